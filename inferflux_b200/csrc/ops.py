@@ -165,7 +165,8 @@ class CudaKernels:
                    "ifx_rmsnorm_pair", "ifx_gate_mul", "ifx_gated_groupnorm", "ifx_pair_combine", "ifx_residual_add_vectors",
                    "ifx_attention_prefill_tcgen05_sink", "ifx_attention_prefill_bf16_sink", "ifx_attention_decode_bf16_sink",
                    "ifx_norm_of_sum", "ifx_row_norm_rope_append", "ifx_rotate_rows", "ifx_gated_scan", "ifx_decay_scan_rate",
-                   "ifx_geglu_mul", "ifx_gemm_skinny_geglu", "ifx_gemm_tcgen05_geglu", "ifx_relu2", "ifx_silu_columns"):
+                   "ifx_geglu_mul", "ifx_gemm_skinny_geglu", "ifx_gemm_tcgen05_geglu", "ifx_relu2", "ifx_silu_columns", "ifx_moe_stream",
+                   "ifx_moe_stream_slices"):
             getattr(self.lib, fn).restype = ctypes.c_int
         self.lib.ifx_delta_rule_scratch_floats.restype = ctypes.c_longlong
         self.lib.ifx_sample_scratch_bytes.restype = ctypes.c_longlong
@@ -1413,9 +1414,11 @@ class CudaKernels:
             _need(h.is_contiguous() and w_up.dtype == h.dtype and w_down.dtype == h.dtype and w_up.is_contiguous()
                   and w_down.is_contiguous() and tuple(w_up.shape) == (experts, 2 * ff, width)
                   and tuple(w_down.shape) == (experts, width, ff), "moe_experts: stacked expert weights in the activations' dtype")
-            if (h.dtype == torch.bfloat16 and T * top >= self.MOE_TILES_MIN_PAIRS and width % 8 == 0 and ff % 8 == 0
-                    and h.data_ptr() % 16 == 0 and os.environ.get("INFERFLUX_B200_MOE_TILES", "1") != "0"):
-                return self._moe_experts_tiles(h, w_up, w_down, ids, weights, experts, out_dtype, glu=glu)
+            if self._moe_on_tensor_cores(h, w_up, w_down, ff, width):
+                way = self.moe_kernels(T * top, int(experts), width, ff, True)
+                if way != "tokens":
+                    return (self._moe_experts_tiles if way == "tiles" else self._moe_experts_stream)(
+                        h, w_up, w_down, ids, weights, experts, out_dtype, glu=glu)
             act = torch.empty((T * top, ff), dtype=h.dtype, device=h.device)
             out = torch.empty((T, width), dtype=out_dtype, device=h.device)
             _check(self.lib.ifx_moe_experts_glu(_ptr(h), _ptr(w_up), _ptr(w_down), _ptr(ids), _ptr(weights), _ptr(act), _ptr(out),
@@ -1428,9 +1431,11 @@ class CudaKernels:
         _need(h.is_contiguous() and (not experts or (w_up.dtype == h.dtype and w_down.dtype == h.dtype and w_up.is_contiguous()
               and w_down.is_contiguous() and tuple(w_up.shape) == (experts, ff, width) and tuple(w_down.shape) == (experts, width, ff))),
               "moe_experts: stacked expert weights in the activations' dtype")
-        if (experts and h.dtype == torch.bfloat16 and T * top >= self.MOE_TILES_MIN_PAIRS and width % 8 == 0 and ff % 8 == 0
-                and h.data_ptr() % 16 == 0 and os.environ.get("INFERFLUX_B200_MOE_TILES", "1") != "0"):
-            return self._moe_experts_tiles(h, w_up, w_down, ids, weights, experts, out_dtype)
+        if experts and self._moe_on_tensor_cores(h, w_up, w_down, ff, width):
+            way = self.moe_kernels(T * top, int(experts), width, ff, False)
+            if way != "tokens":
+                return (self._moe_experts_tiles if way == "tiles" else self._moe_experts_stream)(
+                    h, w_up, w_down, ids, weights, experts, out_dtype)
         act = torch.empty((T * top, ff), dtype=h.dtype, device=h.device)
         out = torch.empty((T, width), dtype=out_dtype, device=h.device)
         _check(self.lib.ifx_moe_experts(_ptr(h), _ptr(w_up if experts else None), _ptr(w_down if experts else None), _ptr(ids),
@@ -1439,8 +1444,50 @@ class CudaKernels:
         self.launches += 2 if experts else 1
         return out
 
-    # From this many (token, choice) pairs on, the experts run as sorted 128-row tiles on the tensor cores.
-    MOE_TILES_MIN_PAIRS = 512
+    # Which kernels make the experts of a bfloat16 step, by the number of (token, choice) pairs.  Measured on a B200 (us; per
+    # token / every chosen expert's weights once / sorted 128-row tiles; 16 experts, four a token):
+    #   1,536 x 2,240 gated   1 token 57 / 46 / 51, 8: 107 / 81 / 92, 24: 240 / 81 / 95, 48: 426 / 93 / 95, 64: 549 / 107 / 95
+    #   1,536 x 3,328         1 token 56 / 46 / 59, 8: 103 / 82 / 91, 24: 227 / 84 / 94, 64: 483 / 89 / 94
+    #   3,584 x 4,736 gated   1 token 150 / 109 / 110, 8: 514 / 312 / 299, 24: 1,100 / 329 / 323, 64: 2,426 / 392 / 321
+    #   512 x 512 gated       1 token 8.5 / 18 / 24, 24: 15 / 19 / 25, 32: 21 / 20 / 25
+    # The tiles are the better once an expert has a dozen tokens (their rows then are not mostly padding, and the stream's
+    # gathering grows), or once its matrices are large enough to keep every SM at whole tiles; work of a few megabytes ends
+    # before the other two have filled their pipelines.
+    MOE_TILES_MIN_PAIRS = 192
+    MOE_TILES_LARGE_EXPERT = 1 << 23
+    MOE_TOKENS_MAX_WORK = 40_000_000
+    MOE_STREAM_MAX_PAIRS = 512
+
+    @classmethod
+    def moe_kernels(cls, pairs, experts, width, ff, gated):
+        """"tokens", "stream" or "tiles"."""
+        if pairs < cls.MOE_STREAM_MAX_PAIRS and pairs * ff * width * (3 if gated else 2) < cls.MOE_TOKENS_MAX_WORK:
+            return "tokens"
+        if pairs >= cls.MOE_TILES_MIN_PAIRS or (ff * width >= cls.MOE_TILES_LARGE_EXPERT and pairs >= 2 * experts):
+            return "tiles"
+        return "stream"
+
+    @staticmethod
+    def _moe_on_tensor_cores(h, w_up, w_down, ff, width):
+        return (h.shape[0] > 0 and h.dtype == torch.bfloat16 and width % 8 == 0 and ff % 8 == 0 and h.data_ptr() % 16 == 0
+                and w_up.data_ptr() % 16 == 0 and w_down.data_ptr() % 16 == 0
+                and os.environ.get("INFERFLUX_B200_MOE_TILES", "1") != "0")
+
+    def _moe_experts_stream(self, h, w_up, w_down, ids, weights, experts, out_dtype, glu=None):
+        """bfloat16, few tokens: every chosen expert's weights once through the tensor cores (csrc/moe_stream_tcgen05.cu)."""
+        T, width = h.shape
+        top, ff = ids.shape[1], w_up.shape[1] // (2 if glu is not None else 1)
+        act = torch.empty((T * top, ff), dtype=torch.bfloat16, device=h.device)
+        slices = int(self.lib.ifx_moe_stream_slices(ff))
+        y = torch.empty((slices, T * top, width), dtype=torch.float32, device=h.device)
+        out = torch.empty((T, width), dtype=out_dtype, device=h.device)
+        limit, slope, offset = glu if glu is not None else (0.0, 0.0, 0.0)
+        _check(self.lib.ifx_moe_stream(_ptr(h), _ptr(w_up), _ptr(w_down), _ptr(ids), _ptr(weights), _ptr(act), _ptr(y), _ptr(out),
+                                       T, top, int(experts), width, ff, _DT[out_dtype], int(glu is not None), ctypes.c_float(limit),
+                                       ctypes.c_float(slope), ctypes.c_float(offset), _ptr(self.error_flag), _stream()),
+               "moe experts (stream)")
+        self.launches += 3
+        return out
 
     def _moe_experts_tiles(self, h, w_up, w_down, ids, weights, experts, out_dtype, glu=None):
         """bfloat16, many tokens: pairs sorted by expert into stretches of whole 128-row tiles, two grouped tcgen05
