@@ -166,9 +166,12 @@ class CudaKernels:
                    "ifx_attention_prefill_tcgen05_sink", "ifx_attention_prefill_bf16_sink", "ifx_attention_decode_bf16_sink",
                    "ifx_norm_of_sum", "ifx_row_norm_rope_append", "ifx_rotate_rows", "ifx_gated_scan", "ifx_decay_scan_rate",
                    "ifx_geglu_mul", "ifx_gemm_skinny_geglu", "ifx_gemm_tcgen05_geglu", "ifx_relu2", "ifx_silu_columns", "ifx_moe_stream",
-                   "ifx_moe_stream_slices"):
+                   "ifx_moe_stream_slices", "ifx_chunk_scan_supports", "ifx_chunk_decay_scan", "ifx_chunk_wkv_scan", "ifx_wkv_norm"):
             getattr(self.lib, fn).restype = ctypes.c_int
         self.lib.ifx_delta_rule_scratch_floats.restype = ctypes.c_longlong
+        self.lib.ifx_chunk_scan_scratch_floats.restype = ctypes.c_longlong
+        # long spans of a bfloat16 run's recurrences by stretches of 64 tokens (0: token after token, for comparisons)
+        self.chunk_scans = os.environ.get("INFERFLUX_B200_CHUNK_SCANS", "1") != "0"
         self.lib.ifx_sample_scratch_bytes.restype = ctypes.c_longlong
         self.lib.ifx_latent_attention_mma_workspace.restype = ctypes.c_longlong
         # latent attention on the tensor-core tiles (0: the per-token kernel, for comparisons)
@@ -1331,6 +1334,16 @@ class CudaKernels:
         self.launches += 1
         return out
 
+    # From spans of this many tokens on, a bfloat16 run takes its recurrences by stretches of 64 tokens (csrc/chunk_scan.cu).
+    CHUNK_SCAN_MIN_SPAN = 128
+
+    def _scans_by_chunks(self, dtype, ctx, heads, dk, dv, *rows):
+        """Whether a recurrence goes by stretches of tokens: long spans, sizes the kernels are made for, rows on 16-byte
+        boundaries, and a bfloat16 run (the order of the sums then depends on how a span was cut into steps)."""
+        return (self.chunk_scans and dtype is torch.bfloat16 and ctx.max_span >= self.CHUNK_SCAN_MIN_SPAN
+                and self.lib.ifx_chunk_scan_supports(ctx.num_requests, int(heads), int(dk), int(dv))
+                and all(t.data_ptr() % 16 == 0 and (t.dim() < 2 or t.stride(0) % 4 == 0) for t in rows))
+
     def wkv_scan(self, r, k, v, w_raw, g, w0, u, norm_w, eps, heads, dim, state, prev_offset, x, ctx, out_dtype):
         """The recurrence of csrc/wkv.cu over every request's tokens.  r, k, v, w_raw, g: float32 [T, heads * dim], each
         contiguous or a column block of a wider matrix (all with the same distance between rows);
@@ -1350,6 +1363,17 @@ class CudaKernels:
               "wkv_scan: the state does not fit the sizes")
         scratch = torch.empty((T, HD), dtype=torch.float32, device=r.device)
         y = torch.empty((T, HD), dtype=out_dtype, device=r.device)
+        if self._scans_by_chunks(out_dtype, ctx, heads, dim, dim, r, k, v, w_raw, w0, u):
+            room = torch.empty(int(self.lib.ifx_chunk_scan_scratch_floats(T, ctx.num_requests, heads, dim, dim, 1)), dtype=torch.float32,
+                               device=r.device)
+            _check(self.lib.ifx_chunk_wkv_scan(
+                _ptr(r), _ptr(k), _ptr(v), _ptr(w_raw), _ptr(w0), _ptr(u), _ptr(state), ctypes.c_void_p(state.data_ptr() + 4 * prev_offset),
+                ctypes.c_longlong(state.shape[1]), _ptr(x), C, _ptr(ctx.cu_seqlens), _ptr(ctx.req_slot), _ptr(scratch),
+                ctx.num_requests, T, heads, dim, ld, ld_w, _ptr(room), _stream()), "wkv_scan (stretches)")
+            _check(self.lib.ifx_wkv_norm(_ptr(scratch), _ptr(g), _ptr(norm_w), ctypes.c_float(eps), _ptr(y), T, heads, dim, ld,
+                                         _DT[out_dtype], _stream()), "wkv_norm")
+            self.launches += 4
+            return y
         _check(self.lib.ifx_wkv_scan(
             _ptr(r), _ptr(k), _ptr(v), _ptr(w_raw), _ptr(g), _ptr(w0), _ptr(u), _ptr(norm_w), ctypes.c_float(eps),
             _ptr(state), ctypes.c_void_p(state.data_ptr() + 4 * prev_offset), ctypes.c_longlong(state.shape[1]), _ptr(x), C,
@@ -1605,6 +1629,17 @@ class CudaKernels:
             _need(vec is None or (vec.dtype == torch.float32 and vec.numel() == heads and vec.is_contiguous()),
                   "decay_scan: per-head vectors are float32 [heads]")
         out = torch.empty((T, heads * dv), dtype=torch.float32, device=q.device)
+        if self._scans_by_chunks(getattr(ctx, "dtype", None), ctx, heads, dk, dv, q, k, v, *([raw] if mode == 0 else [])):
+            room = torch.empty(int(self.lib.ifx_chunk_scan_scratch_floats(T, ctx.num_requests, heads, dk, dv, int(mode == 0))),
+                               dtype=torch.float32, device=q.device)
+            _check(self.lib.ifx_chunk_decay_scan(
+                *self._rows_f32(q, "decay_scan q"), *self._rows_f32(k, "decay_scan k"), *self._rows_f32(v, "decay_scan v"),
+                *(self._rows_f32(raw, "decay_scan raw") if raw is not None else (_ptr(None), _LL(0))), _ptr(state),
+                ctypes.c_longlong(state.stride(0)), _ptr(ctx.req_slot), _ptr(ctx.cu_seqlens), _ptr(out), _ptr(step_bias),
+                _ptr(log_rate), _ptr(skip), ctx.num_requests, T, int(heads), int(groups), int(dk), int(dv), mode,
+                ctypes.c_float(tau), ctypes.c_float(q_scale), _ptr(room), _ptr(rate), _stream()), "decay_scan (stretches)")
+            self.launches += 3
+            return out
         scratch = None                                     # steps with long spans make their decays in a pass of their own
         if ctx.max_span >= 64 and mode != 2:
             scratch = torch.empty(T * (heads * dk if mode == 0 else 2 * heads), dtype=torch.float32, device=q.device)

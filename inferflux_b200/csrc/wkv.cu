@@ -340,4 +340,19 @@ int ifx_wkv_scan(const float* r, const float* k, const float* v, const float* w_
   return 0;
 }
 
+// y = o / sqrt(mean(o^2) + eps) per head * norm_w * silu(g): what the scan does behind its sums, for sums made elsewhere.
+int ifx_wkv_norm(const float* o, const float* g, const float* norm_w, float eps, void* y, int num_tokens, int H, int D, int ld,
+                 int out_dtype, cudaStream_t stream) {
+  if (num_tokens <= 0) return 0;
+  if (H <= 0 || D <= 0 || ld < H * D) return IFX_E_BADARG;
+  const long long items = (long long)num_tokens * H;
+  const unsigned blocks = (unsigned)((items + 7) / 8);
+  if (out_dtype == IFX_DT_F32) wkv_norm_kernel<float><<<blocks, 256, 0, stream>>>(o, g, norm_w, eps, (float*)y, items, H, D, ld);
+  else if (out_dtype == IFX_DT_BF16)
+    wkv_norm_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(o, g, norm_w, eps, (__nv_bfloat16*)y, items, H, D, ld);
+  else return IFX_E_DTYPE;
+  IFX_CHECK_LAUNCH();
+  return 0;
+}
+
 }  // extern "C"
