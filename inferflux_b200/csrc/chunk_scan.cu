@@ -22,9 +22,11 @@
 //
 // The order of the sums depends on where a span is cut into steps, so the float32 run keeps the scans.
 //
-// Bound: the tensor and issue pipes of chunk_local (a third each of splitting operands, mma.sync and decays); the states
-// go through L2 twice (26 MB at 2,048 tokens of 12 heads of 128 x 128).  Measured, us of the whole recurrence, scan -> this:
-// IFX_FILL
+// Bound: issue slots and shared-memory reads of chunk_local, two blocks an SM; mma.sync itself takes a fifth of the time, and the
+// states go through L2 twice (26 MB at 2,048 tokens of 12 heads of 128 x 128).  A warp's tile is 32 x 16, so that an operand
+// is split and read by few warps.  Measured, us, scan -> this (local + carry + reach): 12 heads of 128 x 128 with a constant
+// decay, 1,901 tokens of two prompts 343 -> 96 (58 + 11 + 27); wkv, 24 heads of 64, 2,048 tokens 522 -> 122 (71 + 10 + 19 and
+// its norm).  At 128 tokens 41 -> 33 for either; at 64 the scan is the faster.
 #include "chunk_scan.cuh"
 
 namespace ifx {
@@ -310,76 +312,79 @@ __global__ void __launch_bounds__(256) chunk_local_kernel(const ChunkArgs a) {
     }
   }
   __syncthreads();
-  {                                                        // o: a warp's eight value channels, all tokens
-    float acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
+  {                                                        // o: a warp's 16 value channels, the first and last or the middle 16s of tokens
+    const int m0 = warp >> 2, c0 = (warp & 3) * 16;        // rows of m0 and 3 - m0: ten steps of eight tokens either way
+    float acc[2][2][4] = {};
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks) {
-      FragB fb;
-      load_b_columns(fb, v_s + ks * 8 * kPitchV + warp * 8, kPitchV, lane);
+      if (ks >= 2 * (4 - m0)) break;
+      FragB fb[2];
+      load_b_columns(fb[0], v_s + ks * 8 * kPitchV + c0, kPitchV, lane);
+      load_b_columns(fb[1], v_s + ks * 8 * kPitchV + c0 + 8, kPitchV, lane);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (ks < 2 * (i + 1)) {
+      for (int i = 0; i < 2; ++i) {
+        const int m = i == 0 ? m0 : 3 - m0;
+        if (ks < 2 * (m + 1)) {
           FragA fa;
-          load_a_single(fa, a_s + i * kSub * kPitchA + ks * 8, kPitchA, lane);
-          mma_split(acc[i], fa, fb);
+          load_a_single(fa, a_s + m * kSub * kPitchA + ks * 8, kPitchA, lane);
+          mma_split(acc[i][0], fa, fb[0]);
+          mma_split(acc[i][1], fa, fb[1]);
         }
       }
     }
-    const int c = warp * 8 + 2 * (lane & 3);
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int t = i * kSub + half * 8 + (lane >> 2);
-        if (t < n) {
-          float2 o = make_float2(acc[i][2 * half], acc[i][2 * half + 1]);
-          if (a.skip) {
-            o.x = fmaf(skip, v_s[t * kPitchV + c], o.x);
-            o.y = fmaf(skip, v_s[t * kPitchV + c + 1], o.y);
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          const int t = (i == 0 ? m0 : 3 - m0) * kSub + half * 8 + (lane >> 2), c = c0 + j * 8 + 2 * (lane & 3);
+          if (t < n) {
+            float2 o = make_float2(acc[i][j][2 * half], acc[i][j][2 * half + 1]);
+            if (a.skip) {
+              o.x = fmaf(skip, v_s[t * kPitchV + c], o.x);
+              o.y = fmaf(skip, v_s[t * kPitchV + c + 1], o.y);
+            }
+            *reinterpret_cast<float2*>(out + t * out_row + c) = o;
           }
-          *reinterpret_cast<float2*>(out + t * out_row + c) = o;
         }
-      }
   }
-  // what the stretch adds to the state: value channels as rows, a warp's eight key channels
-  for (int c0 = warp * 8; c0 < DK; c0 += 64) {
-    float acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
-    float rest[4] = {1.0f, 1.0f, 1.0f, 1.0f};              // CHANNEL: decays of the 16s behind the j-th
+  // what the stretch adds to the state: value channels as rows, 32 of them a warp, 16 key channels at a time
+  const int v0 = (warp >> 2) * 32;
+  for (int c0 = (warp & 3) * 16; c0 < DK; c0 += 64) {
+    float acc[2][2][4] = {};
+    float rest[2][4];                                      // CHANNEL: decays of the 16s behind the j-th
     if (L::CHANNEL) {
 #pragma unroll
-      for (int j = 2; j >= 0; --j) rest[j] = rest[j + 1] * small[(j + 1) * DK + c0 + (lane >> 2)];
+      for (int x = 0; x < 2; ++x) {
+        rest[x][3] = 1.0f;
+#pragma unroll
+        for (int j = 2; j >= 0; --j) rest[x][j] = rest[x][j + 1] * small[(j + 1) * DK + c0 + 8 * x + (lane >> 2)];
+      }
     }
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks) {
-      const float* at = k_s + (ks * 8 + (lane & 3)) * PK + c0 + (lane >> 2);
-      float b0 = at[0], b1 = at[4 * PK];
-      if (L::CHANNEL) {
-        b0 *= rest[ks >> 1];
-        b1 *= rest[ks >> 1];
-      } else {
-        b0 *= small[2 * kChunk + ks * 8 + (lane & 3)];
-        b1 *= small[2 * kChunk + ks * 8 + (lane & 3) + 4];
-      }
-      FragB fb;
-      fb.v[0].set(b0);
-      fb.v[1].set(b1);
+      FragA fa[2];
+      load_a_columns(fa[0], v_s + ks * 8 * kPitchV + v0, kPitchV, lane);
+      load_a_columns(fa[1], v_s + ks * 8 * kPitchV + v0 + 16, kPitchV, lane);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        FragA fa;
-        load_a_columns(fa, v_s + ks * 8 * kPitchV + i * 16, kPitchV, lane);
-        mma_split(acc[i], fa, fb);
+      for (int x = 0; x < 2; ++x) {
+        const float* at = k_s + (ks * 8 + (lane & 3)) * PK + c0 + 8 * x + (lane >> 2);
+        FragB fb;
+        fb.v[0].set(at[0] * (L::CHANNEL ? rest[x][ks >> 1] : small[2 * kChunk + ks * 8 + (lane & 3)]));
+        fb.v[1].set(at[4 * PK] * (L::CHANNEL ? rest[x][ks >> 1] : small[2 * kChunk + ks * 8 + (lane & 3) + 4]));
+        mma_split(acc[0][x], fa[0], fb);
+        mma_split(acc[1][x], fa[1], fb);
       }
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float* to = local + (size_t)(i * 16 + (lane >> 2)) * DK + c0 + 2 * (lane & 3);
-      *reinterpret_cast<float2*>(to) = make_float2(acc[i][0], acc[i][1]);
-      *reinterpret_cast<float2*>(to + 8 * DK) = make_float2(acc[i][2], acc[i][3]);
-    }
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        float* to = local + (size_t)(v0 + i * 16 + (lane >> 2)) * DK + c0 + 8 * x + 2 * (lane & 3);
+        *reinterpret_cast<float2*>(to) = make_float2(acc[i][x][0], acc[i][x][1]);
+        *reinterpret_cast<float2*>(to + 8 * DK) = make_float2(acc[i][x][2], acc[i][x][3]);
+      }
   }
 }
 
@@ -471,31 +476,34 @@ __global__ void __launch_bounds__(256) chunk_reach_kernel(const ChunkArgs a) {
     }
     return;
   }
-  float acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
+  const int t0 = (warp >> 2) * 32, c0 = (warp & 3) * 16;   // a warp's 32 tokens and 16 value channels
+  float acc[2][2][4] = {};
 #pragma unroll 4
   for (int kk = 0; kk < DK; kk += 8) {
-    FragB fb;
-    load_b_rows(fb, s_s + warp * 8 * PK + kk, PK, lane);
+    FragB fb[2];
+    load_b_rows(fb[0], s_s + c0 * PK + kk, PK, lane);
+    load_b_rows(fb[1], s_s + (c0 + 8) * PK + kk, PK, lane);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < 2; ++i) {
       FragA fa;
-      load_a_rows(fa, q_s + i * 16 * PK + kk, PK, lane);
-      mma_split(acc[i], fa, fb);
+      load_a_rows(fa, q_s + (t0 + i * 16) * PK + kk, PK, lane);
+      mma_split(acc[i][0], fa, fb[0]);
+      mma_split(acc[i][1], fa, fb[1]);
     }
   }
-  const int c = warp * 8 + 2 * (lane & 3);
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
-      const int t = i * 16 + half * 8 + (lane >> 2);
+      const int t = t0 + i * 16 + half * 8 + (lane >> 2);
       if (t < n) {
         const float f = CHANNEL ? 1.0f : a.reach[(size_t)(first + t) * a.heads + h];
-        float2* to = reinterpret_cast<float2*>(out + t * out_row + c);
-        const float2 o = *to;
-        *to = make_float2(fmaf(f, acc[i][2 * half], o.x), fmaf(f, acc[i][2 * half + 1], o.y));
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          float2* to = reinterpret_cast<float2*>(out + t * out_row + c0 + j * 8 + 2 * (lane & 3));
+          const float2 o = *to;
+          *to = make_float2(fmaf(f, acc[i][j][2 * half], o.x), fmaf(f, acc[i][j][2 * half + 1], o.y));
+        }
       }
     }
 }

@@ -11,17 +11,14 @@ constexpr int kSub = 16;                   // tokens within which decays are mul
 constexpr int kPitchV = 64 + 8;            // floats from a row of 64 to the next: the reads below meet every bank once
 constexpr int kPitchA = 64 + 4;
 
-__device__ __forceinline__ uint32_t to_tf32(float x) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return r;
-}
-// A float32 as the sum of two numbers of 11 bits each: what is left out is below 2^-23 of it.
+// A float32 as the sum of two numbers of 11 bits each, both rounded to the nearest: what is left out is below 2^-22 of it.  By
+// integer additions on the bits, since conversions run at a fraction of their rate; the product does not look at the 13 lowest
+// bits of an operand, so the small part's stay where they are.
 struct Split {
   uint32_t hi, lo;
   __device__ __forceinline__ void set(float x) {
-    hi = to_tf32(x);
-    lo = to_tf32(x - __uint_as_float(hi));
+    hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
+    lo = __float_as_uint(x - __uint_as_float(hi)) + 0x1000u;
   }
 };
 __device__ __forceinline__ void mma_tf32(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -31,7 +28,7 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], uint32_t a0, uint32_t a1
 }
 struct FragA { Split v[4]; };              // 16 rows x 8 of the inner size
 struct FragB { Split v[2]; };              // 8 columns x 8 of the inner size
-// c += a b with both operands split; the product of the two small parts (below 2^-23 of the whole) is left out.
+// c += a b with both operands split; the product of the two small parts (below 2^-22 of the whole) is left out.
 __device__ __forceinline__ void mma_split(float (&c)[4], const FragA& a, const FragB& b) {
   mma_tf32(c, a.v[0].lo, a.v[1].lo, a.v[2].lo, a.v[3].lo, b.v[0].hi, b.v[1].hi);
   mma_tf32(c, a.v[0].hi, a.v[1].hi, a.v[2].hi, a.v[3].hi, b.v[0].lo, b.v[1].lo);
