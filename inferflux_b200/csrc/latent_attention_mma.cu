@@ -328,17 +328,23 @@ __global__ void __launch_bounds__(256) latent_merge_kernel(const float* __restri
   const float* po = part_o + (size_t)row * rank + c;
   const size_t step = (size_t)total_rows * rank;
   float acc = 0.0f;
-  int s = 0;
+  int s = 0;                                                           // a part of weight zero may not have been written
+  auto part = [&](int i) { return w_s[i] != 0.0f ? po[(size_t)i * step] : 0.0f; };
   for (; s + 4 <= splits; s += 4) {
-    const float a0 = po[(size_t)s * step], a1 = po[(size_t)(s + 1) * step], a2 = po[(size_t)(s + 2) * step],
-                a3 = po[(size_t)(s + 3) * step];
+    const float a0 = part(s), a1 = part(s + 1), a2 = part(s + 2), a3 = part(s + 3);
     acc = fmaf(a0, w_s[s], acc);
     acc = fmaf(a1, w_s[s + 1], acc);
     acc = fmaf(a2, w_s[s + 2], acc);
     acc = fmaf(a3, w_s[s + 3], acc);
   }
-  for (; s < splits; ++s) acc = fmaf(po[(size_t)s * step], w_s[s], acc);
+  for (; s < splits; ++s) acc = fmaf(part(s), w_s[s], acc);
   out[(size_t)row * rank + c] = __float2bfloat16_rn(acc * inv_s);
+}
+
+int launch_latent_merge(const float* part_o, const float2* part_ml, const float* sinks, __nv_bfloat16* out, int total_rows, int heads,
+                        int rank, int splits, const float* gate, cudaStream_t stream) {
+  latent_merge_kernel<<<total_rows, 256, 0, stream>>>(part_o, part_ml, sinks, out, total_rows, heads, rank, splits, gate);
+  return (int)cudaGetLastError();
 }
 
 }  // namespace ifx
@@ -402,11 +408,7 @@ int ifx_latent_attention_mma_rot(const void* ql, const void* pool, const int* bl
   }
 #undef IFX_LAUNCH
   IFX_CHECK_LAUNCH();
-  if (splits > 1) {
-    latent_merge_kernel<<<total_rows, 256, 0, stream>>>(
-        part_o, part_ml, sinks, (__nv_bfloat16*)out, total_rows, heads, rank, splits, gate);
-    IFX_CHECK_LAUNCH();
-  }
+  if (splits > 1) return launch_latent_merge(part_o, part_ml, sinks, (__nv_bfloat16*)out, total_rows, heads, rank, splits, gate, stream);
   return 0;
 }
 

@@ -166,7 +166,8 @@ class CudaKernels:
                    "ifx_attention_prefill_tcgen05_sink", "ifx_attention_prefill_bf16_sink", "ifx_attention_decode_bf16_sink",
                    "ifx_norm_of_sum", "ifx_row_norm_rope_append", "ifx_rotate_rows", "ifx_gated_scan", "ifx_decay_scan_rate",
                    "ifx_geglu_mul", "ifx_gemm_skinny_geglu", "ifx_gemm_tcgen05_geglu", "ifx_relu2", "ifx_silu_columns", "ifx_moe_stream",
-                   "ifx_moe_stream_slices", "ifx_chunk_scan_supports", "ifx_chunk_decay_scan", "ifx_chunk_wkv_scan", "ifx_wkv_norm"):
+                   "ifx_moe_stream_slices", "ifx_chunk_scan_supports", "ifx_chunk_decay_scan", "ifx_chunk_wkv_scan", "ifx_wkv_norm",
+                   "ifx_latent_decode", "ifx_latent_decode_supports", "ifx_latent_decode_stretch"):
             getattr(self.lib, fn).restype = ctypes.c_int
         self.lib.ifx_delta_rule_scratch_floats.restype = ctypes.c_longlong
         self.lib.ifx_chunk_scan_scratch_floats.restype = ctypes.c_longlong
@@ -176,6 +177,8 @@ class CudaKernels:
         self.lib.ifx_latent_attention_mma_workspace.restype = ctypes.c_longlong
         # latent attention on the tensor-core tiles (0: the per-token kernel, for comparisons)
         self.latent_tiles = os.environ.get("INFERFLUX_B200_LATENT_TILES", "1") != "0"
+        # decoded tokens on the kernel made for them (0: the tiles of prompt portions, for comparisons)
+        self.latent_decode = os.environ.get("INFERFLUX_B200_LATENT_DECODE", "1") != "0"
         with torch.cuda.device(self.device):
             _check(self.lib.ifx_cublas_init(), "cublas init")
         if os.environ.get("INFERFLUX_B200_CARVEOUT", "") != "":    # for measurements: -1 leaves the split to the driver
@@ -1277,7 +1280,15 @@ class CudaKernels:
         win = 0 if window is None else int(window)
         splits = 1
         max_keys = int(ctx.max_kv_len if not win else min(win, ctx.max_kv_len))
-        if ctx.max_span == 1:                              # decoded tokens only: cut the keys so that the SMs fill
+        decode = (ctx.max_span == 1 and self.latent_decode and self.lib.ifx_latent_decode_supports(rank, int(rot), cache.page_size)
+                  and ql.data_ptr() % 16 == 0 and kv.data_ptr() % 16 == 0)
+        if decode:                                         # decoded tokens only, a kernel of their own
+            stretch = int(self.lib.ifx_latent_decode_stretch(T, heads, max_keys))
+            splits = -(-(max_keys + 15) // stretch)        # (a window may begin inside a tile of 16 keys)
+            decode = splits <= 64
+        if decode:
+            pass
+        elif ctx.max_span == 1:                            # cut the keys so that the SMs fill
             blocks = num_items * -(-heads // 64)                 # about four warps a SM, at least two key tiles each
             splits = max(1, min(592 // max(1, blocks), max_keys // 64, 64))
         else:
@@ -1292,10 +1303,16 @@ class CudaKernels:
             ws = torch.empty(int(self.lib.ifx_latent_attention_mma_workspace(T * heads, rank, splits)), dtype=torch.uint8,
                              device=q_rows.device)
         olat = torch.empty((T, heads * rank), dtype=torch.bfloat16, device=q_rows.device)
-        _check(self.lib.ifx_latent_attention_mma_rot(
-            _ptr(ql), _ptr(kv), _ptr(table), _ptr(items), num_items, int(min(self.LATENT_TILE, ctx.max_span)), _ptr(sinks),
-            _ptr(olat), _ptr(ws), T, heads, rank, int(rot), cache.page_size, table.shape[1], kv.shape[0], win,
-            ctypes.c_float(scale), splits, _ptr(head_gate), _stream()), "latent_attention (tiles)")
+        if decode:
+            _check(self.lib.ifx_latent_decode(
+                _ptr(ql), _ptr(kv), _ptr(table), _ptr(items), num_items, _ptr(sinks), _ptr(olat), _ptr(ws), T, heads, rank, int(rot),
+                cache.page_size, table.shape[1], kv.shape[0], win, ctypes.c_float(scale), stretch, splits, _ptr(head_gate),
+                _ptr(self.error_flag), _stream()), "latent_attention (decode)")
+        else:
+            _check(self.lib.ifx_latent_attention_mma_rot(
+                _ptr(ql), _ptr(kv), _ptr(table), _ptr(items), num_items, int(min(self.LATENT_TILE, ctx.max_span)), _ptr(sinks),
+                _ptr(olat), _ptr(ws), T, heads, rank, int(rot), cache.page_size, table.shape[1], kv.shape[0], win,
+                ctypes.c_float(scale), splits, _ptr(head_gate), _stream()), "latent_attention (tiles)")
         self.launches += 1 + int(splits > 1)
         return self.linear_heads(olat, w_uv, heads, rank, vdim, w_is_nk=True)               # [T, heads * vdim]
 
