@@ -167,7 +167,8 @@ class CudaKernels:
                    "ifx_norm_of_sum", "ifx_row_norm_rope_append", "ifx_rotate_rows", "ifx_gated_scan", "ifx_decay_scan_rate",
                    "ifx_geglu_mul", "ifx_gemm_skinny_geglu", "ifx_gemm_tcgen05_geglu", "ifx_relu2", "ifx_silu_columns", "ifx_moe_stream",
                    "ifx_moe_stream_slices", "ifx_chunk_scan_supports", "ifx_chunk_decay_scan", "ifx_chunk_wkv_scan", "ifx_wkv_norm",
-                   "ifx_latent_decode", "ifx_latent_decode_supports", "ifx_latent_decode_stretch"):
+                   "ifx_latent_decode", "ifx_latent_decode_supports", "ifx_latent_decode_stretch",
+                   "ifx_latent_prompt", "ifx_latent_prompt_supports"):
             getattr(self.lib, fn).restype = ctypes.c_int
         self.lib.ifx_delta_rule_scratch_floats.restype = ctypes.c_longlong
         self.lib.ifx_chunk_scan_scratch_floats.restype = ctypes.c_longlong
@@ -179,6 +180,8 @@ class CudaKernels:
         self.latent_tiles = os.environ.get("INFERFLUX_B200_LATENT_TILES", "1") != "0"
         # decoded tokens on the kernel made for them (0: the tiles of prompt portions, for comparisons)
         self.latent_decode = os.environ.get("INFERFLUX_B200_LATENT_DECODE", "1") != "0"
+        # prompt portions on the tcgen05 kernel (0: the mma.sync tiles, for comparisons)
+        self.latent_prompt = os.environ.get("INFERFLUX_B200_LATENT_PROMPT", "1") != "0"
         with torch.cuda.device(self.device):
             _check(self.lib.ifx_cublas_init(), "cublas init")
         if os.environ.get("INFERFLUX_B200_CARVEOUT", "") != "":    # for measurements: -1 leaves the split to the driver
@@ -1130,6 +1133,7 @@ class CudaKernels:
         return out
 
     # -------------------------------------------------------- latent attention
+    LATENT_PROMPT_MIN_ROWS = 64
     LATENT_TILE = 64           # tokens per work item of the tiled latent attention kernel
 
     def latent_attention_sections(self, ctx):
@@ -1286,8 +1290,15 @@ class CudaKernels:
             stretch = int(self.lib.ifx_latent_decode_stretch(T, heads, max_keys))
             splits = -(-(max_keys + 15) // stretch)        # (a window may begin inside a tile of 16 keys)
             decode = splits <= 64
+        # spans of which a block's 128 rows (a token with all its heads) are a good part: the tcgen05 kernel
+        prompt = (not decode and self.latent_prompt and min(n for _s, n in ctx.spans) * heads >= self.LATENT_PROMPT_MIN_ROWS
+                  and self.lib.ifx_latent_prompt_supports(rank, int(rot), cache.page_size)
+                  and ql.data_ptr() % 16 == 0 and kv.data_ptr() % 16 == 0)
         if decode:
             pass
+        elif prompt:                                       # a block an SM: cut the keys while there are fewer blocks than SMs
+            blocks = sum(-(-n * heads // 128) for _s, n in ctx.spans)
+            splits = max(1, min(148 // blocks, -(-max_keys // 128) // 2, 16))
         elif ctx.max_span == 1:                            # cut the keys so that the SMs fill
             blocks = num_items * -(-heads // 64)                 # about four warps a SM, at least two key tiles each
             splits = max(1, min(592 // max(1, blocks), max_keys // 64, 64))
@@ -1308,6 +1319,11 @@ class CudaKernels:
                 _ptr(ql), _ptr(kv), _ptr(table), _ptr(items), num_items, _ptr(sinks), _ptr(olat), _ptr(ws), T, heads, rank, int(rot),
                 cache.page_size, table.shape[1], kv.shape[0], win, ctypes.c_float(scale), stretch, splits, _ptr(head_gate),
                 _ptr(self.error_flag), _stream()), "latent_attention (decode)")
+        elif prompt:
+            _check(self.lib.ifx_latent_prompt(
+                _ptr(ql), _ptr(kv), _ptr(table), _ptr(items), num_items, int(min(self.LATENT_TILE, ctx.max_span)), _ptr(sinks),
+                _ptr(olat), _ptr(ws), T, heads, rank, int(rot), cache.page_size, table.shape[1], kv.shape[0], win,
+                ctypes.c_float(scale), splits, _ptr(head_gate), _ptr(self.error_flag), _stream()), "latent_attention (prompt)")
         else:
             _check(self.lib.ifx_latent_attention_mma_rot(
                 _ptr(ql), _ptr(kv), _ptr(table), _ptr(items), num_items, int(min(self.LATENT_TILE, ctx.max_span)), _ptr(sinks),
