@@ -540,6 +540,22 @@ static int run_chunks(const ChunkArgs& a, int dk, int mode, int chunks, cudaStre
   return launch_chunks<128, CHUNK_WKV>(a, chunks, stream);
 }
 
+// The last of the three alone, for delta_chunks.cu: heads of 64 x 64, `reach` [T, heads 64] and the states as chunk_carry leaves them.
+int launch_chunk_reach_64(const float* reach, const float* local, float* out, const int* cu_seqlens, int requests, int heads, int chunks,
+                          cudaStream_t stream) {
+  ChunkArgs a = {};
+  a.reach = const_cast<float*>(reach);
+  a.local = const_cast<float*>(local);
+  a.out = out;
+  a.cu_seqlens = cu_seqlens;
+  a.requests = requests;
+  a.heads = a.groups = heads;
+  a.dv = 64;
+  chunk_reach_kernel<64, true><<<dim3(chunks, heads, 1), 256, 2 * kChunk * (64 + 8) * sizeof(float), stream>>>(a);
+  IFX_CHECK_LAUNCH();
+  return 0;
+}
+
 static bool rows_fit(const void* p, long long stride) { return stride % 4 == 0 && reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 
 }  // namespace ifx

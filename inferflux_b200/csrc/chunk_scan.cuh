@@ -13,7 +13,7 @@ constexpr int kPitchA = 64 + 4;
 
 // A float32 as the sum of two numbers of 11 bits each, both rounded to the nearest: what is left out is below 2^-22 of it.  By
 // integer additions on the bits, since conversions run at a fraction of their rate; the product does not look at the 13 lowest
-// bits of an operand, so the small part's stay where they are.
+// bits of an operand, so the small part's stay where they are.  Finite numbers only: a NaN would be lost.
 struct Split {
   uint32_t hi, lo;
   __device__ __forceinline__ void set(float x) {

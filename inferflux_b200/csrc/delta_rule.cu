@@ -247,6 +247,18 @@ __global__ void delta_finish_kernel(const float* __restrict__ o, const float* __
     y[(size_t)t * HD + h * dim + i] = from_f32<TO>(orow[i] * r * norm_w[h * dim + i] * sigmoid_f(g[i]));
 }
 
+int launch_delta_finish(const float* o, const float* proj, int ld, const float* norm_w, float eps, void* y, int num_tokens, int heads,
+                        int dim, int out_dtype, cudaStream_t stream) {
+  const unsigned blocks = (unsigned)(((long long)num_tokens * heads + 3) / 4);
+  if (out_dtype == IFX_DT_F32)
+    delta_finish_kernel<float><<<blocks, 128, 0, stream>>>(o, proj, ld, norm_w, eps, (float*)y, num_tokens, heads, dim);
+  else if (out_dtype == IFX_DT_BF16)
+    delta_finish_kernel<__nv_bfloat16><<<blocks, 128, 0, stream>>>(o, proj, ld, norm_w, eps, (__nv_bfloat16*)y, num_tokens, heads, dim);
+  else return IFX_E_DTYPE;
+  IFX_CHECK_LAUNCH();
+  return 0;
+}
+
 }  // namespace ifx
 
 using namespace ifx;
@@ -310,14 +322,7 @@ int ifx_delta_rule_scan(const float* proj, int ld, const float* w_raw, const flo
   else IFX_SCAN(32);
 #undef IFX_SCAN
   IFX_CHECK_LAUNCH();
-  if (out_dtype == IFX_DT_F32)
-    delta_finish_kernel<float><<<(unsigned)((items + 3) / 4), 128, 0, stream>>>(o, proj, ld, norm_w, eps, (float*)y, T, heads, dim);
-  else if (out_dtype == IFX_DT_BF16)
-    delta_finish_kernel<__nv_bfloat16><<<(unsigned)((items + 3) / 4), 128, 0, stream>>>(o, proj, ld, norm_w, eps,
-                                                                                       (__nv_bfloat16*)y, T, heads, dim);
-  else return IFX_E_DTYPE;
-  IFX_CHECK_LAUNCH();
-  return 0;
+  return launch_delta_finish(o, proj, ld, norm_w, eps, y, T, heads, dim, out_dtype, stream);
 }
 
 }  // extern "C"

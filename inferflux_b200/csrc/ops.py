@@ -168,10 +168,11 @@ class CudaKernels:
                    "ifx_geglu_mul", "ifx_gemm_skinny_geglu", "ifx_gemm_tcgen05_geglu", "ifx_relu2", "ifx_silu_columns", "ifx_moe_stream",
                    "ifx_moe_stream_slices", "ifx_chunk_scan_supports", "ifx_chunk_decay_scan", "ifx_chunk_wkv_scan", "ifx_wkv_norm",
                    "ifx_latent_decode", "ifx_latent_decode_supports", "ifx_latent_decode_stretch",
-                   "ifx_latent_prompt", "ifx_latent_prompt_supports"):
+                   "ifx_latent_prompt", "ifx_latent_prompt_supports", "ifx_delta_chunks_supports", "ifx_delta_chunks_scan"):
             getattr(self.lib, fn).restype = ctypes.c_int
         self.lib.ifx_delta_rule_scratch_floats.restype = ctypes.c_longlong
         self.lib.ifx_chunk_scan_scratch_floats.restype = ctypes.c_longlong
+        self.lib.ifx_delta_chunks_scratch_floats.restype = ctypes.c_longlong
         # long spans of a bfloat16 run's recurrences by stretches of 64 tokens (0: token after token, for comparisons)
         self.chunk_scans = os.environ.get("INFERFLUX_B200_CHUNK_SCANS", "1") != "0"
         self.lib.ifx_sample_scratch_bytes.restype = ctypes.c_longlong
@@ -1369,6 +1370,11 @@ class CudaKernels:
 
     # From spans of this many tokens on, a bfloat16 run takes its recurrences by stretches of 64 tokens (csrc/chunk_scan.cu).
     CHUNK_SCAN_MIN_SPAN = 128
+    # The delta rule's stretches (csrc/delta_chunks.cu) do several times a token's work of the scan; what they gain is that tokens of
+    # one span run side by side.  us, scan and stretches, 24 heads of 64: one span of 2,048 tokens 660 / 241, 300: 101 / 46, 128:
+    # 48 / 41, 96: 38 / 41; four of 500 256 / 219; sixteen of 128 197 / 227 (56 heads: 427 / 492).
+    DELTA_CHUNKS_MIN_SPAN = 128
+    DELTA_CHUNKS_MAX_SPANS = 8
 
     def _scans_by_chunks(self, dtype, ctx, heads, dk, dv, *rows):
         """Whether a recurrence goes by stretches of tokens: long spans, sizes the kernels are made for, rows on 16-byte
@@ -1427,8 +1433,20 @@ class CudaKernels:
             _need(t.dtype == torch.float32 and t.is_contiguous() and t.numel() == HD, "delta_rule_scan: float32 constants of heads * dim")
         _need(state is not None and state.dtype == torch.float32 and state.dim() == 2 and state.stride(1) == 1
               and state.shape[1] >= HD * dim, "delta_rule_scan: the state does not fit the sizes")
-        scratch = torch.empty(int(self.lib.ifx_delta_rule_scratch_floats(T, heads, dim)), dtype=torch.float32, device=proj.device)
         y = torch.empty((T, HD), dtype=out_dtype, device=proj.device)
+        if (self.chunk_scans and out_dtype is torch.bfloat16 and ctx.max_span >= self.DELTA_CHUNKS_MIN_SPAN
+                and T <= self.DELTA_CHUNKS_MAX_SPANS * ctx.max_span
+                and self.lib.ifx_delta_chunks_supports(ctx.num_requests, heads, dim) and proj.shape[1] % 4 == 0
+                and all(t.data_ptr() % 16 == 0 for t in (proj, w_raw, w0, a_bias))):
+            room = torch.empty(int(self.lib.ifx_delta_chunks_scratch_floats(T, ctx.num_requests, heads)), dtype=torch.float32,
+                               device=proj.device)
+            _check(self.lib.ifx_delta_chunks_scan(
+                _ptr(proj), proj.shape[1], _ptr(w_raw), _ptr(w0), _ptr(a_bias), _ptr(norm_w), ctypes.c_float(eps), _ptr(state),
+                ctypes.c_longlong(state.stride(0)), _ptr(ctx.cu_seqlens), _ptr(ctx.req_slot), _ptr(room), _ptr(y), ctx.num_requests, T,
+                heads, dim, _DT[out_dtype], _stream()), "delta_rule_scan (stretches)")
+            self.launches += 4
+            return y
+        scratch = torch.empty(int(self.lib.ifx_delta_rule_scratch_floats(T, heads, dim)), dtype=torch.float32, device=proj.device)
         _check(self.lib.ifx_delta_rule_scan(
             _ptr(proj), proj.shape[1], _ptr(w_raw), _ptr(w0), _ptr(a_bias), _ptr(norm_w), ctypes.c_float(eps), _ptr(state),
             ctypes.c_longlong(state.stride(0)), _ptr(ctx.cu_seqlens), _ptr(ctx.req_slot), _ptr(scratch), _ptr(y),

@@ -1,0 +1,67 @@
+"""The delta rule by stretches of 64 tokens (long spans of a bfloat16 run) against the plain statement and the scan: spans around
+whole stretches, states carried over steps, decays and erasures from none to all, keys that repeat, numbers that are not finite."""
+import pytest
+import torch
+
+from plain.plain_kernels import PlainKernels
+from test_chunk_scan_gpu import STEPS, _Ctx
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+F64 = torch.float64
+BF = torch.bfloat16
+
+
+def _scan(kernels, chunks, *args):
+    before, kernels.chunk_scans = kernels.chunk_scans, chunks
+    try:
+        return kernels.delta_rule_scan(*args)
+    finally:
+        kernels.chunk_scans = before
+
+
+@pytest.mark.parametrize("H,w_shift,a_shift,same_keys", [(3, 0.0, 0.0, False), (1, -8.0, -8.0, False), (2, 8.0, 8.0, False), (2, -8.0, 8.0, True)])
+def test_delta_rule(cuda_kernels, H, w_shift, a_shift, same_keys):
+    D, HD, front = 64, 64 * H, 8
+    g = torch.Generator().manual_seed(H)
+    w0, ab, nw = torch.randn(HD, generator=g) + w_shift, torch.randn(HD, generator=g) + a_shift, 1 + 0.2 * torch.randn(HD, generator=g)
+    states = [torch.zeros(4, front + HD * D, device=DEV) for _ in range(2)]
+    state_p = torch.zeros(4, front + HD * D, dtype=F64)
+    for lens, slots in STEPS:
+        T = sum(lens)
+        proj, w_raw = torch.randn(T, 5 * HD, generator=g), torch.randn(T, HD, generator=g)
+        if same_keys:                                                           # every key nearly the one before: the system at its fullest
+            proj[:, HD:2 * HD] = proj[:1, HD:2 * HD] + 0.05 * proj[:, HD:2 * HD]
+        want = PlainKernels(wide=True).delta_rule_scan(proj.double(), w_raw.double(), w0, ab, nw, 1e-5, H, D, state_p[:, front:],
+                                                       _Ctx(lens, slots, "cpu"), F64)
+        for st, chunks in zip(states, (True, False)):
+            before = cuda_kernels.launches
+            y = _scan(cuda_kernels, chunks, proj.to(DEV), w_raw.to(DEV), w0.to(DEV), ab.to(DEV), nw.to(DEV), 1e-5, H, D, st[:, front:],
+                      _Ctx(lens, slots, DEV), BF)
+            assert cuda_kernels.launches - before == (4 if chunks else 3)
+            assert float((y.double().cpu() - want).abs().max()) <= 2.0 ** -8 * max(1.0, float(want.abs().max()))
+        # both make float32 sums of up to 300 terms: as near to the 64-bit ones as one another
+        errors = [float((st.double().cpu() - state_p).norm() / state_p.norm()) for st in states]
+        assert errors[0] <= 4 * errors[1] + 5e-7, errors
+    assert float(states[0][1].abs().max()) == 0.0 and float(states[0][:, :front].abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("block", range(5))
+def test_a_number_that_is_not_finite_reaches_what_follows_it(cuda_kernels, block):
+    H, D, T, t0 = 2, 64, 200, 70
+    HD = H * D
+    g = torch.Generator().manual_seed(5)
+    proj, w_raw = torch.randn(T, 5 * HD, generator=g), torch.randn(T, HD, generator=g)
+    clean = proj.clone()
+    proj[t0, block * HD + 3] = float("inf") if block < 3 else float("nan")       # r, k, v, g, a
+    vec = [torch.randn(HD, generator=g).to(DEV) for _ in range(3)]
+    results = []
+    for rows, chunks in ((clean, True), (proj, True), (proj, False)):
+        state = torch.zeros(1, HD * D, device=DEV)
+        results.append((_scan(cuda_kernels, chunks, rows.to(DEV), w_raw.to(DEV), *vec, 1e-6, H, D, state, _Ctx((T,), (0,), DEV), BF), state))
+    (y0, _), (y, state), (walk, state_w) = results
+    assert torch.equal(y[:64], y0[:64]) and torch.equal(y[:, D:], y0[:, D:])      # stretches in front, the other head
+    assert torch.equal(torch.isfinite(y), torch.isfinite(walk)) and torch.equal(torch.isfinite(state), torch.isfinite(state_w))
+    fine = torch.isfinite(walk)
+    assert bool(fine[:t0].all()) and not bool(fine.all())
+    assert float((y.float() - walk.float())[fine].abs().max()) <= 2.0 ** -7 * float(walk.float()[fine].abs().max())
