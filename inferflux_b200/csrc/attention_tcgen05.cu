@@ -49,17 +49,6 @@ __device__ __forceinline__ uint64_t desc_mnmajor_sw128(uint32_t addr, uint32_t a
   return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)((atom_stride_bytes >> 4) & 0x3FFF) << 16) |
          ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -89,14 +78,6 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
-__device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&u)[32]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -148,7 +129,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
   const uint32_t bar0 = smem_addr(bars);
   auto bar = [&](int i) { return bar0 + 8 * i; };
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   pdl_launch_dependents();
   if (threadIdx.x == 0) {
     mbar_init(bar(L::B_Q), 1);
@@ -245,42 +226,44 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
         mbar_wait(bar(L::B_FULL + j % SLOTS), (j / SLOTS) & 1);
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issue
-    if (lane == 0) {
+    // ------------------------------------------------------- MMA issue: the warp in step, one lane's instructions by predicate
+    {
+      const uint32_t elected = elect_one();
       const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kBN >> 3) << 17) |
                                ((uint32_t)(kBM >> 4) << 24);                       // both operands K-major
       const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(D >> 3) << 17) |
                                ((uint32_t)(kBM >> 4) << 24);                       // B (values) MN-major
       auto last_q = [&](int kt) { return active(1, kt) ? 1 : 0; };    // the query tile that uses a key tile last
-      bool ok = mbar_wait(bar(L::B_Q), 0);
+      auto wait = [&](int b, int parity) { return (bool)__all_sync(0xffffffffu, mbar_wait(bar(b), parity)); };
+      bool ok = wait(L::B_Q, 0);
       auto issue_s = [&](int q, int kt) -> bool {         // S_q = Q_q . K(kt)^T
         const int j = 2 * visited(kt), s = j % SLOTS;
-        if (!mbar_wait(bar(L::B_FULL + s), (j / SLOTS) & 1)) return false;
+        if (!wait(L::B_FULL + s, (j / SLOTS) & 1)) return false;
         tc_fence_after();
         const uint32_t k_src = kv_s + s * SLOT_BYTES, q_src = q_s + q * Q_BYTES;
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
           const uint32_t half = k / 4, inner = (k % 4) * 32;
-          umma_bf16(tmem_s + q * kBN, desc_kmajor_sw128(q_src + half * kBM * 128) + (inner >> 4),
-                    desc_kmajor_sw128(k_src + half * kBN * 128) + (inner >> 4), idesc_s, k > 0 ? 1u : 0u);
+          umma_ss(tmem_s + q * kBN, desc_kmajor_sw128(q_src + half * kBM * 128) + (inner >> 4),
+                    desc_kmajor_sw128(k_src + half * kBN * 128) + (inner >> 4), idesc_s, k > 0 ? 1u : 0u, elected);
         }
-        umma_commit(bar(L::B_S_FULL + q));
-        if (q == last_q(kt)) umma_commit(bar(L::B_EMPTY + s));      // the keys have been read
+        umma_commit(bar(L::B_S_FULL + q), elected);
+        if (q == last_q(kt)) umma_commit(bar(L::B_EMPTY + s), elected);      // the keys have been read
         return true;
       };
       int done[2] = {0, 0};                                // key tiles of each query tile so far
       auto issue_pv = [&](int q, int kt) -> bool {        // O_q += P_q . V(kt)
         const int j = 2 * visited(kt) + 1, s = j % SLOTS;
-        if (!mbar_wait(bar(L::B_P_FULL + q), done[q] & 1) || !mbar_wait(bar(L::B_FULL + s), (j / SLOTS) & 1))
+        if (!wait(L::B_P_FULL + q, done[q] & 1) || !wait(L::B_FULL + s, (j / SLOTS) & 1))
           return false;
         tc_fence_after();
         const uint32_t v_src = kv_s + s * SLOT_BYTES;
 #pragma unroll
         for (int k = 0; k < kBN / 16; ++k)                 // 16 keys (8 columns of pairs) a step
-          umma_bf16_ts(tmem_o + q * D, tmem_s + q * kBN + k * 8, desc_mnmajor_sw128(v_src + k * 2048, kBN * 128),
-                       idesc_o, (done[q] > 0 || k > 0) ? 1u : 0u);
-        umma_commit(bar(L::B_O_FULL + q));
-        if (q == last_q(kt)) umma_commit(bar(L::B_EMPTY + s));      // the values have been read
+          umma_ts(tmem_o + q * D, tmem_s + q * kBN + k * 8, desc_mnmajor_sw128(v_src + k * 2048, kBN * 128),
+                       idesc_o, (done[q] > 0 || k > 0) ? 1u : 0u, elected);
+        umma_commit(bar(L::B_O_FULL + q), elected);
+        if (q == last_q(kt)) umma_commit(bar(L::B_EMPTY + s), elected);      // the values have been read
         ++done[q];
         return true;
       };
@@ -297,7 +280,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
           if (ok && active(q, next_tile(kt))) ok = issue_s(q, next_tile(kt));
         }
       }
-      if (!ok) atomicExch(error_flag, 8);
+      if (!ok && lane == 0) atomicExch(error_flag, 8);
     }
     __syncwarp();
   } else {

@@ -42,23 +42,6 @@ __device__ __forceinline__ uint64_t lp_desc_k(uint32_t addr) {
 __device__ __forceinline__ uint64_t lp_desc_mn(uint32_t addr) {          // the next 64 columns lie a box further
   return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(kLpBox >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
-__device__ __forceinline__ void lp_mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void lp_mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void lp_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
 __device__ __forceinline__ void lp_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 __device__ __forceinline__ void lp_ld32(uint32_t taddr, float* r) {
   uint32_t* u = reinterpret_cast<uint32_t*>(r);
@@ -120,7 +103,7 @@ __global__ void __launch_bounds__(kLpThreads, 1) latent_prompt_kernel(
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(smem + L::HOLDER);
   float* maxima = reinterpret_cast<float*>(smem + L::MAXIMA);          // [half][128]
   __shared__ int odd_s;                                                // a cleared row held a number that is not finite
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int bx = gridDim.x - 1 - blockIdx.x;                           // later tokens see more keys: they start first
   const int4 item = items[bx / tiles_per_item];
   const int r0 = (bx % tiles_per_item) * kLpRows, rows_item = item.z * heads;
@@ -202,43 +185,45 @@ __global__ void __launch_bounds__(kLpThreads, 1) latent_prompt_kernel(
     }
     __syncwarp();
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issue
-    if (lane == 0) {
+    // ------------------------------------------------------- MMA issue: the warp in step, one lane's instructions by predicate
+    {
+      const uint32_t elected = elect_one();
+      auto wait = [&](int b, int parity) { return (bool)__all_sync(0xffffffffu, mbar_wait(bar(b), parity)); };
       const uint32_t common = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kLpRows >> 4) << 24);
       const uint32_t idesc_s = common | ((uint32_t)(kLpKeys >> 3) << 17), idesc_o = common | (1u << 16) | ((uint32_t)(kLpRank >> 3) << 17);
-      bool ok = mbar_wait(bar(L::B_Q), 0);
+      bool ok = wait(L::B_Q, 0);
       auto scores = [&](int i) -> bool {
         const uint32_t k_src = base + L::KV + (i & 1) * L::KV_BYTES, d = tmem + (i & 1) * kLpKeys;
-        if (!mbar_wait(bar(L::B_KV_FULL + (i & 1)), (i >> 1) & 1)) return false;
+        if (!wait(L::B_KV_FULL + (i & 1), (i >> 1) & 1)) return false;
         lp_after();
 #pragma unroll
         for (int k = 0; k < kLpRank / 16; ++k)
-          lp_mma_ss(d, lp_desc_k(base + L::Q + (k / 4) * kLpBox) + (k % 4) * 2, lp_desc_k(k_src + (k / 4) * kLpBox) + (k % 4) * 2, idesc_s,
-                    k > 0 ? 1u : 0u);
+          umma_ss(d, lp_desc_k(base + L::Q + (k / 4) * kLpBox) + (k % 4) * 2, lp_desc_k(k_src + (k / 4) * kLpBox) + (k % 4) * 2, idesc_s,
+                    k > 0 ? 1u : 0u, elected);
         if (ROT) {
-          if (!mbar_wait(bar(L::B_ROT_FULL), i & 1)) return false;
+          if (!wait(L::B_ROT_FULL, i & 1)) return false;
           lp_after();
 #pragma unroll
           for (int k = 0; k < ROT / 16; ++k)
-            lp_mma_ss(d, lp_desc_k(base + L::Q + 4 * kLpBox) + k * 2, lp_desc_k(base + L::TURNED) + k * 2, idesc_s, 1u);
+            umma_ss(d, lp_desc_k(base + L::Q + 4 * kLpBox) + k * 2, lp_desc_k(base + L::TURNED) + k * 2, idesc_s, 1u, elected);
         }
-        lp_commit(bar(L::B_S_FULL + (i & 1)));
-        if (ROT) lp_commit(bar(L::B_ROT_EMPTY));
+        umma_commit(bar(L::B_S_FULL + (i & 1)), elected);
+        if (ROT) umma_commit(bar(L::B_ROT_EMPTY), elected);
         return true;
       };
       if (ok) ok = scores(0);
       for (int i = 0; i < n && ok; ++i) {
         if (i + 1 < n) ok = scores(i + 1);                             // over the weights of tile i - 1, whose product was issued before
-        if (!ok || !(ok = mbar_wait(bar(L::B_P_FULL + (i & 1)), (i >> 1) & 1))) break;
+        if (!ok || !(ok = wait(L::B_P_FULL + (i & 1), (i >> 1) & 1))) break;
         lp_after();
         const uint32_t v_src = base + L::KV + (i & 1) * L::KV_BYTES;
 #pragma unroll
         for (int k = 0; k < kLpKeys / 16; ++k)
-          lp_mma_ts(tmem_o, tmem + (i & 1) * kLpKeys + k * 8, lp_desc_mn(v_src + k * 2048), idesc_o, (i > 0 || k > 0) ? 1u : 0u);
-        lp_commit(bar(L::B_KV_EMPTY + (i & 1)));
-        lp_commit(bar(L::B_O_FULL));
+          umma_ts(tmem_o, tmem + (i & 1) * kLpKeys + k * 8, lp_desc_mn(v_src + k * 2048), idesc_o, (i > 0 || k > 0) ? 1u : 0u, elected);
+        umma_commit(bar(L::B_KV_EMPTY + (i & 1)), elected);
+        umma_commit(bar(L::B_O_FULL), elected);
       }
-      if (!ok) atomicExch(error_flag, 62);
+      if (!ok && lane == 0) atomicExch(error_flag, 62);
     }
     __syncwarp();
   } else {

@@ -61,6 +61,42 @@ __device__ __forceinline__ uint64_t l2_evict_first_policy() {
   return p;
 }
 
+// 1 in one lane of a converged warp, 0 in the others.  tcgen05.mma and its commit are issued by a whole warp in step, the one
+// lane's by a predicate: descriptors then live in uniform registers.  From a branch that one lane takes, every issue moves them
+// there first: 172 cycles for an M 128, N 256, K 16 product whose operands lie in shared memory, and 108 for N 128; by predicate
+// 129 and 65, the tensor pipe's own 128 and 64.
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r;
+}
+// D (+)= A B^T for the elected lane: operands in shared memory, or A in tensor memory.
+__device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate,
+                                        uint32_t elected) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(elected)
+      : "memory");
+}
+__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate,
+                                        uint32_t elected) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(elected)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit(uint32_t bar, uint32_t elected) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+      ::"r"(bar), "r"(elected)
+      : "memory");
+}
+// This thread's warp, the same for all its lanes as far as the compiler can tell.
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 // Generic-proxy accesses to shared memory (ldmatrix, stores) that came before are ordered
 // before asynchronous-proxy accesses (TMA writes) that come after.
 __device__ __forceinline__ void fence_proxy_async_smem() {
