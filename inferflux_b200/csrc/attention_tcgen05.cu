@@ -25,6 +25,12 @@
 // [16 keys x 64 elements] through the block table, into a ring of slots (a slot holds the keys
 // or the values of one tile).  Warp 1 issues the MMAs.  Warps 2-5 and 6-9 are the softmax groups.
 //
+// Bound: the tensor pipe and the exponentials, each busy 43 % of the time a block is resident (a key tile takes a block 2.1 us),
+// waiting for one another at the hand-overs.  A warp in step issues the products, one lane of it by predicate: with a single thread in a
+// branch of its own a product took 108 clocks to issue instead of 65 (2,500 tokens behind 4,000, 28 heads: 211 us, then 192).
+// A block has an SM to itself, so blocks left over behind whole rounds of 148 cost a round: they are cut into parts of their keys
+// that prefill_merge_kernel adds up (192 -> 162; 512 tokens behind 3,000 of 12 heads, where 24 blocks are all there is, 62 -> 30).
+//
 // Keys outside a row's range get weight zero; what the cache holds there is finite (the pool
 // starts as zeros and only finite values are written to it).  Page sizes: powers of two from
 // 16; head sizes 64 and 128.  Every wait is bounded; a wait that runs out sets *error_flag.
@@ -94,6 +100,7 @@ __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+constexpr int kSms = 148;                  // blocks of a round: one an SM
 constexpr float kRescaleStep = 8.0f;      // log2 units the maximum may outgrow its reference before O is rescaled
 constexpr uint32_t kTmemCols = 512;       // per query tile: scores (128 columns) and output (head size)
 constexpr int kThreads = 320;             // fetch warp, MMA warp, two softmax groups of four warps
@@ -109,6 +116,15 @@ struct PrefillLayout {
   static constexpr size_t SMEM = 1024 + 2 * Q_BYTES + (size_t)SLOTS * SLOT_BYTES + B_COUNT * 8 + 16;
 };
 
+// What is left over when whole rounds of blocks, one an SM, have been taken off a grid runs as `parts` blocks each, every one over a
+// part of the keys, and leaves an unnormalised sum, its reference and its denominator for prefill_merge_kernel.  A plain grid has
+// full = its blocks.  (28 heads x 11 items on 148 SMs are two rounds and 12 blocks, which alone took a third round.)
+struct PrefillParts {
+  int full, parts;
+  float* o;                  // [left over x parts][256][D]
+  float2* ml;                // [left over x parts][256]: reference in units of log2, sum
+};
+
 // KEPT: the mask has kept first keys (without them the walk over the key tiles is a plain range).
 template <int D, bool KEPT>
 __global__ void __launch_bounds__(kThreads)
@@ -116,7 +132,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
                             const int* __restrict__ block_table, const int* __restrict__ tiles,
                             const int* __restrict__ req_slot, bf16* __restrict__ out, int nq, int nkv, int page_size,
                             int page_shift, int max_blocks, int num_pages, KeyMask window, HeadOutput post, float scale_log2,
-                            int* __restrict__ error_flag) {
+                            int* __restrict__ error_flag, int num_tiles, PrefillParts split) {
   using L = PrefillLayout<D>;
   constexpr int HALVES = L::HALVES, SLOTS = L::SLOTS;
   constexpr uint32_t Q_BYTES = L::Q_BYTES, SLOT_BYTES = L::SLOT_BYTES;
@@ -158,16 +174,30 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
   pdl_wait();
 
   // the last items of a prompt see the most keys: they go first; the heads of an item run side by side
-  const int* tile = tiles + (size_t)(gridDim.y - 1 - blockIdx.y) * 4;
+  int block = blockIdx.x, part = 0;
+  const int slot = block - split.full;                     // < 0: a block with all of its keys
+  if (slot >= 0) {
+    block = split.full + slot / split.parts;
+    part = slot % split.parts;
+  }
+  const int* tile = tiles + (size_t)(num_tiles - 1 - block / nq) * 4;
   const int r = tile[0], row0 = tile[1], rows = tile[2], pos0 = tile[3];
-  const int h = blockIdx.x;
+  const int h = block % nq;
   const int g = h / (nq / nkv);
   // key tiles [tb_q, te_q) of query tile q (rows q * 128 ...); tile 1 may be absent
   const int rows_1 = max(rows - kBM, 0);
-  const int tb_0 = window.first(pos0) / kBN;
-  const int te_0 = (pos0 + min(rows, kBM) + kBN - 1) / kBN;
-  const int tb_1 = window.first(pos0 + kBM) / kBN;
-  const int te_1 = rows_1 > 0 ? (pos0 + rows + kBN - 1) / kBN : tb_1;
+  int tb_0 = window.first(pos0) / kBN;
+  int te_0 = (pos0 + min(rows, kBM) + kBN - 1) / kBN;
+  int tb_1 = window.first(pos0 + kBM) / kBN;
+  int te_1 = rows_1 > 0 ? (pos0 + rows + kBN - 1) / kBN : tb_1;
+  if (!KEPT && slot >= 0) {                                // this block's part of the key tiles (tile 0 begins first)
+    const int last = max(te_0, te_1), per = (last - tb_0 + split.parts - 1) / split.parts;
+    const int lo = min(last, tb_0 + part * per), hi = min(last, lo + per);
+    tb_0 = lo;
+    te_0 = max(lo, min(te_0, hi));
+    tb_1 = max(lo, min(tb_1, hi));
+    te_1 = max(tb_1, min(te_1, hi));
+  }
   const int te = max(te_0, te_1);
   // Key tiles are visited in order: with kept keys first [0, nk), then [tb_0, te); query tile q uses those that hold kept keys
   // and those of its own window.
@@ -386,7 +416,25 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
     }
     if (ok && i > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar(L::B_O_FULL + q), (i - 1) & 1));
     if (!ok && lane == 0) atomicExch(error_flag, 9);
-    if (ok && i > 0) {
+    if (!KEPT && slot >= 0) {                              // the sum as it is, for the merge
+      const size_t at = (size_t)slot * 2 * kBM + q * kBM + row;
+      if (row < rows_q)
+        split.ml[at] = ok && i > 0 ? make_float2(m_ref > -INFINITY ? m_ref * scale_log2 : -INFINITY, l_run) : make_float2(-INFINITY, 0.0f);
+      if (ok && i > 0) {
+        tc_fence_after();
+#pragma unroll 1
+        for (int c = 0; c < D; c += 32) {
+          float t[32];
+          tmem_ld32(o_addr + c, t);
+          tmem_wait_ld();
+          if (row < rows_q) {
+#pragma unroll
+            for (int j = 0; j < 32; j += 4)
+              *reinterpret_cast<float4*>(split.o + at * D + c + j) = make_float4(t[j], t[j + 1], t[j + 2], t[j + 3]);
+          }
+        }
+      }
+    } else if (ok && i > 0) {
       tc_fence_after();
       if (window.sink && m_ref > -INFINITY) l_run += exp2f(window.sink_log2(h) - m_ref * scale_log2);     // the sink's share
       const float inv = (l_run > 0.0f ? 1.0f / l_run : 0.0f) * post.factor(row0 + q * kBM + min(row, max(rows_q - 1, 0)), h);
@@ -461,11 +509,44 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
   }
 }
 
+// grid (left over blocks, 32): a warp a row; parts in order.
+template <int D>
+__global__ void __launch_bounds__(256) prefill_merge_kernel(const int* __restrict__ tiles, bf16* __restrict__ out, int nq, int num_tiles,
+                                                            PrefillParts split) {
+  pdl_wait();
+  const int block = split.full + blockIdx.x, row = blockIdx.y * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int* tile = tiles + (size_t)(num_tiles - 1 - block / nq) * 4;
+  if (row >= tile[2]) return;
+  const size_t at = (size_t)blockIdx.x * split.parts * 2 * kBM + row;
+  float m = -INFINITY, l = 0.0f;
+  for (int p = 0; p < split.parts; ++p) m = fmaxf(m, split.ml[at + (size_t)p * 2 * kBM].x);
+  float acc[D / 32];
+#pragma unroll
+  for (int j = 0; j < D / 32; ++j) acc[j] = 0.0f;
+  for (int p = 0; p < split.parts; ++p) {
+    const float2 ml = split.ml[at + (size_t)p * 2 * kBM];
+    if (ml.x == -INFINITY && !isnan(ml.y)) continue;       // no key of this part: its sums were not written
+    const float w = ml.x == -INFINITY ? 1.0f : exp2f(ml.x - m);
+    l = fmaf(ml.y, w, l);
+    const float* o = split.o + (at + (size_t)p * 2 * kBM) * D + lane * (D / 32);
+#pragma unroll
+    for (int j = 0; j < D / 32; j += 2) {
+      const float2 v = *reinterpret_cast<const float2*>(o + j);
+      acc[j] = fmaf(v.x, w, acc[j]);
+      acc[j + 1] = fmaf(v.y, w, acc[j + 1]);
+    }
+  }
+  const float inv = l > 0.0f || isnan(l) ? 1.0f / l : 0.0f;
+  bf16* to = out + ((size_t)(tile[1] + row) * nq + block % nq) * D + lane * (D / 32);
+#pragma unroll
+  for (int j = 0; j < D / 32; j += 2) *reinterpret_cast<__nv_bfloat162*>(to + j) = __floats2bfloat162_rn(acc[j] * inv, acc[j + 1] * inv);
+}
+
 template <int D, bool KEPT>
 static int launch_prefill_tcgen05(const bf16* q, int num_tokens, const bf16* kv_pool, const int* block_table,
                                   const int* tiles, const int* req_slot, bf16* out, int num_tiles, int nq, int nkv,
                                   int page_size, int page_shift, int max_blocks, int num_pages, KeyMask window, HeadOutput post,
-                                  float scale_log2, int* error_flag, cudaStream_t stream) {
+                                  float scale_log2, int* error_flag, cudaStream_t stream, int parts, void* workspace) {
   CUtensorMap q_map, pool_map;
   int rc = make_tensor_map_bf16(&q_map, q, num_tokens, nq * D, kBM);
   if (rc) return rc;
@@ -479,9 +560,14 @@ static int launch_prefill_tcgen05(const bf16* q, int num_tokens, const bf16* kv_
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  return launch_pdl(attn_prefill_tcgen05_kernel<D, KEPT>, dim3(nq, num_tiles), dim3(kThreads), smem, stream, 1, q_map,
-                    pool_map, block_table, tiles, req_slot, out, nq, nkv, page_size, page_shift, max_blocks,
-                    num_pages, window, post, scale_log2, error_flag);
+  const int blocks = nq * num_tiles, left = parts > 1 ? blocks % kSms : 0;
+  PrefillParts split{blocks - left, parts, (float*)workspace, nullptr};
+  if (left) split.ml = reinterpret_cast<float2*>(split.o + (size_t)left * parts * 2 * kBM * D);
+  rc = launch_pdl(attn_prefill_tcgen05_kernel<D, KEPT>, dim3(split.full + left * parts), dim3(kThreads), smem, stream, 1, q_map,
+                  pool_map, block_table, tiles, req_slot, out, nq, nkv, page_size, page_shift, max_blocks,
+                  num_pages, window, post, scale_log2, error_flag, num_tiles, split);
+  if (rc || !left) return rc;
+  return launch_pdl(prefill_merge_kernel<D>, dim3(left, 2 * kBM / 8), dim3(256), 0, stream, 1, tiles, out, nq, num_tiles, split);
 }
 
 }  // namespace ifx
@@ -517,7 +603,7 @@ int ifx_attention_prefill_tcgen05_sink(const void* q, int num_tokens, const void
   const float scale_log2 = scale * 1.4426950408889634f;
   auto run = [&](auto launch) {
     return launch((const bf16*)q, num_tokens, (const bf16*)kv_pool, block_table, tiles, req_slot, (bf16*)out, num_tiles, nq, nkv,
-                  page_size, ps, max_blocks, num_pages, window, post, scale_log2, error_flag, stream);
+                  page_size, ps, max_blocks, num_pages, window, post, scale_log2, error_flag, stream, 1, nullptr);
   };
   if (d == 64) return keep_first > 0 ? run(launch_prefill_tcgen05<64, true>) : run(launch_prefill_tcgen05<64, false>);
   return keep_first > 0 ? run(launch_prefill_tcgen05<128, true>) : run(launch_prefill_tcgen05<128, false>);
@@ -538,6 +624,32 @@ int ifx_attention_prefill_tcgen05(const void* q, int num_tokens, const void* kv_
                                   int* error_flag, cudaStream_t stream) {
   return ifx_attention_prefill_tcgen05_ex(q, num_tokens, kv_pool, block_table, tiles, req_slot, out, num_tiles, nq, nkv, d,
                                           page_size, max_blocks, num_pages, window, 0, 0, scale, error_flag, stream);
+}
+
+// Bytes of workspace that cutting the left over blocks into `parts` (at least two) needs.
+long long ifx_attention_prefill_tcgen05_parts_bytes(int num_tiles, int nq, int d, int parts) {
+  return parts > 1 ? (long long)((long long)num_tiles * nq % kSms) * parts * 2 * kBM * (d + 2) * 4 : 0;
+}
+
+// The plain form with the blocks left over behind whole rounds cut into `parts` parts of their keys (1: none; two launches with more).
+int ifx_attention_prefill_tcgen05_parts(const void* q, int num_tokens, const void* kv_pool, const int* block_table, const int* tiles,
+                                        const int* req_slot, void* out, int num_tiles, int nq, int nkv, int d, int page_size,
+                                        int max_blocks, int num_pages, int window, float scale, int parts, void* workspace,
+                                        int* error_flag, cudaStream_t stream) {
+  if (parts <= 1)
+    return ifx_attention_prefill_tcgen05(q, num_tokens, kv_pool, block_table, tiles, req_slot, out, num_tiles, nq, nkv, d, page_size,
+                                         max_blocks, num_pages, window, scale, error_flag, stream);
+  if (num_tiles <= 0) return 0;
+  if (!ifx_attention_prefill_tcgen05_supports(d, page_size) || nq <= 0 || nkv <= 0 || nq % nkv || max_blocks <= 0 || num_tiles > 65535 ||
+      !(scale > 0.0f) || error_flag == nullptr || parts > 16 || workspace == nullptr || (uintptr_t)workspace % 16)
+    return IFX_E_BADARG;
+  int ps = 0;
+  while ((1 << ps) < page_size) ++ps;
+  const KeyMask mask{window, 0, 0, nullptr, 0};
+  const HeadOutput post{nullptr, 0, nullptr, nq};
+  auto launch = d == 64 ? launch_prefill_tcgen05<64, false> : launch_prefill_tcgen05<128, false>;
+  return launch((const bf16*)q, num_tokens, (const bf16*)kv_pool, block_table, tiles, req_slot, (bf16*)out, num_tiles, nq, nkv, page_size, ps,
+                max_blocks, num_pages, mask, post, scale * 1.4426950408889634f, error_flag, stream, parts, workspace);
 }
 
 }  // extern "C"

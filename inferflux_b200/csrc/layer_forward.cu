@@ -26,8 +26,9 @@ int ifx_rope_append(const void*, const float*, int, const float*, const float*, 
                     const int*, int, int, int, void*, void*, int, int, int, int, int, int, int, cudaStream_t);
 int ifx_attention_mma_supports(int);
 int ifx_attention_prefill_tcgen05_supports(int, int);
-int ifx_attention_prefill_tcgen05(const void*, int, const void*, const int*, const int*, const int*, void*, int, int, int, int,
-                                  int, int, int, int, float, int*, cudaStream_t);
+int ifx_attention_prefill_tcgen05_parts(const void*, int, const void*, const int*, const int*, const int*, void*, int, int, int, int, int,
+                                        int, int, int, float, int, void*, int*, cudaStream_t);
+long long ifx_attention_prefill_tcgen05_parts_bytes(int, int, int, int);
 int ifx_attention_prefill_bf16(const void*, const void*, const int*, const int*, const int*, void*, int, int, int, int, int,
                                int, int, int, float, int, int*, cudaStream_t);
 int ifx_attention_decode_max_splits(int, int);
@@ -73,7 +74,8 @@ struct IfxLayerIO {
   long long ws_bytes;
   void* out_tensor;           // this layer's last delta, unadded: one of the two forms again
   float* out_parts;
-  int out_splits, launches, library_calls, pad0;
+  int out_splits, launches, library_calls;
+  int prefill_parts;          // in: parts of the prompt attention's left over blocks (CudaKernels.prefill_parts)
 };
 
 namespace {
@@ -243,6 +245,7 @@ extern "C" long long ifx_layer_workspace_bytes(int T, int hidden, int q_dim, int
   total += 2 * ((size_t)T * hidden * 2 + 256) + 2 * ((size_t)T * chunks * 4 + 256);      // normed rows, sums of squares
   total += delta(qkv) + 2 * ((size_t)T * q_dim * 2 + 256) + delta(hidden);               // q/k/v, q, attention, o
   total += (size_t)T * 2 * inter * 2 + (size_t)T * inter * 2 + 512;                      // gate|up, activation
+  total += (size_t)148 * 256 * (128 + 2) * 4 + 256;                                     // parts of the prompt attention
   return (long long)total + 1024;
 }
 
@@ -304,11 +307,15 @@ extern "C" int ifx_layer_forward(const IfxStepArgs* s, const IfxLayerArgs* l, If
       }
     }
     if (s->num_tiles > 0) {
-      if (s->tensor_core_prefill && ifx_attention_prefill_tcgen05_supports(d, l->page_size))
-        RUN(ifx_attention_prefill_tcgen05(q, T, l->kv_pool, l->block_table, s->prefill_tiles, s->req_slot, attn, s->num_tiles,
-                                          nq, nkv, d, l->page_size, l->max_blocks, l->num_pages, l->window, l->scale,
-                                          s->error_flag, st));
-      else
+      if (s->tensor_core_prefill && ifx_attention_prefill_tcgen05_supports(d, l->page_size)) {
+        const size_t bytes = (size_t)ifx_attention_prefill_tcgen05_parts_bytes(s->num_tiles, nq, d, io->prefill_parts);
+        void* room = bytes ? c.ws.take(bytes) : nullptr;
+        if (bytes && !room) return IFX_E_TOOBIG;
+        RUN(ifx_attention_prefill_tcgen05_parts(q, T, l->kv_pool, l->block_table, s->prefill_tiles, s->req_slot, attn, s->num_tiles, nq,
+                                                nkv, d, l->page_size, l->max_blocks, l->num_pages, l->window, l->scale,
+                                                bytes ? io->prefill_parts : 1, room, s->error_flag, st));
+        if (bytes) ++io->launches;
+      } else
         RUN(ifx_attention_prefill_bf16(q, l->kv_pool, l->block_table, s->prefill_tiles, s->req_slot, attn, s->num_tiles, nq,
                                        nkv, d, l->page_size, l->max_blocks, l->num_pages, l->window, l->scale, s->max_kv_len,
                                        s->error_flag, st));

@@ -129,7 +129,7 @@ class _LayerIO(ctypes.Structure):
     """IfxLayerIO: what changes from call to call, and what comes back."""
     _fields_ = [("x", _P), ("pending_tensor", _P), ("pending_parts", _P), ("pending_splits", _I), ("parity", _I),
                 ("ws", _P), ("ws_bytes", _LL), ("out_tensor", _P), ("out_parts", _P), ("out_splits", _I),
-                ("launches", _I), ("library_calls", _I), ("pad0", _I)]
+                ("launches", _I), ("library_calls", _I), ("prefill_parts", _I)]
 
 
 class CudaKernels:
@@ -168,11 +168,13 @@ class CudaKernels:
                    "ifx_geglu_mul", "ifx_gemm_skinny_geglu", "ifx_gemm_tcgen05_geglu", "ifx_relu2", "ifx_silu_columns", "ifx_moe_stream",
                    "ifx_moe_stream_slices", "ifx_chunk_scan_supports", "ifx_chunk_decay_scan", "ifx_chunk_wkv_scan", "ifx_wkv_norm",
                    "ifx_latent_decode", "ifx_latent_decode_supports", "ifx_latent_decode_stretch",
-                   "ifx_latent_prompt", "ifx_latent_prompt_supports", "ifx_delta_chunks_supports", "ifx_delta_chunks_scan"):
+                   "ifx_latent_prompt", "ifx_latent_prompt_supports", "ifx_delta_chunks_supports", "ifx_delta_chunks_scan",
+                   "ifx_attention_prefill_tcgen05_parts"):
             getattr(self.lib, fn).restype = ctypes.c_int
         self.lib.ifx_delta_rule_scratch_floats.restype = ctypes.c_longlong
         self.lib.ifx_chunk_scan_scratch_floats.restype = ctypes.c_longlong
         self.lib.ifx_delta_chunks_scratch_floats.restype = ctypes.c_longlong
+        self.lib.ifx_attention_prefill_tcgen05_parts_bytes.restype = ctypes.c_longlong
         # long spans of a bfloat16 run's recurrences by stretches of 64 tokens (0: token after token, for comparisons)
         self.chunk_scans = os.environ.get("INFERFLUX_B200_CHUNK_SCANS", "1") != "0"
         self.lib.ifx_sample_scratch_bytes.restype = ctypes.c_longlong
@@ -677,6 +679,7 @@ class CudaKernels:
             io.pending_tensor, io.pending_parts, io.pending_splits = pending.data_ptr(), 0, 0
         parity = self._layer_parity = 1 - self._layer_parity
         io.parity = parity
+        io.prefill_parts = self.prefill_parts(ctx, m.nq, int(m.window or 0))
         io.ws, io.ws_bytes = ws.data_ptr(), ws.numel()
         rc = self.lib.ifx_layer_forward(step, layer, self._layer_io_ref, _stream())
         self.launches += io.launches
@@ -834,9 +837,15 @@ class CudaKernels:
             return out
         if num_tiles and self.tensor_core_prefill and self.lib.ifx_attention_prefill_tcgen05_supports(
                 d, cache.page_size):
-            _check(self.lib.ifx_attention_prefill_tcgen05(
+            parts = self.prefill_parts(ctx, nq, win)
+            room = None
+            if parts > 1:
+                room = torch.empty(int(self.lib.ifx_attention_prefill_tcgen05_parts_bytes(num_tiles, nq, d, parts)), dtype=torch.uint8,
+                                   device=q.device)
+                self.launches += 1
+            _check(self.lib.ifx_attention_prefill_tcgen05_parts(
                 _ptr(q), T, _ptr(kv), _ptr(table), _ptr(tiles), _ptr(ctx.req_slot), _ptr(out),
-                num_tiles, nq, nkv, d, *common, _ptr(self.error_flag), _stream()),
+                num_tiles, nq, nkv, d, *common, parts, _ptr(room), _ptr(self.error_flag), _stream()),
                 "attention (prompt portions, tcgen05)")
             self.launches += 1
         elif num_tiles:
@@ -857,6 +866,32 @@ class CudaKernels:
                 max_keys, _ptr(self.error_flag), _stream()), "attention (decoded tokens)")
             self.launches += 1
         return out
+
+    PREFILL_PART_TILES = 4     # key tiles (of 128) that a part of a prompt attention block keeps at least
+
+    def prefill_parts(self, ctx, nq, window):
+        """Parts of their keys that the prompt attention's left over blocks are cut into (1: whole).  A block takes up to 256 tokens of a
+        head and an SM to itself, so what is left behind whole rounds of 148 blocks leaves SMs idle for as long as its longest
+        block walks; with few blocks that is the whole grid.  Cut while every part keeps four tiles of 128 keys: with parts of
+        three or of six the times below are the same or up to 3 % longer, and below that adding the parts up takes what they save.
+        us, whole and cut: 28 heads, two requests' 2,500 tokens behind up to 4,000 (12 of 308 blocks left) 191 and 162, 384 tokens
+        behind 2,000 39.0 and 32.4; 12 heads, 512 tokens behind 3,000 (24 blocks, six parts) 61.9 and 30.2, 600 tokens behind 900
+        26.9 and 24.6, 1,024 tokens 24.4 and 23.8."""
+        blocks = ctx.extra_len["attn.prefill_tiles"] // 4 * nq
+        left = blocks % 148
+        if not 0 < left <= 74:
+            return 1
+        items, longest = -(-left // nq), 0                 # the first items' blocks run last
+        for start, n in ctx.spans:
+            if n == 1:
+                continue
+            for off in range(0, n, self.PREFILL_TILE):
+                first, end = start + off, start + min(n, off + self.PREFILL_TILE)
+                longest = max(longest, -(-end // 128) - (max(0, first - window + 1) // 128 if window else 0))
+                items -= 1
+                if not items:
+                    return max(1, min(148 // left, longest // self.PREFILL_PART_TILES, 8))
+        return 1
 
     @staticmethod
     def decode_splits(num_tokens, nkv, max_keys, max_splits=8):
