@@ -76,6 +76,7 @@ struct IfxLayerIO {
   float* out_parts;
   int out_splits, launches, library_calls;
   int prefill_parts;          // in: parts of the prompt attention's left over blocks (CudaKernels.prefill_parts)
+  int least_decode_splits, pad0;   // in: parts of a decoded token's keys at least (CudaKernels.least_decode_splits)
 };
 
 namespace {
@@ -327,7 +328,9 @@ extern "C" int ifx_layer_forward(const IfxStepArgs* s, const IfxLayerArgs* l, If
                                   l->scale, IFX_DT_BF16, st));
       } else {
         const int max_keys = l->window > 0 && l->window < s->max_kv_len ? l->window : s->max_kv_len;
-        const int splits = decode_splits(s->num_decode, nkv, max_keys, ifx_attention_decode_max_splits(d, l->page_size));
+        const int most = ifx_attention_decode_max_splits(d, l->page_size);
+        int splits = decode_splits(s->num_decode, nkv, max_keys, most);
+        if (splits < io->least_decode_splits) splits = io->least_decode_splits < most ? io->least_decode_splits : most;
         RUN(ifx_attention_decode_bf16(q, l->kv_pool, l->block_table, s->decode_meta, attn, s->num_decode, nq, nkv, d,
                                       l->page_size, l->max_blocks, l->num_pages, l->window, l->scale, splits, max_keys,
                                       s->error_flag, decode_st));

@@ -129,7 +129,7 @@ class _LayerIO(ctypes.Structure):
     """IfxLayerIO: what changes from call to call, and what comes back."""
     _fields_ = [("x", _P), ("pending_tensor", _P), ("pending_parts", _P), ("pending_splits", _I), ("parity", _I),
                 ("ws", _P), ("ws_bytes", _LL), ("out_tensor", _P), ("out_parts", _P), ("out_splits", _I),
-                ("launches", _I), ("library_calls", _I), ("prefill_parts", _I)]
+                ("launches", _I), ("library_calls", _I), ("prefill_parts", _I), ("least_decode_splits", _I), ("pad0", _I)]
 
 
 class CudaKernels:
@@ -679,6 +679,7 @@ class CudaKernels:
             io.pending_tensor, io.pending_parts, io.pending_splits = pending.data_ptr(), 0, 0
         parity = self._layer_parity = 1 - self._layer_parity
         io.parity = parity
+        io.least_decode_splits = self.least_decode_splits(ctx, ctx.extra_len.get("attn.decode_rows", 0), m.nkv, m.d, int(m.window or 0))
         io.prefill_parts = self.prefill_parts(ctx, m.nq, int(m.window or 0))
         io.ws, io.ws_bytes = ws.data_ptr(), ws.numel()
         rc = self.lib.ifx_layer_forward(step, layer, self._layer_io_ref, _stream())
@@ -706,16 +707,22 @@ class CudaKernels:
         attn.decode_rows[D] (flat indices of spans of one token), attn.decode_meta[D,4] (flat index,
         position, slot, 0: what the decode kernel needs of a token, in one 16-byte load),
         attn.prefill_tiles[P,4] (request, first flat row, rows, first position) for longer spans."""
-        rows, meta, tiles, base = [], [], [], 0
+        rows, single, tiles, base = [], [], [], 0
         for r, ((start, n), slot) in enumerate(zip(ctx.spans, ctx.slots_host)):
             if n == 1:
                 rows.append(base)
-                meta.extend((base, start, int(slot), 0))
+                single.append((base, start, int(slot), 0))
             else:
                 for off in range(0, n, self.PREFILL_TILE):
                     tiles.extend((r, base + off, min(self.PREFILL_TILE, n - off), start + off))
             base += n
-        return {"attn.decode_rows": rows, "attn.decode_meta": meta, "attn.prefill_tiles": tiles}
+        # Longest first, for then no long one starts when the others end (28 heads, 40 tokens at up to 4,200 keys: 62.0 -> 56.4 us;
+        # 64 at up to 8,000: 108 -> 105).  Up to 16 tokens all blocks run at once whatever the order (8 tokens: 22.4, sorted 23.6).
+        if len(single) > 16:
+            single.sort(key=lambda m: -m[1])
+        # (longest, sum) of the decoded tokens' keys, for least_decode_splits; a captured step takes it back
+        ctx.decode_keys = (1 + max(m[1] for m in single), len(single) + sum(m[1] for m in single)) if single else None
+        return {"attn.decode_rows": rows, "attn.decode_meta": [v for m in single for v in m], "attn.prefill_tiles": tiles}
 
     @staticmethod
     def small_attention_grid(ctx, nkv):
@@ -860,7 +867,8 @@ class CudaKernels:
                 self._attention_generic(q, kv, table, ctx, decode_rows, n, out, nq, nkv, d, common)
                 return out
             max_keys = int(ctx.max_kv_len if not win else min(win, ctx.max_kv_len))
-            splits = self.decode_splits(n, nkv, max_keys, int(self.lib.ifx_attention_decode_max_splits(d, cache.page_size)))
+            most = int(self.lib.ifx_attention_decode_max_splits(d, cache.page_size))
+            splits = max(self.decode_splits(n, nkv, max_keys, most), min(most, self.least_decode_splits(ctx, n, nkv, d, win)))
             _check(self.lib.ifx_attention_decode_bf16(
                 _ptr(q), _ptr(kv), _ptr(table), _ptr(decode_meta), _ptr(out), n, nq, nkv, d, *common, splits,
                 max_keys, _ptr(self.error_flag), _stream()), "attention (decoded tokens)")
@@ -892,6 +900,21 @@ class CudaKernels:
                 if not items:
                     return max(1, min(148 // left, longest // self.PREFILL_PART_TILES, 8))
         return 1
+
+    @staticmethod
+    def least_decode_splits(ctx, num_tokens, nkv, d, window):
+        """Parts that a decoded token's keys are cut into at least, where the tokens of a step have uneven numbers of keys: with a
+        block a token and head the longest alone decides how long the step takes, and the others' SMs idle.  Parts cost a
+        prologue and a merge each, so a token's keys have to be long, and even steps, whose blocks end together, keep
+        decode_splits.  us, heads of 128, with 1 / 2 / 4 parts, longest first: 28 + 4 heads, 40 tokens at 4,400 keys in the
+        mean and 7,800 at most 87 / 65 / 62, 48 at 4,100 and 7,900 97 / 75 / 70, 64 at 4,400 and 7,900 105 / 102 / 97, 48 at 2,200 and
+        4,100 63 / 56 / 58, 64 at 1,700 and 3,000 53.8 / 55.5 / 61; even, 64 at 4,096 82 / 90 / 100, 40 at 7,900 102 / 136 / 117;
+        12 + 2 heads, 40 at 4,400 and 7,800 64 / 54 / 46, 48 at 2,900 and 5,800 51 / 46 / 40."""
+        keys = getattr(ctx, "decode_keys", None)
+        if keys is None or window or num_tokens * nkv > 296 or keys[0] * num_tokens * 2 < keys[1] * 3:
+            return 1
+        size = keys[0] * d
+        return 4 if size >= 5600 * 128 else 2 if size >= 4000 * 128 else 1
 
     @staticmethod
     def decode_splits(num_tokens, nkv, max_keys, max_splits=8):

@@ -192,6 +192,7 @@ class ModelRunner:
             ctx.rebind(static)
             self._relay(ctx)
             ctx.max_kv_len = bucket                        # what depends on the context is fixed per bucket
+            ctx.decode_keys = None                         # and how uneven it is does not hold for later steps
             torch.cuda.synchronize(self.device)
             graph = torch.cuda.CUDAGraph()
             launches = self.kernels.launches
