@@ -15,6 +15,9 @@
 // per token and head) norms and gates.  Everything is float32, and every sum's order is a function of the head size
 // alone, so a token's result does not depend on how its request's tokens were cut into steps or on what else is in the
 // batch.
+//
+// Long spans of a bfloat16 run go to delta_chunks.cu instead of delta_scan (DELTA_CHUNKS_MIN_SPAN in ops.py), where stretches of 64
+// tokens are products on the tensor cores; preparation and finish are these.
 #include "common.cuh"
 
 namespace ifx {

@@ -1,5 +1,6 @@
 // Attention over cached latents on the tensor cores (bfloat16), for prompt portions
-// and decoded tokens alike.  The latent of a key serves all heads as key and as
+// and decoded tokens alike: every size that latent_prompt_tcgen05.cu (prompt portions) and
+// latent_decode.cu (decoded tokens) do not take, and steps that mix the two.  The latent of a key serves all heads as key and as
 // value, so a thread block takes a tile of one request's tokens with ALL their heads
 // as its rows, (token, head) pairs, and every latent tile it stages in shared memory
 // is used by all of them, for the scores and for the weighted sum:

@@ -25,8 +25,8 @@
 // Every wait is bounded; a wait that runs out sets *error_flag.
 //
 // Bound: the tensor pipe (576 multiply-adds a score) beside 64 exponentials a thread and tile.  2,048 tokens of 12 heads:
-// latent_attention_mma_kernel and its merge 302 us, this 55 (a block with the last tokens walks 16 tiles at 3.2 us; the heads of
-// 192 blocks on 148 SMs).  100 tokens behind 2,000: 17 us and 4 of merge.
+// latent_attention_mma_kernel and its merge 302 us, this 55 (192 blocks on 148 SMs; one that holds the last tokens
+// walks 16 tiles at 3.2 us).  100 tokens behind 2,000: 17 us and 4 of merge.
 #include "common.cuh"
 #include "ptx_sm100.cuh"
 

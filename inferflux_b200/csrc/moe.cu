@@ -12,8 +12,9 @@
 //   moe_down      out[t] = sum over the token's choices, in their order, of weight * (W_down[e] act[p]), or
 //                 weight * h[t] for an expert without weights
 //
-// Steps with many tokens in bfloat16 sort their (token, choice) pairs by expert instead and multiply whole tiles on the
-// tensor cores (the grouped modes of gemm_tcgen05.cu):
+// In bfloat16 the work goes one of three ways (CudaKernels.moe_kernels has the rule and its measurements): the kernels of this file
+// for a few tokens, the stream of moe_stream_tcgen05.cu up to a few hundred pairs, whole tiles above.  The tiles sort their
+// (token, choice) pairs by expert first and multiply on the tensor cores (the grouped modes of gemm_tcgen05.cu):
 //
 //   moe_sort      every expert's pairs get a stretch of rows that starts on a multiple of 128; per row the pair it
 //                 holds (or -1) and the pair's weight (or 0); per 128-row tile its expert (or -1); per pair its row
