@@ -290,7 +290,8 @@ __global__ void __launch_bounds__(128, 3) latent_attention_mma_kernel(   // 32 .
 
 // One block per (token, head), a thread per latent column: adds the parts in split order, counts the sink,
 // normalises.  The parts' maxima and sums go through shared memory once; the columns' loads of different parts
-// are independent, four in flight.
+// are independent, four in flight.  A part that its kernel left unwritten is marked by a denominator below zero; every other
+// part is read whatever its weight, since 0 times a number that is not finite has to arrive in the result.
 constexpr int kMaxSplits = 64;
 
 __global__ void __launch_bounds__(256) latent_merge_kernel(const float* __restrict__ part_o,
@@ -299,6 +300,7 @@ __global__ void __launch_bounds__(256) latent_merge_kernel(const float* __restri
                                                            __nv_bfloat16* __restrict__ out, int total_rows, int heads,
                                                            int rank, int splits, const float* __restrict__ gate) {
   __shared__ float w_s[kMaxSplits];
+  __shared__ bool written_s[kMaxSplits];
   __shared__ float inv_s;
   const int row = blockIdx.x, c = threadIdx.x;
   if (c < 32) {                                                        // one warp: weights of the parts and the denominator
@@ -317,7 +319,10 @@ __global__ void __launch_bounds__(256) latent_merge_kernel(const float* __restri
     for (int i = 0; i < kMaxSplits / 32; ++i) {
       const int s = c + 32 * i;
       const float w = (ml[i].x == -INFINITY || m == -INFINITY) ? 0.0f : exp2f(ml[i].x - m);
-      if (s < splits) w_s[s] = w;
+      if (s < splits) {
+        w_s[s] = w;
+        written_s[s] = !(ml[i].y < 0.0f);                                // (a denominator that is not a number was written)
+      }
       l = fmaf(ml[i].y, w, l);
     }
     l = warp_sum(l);
@@ -329,8 +334,8 @@ __global__ void __launch_bounds__(256) latent_merge_kernel(const float* __restri
   const float* po = part_o + (size_t)row * rank + c;
   const size_t step = (size_t)total_rows * rank;
   float acc = 0.0f;
-  int s = 0;                                                           // a part of weight zero may not have been written
-  auto part = [&](int i) { return w_s[i] != 0.0f ? po[(size_t)i * step] : 0.0f; };
+  int s = 0;
+  auto part = [&](int i) { return written_s[i] ? po[(size_t)i * step] : 0.0f; };
   for (; s + 4 <= splits; s += 4) {
     const float a0 = part(s), a1 = part(s + 1), a2 = part(s + 2), a3 = part(s + 3);
     acc = fmaf(a0, w_s[s], acc);

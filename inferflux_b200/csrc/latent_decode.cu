@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(kLdWarps * 32, 2) latent_decode_kernel(
   const int k0 = (lo & ~(kLdKeys - 1)) + blockIdx.z * stretch, k1 = min(hi, k0 + stretch);
   const size_t row0 = (size_t)item.y * heads + h0;                     // (token, head)
   if (k0 >= hi) {                                                      // this token's keys are fewer
-    if (gridDim.z > 1 && tid < nh) part_ml[(size_t)blockIdx.z * total_rows + row0 + tid] = make_float2(-INFINITY, 0.0f);
+    if (gridDim.z > 1 && tid < nh) part_ml[(size_t)blockIdx.z * total_rows + row0 + tid] = make_float2(-INFINITY, -1.0f);     // not written
     return;
   }
   const int tiles = (k1 - k0 + kLdKeys - 1) / kLdKeys;
@@ -221,8 +221,8 @@ __global__ void __launch_bounds__(kLdWarps * 32, 2) latent_decode_kernel(
       m = fmaxf(m, ml_s[w * 16 + r].x);
     }
 #pragma unroll
-    for (int w = 0; w < kLdWarps; ++w)
-      if (ml_s[w * 16 + r].x > -INFINITY) l = fmaf(ml_s[w * 16 + r].y, exp2f(ml_s[w * 16 + r].x - m), l);
+    for (int w = 0; w < kLdWarps; ++w)                                  // (0 times a sum that is not a number stays none)
+      l = fmaf(ml_s[w * 16 + r].y, ml_s[w * 16 + r].x == -INFINITY ? 0.0f : exp2f(ml_s[w * 16 + r].x - m), l);
     if (gridDim.z > 1) {
       *reinterpret_cast<float2*>(part_o + ((size_t)blockIdx.z * total_rows + row0 + r) * kLdRank + c) = v;
       if (c == 0) part_ml[(size_t)blockIdx.z * total_rows + row0 + r] = make_float2(m, l);

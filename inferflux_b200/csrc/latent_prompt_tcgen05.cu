@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(kLpThreads, 1) latent_prompt_kernel(
     tb += blockIdx.z * per;
     te = min(te, tb + per);
     if (tb >= te) {
-      if ((int)threadIdx.x < rows) part_ml[(size_t)blockIdx.z * total_rows + row0 + threadIdx.x] = make_float2(-INFINITY, 0.0f);
+      if ((int)threadIdx.x < rows) part_ml[(size_t)blockIdx.z * total_rows + row0 + threadIdx.x] = make_float2(-INFINITY, -1.0f);   // not written
       return;
     }
   }

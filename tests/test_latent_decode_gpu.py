@@ -76,3 +76,50 @@ def test_against_64_bits(cuda_kernels, lens, heads, rot, page, window, extras):
     assert bool(torch.isfinite(got).all())
     assert float((got - want).abs().max()) <= 2.0 ** -7 * max(1.0, float(want.abs().max()))
     assert float((got - want).norm() / want.norm()) <= 2.0 ** -8
+
+
+@pytest.mark.parametrize("tiles", [False, True])                         # the kernel for decoded tokens, the tiles that share its merge
+@pytest.mark.parametrize("keys", [40, 700])                              # one part, several
+@pytest.mark.parametrize("what", ["query", "tile", "stretch", "outweighed"])
+def test_what_is_not_finite_arrives_in_the_result(cuda_kernels, what, keys, tiles):
+    """A query that is not a number, and keys that fill a warp's tile or a whole part, make their token's result no number, with
+    the keys in one part or in several; so does an infinity of weight zero in a part that another part outweighs."""
+    heads, rot, scale = 12, 64, 0.2
+    ctx, cache, view, rows, g = _setup(cuda_kernels, (keys, keys), rot, 16, None, 7)
+    ql = torch.randn(2, heads, 256 + rot, generator=g).to(BF)
+    if what == "outweighed":
+        ql[0, :, 7] = -1.0
+    w = torch.eye(256, dtype=BF).repeat(heads, 1).to(DEV)
+    from inferflux_b200.csrc.ops import TurnedQueries
+
+    def run():
+        flat = torch.cat((ql[..., :256], torch.zeros(2, heads, rot, dtype=BF)), -1).to(DEV).reshape(2, -1)
+        before, cuda_kernels.latent_decode = cuda_kernels.latent_decode, not tiles
+        try:
+            got = cuda_kernels.latent_attention(TurnedQueries(flat, ql.to(DEV).reshape(2, -1).clone()), w, w, None, heads, 256, 256, 256,
+                                                None, scale, ctx, view, rot=rot)
+        finally:
+            cuda_kernels.latent_decode = before
+        cuda_kernels.check_errors()
+        return got.view(2, heads, 256).float().cpu()
+
+    def row(key, value):
+        view.kv[cache.pages_of(0)[key // 16], 0, 0, key % 16] = value
+
+    clean = run()
+    assert bool(torch.isfinite(clean).all())
+    fine = torch.ones_like(clean, dtype=torch.bool)
+    if what == "query":
+        ql[0, 3] = float("nan")
+        fine[0, 3] = False
+    elif what in ("tile", "stretch"):
+        for key in range(16, 32) if what == "tile" else range(min(keys, 64)):
+            row(key, float("nan"))
+        fine[0] = False
+    else:
+        view.kv[cache.pages_of(0)[0], 0, 0, 5, 7] = float("inf")             # a score of -inf, a value of inf
+        row(keys - 1, (8.0 * ql[0, 0].float()).to(BF).to(DEV))               # head 0: the last key is all there is
+        fine[0] = False                                                  # (the product behind the sums spreads it over the columns)
+    got = run()
+    assert torch.equal(torch.isfinite(got), fine)
+    assert torch.equal(got[1], clean[1])

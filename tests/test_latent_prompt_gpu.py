@@ -118,3 +118,31 @@ def test_a_row_that_is_not_finite_reaches_those_who_see_it(cuda_kernels, value, 
         sees &= torch.arange(30, 430) < at + window
     assert torch.equal(got[~sees], clean[~sees])
     assert not bool(torch.isfinite(got[sees]).all(-1).any())
+
+
+@pytest.mark.parametrize("tiles", [False, True])                         # tcgen05, the mma.sync tiles that share its merge
+@pytest.mark.parametrize("context", [0, 1000])                           # one part, several
+@pytest.mark.parametrize("what", ["query", "keys"])
+def test_what_is_not_a_number_arrives_in_the_result(cuda_kernels, what, context, tiles):
+    """A query that is not a number, and keys that fill the first part, make the result of those who see them no number, with the
+    keys in one part or in several."""
+    spans, heads, rot, scale, at = [(context, 40)], 12, 64, 0.2, 17
+    ctx, cache, view, rows, g = _setup(cuda_kernels, spans, rot, 16, None, 8)
+    ql = torch.randn(40, heads, 256 + rot, generator=g).to(BF)
+    before, cuda_kernels.latent_prompt = cuda_kernels.latent_prompt, not tiles
+    try:
+        clean = _run(cuda_kernels, ctx, view, ql, heads, rot, None, scale, None, None)
+        bad = torch.zeros(40, heads, dtype=torch.bool)
+        if what == "query":
+            ql[at, 3] = float("nan")
+            bad[at, 3] = True
+        else:
+            for key in range(512 if context else 1):                     # with context: all that the first parts hold
+                view.kv[cache.pages_of(0)[key // 16], 0, 0, key % 16] = float("nan")
+            bad[:] = True
+        got = _run(cuda_kernels, ctx, view, ql, heads, rot, None, scale, None, None)
+    finally:
+        cuda_kernels.latent_prompt = before
+    assert bool(torch.isfinite(clean).all())
+    assert torch.equal(torch.isfinite(got), (~bad)[..., None].expand_as(got))
+    assert torch.equal(got[~bad], clean[~bad])
