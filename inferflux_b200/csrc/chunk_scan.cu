@@ -15,18 +15,22 @@
 // logarithm is taken: products of decays are multiplied up, so a decay may be zero and the error is that of the scan.
 // With a decay per key channel, pairs (t, s) within 16 tokens are multiplied up one by one; for pairs further apart the
 // product is cut at the beginnings of the 16s, q_t taking what lies in its own 16, k_s the rest of its own, and whole 16s
-// between as factors.  Matrix products run on the tensor cores with both operands split into two (chunk_scan.cuh).
+// between as factors.  Matrix products run on the tensor cores with both operands split into three (chunk_scan.cuh).
 //
 // A stretch that holds a number that is not finite is walked token by token by its block, so that such a number reaches
 // what it would reach in a scan and nothing in front of it.
 //
 // The order of the sums depends on where a span is cut into steps, so the float32 run keeps the scans.
 //
-// Bound: issue slots and shared-memory reads of chunk_local, two blocks an SM; mma.sync itself takes a fifth of the time, and the
-// states go through L2 twice (26 MB at 2,048 tokens of 12 heads of 128 x 128).  A warp's tile is 32 x 16, so that an operand
-// is split and read by few warps.  Measured, us, scan -> this (local + carry + reach): 12 heads of 128 x 128 with a constant
-// decay, 1,901 tokens of two prompts 343 -> 96 (58 + 11 + 27); wkv, 24 heads of 64, 2,048 tokens 522 -> 122 (71 + 10 + 19 and
-// its norm).  At 128 tokens 41 -> 33 for either; at 64 the scan is the faster.
+// Bound: issue slots of chunk_local, which split every operand into three and make eight products of them, and the states, which go
+// through L2 twice (26 MB at 2,048 tokens of 12 heads of 128 x 128).  A warp's tile is 32 x 16, so that an operand is split and read
+// by few warps.  Measured, us, scan -> this, one span of 2,048 tokens: constant decay, 12 heads of 128 x 128 590 -> 119; wkv, 24
+// heads of 64 (with its norm) 521 -> 123; a decay per token, 24 heads of 128 x 64 693 -> 116; per key channel, 12 heads of
+// 64 x 128 491 -> 92.  At 130 tokens 42 -> 31, 41 -> 30, 50 -> 31, 36 -> 25; at 64 the scan is the faster.
+// Errors of outputs and of the state against 64 bits (2-norm, scan and this, parameters where trained models have them, 2,048
+// tokens): constant decay 3.5e-7 and 1.1e-7, 3.8e-7 and 0.8e-7; a decay per token 1.65e-7 and 1.53e-7, 1.30e-7 and 1.22e-7; per key
+// channel 3.20e-6 and 3.16e-6, 3.98e-6 and 3.96e-6; wkv's state 9.14e-7 and 9.17e-7.  (With operands of 22 bits and sums left in the
+// tensor cores' accumulators it was 15, 9.8, 2.9 and 8.9e-7, a fifth faster.)
 #include "chunk_scan.cuh"
 
 namespace ifx {
@@ -46,7 +50,7 @@ struct ChunkArgs {
   int requests, heads, groups, dv;
   float inv_tau, q_scale;
   float* local;                                 // [stretches, heads, dv, dk]: what a stretch adds, then the state in front of it
-  float* total;                                 // decays of a whole stretch: [stretches, heads, dk], or [stretches, heads]
+  float* total;                                 // decays of a whole stretch: [stretches, heads, dk], or [stretches, heads] as two numbers each
   float* reach;                                 // queries times decays since the stretch's beginning [T, heads dk], or decays [T, heads]
   int key_rows;                                 // the request's state is [head, key channel, value channel]
   const float* x; float* prev_state; int C;     // CHUNK_WKV: the step's input rows, where the last one of a request goes
@@ -220,13 +224,17 @@ __global__ void __launch_bounds__(256) chunk_local_kernel(const ChunkArgs a) {
     }
   } else {
     if (tid < kChunk) {                                    // column s of the decays from s + 1 to t
-      float p = 1.0f;
+      Product p;
       for (int t = tid; t < kChunk; ++t) {
-        if (t > tid) p *= small[t];
-        a_s[t * kPitchA + tid] = p;
+        if (t > tid) p.times(small[t]);
+        a_s[t * kPitchA + tid] = p.value();
       }
-      small[2 * kChunk + tid] = p;                         // to the end
-      if (tid == 0 && z == 0) a.total[item] = p * small[0];
+      small[2 * kChunk + tid] = p.value();                 // to the end
+      if (tid == 0 && z == 0) {
+        p.times(small[0]);
+        a.total[2 * item] = p.value();
+        a.total[2 * item + 1] = (p.hi - p.value()) + p.lo;
+      }
     }
     __syncthreads();
     if (z == 0 && tid < n) a.reach[(size_t)(first + tid) * a.heads + h] = a_s[tid * kPitchA] * small[0];
@@ -269,19 +277,22 @@ __global__ void __launch_bounds__(256) chunk_local_kernel(const ChunkArgs a) {
       const int pair = task >> 1, i = pair == 0 ? 1 : pair < 3 ? 2 : 3, j = pair == 0 ? 0 : pair < 3 ? pair - 1 : pair - 3;
       const int r0 = i * kSub, c0 = j * kSub + (task & 1) * 8;
       float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll 4
-      for (int kk = 0; kk < DK; kk += 8) {
+#pragma unroll 2
+      for (int kk = 0; kk < DK; kk += 16) {
         FragA fa;
         FragB fb;
         load_a_rows(fa, q_s + r0 * PK + kk, PK, lane);
-        float2 b = read_b_rows(k_s + c0 * PK + kk, PK, lane);
+        float2 b[2] = {read_b_rows(k_s + c0 * PK + kk, PK, lane), read_b_rows(k_s + c0 * PK + kk + 8, PK, lane)};
         for (int m = j + 1; m < i; ++m) {
-          const float2 f = *reinterpret_cast<const float2*>(small + m * DK + kk + 2 * (lane & 3));
-          b.x *= f.x;
-          b.y *= f.y;
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            const float2 f = *reinterpret_cast<const float2*>(small + m * DK + kk + 8 * x + 2 * (lane & 3));
+            b[x].x *= f.x;
+            b[x].y *= f.y;
+          }
         }
-        fb.v[0].set(b.x);
-        fb.v[1].set(b.y);
+        fb.v[0].set(b[0].x, b[1].x);
+        fb.v[1].set(b[0].y, b[1].y);
         mma_split(c, fa, fb);
       }
       float* to = a_s + (r0 + (lane >> 2)) * kPitchA + c0 + 2 * (lane & 3);
@@ -295,8 +306,8 @@ __global__ void __launch_bounds__(256) chunk_local_kernel(const ChunkArgs a) {
       const int i = task < 2 ? 0 : task < 6 ? 1 : task < 12 ? 2 : 3;
       const int r0 = i * kSub, c0 = (task - i * (i + 1)) * 8;
       float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll 4
-      for (int kk = 0; kk < DK; kk += 8) {
+#pragma unroll 2
+      for (int kk = 0; kk < DK; kk += 16) {
         FragA fa;
         FragB fb;
         load_a_rows(fa, q_s + r0 * PK + kk, PK, lane);
@@ -313,20 +324,20 @@ __global__ void __launch_bounds__(256) chunk_local_kernel(const ChunkArgs a) {
   }
   __syncthreads();
   {                                                        // o: a warp's 16 value channels, the first and last or the middle 16s of tokens
-    const int m0 = warp >> 2, c0 = (warp & 3) * 16;        // rows of m0 and 3 - m0: ten steps of eight tokens either way
+    const int m0 = warp >> 2, c0 = (warp & 3) * 16;        // rows of m0 and 3 - m0: five steps of 16 tokens either way
     float acc[2][2][4] = {};
 #pragma unroll
-    for (int ks = 0; ks < 8; ++ks) {
-      if (ks >= 2 * (4 - m0)) break;
+    for (int ks = 0; ks < 4; ++ks) {
+      if (ks >= 4 - m0) break;
       FragB fb[2];
-      load_b_columns(fb[0], v_s + ks * 8 * kPitchV + c0, kPitchV, lane);
-      load_b_columns(fb[1], v_s + ks * 8 * kPitchV + c0 + 8, kPitchV, lane);
+      load_b_columns(fb[0], v_s + ks * 16 * kPitchV + c0, kPitchV, lane);
+      load_b_columns(fb[1], v_s + ks * 16 * kPitchV + c0 + 8, kPitchV, lane);
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         const int m = i == 0 ? m0 : 3 - m0;
-        if (ks < 2 * (m + 1)) {
+        if (ks <= m) {
           FragA fa;
-          load_a_single(fa, a_s + m * kSub * kPitchA + ks * 8, kPitchA, lane);
+          load_a_single(fa, a_s + m * kSub * kPitchA + ks * 16, kPitchA, lane);
           mma_split(acc[i][0], fa, fb[0]);
           mma_split(acc[i][1], fa, fb[1]);
         }
@@ -363,16 +374,20 @@ __global__ void __launch_bounds__(256) chunk_local_kernel(const ChunkArgs a) {
       }
     }
 #pragma unroll
-    for (int ks = 0; ks < 8; ++ks) {
+    for (int ks = 0; ks < 4; ++ks) {
       FragA fa[2];
-      load_a_columns(fa[0], v_s + ks * 8 * kPitchV + v0, kPitchV, lane);
-      load_a_columns(fa[1], v_s + ks * 8 * kPitchV + v0 + 16, kPitchV, lane);
+      load_a_columns(fa[0], v_s + ks * 16 * kPitchV + v0, kPitchV, lane);
+      load_a_columns(fa[1], v_s + ks * 16 * kPitchV + v0 + 16, kPitchV, lane);
+      float tail[4];                                       // decays from this lane's four tokens to the end
+#pragma unroll
+      for (int i = 0; i < 4; ++i) tail[i] = L::CHANNEL ? 1.0f : small[2 * kChunk + ks * 16 + (lane & 3) + 4 * i];
 #pragma unroll
       for (int x = 0; x < 2; ++x) {
-        const float* at = k_s + (ks * 8 + (lane & 3)) * PK + c0 + 8 * x + (lane >> 2);
+        const float* at = k_s + (ks * 16 + (lane & 3)) * PK + c0 + 8 * x + (lane >> 2);
+        auto key = [&](int i) { return at[4 * i * PK] * (L::CHANNEL ? rest[x][ks] : tail[i]); };
         FragB fb;
-        fb.v[0].set(at[0] * (L::CHANNEL ? rest[x][ks >> 1] : small[2 * kChunk + ks * 8 + (lane & 3)]));
-        fb.v[1].set(at[4 * PK] * (L::CHANNEL ? rest[x][ks >> 1] : small[2 * kChunk + ks * 8 + (lane & 3) + 4]));
+        fb.v[0].set(key(0), key(2));
+        fb.v[1].set(key(1), key(3));
         mma_split(acc[0][x], fa[0], fb);
         mma_split(acc[1][x], fa[1], fb);
       }
@@ -408,17 +423,29 @@ __global__ void __launch_bounds__(256) chunk_carry_kernel(const ChunkArgs a, int
   constexpr int U = 8;
   for (int c0 = 0; c0 < chunks; c0 += U) {
     float4 add[U], w[U];
+    float rest[U];                                         // what the one decay of a head lacks
 #pragma unroll
     for (int i = 0; i < U; ++i) {
       const size_t item = base + (size_t)min(c0 + i, chunks - 1) * a.heads;
       add[i] = *reinterpret_cast<const float4*>(a.local + (item * a.dv + v) * dk + c);
       if (CHANNEL) w[i] = *reinterpret_cast<const float4*>(a.total + item * dk + c);
-      else { const float f = a.total[item]; w[i] = make_float4(f, f, f, f); }
+      else {
+        const float2 f = *reinterpret_cast<const float2*>(a.total + 2 * item);
+        w[i] = make_float4(f.x, f.x, f.x, f.x);
+        rest[i] = f.y;
+      }
     }
 #pragma unroll
     for (int i = 0; i < U; ++i) {
       if (c0 + i < chunks) {
         *reinterpret_cast<float4*>(a.local + ((base + (size_t)(c0 + i) * a.heads) * a.dv + v) * dk + c) = S;
+        if (!CHANNEL) {
+          auto with_rest = [&](float s, float a) { return isfinite(s) ? fmaf(rest[i], s, a) : a; };
+          add[i].x = with_rest(S.x, add[i].x);
+          add[i].y = with_rest(S.y, add[i].y);
+          add[i].z = with_rest(S.z, add[i].z);
+          add[i].w = with_rest(S.w, add[i].w);
+        }
         S.x = fmaf(w[i].x, S.x, add[i].x);
         S.y = fmaf(w[i].y, S.y, add[i].y);
         S.z = fmaf(w[i].z, S.z, add[i].z);
@@ -478,8 +505,8 @@ __global__ void __launch_bounds__(256) chunk_reach_kernel(const ChunkArgs a) {
   }
   const int t0 = (warp >> 2) * 32, c0 = (warp & 3) * 16;   // a warp's 32 tokens and 16 value channels
   float acc[2][2][4] = {};
-#pragma unroll 4
-  for (int kk = 0; kk < DK; kk += 8) {
+#pragma unroll 2
+  for (int kk = 0; kk < DK; kk += 16) {
     FragB fb[2];
     load_b_rows(fb[0], s_s + c0 * PK + kk, PK, lane);
     load_b_rows(fb[1], s_s + (c0 + 8) * PK + kk, PK, lane);
@@ -572,7 +599,7 @@ int ifx_chunk_scan_supports(int requests, int heads, int dk, int dv) {
 // Floats of scratch.  per_channel: a decay per key channel (mode 0 and wkv).
 long long ifx_chunk_scan_scratch_floats(int num_tokens, int requests, int heads, int dk, int dv, int per_channel) {
   const long long chunks = chunks_at_most(num_tokens, requests);
-  const long long total = ((per_channel ? chunks * heads * dk : chunks * heads) + 3) / 4 * 4;
+  const long long total = ((per_channel ? chunks * heads * dk : 2 * chunks * heads) + 3) / 4 * 4;
   return chunks * heads * dv * dk + total + (per_channel ? (long long)num_tokens * heads * dk : (long long)num_tokens * heads);
 }
 
@@ -600,7 +627,7 @@ int ifx_chunk_decay_scan(const float* q, long long q_stride, const float* k, lon
   a.q_scale = q_scale;
   a.local = scratch;
   a.total = scratch + (size_t)chunks * heads * dv * dk;
-  a.reach = a.total + ((mode == 0 ? (size_t)chunks * heads * dk : (size_t)chunks * heads) + 3) / 4 * 4;
+  a.reach = a.total + ((mode == 0 ? (size_t)chunks * heads * dk : (size_t)2 * chunks * heads) + 3) / 4 * 4;
   return run_chunks(a, dk, mode, chunks, stream);
 }
 

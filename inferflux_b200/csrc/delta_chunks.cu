@@ -24,9 +24,11 @@
 // A stretch that holds a number that is not finite is walked token by token.  The order of the sums depends on where a span is
 // cut into steps, so the float32 run keeps the scan.
 //
-// Bound: delta_local, one block of 16 warps an SM (128 KB): issue slots for the splitting of operands (82,000 warp instructions a
-// stretch, the pipes of which are busy 37 % of the time) and twenty barriers.  2,048 tokens of 24 heads: delta_rule.cu's
-// three kernels 656 us, these 241 (154 + 47 + 23 + 18).
+// Bound: delta_local, one block of 16 warps an SM (128 KB): issue slots for the splitting of operands and twenty barriers.  2,048 tokens
+// of 24 heads: delta_rule.cu's three kernels 658 us, these 297.  Error of the state against 64 bits (2-norm, scan and this, 2,048
+// tokens): parameters where trained models have them 5.2e-7 and 4.6e-7, decays near one 1.76e-6 and 1.70e-6, random ones 0.95e-7
+// and 1.00e-7.  (With operands of 22 bits 241 us, 1.4e-7 in the last case, and 1.0e-6 in place of the scan's 4.6e-7 where 130 keys are
+// nearly the same.)
 #include "chunk_scan.cuh"
 
 namespace ifx {
@@ -53,7 +55,7 @@ struct DeltaChunkLayout {
 // acc = rows . columns^T of two tiles whose inner size runs along the rows; 16 rows x 16 columns a warp.
 __device__ __forceinline__ void dc_pairs(float (&acc)[2][4], const float* x, const float* y, int lane) {
 #pragma unroll
-  for (int kk = 0; kk < kDcD; kk += 8) {
+  for (int kk = 0; kk < kDcD; kk += 16) {
     FragA fa;
     FragB fb;
     load_a_rows(fa, x + kk, kDcP, lane);
@@ -64,15 +66,15 @@ __device__ __forceinline__ void dc_pairs(float (&acc)[2][4], const float* x, con
     }
   }
 }
-// acc += the first `steps` eights of a row of the matrix times the rows of a tile.
+// acc += the first `steps` sixteens of a row of the matrix times the rows of a tile.
 __device__ __forceinline__ void dc_times(float (&acc)[2][4], const float* a, const float* tile, int steps, int lane) {
   for (int ks = 0; ks < steps; ++ks) {
     FragA fa;
     FragB fb;
-    load_a_single(fa, a + ks * 8, kPitchA, lane);
+    load_a_single(fa, a + ks * 16, kPitchA, lane);
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-      load_b_columns(fb, tile + ks * 8 * kDcP + j * 8, kDcP, lane);
+      load_b_columns(fb, tile + ks * 16 * kDcP + j * 8, kDcP, lane);
       mma_split(acc[j], fa, fb);
     }
   }
@@ -80,13 +82,13 @@ __device__ __forceinline__ void dc_times(float (&acc)[2][4], const float* a, con
 // acc = columns of one tile . columns of another, over the tokens.
 __device__ __forceinline__ void dc_over_tokens(float (&acc)[2][4], const float* x, const float* y, int lane) {
 #pragma unroll
-  for (int ks = 0; ks < 8; ++ks) {
+  for (int ks = 0; ks < 4; ++ks) {
     FragA fa;
     FragB fb;
-    load_a_columns(fa, x + ks * 8 * kDcP, kDcP, lane);
+    load_a_columns(fa, x + ks * 16 * kDcP, kDcP, lane);
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-      load_b_columns(fb, y + ks * 8 * kDcP + j * 8, kDcP, lane);
+      load_b_columns(fb, y + ks * 16 * kDcP + j * 8, kDcP, lane);
       mma_split(acc[j], fa, fb);
     }
   }
@@ -176,22 +178,23 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_local_kernel(const DeltaC
   // ---------------------------------------------------------- decays from the middle: x_s holds G_t / G_31 for t > 31, its reciprocal up to there
   if (tid < 2 * kDcD) {
     const int c = tid & (kDcD - 1);
-    float p = 1.0f;
+    Product p;
     if (tid < kDcD) {
       x_s[31 * kDcP + c] = 1.0f;
 #pragma unroll 8
       for (int t = 30; t >= 0; --t) {
-        p *= a_s[(t + 1) * kPitchA + c];
-        x_s[t * kDcP + c] = p;
+        p.times(a_s[(t + 1) * kPitchA + c]);
+        x_s[t * kDcP + c] = p.value();
       }
-      mid[c] = p * a_s[c];                                 // from the stretch's beginning to the middle
+      p.times(a_s[c]);
+      mid[c] = p.value();                                  // from the stretch's beginning to the middle
     } else {
 #pragma unroll 8
       for (int t = 32; t < kChunk; ++t) {
-        p *= a_s[t * kPitchA + c];
-        x_s[t * kDcP + c] = p;
+        p.times(a_s[t * kPitchA + c]);
+        x_s[t * kDcP + c] = p.value();
       }
-      end[c] = p;
+      end[c] = p.value();
     }
   }
   __syncthreads();
@@ -207,7 +210,7 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_local_kernel(const DeltaC
   }
   __syncthreads();
 
-  const int wm = warp >> 2, wn = warp & 3, steps = 2 * (wm + 1);          // this warp's 16 rows and 16 columns
+  const int wm = warp >> 2, wn = warp & 3, steps = wm + 1;          // this warp's 16 rows and 16 columns
   const int tr = wm * 16 + (lane >> 2), tc = wn * 16 + 2 * (lane & 3);    // its first numbers: rows tr and tr + 8, columns tc + 8 j, + 1
   auto lower = [&](const float* rows, const float* cols, bool strict) {   // a_s = the lower triangle of rows . cols^T
     if (wn <= wm) {
@@ -261,7 +264,7 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_local_kernel(const DeltaC
       const int j = i + 1 + (task >> 3), c = (task & 7) * 16;
       float* tile = (c < kDcD ? x_s : u_s) + (c & (kDcD - 1));
       float acc[2][4] = {};
-      dc_times(acc, a_s + j * 16 * kPitchA + i * 16, tile + i * 16 * kDcP, 2, lane);
+      dc_times(acc, a_s + j * 16 * kPitchA + i * 16, tile + i * 16 * kDcP, 1, lane);
 #pragma unroll
       for (int x = 0; x < 2; ++x)
 #pragma unroll
@@ -359,12 +362,12 @@ __global__ void __launch_bounds__(kCarryThreads) delta_carry_kernel(const DeltaC
         for (int i = 0; i < 4; ++i) acc[0][i] = fmaf(p[(k0 + (i >> 1) * 8) * kDcP + j], s_s[(vc + (i & 1)) * kDcP + j], acc[0][i]);
     } else {
 #pragma unroll
-      for (int kk = 0; kk < kDcD; kk += 8) {
+      for (int kk = 0; kk < kDcD; kk += 16) {
         FragA fa;
         FragB fb;
         load_a_rows(fa, p + wm * 16 * kDcP + kk, kDcP, lane);
         load_b_rows(fb, s_s + wn * 8 * kDcP + kk, kDcP, lane);
-        mma_split(acc[(kk >> 3) & 1], fa, fb);
+        mma_split(acc[(kk >> 4) & 1], fa, fb);
       }
     }
     __syncthreads();                                       // the state has been read by all

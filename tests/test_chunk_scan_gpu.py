@@ -127,3 +127,29 @@ def test_which_spans_go_by_stretches(cuda_kernels):
     assert not fits(long, torch.float32) and not fits(short, torch.bfloat16)
     assert not fits(long, torch.bfloat16, 96) and not fits(long, torch.bfloat16, 64, 96)
     assert not fits(long, torch.bfloat16, rows=row[:, 1:]) and not fits(long, torch.bfloat16, rows=row[:, :64])
+
+
+@pytest.mark.parametrize("mode,H,G,dk,dv", [("sigmoid_root", 2, 2, 64, 128), ("softplus_step", 4, 1, 128, 64), ("constant", 3, 3, 128, 128),
+                                            ("constant", 3, 3, 64, 128)])
+def test_no_less_exact_than_the_scan(cuda_kernels, mode, H, G, dk, dv):
+    """Parameters where trained models have them.  Both make float32 sums of the same numbers; a tenth for chance."""
+    T = 500
+    g = torch.Generator().manual_seed(dk + dv)
+    uniform = lambda lo, hi, *s: torch.rand(*s, generator=g) * (hi - lo) + lo
+    wide, raw = _decay_inputs(mode, T, H, G, dk, dv, g, 0.5)
+    if mode == "sigmoid_root":
+        raw += uniform(-2.0, 4.0, H * dk)
+    kw = {"sigmoid_root": {"tau": 16.0, "q_scale": dk ** -0.5}, "constant": {"rate": torch.tensor([1 - 2 ** (-5 - 5 * i / H) for i in range(H)])},
+          "softplus_step": {"step_bias": uniform(-6, -2, H), "log_rate": uniform(0, 2.7, H), "skip": uniform(0, 0.2, H)}}[mode]
+    on = {k: v.to(DEV) if torch.is_tensor(v) else v for k, v in kw.items()}
+    cut = lambda t: (t[:, :G * dk], t[:, G * dk:2 * G * dk], t[:, 2 * G * dk:2 * G * dk + H * dv])
+    state_p = torch.zeros(1, H * dk * dv, dtype=F64)
+    want = PlainKernels(wide=True).decay_scan(*cut(wide.double()), None if raw is None else raw.double(), state_p, _Ctx((T,), (0,), "cpu"),
+                                              heads=H, groups=G, dk=dk, dv=dv, decay=mode, **kw).double()
+    errors = []
+    for dtype in (torch.bfloat16, torch.float32):
+        state = torch.zeros(1, H * dk * dv, device=DEV)
+        out = cuda_kernels.decay_scan(*cut(wide.to(DEV)), None if raw is None else raw.to(DEV), state, _Ctx((T,), (0,), DEV, dtype), heads=H,
+                                      groups=G, dk=dk, dv=dv, decay=mode, **on)
+        errors.append([float((a.double().cpu() - b).norm() / b.norm()) for a, b in ((out, want), (state, state_p))])
+    assert errors[0][0] <= 1.1 * errors[1][0] and errors[0][1] <= 1.1 * errors[1][1], errors

@@ -65,3 +65,21 @@ def test_a_number_that_is_not_finite_reaches_what_follows_it(cuda_kernels, block
     fine = torch.isfinite(walk)
     assert bool(fine[:t0].all()) and not bool(fine.all())
     assert float((y.float() - walk.float())[fine].abs().max()) <= 2.0 ** -7 * float(walk.float()[fine].abs().max())
+
+
+@pytest.mark.parametrize("tokens", [130, 640])
+def test_no_less_exact_than_the_scan(cuda_kernels, tokens):
+    """Parameters where trained models have them.  Both make float32 sums of the same numbers; a tenth for chance."""
+    H, D = 4, 64
+    HD = H * D
+    g = torch.Generator().manual_seed(tokens)
+    proj, w_raw = torch.randn(tokens, 5 * HD, generator=g), 0.5 * torch.randn(tokens, HD, generator=g)
+    w0, ab, nw = torch.rand(HD, generator=g) * 7 - 6, 0.5 * torch.rand(HD, generator=g), torch.ones(HD)
+    state_p = torch.zeros(1, HD * D, dtype=F64)
+    PlainKernels(wide=True).delta_rule_scan(proj.double(), w_raw.double(), w0, ab, nw, 1e-6, H, D, state_p, _Ctx((tokens,), (0,), "cpu"), F64)
+    errors = []
+    for chunks in (True, False):
+        state = torch.zeros(1, HD * D, device=DEV)
+        _scan(cuda_kernels, chunks, *(t.to(DEV) for t in (proj, w_raw, w0, ab, nw)), 1e-6, H, D, state, _Ctx((tokens,), (0,), DEV), BF)
+        errors.append(float((state.double().cpu() - state_p).norm() / state_p.norm()))
+    assert errors[0] <= 1.1 * errors[1], errors
