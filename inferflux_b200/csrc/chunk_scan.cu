@@ -17,8 +17,9 @@
 // product is cut at the beginnings of the 16s, q_t taking what lies in its own 16, k_s the rest of its own, and whole 16s
 // between as factors.  Matrix products run on the tensor cores with both operands split into three (chunk_scan.cuh).
 //
-// A stretch that holds a number that is not finite is walked token by token by its block, so that such a number reaches
-// what it would reach in a scan and nothing in front of it.
+// A stretch that holds a number that is not finite, or in which the product of a query and a key is none, is walked token by
+// token by its block, so that such a number reaches what it would reach in a scan and nothing in front of it, and so that a product
+// that a scan would not have formed spoils nothing.
 //
 // The order of the sums depends on where a span is cut into steps, so the float32 run keeps the scans.
 //
@@ -96,7 +97,7 @@ __global__ void __launch_bounds__(256) chunk_local_kernel(const ChunkArgs a) {
     }
     __syncthreads();
   }
-  bool bad = !L::CHANNEL && tid < kChunk && !isfinite(small[tid]);
+  bool bad = !L::CHANNEL && tid < kChunk && !splits(small[tid]);
   for (int e = tid; e < kChunk * DK / 4; e += 256) {
     const int t = e / (DK / 4), c = e % (DK / 4) * 4;
     const size_t row = (size_t)(first + t);
@@ -119,10 +120,10 @@ __global__ void __launch_bounds__(256) chunk_local_kernel(const ChunkArgs a) {
           w.x = expf(-expf(r.x + w0.x)); w.y = expf(-expf(r.y + w0.y));
           w.z = expf(-expf(r.z + w0.z)); w.w = expf(-expf(r.w + w0.w));
         }
-        bad = bad || !all_finite(w);
+        bad = bad || !splits(w);
       }
     }
-    bad = bad || !all_finite(q) || !all_finite(k);
+    bad = bad || !splits(q) || !splits(k);
     *reinterpret_cast<float4*>(q_s + t * PK + c) = q;
     *reinterpret_cast<float4*>(k_s + t * PK + c) = k;
     if (L::CHANNEL) *reinterpret_cast<float4*>(w_s + t * PK + c) = w;
@@ -131,11 +132,12 @@ __global__ void __launch_bounds__(256) chunk_local_kernel(const ChunkArgs a) {
     const int t = e >> 4, c = (e & 15) * 4;
     float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (t < n) v = *reinterpret_cast<const float4*>(a.v + (size_t)(first + t) * a.v_stride + (size_t)h * dv + z * 64 + c);
-    bad = bad || !all_finite(v);
+    bad = bad || !splits(v);
     *reinterpret_cast<float4*>(v_s + t * kPitchV + c) = v;
   }
   bad = __syncthreads_or(bad);
 
+  uint32_t largest = 0;                                    // of what is made here to be split
   // ---------------------------------------------------------- decays multiplied up; pairs of tokens within 16
   if (L::CHANNEL && !bad) {
     const int i = tid >> 6, s = (tid >> 2) & 15, part = tid & 3, tok = i * kSub + s;       // four lanes share a key
@@ -175,7 +177,9 @@ __global__ void __launch_bounds__(256) chunk_local_kernel(const ChunkArgs a) {
       }
       acc += __shfl_xor_sync(0xffffffffu, acc, 1);
       acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-      if (part == 0) a_s[row * kPitchA + tok] = t >= s ? acc : 0.0f;
+      acc = t >= s ? acc : 0.0f;
+      largest = max(largest, magnitude(acc));
+      if (part == 0) a_s[row * kPitchA + tok] = acc;
     }
     __syncthreads();
   }
@@ -230,6 +234,7 @@ __global__ void __launch_bounds__(256) chunk_local_kernel(const ChunkArgs a) {
         a_s[t * kPitchA + tid] = p.value();
       }
       small[2 * kChunk + tid] = p.value();                 // to the end
+      largest = magnitude(p.value());
       if (tid == 0 && z == 0) {
         p.times(small[0]);
         a.total[2 * item] = p.value();
@@ -244,35 +249,8 @@ __global__ void __launch_bounds__(256) chunk_local_kernel(const ChunkArgs a) {
   float* local = a.local + (item * dv + z * 64) * DK;
   const float skip = a.skip ? a.skip[h] : 0.0f;
 
-  if (bad) {                                               // token by token, a thread per value channel
-    if (tid < 64) {
-      float S[DK];                                         // in local memory: this path is for correctness
-#pragma unroll 1
-      for (int c = 0; c < DK; ++c) S[c] = 0.0f;
-      for (int t = 0; t < n; ++t) {
-        const float v = v_s[t * kPitchV + tid];
-        float acc = 0.0f, bonus = 0.0f;
-#pragma unroll 1
-        for (int c = 0; c < DK; ++c) {
-          const float q = q_s[t * PK + c], k = k_s[t * PK + c], w = L::CHANNEL ? w_s[t * PK + c] : small[t];
-          if (MODE == CHUNK_WKV) {
-            acc = fmaf(q, S[c], acc);
-            bonus = fmaf(q * a.u[(size_t)h * DK + c], k, bonus);
-          }
-          S[c] = fmaf(w, S[c], k * v);
-          if (MODE != CHUNK_WKV) acc = fmaf(q, S[c], acc);
-        }
-        if (MODE == CHUNK_WKV) acc = fmaf(bonus, v, acc);
-        out[t * out_row + tid] = a.skip ? fmaf(skip, v, acc) : acc;
-      }
-#pragma unroll 1
-      for (int c = 0; c < DK; ++c) local[(size_t)tid * DK + c] = S[c];
-    }
-    return;
-  }
-
   // ---------------------------------------------------------- pairs of tokens: 16 x 8 tiles of q . k
-  if (L::CHANNEL) {
+  if (!bad && L::CHANNEL) {
     for (int task = warp; task < 12; task += 8) {          // (i, j < i, half): rows of the i-th 16, columns of the j-th
       const int pair = task >> 1, i = pair == 0 ? 1 : pair < 3 ? 2 : 3, j = pair == 0 ? 0 : pair < 3 ? pair - 1 : pair - 3;
       const int r0 = i * kSub, c0 = j * kSub + (task & 1) * 8;
@@ -300,8 +278,10 @@ __global__ void __launch_bounds__(256) chunk_local_kernel(const ChunkArgs a) {
       to[1] = c[1];
       to[8 * kPitchA] = c[2];
       to[8 * kPitchA + 1] = c[3];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) largest = max(largest, magnitude(c[i]));
     }
-  } else {
+  } else if (!bad) {
     for (int task = warp; task < 20; task += 8) {          // the tiles at and below the diagonal
       const int i = task < 2 ? 0 : task < 6 ? 1 : task < 12 ? 2 : 3;
       const int r0 = i * kSub, c0 = (task - i * (i + 1)) * 8;
@@ -316,13 +296,48 @@ __global__ void __launch_bounds__(256) chunk_local_kernel(const ChunkArgs a) {
       }
       const int t = r0 + (lane >> 2), s = c0 + 2 * (lane & 3);
       float* to = a_s + t * kPitchA + s;
-      to[0] = s <= t ? to[0] * c[0] : 0.0f;
-      to[1] = s + 1 <= t ? to[1] * c[1] : 0.0f;
-      to[8 * kPitchA] = s <= t + 8 ? to[8 * kPitchA] * c[2] : 0.0f;
-      to[8 * kPitchA + 1] = s + 1 <= t + 8 ? to[8 * kPitchA + 1] * c[3] : 0.0f;
+      c[0] = s <= t ? to[0] * c[0] : 0.0f;
+      c[1] = s + 1 <= t ? to[1] * c[1] : 0.0f;
+      c[2] = s <= t + 8 ? to[8 * kPitchA] * c[2] : 0.0f;
+      c[3] = s + 1 <= t + 8 ? to[8 * kPitchA + 1] * c[3] : 0.0f;
+      to[0] = c[0];
+      to[1] = c[1];
+      to[8 * kPitchA] = c[2];
+      to[8 * kPitchA + 1] = c[3];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) largest = max(largest, magnitude(c[i]));
     }
   }
-  __syncthreads();
+  bad = __syncthreads_or(bad || largest >= kSplitLimit);
+  if (bad) {                                               // token by token, a thread per value channel (CHANNEL: q_s, k_s may be scaled)
+    if (tid < 64) {
+      float S[DK];                                         // in local memory: this path is for correctness
+#pragma unroll 1
+      for (int c = 0; c < DK; ++c) S[c] = 0.0f;
+      for (int t = 0; t < n; ++t) {
+        const float v = v_s[t * kPitchV + tid];
+        float acc = 0.0f, bonus = 0.0f;
+#pragma unroll 1
+        for (int c = 0; c < DK; ++c) {
+          const float q = L::CHANNEL ? a.q[(size_t)(first + t) * a.q_stride + (size_t)g * DK + c] * a.q_scale : q_s[t * PK + c];
+          const float k = L::CHANNEL ? a.k[(size_t)(first + t) * a.k_stride + (size_t)g * DK + c] : k_s[t * PK + c];
+          const float w = L::CHANNEL ? w_s[t * PK + c] : small[t];
+          if (MODE == CHUNK_WKV) {
+            acc = fmaf(q, S[c], acc);
+            bonus = fmaf(q * a.u[(size_t)h * DK + c], k, bonus);
+          }
+          S[c] = fmaf(w, S[c], k * v);
+          if (MODE != CHUNK_WKV) acc = fmaf(q, S[c], acc);
+        }
+        if (MODE == CHUNK_WKV) acc = fmaf(bonus, v, acc);
+        out[t * out_row + tid] = a.skip ? fmaf(skip, v, acc) : acc;
+      }
+#pragma unroll 1
+      for (int c = 0; c < DK; ++c) local[(size_t)tid * DK + c] = S[c];
+    }
+    return;
+  }
+
   {                                                        // o: a warp's 16 value channels, the first and last or the middle 16s of tokens
     const int m0 = warp >> 2, c0 = (warp & 3) * 16;        // rows of m0 and 3 - m0: five steps of 16 tokens either way
     float acc[2][2][4] = {};
@@ -486,7 +501,7 @@ __global__ void __launch_bounds__(256) chunk_reach_kernel(const ChunkArgs a) {
       }
     }
     const float4 s = *reinterpret_cast<const float4*>(state + (size_t)t * DK + c);        // row t: a value channel
-    bad = bad || !all_finite(q) || !all_finite(s);
+    bad = bad || !splits(q) || !splits(s);
     *reinterpret_cast<float4*>(q_s + t * PK + c) = q;
     *reinterpret_cast<float4*>(s_s + t * PK + c) = s;
   }

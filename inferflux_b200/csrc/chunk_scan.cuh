@@ -11,6 +11,12 @@ constexpr int kSub = 16;                   // tokens within which decays are mul
 constexpr int kPitchV = 64 + 8;            // floats from a row of 64 to the next: the reads below meet every bank once
 constexpr int kPitchA = 64 + 4;
 
+// What `splits` refuses, infinities and what is not a number, would come out of a product as something else than of a scan.
+// Whoever makes a number that is to be split looks at it first, and a stretch that holds another one goes token by token.
+constexpr uint32_t kSplitLimit = 0x7f800000u;
+__device__ __forceinline__ uint32_t magnitude(float x) { return __float_as_uint(x) & 0x7fffffffu; }
+__device__ __forceinline__ bool splits(float x) { return magnitude(x) < kSplitLimit; }
+__device__ __forceinline__ bool splits(float4 v) { return splits(v.x) && splits(v.y) && splits(v.z) && splits(v.w); }
 // Two float32, each as the sum of three bfloat16 of 8 bits: the upper half of its bits, the upper half of what that leaves, the
 // rest.  All 24 bits are kept.
 struct Split {
@@ -126,7 +132,5 @@ __device__ __forceinline__ int chunks_before(const int* __restrict__ cu_seqlens,
 }
 // The most stretches that num_tokens of num_requests can make.
 inline int chunks_at_most(int num_tokens, int num_requests) { return num_tokens / kChunk + num_requests; }
-
-__device__ __forceinline__ bool all_finite(float4 v) { return isfinite(v.x) && isfinite(v.y) && isfinite(v.z) && isfinite(v.w); }
 
 }  // namespace ifx

@@ -21,7 +21,8 @@
 // a product on the one side and a reciprocal on the other, both counted from the middle of the stretch.  Products run on the tensor
 // cores with split operands (chunk_scan.cuh); the triangular system goes by blocks of 16 rows, substituted in the blocks.
 //
-// A stretch that holds a number that is not finite is walked token by token.  The order of the sums depends on where a span is
+// A stretch that holds a number that is not finite, or in which one comes up that a scan would not have formed, is walked token by
+// token.  The order of the sums depends on where a span is
 // cut into steps, so the float32 run keeps the scan.
 //
 // Bound: delta_local, one block of 16 warps an SM (128 KB): issue slots for the splitting of operands and twenty barriers.  2,048 tokens
@@ -106,43 +107,46 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_local_kernel(const DeltaC
   const size_t item = (size_t)blockIdx.x * a.heads + h;
 
   // ---------------------------------------------------------- rows: queries, keys, values, how much is erased, unit keys, decays
-  bool bad = false;
+  auto load = [&]() {
+    bool bad = false;
 #pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    const int t = half * 32 + (tid >> 4), c = (tid & 15) * 4;             // sixteen neighbouring lanes a token
-    float4 r = make_float4(0.0f, 0.0f, 0.0f, 0.0f), k = r, v = r, e = r, w = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
-    if (t < n) {
-      const float* row = a.proj + (size_t)(first + t) * a.ld + h * kDcD + c;
-      r = *reinterpret_cast<const float4*>(row);
-      k = *reinterpret_cast<const float4*>(row + HD);
-      v = *reinterpret_cast<const float4*>(row + 2 * HD);
-      e = *reinterpret_cast<const float4*>(row + 4 * HD);
-      w = *reinterpret_cast<const float4*>(a.w_raw + (size_t)(first + t) * HD + h * kDcD + c);
-      const float4 b = *reinterpret_cast<const float4*>(a.a_bias + h * kDcD + c), w0 = *reinterpret_cast<const float4*>(a.w0 + h * kDcD + c);
-      e.x = dc_sigmoid(e.x + b.x); e.y = dc_sigmoid(e.y + b.y); e.z = dc_sigmoid(e.z + b.z); e.w = dc_sigmoid(e.w + b.w);
-      w.x = expf(-kDcFloor * dc_sigmoid(w.x + w0.x)); w.y = expf(-kDcFloor * dc_sigmoid(w.y + w0.y));
-      w.z = expf(-kDcFloor * dc_sigmoid(w.z + w0.z)); w.w = expf(-kDcFloor * dc_sigmoid(w.w + w0.w));
+    for (int half = 0; half < 2; ++half) {
+      const int t = half * 32 + (tid >> 4), c = (tid & 15) * 4;             // sixteen neighbouring lanes a token
+      float4 r = make_float4(0.0f, 0.0f, 0.0f, 0.0f), k = r, v = r, e = r, w = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+      if (t < n) {
+        const float* row = a.proj + (size_t)(first + t) * a.ld + h * kDcD + c;
+        r = *reinterpret_cast<const float4*>(row);
+        k = *reinterpret_cast<const float4*>(row + HD);
+        v = *reinterpret_cast<const float4*>(row + 2 * HD);
+        e = *reinterpret_cast<const float4*>(row + 4 * HD);
+        w = *reinterpret_cast<const float4*>(a.w_raw + (size_t)(first + t) * HD + h * kDcD + c);
+        const float4 b = *reinterpret_cast<const float4*>(a.a_bias + h * kDcD + c), w0 = *reinterpret_cast<const float4*>(a.w0 + h * kDcD + c);
+        e.x = dc_sigmoid(e.x + b.x); e.y = dc_sigmoid(e.y + b.y); e.z = dc_sigmoid(e.z + b.z); e.w = dc_sigmoid(e.w + b.w);
+        w.x = expf(-kDcFloor * dc_sigmoid(w.x + w0.x)); w.y = expf(-kDcFloor * dc_sigmoid(w.y + w0.y));
+        w.z = expf(-kDcFloor * dc_sigmoid(w.z + w0.z)); w.w = expf(-kDcFloor * dc_sigmoid(w.w + w0.w));
+      }
+      float ss = fmaf(k.x, k.x, fmaf(k.y, k.y, fmaf(k.z, k.z, k.w * k.w)));
+#pragma unroll
+      for (int o = 1; o < 16; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      const float inv = 1.0f / sqrtf(ss + 1e-6f);
+      const float4 u = make_float4(k.x * inv, k.y * inv, k.z * inv, k.w * inv);
+      e.x *= u.x; e.y *= u.y; e.z *= u.z; e.w *= u.w;
+      bad = bad || !splits(r) || !splits(k) || !splits(v) || !splits(e) || !splits(w) || !isfinite(ss);
+      *reinterpret_cast<float4*>(r_s + t * kDcP + c) = r;
+      *reinterpret_cast<float4*>(k_s + t * kDcP + c) = k;
+      *reinterpret_cast<float4*>(v_s + t * kDcP + c) = v;
+      *reinterpret_cast<float4*>(e_s + t * kDcP + c) = e;
+      *reinterpret_cast<float4*>(u_s + t * kDcP + c) = u;
+      *reinterpret_cast<float4*>(a_s + t * kPitchA + c) = w;
     }
-    float ss = fmaf(k.x, k.x, fmaf(k.y, k.y, fmaf(k.z, k.z, k.w * k.w)));
-#pragma unroll
-    for (int o = 1; o < 16; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    const float inv = 1.0f / sqrtf(ss + 1e-6f);
-    const float4 u = make_float4(k.x * inv, k.y * inv, k.z * inv, k.w * inv);
-    e.x *= u.x; e.y *= u.y; e.z *= u.z; e.w *= u.w;
-    bad = bad || !all_finite(r) || !all_finite(k) || !all_finite(v) || !all_finite(e) || !all_finite(w) || !isfinite(ss);
-    *reinterpret_cast<float4*>(r_s + t * kDcP + c) = r;
-    *reinterpret_cast<float4*>(k_s + t * kDcP + c) = k;
-    *reinterpret_cast<float4*>(v_s + t * kDcP + c) = v;
-    *reinterpret_cast<float4*>(e_s + t * kDcP + c) = e;
-    *reinterpret_cast<float4*>(u_s + t * kDcP + c) = u;
-    *reinterpret_cast<float4*>(a_s + t * kPitchA + c) = w;
-  }
-  bad = __syncthreads_or(bad);
+    return bad;
+  };
+  bool bad = __syncthreads_or(load());
   float* out = a.out + (size_t)first * HD + h * kDcD;
   float* reach = a.reach + (size_t)first * HD + h * kDcD;
   float *local = a.local + item * kDcD * kDcD, *trans = a.trans + item * kDcD * kDcD;
 
-  if (bad) {                                               // token by token: 64 columns of values, 64 of the unit matrix
+  auto walk = [&]() {                                      // token by token: 64 columns of values, 64 of the unit matrix
     if (tid < 2 * kDcD) {
       const bool unit = tid >= kDcD;
       const int j = tid & (kDcD - 1);
@@ -172,6 +176,9 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_local_kernel(const DeltaC
 #pragma unroll 1
       for (int i = 0; i < kDcD; ++i) (unit ? trans[i * kDcD + j] : local[j * kDcD + i]) = S[i];
     }
+  };
+  if (bad) {
+    walk();
     return;
   }
 
@@ -198,6 +205,8 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_local_kernel(const DeltaC
     }
   }
   __syncthreads();
+  uint32_t largest = 0;                                    // of what is made here to be split
+  auto note = [&](float x) { largest = max(largest, magnitude(x)); };
 #pragma unroll
   for (int e8 = 0; e8 < kChunk * kDcD / kDcThreads; ++e8) {
     const int e = e8 * kDcThreads + tid, t = e >> 6, c = e & 63;
@@ -207,6 +216,10 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_local_kernel(const DeltaC
     u_s[t * kDcP + c] *= before;
     k_s[t * kDcP + c] *= back;
     e_s[t * kDcP + c] *= back;
+    note(r_s[t * kDcP + c]);
+    note(u_s[t * kDcP + c]);
+    note(k_s[t * kDcP + c]);
+    note(e_s[t * kDcP + c]);
   }
   __syncthreads();
 
@@ -221,7 +234,9 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_local_kernel(const DeltaC
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int t = tr + (i >> 1) * 8, s = tc + j * 8 + (i & 1);
-          a_s[t * kPitchA + s] = (strict ? s < t : s <= t) ? acc[j][i] : 0.0f;
+          const float x = (strict ? s < t : s <= t) ? acc[j][i] : 0.0f;
+          a_s[t * kPitchA + s] = x;
+          note(x);
         }
     }
   };
@@ -252,11 +267,13 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_local_kernel(const DeltaC
       float x[16];
 #pragma unroll
       for (int r = 0; r < 16; ++r) x[r] = col[r * kDcP];
+      note(x[0]);
 #pragma unroll
       for (int r = 1; r < 16; ++r) {
 #pragma unroll
         for (int q = 0; q < r; ++q) x[r] = fmaf(-m[r * kPitchA + q], x[q], x[r]);
         col[r * kDcP] = x[r];
+        note(x[r]);
       }
     }
     __syncthreads();
@@ -274,7 +291,12 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_local_kernel(const DeltaC
     __syncthreads();
   }
   lower(r_s, e_s, false);                                  // B
-  __syncthreads();
+  if (__syncthreads_or(largest >= kSplitLimit)) {
+    load();
+    __syncthreads();
+    walk();
+    return;
+  }
   {
     float bx[2][4] = {}, bu[2][4] = {};
     dc_times(bx, a_s + wm * 16 * kPitchA, x_s + wn * 16, steps, lane);
@@ -329,7 +351,7 @@ __global__ void __launch_bounds__(kCarryThreads) delta_carry_kernel(const DeltaC
   bool bad = false;                                        // numbers of the state, the matrix that are not finite: split products would lose them
   for (int e = tid; e < 16 * kDcD; e += kCarryThreads) {
     const float v = st[(e >> 4) * kDcD + v0 + (e & 15)];
-    bad = bad || !isfinite(v);
+    bad = bad || !splits(v);
     s_s[(e & 15) * kDcP + (e >> 4)] = v;
   }
   auto copy = [](float* to, const float* from) {
@@ -349,7 +371,7 @@ __global__ void __launch_bounds__(kCarryThreads) delta_carry_kernel(const DeltaC
     asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 1;" ::: "memory");
     const float *p = p_s + (c & 1) * kCarryTrans, *l = l_s + (c & 1) * kCarryState;
     for (int e = tid; e < kDcD * 16; e += kCarryThreads)
-      bad = bad || !all_finite(*reinterpret_cast<const float4*>(p + (e >> 4) * kDcP + (e & 15) * 4));
+      bad = bad || !splits(*reinterpret_cast<const float4*>(p + (e >> 4) * kDcP + (e & 15) * 4));
     bad = __syncthreads_or(bad);
     *reinterpret_cast<float4*>(a.local + (base + (size_t)c * a.heads) * kDcD * kDcD + (size_t)v0 * kDcD + tid * 4) =
         *reinterpret_cast<const float4*>(s_s + (tid >> 4) * kDcP + (tid & 15) * 4);       // the state in front of the stretch
@@ -376,7 +398,7 @@ __global__ void __launch_bounds__(kCarryThreads) delta_carry_kernel(const DeltaC
     for (int i = 0; i < 4; ++i) {
       const int k = k0 + (i >> 1) * 8, v = vc + (i & 1);
       const float x = acc[0][i] + acc[1][i] + l[v * kDcP + k];
-      bad = bad || !isfinite(x);
+      bad = bad || !splits(x);
       s_s[v * kDcP + k] = x;
     }
     __syncthreads();

@@ -153,3 +153,29 @@ def test_no_less_exact_than_the_scan(cuda_kernels, mode, H, G, dk, dv):
                                       groups=G, dk=dk, dv=dv, decay=mode, **on)
         errors.append([float((a.double().cpu() - b).norm() / b.norm()) for a, b in ((out, want), (state, state_p))])
     assert errors[0][0] <= 1.1 * errors[1][0] and errors[0][1] <= 1.1 * errors[1][1], errors
+
+
+@pytest.mark.parametrize("mode,H,G,dk,dv", [("sigmoid_root", 2, 2, 64, 64), ("softplus_step", 2, 1, 128, 64), ("constant", 2, 2, 64, 64)])
+def test_products_that_a_scan_does_not_form(cuda_kernels, mode, H, G, dk, dv):
+    """A query and a key whose product is beyond float32, beside a value that brings the state back into range: finite in the scan."""
+    T, t0 = 200, 70
+    g = torch.Generator().manual_seed(6)
+    wide, raw = _decay_inputs(mode, T, H, G, dk, dv, g, 1.0)
+    wide[t0, :2 * G * dk] *= 1e25
+    wide[t0, 2 * G * dk:] *= 1e-30
+    wide = wide.to(DEV)
+    vec = [torch.rand(H, generator=g).to(DEV) for _ in range(3)]
+    kw = {"sigmoid_root": {"tau": 3.0}, "softplus_step": {"step_bias": vec[0], "log_rate": vec[1], "skip": vec[2]},
+          "constant": {"rate": vec[0]}}[mode]
+    results = []
+    for dtype in (torch.bfloat16, torch.float32):
+        state = torch.zeros(1, H * dk * dv, device=DEV)
+        out = cuda_kernels.decay_scan(wide[:, :G * dk], wide[:, G * dk:2 * G * dk], wide[:, 2 * G * dk:2 * G * dk + H * dv],
+                                      None if raw is None else raw.to(DEV), state, _Ctx((T,), (0,), DEV, dtype), heads=H, groups=G, dk=dk,
+                                      dv=dv, decay=mode, **kw)
+        results.append((out.double(), state.double()))
+    (out, state), (walk, state_w) = results
+    assert bool(torch.isfinite(walk).all()) and bool(torch.isfinite(out).all())
+    size = walk.abs().amax(-1, keepdim=True)                                    # float32 sums of up to 200 terms
+    assert float(((out - walk).abs() / size).max()) <= 1e-4
+    assert float((state - state_w).abs().max()) <= 1e-5 * float(state_w.abs().max())

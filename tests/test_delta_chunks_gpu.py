@@ -83,3 +83,27 @@ def test_no_less_exact_than_the_scan(cuda_kernels, tokens):
         _scan(cuda_kernels, chunks, *(t.to(DEV) for t in (proj, w_raw, w0, ab, nw)), 1e-6, H, D, state, _Ctx((tokens,), (0,), DEV), BF)
         errors.append(float((state.double().cpu() - state_p).norm() / state_p.norm()))
     assert errors[0] <= 1.1 * errors[1], errors
+
+
+@pytest.mark.parametrize("block", [0, 1])
+def test_products_that_a_scan_does_not_form(cuda_kernels, block):
+    """Decays at their strongest, counted from a stretch's middle, take a query (a key) beyond float32 that a scan never scales."""
+    H, D, T, t0 = 2, 64, 200, 64 if block == 0 else 127
+    HD = H * D
+    g = torch.Generator().manual_seed(7)
+    proj, w_raw = torch.randn(T, 5 * HD, generator=g), torch.randn(T, HD, generator=g)
+    proj[t0, block * HD:(block + 1) * HD] *= 1e33 if block == 0 else 1e18
+    proj[t0, 2 * HD:3 * HD] *= 1.0 if block == 0 else 1e-18
+    if block == 1:                                                              # k k^T beyond float32 only where the stretch multiplies
+        proj[:, :HD] *= 1e18
+    w0, ab, nw = torch.full((HD,), 8.0), torch.randn(HD, generator=g), torch.ones(HD)
+    results = []
+    for chunks in (True, False):
+        state = torch.zeros(1, HD * D, device=DEV)
+        y = _scan(cuda_kernels, chunks, *(t.to(DEV) for t in (proj, w_raw, w0, ab, nw)), 1e-6, H, D, state, _Ctx((T,), (0,), DEV), BF)
+        results.append((y.double(), state.double()))
+    (y, state), (walk, state_w) = results
+    assert torch.equal(torch.isfinite(y), torch.isfinite(walk)) and bool(torch.isfinite(state_w).all())
+    fine = torch.isfinite(walk)
+    assert float((y - walk)[fine].abs().max()) <= 2.0 ** -7 * float(walk[fine].abs().max())
+    assert float((state - state_w).abs().max()) <= 1e-5 * float(state_w.abs().max())
