@@ -242,7 +242,10 @@ __global__ void __launch_bounds__(256) chunk_local_kernel(const ChunkArgs a) {
       }
     }
     __syncthreads();
-    if (z == 0 && tid < n) a.reach[(size_t)(first + tid) * a.heads + h] = a_s[tid * kPitchA] * small[0];
+    if (z == 0) {
+      if (tid < n) a.reach[(size_t)(first + tid) * a.heads + h] = a_s[tid * kPitchA] * small[0];
+      __syncthreads();                                     // read, before the products below go over it
+    }
   }
   float* out = a.out + (size_t)first * a.heads * dv + (size_t)h * dv + z * 64;
   const size_t out_row = (size_t)a.heads * dv;
