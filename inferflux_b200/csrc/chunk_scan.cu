@@ -48,7 +48,7 @@ struct ChunkArgs {
   float* out;                                   // [T, heads dv]
   const float* step_bias; const float* log_rate; const float* skip; const float* rate;      // per head
   const float* w0; const float* u;              // CHUNK_WKV: per head and key channel
-  int requests, heads, groups, dv;
+  int requests, min_span, heads, groups, dv;    // shorter spans are left to the scans token by token
   float inv_tau, q_scale;
   float* local;                                 // [stretches, heads, dv, dk]: what a stretch adds, then the state in front of it
   float* total;                                 // decays of a whole stretch: [stretches, heads, dk], or [stretches, heads] as two numbers each
@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(256) chunk_local_kernel(const ChunkArgs a) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int h = blockIdx.y, z = blockIdx.z, g = h / (a.heads / a.groups), dv = a.dv;
   int first, n;
-  if (!chunk_of(a.cu_seqlens, a.requests, blockIdx.x, first, n)) return;
+  if (!chunk_of(a.cu_seqlens, a.requests, a.min_span, blockIdx.x, first, n)) return;
   const size_t item = (size_t)blockIdx.x * a.heads + h;
 
   if (!L::CHANNEL) {                                       // decays and steps of the tokens; rows behind the last leave the state alone
@@ -426,18 +426,19 @@ __global__ void __launch_bounds__(256) chunk_local_kernel(const ChunkArgs a) {
 template <bool CHANNEL>
 __global__ void __launch_bounds__(256) chunk_carry_kernel(const ChunkArgs a, int dk) {
   const int r = blockIdx.x, h = blockIdx.y, e = blockIdx.z * 256 + threadIdx.x;
-  const int lo = a.cu_seqlens[r], span = a.cu_seqlens[r + 1] - lo, chunks = (span + kChunk - 1) / kChunk;
-  if (a.x != nullptr && h == 0 && blockIdx.z == 0 && span > 0) {           // the step's last input row
+  const int lo = a.cu_seqlens[r], span = a.cu_seqlens[r + 1] - lo, chunks = chunks_of(span, a.min_span);
+  if (chunks == 0) return;
+  if (a.x != nullptr && h == 0 && blockIdx.z == 0) {                       // the step's last input row
     float* to = a.prev_state + (long long)a.req_slot[r] * a.state_slot_stride;
     for (int i = threadIdx.x; i < a.C; i += 256) to[i] = a.x[(size_t)(lo + span - 1) * a.C + i];
   }
-  if (e >= a.dv * (dk / 4) || span == 0) return;
+  if (e >= a.dv * (dk / 4)) return;
   const int v = e / (dk / 4), c = e % (dk / 4) * 4;
   float* st = a.state + (long long)a.req_slot[r] * a.state_slot_stride + (size_t)h * a.dv * dk;
   float4 S;
   if (a.key_rows) S = make_float4(st[(size_t)c * a.dv + v], st[(size_t)(c + 1) * a.dv + v], st[(size_t)(c + 2) * a.dv + v], st[(size_t)(c + 3) * a.dv + v]);
   else S = make_float4(st[(size_t)v * dk + c], st[(size_t)v * dk + c + 1], st[(size_t)v * dk + c + 2], st[(size_t)v * dk + c + 3]);
-  const size_t base = (size_t)chunks_before(a.cu_seqlens, r) * a.heads + h;
+  const size_t base = (size_t)chunks_before(a.cu_seqlens, a.min_span, r) * a.heads + h;
   constexpr int U = 8;
   for (int c0 = 0; c0 < chunks; c0 += U) {
     float4 add[U], w[U];
@@ -488,7 +489,7 @@ __global__ void __launch_bounds__(256) chunk_reach_kernel(const ChunkArgs a) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int h = blockIdx.y, z = blockIdx.z, g = h / (a.heads / a.groups), dv = a.dv;
   int first, n;
-  if (!chunk_of(a.cu_seqlens, a.requests, blockIdx.x, first, n)) return;
+  if (!chunk_of(a.cu_seqlens, a.requests, a.min_span, blockIdx.x, first, n)) return;
   const float* state = a.local + (((size_t)blockIdx.x * a.heads + h) * dv + z * 64) * DK;
   bool bad = false;
   for (int e = tid; e < kChunk * DK / 4; e += 256) {
@@ -586,14 +587,15 @@ static int run_chunks(const ChunkArgs& a, int dk, int mode, int chunks, cudaStre
 }
 
 // The last of the three alone, for delta_chunks.cu: heads of 64 x 64, `reach` [T, heads 64] and the states as chunk_carry leaves them.
-int launch_chunk_reach_64(const float* reach, const float* local, float* out, const int* cu_seqlens, int requests, int heads, int chunks,
-                          cudaStream_t stream) {
+int launch_chunk_reach_64(const float* reach, const float* local, float* out, const int* cu_seqlens, int requests, int min_span, int heads,
+                          int chunks, cudaStream_t stream) {
   ChunkArgs a = {};
   a.reach = const_cast<float*>(reach);
   a.local = const_cast<float*>(local);
   a.out = out;
   a.cu_seqlens = cu_seqlens;
   a.requests = requests;
+  a.min_span = min_span;
   a.heads = a.groups = heads;
   a.dv = 64;
   chunk_reach_kernel<64, true><<<dim3(chunks, heads, 1), 256, 2 * kChunk * (64 + 8) * sizeof(float), stream>>>(a);
@@ -614,9 +616,10 @@ int ifx_chunk_scan_supports(int requests, int heads, int dk, int dv) {
   return requests > 0 && requests <= 64 && heads > 0 && heads <= 65535 && (dk == 64 || dk == 128) && dv > 0 && dv % 64 == 0 && dv / 64 <= 65535;
 }
 
-// Floats of scratch.  per_channel: a decay per key channel (mode 0 and wkv).
-long long ifx_chunk_scan_scratch_floats(int num_tokens, int requests, int heads, int dk, int dv, int per_channel) {
-  const long long chunks = chunks_at_most(num_tokens, requests);
+// Floats of scratch.  per_channel: a decay per key channel (mode 0 and wkv).  min_span here and below: spans with fewer tokens are
+// not touched (1: none are left out).
+long long ifx_chunk_scan_scratch_floats(int num_tokens, int requests, int min_span, int heads, int dk, int dv, int per_channel) {
+  const long long chunks = chunks_at_most(num_tokens, requests, min_span);
   const long long total = ((per_channel ? chunks * heads * dk : 2 * chunks * heads) + 3) / 4 * 4;
   return chunks * heads * dv * dk + total + (per_channel ? (long long)num_tokens * heads * dk : (long long)num_tokens * heads);
 }
@@ -625,9 +628,9 @@ long long ifx_chunk_scan_scratch_floats(int num_tokens, int requests, int heads,
 int ifx_chunk_decay_scan(const float* q, long long q_stride, const float* k, long long k_stride, const float* v, long long v_stride,
                          const float* raw, long long raw_stride, float* state, long long state_slot_stride, const int* req_slot,
                          const int* cu_seqlens, float* out, const float* step_bias, const float* log_rate, const float* skip,
-                         int num_requests, int num_tokens, int heads, int groups, int dk, int dv, int mode, float tau,
+                         int num_requests, int num_tokens, int min_span, int heads, int groups, int dk, int dv, int mode, float tau,
                          float q_scale, float* scratch, const float* rate, cudaStream_t stream) {
-  if (num_requests <= 0 || num_tokens <= 0) return 0;
+  if (num_requests <= 0 || num_tokens <= 0 || num_tokens < min_span) return 0;
   if (!ifx_chunk_scan_supports(num_requests, heads, dk, dv) || groups <= 0 || heads % groups || mode < 0 || mode > 2 || scratch == nullptr)
     return IFX_E_BADARG;
   if ((mode == 0 && !(tau > 0.0f)) || (mode == 1 && (step_bias == nullptr || log_rate == nullptr)) || (mode == 2 && rate == nullptr))
@@ -635,12 +638,12 @@ int ifx_chunk_decay_scan(const float* q, long long q_stride, const float* k, lon
   if (!rows_fit(q, q_stride) || !rows_fit(k, k_stride) || !rows_fit(v, v_stride) || (mode == 0 && !rows_fit(raw, raw_stride)) ||
       !rows_fit(scratch, 0) || !rows_fit(out, 0))
     return IFX_E_ALIGN;
-  const int chunks = chunks_at_most(num_tokens, num_requests);
+  const int chunks = chunks_at_most(num_tokens, num_requests, min_span);
   ChunkArgs a = {};
   a.q = q; a.q_stride = q_stride; a.k = k; a.k_stride = k_stride; a.v = v; a.v_stride = v_stride; a.raw = raw; a.raw_stride = raw_stride;
   a.state = state; a.state_slot_stride = state_slot_stride; a.req_slot = req_slot; a.cu_seqlens = cu_seqlens; a.out = out;
   a.step_bias = step_bias; a.log_rate = log_rate; a.skip = skip; a.rate = rate;
-  a.requests = num_requests; a.heads = heads; a.groups = groups; a.dv = dv;
+  a.requests = num_requests; a.min_span = min_span; a.heads = heads; a.groups = groups; a.dv = dv;
   a.inv_tau = mode == 0 ? 1.0f / tau : 0.0f;
   a.q_scale = q_scale;
   a.local = scratch;
@@ -652,19 +655,19 @@ int ifx_chunk_decay_scan(const float* q, long long q_stride, const float* k, lon
 // As the recurrence of ifx_wkv_scan (wkv.cu) without the norm and gate behind it: out [T, heads dim] float32.
 int ifx_chunk_wkv_scan(const float* r, const float* k, const float* v, const float* w_raw, const float* w0, const float* u,
                        float* s_state, float* prev_state, long long slot_stride, const float* x, int C, const int* cu_seqlens,
-                       const int* req_slot, float* out, int num_requests, int num_tokens, int heads, int dim, int ld, int ld_w,
-                       float* scratch, cudaStream_t stream) {
-  if (num_requests <= 0 || num_tokens <= 0) return 0;
+                       const int* req_slot, float* out, int num_requests, int num_tokens, int min_span, int heads, int dim, int ld,
+                       int ld_w, float* scratch, cudaStream_t stream) {
+  if (num_requests <= 0 || num_tokens <= 0 || num_tokens < min_span) return 0;
   if (!ifx_chunk_scan_supports(num_requests, heads, dim, dim) || scratch == nullptr) return IFX_E_BADARG;
   if (!rows_fit(r, ld) || !rows_fit(k, ld) || !rows_fit(v, ld) || !rows_fit(w_raw, ld_w) || !rows_fit(w0, 0) || !rows_fit(u, 0) ||
       !rows_fit(scratch, 0) || !rows_fit(out, 0))
     return IFX_E_ALIGN;
-  const int chunks = chunks_at_most(num_tokens, num_requests);
+  const int chunks = chunks_at_most(num_tokens, num_requests, min_span);
   ChunkArgs a = {};
   a.q = r; a.q_stride = ld; a.k = k; a.k_stride = ld; a.v = v; a.v_stride = ld; a.raw = w_raw; a.raw_stride = ld_w;
   a.state = s_state; a.state_slot_stride = slot_stride; a.req_slot = req_slot; a.cu_seqlens = cu_seqlens; a.out = out;
   a.w0 = w0; a.u = u; a.x = x; a.prev_state = prev_state; a.C = C;
-  a.requests = num_requests; a.heads = heads; a.groups = heads; a.dv = dim;
+  a.requests = num_requests; a.min_span = min_span; a.heads = heads; a.groups = heads; a.dv = dim;
   a.q_scale = 1.0f;
   a.key_rows = 1;
   a.local = scratch;

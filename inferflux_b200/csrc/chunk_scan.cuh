@@ -111,11 +111,13 @@ __device__ __forceinline__ void load_b_columns(FragB& f, const float* p, int pit
   f.v[1].set(at[4 * pitch], at[12 * pitch]);
 }
 
-// Stretch `index` of the step: its request, first flat token and tokens.  Stretches of a request lie side by side.
-__device__ __forceinline__ bool chunk_of(const int* __restrict__ cu_seqlens, int requests, int index, int& first, int& n) {
+// Stretch `index` of the step's spans of min_span tokens and more: its request, first flat token and tokens.  Stretches of a
+// request lie side by side.
+__device__ __forceinline__ int chunks_of(int span, int min_span) { return span < min_span ? 0 : (span + kChunk - 1) / kChunk; }
+__device__ __forceinline__ bool chunk_of(const int* __restrict__ cu_seqlens, int requests, int min_span, int index, int& first, int& n) {
   int before = 0;
   for (int r = 0; r < requests; ++r) {
-    const int lo = cu_seqlens[r], span = cu_seqlens[r + 1] - lo, chunks = (span + kChunk - 1) / kChunk;
+    const int lo = cu_seqlens[r], span = cu_seqlens[r + 1] - lo, chunks = chunks_of(span, min_span);
     if (index < before + chunks) {
       first = lo + (index - before) * kChunk;
       n = min(kChunk, span - (index - before) * kChunk);
@@ -125,12 +127,15 @@ __device__ __forceinline__ bool chunk_of(const int* __restrict__ cu_seqlens, int
   }
   return false;
 }
-__device__ __forceinline__ int chunks_before(const int* __restrict__ cu_seqlens, int request) {
+__device__ __forceinline__ int chunks_before(const int* __restrict__ cu_seqlens, int min_span, int request) {
   int before = 0;
-  for (int r = 0; r < request; ++r) before += (cu_seqlens[r + 1] - cu_seqlens[r] + kChunk - 1) / kChunk;
+  for (int r = 0; r < request; ++r) before += chunks_of(cu_seqlens[r + 1] - cu_seqlens[r], min_span);
   return before;
 }
 // The most stretches that num_tokens of num_requests can make.
-inline int chunks_at_most(int num_tokens, int num_requests) { return num_tokens / kChunk + num_requests; }
+inline int chunks_at_most(int num_tokens, int num_requests, int min_span) {
+  const int spans = num_tokens / (min_span > 1 ? min_span : 1);
+  return num_tokens / kChunk + (spans < num_requests ? spans : num_requests);
+}
 
 }  // namespace ifx

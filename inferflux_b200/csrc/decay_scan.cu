@@ -22,7 +22,7 @@
 // worked on (the exponentials are taken there, once per token and channel).  Every sum's order depends on (dk, R, KS)
 // only, never on how the tokens were cut into steps or which other requests are in the batch.
 // Long spans of a bfloat16 run go to chunk_scan.cu instead (CHUNK_SCAN_MIN_SPAN in ops.py); this is the scan of a float32 run, of
-// decoded tokens and of short spans.
+// decoded tokens and of short spans.  With `part` spans of more than `max_span` tokens are in the step and are not touched.
 #include "common.cuh"
 
 namespace ifx {
@@ -46,6 +46,7 @@ struct DecayScanArgs {
   // front, its step sizes behind), made by decay_prepare_kernel for steps with long spans
   int ready;
   int vec;                                     // rows, strides and sizes allow copies of four floats at a time
+  int part, max_span;                          // part: longer spans than max_span are left to chunk_scan.cu
 };
 
 __device__ __forceinline__ float log_sigmoid(float x) { return fminf(x, 0.0f) - log1pf(expf(-fabsf(x))); }
@@ -69,7 +70,9 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // four floats of padding behind every 32 keep the KS lanes of a column on banks of their own.
 __device__ __forceinline__ int padded(int c) { return c + ((c >> 5) << 2); }
 
-template <int R, int MODE>
+// PART: spans of more than max_span tokens are left to chunk_scan.cu.  Compiled apart, since with that test the scan of long spans is
+// slower (a decay per key channel, 2,048 tokens of 12 heads: 491 -> 504 us).
+template <int R, int MODE, bool PART>
 __global__ void __launch_bounds__(256) decay_scan_kernel(const DecayScanArgs a) {
   extern __shared__ __align__(16) float smem[];
   static_assert(R % 4 == 0, "a lane reads its key channels four at a time");
@@ -87,6 +90,7 @@ __global__ void __launch_bounds__(256) decay_scan_kernel(const DecayScanArgs a) 
   const int dk = a.dk, dv = a.dv;
   const int g = h / (a.heads / a.groups);
   const int first = a.cu_seqlens[r], n = a.cu_seqlens[r + 1] - first;
+  if (PART && n > a.max_span) return;
   float* st = a.state + (long long)a.req_slot[r] * a.state_slot_stride + ((size_t)h * dv + (live ? j : 0)) * dk;
   const int c0 = s * R;                                      // this lane's first key channel
 
@@ -259,16 +263,21 @@ __global__ void decay_prepare_kernel(const float* __restrict__ raw, long long ra
 
 template <int MODE>
 static int launch_decay_scan(const DecayScanArgs& a, int R, dim3 grid, int threads, size_t smem, cudaStream_t stream) {
-#define IFX_SCAN(RR)                                                                                          \
+#define IFX_SCAN(RR, PART)                                                                                    \
   do {                                                                                                        \
-    auto kern = decay_scan_kernel<RR, MODE>;                                                                  \
+    auto kern = decay_scan_kernel<RR, MODE, PART>;                                                            \
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
     kern<<<grid, threads, smem, stream>>>(a);                                                                 \
   } while (0)
+  if (a.part) {                                              // beside chunk_scan.cu: 64 or 128 key channels
+    if (R != 8) return IFX_E_BADARG;
+    IFX_SCAN(8, true);
+    return 0;
+  }
   switch (R) {
-    case 4: IFX_SCAN(4); break;
-    case 8: IFX_SCAN(8); break;
-    case 16: IFX_SCAN(16); break;
+    case 4: IFX_SCAN(4, false); break;
+    case 8: IFX_SCAN(8, false); break;
+    case 16: IFX_SCAN(16, false); break;
     default: return IFX_E_BADARG;
   }
 #undef IFX_SCAN
@@ -309,7 +318,7 @@ int ifx_decay_scan_split(int dk, int* R_out, int* KS_out) {
 int ifx_decay_scan_rate(const float* q, long long q_stride, const float* k, long long k_stride, const float* v, long long v_stride,
                    const float* raw, long long raw_stride, float* state, long long state_slot_stride, const int* req_slot,
                    const int* cu_seqlens, float* out, const float* step_bias, const float* log_rate, const float* skip,
-                   int num_requests, int num_tokens, int max_span, int heads, int groups, int dk, int dv, int mode, float tau,
+                   int num_requests, int num_tokens, int max_span, int part, int heads, int groups, int dk, int dv, int mode, float tau,
                    float q_scale, int blocks_wanted, float* scratch, const float* rate, cudaStream_t stream) {
   if (num_requests <= 0) return 0;
   if (heads <= 0 || groups <= 0 || heads % groups || dk <= 0 || dv <= 0 || mode < 0 || mode > 2 || max_span <= 0)
@@ -360,6 +369,8 @@ int ifx_decay_scan_rate(const float* q, long long q_stride, const float* k, long
   a.inv_tau = mode == 0 ? 1.0f / tau : 0.0f;
   a.q_scale = q_scale;
   a.ready = ready ? 1 : 0;
+  a.part = part;
+  a.max_span = max_span;
   auto by16 = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
   a.vec = (dk % 4 == 0 && q_stride % 4 == 0 && k_stride % 4 == 0 && (mode != 0 || raw_stride % 4 == 0) && by16(q) && by16(k) &&
            (mode != 0 || by16(raw))) ? 1 : 0;
@@ -379,7 +390,7 @@ int ifx_decay_scan(const float* q, long long q_stride, const float* k, long long
                    float q_scale, int blocks_wanted, float* scratch, cudaStream_t stream) {
   if (mode != 0 && mode != 1) return IFX_E_BADARG;
   return ifx_decay_scan_rate(q, q_stride, k, k_stride, v, v_stride, raw, raw_stride, state, state_slot_stride, req_slot, cu_seqlens,
-                             out, step_bias, log_rate, skip, num_requests, num_tokens, max_span, heads, groups, dk, dv, mode, tau,
+                             out, step_bias, log_rate, skip, num_requests, num_tokens, max_span, 0, heads, groups, dk, dv, mode, tau,
                              q_scale, blocks_wanted, scratch, nullptr, stream);
 }
 

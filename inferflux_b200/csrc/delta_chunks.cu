@@ -42,7 +42,7 @@ struct DeltaChunkArgs {
   const float* w_raw; const float* w0; const float* a_bias;
   float* state; long long state_slot_stride; const int* req_slot; const int* cu_seqlens;
   float* out;                                               // [T, heads 64]
-  int requests, heads;
+  int requests, min_span, heads;                            // shorter spans are left to delta_scan
   float *local, *trans, *reach;                             // [stretches, heads, v, k], [stretches, heads, k, k], [T, heads 64]
 };
 
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_local_kernel(const DeltaC
         *a_s = smem + L::A, *mid = smem + L::MID, *end = smem + L::END;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y, HD = a.heads * kDcD;
   int first, n;
-  if (!chunk_of(a.cu_seqlens, a.requests, blockIdx.x, first, n)) return;
+  if (!chunk_of(a.cu_seqlens, a.requests, a.min_span, blockIdx.x, first, n)) return;
   const size_t item = (size_t)blockIdx.x * a.heads + h;
 
   // ---------------------------------------------------------- rows: queries, keys, values, how much is erased, unit keys, decays
@@ -344,9 +344,9 @@ __global__ void __launch_bounds__(kCarryThreads) delta_carry_kernel(const DeltaC
   float* s_s = l_s + 2 * kCarryState;                      // [16][72]: the state, a value channel a row
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int r = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * 16;
-  const int span = a.cu_seqlens[r + 1] - a.cu_seqlens[r], chunks = (span + kChunk - 1) / kChunk;
+  const int chunks = chunks_of(a.cu_seqlens[r + 1] - a.cu_seqlens[r], a.min_span);
   if (chunks == 0) return;
-  const size_t base = (size_t)chunks_before(a.cu_seqlens, r) * a.heads + h;
+  const size_t base = (size_t)chunks_before(a.cu_seqlens, a.min_span, r) * a.heads + h;
   float* st = a.state + (long long)a.req_slot[r] * a.state_slot_stride + (size_t)h * kDcD * kDcD;      // [k, v]
   bool bad = false;                                        // numbers of the state, the matrix that are not finite: split products would lose them
   for (int e = tid; e < 16 * kDcD; e += kCarryThreads) {
@@ -406,8 +406,11 @@ __global__ void __launch_bounds__(kCarryThreads) delta_carry_kernel(const DeltaC
   for (int e = tid; e < 16 * kDcD; e += kCarryThreads) st[(e >> 4) * kDcD + v0 + (e & 15)] = s_s[(e & 15) * kDcP + (e >> 4)];
 }
 
-int launch_chunk_reach_64(const float* reach, const float* local, float* out, const int* cu_seqlens, int requests, int heads, int chunks,
-                          cudaStream_t stream);                                             // chunk_scan.cu
+int launch_chunk_reach_64(const float* reach, const float* local, float* out, const int* cu_seqlens, int requests, int min_span, int heads,
+                          int chunks, cudaStream_t stream);                                 // chunk_scan.cu
+int launch_delta_scan(const float* proj, int ld, const float* w_raw, const float* w0, const float* a_bias, float* state,
+                      long long slot_stride, const int* cu_seqlens, const int* req_slot, float* scratch, float* o, int num_requests, int T,
+                      int heads, int dim, int max_span, cudaStream_t stream);               // delta_rule.cu
 int launch_delta_finish(const float* o, const float* proj, int ld, const float* norm_w, float eps, void* y, int num_tokens, int heads,
                         int dim, int out_dtype, cudaStream_t stream);                       // delta_rule.cu
 
@@ -420,24 +423,26 @@ extern "C" {
 int ifx_delta_chunks_supports(int requests, int heads, int dim) {
   return requests > 0 && requests <= 64 && heads > 0 && heads <= 65535 && dim == kDcD;
 }
-long long ifx_delta_chunks_scratch_floats(int num_tokens, int requests, int heads) {
-  return 2LL * chunks_at_most(num_tokens, requests) * heads * kDcD * kDcD + 2LL * num_tokens * heads * kDcD;
+long long ifx_delta_chunks_scratch_floats(int num_tokens, int requests, int min_span, int heads) {
+  return 2LL * chunks_at_most(num_tokens, requests, min_span) * heads * kDcD * kDcD + 2LL * num_tokens * heads * kDcD;
 }
 
-// As ifx_delta_rule_scan (delta_rule.cu) for heads of 64 channels, with scratch as above; rows on 16-byte boundaries.
+// As ifx_delta_rule_scan (delta_rule.cu) for heads of 64 channels, with scratch as above; rows on 16-byte boundaries.  Spans of
+// fewer than min_span tokens go through delta_scan, with scan_scratch as ifx_delta_rule_scratch_floats says (null: there are none).
 int ifx_delta_chunks_scan(const float* proj, int ld, const float* w_raw, const float* w0, const float* a_bias, const float* norm_w,
                           float eps, float* state, long long slot_stride, const int* cu_seqlens, const int* req_slot, float* scratch,
-                          void* y, int num_requests, int num_tokens, int heads, int dim, int out_dtype, cudaStream_t stream) {
+                          void* y, int num_requests, int num_tokens, int min_span, int heads, int dim, int out_dtype, float* scan_scratch,
+                          cudaStream_t stream) {
   if (num_tokens <= 0 || num_requests <= 0) return 0;
   if (!ifx_delta_chunks_supports(num_requests, heads, dim) || ld < 5 * heads * dim || slot_stride < (long long)heads * dim * dim ||
-      scratch == nullptr)
+      scratch == nullptr || min_span < 1 || min_span > num_tokens)
     return IFX_E_BADARG;
   if (ld % 4 || ((uintptr_t)proj | (uintptr_t)w_raw | (uintptr_t)w0 | (uintptr_t)a_bias | (uintptr_t)scratch) % 16) return IFX_E_ALIGN;
-  const int chunks = chunks_at_most(num_tokens, num_requests);
+  const int chunks = chunks_at_most(num_tokens, num_requests, min_span);
   DeltaChunkArgs a;
   a.proj = proj; a.ld = ld; a.w_raw = w_raw; a.w0 = w0; a.a_bias = a_bias;
   a.state = state; a.state_slot_stride = slot_stride; a.req_slot = req_slot; a.cu_seqlens = cu_seqlens;
-  a.requests = num_requests; a.heads = heads;
+  a.requests = num_requests; a.min_span = min_span; a.heads = heads;
   const size_t states = (size_t)chunks * heads * kDcD * kDcD, rows = (size_t)num_tokens * heads * kDcD;
   a.local = scratch;
   a.trans = a.local + states;
@@ -447,11 +452,16 @@ int ifx_delta_chunks_scan(const float* proj, int ld, const float* w_raw, const f
   cudaError_t e = cudaFuncSetAttribute(delta_local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DeltaChunkLayout::BYTES);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_carry_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)carry_bytes);
   if (e != cudaSuccess) return (int)e;
+  if (scan_scratch != nullptr) {
+    const int rc = launch_delta_scan(proj, ld, w_raw, w0, a_bias, state, slot_stride, cu_seqlens, req_slot, scan_scratch, a.out, num_requests,
+                                     num_tokens, heads, dim, min_span - 1, stream);
+    if (rc) return rc;
+  }
   delta_local_kernel<<<dim3(chunks, heads), kDcThreads, DeltaChunkLayout::BYTES, stream>>>(a);
   IFX_CHECK_LAUNCH();
   delta_carry_kernel<<<dim3(num_requests, heads, 4), kCarryThreads, carry_bytes, stream>>>(a);
   IFX_CHECK_LAUNCH();
-  const int rc = launch_chunk_reach_64(a.reach, a.local, a.out, cu_seqlens, num_requests, heads, chunks, stream);
+  const int rc = launch_chunk_reach_64(a.reach, a.local, a.out, cu_seqlens, num_requests, min_span, heads, chunks, stream);
   if (rc) return rc;
   return launch_delta_finish(a.out, proj, ld, norm_w, eps, y, num_tokens, heads, dim, out_dtype, stream);
 }

@@ -32,11 +32,20 @@ __device__ __forceinline__ float sigmoid_f(float z) { return 1.0f / (1.0f + expf
 __global__ void delta_prepare_kernel(const float* __restrict__ proj, int ld, const float* __restrict__ w_raw,
                                      const float* __restrict__ w0, const float* __restrict__ a_bias,
                                      float* __restrict__ decay, float* __restrict__ au, float* __restrict__ unit,
-                                     float* __restrict__ rw, float2* __restrict__ c, int num_tokens, int heads, int dim) {
+                                     float* __restrict__ rw, float2* __restrict__ c, int num_tokens, int heads, int dim,
+                                     const int* __restrict__ cu_seqlens, int requests, int max_span) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + warp;
   if (item >= (long long)num_tokens * heads) return;
   const int t = (int)(item / heads), h = (int)(item % heads);
+  if (max_span < num_tokens) {                             // tokens of longer spans are left out
+    int r = 0, end = requests;
+    while (end - r > 1) {
+      const int m = (r + end) >> 1;
+      if (cu_seqlens[m] <= t) r = m; else end = m;
+    }
+    if (cu_seqlens[r + 1] - cu_seqlens[r] > max_span) return;
+  }
   const int HD = heads * dim;
   const float* r = proj + (size_t)t * ld + h * dim;
   const float* k = proj + (size_t)t * ld + HD + h * dim;
@@ -82,12 +91,14 @@ constexpr int kDeltaNC = 2;           // columns a thread keeps: one's shuffles 
 // an order that the head size alone decides.  Both sums of a token, u^T S and (r * decay)^T S, are taken of the state
 // before the token, so they run side by side and their shuffles overlap.  Block: 128 threads, of which the first cols * KS (whole warps) compute;
 // all of them bring the vectors of the next `stage` tokens into the other buffer by cp.async while these are worked on.
-template <int KS>
+// PART: spans of more than max_span tokens are left to delta_chunks.cu.  Compiled apart, since with that test the scan of long spans is a
+// tenth slower (2,048 tokens of 24 heads 658 -> 733 us).
+template <int KS, bool PART>
 __global__ void __launch_bounds__(kDeltaThreads) delta_scan_kernel(
     const float* __restrict__ proj, int ld, const float* __restrict__ decay, const float* __restrict__ au,
     const float* __restrict__ unit, const float* __restrict__ rw, const float2* __restrict__ c12,
     float* __restrict__ state, long long slot_stride, const int* __restrict__ cu_seqlens,
-    const int* __restrict__ req_slot, float* __restrict__ o, int heads, int dim, int cols, int stage, int vec) {
+    const int* __restrict__ req_slot, float* __restrict__ o, int heads, int dim, int cols, int stage, int vec, int max_span) {
   constexpr int R = kDeltaR;
   constexpr int DP = KS * (R + kDeltaPad);               // a staged row: slice s at s * (R + pad), zeros beyond dim
   extern __shared__ __align__(16) float smem[];          // 2 x ([stage][5][DP]: r * decay, k, decay, au, u ; [stage][cols]: v ; [stage][2])
@@ -102,6 +113,7 @@ __global__ void __launch_bounds__(kDeltaThreads) delta_scan_kernel(
   for (int cc = 0; cc < NC; ++cc) live[cc] = c * NC + cc < cols && j + cc < dim;
   const int HD = heads * dim;
   const int lo = cu_seqlens[req], hi = cu_seqlens[req + 1];
+  if (PART && hi - lo > max_span) return;
   float* S_mem = state + (long long)req_slot[req] * slot_stride + (size_t)h * dim * dim;
   float S[NC][R];
 #pragma unroll
@@ -262,31 +274,17 @@ int launch_delta_finish(const float* o, const float* proj, int ld, const float* 
   return 0;
 }
 
-}  // namespace ifx
-
-using namespace ifx;
-
-extern "C" {
-
-// Floats of scratch the scan needs for T tokens: decay, a * u, u, o and r * decay, [T, heads * dim] each, and two numbers per
-// token and head.
-long long ifx_delta_rule_scratch_floats(int T, int heads, int dim) { return 5LL * T * heads * dim + 2LL * T * heads + 4; }
-
-// proj: float32 [T, ld], the projections r, k, v, g, a in column blocks of heads * dim; w_raw: float32 [T, heads * dim];
-// state: float32, slot s at state + s * slot_stride holds [heads, dim, dim]; y: [T, heads * dim] in out_dtype.
-int ifx_delta_rule_scan(const float* proj, int ld, const float* w_raw, const float* w0, const float* a_bias,
-                        const float* norm_w, float eps, float* state, long long slot_stride, const int* cu_seqlens,
-                        const int* req_slot, float* scratch, void* y, int num_requests, int T, int heads, int dim,
-                        int out_dtype, cudaStream_t stream) {
-  if (T <= 0 || num_requests <= 0) return 0;
-  if (heads <= 0 || dim <= 0 || ld < 5 * heads * dim || slot_stride < (long long)heads * dim * dim) return IFX_E_BADARG;
-  if (dim > 256) return IFX_E_TOOBIG;
+// Preparation and scan of the spans of up to max_span tokens: their rows of o and their states.  scratch: as
+// ifx_delta_rule_scratch_floats says (o may be its fourth block).
+int launch_delta_scan(const float* proj, int ld, const float* w_raw, const float* w0, const float* a_bias, float* state,
+                      long long slot_stride, const int* cu_seqlens, const int* req_slot, float* scratch, float* o, int num_requests, int T,
+                      int heads, int dim, int max_span, cudaStream_t stream) {
   const size_t n = (size_t)T * heads * dim;
-  float *decay = scratch, *au = scratch + n, *unit = scratch + 2 * n, *o = scratch + 3 * n, *rw = scratch + 4 * n;
+  float *decay = scratch, *au = scratch + n, *unit = scratch + 2 * n, *rw = scratch + 4 * n;
   float2* c12 = reinterpret_cast<float2*>(scratch + ((5 * n + 1) & ~(size_t)1));
   const long long items = (long long)T * heads;
   delta_prepare_kernel<<<(unsigned)((items + 3) / 4), 128, 0, stream>>>(proj, ld, w_raw, w0, a_bias, decay, au, unit, rw, c12, T, heads,
-                                                                        dim);
+                                                                        dim, cu_seqlens, num_requests, max_span);
   IFX_CHECK_LAUNCH();
   // slices of 8 key channels: a function of the head size alone, so that no sum's order depends on anything else
   const int KS = dim <= 8 ? 1 : dim <= 16 ? 2 : dim <= 32 ? 4 : dim <= 64 ? 8 : dim <= 128 ? 16 : 32;
@@ -312,10 +310,10 @@ int ifx_delta_rule_scan(const float* proj, int ld, const float* w_raw, const flo
   const size_t smem = bytes_for(cols);
 #define IFX_SCAN(KK)                                                                                              \
   do {                                                                                                            \
-    auto kern = delta_scan_kernel<KK>;                                                                            \
+    auto kern = max_span < T ? delta_scan_kernel<KK, true> : delta_scan_kernel<KK, false>;                        \
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);     \
     kern<<<grid, kDeltaThreads, smem, stream>>>(proj, ld, decay, au, unit, rw, c12, state, slot_stride, cu_seqlens,  \
-                                                req_slot, o, heads, dim, cols, stage, vec);                       \
+                                                req_slot, o, heads, dim, cols, stage, vec, max_span);             \
   } while (0)
   if (KS == 1) IFX_SCAN(1);
   else if (KS == 2) IFX_SCAN(2);
@@ -325,6 +323,32 @@ int ifx_delta_rule_scan(const float* proj, int ld, const float* w_raw, const flo
   else IFX_SCAN(32);
 #undef IFX_SCAN
   IFX_CHECK_LAUNCH();
+  return 0;
+}
+
+}  // namespace ifx
+
+using namespace ifx;
+
+extern "C" {
+
+// Floats of scratch the scan needs for T tokens: decay, a * u, u, o and r * decay, [T, heads * dim] each, and two numbers per
+// token and head.
+long long ifx_delta_rule_scratch_floats(int T, int heads, int dim) { return 5LL * T * heads * dim + 2LL * T * heads + 4; }
+
+// proj: float32 [T, ld], the projections r, k, v, g, a in column blocks of heads * dim; w_raw: float32 [T, heads * dim];
+// state: float32, slot s at state + s * slot_stride holds [heads, dim, dim]; y: [T, heads * dim] in out_dtype.
+int ifx_delta_rule_scan(const float* proj, int ld, const float* w_raw, const float* w0, const float* a_bias,
+                        const float* norm_w, float eps, float* state, long long slot_stride, const int* cu_seqlens,
+                        const int* req_slot, float* scratch, void* y, int num_requests, int T, int heads, int dim,
+                        int out_dtype, cudaStream_t stream) {
+  if (T <= 0 || num_requests <= 0) return 0;
+  if (heads <= 0 || dim <= 0 || ld < 5 * heads * dim || slot_stride < (long long)heads * dim * dim) return IFX_E_BADARG;
+  if (dim > 256) return IFX_E_TOOBIG;
+  float* o = scratch + 3 * (size_t)T * heads * dim;
+  const int rc = launch_delta_scan(proj, ld, w_raw, w0, a_bias, state, slot_stride, cu_seqlens, req_slot, scratch, o, num_requests, T, heads,
+                                   dim, T, stream);
+  if (rc) return rc;
   return launch_delta_finish(o, proj, ld, norm_w, eps, y, T, heads, dim, out_dtype, stream);
 }
 

@@ -1429,20 +1429,46 @@ class CudaKernels:
         self.launches += 1
         return out
 
-    # From spans of this many tokens on, a bfloat16 run takes its recurrences by stretches of 64 tokens (csrc/chunk_scan.cu).
+    # Spans of this many tokens and more can go by stretches of 64 tokens in a bfloat16 run (csrc/chunk_scan.cu, delta_chunks.cu).  The
+    # other spans of the same step then go through the scans token by token, in launches of their own: a stretch costs the same
+    # with one token as with 64.
     CHUNK_SCAN_MIN_SPAN = 128
-    # The delta rule's stretches (csrc/delta_chunks.cu) do several times a token's work of the scan; what they gain is that tokens of
-    # one span run side by side.  us, scan and stretches, 24 heads of 64: one span of 2,048 tokens 660 / 241, 300: 101 / 46, 128:
-    # 48 / 41, 96: 38 / 41; four of 500 256 / 219; sixteen of 128 197 / 227 (56 heads: 427 / 492).
-    DELTA_CHUNKS_MIN_SPAN = 128
-    DELTA_CHUNKS_MAX_SPANS = 8
 
-    def _scans_by_chunks(self, dtype, ctx, heads, dk, dv, *rows):
-        """Whether a recurrence goes by stretches of tokens: long spans, sizes the kernels are made for, rows on 16-byte
-        boundaries, and a bfloat16 run (the order of the sums then depends on how a span was cut into steps)."""
-        return (self.chunk_scans and dtype is torch.bfloat16 and ctx.max_span >= self.CHUNK_SCAN_MIN_SPAN
-                and self.lib.ifx_chunk_scan_supports(ctx.num_requests, int(heads), int(dk), int(dv))
-                and all(t.data_ptr() % 16 == 0 and (t.dim() < 2 or t.stride(0) % 4 == 0) for t in rows))
+    def _long_spans(self, ctx):
+        """(longest, tokens, number) of a step's spans of fewer than CHUNK_SCAN_MIN_SPAN tokens and the stretches of the others, found
+        once a step; None for a context without a host list of spans, whose spans all go the same way."""
+        got = getattr(ctx, "long_spans", None)
+        if got is None and getattr(ctx, "spans", None):
+            short = [n for _s, n in ctx.spans if n < self.CHUNK_SCAN_MIN_SPAN]
+            got = ctx.long_spans = (max(short, default=0), sum(short), len(short),
+                                    sum(-(-n // 64) for _s, n in ctx.spans if n >= self.CHUNK_SCAN_MIN_SPAN))
+        return got
+
+    def _scans_by_chunks(self, dtype, ctx, heads, dk, dv, *rows, constant=False):
+        """Whether a recurrence's long spans go by stretches of tokens: where that pays, with sizes the kernels are made for, rows
+        on 16-byte boundaries, and in a bfloat16 run (the order of the sums then depends on how a span was cut into steps)."""
+        if not (self.chunk_scans and dtype is torch.bfloat16 and ctx.max_span >= self.CHUNK_SCAN_MIN_SPAN):
+            return False
+        spans = self._long_spans(ctx)
+        return bool((spans is None or self.stretches_pay(ctx.max_span, spans[0], spans[3], constant and dk == 64))
+                    and self.lib.ifx_chunk_scan_supports(ctx.num_requests, int(heads), int(dk), int(dv))
+                    and all(t.data_ptr() % 16 == 0 and (t.dim() < 2 or t.stride(0) % 4 == 0) for t in rows))
+
+    @staticmethod
+    def stretches_pay(longest, short, stretches, cheap):
+        """For a step whose longest span has `longest` tokens, the longest of fewer than CHUNK_SCAN_MIN_SPAN `short` (0: none).  What is
+        gained is the time between the two; a launch for the short spans costs a few us beside them.  us, the scan alone and this
+        (12 heads of 128 x 128 with a constant decay; wkv, 24 heads of 64): 128 tokens 41 / 32; 40 / 29; 128 and 31 of one
+        75 / 66; 96 / 63; 512 and 31 of one 237 / 78; 260 / 75; 128 and 20 47 / 44; 44 / 41; 192 and 60 68 / 56; 62 / 52; 228 and 100
+        80 / 81; 73 / 74; 512, 100, 80 and 29 of one 229 / 123; 268 / 127; sixteen of 128 213 / 151; 184 / 148; at 56 heads 128 and 63 of
+        one 192 / 198; 242 / 174.  `cheap`, a constant decay and keys of 64 numbers: its scan wins where very many stretches are
+        of short spans (28 heads, 32 of 128: 442 / 493; sixteen of 256 458 / 375)."""
+        return (short < 24 or longest >= short + 128) and not (cheap and stretches > 24 + longest // 4)
+
+    def _parting(self, ctx):
+        """(the fewest tokens of a span that goes by stretches, the most tokens of one that does not or 0)."""
+        spans = self._long_spans(ctx)
+        return (1, 0) if spans is None else (self.CHUNK_SCAN_MIN_SPAN, spans[0])
 
     def wkv_scan(self, r, k, v, w_raw, g, w0, u, norm_w, eps, heads, dim, state, prev_offset, x, ctx, out_dtype):
         """The recurrence of csrc/wkv.cu over every request's tokens.  r, k, v, w_raw, g: float32 [T, heads * dim], each
@@ -1464,12 +1490,20 @@ class CudaKernels:
         scratch = torch.empty((T, HD), dtype=torch.float32, device=r.device)
         y = torch.empty((T, HD), dtype=out_dtype, device=r.device)
         if self._scans_by_chunks(out_dtype, ctx, heads, dim, dim, r, k, v, w_raw, w0, u):
-            room = torch.empty(int(self.lib.ifx_chunk_scan_scratch_floats(T, ctx.num_requests, heads, dim, dim, 1)), dtype=torch.float32,
-                               device=r.device)
+            least, short = self._parting(ctx)
+            if short:
+                _check(self.lib.ifx_wkv_scan(
+                    _ptr(r), _ptr(k), _ptr(v), _ptr(w_raw), _ptr(g), _ptr(w0), _ptr(u), _ptr(norm_w), ctypes.c_float(eps),
+                    _ptr(state), ctypes.c_void_p(state.data_ptr() + 4 * prev_offset), ctypes.c_longlong(state.shape[1]), _ptr(x), C,
+                    _ptr(ctx.cu_seqlens), _ptr(ctx.req_slot), _ptr(scratch), _ptr(y), ctx.num_requests, T, heads, dim, ld, ld_w,
+                    _DT[out_dtype], short, _stream()), "wkv_scan (short spans)")
+                self.launches += 1
+            room = torch.empty(int(self.lib.ifx_chunk_scan_scratch_floats(T, ctx.num_requests, least, heads, dim, dim, 1)),
+                               dtype=torch.float32, device=r.device)
             _check(self.lib.ifx_chunk_wkv_scan(
                 _ptr(r), _ptr(k), _ptr(v), _ptr(w_raw), _ptr(w0), _ptr(u), _ptr(state), ctypes.c_void_p(state.data_ptr() + 4 * prev_offset),
                 ctypes.c_longlong(state.shape[1]), _ptr(x), C, _ptr(ctx.cu_seqlens), _ptr(ctx.req_slot), _ptr(scratch),
-                ctx.num_requests, T, heads, dim, ld, ld_w, _ptr(room), _stream()), "wkv_scan (stretches)")
+                ctx.num_requests, T, least, heads, dim, ld, ld_w, _ptr(room), _stream()), "wkv_scan (stretches)")
             _check(self.lib.ifx_wkv_norm(_ptr(scratch), _ptr(g), _ptr(norm_w), ctypes.c_float(eps), _ptr(y), T, heads, dim, ld,
                                          _DT[out_dtype], _stream()), "wkv_norm")
             self.launches += 4
@@ -1478,9 +1512,35 @@ class CudaKernels:
             _ptr(r), _ptr(k), _ptr(v), _ptr(w_raw), _ptr(g), _ptr(w0), _ptr(u), _ptr(norm_w), ctypes.c_float(eps),
             _ptr(state), ctypes.c_void_p(state.data_ptr() + 4 * prev_offset), ctypes.c_longlong(state.shape[1]), _ptr(x), C,
             _ptr(ctx.cu_seqlens), _ptr(ctx.req_slot), _ptr(scratch), _ptr(y), ctx.num_requests, T, heads, dim, ld, ld_w, _DT[out_dtype],
-            _stream()), "wkv_scan")
+            0, _stream()), "wkv_scan")
         self.launches += 1
         return y
+
+    def _delta_by_chunks(self, dtype, ctx, tokens, heads, dim):
+        """Whether the delta rule's long spans go by stretches."""
+        if not (self.chunk_scans and dtype is torch.bfloat16 and ctx.max_span >= self.CHUNK_SCAN_MIN_SPAN):
+            return False
+        spans = self._long_spans(ctx)
+        pays = tokens <= 8 * ctx.max_span if spans is None else self.delta_stretches_pay(heads, tokens, ctx.num_requests, ctx.max_span, *spans)
+        return bool(pays and self.lib.ifx_delta_chunks_supports(ctx.num_requests, heads, dim))
+
+    @staticmethod
+    def delta_stretches_pay(heads, tokens, requests, longest, short, short_tokens, short_requests, stretches):
+        """A stretch of the delta rule does several times a token's work of the scan; what is gained is that the tokens of one span run
+        side by side, so this compares what both ways take.  us, fitted to what follows within a tenth: the scan walks its longest
+        span at 0.3 a token and more with more columns at once; the stretches go in rounds of 148 blocks (a head's stretch each).
+        us, 24 heads of 64, the scan alone and this: 128 tokens 47 / 48; 256 87 / 53; 512 165 / 96; 2,048 659 / 304; two of 256
+        99 / 92; four of 256 128 / 139; four of 512 262 / 277; eight of 512 377 / 509; with 31 of one 128 68 / 72, 256 115 / 81, 512
+        211 / 129; with 63 of one 512 225 / 144; 256 and 100 106 / 102; 512, 100, 80 and 29 of one 222 / 176.  56 heads: 192 82 / 90;
+        256 105 / 93; 2,048 841 / 608; four of 256 267 / 320; with 31 of one 512 280 / 249."""
+        def scan(longest, tokens, requests):
+            columns = tokens * heads / longest             # heads at work at once, on average
+            return longest * max(0.3 + 0.0019 * columns, columns / 275) + 0.018 * requests * heads
+        blocks = stretches * heads
+        chunks = 37 * -(-blocks // 148) + 1.5 * (longest / 64) + 0.055 * blocks + 8
+        if short:
+            chunks += 10 + scan(short, short_tokens, short_requests)
+        return 1.1 * chunks < 6 + scan(longest, tokens, requests - 1)
 
     def delta_rule_scan(self, proj, w_raw, w0, a_bias, norm_w, eps, heads, dim, state, ctx, out_dtype):
         """The recurrence of csrc/delta_rule.cu over every request's tokens.  `proj`: float32 [T, 5 heads dim], the
@@ -1495,16 +1555,19 @@ class CudaKernels:
         _need(state is not None and state.dtype == torch.float32 and state.dim() == 2 and state.stride(1) == 1
               and state.shape[1] >= HD * dim, "delta_rule_scan: the state does not fit the sizes")
         y = torch.empty((T, HD), dtype=out_dtype, device=proj.device)
-        if (self.chunk_scans and out_dtype is torch.bfloat16 and ctx.max_span >= self.DELTA_CHUNKS_MIN_SPAN
-                and T <= self.DELTA_CHUNKS_MAX_SPANS * ctx.max_span
-                and self.lib.ifx_delta_chunks_supports(ctx.num_requests, heads, dim) and proj.shape[1] % 4 == 0
+        if (self._delta_by_chunks(out_dtype, ctx, T, heads, dim) and proj.shape[1] % 4 == 0
                 and all(t.data_ptr() % 16 == 0 for t in (proj, w_raw, w0, a_bias))):
-            room = torch.empty(int(self.lib.ifx_delta_chunks_scratch_floats(T, ctx.num_requests, heads)), dtype=torch.float32,
+            least, short = self._parting(ctx)
+            room = torch.empty(int(self.lib.ifx_delta_chunks_scratch_floats(T, ctx.num_requests, least, heads)), dtype=torch.float32,
                                device=proj.device)
+            scan_room = None
+            if short:
+                scan_room = torch.empty(int(self.lib.ifx_delta_rule_scratch_floats(T, heads, dim)), dtype=torch.float32, device=proj.device)
+                self.launches += 2
             _check(self.lib.ifx_delta_chunks_scan(
                 _ptr(proj), proj.shape[1], _ptr(w_raw), _ptr(w0), _ptr(a_bias), _ptr(norm_w), ctypes.c_float(eps), _ptr(state),
                 ctypes.c_longlong(state.stride(0)), _ptr(ctx.cu_seqlens), _ptr(ctx.req_slot), _ptr(room), _ptr(y), ctx.num_requests, T,
-                heads, dim, _DT[out_dtype], _stream()), "delta_rule_scan (stretches)")
+                least, heads, dim, _DT[out_dtype], _ptr(scan_room), _stream()), "delta_rule_scan (stretches)")
             self.launches += 4
             return y
         scratch = torch.empty(int(self.lib.ifx_delta_rule_scratch_floats(T, heads, dim)), dtype=torch.float32, device=proj.device)
@@ -1741,25 +1804,30 @@ class CudaKernels:
             _need(vec is None or (vec.dtype == torch.float32 and vec.numel() == heads and vec.is_contiguous()),
                   "decay_scan: per-head vectors are float32 [heads]")
         out = torch.empty((T, heads * dv), dtype=torch.float32, device=q.device)
-        if self._scans_by_chunks(getattr(ctx, "dtype", None), ctx, heads, dk, dv, q, k, v, *([raw] if mode == 0 else [])):
-            room = torch.empty(int(self.lib.ifx_chunk_scan_scratch_floats(T, ctx.num_requests, heads, dk, dv, int(mode == 0))),
+        if self._scans_by_chunks(getattr(ctx, "dtype", None), ctx, heads, dk, dv, q, k, v, *([raw] if mode == 0 else []), constant=mode == 2):
+            least, short = self._parting(ctx)
+            room = torch.empty(int(self.lib.ifx_chunk_scan_scratch_floats(T, ctx.num_requests, least, heads, dk, dv, int(mode == 0))),
                                dtype=torch.float32, device=q.device)
             _check(self.lib.ifx_chunk_decay_scan(
                 *self._rows_f32(q, "decay_scan q"), *self._rows_f32(k, "decay_scan k"), *self._rows_f32(v, "decay_scan v"),
                 *(self._rows_f32(raw, "decay_scan raw") if raw is not None else (_ptr(None), _LL(0))), _ptr(state),
                 ctypes.c_longlong(state.stride(0)), _ptr(ctx.req_slot), _ptr(ctx.cu_seqlens), _ptr(out), _ptr(step_bias),
-                _ptr(log_rate), _ptr(skip), ctx.num_requests, T, int(heads), int(groups), int(dk), int(dv), mode,
+                _ptr(log_rate), _ptr(skip), ctx.num_requests, T, least, int(heads), int(groups), int(dk), int(dv), mode,
                 ctypes.c_float(tau), ctypes.c_float(q_scale), _ptr(room), _ptr(rate), _stream()), "decay_scan (stretches)")
             self.launches += 3
-            return out
+            if not short:
+                return out
+            longest = short                                # the other spans, token by token
+        else:
+            longest = int(ctx.max_span)
         scratch = None                                     # steps with long spans make their decays in a pass of their own
-        if ctx.max_span >= 64 and mode != 2:
+        if longest >= 64 and mode != 2:
             scratch = torch.empty(T * (heads * dk if mode == 0 else 2 * heads), dtype=torch.float32, device=q.device)
         _check(self.lib.ifx_decay_scan_rate(*self._rows_f32(q, "decay_scan q"), *self._rows_f32(k, "decay_scan k"),
                                        *self._rows_f32(v, "decay_scan v"),
                                        *(self._rows_f32(raw, "decay_scan raw") if raw is not None else (_ptr(None), _LL(0))), _ptr(state),
                                        ctypes.c_longlong(state.stride(0)), _ptr(ctx.req_slot), _ptr(ctx.cu_seqlens), _ptr(out),
-                                       _ptr(step_bias), _ptr(log_rate), _ptr(skip), ctx.num_requests, T, int(ctx.max_span), int(heads),
+                                       _ptr(step_bias), _ptr(log_rate), _ptr(skip), ctx.num_requests, T, longest, int(longest < ctx.max_span), int(heads),
                                        int(groups), int(dk), int(dv), mode, ctypes.c_float(tau), ctypes.c_float(q_scale), 296,
                                        _ptr(scratch), _ptr(rate), _stream()), "decay_scan")
         self.launches += 1 + int(scratch is not None)

@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(kScanThreads) wkv_scan_kernel(
     const float* __restrict__ u, const float* __restrict__ norm_w, float eps, float* __restrict__ s_state,
     float* __restrict__ prev_state, long long slot_stride, const float* __restrict__ x, int C,
     const int* __restrict__ cu_seqlens, const int* __restrict__ req_slot, float* __restrict__ o_scratch,
-    TO* __restrict__ y, int H, int D, int DC, int TB, int fused_norm, int wide_copies, int ld, int ld_w) {
+    TO* __restrict__ y, int H, int D, int DC, int TB, int fused_norm, int wide_copies, int ld, int ld_w, int max_span) {
   extern __shared__ __align__(16) float smem[];
   constexpr int DP = KS * R;                         // a staged row of r, k or w: D numbers, then zeros up to KS * R
   const int per_buf = TB * (3 * DP + DC);
@@ -101,6 +101,7 @@ __global__ void __launch_bounds__(kScanThreads) wkv_scan_kernel(
   const int req = blockIdx.x, head = blockIdx.y, j0 = blockIdx.z * DC;
   const int cols = min(DC, D - j0);                  // value channels of this block
   const int lo = cu_seqlens[req], hi = cu_seqlens[req + 1];
+  if (hi - lo > max_span) return;                    // left to chunk_scan.cu
   const int slot = req_slot[req];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
   const int jl = tid / KS, s = tid % KS;
@@ -272,19 +273,24 @@ int ifx_tanh_rows(void* z, long long n, int dtype, cudaStream_t stream) {
 // r, k, v, w_raw, g: float32 [T, H * D] in rows `ld` floats apart (`ld_w` for w_raw): they may be column
 // blocks of one wider matrix.  s_state / prev_state: slot 0's matrix block [H, D, D] and input row [C]
 // inside the state tensor, slots slot_stride floats apart.  o_scratch: float32 [T, H * D].  y: [T, H * D].
+// max_span: 0, or only spans of up to that many tokens are worked on, and only as far as o_scratch (ifx_wkv_norm follows
+// when the other spans' sums are there too).
 int ifx_wkv_scan(const float* r, const float* k, const float* v, const float* w_raw, const float* g, const float* w0,
                  const float* u, const float* norm_w, float eps, float* s_state, float* prev_state,
                  long long slot_stride, const float* x, int C, const int* cu_seqlens, const int* req_slot,
                  float* o_scratch, void* y, int num_requests, int num_tokens, int H, int D, int ld, int ld_w, int out_dtype,
-                 cudaStream_t stream) {
+                 int max_span, cudaStream_t stream) {
   if (num_requests <= 0 || num_tokens <= 0) return 0;
-  if (H <= 0 || D <= 0 || D > 256 || H > 65535 || ld < H * D || ld_w < H * D) return IFX_E_BADARG;
+  if (H <= 0 || D <= 0 || D > 256 || H > 65535 || ld < H * D || ld_w < H * D || max_span < 0) return IFX_E_BADARG;
   // threads per value channel (a power of two that depends on the head size alone, so that a sum's order does too)
   // and key channels per thread: four, eight for the largest heads
   int ks = 1;
   while (ks < 32 && ks * 4 < D) ks *= 2;
   int rows = ks * 4 >= D ? 4 : 8;
-  const int longest = num_tokens - (num_requests - 1);                 // no span is longer than this
+  const bool all = max_span == 0;
+  int longest = num_tokens - (num_requests - 1);                       // no span is longer than this
+  if (all) max_span = longest;
+  if (longest > max_span) longest = max_span;
   // A bfloat16 run's long spans (prompt portions) are bound by the latency of one warp's instructions per token:
   // two key channels a thread make twice the warps with half the work each.  The float32 run keeps one split per
   // head size, so that its sums have one order however the tokens are cut.
@@ -306,15 +312,15 @@ int ifx_wkv_scan(const float* r, const float* k, const float* v, const float* w_
   while (tb > 4 && ((size_t)2 * tb * (3 * dp + dc) + tb) * sizeof(float) > 160 * 1024) tb /= 2;
   const size_t smem = ((size_t)2 * tb * (3 * dp + dc) + tb) * sizeof(float);
   const int wide = (D % 4 == 0 && dc % 4 == 0 && ld % 4 == 0 && ld_w % 4 == 0 && ((uintptr_t)r | (uintptr_t)k | (uintptr_t)v | (uintptr_t)w_raw) % 16 == 0) ? 1 : 0;
-  const int fused = groups == 1 ? 1 : 0;
+  const int fused = groups == 1 && all ? 1 : 0;
   dim3 grid(num_requests, H, groups);
 #define IFX_SCAN(KS_, R_, TO)                                                                                    \
   do {                                                                                                           \
     auto kern = wkv_scan_kernel<KS_, R_, TO>;                                                                    \
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);    \
     kern<<<grid, threads, smem, stream>>>(r, k, v, w_raw, g, w0, u, norm_w, eps, s_state, prev_state, slot_stride, \
-                                          x, C, cu_seqlens, req_slot, o_scratch, (TO*)y, H, D, dc, tb, fused, wide, ld, ld_w); \
-    if (!fused) {                                                                                                \
+                                          x, C, cu_seqlens, req_slot, o_scratch, (TO*)y, H, D, dc, tb, fused, wide, ld, ld_w, max_span); \
+    if (all && !fused) {                                                                                           \
       const long long items = (long long)num_tokens * H;                                                        \
       wkv_norm_kernel<TO><<<(unsigned)((items + 7) / 8), 256, 0, stream>>>(o_scratch, g, norm_w, eps, (TO*)y, items, H, D, ld); \
     }                                                                                                            \

@@ -179,3 +179,68 @@ def test_products_that_a_scan_does_not_form(cuda_kernels, mode, H, G, dk, dv):
     size = walk.abs().amax(-1, keepdim=True)                                    # float32 sums of up to 200 terms
     assert float(((out - walk).abs() / size).max()) <= 1e-4
     assert float((state - state_w).abs().max()) <= 1e-5 * float(state_w.abs().max())
+
+
+MIXED = [((300, 1, 130, 90), (3, 0, 2, 1)), ((1, 300, 1, 5), (3, 2, 0, 1)), ((1, 1, 1, 1), (0, 1, 2, 3))]
+
+
+def _mixed_ctx(lens, slots, device):
+    ctx = _Ctx(lens, slots, device)
+    ctx.spans = [(0, n) for n in lens]
+    return ctx
+
+
+@pytest.mark.parametrize("mode,H,G,dk,dv", [("sigmoid_root", 2, 2, 64, 128), ("softplus_step", 2, 1, 128, 64), ("constant", 3, 3, 64, 64)])
+def test_long_spans_by_stretches_beside_short_ones_by_the_scan(cuda_kernels, mode, H, G, dk, dv):
+    g = torch.Generator().manual_seed(dk)
+    vec = [torch.rand(H, generator=g) for _ in range(3)]
+    kw = {"sigmoid_root": {"tau": 3.0}, "softplus_step": {"step_bias": vec[0], "log_rate": vec[1], "skip": vec[2]},
+          "constant": {"rate": vec[0]}}[mode]
+    on = {k: v.to(DEV) if torch.is_tensor(v) else v for k, v in kw.items()}
+    state, state_p = torch.zeros(4, H * dk * dv, device=DEV), torch.zeros(4, H * dk * dv, dtype=F64)
+    for step, (lens, slots) in enumerate(MIXED):
+        wide, raw = _decay_inputs(mode, sum(lens), H, G, dk, dv, g, 1.0)
+        cut = lambda t: (t[:, :G * dk], t[:, G * dk:2 * G * dk], t[:, 2 * G * dk:2 * G * dk + H * dv])
+        want = PlainKernels(wide=True).decay_scan(*cut(wide.double()), None if raw is None else raw.double(), state_p, _Ctx(lens, slots, "cpu"),
+                                                  heads=H, groups=G, dk=dk, dv=dv, decay=mode, **kw).double()
+        before = cuda_kernels.launches
+        got = cuda_kernels.decay_scan(*cut(wide.to(DEV)), None if raw is None else raw.to(DEV), state, _mixed_ctx(lens, slots, DEV), heads=H,
+                                      groups=G, dk=dk, dv=dv, decay=mode, **on)
+        # three for the stretches, the scan, and its decays ahead of it where its longest span has 64 tokens and they are not constant
+        assert cuda_kernels.launches - before == ((5 if mode != "constant" else 4), 4, 1)[step]
+        for a, b in ((got, want), (state, state_p)):                            # float32 sums of up to 300 terms
+            assert float((a.double().cpu() - b).abs().max()) <= 5e-6 * max(1.0, float(b.abs().max()))
+
+
+@pytest.mark.parametrize("H,D", [(3, 64), (1, 128)])
+def test_wkv_of_long_and_short_spans(cuda_kernels, H, D):
+    HD, C = H * D, 40
+    g = torch.Generator().manual_seed(H)
+    w0, u, nw = torch.randn(HD, generator=g), 0.5 * torch.randn(HD, generator=g), 1 + 0.2 * torch.randn(HD, generator=g)
+    state, state_p = torch.zeros(4, HD * D + C, device=DEV), torch.zeros(4, HD * D + C, dtype=F64)
+    for step, (lens, slots) in enumerate(MIXED):
+        T = sum(lens)
+        r, k, v, gate, w_raw = (torch.randn(T, HD, generator=g) for _ in range(5))
+        x = torch.randn(T, C, generator=g)
+        want = PlainKernels(wide=True).wkv_scan(r, k, v, w_raw, gate, w0, u, nw, 1e-5, H, D, state_p, HD * D, x.double(),
+                                                _Ctx(lens, slots, "cpu"), F64)
+        before = cuda_kernels.launches
+        y = cuda_kernels.wkv_scan(*(t.to(DEV) for t in (r, k, v, w_raw, gate, w0, u, nw)), 1e-5, H, D, state, HD * D, x.to(DEV),
+                                  _mixed_ctx(lens, slots, DEV), torch.bfloat16)
+        assert cuda_kernels.launches - before == (5, 5, 1)[step]
+        assert float((y.double().cpu() - want).abs().max()) <= 2.0 ** -8 * max(1.0, float(want.abs().max()))
+        assert float((state.double().cpu() - state_p).abs().max()) <= 5e-6 * max(1.0, float(state_p.abs().max()))
+
+
+def test_rows_off_a_16_byte_boundary_go_by_the_scan(cuda_kernels):
+    """The kernels of long spans refuse them before they touch anything; nothing is done twice."""
+    T, H, d = 200, 2, 64
+    g = torch.Generator().manual_seed(9)
+    rows, rate = torch.randn(T, 3 * H * d + 1, generator=g).to(DEV), torch.full((H,), 0.9, device=DEV)
+    results = []
+    for dtype in (torch.bfloat16, torch.float32):
+        state = torch.ones(1, H * d * d, device=DEV)
+        cut = [rows[:, 1 + i * H * d:1 + (i + 1) * H * d] for i in range(3)]
+        results.append((cuda_kernels.decay_scan(*cut, None, state, _Ctx((T,), (0,), DEV, dtype), heads=H, groups=H, dk=d, dv=d,
+                                                decay="constant", rate=rate), state))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])

@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from plain.plain_kernels import PlainKernels
-from test_chunk_scan_gpu import STEPS, _Ctx
+from test_chunk_scan_gpu import MIXED, STEPS, _Ctx, _mixed_ctx
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -107,3 +107,23 @@ def test_products_that_a_scan_does_not_form(cuda_kernels, block):
     fine = torch.isfinite(walk)
     assert float((y - walk)[fine].abs().max()) <= 2.0 ** -7 * float(walk[fine].abs().max())
     assert float((state - state_w).abs().max()) <= 1e-5 * float(state_w.abs().max())
+
+
+def test_long_spans_by_stretches_beside_short_ones_by_the_scan(cuda_kernels, monkeypatch):
+    monkeypatch.setattr(cuda_kernels, "delta_stretches_pay", lambda *a: True)
+    H, D = 3, 64
+    HD = H * D
+    g = torch.Generator().manual_seed(8)
+    vec = [torch.randn(HD, generator=g) for _ in range(3)]
+    state, state_p = torch.zeros(4, HD * D, device=DEV), torch.zeros(4, HD * D, dtype=F64)
+    for step, (lens, slots) in enumerate(MIXED):
+        T = sum(lens)
+        proj, w_raw = torch.randn(T, 5 * HD, generator=g), torch.randn(T, HD, generator=g)
+        want = PlainKernels(wide=True).delta_rule_scan(proj.double(), w_raw.double(), *vec, 1e-5, H, D, state_p, _Ctx(lens, slots, "cpu"), F64)
+        before = cuda_kernels.launches
+        y = cuda_kernels.delta_rule_scan(proj.to(DEV), w_raw.to(DEV), *(t.to(DEV) for t in vec), 1e-5, H, D, state,
+                                         _mixed_ctx(lens, slots, DEV), BF)
+        assert cuda_kernels.launches - before == (6, 6, 3)[step]                # two more for the short spans; the scan alone
+        # the norm divides by the size of a head's sums, which may be small
+        assert float((y.double().cpu() - want).abs().max()) <= 2.0 ** -8 * max(1.0, float(want.abs().max()))
+        assert float((state.double().cpu() - state_p).abs().max()) <= 5e-6 * max(1.0, float(state_p.abs().max()))
