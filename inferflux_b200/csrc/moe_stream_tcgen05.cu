@@ -15,8 +15,9 @@
 //   warps 2-5  epilogue: activation or weight, rows of act / y
 //   warp 6     the pairs' rows into the stages by cp.async, swizzled as TMA would, AHEAD stages before they are handed over
 //
-// An expert with more pairs than a block takes at once (`nmax`) goes through its weights again.  Blocks of experts that no
-// token chose leave at once.
+// An expert with more pairs than a block takes at once (`nmax`) goes through its weights again.  A step with fewer than two pairs
+// an expert has blocks for as many experts as it has pairs, and the i-th of them finds the i-th expert that some token chose
+// (blocks for all experts, most of which leave at once, cost 7 ns each: 110 us with 256 experts of 2,048 x 1,024).
 //
 // Bound: reading the chosen experts' weights.  24 tokens, 16 gated experts of 1,536 x 2,240, four a token (330 MB): the
 // per-token kernels 244 us (up 146, down 98), these 81 (4.1 TB/s; 5.1 TB/s on matrices five times as large: what is lost is
@@ -27,6 +28,7 @@
 namespace ifx {
 
 constexpr int kStreamMaxPairs = 512;          // pairs of a step
+constexpr int kStreamMaxExperts = 1024;
 constexpr int kStreamThreads = 224;
 constexpr uint32_t kStreamWeightBytes = 128 * 128;
 enum { STREAM_RELU2 = 0, STREAM_GLU = 1, STREAM_DOWN = 2 };
@@ -63,18 +65,50 @@ struct StreamArgs {
   const float* weights;
   void* out;                       // up: act [pairs, N] bfloat16; down: y [pairs, N] float32
   int pairs, top, N, K, group_rows, nmax, stages, slice;               // slice: k-blocks of a block
-  int early;                       // fetch the first weights before it is known whether the expert has pairs
+  int experts;
+  int early;                       // blocks for every expert, which fetch the first weights before it is known whether it has pairs
   float limit, slope, offset;
   int* error_flag;
 };
 
-// grid (tiles of N, experts, slices of K)
+// The place-th expert that some pair chose, -1 if there are fewer: bits of chosen experts, counted by the first warp.
+__device__ __forceinline__ int chosen_expert(const int* __restrict__ ids, int pairs, int experts, int place, uint32_t* bits_s, int* found_s) {
+  for (int i = threadIdx.x; i < kStreamMaxExperts / 32; i += kStreamThreads) bits_s[i] = 0u;
+  if (threadIdx.x == 0) *found_s = -1;
+  __syncthreads();
+  for (int p = threadIdx.x; p < pairs; p += kStreamThreads) {
+    const int e = ids[p];
+    if (e >= 0 && e < experts) atomicOr(&bits_s[e >> 5], 1u << (e & 31));
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    static_assert(kStreamMaxExperts == 32 * 32, "a lane a word");
+    uint32_t word = bits_s[threadIdx.x];
+    int before = __popc(word);                                         // experts in front of this lane's
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, before, o);
+      if ((int)threadIdx.x >= o) before += x;
+    }
+    before -= __popc(word);
+    int left = place - before;
+    if (left >= 0 && left < __popc(word)) {
+      for (; left > 0; --left) word &= word - 1;
+      *found_s = (int)threadIdx.x * 32 + __ffs(word) - 1;
+    }
+  }
+  __syncthreads();
+  return *found_s;
+}
+
+// grid (tiles of N, experts or at most as many as there are pairs, slices of K)
 template <int KIND, int AHEAD>
 __global__ void __launch_bounds__(kStreamThreads) moe_stream_kernel(const __grid_constant__ CUtensorMap map_w, const StreamArgs a) {
   constexpr int TILE = KIND == STREAM_GLU ? 64 : 128;                  // outputs of a block
   extern __shared__ unsigned char smem_raw[];
   __shared__ int list_s[kStreamMaxPairs];                              // this expert's pairs, in any order
-  __shared__ int count_s;
+  __shared__ int count_s, found_s;
+  __shared__ uint32_t bits_s[kStreamMaxExperts / 32];
   __shared__ float up_rows[KIND == STREAM_GLU ? 64 : 1][17];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const uint32_t stage_bytes = kStreamWeightBytes + a.nmax * 128;
@@ -83,7 +117,8 @@ __global__ void __launch_bounds__(kStreamThreads) moe_stream_kernel(const __grid
   const uint32_t ring = smem_addr(smem), full0 = smem_addr(bars), empty0 = full0 + 8 * a.stages, done_bar = empty0 + 8 * a.stages,
                  free_bar = done_bar + 8;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = blockIdx.x * TILE, expert = blockIdx.y;
+  const int n0 = blockIdx.x * TILE;
+  int expert = blockIdx.y;
   const uint32_t tmem_cols = a.nmax < 32 ? 32 : a.nmax;                // nmax: a power of two
 
   pdl_launch_dependents();
@@ -119,8 +154,9 @@ __global__ void __launch_bounds__(kStreamThreads) moe_stream_kernel(const __grid
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_holder;
+  if (!a.early) expert = chosen_expert(a.ids, a.pairs, a.experts, blockIdx.y, bits_s, &found_s);
   for (int p = threadIdx.x; p < a.pairs; p += kStreamThreads)
-    if (a.ids[p] == expert) list_s[atomicAdd(&count_s, 1)] = p;        // a pair's place among the others changes no result
+    if (expert >= 0 && a.ids[p] == expert) list_s[atomicAdd(&count_s, 1)] = p;        // a pair's place among the others changes no result
   __syncthreads();
   const int count = count_s;
   const int passes = (count + a.nmax - 1) / a.nmax, total = passes * kblocks;
@@ -306,7 +342,7 @@ static int launch_stream_ahead(const CUtensorMap& mw, const StreamArgs& a, int e
   auto kern = moe_stream_kernel<KIND, AHEAD>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  return launch_pdl(kern, dim3((a.N + tile - 1) / tile, experts, slices), dim3(kStreamThreads), smem, stream, 1, mw, a);
+  return launch_pdl(kern, dim3((a.N + tile - 1) / tile, a.early || experts < a.pairs ? experts : a.pairs, slices), dim3(kStreamThreads), smem, stream, 1, mw, a);
 }
 
 template <int KIND>
@@ -340,8 +376,8 @@ int ifx_moe_stream(const void* h, const void* w_up, const void* w_down, const in
                    void* out, int T, int top, int experts, int width, int ff, int out_dtype, int glu, float limit, float slope,
                    float offset, int* error_flag, cudaStream_t stream) {
   if (T <= 0) return 0;
-  if (top <= 0 || experts <= 0 || experts > 65535 || width <= 0 || ff <= 0 || error_flag == nullptr) return IFX_E_BADARG;
-  if ((long long)T * top > kStreamMaxPairs) return IFX_E_TOOBIG;
+  if (top <= 0 || experts <= 0 || width <= 0 || ff <= 0 || error_flag == nullptr) return IFX_E_BADARG;
+  if ((long long)T * top > kStreamMaxPairs || experts > kStreamMaxExperts) return IFX_E_TOOBIG;
   if (width % 8 || ff % 8 || ((uintptr_t)h | (uintptr_t)w_up | (uintptr_t)w_down | (uintptr_t)act | (uintptr_t)y | (uintptr_t)out) % 16)
     return IFX_E_ALIGN;
   if (out_dtype != IFX_DT_F32 && out_dtype != IFX_DT_BF16) return IFX_E_DTYPE;
@@ -355,6 +391,7 @@ int ifx_moe_stream(const void* h, const void* w_up, const void* w_down, const in
   a.weights = weights;
   a.pairs = T * top;
   a.top = top;
+  a.experts = experts;
   a.early = a.pairs >= 2 * experts;                                    // then nearly every expert has some
   a.nmax = T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : 128;           // a token chooses an expert once
   a.stages = 0;

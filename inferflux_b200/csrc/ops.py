@@ -1613,9 +1613,9 @@ class CudaKernels:
             _need(h.is_contiguous() and w_up.dtype == h.dtype and w_down.dtype == h.dtype and w_up.is_contiguous()
                   and w_down.is_contiguous() and tuple(w_up.shape) == (experts, 2 * ff, width)
                   and tuple(w_down.shape) == (experts, width, ff), "moe_experts: stacked expert weights in the activations' dtype")
-            if self._moe_on_tensor_cores(h, w_up, w_down, ff, width):
+            if h.dtype == torch.bfloat16:
                 way = self.moe_kernels(T * top, int(experts), width, ff, True)
-                if way != "tokens":
+                if way != "tokens" and self._moe_on_tensor_cores(h, w_up, w_down, ff, width):
                     return (self._moe_experts_tiles if way == "tiles" else self._moe_experts_stream)(
                         h, w_up, w_down, ids, weights, experts, out_dtype, glu=glu)
             act = torch.empty((T * top, ff), dtype=h.dtype, device=h.device)
@@ -1630,9 +1630,9 @@ class CudaKernels:
         _need(h.is_contiguous() and (not experts or (w_up.dtype == h.dtype and w_down.dtype == h.dtype and w_up.is_contiguous()
               and w_down.is_contiguous() and tuple(w_up.shape) == (experts, ff, width) and tuple(w_down.shape) == (experts, width, ff))),
               "moe_experts: stacked expert weights in the activations' dtype")
-        if experts and self._moe_on_tensor_cores(h, w_up, w_down, ff, width):
+        if experts and h.dtype == torch.bfloat16:
             way = self.moe_kernels(T * top, int(experts), width, ff, False)
-            if way != "tokens":
+            if way != "tokens" and self._moe_on_tensor_cores(h, w_up, w_down, ff, width):
                 return (self._moe_experts_tiles if way == "tiles" else self._moe_experts_stream)(
                     h, w_up, w_down, ids, weights, experts, out_dtype)
         act = torch.empty((T * top, ff), dtype=h.dtype, device=h.device)
@@ -1643,26 +1643,37 @@ class CudaKernels:
         self.launches += 2 if experts else 1
         return out
 
-    # Which kernels make the experts of a bfloat16 step, by the number of (token, choice) pairs.  Measured on a B200 (us; per
-    # token / every chosen expert's weights once / sorted 128-row tiles; 16 experts, four a token):
-    #   1,536 x 2,240 gated   1 token 57 / 46 / 51, 8: 107 / 81 / 92, 24: 240 / 81 / 95, 48: 426 / 93 / 95, 64: 549 / 107 / 95
-    #   1,536 x 3,328         1 token 56 / 46 / 59, 8: 103 / 82 / 91, 24: 227 / 84 / 94, 64: 483 / 89 / 94
-    #   3,584 x 4,736 gated   1 token 150 / 109 / 110, 8: 514 / 312 / 299, 24: 1,100 / 329 / 323, 64: 2,426 / 392 / 321
-    #   512 x 512 gated       1 token 8.5 / 18 / 24, 24: 15 / 19 / 25, 32: 21 / 20 / 25
-    # The tiles are the better once an expert has a dozen tokens (their rows then are not mostly padding, and the stream's
-    # gathering grows), or once its matrices are large enough to keep every SM at whole tiles; work of a few megabytes ends
-    # before the other two have filled their pipelines.
+    # Which kernels make the experts of a bfloat16 step, by the number of (token, choice) pairs.  Measured on a B200 with every
+    # expert's weights in HBM (us; per token / every chosen expert's weights once / sorted 128-row tiles):
+    #    16 experts, 1,536 x 2,240 gated, four a token   1 token 71 / 48 / 69, 8: 122 / 93 / 111, 24: 255 / 95 / 118, 64: 560 / 114 / 116
+    #     8 experts, the same, two a token               1 token 46 / 46 / 62, 16: 108 / 52 / 87, 64: 300 / 60 / 87
+    #    32 experts, the same, four a token              8 tokens 132 / 128 / 150, 24: 279 / 169 / 177, 64: 585 / 167 / 185
+    #    64 experts, 2,048 x 1,408 gated, six a token    1 token 83 / 54 / 99, 4: 124 / 118 / 144, 16: 290 / 230 / 251, 48: 610 / 267 / 280
+    #   128 experts, 2,048 x 768 gated, eight a token    4 tokens 88 / 116 / 134, 16: 216 / 249 / 255, 32: 343 / 308 / 329
+    #   256 experts, 2,048 x 1,024 gated, eight a token  1 token 75 / 60 / 110, 8: 196 / 216 / 245, 32: 494 / 572 / 607, 48: 669 / 621 / 710
+    #   256 experts, 3,584 x 1,024, eight a token        1 token 79 / 85 / 153, 16: 364 / 388 / 464, 48: 844 / 724 / 851
+    #    64 experts, 1,536 x 512, four a token           4 tokens 34 / 42 / 65, 16: 58 / 54 / 89, 64: 134 / 62 / 103
+    # (3,584 x 4,736 gated, 16 experts: 1 token 150 / 109 / 110, 8: 514 / 312 / 299, 24: 1,100 / 329 / 323, from L2.)
+    # Per token, where an expert seldom has more than one pair: nothing is read twice then, and the other two have a block for every
+    # tile of an expert all the same; and where the work is a few megabytes, which end before the other two have filled their
+    # pipelines.  Tiles once an expert has a dozen tokens (their rows then are not mostly padding, and the stream's gathering grows), or
+    # once its matrices are large enough to keep every SM at whole tiles.
     MOE_TILES_MIN_PAIRS = 192
     MOE_TILES_LARGE_EXPERT = 1 << 23
     MOE_TOKENS_MAX_WORK = 40_000_000
     MOE_STREAM_MAX_PAIRS = 512
+    MOE_MAX_EXPERTS = 1024     # of the stream and the tiles
 
     @classmethod
     def moe_kernels(cls, pairs, experts, width, ff, gated):
         """"tokens", "stream" or "tiles"."""
-        if pairs < cls.MOE_STREAM_MAX_PAIRS and pairs * ff * width * (3 if gated else 2) < cls.MOE_TOKENS_MAX_WORK:
+        if pairs >= cls.MOE_STREAM_MAX_PAIRS:
+            return "tiles"
+        if (experts > cls.MOE_MAX_EXPERTS or pairs * ff * width * (3 if gated else 2) < cls.MOE_TOKENS_MAX_WORK
+                or not (4 * pairs >= 5 * experts or (pairs <= 16 and experts <= 64))):
             return "tokens"
-        if pairs >= cls.MOE_TILES_MIN_PAIRS or (ff * width >= cls.MOE_TILES_LARGE_EXPERT and pairs >= 2 * experts):
+        if ((pairs >= cls.MOE_TILES_MIN_PAIRS and pairs >= 12 * experts)
+                or (ff * width >= cls.MOE_TILES_LARGE_EXPERT and pairs >= 2 * experts)):
             return "tiles"
         return "stream"
 

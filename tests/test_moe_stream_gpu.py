@@ -38,7 +38,8 @@ def _plain(h, up, down, ids, weights, experts, glu):
 @pytest.mark.parametrize("glu", [None, (7.0, 1.702, 1.0), (float("inf"), 1.0, 0.0)])
 @pytest.mark.parametrize("T,width,ff,experts,identity,top", [
     (1, 64, 64, 4, 0, 2), (5, 72, 40, 5, 2, 3), (16, 136, 200, 3, 0, 3), (17, 256, 136, 6, 1, 2), (33, 64, 1032, 16, 0, 4),
-    (65, 320, 72, 9, 0, 3), (127, 128, 96, 4, 0, 4), (300, 64, 72, 7, 1, 1)])
+    (65, 320, 72, 9, 0, 3), (127, 128, 96, 4, 0, 4), (300, 64, 72, 7, 1, 1),
+    (1, 64, 72, 1024, 0, 2), (3, 72, 64, 33, 1, 4), (20, 64, 72, 300, 2, 3)])                    # fewer pairs than experts
 def test_stream_against_64_bits(cuda_kernels, T, width, ff, experts, identity, top, glu):
     args = _inputs(T, width, ff, experts, experts + identity, top, glu, T + width)
     want = _plain(*args, experts, glu)
@@ -81,3 +82,22 @@ def test_a_token_that_is_not_finite_touches_no_other(cuda_kernels):
     (32, 16, 3584, 4736, True, "tiles"), (300, 3, 64, 32, False, "tokens"), (520, 3, 64, 32, False, "tiles")])
 def test_which_kernels_run(cuda_kernels, pairs, experts, width, ff, gated, want):
     assert cuda_kernels.moe_kernels(pairs, experts, width, ff, gated) == want
+
+
+@pytest.mark.parametrize("pairs,experts,width,ff,gated,want", [
+    (8, 64, 2048, 1408, True, "stream"), (24, 64, 2048, 1408, True, "tokens"), (96, 64, 2048, 1408, True, "stream"),
+    (300, 64, 2048, 1408, True, "stream"), (64, 256, 2048, 1024, True, "tokens"), (192, 256, 2048, 1024, True, "tokens"),
+    (384, 256, 2048, 1024, True, "stream"), (511, 16, 2048, 1024, True, "tiles"), (200, 1025, 1024, 512, True, "tokens"),
+    (512, 256, 2048, 1024, True, "tiles")])
+def test_which_kernels_run_with_many_experts(cuda_kernels, pairs, experts, width, ff, gated, want):
+    """An expert that has one pair at most is read once per token too, without a block for every tile of every expert."""
+    assert cuda_kernels.moe_kernels(pairs, experts, width, ff, gated) == want
+
+
+def test_more_experts_than_the_stream_and_the_tiles_take(cuda_kernels):
+    """Between 192 and 511 pairs they go per token."""
+    T, width, ff, experts = 100, 64, 72, 1100
+    h, up, down, ids, weights = _inputs(T, width, ff, experts, experts, 2, None, 3)
+    want = _plain(h, up, down, ids, weights, experts, None)
+    got = cuda_kernels.moe_experts(h.to(DEV), up.to(DEV), down.to(DEV), ids.to(DEV), weights.to(DEV), experts, torch.float32)
+    assert float((got.double().cpu() - want).abs().max()) <= 4 * 2.0 ** -8 * ff ** -0.5 * max(1.0, float(want.abs().max()))
