@@ -721,6 +721,7 @@ class CudaKernels:
         if len(single) > 16:
             single.sort(key=lambda m: -m[1])
         # (longest, sum) of the decoded tokens' keys, for least_decode_splits; a captured step takes it back
+        ctx.__dict__.pop("prefill_parts", None)            # what an earlier list of spans gave
         ctx.decode_keys = (1 + max(m[1] for m in single), len(single) + sum(m[1] for m in single)) if single else None
         return {"attn.decode_rows": rows, "attn.decode_meta": [v for m in single for v in m], "attn.prefill_tiles": tiles}
 
@@ -847,8 +848,7 @@ class CudaKernels:
             parts = self.prefill_parts(ctx, nq, win)
             room = None
             if parts > 1:
-                room = torch.empty(int(self.lib.ifx_attention_prefill_tcgen05_parts_bytes(num_tiles, nq, d, parts)), dtype=torch.uint8,
-                                   device=q.device)
+                room = torch.empty(self.prefill_parts_bytes(num_tiles, nq, d, parts), dtype=torch.uint8, device=q.device)
                 self.launches += 1
             _check(self.lib.ifx_attention_prefill_tcgen05_parts(
                 _ptr(q), T, _ptr(kv), _ptr(table), _ptr(tiles), _ptr(ctx.req_slot), _ptr(out),
@@ -877,14 +877,27 @@ class CudaKernels:
 
     PREFILL_PART_TILES = 4     # key tiles (of 128) that a part of a prompt attention block keeps at least
 
+    @staticmethod
+    def prefill_parts_bytes(num_tiles, nq, d, parts):
+        """What ifx_attention_prefill_tcgen05_parts_bytes says: a sum of d numbers, a reference and a denominator per row of a part."""
+        return num_tiles * nq % 148 * parts * 256 * (d + 2) * 4
+
     def prefill_parts(self, ctx, nq, window):
-        """Parts of their keys that the prompt attention's left over blocks are cut into (1: whole).  A block takes up to 256 tokens of a
-        head and an SM to itself, so what is left behind whole rounds of 148 blocks leaves SMs idle for as long as its longest
+        """Parts of their keys that the prompt attention's left over blocks are cut into (1: whole), found once a step and kind of layer."""
+        known = ctx.__dict__.setdefault("prefill_parts", {})
+        parts = known.get((nq, window))
+        if parts is None:
+            parts = known[nq, window] = self._prefill_parts(ctx, nq, window)
+        return parts
+
+    def _prefill_parts(self, ctx, nq, window):
+        """A block takes up to 256 tokens of a head and an SM to itself, so what is left behind whole rounds of 148 blocks leaves SMs idle for as long as its longest
         block walks; with few blocks that is the whole grid.  Cut while every part keeps four tiles of 128 keys: with parts of
         three or of six the times below are the same or up to 3 % longer, and below that adding the parts up takes what they save.
+        Eight tiles stay whole too: two parts of four save 0.6 us, and the launch that adds them up costs the host 3.
         us, whole and cut: 28 heads, two requests' 2,500 tokens behind up to 4,000 (12 of 308 blocks left) 191 and 162, 384 tokens
         behind 2,000 39.0 and 32.4; 12 heads, 512 tokens behind 3,000 (24 blocks, six parts) 61.9 and 30.2, 600 tokens behind 900
-        26.9 and 24.6, 1,024 tokens 24.4 and 23.8."""
+        26.9 and 24.6."""
         blocks = ctx.extra_len["attn.prefill_tiles"] // 4 * nq
         left = blocks % 148
         if not 0 < left <= 74:
@@ -898,7 +911,7 @@ class CudaKernels:
                 longest = max(longest, -(-end // 128) - (max(0, first - window + 1) // 128 if window else 0))
                 items -= 1
                 if not items:
-                    return max(1, min(148 // left, longest // self.PREFILL_PART_TILES, 8))
+                    return max(1, min(148 // left, longest // self.PREFILL_PART_TILES, 8)) if longest > 2 * self.PREFILL_PART_TILES else 1
         return 1
 
     @staticmethod

@@ -40,3 +40,8 @@ def test_parts_of_keys(cuda_kernels, nq, nkv, d, page, window, lens, spans, part
             bound = (2 ** -8 + 1e-4) * size + 2 ** -8 * want.abs() + 1e-6
             assert ((got[t:t + s, h] - want).abs() <= 1.1 * bound).all(), (h, t)
         t += s
+
+
+def test_bytes_of_the_parts(cuda_kernels):
+    for case in ((2, 12, 128, 2), (7, 28, 128, 2), (1, 4, 64, 6), (37, 4, 64, 3)):
+        assert cuda_kernels.prefill_parts_bytes(*case) == cuda_kernels.lib.ifx_attention_prefill_tcgen05_parts_bytes(*case)

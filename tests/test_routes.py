@@ -46,3 +46,34 @@ def test_a_constant_decay_with_small_keys_and_very_many_stretches_stays_with_the
     for lens, way in (((128,) * 32, False), ((256,) * 16, True), ((128,) * 16, True)):
         assert table._scans_by_chunks(torch.bfloat16, _Ctx(lens), 28, 64, 128, constant=True) == way
         assert table._scans_by_chunks(torch.bfloat16, _Ctx(lens), 28, 64, 128)
+
+
+class _Counted(list):
+    walks = 0
+
+    def __iter__(self):
+        self.walks += 1
+        return super().__iter__()
+
+
+def test_parts_of_the_prompt_attention_are_found_once_a_step_and_kind_of_layer():
+    """Every layer asks; the spans are walked for the first one of a kind."""
+    table = type("T", (), {"PREFILL_TILE": CudaKernels.PREFILL_TILE, "PREFILL_PART_TILES": CudaKernels.PREFILL_PART_TILES,
+                           "prefill_parts": CudaKernels.prefill_parts, "_prefill_parts": CudaKernels._prefill_parts,
+                           "attention_sections": CudaKernels.attention_sections})()
+
+    def step(*spans):
+        ctx = type("C", (), {})()
+        ctx.spans, ctx.slots_host = _Counted(spans), list(range(len(spans)))
+        ctx.extra_len = {k: len(v) for k, v in table.attention_sections(ctx).items()}
+        ctx.spans.walks = 0
+        return ctx
+
+    ctx = step((1100, 300))
+    assert [table.prefill_parts(ctx, 12, 0) for _ in range(5)] == [2] * 5 and ctx.spans.walks == 1
+    assert table.prefill_parts(ctx, 12, 600) == 1 and table.prefill_parts(ctx, 12, 600) == 1 and ctx.spans.walks == 2
+    ctx.spans = _Counted([(3000, 512)])                                         # another step's spans
+    ctx.extra_len = {k: len(v) for k, v in table.attention_sections(ctx).items()}
+    assert table.prefill_parts(ctx, 12, 0) == 6
+    for spans, parts in ((((0, 900),), 1), (((0, 1152),), 2), (((5, 1), (9, 1)), 1)):     # eight tiles of keys stay whole
+        assert table.prefill_parts(step(*spans), 12, 0) == parts
