@@ -4,7 +4,9 @@ where the reference uses it too).
 
 There is no CPU path and no library model code here: making a `CudaKernels`
 without a CUDA device, or without being able to build or load the library, raises.
-Tensors are passed as raw device pointers on torch's current stream.
+Tensors are passed as raw device pointers on torch's current stream.  What a call costs the host
+matters where a layer's kernels are short: sizes go to `torch.empty` one by one (as a tuple they
+take a microsecond more), and messages with values in them are made when something is wrong.
 """
 from __future__ import annotations
 
@@ -17,6 +19,7 @@ import torch
 from .build import BuildError, load_library
 
 _DT = {torch.float32: 0, torch.bfloat16: 1}
+_DECAYS = {"sigmoid_root": 0, "softplus_step": 1, "constant": 2}
 
 _ERRORS = {-1: "a size or option the kernel does not take", -2: "unknown dtype",
            -3: "a pointer or stride breaks an alignment rule", -4: "a size beyond the kernel's stated maximum"}
@@ -220,7 +223,7 @@ class CudaKernels:
     # ------------------------------------------------------------- elementwise
     def embed(self, table, token_ids, vocab, scale=1.0):
         T, H = token_ids.numel(), table.shape[1]
-        out = torch.empty((T, H), dtype=torch.float32, device=table.device)
+        out = torch.empty(T, H, dtype=torch.float32, device=table.device)
         if scale != 1.0:
             _check(self.lib.ifx_embed_scaled(_ptr(table), _ptr(token_ids), _ptr(out), T, H, int(vocab), ctypes.c_float(scale),
                                              _DT[table.dtype], _stream()), "embed")
@@ -234,7 +237,7 @@ class CudaKernels:
     def rmsnorm(self, x, w, eps, out_dtype, groups=1):
         _need(x.dtype == torch.float32 and w.dtype == torch.float32, "rmsnorm: x and w must be float32")
         T, H = x.shape
-        out = torch.empty((T, H), dtype=out_dtype, device=x.device)
+        out = torch.empty(T, H, dtype=out_dtype, device=x.device)
         if groups > 1:
             _need(x.is_contiguous() and H % groups == 0, "rmsnorm: the groups must cut a contiguous row evenly")
             _check(self.lib.ifx_groupnorm_stream(
@@ -253,7 +256,7 @@ class CudaKernels:
         dtype or a PartialSum, whose slices are added in the same pass."""
         _need(x.dtype == torch.float32 and w.dtype == torch.float32, "add_rmsnorm: x and w must be float32")
         T, H = x.shape
-        out = torch.empty((T, H), dtype=out_dtype, device=x.device)
+        out = torch.empty(T, H, dtype=out_dtype, device=x.device)
         if isinstance(delta, PartialSum):
             _need(tuple(delta.shape) == (T, H), "add_rmsnorm: partial sums do not match x")
             chunks = -(-H // 512)
@@ -279,8 +282,8 @@ class CudaKernels:
         T, H = x.shape
         if out_dtype != torch.bfloat16 or T > self.SKINNY_MAX_ROWS or H % 8:
             return self.rmsnorm(x, w, eps, out_dtype) if delta is None else self.add_rmsnorm(x, delta, w, eps, out_dtype)
-        pre = torch.empty((T, H), dtype=out_dtype, device=x.device)
-        sumsq = torch.empty((T, -(-H // 512)), dtype=torch.float32, device=x.device)
+        pre = torch.empty(T, H, dtype=out_dtype, device=x.device)
+        sumsq = torch.empty(T, -(-H // 512), dtype=torch.float32, device=x.device)
         if isinstance(delta, PartialSum):
             _need(tuple(delta.shape) == (T, H), "prenorm: partial sums do not match x")
             src, splits = delta.parts, delta.splits
@@ -297,7 +300,7 @@ class CudaKernels:
         if not isinstance(h, ScaledRows):
             return h
         T, H = h.shape
-        out = torch.empty((T, H), dtype=h.dtype, device=h.pre.device)
+        out = torch.empty(T, H, dtype=h.dtype, device=h.pre.device)
         _check(self.lib.ifx_scale_rows(_ptr(h.pre), _ptr(h.sumsq), _ptr(out), T, H, ctypes.c_float(h.eps),
                                        _DT[h.dtype], _stream()), "scale_rows")
         self.launches += 1
@@ -317,7 +320,7 @@ class CudaKernels:
         if not isinstance(value, PartialSum):
             return value if bias is None else value + bias.to(value.dtype)
         T, N = value.shape
-        out = torch.empty((T, N), dtype=value.dtype, device=value.parts.device)
+        out = torch.empty(T, N, dtype=value.dtype, device=value.parts.device)
         _check(self.lib.ifx_reduce_partial(_ptr(value.parts), _ptr(bias), _ptr(out), T, N, value.splits,
                                            _DT[value.dtype], _stream()), "reduce_partial")
         self.launches += 1
@@ -325,7 +328,7 @@ class CudaKernels:
 
     def silu_mul(self, gate_up):
         T, two_i = gate_up.shape
-        out = torch.empty((T, two_i // 2), dtype=gate_up.dtype, device=gate_up.device)
+        out = torch.empty(T, two_i // 2, dtype=gate_up.dtype, device=gate_up.device)
         _check(self.lib.ifx_silu_mul(_ptr(gate_up), _ptr(out), T, two_i // 2, _DT[gate_up.dtype], _stream()),
                "silu_mul")
         self.launches += 1
@@ -333,7 +336,7 @@ class CudaKernels:
 
     def gather_rows(self, x, rows):
         R, H = rows.numel(), x.shape[1]
-        out = torch.empty((R, H), dtype=torch.float32, device=x.device)
+        out = torch.empty(R, H, dtype=torch.float32, device=x.device)
         _check(self.lib.ifx_gather_rows(_ptr(x), _ptr(rows), _ptr(out), R, H, x.shape[0], _stream()), "gather_rows")
         self.launches += 1
         return out
@@ -365,19 +368,21 @@ class CudaKernels:
         rows = a if isinstance(a, ScaledRows) else None
         if rows is not None:
             a = rows.pre
-        _need(a.dtype == w.dtype, f"linear: activations are {a.dtype}, weights {w.dtype}")
+        if a.dtype != w.dtype:                             # (messages with values in them are made when they are needed)
+            raise KernelError(f"linear: activations are {a.dtype}, weights {w.dtype}")
         _need(a.is_contiguous() and w.is_contiguous(), "linear: operands must be contiguous")
         T, K = a.shape
         N = w.shape[0]
-        _need(w.shape[1] == K, f"linear: inner sizes differ ({K} vs {w.shape[1]})")
+        if w.shape[1] != K:
+            raise KernelError(f"linear: inner sizes differ ({K} vs {w.shape[1]})")
         out_dtype = out_dtype or a.dtype
         if T == 0:
-            return torch.empty((T, N), dtype=out_dtype, device=a.device)
+            return torch.empty(T, N, dtype=out_dtype, device=a.device)
         if rows is not None and not (T <= self.SKINNY_MAX_ROWS and K % 8 == 0 and w.data_ptr() % 16 == 0):
             a, rows = self.materialize_rows(rows), None
         if a.dtype == torch.float32:
             _need(out_dtype == torch.float32, "linear: a float32 product gives float32")
-            out = torch.empty((T, N), dtype=out_dtype, device=a.device)
+            out = torch.empty(T, N, dtype=out_dtype, device=a.device)
             _check(self.lib.ifx_gemm_generic(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), T, N, K, 0, 0, _stream()),
                    "gemm (float32)")
             self.launches += 1
@@ -394,7 +399,7 @@ class CudaKernels:
                 return PartialSum(parts, out_dtype)
             if tiles >= 74 or allow_partial or rows is not None:
                 return self.linear_skinny(a, w, bias, out_dtype=out_dtype, splits=1, mode=0, rows=rows)
-        out = torch.empty((T, N), dtype=out_dtype, device=a.device)
+        out = torch.empty(T, N, dtype=out_dtype, device=a.device)
         _check(self.lib.ifx_gemm_cublas_bf16(_ptr(a), _ptr(w), _ptr(out), T, N, K, _DT[out_dtype], _stream()),
                "gemm (bfloat16)")
         self.library_calls += 1
@@ -438,14 +443,14 @@ class CudaKernels:
         if (T and a.dtype == torch.bfloat16 and K % 8 == 0 and a.data_ptr() % 16 == 0 and w_gate_up.data_ptr() % 16 == 0):
             few = T <= self.SKINNY_MAX_ROWS
             if few or (self.swiglu_tiles and K <= self.SWIGLU_TILES_MAX_K):
-                out = torch.empty((T, inter), dtype=torch.bfloat16, device=a.device)
+                out = torch.empty(T, inter, dtype=torch.bfloat16, device=a.device)
                 product = self.lib.ifx_gemm_skinny_geglu if few else self.lib.ifx_gemm_tcgen05_geglu
                 _check(product(_ptr(a), _ptr(w_gate_up), _ptr(bias), _ptr(out), T, inter, K, _ptr(self.error_flag), _stream()),
                        "linear_geglu")
                 self.launches += 1
                 return out
         both = self.linear(a, w_gate_up)
-        out = torch.empty((T, inter), dtype=a.dtype, device=a.device)
+        out = torch.empty(T, inter, dtype=a.dtype, device=a.device)
         _check(self.lib.ifx_geglu_mul(_ptr(both), _ptr(bias), _ptr(out), T, inter, _DT[a.dtype], _stream()), "geglu_mul")
         self.launches += 1
         return out
@@ -459,7 +464,7 @@ class CudaKernels:
         if (a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and 0 < T <= self.SKINNY_MAX_ROWS and K % 8 == 0
                 and a.is_contiguous() and w.is_contiguous() and w.shape[1] == K and a.data_ptr() % 16 == 0
                 and w.data_ptr() % 16 == 0 and -(-N // 128) >= 74):
-            out = torch.empty((T, N), dtype=torch.bfloat16, device=a.device)
+            out = torch.empty(T, N, dtype=torch.bfloat16, device=a.device)
             _check(self.lib.ifx_gemm_skinny_act(_ptr(a), _ptr(w), _ptr(None), _ptr(out), T, N, K, w.shape[0], 0, _ptr(None), 0,
                                                 ctypes.c_float(0.0), 1, ctypes.c_float(a_pos), ctypes.c_float(a_neg),
                                                 _ptr(self.error_flag), _stream()), "gemm_skinny (xielu)")
@@ -476,12 +481,12 @@ class CudaKernels:
                 and w.shape[1] == K and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
             out = None
             if T <= self.SKINNY_MAX_ROWS and -(-N // 128) >= 74:
-                out = torch.empty((T, N), dtype=torch.bfloat16, device=a.device)
+                out = torch.empty(T, N, dtype=torch.bfloat16, device=a.device)
                 _check(self.lib.ifx_gemm_skinny_act(_ptr(a), _ptr(w), _ptr(None), _ptr(out), T, N, K, N, 0, _ptr(None), 0,
                                                     ctypes.c_float(0.0), 3, ctypes.c_float(0.0), ctypes.c_float(0.0),
                                                     _ptr(self.error_flag), _stream()), "gemm_skinny (relu2)")
             elif T > self.SKINNY_MAX_ROWS and self.swiglu_tiles and K <= self.SWIGLU_TILES_MAX_K:
-                out = torch.empty((T, N), dtype=torch.bfloat16, device=a.device)
+                out = torch.empty(T, N, dtype=torch.bfloat16, device=a.device)
                 _check(self.lib.ifx_gemm_tcgen05(_ptr(a), _ptr(w), _ptr(out), T, N, K, N, 6, 0, _ptr(self.error_flag), _stream()),
                        "gemm_tcgen05 (relu2)")
             if out is not None:
@@ -519,9 +524,9 @@ class CudaKernels:
         out_dtype = out_dtype or torch.bfloat16
         out = partials = None
         if mode == 1:
-            partials = torch.empty((splits, T, N), dtype=torch.float32, device=a.device)
+            partials = torch.empty(splits, T, N, dtype=torch.float32, device=a.device)
         else:
-            out = torch.empty((T, N), dtype=out_dtype, device=a.device)
+            out = torch.empty(T, N, dtype=out_dtype, device=a.device)
         _check(self.lib.ifx_gemm_skinny(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), _ptr(partials), T, N, K, w.shape[0],
                                         splits, mode, up_row_offset, int(out_dtype == torch.float32),
                                         _ptr(None if rows is None else rows.sumsq),
@@ -538,7 +543,7 @@ class CudaKernels:
         _need(a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16, "linear_tiles: bfloat16 only")
         _need(a.is_contiguous() and w.is_contiguous() and w.shape[1] == K and K % 8 == 0, "linear_tiles: bad operands")
         N = w.shape[0] // 2 if swiglu else w.shape[0]
-        out = torch.empty((T, N), dtype=torch.bfloat16, device=a.device)
+        out = torch.empty(T, N, dtype=torch.bfloat16, device=a.device)
         _check(self.lib.ifx_gemm_tcgen05(_ptr(a), _ptr(w), _ptr(out), T, N, K, w.shape[0], int(bool(swiglu)),
                                          N if swiglu else 0, _ptr(self.error_flag), _stream()), "gemm_tcgen05")
         self.launches += 1
@@ -549,7 +554,7 @@ class CudaKernels:
         T, K = a.shape
         N = w.shape[0]
         out_dtype = out_dtype or a.dtype
-        out = torch.empty((T, N), dtype=out_dtype, device=a.device)
+        out = torch.empty(T, N, dtype=out_dtype, device=a.device)
         _check(self.lib.ifx_gemm_generic(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), T, N, K, _DT[a.dtype],
                                          _DT[out_dtype], _stream()), "gemm_generic")
         self.launches += 1
@@ -755,11 +760,12 @@ class CudaKernels:
             dtype, device = qkv.dtype, qkv.device
             T, width = qkv.shape
         _need(width == (nq + 2 * nkv) * d, "rope_append: qkv width does not fit the head counts")
-        q_out = torch.empty((T, nq * d), dtype=dtype, device=device)
+        q_out = torch.empty(T, nq * d, dtype=dtype, device=device)
         write = bool(cache.writes and cache.kv is not None)
         kv, table = cache.kv, cache.block_table
         if write:
-            _need(kv.dtype == dtype, f"rope_append: cache is {kv.dtype}, activations {dtype}")
+            if kv.dtype != dtype:
+                raise KernelError(f"rope_append: cache is {kv.dtype}, activations {dtype}")
         rot = 0 if rotary is None else int(rotary.rotary_dim)
         _need(rot <= d, "rope_append: rotary_dim exceeds the head size")
         _check(self.lib.ifx_rope_append(
@@ -786,12 +792,13 @@ class CudaKernels:
         _need(width == (nq + src_kv) * d + src_kv * dv, "rope_append: the rows' width does not fit the head counts")
         for w in (q_norm, k_norm):
             _need(w is None or (w.dtype == torch.float32 and w.numel() == d), "rope_append: a head norm weight is float32 [d]")
-        q_out = torch.empty((T, nq * d), dtype=dtype, device=device)
+        q_out = torch.empty(T, nq * d, dtype=dtype, device=device)
         kv, table = cache.kv, cache.block_table
         write = bool(own_kv and cache.writes and kv is not None)
         d_row = d
         if write:
-            _need(kv.dtype == dtype, f"rope_append: cache is {kv.dtype}, activations {dtype}")
+            if kv.dtype != dtype:
+                raise KernelError(f"rope_append: cache is {kv.dtype}, activations {dtype}")
             d_row = kv.shape[-1]
             _need(kv.shape[1] == 2 and kv.shape[2] == nkv and d_row >= max(d, dv), "rope_append: the cache does not fit the heads")
         rot = 0 if rotary is None else int(rotary.rotary_dim)
@@ -827,10 +834,12 @@ class CudaKernels:
         T = q.shape[0]
         kv, table = cache.kv, cache.block_table
         _need(kv is not None and table is not None, "attention: the mixer has no key/value cache")
-        _need(kv.dtype == q.dtype, f"attention: cache is {kv.dtype}, queries {q.dtype}")
-        _need(d % 8 == 0 and d <= 256, f"attention: head size {d} is not a multiple of 8 up to 256")
+        if kv.dtype != q.dtype:
+            raise KernelError(f"attention: cache is {kv.dtype}, queries {q.dtype}")
+        if d % 8 or d > 256:
+            raise KernelError(f"attention: head size {d} is not a multiple of 8 up to 256")
         _need(q.is_contiguous() and q.shape[1] == nq * d, "attention: queries must be one [tokens, heads * size] block")
-        out = torch.empty((T, nq * d), dtype=q.dtype, device=q.device)
+        out = torch.empty(T, nq * d, dtype=q.dtype, device=q.device)
         win = 0 if window is None else int(window)
         common = (cache.page_size, table.shape[1], kv.shape[0], win, ctypes.c_float(scale))
         tiled = q.dtype == torch.bfloat16 and bool(self.lib.ifx_attention_mma_supports(d))
@@ -951,12 +960,13 @@ class CudaKernels:
         T = q.shape[0]
         kv, table = cache.kv, cache.block_table
         _need(kv is not None and table is not None, "attention: the mixer has no key/value cache")
-        _need(kv.dtype == q.dtype, f"attention: cache is {kv.dtype}, queries {q.dtype}")
+        if kv.dtype != q.dtype:
+            raise KernelError(f"attention: cache is {kv.dtype}, queries {q.dtype}")
         _need(q.is_contiguous() and q.shape[1] == nq * d, "attention: queries must be one [tokens, heads * size] block")
         d_row = kv.shape[-1]
         _need(kv.shape[1] == 2 and kv.shape[2] == nkv and d_row >= max(d, dv) and d_row % 8 == 0 and d_row <= 256,
               "attention: the cache does not fit the heads")
-        out = torch.empty((T, nq * dv), dtype=q.dtype, device=q.device)
+        out = torch.empty(T, nq * dv, dtype=q.dtype, device=q.device)
         win = 0 if window is None else int(window)
         sink_values = sink if torch.is_tensor(sink) else None
         if sink_values is not None:
@@ -1043,7 +1053,7 @@ class CudaKernels:
         _need(w_post.dtype == torch.float32 and (w_next is None or w_next.dtype == torch.float32),
               "postnorm_add: norm weights must be float32")
         T, H = x.shape
-        out = None if (w_next is None and not cast_out) else torch.empty((T, H), dtype=out_dtype or y.dtype, device=x.device)
+        out = None if (w_next is None and not cast_out) else torch.empty(T, H, dtype=out_dtype or y.dtype, device=x.device)
         cw, taps, st_ptr, stride, treq, rslot = None, 0, ctypes.c_void_p(0), 0, None, None
         if conv is not None:
             cw, taps, state, index, ctx = conv
@@ -1075,7 +1085,7 @@ class CudaKernels:
               "postnorm_add: a norm over groups needs both float32 norm weights")
         T, H = x.shape
         out_dtype = out_dtype or y.dtype
-        out = torch.empty((T, H), dtype=out_dtype, device=x.device)
+        out = torch.empty(T, H, dtype=out_dtype, device=x.device)
         out2, cw, taps, st_ptr, stride, treq, rslot = None, None, 0, ctypes.c_void_p(0), 0, None, None
         if conv is not None:
             cw, taps, state, index, ctx = conv
@@ -1088,7 +1098,7 @@ class CudaKernels:
                 stride = state.stride(0)
                 st_ptr = ctypes.c_void_p(state.data_ptr() + 4 * index * state.stride(1))
             treq, rslot = ctx.token_req, ctx.req_slot
-            out2 = torch.empty((T, H), dtype=out_dtype, device=x.device)
+            out2 = torch.empty(T, H, dtype=out_dtype, device=x.device)
         _check(self.lib.ifx_groupnorm_stream(
             _ptr(x), _ptr(y), _ptr(w_post), ctypes.c_float(eps_post), _ptr(w_next), ctypes.c_float(eps_next), int(groups),
             _ptr(out), _ptr(out2), T, H, _DT[y.dtype], _DT[out_dtype], splits, _ptr(cw), taps, st_ptr,
@@ -1114,7 +1124,7 @@ class CudaKernels:
             return v, _DT[v.dtype], 1
         pa, da, sa = operand(a)
         pb, db, sb = operand(b)
-        out = None if out_dtype is None else torch.empty((T, H), dtype=out_dtype, device=x.device)
+        out = None if out_dtype is None else torch.empty(T, H, dtype=out_dtype, device=x.device)
         _check(self.lib.ifx_residual_add_scaled(_ptr(x), _ptr(pa), da, sa, _ptr(pb), db, sb, ctypes.c_float(scale), _ptr(out),
                                                 0 if out is None else _DT[out_dtype], T, H, _stream()), "residual_add_scaled")
         self.launches += 1
@@ -1142,7 +1152,7 @@ class CudaKernels:
         T, ld = rows.shape
         _need(rows.is_contiguous() and w.dtype == torch.float32 and w.numel() == n and col0 + n <= ld,
               "rmsnorm_columns: the columns must lie inside contiguous rows")
-        out = torch.empty((T, n), dtype=rows.dtype, device=rows.device)
+        out = torch.empty(T, n, dtype=rows.dtype, device=rows.device)
         _check(self.lib.ifx_latent_norm_append(
             _ptr(rows), ld, int(col0), _ptr(w), ctypes.c_float(eps), _ptr(None), _ptr(None), _ptr(None), _ptr(None), 0, 0, 0,
             _ptr(None), _ptr(out), T, n, _DT[rows.dtype], _stream()), "rmsnorm_columns")
@@ -1154,7 +1164,7 @@ class CudaKernels:
         _need(a.dtype == torch.float32 and b.dtype == torch.float32 and a.shape == b.shape and a.is_contiguous()
               and b.is_contiguous(), "concat_cast: two float32 tensors of one shape")
         T, H = a.shape
-        out = torch.empty((T, 2 * H), dtype=dtype, device=a.device)
+        out = torch.empty(T, 2 * H, dtype=dtype, device=a.device)
         _check(self.lib.ifx_concat_cast(_ptr(a), _ptr(b), _ptr(out), T, H, _DT[dtype], _stream()), "concat_cast")
         self.launches += 1
         return out
@@ -1195,7 +1205,7 @@ class CudaKernels:
                   "short_conv: the state does not fit the convolution")
             stride = state.stride(0)                       # a slot's rows may be part of a longer state row
             st_ptr = ctypes.c_void_p(state.data_ptr() + 4 * index * state.stride(1))
-        out = torch.empty((T, C), dtype=h.dtype, device=h.device)
+        out = torch.empty(T, C, dtype=h.dtype, device=h.device)
         _check(self.lib.ifx_short_conv_ex(ctypes.c_void_p(h.data_ptr() + col0 * h.element_size()), ctypes.c_longlong(width),
                                           _ptr(w), _ptr(bias), st_ptr, ctypes.c_longlong(stride), _ptr(ctx.token_req),
                                           _ptr(ctx.req_slot), _ptr(ctx.cu_seqlens), _ptr(out), T, ctx.num_requests, C,
@@ -1232,7 +1242,7 @@ class CudaKernels:
               "linear_heads: shapes do not fit")
         so = n if out_head_stride is None else int(out_head_stride)
         if out is None:
-            out = torch.empty((T, heads * so), dtype=torch.bfloat16, device=a.device)
+            out = torch.empty(T, heads * so, dtype=torch.bfloat16, device=a.device)
         _need(out.dtype == torch.bfloat16 and out.is_contiguous() and out.shape[0] == T and so >= n
               and out.shape[1] >= (heads - 1) * so + n, "linear_heads: the output does not fit")
         ldw = k if w_is_nk else n
@@ -1264,7 +1274,7 @@ class CudaKernels:
         rows of queries in latent space, [T, heads (rank + rot)], whose other columns `latent_attention` fills.  With
         `gate_col` returns (that, sigmoid of the `heads` columns of `rows` from gate_col on as float32 [T, heads])."""
         T, ld = rows.shape
-        gate = None if gate_col is None else torch.empty((T, heads), dtype=torch.float32, device=rows.device)
+        gate = None if gate_col is None else torch.empty(T, heads, dtype=torch.float32, device=rows.device)
         kv, table = cache.kv, cache.block_table
         _need(kv is not None and table is not None and kv.dtype == rows.dtype and q.dtype == rows.dtype,
               "latent_rope_append: no cache of the run's dtype")
@@ -1281,7 +1291,7 @@ class CudaKernels:
         dst, ld_dst, head_stride, offset, result = q, q.shape[1], dim + rot, dim, q
         if (rot and vdim is not None and self.latent_tiles and rows.dtype == torch.bfloat16 and dim % 8 == 0 and vdim % 8 == 0
                 and q.shape[1] % 8 == 0 and self.lib.ifx_latent_attention_mma_supports_rot(rank, rot)):
-            dst = torch.empty((T, heads * (rank + rot)), dtype=torch.bfloat16, device=rows.device)
+            dst = torch.empty(T, heads * (rank + rot), dtype=torch.bfloat16, device=rows.device)
             ld_dst, head_stride, offset, result = heads * (rank + rot), rank + rot, rank, TurnedQueries(q, dst)
         _check(self.lib.ifx_latent_rope_append(
             _ptr(rows), ld, int(col0), _ptr(w), ctypes.c_float(eps), _ptr(q), q.shape[1], _ptr(dst), ld_dst, head_stride, offset,
@@ -1315,7 +1325,7 @@ class CudaKernels:
         tiled = (self.latent_tiles and not rot and q_rows.dtype == torch.bfloat16 and dim % 8 == 0 and vdim % 8 == 0
                  and ldq % 8 == 0 and self.lib.ifx_latent_attention_mma_supports(rank))
         if rot or (head_gate is not None and not tiled):
-            out = torch.empty((T, heads * vdim), dtype=q_rows.dtype, device=q_rows.device)
+            out = torch.empty(T, heads * vdim, dtype=q_rows.dtype, device=q_rows.device)
             _check(self.lib.ifx_latent_attention_generic_rot(
                 _ptr(q_rows), ldq, _ptr(w_uk), _ptr(w_uv), _ptr(sinks), _ptr(kv), _ptr(table), _ptr(ctx.positions),
                 _ptr(ctx.token_req), _ptr(ctx.req_slot), _ptr(None), _ptr(out), T, heads, dim, vdim, rank, cache.page_size,
@@ -1326,7 +1336,7 @@ class CudaKernels:
         if tiled:
             return self._latent_attention_tiles(q_rows, w_uk, w_uv, sinks, heads, dim, vdim, rank, window, scale, ctx, cache,
                                                 head_gate=head_gate)
-        out = torch.empty((T, heads * vdim), dtype=q_rows.dtype, device=q_rows.device)
+        out = torch.empty(T, heads * vdim, dtype=q_rows.dtype, device=q_rows.device)
         _check(self.lib.ifx_latent_attention_generic(
             _ptr(q_rows), ldq, _ptr(w_uk), _ptr(w_uv), _ptr(sinks), _ptr(kv), _ptr(table), _ptr(ctx.positions),
             _ptr(ctx.token_req), _ptr(ctx.req_slot), _ptr(None), _ptr(out), T, heads, dim, vdim, rank, cache.page_size,
@@ -1388,7 +1398,7 @@ class CudaKernels:
         if splits > 1:
             ws = torch.empty(int(self.lib.ifx_latent_attention_mma_workspace(T * heads, rank, splits)), dtype=torch.uint8,
                              device=q_rows.device)
-        olat = torch.empty((T, heads * rank), dtype=torch.bfloat16, device=q_rows.device)
+        olat = torch.empty(T, heads * rank, dtype=torch.bfloat16, device=q_rows.device)
         if decode:
             _check(self.lib.ifx_latent_decode(
                 _ptr(ql), _ptr(kv), _ptr(table), _ptr(items), num_items, _ptr(sinks), _ptr(olat), _ptr(ws), T, heads, rank, int(rot),
@@ -1434,7 +1444,7 @@ class CudaKernels:
               and mu.shape[1] == C, "token_shift_mix: float32 rows and weights of one width")
         _need(state is not None and state.dtype == torch.float32 and state.is_contiguous() and state.dim() == 2
               and prev_offset + C <= state.shape[1], "token_shift_mix: the state does not hold a row")
-        out = torch.empty((mu.shape[0], T, C), dtype=out_dtype, device=x.device)
+        out = torch.empty(mu.shape[0], T, C, dtype=out_dtype, device=x.device)
         _check(self.lib.ifx_token_shift_mix(
             _ptr(x), _ptr(mu), ctypes.c_void_p(state.data_ptr() + 4 * prev_offset), ctypes.c_longlong(state.shape[1]),
             _ptr(ctx.token_req), _ptr(ctx.req_slot), _ptr(ctx.cu_seqlens), _ptr(out), T, C, mu.shape[0], _DT[out_dtype],
@@ -1500,8 +1510,8 @@ class CudaKernels:
         _need(HD == heads * dim and prev_offset == heads * dim * dim and state.dtype == torch.float32 and state.is_contiguous()
               and state.dim() == 2 and state.shape[1] == prev_offset + C and x.dtype == torch.float32 and x.is_contiguous(),
               "wkv_scan: the state does not fit the sizes")
-        scratch = torch.empty((T, HD), dtype=torch.float32, device=r.device)
-        y = torch.empty((T, HD), dtype=out_dtype, device=r.device)
+        scratch = torch.empty(T, HD, dtype=torch.float32, device=r.device)
+        y = torch.empty(T, HD, dtype=out_dtype, device=r.device)
         if self._scans_by_chunks(out_dtype, ctx, heads, dim, dim, r, k, v, w_raw, w0, u):
             least, short = self._parting(ctx)
             if short:
@@ -1567,7 +1577,7 @@ class CudaKernels:
             _need(t.dtype == torch.float32 and t.is_contiguous() and t.numel() == HD, "delta_rule_scan: float32 constants of heads * dim")
         _need(state is not None and state.dtype == torch.float32 and state.dim() == 2 and state.stride(1) == 1
               and state.shape[1] >= HD * dim, "delta_rule_scan: the state does not fit the sizes")
-        y = torch.empty((T, HD), dtype=out_dtype, device=proj.device)
+        y = torch.empty(T, HD, dtype=out_dtype, device=proj.device)
         if (self._delta_by_chunks(out_dtype, ctx, T, heads, dim) and proj.shape[1] % 4 == 0
                 and all(t.data_ptr() % 16 == 0 for t in (proj, w_raw, w0, a_bias))):
             least, short = self._parting(ctx)
@@ -1602,8 +1612,8 @@ class CudaKernels:
         T, n = z.shape
         _need(z.dtype == torch.float32 and z.is_contiguous() and (correction is None or (correction.dtype == torch.float32
               and correction.numel() == n)), "moe_route: float32 logits and corrections")
-        ids = torch.empty((T, top), dtype=torch.int32, device=z.device)
-        weights = torch.empty((T, top), dtype=torch.float32, device=z.device)
+        ids = torch.empty(T, top, dtype=torch.int32, device=z.device)
+        weights = torch.empty(T, top, dtype=torch.float32, device=z.device)
         _check(self.lib.ifx_moe_route_kind(_ptr(z), _ptr(correction), _ptr(ids), _ptr(weights), T, n, int(top),
                                            2 if kind == "sigmoid_normalized" else int(bool(of_chosen)), ctypes.c_float(floor),
                                            _stream()), "moe_route")
@@ -1631,8 +1641,8 @@ class CudaKernels:
                 if way != "tokens" and self._moe_on_tensor_cores(h, w_up, w_down, ff, width):
                     return (self._moe_experts_tiles if way == "tiles" else self._moe_experts_stream)(
                         h, w_up, w_down, ids, weights, experts, out_dtype, glu=glu)
-            act = torch.empty((T * top, ff), dtype=h.dtype, device=h.device)
-            out = torch.empty((T, width), dtype=out_dtype, device=h.device)
+            act = torch.empty(T * top, ff, dtype=h.dtype, device=h.device)
+            out = torch.empty(T, width, dtype=out_dtype, device=h.device)
             _check(self.lib.ifx_moe_experts_glu(_ptr(h), _ptr(w_up), _ptr(w_down), _ptr(ids), _ptr(weights), _ptr(act), _ptr(out),
                                                 T, top, int(experts), width, ff, _DT[h.dtype], _DT[out_dtype], 1,
                                                 ctypes.c_float(glu[0]), ctypes.c_float(glu[1]), ctypes.c_float(glu[2]),
@@ -1648,8 +1658,8 @@ class CudaKernels:
             if way != "tokens" and self._moe_on_tensor_cores(h, w_up, w_down, ff, width):
                 return (self._moe_experts_tiles if way == "tiles" else self._moe_experts_stream)(
                     h, w_up, w_down, ids, weights, experts, out_dtype)
-        act = torch.empty((T * top, ff), dtype=h.dtype, device=h.device)
-        out = torch.empty((T, width), dtype=out_dtype, device=h.device)
+        act = torch.empty(T * top, ff, dtype=h.dtype, device=h.device)
+        out = torch.empty(T, width, dtype=out_dtype, device=h.device)
         _check(self.lib.ifx_moe_experts(_ptr(h), _ptr(w_up if experts else None), _ptr(w_down if experts else None), _ptr(ids),
                                         _ptr(weights), _ptr(act), _ptr(out), T, top, int(experts), width, ff, _DT[h.dtype],
                                         _DT[out_dtype], _stream()), "moe_experts")
@@ -1700,10 +1710,10 @@ class CudaKernels:
         """bfloat16, few tokens: every chosen expert's weights once through the tensor cores (csrc/moe_stream_tcgen05.cu)."""
         T, width = h.shape
         top, ff = ids.shape[1], w_up.shape[1] // (2 if glu is not None else 1)
-        act = torch.empty((T * top, ff), dtype=torch.bfloat16, device=h.device)
+        act = torch.empty(T * top, ff, dtype=torch.bfloat16, device=h.device)
         slices = int(self.lib.ifx_moe_stream_slices(ff))
-        y = torch.empty((slices, T * top, width), dtype=torch.float32, device=h.device)
-        out = torch.empty((T, width), dtype=out_dtype, device=h.device)
+        y = torch.empty(slices, T * top, width, dtype=torch.float32, device=h.device)
+        out = torch.empty(T, width, dtype=out_dtype, device=h.device)
         limit, slope, offset = glu if glu is not None else (0.0, 0.0, 0.0)
         _check(self.lib.ifx_moe_stream(_ptr(h), _ptr(w_up), _ptr(w_down), _ptr(ids), _ptr(weights), _ptr(act), _ptr(y), _ptr(out),
                                        T, top, int(experts), width, ff, _DT[out_dtype], int(glu is not None), ctypes.c_float(limit),
@@ -1727,9 +1737,9 @@ class CudaKernels:
         pair_row = torch.empty(pairs, dtype=torch.int32, device=dev)
         _check(self.lib.ifx_moe_sort(_ptr(ids), _ptr(weights), pairs, int(experts), _ptr(row_pair), _ptr(row_scale),
                                      _ptr(tile_group), _ptr(pair_row), cap, _stream()), "moe_sort")
-        rows = torch.empty((cap, width), dtype=torch.bfloat16, device=dev)
+        rows = torch.empty(cap, width, dtype=torch.bfloat16, device=dev)
         _check(self.lib.ifx_moe_gather(_ptr(h), _ptr(row_pair), _ptr(rows), cap, top, width, _stream()), "moe_gather")
-        act = torch.empty((cap, ff), dtype=torch.bfloat16, device=dev)
+        act = torch.empty(cap, ff, dtype=torch.bfloat16, device=dev)
         if glu is not None:
             _check(self.lib.ifx_gemm_tcgen05_grouped_glu_offset(
                 _ptr(rows), _ptr(w_up), _ptr(act), cap, ff, width, int(experts), _ptr(tile_group), ctypes.c_float(glu[0]),
@@ -1739,11 +1749,11 @@ class CudaKernels:
             _check(self.lib.ifx_gemm_tcgen05_grouped(_ptr(rows), _ptr(w_up), _ptr(act), cap, ff, width, int(experts), ff,
                                                      _ptr(tile_group), _ptr(None), 2, _ptr(self.error_flag), _stream()),
                    "moe experts (up, tiles)")
-        y = torch.empty((cap, width), dtype=torch.float32, device=dev)
+        y = torch.empty(cap, width, dtype=torch.float32, device=dev)
         _check(self.lib.ifx_gemm_tcgen05_grouped(_ptr(act), _ptr(w_down), _ptr(y), cap, width, ff, int(experts), width,
                                                  _ptr(tile_group), _ptr(row_scale), 3, _ptr(self.error_flag), _stream()),
                "moe experts (down, tiles)")
-        out = torch.empty((T, width), dtype=out_dtype, device=dev)
+        out = torch.empty(T, width, dtype=out_dtype, device=dev)
         _check(self.lib.ifx_moe_combine(_ptr(h), _ptr(y), _ptr(ids), _ptr(weights), _ptr(pair_row), _ptr(out), T, top,
                                         int(experts), width, _DT[out_dtype], _stream()), "moe_combine")
         self.launches += 5
@@ -1779,8 +1789,8 @@ class CudaKernels:
                   and (vb2 is None or (vb is not None and vb2.is_contiguous())), "rmsnorm_pair: the sum's rows do not fit")
         _need(x.dtype == torch.float32 and x.is_contiguous() and w_a.numel() == H and w_b.numel() == H
               and w_a.dtype == torch.float32 and w_b.dtype == torch.float32, "rmsnorm_pair: bad operands")
-        out_a = torch.empty((T, H), dtype=out_dtype, device=x.device)
-        out_b = torch.empty((T, H), dtype=out_dtype, device=x.device)
+        out_a = torch.empty(T, H, dtype=out_dtype, device=x.device)
+        out_b = torch.empty(T, H, dtype=out_dtype, device=x.device)
         _check(self.lib.ifx_rmsnorm_pair(_ptr(x), _ptr(w_a), ctypes.c_float(eps_a), _ptr(w_b), ctypes.c_float(eps_b), _ptr(out_a),
                                          _ptr(out_b), T, H, _DT[out_dtype], _ptr(va), _DT[va.dtype] if va is not None else 0,
                                          _ptr(vsa), _ptr(vb), _ptr(vb2), _DT[vb.dtype] if vb is not None else 0, _ptr(vsb),
@@ -1800,7 +1810,8 @@ class CudaKernels:
 
     @staticmethod
     def _rows_f32(t, what):
-        _need(t.dtype == torch.float32 and t.dim() == 2 and t.stride(1) == 1, f"{what}: float32 rows with unit column stride")
+        if t.dtype != torch.float32 or t.dim() != 2 or t.stride(1) != 1:
+            raise KernelError(f"{what}: float32 rows with unit column stride")
         return ctypes.c_void_p(t.data_ptr()), ctypes.c_longlong(t.stride(0))
 
     def decay_scan(self, q, k, v, raw, state, ctx, heads, groups, dk, dv, decay, tau=1.0, q_scale=1.0, step_bias=None,
@@ -1814,9 +1825,9 @@ class CudaKernels:
         head, k is multiplied by dt, and skip[h] v_t is added to o_t.
         decay `constant`: raw None, w = rate[h] whatever the token."""
         T = q.shape[0]
-        modes = {"sigmoid_root": 0, "softplus_step": 1, "constant": 2}
-        _need(decay in modes, f"decay_scan: unknown decay {decay!r}")
-        mode = modes[decay]
+        mode = _DECAYS.get(decay)
+        if mode is None:
+            raise KernelError(f"decay_scan: unknown decay {decay!r}")
         _need((raw is None) == (mode == 2) == (rate is not None), "decay_scan: a constant decay comes from `rate`, any other from `raw`")
         _need(q.shape[1] == groups * dk and k.shape[1] == groups * dk and v.shape[1] == heads * dv
               and k.shape[0] == T and v.shape[0] == T
@@ -1827,7 +1838,7 @@ class CudaKernels:
         for vec in (step_bias, log_rate, skip, rate):
             _need(vec is None or (vec.dtype == torch.float32 and vec.numel() == heads and vec.is_contiguous()),
                   "decay_scan: per-head vectors are float32 [heads]")
-        out = torch.empty((T, heads * dv), dtype=torch.float32, device=q.device)
+        out = torch.empty(T, heads * dv, dtype=torch.float32, device=q.device)
         if self._scans_by_chunks(getattr(ctx, "dtype", None), ctx, heads, dk, dv, q, k, v, *([raw] if mode == 0 else []), constant=mode == 2):
             least, short = self._parting(ctx)
             room = torch.empty(int(self.lib.ifx_chunk_scan_scratch_floats(T, ctx.num_requests, least, heads, dk, dv, int(mode == 0))),
@@ -1865,7 +1876,7 @@ class CudaKernels:
         _need(y.dtype == torch.float32 and y.is_contiguous() and tuple(gate.shape) == (T, C) and C % groups == 0
               and (w is None or (w.dtype == torch.float32 and w.is_contiguous() and w.numel() in (C, C // groups)))
               and kind in ("silu", "sigmoid"), "gated_groupnorm: bad operands")
-        out = torch.empty((T, C), dtype=out_dtype, device=y.device)
+        out = torch.empty(T, C, dtype=out_dtype, device=y.device)
         gp, gs = self._rows_f32(gate, "gated_groupnorm gate")
         _check(self.lib.ifx_gated_groupnorm(_ptr(y), gp, gs, _ptr(w), 0 if w is None else int(w.numel()), ctypes.c_float(eps), _ptr(out), T, C,
                                             int(groups), int(bool(gate_first)), int(kind == "sigmoid"), _DT[out_dtype], _stream()),
@@ -1878,7 +1889,7 @@ class CudaKernels:
         T, C = a.shape
         _need(a.is_contiguous() and b.is_contiguous() and a.shape == b.shape and (w_a is None) == (w_b is None),
               "pair_combine: rows of one shape")
-        out = torch.empty((T, C), dtype=torch.float32, device=a.device)
+        out = torch.empty(T, C, dtype=torch.float32, device=a.device)
         _check(self.lib.ifx_pair_combine(_ptr(a), _DT[a.dtype], _ptr(b), _DT[b.dtype], _ptr(w_a), _ptr(w_b), ctypes.c_float(c_a),
                                          ctypes.c_float(c_b), ctypes.c_float(eps), _ptr(out), T, C, _stream()), "pair_combine")
         self.launches += 1
@@ -1918,7 +1929,7 @@ class CudaKernels:
                   and (bias is None or (bias.dtype == torch.float32 and bias.numel() == H and bias.is_contiguous())),
                   "norm_of_sum: a term does not match x")
             flat += [_ptr(y), 0 if y is None else _DT[y.dtype], splits, ctypes.c_float(c), _ptr(bias)]
-        out = None if out_dtype is None else torch.empty((T, H), dtype=out_dtype, device=x.device)
+        out = None if out_dtype is None else torch.empty(T, H, dtype=out_dtype, device=x.device)
         _check(self.lib.ifx_norm_of_sum(_ptr(x), ctypes.c_float(alpha), *flat, _ptr(w), ctypes.c_float(eps), _ptr(out),
                                         0 if out is None else _DT[out_dtype], T, H, _stream()), "norm_of_sum")
         self.launches += 1
@@ -1958,9 +1969,9 @@ class CudaKernels:
         _need(turn is None or turn.rotary_dim == dv, "row_norm_rope_append: values are turned as a whole")
         src, code, part, splits, ld = self._row_source(rows)
         dev = kv.device
-        q_out = torch.empty((T, nq * d), dtype=kv.dtype, device=dev)
-        back = None if turn is None else torch.empty((T, dv // 2, 2), dtype=torch.float32, device=dev)
-        gate = None if gate_col is None else torch.empty((T, nq), dtype=torch.float32, device=dev)
+        q_out = torch.empty(T, nq * d, dtype=kv.dtype, device=dev)
+        back = None if turn is None else torch.empty(T, dv // 2, 2, dtype=torch.float32, device=dev)
+        gate = None if gate_col is None else torch.empty(T, nq, dtype=torch.float32, device=dev)
         _check(self.lib.ifx_row_norm_rope_append(
             src, code, part, splits, _LL(ld), int(col0), _ptr(bias), _ptr(q_norm), _ptr(k_norm), ctypes.c_float(norm_eps),
             _ptr(None if rotary is None else rotary.inv_freq), 0 if rotary is None else int(rotary.rotary_dim),
@@ -1980,7 +1991,7 @@ class CudaKernels:
         src, code, part, splits, ld = self._row_source(rows)
         plain = not isinstance(rows, PartialSum)
         _need(not plain or rows.dtype == torch.float32, "silu_columns: float32 rows")
-        out = rows if plain else torch.empty((T, ld), dtype=torch.float32, device=rows.parts.device)
+        out = rows if plain else torch.empty(T, ld, dtype=torch.float32, device=rows.parts.device)
         _check(self.lib.ifx_silu_columns(src, part, splits, _LL(ld), 0, _ptr(out), T, int(ld), int(acted), _stream()), "silu_columns")
         self.launches += 1
         return out
@@ -1995,7 +2006,7 @@ class CudaKernels:
         _need(not plain or rows.dtype == torch.float32, "rotate_rows: float32 rows")
         _need(rotary is None or (rotary.magnitude == 1.0 and rotary.rotary_dim <= dk), "rotate_rows: the table does not fit")
         device = rows.device if plain else rows.parts.device
-        out = rows if plain and ld == width and col0 == 0 else torch.empty((T, width), dtype=torch.float32, device=device)
+        out = rows if plain and ld == width and col0 == 0 else torch.empty(T, width, dtype=torch.float32, device=device)
         _check(self.lib.ifx_rotate_rows(
             src, part, splits, _LL(ld), int(col0), _ptr(None if rotary is None else rotary.inv_freq),
             0 if rotary is None else int(rotary.rotary_dim), int(rotary is not None and rotary.interleaved), _ptr(ctx.positions),
@@ -2013,7 +2024,7 @@ class CudaKernels:
               "gated_scan: bad operands")
         src, splits = (rows.parts, rows.splits) if isinstance(rows, PartialSum) else (rows, 1)
         _need(src.dtype == torch.float32 and src.is_contiguous(), "gated_scan: float32 rows")
-        out = torch.empty((T, width), dtype=out_dtype, device=src.device)
+        out = torch.empty(T, width, dtype=out_dtype, device=src.device)
         _check(self.lib.ifx_gated_scan(_ptr(src), splits, _ptr(bias), _ptr(state), _LL(state.stride(0)), _ptr(ctx.req_slot),
                                        _ptr(ctx.cu_seqlens), _ptr(out), ctx.num_requests, T, int(ctx.max_span), int(width),
                                        _DT[out_dtype], _stream()), "gated_scan")
@@ -2023,7 +2034,7 @@ class CudaKernels:
     # ---------------------------------------------------------------- sampling
     def argmax(self, logits):
         R, V = logits.shape
-        out = torch.empty((R,), dtype=torch.int32, device=logits.device)
+        out = torch.empty(R, dtype=torch.int32, device=logits.device)
         if V >= 16384 and R <= 256:                      # long rows, few of them: many blocks per row
             _check(self.lib.ifx_argmax_chunks(_ptr(logits), _ptr(out), R, V, 32, _ptr(self._argmax_val),
                                               _ptr(self._argmax_idx), _ptr(self._argmax_tickets), _stream()), "argmax")
@@ -2049,7 +2060,7 @@ class CudaKernels:
         """One draw per row (see sampling.cu).  Rows are spread over many blocks; `features` says which
         filters any row uses (bit 0: top-k, bit 1: top-p) so that the passes of the others are not launched."""
         R, V = logits.shape
-        out = torch.empty((R,), dtype=torch.int32, device=logits.device)
+        out = torch.empty(R, dtype=torch.int32, device=logits.device)
         if R > self._sample_capacity:                    # the scratch's layout goes with its capacity
             self._sample_capacity = max(64, 1 << (R - 1).bit_length())
             self._sample_scratch = torch.zeros(int(self.lib.ifx_sample_scratch_bytes(self._sample_capacity)),
@@ -2064,8 +2075,8 @@ class CudaKernels:
     def sample_one_block(self, logits, temperature, top_k, top_p, min_p, seed_lo, seed_hi, step):
         """The same draw with one block per row and thresholds by bisection (kept for comparison)."""
         R, V = logits.shape
-        probs = torch.empty((R, V), dtype=torch.float32, device=logits.device)
-        out = torch.empty((R,), dtype=torch.int32, device=logits.device)
+        probs = torch.empty(R, V, dtype=torch.float32, device=logits.device)
+        out = torch.empty(R, dtype=torch.int32, device=logits.device)
         _check(self.lib.ifx_sample(_ptr(logits), _ptr(probs), _ptr(temperature), _ptr(top_k), _ptr(top_p),
                                    _ptr(min_p), _ptr(seed_lo), _ptr(seed_hi), _ptr(step), _ptr(out), R, V,
                                    _stream()), "sample")
