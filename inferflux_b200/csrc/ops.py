@@ -19,6 +19,7 @@ import torch
 from .build import BuildError, load_library
 
 _DT = {torch.float32: 0, torch.bfloat16: 1}
+_MISALIGNED = -3             # what the kernels of long spans say of rows off a 16-byte boundary, before they touch anything
 _DECAYS = {"sigmoid_root": 0, "softplus_step": 1, "constant": 2}
 
 _ERRORS = {-1: "a size or option the kernel does not take", -2: "unknown dtype",
@@ -1469,13 +1470,15 @@ class CudaKernels:
 
     def _scans_by_chunks(self, dtype, ctx, heads, dk, dv, *rows, constant=False):
         """Whether a recurrence's long spans go by stretches of tokens: where that pays, with sizes the kernels are made for, rows
-        on 16-byte boundaries, and in a bfloat16 run (the order of the sums then depends on how a span was cut into steps)."""
+        on 16-byte boundaries (those given here; the kernels look at theirs themselves), and in a bfloat16 run (the order of the sums
+        then depends on how a span was cut into steps)."""
         if not (self.chunk_scans and dtype is torch.bfloat16 and ctx.max_span >= self.CHUNK_SCAN_MIN_SPAN):
             return False
+        if dk not in (64, 128) or dv % 64 or ctx.num_requests > 64:              # ifx_chunk_scan_supports, without a call
+            return False
         spans = self._long_spans(ctx)
-        return bool((spans is None or self.stretches_pay(ctx.max_span, spans[0], spans[3], constant and dk == 64))
-                    and self.lib.ifx_chunk_scan_supports(ctx.num_requests, int(heads), int(dk), int(dv))
-                    and all(t.data_ptr() % 16 == 0 and (t.dim() < 2 or t.stride(0) % 4 == 0) for t in rows))
+        return ((spans is None or self.stretches_pay(ctx.max_span, spans[0], spans[3], constant and dk == 64))
+                and all(t.data_ptr() % 16 == 0 and (t.dim() < 2 or t.stride(0) % 4 == 0) for t in rows))
 
     @staticmethod
     def stretches_pay(longest, short, stretches, cheap):
@@ -1510,32 +1513,32 @@ class CudaKernels:
         _need(HD == heads * dim and prev_offset == heads * dim * dim and state.dtype == torch.float32 and state.is_contiguous()
               and state.dim() == 2 and state.shape[1] == prev_offset + C and x.dtype == torch.float32 and x.is_contiguous(),
               "wkv_scan: the state does not fit the sizes")
-        scratch = torch.empty(T, HD, dtype=torch.float32, device=r.device)
-        y = torch.empty(T, HD, dtype=out_dtype, device=r.device)
-        if self._scans_by_chunks(out_dtype, ctx, heads, dim, dim, r, k, v, w_raw, w0, u):
+        by_chunks, size = self._scans_by_chunks(out_dtype, ctx, heads, dim, dim), T * HD
+        if by_chunks:
             least, short = self._parting(ctx)
-            if short:
-                _check(self.lib.ifx_wkv_scan(
-                    _ptr(r), _ptr(k), _ptr(v), _ptr(w_raw), _ptr(g), _ptr(w0), _ptr(u), _ptr(norm_w), ctypes.c_float(eps),
-                    _ptr(state), ctypes.c_void_p(state.data_ptr() + 4 * prev_offset), ctypes.c_longlong(state.shape[1]), _ptr(x), C,
-                    _ptr(ctx.cu_seqlens), _ptr(ctx.req_slot), _ptr(scratch), _ptr(y), ctx.num_requests, T, heads, dim, ld, ld_w,
-                    _DT[out_dtype], short, _stream()), "wkv_scan (short spans)")
-                self.launches += 1
-            room = torch.empty(int(self.lib.ifx_chunk_scan_scratch_floats(T, ctx.num_requests, least, heads, dim, dim, 1)),
-                               dtype=torch.float32, device=r.device)
-            _check(self.lib.ifx_chunk_wkv_scan(
-                _ptr(r), _ptr(k), _ptr(v), _ptr(w_raw), _ptr(w0), _ptr(u), _ptr(state), ctypes.c_void_p(state.data_ptr() + 4 * prev_offset),
-                ctypes.c_longlong(state.shape[1]), _ptr(x), C, _ptr(ctx.cu_seqlens), _ptr(ctx.req_slot), _ptr(scratch),
-                ctx.num_requests, T, least, heads, dim, ld, ld_w, _ptr(room), _stream()), "wkv_scan (stretches)")
-            _check(self.lib.ifx_wkv_norm(_ptr(scratch), _ptr(g), _ptr(norm_w), ctypes.c_float(eps), _ptr(y), T, heads, dim, ld,
-                                         _DT[out_dtype], _stream()), "wkv_norm")
-            self.launches += 4
-            return y
-        _check(self.lib.ifx_wkv_scan(
-            _ptr(r), _ptr(k), _ptr(v), _ptr(w_raw), _ptr(g), _ptr(w0), _ptr(u), _ptr(norm_w), ctypes.c_float(eps),
-            _ptr(state), ctypes.c_void_p(state.data_ptr() + 4 * prev_offset), ctypes.c_longlong(state.shape[1]), _ptr(x), C,
-            _ptr(ctx.cu_seqlens), _ptr(ctx.req_slot), _ptr(scratch), _ptr(y), ctx.num_requests, T, heads, dim, ld, ld_w, _DT[out_dtype],
-            0, _stream()), "wkv_scan")
+            size += int(self.lib.ifx_chunk_scan_scratch_floats(T, ctx.num_requests, least, heads, dim, dim, 1))
+        scratch = torch.empty(size, dtype=torch.float32, device=r.device)         # the sums, and what the stretches need
+        y = torch.empty(T, HD, dtype=out_dtype, device=r.device)
+        common = (_ptr(state), ctypes.c_void_p(state.data_ptr() + 4 * prev_offset), _LL(state.shape[1]), _ptr(x), C, _ptr(ctx.cu_seqlens),
+                  _ptr(ctx.req_slot), _ptr(scratch))
+        rows = (_ptr(r), _ptr(k), _ptr(v), _ptr(w_raw))
+        if by_chunks:
+            room = ctypes.c_void_p(scratch.data_ptr() + 4 * T * HD)               # (heads of 64 or 128: still on 16 bytes)
+            rc = self.lib.ifx_chunk_wkv_scan(*rows, _ptr(w0), _ptr(u), *common, ctx.num_requests, T, least, heads, dim, ld, ld_w, room,
+                                             _stream())
+            if rc != _MISALIGNED:
+                _check(rc, "wkv_scan (stretches)")
+                if short:
+                    _check(self.lib.ifx_wkv_scan(*rows, _ptr(g), _ptr(w0), _ptr(u), _ptr(norm_w), ctypes.c_float(eps), *common, _ptr(y),
+                                                 ctx.num_requests, T, heads, dim, ld, ld_w, _DT[out_dtype], short, _stream()),
+                           "wkv_scan (short spans)")
+                    self.launches += 1
+                _check(self.lib.ifx_wkv_norm(_ptr(scratch), _ptr(g), _ptr(norm_w), ctypes.c_float(eps), _ptr(y), T, heads, dim, ld,
+                                             _DT[out_dtype], _stream()), "wkv_norm")
+                self.launches += 4
+                return y
+        _check(self.lib.ifx_wkv_scan(*rows, _ptr(g), _ptr(w0), _ptr(u), _ptr(norm_w), ctypes.c_float(eps), *common, _ptr(y), ctx.num_requests,
+                                     T, heads, dim, ld, ld_w, _DT[out_dtype], 0, _stream()), "wkv_scan")
         self.launches += 1
         return y
 
@@ -1545,7 +1548,7 @@ class CudaKernels:
             return False
         spans = self._long_spans(ctx)
         pays = tokens <= 8 * ctx.max_span if spans is None else self.delta_stretches_pay(heads, tokens, ctx.num_requests, ctx.max_span, *spans)
-        return bool(pays and self.lib.ifx_delta_chunks_supports(ctx.num_requests, heads, dim))
+        return pays and dim == 64 and ctx.num_requests <= 64                     # ifx_delta_chunks_supports, without a call
 
     @staticmethod
     def delta_stretches_pay(heads, tokens, requests, longest, short, short_tokens, short_requests, stretches):
@@ -1578,21 +1581,21 @@ class CudaKernels:
         _need(state is not None and state.dtype == torch.float32 and state.dim() == 2 and state.stride(1) == 1
               and state.shape[1] >= HD * dim, "delta_rule_scan: the state does not fit the sizes")
         y = torch.empty(T, HD, dtype=out_dtype, device=proj.device)
-        if (self._delta_by_chunks(out_dtype, ctx, T, heads, dim) and proj.shape[1] % 4 == 0
-                and all(t.data_ptr() % 16 == 0 for t in (proj, w_raw, w0, a_bias))):
+        if self._delta_by_chunks(out_dtype, ctx, T, heads, dim):
             least, short = self._parting(ctx)
             room = torch.empty(int(self.lib.ifx_delta_chunks_scratch_floats(T, ctx.num_requests, least, heads)), dtype=torch.float32,
                                device=proj.device)
             scan_room = None
             if short:
                 scan_room = torch.empty(int(self.lib.ifx_delta_rule_scratch_floats(T, heads, dim)), dtype=torch.float32, device=proj.device)
-                self.launches += 2
-            _check(self.lib.ifx_delta_chunks_scan(
+            rc = self.lib.ifx_delta_chunks_scan(
                 _ptr(proj), proj.shape[1], _ptr(w_raw), _ptr(w0), _ptr(a_bias), _ptr(norm_w), ctypes.c_float(eps), _ptr(state),
                 ctypes.c_longlong(state.stride(0)), _ptr(ctx.cu_seqlens), _ptr(ctx.req_slot), _ptr(room), _ptr(y), ctx.num_requests, T,
-                least, heads, dim, _DT[out_dtype], _ptr(scan_room), _stream()), "delta_rule_scan (stretches)")
-            self.launches += 4
-            return y
+                least, heads, dim, _DT[out_dtype], _ptr(scan_room), _stream())
+            if rc != _MISALIGNED:
+                _check(rc, "delta_rule_scan (stretches)")
+                self.launches += 6 if short else 4
+                return y
         scratch = torch.empty(int(self.lib.ifx_delta_rule_scratch_floats(T, heads, dim)), dtype=torch.float32, device=proj.device)
         _check(self.lib.ifx_delta_rule_scan(
             _ptr(proj), proj.shape[1], _ptr(w_raw), _ptr(w0), _ptr(a_bias), _ptr(norm_w), ctypes.c_float(eps), _ptr(state),
@@ -1839,32 +1842,28 @@ class CudaKernels:
             _need(vec is None or (vec.dtype == torch.float32 and vec.numel() == heads and vec.is_contiguous()),
                   "decay_scan: per-head vectors are float32 [heads]")
         out = torch.empty(T, heads * dv, dtype=torch.float32, device=q.device)
-        if self._scans_by_chunks(getattr(ctx, "dtype", None), ctx, heads, dk, dv, q, k, v, *([raw] if mode == 0 else []), constant=mode == 2):
+        rows = (*self._rows_f32(q, "decay_scan q"), *self._rows_f32(k, "decay_scan k"), *self._rows_f32(v, "decay_scan v"),
+                *(self._rows_f32(raw, "decay_scan raw") if raw is not None else (_ptr(None), _LL(0))), _ptr(state), _LL(state.stride(0)),
+                _ptr(ctx.req_slot), _ptr(ctx.cu_seqlens), _ptr(out), _ptr(step_bias), _ptr(log_rate), _ptr(skip))
+        longest = int(ctx.max_span)
+        if self._scans_by_chunks(getattr(ctx, "dtype", None), ctx, heads, dk, dv, constant=mode == 2):
             least, short = self._parting(ctx)
             room = torch.empty(int(self.lib.ifx_chunk_scan_scratch_floats(T, ctx.num_requests, least, heads, dk, dv, int(mode == 0))),
                                dtype=torch.float32, device=q.device)
-            _check(self.lib.ifx_chunk_decay_scan(
-                *self._rows_f32(q, "decay_scan q"), *self._rows_f32(k, "decay_scan k"), *self._rows_f32(v, "decay_scan v"),
-                *(self._rows_f32(raw, "decay_scan raw") if raw is not None else (_ptr(None), _LL(0))), _ptr(state),
-                ctypes.c_longlong(state.stride(0)), _ptr(ctx.req_slot), _ptr(ctx.cu_seqlens), _ptr(out), _ptr(step_bias),
-                _ptr(log_rate), _ptr(skip), ctx.num_requests, T, least, int(heads), int(groups), int(dk), int(dv), mode,
-                ctypes.c_float(tau), ctypes.c_float(q_scale), _ptr(room), _ptr(rate), _stream()), "decay_scan (stretches)")
-            self.launches += 3
-            if not short:
-                return out
-            longest = short                                # the other spans, token by token
-        else:
-            longest = int(ctx.max_span)
+            rc = self.lib.ifx_chunk_decay_scan(*rows, ctx.num_requests, T, least, int(heads), int(groups), int(dk), int(dv), mode,
+                                               ctypes.c_float(tau), ctypes.c_float(q_scale), _ptr(room), _ptr(rate), _stream())
+            if rc != _MISALIGNED:
+                _check(rc, "decay_scan (stretches)")
+                self.launches += 3
+                if not short:
+                    return out
+                longest = short                            # the other spans, token by token
         scratch = None                                     # steps with long spans make their decays in a pass of their own
         if longest >= 64 and mode != 2:
             scratch = torch.empty(T * (heads * dk if mode == 0 else 2 * heads), dtype=torch.float32, device=q.device)
-        _check(self.lib.ifx_decay_scan_rate(*self._rows_f32(q, "decay_scan q"), *self._rows_f32(k, "decay_scan k"),
-                                       *self._rows_f32(v, "decay_scan v"),
-                                       *(self._rows_f32(raw, "decay_scan raw") if raw is not None else (_ptr(None), _LL(0))), _ptr(state),
-                                       ctypes.c_longlong(state.stride(0)), _ptr(ctx.req_slot), _ptr(ctx.cu_seqlens), _ptr(out),
-                                       _ptr(step_bias), _ptr(log_rate), _ptr(skip), ctx.num_requests, T, longest, int(longest < ctx.max_span), int(heads),
-                                       int(groups), int(dk), int(dv), mode, ctypes.c_float(tau), ctypes.c_float(q_scale), 296,
-                                       _ptr(scratch), _ptr(rate), _stream()), "decay_scan")
+        _check(self.lib.ifx_decay_scan_rate(*rows, ctx.num_requests, T, longest, int(longest < ctx.max_span), int(heads), int(groups), int(dk),
+                                            int(dv), mode, ctypes.c_float(tau), ctypes.c_float(q_scale), 296, _ptr(scratch), _ptr(rate), _stream()),
+               "decay_scan")
         self.launches += 1 + int(scratch is not None)
         return out
 
