@@ -183,6 +183,7 @@ class CudaKernels:
         self.chunk_scans = os.environ.get("INFERFLUX_B200_CHUNK_SCANS", "1") != "0"
         self.lib.ifx_sample_scratch_bytes.restype = ctypes.c_longlong
         self.lib.ifx_latent_attention_mma_workspace.restype = ctypes.c_longlong
+        self._latent_sizes = {}
         # latent attention on the tensor-core tiles (0: the per-token kernel, for comparisons)
         self.latent_tiles = os.environ.get("INFERFLUX_B200_LATENT_TILES", "1") != "0"
         # decoded tokens on the kernel made for them (0: the tiles of prompt portions, for comparisons)
@@ -1346,6 +1347,13 @@ class CudaKernels:
         self.launches += 1
         return out
 
+    def _latent_by_tma(self, rank, rot, page_size):
+        """Whether the kernels whose tiles come by TMA take these sizes; asked of them once per sizes."""
+        key = rank, rot, page_size
+        if key not in self._latent_sizes:
+            self._latent_sizes[key] = bool(self.lib.ifx_latent_decode_supports(*key) and self.lib.ifx_latent_prompt_supports(*key))
+        return self._latent_sizes[key]
+
     def _latent_attention_tiles(self, q_rows, w_uk, w_uv, sinks, heads, dim, vdim, rank, window, scale, ctx, cache, rot=0,
                                 ql=None, head_gate=None):
         """bfloat16: queries into latent space (a product per head), the tensor-core kernel over cached latents
@@ -1367,16 +1375,16 @@ class CudaKernels:
         win = 0 if window is None else int(window)
         splits = 1
         max_keys = int(ctx.max_kv_len if not win else min(win, ctx.max_kv_len))
-        decode = (ctx.max_span == 1 and self.latent_decode and self.lib.ifx_latent_decode_supports(rank, int(rot), cache.page_size)
-                  and ql.data_ptr() % 16 == 0 and kv.data_ptr() % 16 == 0)
+        by_tma = self._latent_by_tma(rank, int(rot), cache.page_size) and (ql.data_ptr() | kv.data_ptr()) % 16 == 0
+        decode = by_tma and ctx.max_span == 1 and self.latent_decode
         if decode:                                         # decoded tokens only, a kernel of their own
             stretch = int(self.lib.ifx_latent_decode_stretch(T, heads, max_keys))
             splits = -(-(max_keys + 15) // stretch)        # (a window may begin inside a tile of 16 keys)
             decode = splits <= 64
         # spans of which a block's 128 rows (a token with all its heads) are a good part: the tcgen05 kernel
-        prompt = (not decode and self.latent_prompt and min(n for _s, n in ctx.spans) * heads >= self.LATENT_PROMPT_MIN_ROWS
-                  and self.lib.ifx_latent_prompt_supports(rank, int(rot), cache.page_size)
-                  and ql.data_ptr() % 16 == 0 and kv.data_ptr() % 16 == 0)
+        # (whose running maximum is of the scores before they are scaled, so that a scale has to be positive)
+        prompt = (by_tma and not decode and self.latent_prompt and scale > 0.0
+                  and min(n for _s, n in ctx.spans) * heads >= self.LATENT_PROMPT_MIN_ROWS)
         if decode:
             pass
         elif prompt:                                       # a block an SM: cut the keys while there are fewer blocks than SMs

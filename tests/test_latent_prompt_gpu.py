@@ -146,3 +146,14 @@ def test_what_is_not_a_number_arrives_in_the_result(cuda_kernels, what, context,
     assert bool(torch.isfinite(clean).all())
     assert torch.equal(torch.isfinite(got), (~bad)[..., None].expand_as(got))
     assert torch.equal(got[~bad], clean[~bad])
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.2])
+def test_a_scale_that_is_not_positive_keeps_the_tiles(cuda_kernels, scale):
+    """The running maximum of the tcgen05 kernel is of the scores before they are scaled."""
+    spans, heads, rot = [(30, 70)], 12, 64
+    ctx, cache, view, rows, g = _setup(cuda_kernels, spans, rot, 16, None, 9)
+    ql = torch.randn(70, heads, 256 + rot, generator=g).to(BF)
+    want = _plain(ql, spans, rows, None, scale, None, None)
+    got = _run(cuda_kernels, ctx, view, ql, heads, rot, None, scale, None, None)
+    assert float((got - want).abs().max()) <= 2.0 ** -7 * max(1.0, float(want.abs().max()))
