@@ -1721,12 +1721,12 @@ class CudaKernels:
         """bfloat16, few tokens: every chosen expert's weights once through the tensor cores (csrc/moe_stream_tcgen05.cu)."""
         T, width = h.shape
         top, ff = ids.shape[1], w_up.shape[1] // (2 if glu is not None else 1)
-        act = torch.empty(T * top, ff, dtype=torch.bfloat16, device=h.device)
-        slices = int(self.lib.ifx_moe_stream_slices(ff))
-        y = torch.empty(slices, T * top, width, dtype=torch.float32, device=h.device)
+        sums = int(self.lib.ifx_moe_stream_slices(ff)) * T * top * width           # float32, then the activations in bfloat16
+        room = torch.empty(sums + T * top * ff // 2, dtype=torch.float32, device=h.device)
         out = torch.empty(T, width, dtype=out_dtype, device=h.device)
         limit, slope, offset = glu if glu is not None else (0.0, 0.0, 0.0)
-        _check(self.lib.ifx_moe_stream(_ptr(h), _ptr(w_up), _ptr(w_down), _ptr(ids), _ptr(weights), _ptr(act), _ptr(y), _ptr(out),
+        act = ctypes.c_void_p(room.data_ptr() + 4 * sums)
+        _check(self.lib.ifx_moe_stream(_ptr(h), _ptr(w_up), _ptr(w_down), _ptr(ids), _ptr(weights), act, _ptr(room), _ptr(out),
                                        T, top, int(experts), width, ff, _DT[out_dtype], int(glu is not None), ctypes.c_float(limit),
                                        ctypes.c_float(slope), ctypes.c_float(offset), _ptr(self.error_flag), _stream()),
                "moe experts (stream)")
