@@ -23,11 +23,12 @@
 //
 // The order of the sums depends on where a span is cut into steps, so the float32 run keeps the scans.
 //
-// Bound: issue slots of chunk_local, which split every operand into three and make eight products of them, and the states, which go
-// through L2 twice (26 MB at 2,048 tokens of 12 heads of 128 x 128).  A warp's tile is 32 x 16, so that an operand is split and read
-// by few warps.  Measured, us, scan -> this, one span of 2,048 tokens: constant decay, 12 heads of 128 x 128 590 -> 119; wkv, 24
-// heads of 64 (with its norm) 521 -> 123; a decay per token, 24 heads of 128 x 64 693 -> 116; per key channel, 12 heads of
-// 64 x 128 491 -> 92.  At 130 tokens 42 -> 31, 41 -> 30, 50 -> 31, 36 -> 25; at 64 the scan is the faster.
+// Bound: no unit alone.  chunk_local splits every operand into three and makes eight products of them: issue slots 44 % busy, ALU 35 %,
+// tensor pipe 31 %, with 14 warps an SM that wait for barriers, for the latency of that chain and for states, which go through L2
+// twice (26 MB at 2,048 tokens of 12 heads of 128 x 128).  A warp's tile is 32 x 16, so that an operand is split and read
+// by few warps.  Measured, us, scan -> this, one span of 2,048 tokens: constant decay, 12 heads of 128 x 128 590 -> 120; wkv, 24
+// heads of 64 (with its norm) 521 -> 127; a decay per token, 24 heads of 128 x 64 693 -> 117; per key channel, 12 heads of
+// 64 x 128 491 -> 93.  At 130 tokens 42 -> 32, 41 -> 30, 50 -> 32, 36 -> 25; at 64 the scan is the faster.
 // Errors of outputs and of the state against 64 bits (2-norm, scan and this, parameters where trained models have them, 2,048
 // tokens): constant decay 3.5e-7 and 1.1e-7, 3.8e-7 and 0.8e-7; a decay per token 1.65e-7 and 1.53e-7, 1.30e-7 and 1.22e-7; per key
 // channel 3.20e-6 and 3.16e-6, 3.98e-6 and 3.96e-6; wkv's state 9.14e-7 and 9.17e-7.  (With operands of 22 bits and sums left in the

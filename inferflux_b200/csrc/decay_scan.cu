@@ -21,7 +21,7 @@
 // stretch of tokens' q, k, raw decay and v arrives in shared memory by cp.async, one stretch ahead of the one being
 // worked on (the exponentials are taken there, once per token and channel).  Every sum's order depends on (dk, R, KS)
 // only, never on how the tokens were cut into steps or which other requests are in the batch.
-// Long spans of a bfloat16 run go to chunk_scan.cu instead (CHUNK_SCAN_MIN_SPAN in ops.py); this is the scan of a float32 run, of
+// Long spans of a bfloat16 run go to chunk_scan.cu instead (stretches_pay in ops.py); this is the scan of a float32 run, of
 // decoded tokens and of short spans.  With `part` spans of more than `max_span` tokens are in the step and are not touched.
 #include "common.cuh"
 

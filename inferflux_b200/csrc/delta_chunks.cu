@@ -22,14 +22,13 @@
 // cores with split operands (chunk_scan.cuh); the triangular system goes by blocks of 16 rows, substituted in the blocks.
 //
 // A stretch that holds a number that is not finite, or in which one comes up that a scan would not have formed, is walked token by
-// token.  The order of the sums depends on where a span is
-// cut into steps, so the float32 run keeps the scan.
+// token.  The order of the sums depends on where a span is cut into steps, so the float32 run keeps the scan.
 //
-// Bound: delta_local, one block of 16 warps an SM (128 KB): issue slots for the splitting of operands and twenty barriers.  2,048 tokens
-// of 24 heads: delta_rule.cu's three kernels 658 us, these 297.  Error of the state against 64 bits (2-norm, scan and this, 2,048
-// tokens): parameters where trained models have them 5.2e-7 and 4.6e-7, decays near one 1.76e-6 and 1.70e-6, random ones 0.95e-7
-// and 1.00e-7.  (With operands of 22 bits 241 us, 1.4e-7 in the last case, and 1.0e-6 in place of the scan's 4.6e-7 where 130 keys are
-// nearly the same.)
+// Bound: delta_local, one block of 16 warps an SM (128 KB): twenty barriers and the chain split -> product -> sum between them (issue
+// slots 44 % busy, tensor pipe 29 %).  2,048 tokens of 24 heads: delta_rule.cu's three kernels 658 us, these 303.
+// Error of the state against 64 bits (2-norm, scan and this, 2,048 tokens): parameters where trained models have them 5.2e-7 and
+// 4.6e-7, decays near one 1.76e-6 and 1.70e-6, random ones 0.95e-7 and 1.00e-7.  (With operands of 22 bits 241 us, 1.4e-7 in the last
+// case, and 1.0e-6 in place of the scan's 4.6e-7 where 130 keys are nearly the same.)
 #include "chunk_scan.cuh"
 
 namespace ifx {

@@ -16,7 +16,7 @@
 // alone, so a token's result does not depend on how its request's tokens were cut into steps or on what else is in the
 // batch.
 //
-// Long spans of a bfloat16 run go to delta_chunks.cu instead of delta_scan (DELTA_CHUNKS_MIN_SPAN in ops.py), where stretches of 64
+// Long spans of a bfloat16 run go to delta_chunks.cu instead of delta_scan (delta_stretches_pay in ops.py), where stretches of 64
 // tokens are products on the tensor cores; preparation and finish are these.
 #include "common.cuh"
 

@@ -902,10 +902,11 @@ class CudaKernels:
         return parts
 
     def _prefill_parts(self, ctx, nq, window):
-        """A block takes up to 256 tokens of a head and an SM to itself, so what is left behind whole rounds of 148 blocks leaves SMs idle for as long as its longest
-        block walks; with few blocks that is the whole grid.  Cut while every part keeps four tiles of 128 keys: with parts of
-        three or of six the times below are the same or up to 3 % longer, and below that adding the parts up takes what they save.
-        Eight tiles stay whole too: two parts of four save 0.6 us, and the launch that adds them up costs the host 3.
+        """A block takes up to 256 tokens of a head and an SM to itself, so what is left behind whole rounds of 148 blocks leaves SMs idle
+        for as long as its longest block walks; with few blocks that is the whole grid.  Cut while every part keeps four tiles of 128
+        keys: with parts of three or of six the times below are the same or up to 3 % longer, and below that adding the parts up takes
+        what they save.  Eight tiles stay whole too: two parts of four save 0.6 us, and the launch that adds them up and its workspace
+        cost the host 5.
         us, whole and cut: 28 heads, two requests' 2,500 tokens behind up to 4,000 (12 of 308 blocks left) 191 and 162, 384 tokens
         behind 2,000 39.0 and 32.4; 12 heads, 512 tokens behind 3,000 (24 blocks, six parts) 61.9 and 30.2, 600 tokens behind 900
         26.9 and 24.6."""
@@ -1462,47 +1463,50 @@ class CudaKernels:
         return out
 
     # Spans of this many tokens and more can go by stretches of 64 tokens in a bfloat16 run (csrc/chunk_scan.cu, delta_chunks.cu).  The
-    # other spans of the same step then go through the scans token by token, in launches of their own: a stretch costs the same
-    # with one token as with 64.
+    # other spans of the same step then go along, or through the scans token by token in launches of their own: a stretch costs the
+    # same with one token as with 64.
     CHUNK_SCAN_MIN_SPAN = 128
 
     def _long_spans(self, ctx):
-        """(longest, tokens, number) of a step's spans of fewer than CHUNK_SCAN_MIN_SPAN tokens and the stretches of the others, found
-        once a step; None for a context without a host list of spans, whose spans all go the same way."""
+        """(longest, tokens, number, stretches) of a step's spans of fewer than CHUNK_SCAN_MIN_SPAN tokens and the stretches of the others,
+        found once a step; None for a context without a host list of spans, whose spans all go the same way."""
         got = getattr(ctx, "long_spans", None)
         if got is None and getattr(ctx, "spans", None):
             short = [n for _s, n in ctx.spans if n < self.CHUNK_SCAN_MIN_SPAN]
-            got = ctx.long_spans = (max(short, default=0), sum(short), len(short),
+            got = ctx.long_spans = (max(short, default=0), sum(short), len(short), sum(-(-n // 64) for n in short),
                                     sum(-(-n // 64) for _s, n in ctx.spans if n >= self.CHUNK_SCAN_MIN_SPAN))
         return got
 
     def _scans_by_chunks(self, dtype, ctx, heads, dk, dv, *rows, constant=False):
-        """Whether a recurrence's long spans go by stretches of tokens: where that pays, with sizes the kernels are made for, rows
-        on 16-byte boundaries (those given here; the kernels look at theirs themselves), and in a bfloat16 run (the order of the sums
-        then depends on how a span was cut into steps)."""
+        """Which of a recurrence's spans go by stretches of tokens: False, none; else (the fewest tokens of one that does, the most
+        tokens of one that does not or 0).  Where that pays, with sizes the kernels are made for, rows on 16-byte boundaries (those
+        given here; the kernels look at theirs themselves), and in a bfloat16 run (the order of the sums then depends on how a span
+        was cut into steps)."""
         if not (self.chunk_scans and dtype is torch.bfloat16 and ctx.max_span >= self.CHUNK_SCAN_MIN_SPAN):
             return False
         if dk not in (64, 128) or dv % 64 or ctx.num_requests > 64:              # ifx_chunk_scan_supports, without a call
             return False
         spans = self._long_spans(ctx)
-        return ((spans is None or self.stretches_pay(ctx.max_span, spans[0], spans[3], constant and dk == 64))
-                and all(t.data_ptr() % 16 == 0 and (t.dim() < 2 or t.stride(0) % 4 == 0) for t in rows))
+        plan = (1, 0) if spans is None else self.stretches_pay(ctx.max_span, heads * dv // 64, constant and dk == 64, *spans)
+        return plan if plan and all(t.data_ptr() % 16 == 0 and (t.dim() < 2 or t.stride(0) % 4 == 0) for t in rows) else False
 
-    @staticmethod
-    def stretches_pay(longest, short, stretches, cheap):
-        """For a step whose longest span has `longest` tokens, the longest of fewer than CHUNK_SCAN_MIN_SPAN `short` (0: none).  What is
-        gained is the time between the two; a launch for the short spans costs a few us beside them.  us, the scan alone and this
-        (12 heads of 128 x 128 with a constant decay; wkv, 24 heads of 64): 128 tokens 41 / 32; 40 / 29; 128 and 31 of one
-        75 / 66; 96 / 63; 512 and 31 of one 237 / 78; 260 / 75; 128 and 20 47 / 44; 44 / 41; 192 and 60 68 / 56; 62 / 52; 228 and 100
-        80 / 81; 73 / 74; 512, 100, 80 and 29 of one 229 / 123; 268 / 127; sixteen of 128 213 / 151; 184 / 148; at 56 heads 128 and 63 of
-        one 192 / 198; 242 / 174.  `cheap`, a constant decay and keys of 64 numbers: its scan wins where very many stretches are
-        of short spans (28 heads, 32 of 128: 442 / 493; sixteen of 256 458 / 375)."""
-        return (short < 24 or longest >= short + 128) and not (cheap and stretches > 24 + longest // 4)
-
-    def _parting(self, ctx):
-        """(the fewest tokens of a span that goes by stretches, the most tokens of one that does not or 0)."""
-        spans = self._long_spans(ctx)
-        return (1, 0) if spans is None else (self.CHUNK_SCAN_MIN_SPAN, spans[0])
+    @classmethod
+    def stretches_pay(cls, longest, blocks, cheap, short, short_tokens, short_spans, short_stretches, stretches):
+        """The plan for a step whose longest span has `longest` tokens, with `blocks` blocks a stretch.  Short spans go along where their
+        stretches (0.13 us a block) take less than a launch of the scan for them.  Otherwise what is gained is the time between the
+        longest span and the longest short one.  us, the scan alone and this (12 heads of 128 x 128 with a constant decay; wkv, 24
+        heads of 64): 128 tokens 41 / 32; 40 / 29; sixteen of 128 213 / 152; 183 / 148; short spans along: 128 and 20 46 / 33; 44 / 30;
+        228 and 100 80 / 45 (81 beside); 73 / 42 (74); beside the scan: 128 and 31 of one 75 / 66; 96 / 62 (146; 121 along); 512 and 31
+        of one 239 / 79; 260 / 76; 512, 100, 80 and 29 of one 226 / 124; 267 / 127.  At 56 heads 128 and 31 of one 123 / 117; 154 / 109,
+        but 63 of one 187 / 199; 242 / 174: what the launch for very many states costs has to be gained.  `cheap`, a constant decay and
+        keys of 64 numbers: its scan wins where very many stretches are of short spans (28 heads, 32 of 128 442 / 493; sixteen of 256
+        456 / 374)."""
+        if cheap and stretches > 24 + longest // 4:
+            return False
+        if 0.13 * short_stretches * blocks <= 8 + 0.22 * short + 0.035 * short_spans * blocks:
+            return 1, 0
+        beside = longest >= short + 128 or (short < 24 and (longest >= 192 or short_spans * blocks <= 2500))
+        return (cls.CHUNK_SCAN_MIN_SPAN, short) if beside else False
 
     def wkv_scan(self, r, k, v, w_raw, g, w0, u, norm_w, eps, heads, dim, state, prev_offset, x, ctx, out_dtype):
         """The recurrence of csrc/wkv.cu over every request's tokens.  r, k, v, w_raw, g: float32 [T, heads * dim], each
@@ -1523,7 +1527,7 @@ class CudaKernels:
               "wkv_scan: the state does not fit the sizes")
         by_chunks, size = self._scans_by_chunks(out_dtype, ctx, heads, dim, dim), T * HD
         if by_chunks:
-            least, short = self._parting(ctx)
+            least, short = by_chunks
             size += int(self.lib.ifx_chunk_scan_scratch_floats(T, ctx.num_requests, least, heads, dim, dim, 1))
         scratch = torch.empty(size, dtype=torch.float32, device=r.device)         # the sums, and what the stretches need
         y = torch.empty(T, HD, dtype=out_dtype, device=r.device)
@@ -1551,30 +1555,39 @@ class CudaKernels:
         return y
 
     def _delta_by_chunks(self, dtype, ctx, tokens, heads, dim):
-        """Whether the delta rule's long spans go by stretches."""
+        """Which spans of the delta rule go by stretches, as above."""
         if not (self.chunk_scans and dtype is torch.bfloat16 and ctx.max_span >= self.CHUNK_SCAN_MIN_SPAN):
             return False
+        if dim != 64 or ctx.num_requests > 64:                                   # ifx_delta_chunks_supports, without a call
+            return False
         spans = self._long_spans(ctx)
-        pays = tokens <= 8 * ctx.max_span if spans is None else self.delta_stretches_pay(heads, tokens, ctx.num_requests, ctx.max_span, *spans)
-        return pays and dim == 64 and ctx.num_requests <= 64                     # ifx_delta_chunks_supports, without a call
+        if spans is None:
+            return tokens <= 8 * ctx.max_span and (1, 0)
+        return self.delta_stretches_pay(heads, tokens, ctx.num_requests, ctx.max_span, *spans)
 
-    @staticmethod
-    def delta_stretches_pay(heads, tokens, requests, longest, short, short_tokens, short_requests, stretches):
+    @classmethod
+    def delta_stretches_pay(cls, heads, tokens, requests, longest, short, short_tokens, short_spans, short_stretches, stretches):
         """A stretch of the delta rule does several times a token's work of the scan; what is gained is that the tokens of one span run
-        side by side, so this compares what both ways take.  us, fitted to what follows within a tenth: the scan walks its longest
-        span at 0.3 a token and more with more columns at once; the stretches go in rounds of 148 blocks (a head's stretch each).
-        us, 24 heads of 64, the scan alone and this: 128 tokens 47 / 48; 256 87 / 53; 512 165 / 96; 2,048 659 / 304; two of 256
-        99 / 92; four of 256 128 / 139; four of 512 262 / 277; eight of 512 377 / 509; with 31 of one 128 68 / 72, 256 115 / 81, 512
-        211 / 129; with 63 of one 512 225 / 144; 256 and 100 106 / 102; 512, 100, 80 and 29 of one 222 / 176.  56 heads: 192 82 / 90;
-        256 105 / 93; 2,048 841 / 608; four of 256 267 / 320; with 31 of one 512 280 / 249."""
+        side by side, so this compares what the ways take: the scan for all, stretches for all, stretches for the long spans beside
+        the scan for the others.  us, fitted to what follows within a tenth: the scan walks its longest span at 0.3 a token and more
+        with more columns at once; the stretches go in rounds of 148 blocks (a head's stretch each).
+        us, 24 heads of 64, the scan alone and the stretches (beside the scan): 128 tokens 47 / 48; 256 87 / 53; 512 165 / 96; 2,048
+        659 / 304; two of 256 99 / 92; four of 256 128 / 139; four of 512 262 / 277; eight of 512 377 / 509; with 31 of one 128 68 / 72,
+        256 115 / 81, 512 211 / 129; with 63 of one 512 225 / 144; 256 and 100 106 / 102; 512, 100, 80 and 29 of one 222 / 176.
+        56 heads: 192 82 / 90; 256 105 / 93; 2,048 841 / 608; four of 256 267 / 320; with 31 of one 512 280 / 249."""
         def scan(longest, tokens, requests):
             columns = tokens * heads / longest             # heads at work at once, on average
             return longest * max(0.3 + 0.0019 * columns, columns / 275) + 0.018 * requests * heads
-        blocks = stretches * heads
-        chunks = 37 * -(-blocks // 148) + 1.5 * (longest / 64) + 0.055 * blocks + 8
+
+        def chunks(blocks):
+            return 37 * -(-blocks // 148) + 1.5 * (longest / 64) + 0.055 * blocks + 8
+        least, alone = 1, 6 + scan(longest, tokens, requests - 1)
+        best = chunks((stretches + short_stretches) * heads)
         if short:
-            chunks += 10 + scan(short, short_tokens, short_requests)
-        return 1.1 * chunks < 6 + scan(longest, tokens, requests - 1)
+            beside = chunks(stretches * heads) + 10 + scan(short, short_tokens, short_spans)
+            if beside < best:
+                least, best = cls.CHUNK_SCAN_MIN_SPAN, beside
+        return 1.1 * best < alone and (least, short if least > 1 else 0)
 
     def delta_rule_scan(self, proj, w_raw, w0, a_bias, norm_w, eps, heads, dim, state, ctx, out_dtype):
         """The recurrence of csrc/delta_rule.cu over every request's tokens.  `proj`: float32 [T, 5 heads dim], the
@@ -1589,8 +1602,9 @@ class CudaKernels:
         _need(state is not None and state.dtype == torch.float32 and state.dim() == 2 and state.stride(1) == 1
               and state.shape[1] >= HD * dim, "delta_rule_scan: the state does not fit the sizes")
         y = torch.empty(T, HD, dtype=out_dtype, device=proj.device)
-        if self._delta_by_chunks(out_dtype, ctx, T, heads, dim):
-            least, short = self._parting(ctx)
+        by_chunks = self._delta_by_chunks(out_dtype, ctx, T, heads, dim)
+        if by_chunks:
+            least, short = by_chunks
             room = torch.empty(int(self.lib.ifx_delta_chunks_scratch_floats(T, ctx.num_requests, least, heads)), dtype=torch.float32,
                                device=proj.device)
             scan_room = None
@@ -1854,8 +1868,9 @@ class CudaKernels:
                 *(self._rows_f32(raw, "decay_scan raw") if raw is not None else (_ptr(None), _LL(0))), _ptr(state), _LL(state.stride(0)),
                 _ptr(ctx.req_slot), _ptr(ctx.cu_seqlens), _ptr(out), _ptr(step_bias), _ptr(log_rate), _ptr(skip))
         longest = int(ctx.max_span)
-        if self._scans_by_chunks(getattr(ctx, "dtype", None), ctx, heads, dk, dv, constant=mode == 2):
-            least, short = self._parting(ctx)
+        by_chunks = self._scans_by_chunks(getattr(ctx, "dtype", None), ctx, heads, dk, dv, constant=mode == 2)
+        if by_chunks:
+            least, short = by_chunks
             room = torch.empty(int(self.lib.ifx_chunk_scan_scratch_floats(T, ctx.num_requests, least, heads, dk, dv, int(mode == 0))),
                                dtype=torch.float32, device=q.device)
             rc = self.lib.ifx_chunk_decay_scan(*rows, ctx.num_requests, T, least, int(heads), int(groups), int(dk), int(dv), mode,

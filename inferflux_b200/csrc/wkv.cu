@@ -19,7 +19,7 @@
 // key channels i = s, s + KS, s + 2 KS, ... of S in registers (KS a power of two up to 32 that depends on the
 // head size alone; the KS threads of a channel are neighbours in a warp and add their shares by shuffles).  r, k, w and v of up to 32 tokens arrive in shared
 // memory at a time, so the block synchronises three times per 32 tokens, not per token.
-// Long spans of a bfloat16 run go to chunk_scan.cu instead (CHUNK_SCAN_MIN_SPAN in ops.py), followed by wkv_norm below.
+// Long spans of a bfloat16 run go to chunk_scan.cu instead (stretches_pay in ops.py), followed by wkv_norm below.
 #include "common.cuh"
 
 namespace ifx {

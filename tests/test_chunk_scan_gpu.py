@@ -190,8 +190,17 @@ def _mixed_ctx(lens, slots, device):
     return ctx
 
 
+def _part(cuda_kernels, monkeypatch, beside):
+    """All spans of a step by stretches, or the long ones beside the scan for the others."""
+    plan = lambda short: (128, short) if beside and short else (1, 0)
+    monkeypatch.setattr(cuda_kernels, "stretches_pay", lambda longest, blocks, cheap, short, *more: plan(short))
+    monkeypatch.setattr(cuda_kernels, "delta_stretches_pay", lambda heads, tokens, requests, longest, short, *more: plan(short))
+
+
+@pytest.mark.parametrize("beside", [False, True])
 @pytest.mark.parametrize("mode,H,G,dk,dv", [("sigmoid_root", 2, 2, 64, 128), ("softplus_step", 2, 1, 128, 64), ("constant", 3, 3, 64, 64)])
-def test_long_spans_by_stretches_beside_short_ones_by_the_scan(cuda_kernels, mode, H, G, dk, dv):
+def test_long_spans_by_stretches_beside_short_ones(cuda_kernels, monkeypatch, mode, H, G, dk, dv, beside):
+    _part(cuda_kernels, monkeypatch, beside)
     g = torch.Generator().manual_seed(dk)
     vec = [torch.rand(H, generator=g) for _ in range(3)]
     kw = {"sigmoid_root": {"tau": 3.0}, "softplus_step": {"step_bias": vec[0], "log_rate": vec[1], "skip": vec[2]},
@@ -207,13 +216,15 @@ def test_long_spans_by_stretches_beside_short_ones_by_the_scan(cuda_kernels, mod
         got = cuda_kernels.decay_scan(*cut(wide.to(DEV)), None if raw is None else raw.to(DEV), state, _mixed_ctx(lens, slots, DEV), heads=H,
                                       groups=G, dk=dk, dv=dv, decay=mode, **on)
         # three for the stretches, the scan, and its decays ahead of it where its longest span has 64 tokens and they are not constant
-        assert cuda_kernels.launches - before == ((5 if mode != "constant" else 4), 4, 1)[step]
+        assert cuda_kernels.launches - before == (((5 if mode != "constant" else 4), 4, 1) if beside else (3, 3, 1))[step]
         for a, b in ((got, want), (state, state_p)):                            # float32 sums of up to 300 terms
             assert float((a.double().cpu() - b).abs().max()) <= 5e-6 * max(1.0, float(b.abs().max()))
 
 
+@pytest.mark.parametrize("beside", [False, True])
 @pytest.mark.parametrize("H,D", [(3, 64), (1, 128)])
-def test_wkv_of_long_and_short_spans(cuda_kernels, H, D):
+def test_wkv_of_long_and_short_spans(cuda_kernels, monkeypatch, H, D, beside):
+    _part(cuda_kernels, monkeypatch, beside)
     HD, C = H * D, 40
     g = torch.Generator().manual_seed(H)
     w0, u, nw = torch.randn(HD, generator=g), 0.5 * torch.randn(HD, generator=g), 1 + 0.2 * torch.randn(HD, generator=g)
@@ -227,7 +238,7 @@ def test_wkv_of_long_and_short_spans(cuda_kernels, H, D):
         before = cuda_kernels.launches
         y = cuda_kernels.wkv_scan(*(t.to(DEV) for t in (r, k, v, w_raw, gate, w0, u, nw)), 1e-5, H, D, state, HD * D, x.to(DEV),
                                   _mixed_ctx(lens, slots, DEV), torch.bfloat16)
-        assert cuda_kernels.launches - before == (5, 5, 1)[step]
+        assert cuda_kernels.launches - before == ((5, 5, 1) if beside else (4, 4, 1))[step]
         assert float((y.double().cpu() - want).abs().max()) <= 2.0 ** -8 * max(1.0, float(want.abs().max()))
         assert float((state.double().cpu() - state_p).abs().max()) <= 5e-6 * max(1.0, float(state_p.abs().max()))
 

@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from plain.plain_kernels import PlainKernels
-from test_chunk_scan_gpu import MIXED, STEPS, _Ctx, _mixed_ctx
+from test_chunk_scan_gpu import MIXED, STEPS, _Ctx, _mixed_ctx, _part
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -109,8 +109,9 @@ def test_products_that_a_scan_does_not_form(cuda_kernels, block):
     assert float((state - state_w).abs().max()) <= 1e-5 * float(state_w.abs().max())
 
 
-def test_long_spans_by_stretches_beside_short_ones_by_the_scan(cuda_kernels, monkeypatch):
-    monkeypatch.setattr(cuda_kernels, "delta_stretches_pay", lambda *a: True)
+@pytest.mark.parametrize("beside", [False, True])
+def test_long_spans_by_stretches_beside_short_ones(cuda_kernels, monkeypatch, beside):
+    _part(cuda_kernels, monkeypatch, beside)
     H, D = 3, 64
     HD = H * D
     g = torch.Generator().manual_seed(8)
@@ -123,7 +124,7 @@ def test_long_spans_by_stretches_beside_short_ones_by_the_scan(cuda_kernels, mon
         before = cuda_kernels.launches
         y = cuda_kernels.delta_rule_scan(proj.to(DEV), w_raw.to(DEV), *(t.to(DEV) for t in vec), 1e-5, H, D, state,
                                          _mixed_ctx(lens, slots, DEV), BF)
-        assert cuda_kernels.launches - before == (6, 6, 3)[step]                # two more for the short spans; the scan alone
+        assert cuda_kernels.launches - before == ((6, 6, 3) if beside else (4, 4, 3))[step]     # two more for the short spans; the scan alone
         # the norm divides by the size of a head's sums, which may be small
         assert float((y.double().cpu() - want).abs().max()) <= 2.0 ** -8 * max(1.0, float(want.abs().max()))
         assert float((state.double().cpu() - state_p).abs().max()) <= 5e-6 * max(1.0, float(state_p.abs().max()))

@@ -9,12 +9,10 @@ class _Table:
     """The rules of a kernel table that was never made."""
     chunk_scans = True
     CHUNK_SCAN_MIN_SPAN = CudaKernels.CHUNK_SCAN_MIN_SPAN
-    stretches_pay, delta_stretches_pay = staticmethod(CudaKernels.stretches_pay), staticmethod(CudaKernels.delta_stretches_pay)
-    _long_spans, _parting = CudaKernels._long_spans, CudaKernels._parting
+    stretches_pay, delta_stretches_pay = CudaKernels.stretches_pay, CudaKernels.delta_stretches_pay
+    _long_spans = CudaKernels._long_spans
     _scans_by_chunks, _delta_by_chunks = CudaKernels._scans_by_chunks, CudaKernels._delta_by_chunks
 
-    class lib:
-        ifx_chunk_scan_supports = ifx_delta_chunks_supports = staticmethod(lambda *a: 1)
 
 
 class _Ctx:
@@ -22,29 +20,36 @@ class _Ctx:
         self.spans, self.num_requests, self.max_span = [(7, n) for n in lens], len(lens), max(lens)
 
 
-SPANS = {"prompt": (2048,), "short prompt": (127,), "prompts": (500, 400), "portion and decoded": (512,) + (1,) * 31,
-         "small portion and decoded": (128,) + (1,) * 31, "portion and a short span": (200, 100), "many": (128,) * 32, "decoded": (1,) * 32}
+ALL, NONE = (1, 0), False
 
 
-@pytest.mark.parametrize("kind,scans,deltas", [
-    ("prompt", True, True), ("short prompt", False, False), ("prompts", True, True), ("portion and decoded", True, True),
-    ("small portion and decoded", True, False), ("portion and a short span", False, False), ("many", True, False), ("decoded", False, False)])
-def test_recurrences_by_stretches(kind, scans, deltas):
-    """A decoded token is a stretch of its own, so what counts is stretches and what the scan would take, not the longest span alone."""
-    table, lens = _Table(), SPANS[kind]
+@pytest.mark.parametrize("lens,scans,deltas", [
+    ((2048,), ALL, ALL), ((127,), NONE, NONE), ((500, 400), ALL, ALL), ((512,) + (1,) * 31, (128, 1), (128, 1)),
+    ((128,) + (1,) * 31, (128, 1), NONE), ((512, 1), ALL, ALL), ((200, 100), ALL, ALL), ((150, 71), ALL, ALL),
+    ((512, 100, 80) + (1,) * 29, (128, 100), (128, 100)), ((200,) + (100,) * 30, NONE, NONE), ((128,) * 32, ALL, NONE), ((1,) * 32, NONE, NONE)])
+def test_recurrences_by_stretches(lens, scans, deltas):
+    """A decoded token is a stretch of its own, so what counts is stretches and what the scan would take, not the longest span alone:
+    all spans by stretches, the long ones beside the scan for the others, or the scan."""
+    table = _Table()
     ctx = _Ctx(lens)
     assert table._scans_by_chunks(torch.bfloat16, ctx, 12, 128, 128, constant=True) == scans
     assert table._delta_by_chunks(torch.bfloat16, ctx, sum(lens), 24, 64) == deltas
-    assert not table._scans_by_chunks(torch.float32, ctx, 12, 128, 128)
+    assert not table._scans_by_chunks(torch.float32, ctx, 12, 128, 128) and not table._scans_by_chunks(torch.bfloat16, ctx, 12, 96, 128)
     short = [n for n in lens if n < 128]
-    assert table._parting(ctx) == (128, max(short, default=0))
-    assert table._long_spans(ctx) == (max(short, default=0), sum(short), len(short), sum(-(-n // 64) for n in lens if n >= 128))
+    count = lambda spans: sum(-(-n // 64) for n in spans)
+    assert table._long_spans(ctx) == (max(short, default=0), sum(short), len(short), count(short), count(n for n in lens if n >= 128))
+
+
+def test_very_many_states_beside_the_shortest_long_span():
+    table = _Table()
+    for lens, way in (((128,) + (1,) * 63, NONE), ((192,) + (1,) * 63, (128, 1)), ((128,) + (1,) * 31, (128, 1))):
+        assert table._scans_by_chunks(torch.bfloat16, _Ctx(lens), 28, 128, 128) == way
 
 
 def test_a_constant_decay_with_small_keys_and_very_many_stretches_stays_with_the_scan():
     table = _Table()
     for lens, way in (((128,) * 32, False), ((256,) * 16, True), ((128,) * 16, True)):
-        assert table._scans_by_chunks(torch.bfloat16, _Ctx(lens), 28, 64, 128, constant=True) == way
+        assert bool(table._scans_by_chunks(torch.bfloat16, _Ctx(lens), 28, 64, 128, constant=True)) == way
         assert table._scans_by_chunks(torch.bfloat16, _Ctx(lens), 28, 64, 128)
 
 
