@@ -300,7 +300,6 @@ __global__ void __launch_bounds__(256) latent_merge_kernel(const float* __restri
                                                            __nv_bfloat16* __restrict__ out, int total_rows, int heads,
                                                            int rank, int splits, const float* __restrict__ gate) {
   __shared__ float w_s[kMaxSplits];
-  __shared__ bool written_s[kMaxSplits];
   __shared__ float inv_s;
   const int row = blockIdx.x, c = threadIdx.x;
   if (c < 32) {                                                        // one warp: weights of the parts and the denominator
@@ -319,10 +318,7 @@ __global__ void __launch_bounds__(256) latent_merge_kernel(const float* __restri
     for (int i = 0; i < kMaxSplits / 32; ++i) {
       const int s = c + 32 * i;
       const float w = (ml[i].x == -INFINITY || m == -INFINITY) ? 0.0f : exp2f(ml[i].x - m);
-      if (s < splits) {
-        w_s[s] = w;
-        written_s[s] = !(ml[i].y < 0.0f);                                // (a denominator that is not a number was written)
-      }
+      if (s < splits) w_s[s] = ml[i].y < 0.0f ? -1.0f : w;
       l = fmaf(ml[i].y, w, l);
     }
     l = warp_sum(l);
@@ -335,7 +331,7 @@ __global__ void __launch_bounds__(256) latent_merge_kernel(const float* __restri
   const size_t step = (size_t)total_rows * rank;
   float acc = 0.0f;
   int s = 0;
-  auto part = [&](int i) { return written_s[i] ? po[(size_t)i * step] : 0.0f; };
+  auto part = [&](int i) { return w_s[i] >= 0.0f ? po[(size_t)i * step] : 0.0f; };       // (0 times a weight that is no number is none)
   for (; s + 4 <= splits; s += 4) {
     const float a0 = part(s), a1 = part(s + 1), a2 = part(s + 2), a3 = part(s + 3);
     acc = fmaf(a0, w_s[s], acc);
