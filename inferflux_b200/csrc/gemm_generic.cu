@@ -1,8 +1,8 @@
 // C[M, N] = A[M, K] . W[N, K]^T (+ bias[N]) on the CUDA cores, accumulating in
 // float32 with one fused multiply-add per product, k ascending.
 //
-// This is the matrix product of the true 32-bit path (no tensor cores, no reduced
-// precision mode) and it takes every M, N and K.  The additions that make one
+// This is the matrix product of the 32-bit path (its large products run in gemm_f32_split.cu)
+// and it takes every M, N and K.  The additions that make one
 // output element happen in an order that depends on K alone, so a row's result is
 // bit-for-bit the same whatever other rows share the launch.
 //

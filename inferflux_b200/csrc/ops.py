@@ -173,12 +173,13 @@ class CudaKernels:
                    "ifx_moe_stream_slices", "ifx_chunk_scan_supports", "ifx_chunk_decay_scan", "ifx_chunk_wkv_scan", "ifx_wkv_norm",
                    "ifx_latent_decode", "ifx_latent_decode_supports", "ifx_latent_decode_stretch",
                    "ifx_latent_prompt", "ifx_latent_prompt_supports", "ifx_delta_chunks_supports", "ifx_delta_chunks_scan",
-                   "ifx_attention_prefill_tcgen05_parts"):
+                   "ifx_attention_prefill_tcgen05_parts", "ifx_gemm_f32_split", "ifx_gemm_f32_split_launches"):
             getattr(self.lib, fn).restype = ctypes.c_int
         self.lib.ifx_delta_rule_scratch_floats.restype = ctypes.c_longlong
         self.lib.ifx_chunk_scan_scratch_floats.restype = ctypes.c_longlong
         self.lib.ifx_delta_chunks_scratch_floats.restype = ctypes.c_longlong
         self.lib.ifx_attention_prefill_tcgen05_parts_bytes.restype = ctypes.c_longlong
+        self.lib.ifx_gemm_f32_split_scratch.restype = ctypes.c_longlong
         # long spans of a bfloat16 run's recurrences by stretches of 64 tokens (0: token after token, for comparisons)
         self.chunk_scans = os.environ.get("INFERFLUX_B200_CHUNK_SCANS", "1") != "0"
         self.lib.ifx_sample_scratch_bytes.restype = ctypes.c_longlong
@@ -364,7 +365,7 @@ class CudaKernels:
 
     def linear(self, a, w, bias=None, out_dtype=None, allow_partial=False):
         """out[T, N] = a[T, K] . w[N, K]^T (+ bias), float32 accumulation.  float32 runs use
-        the CUDA-core product.  bfloat16 runs with up to 256 rows use the tcgen05 weight-streaming
+        the CUDA-core product, or operands in parts on the tensor cores (`float32_by_parts`).  bfloat16 runs with up to 256 rows use the tcgen05 weight-streaming
         kernel; with `allow_partial` a narrow product is split over K and comes back as a
         PartialSum for a consumer that adds the slices itself.  More rows go to cuBLAS."""
         rows = a if isinstance(a, ScaledRows) else None
@@ -385,6 +386,13 @@ class CudaKernels:
         if a.dtype == torch.float32:
             _need(out_dtype == torch.float32, "linear: a float32 product gives float32")
             out = torch.empty(T, N, dtype=out_dtype, device=a.device)
+            if self.float32_by_parts(N, K) and (a.data_ptr() | w.data_ptr()) % 16 == 0:
+                room = self.lib.ifx_gemm_f32_split_scratch(T, N, K)
+                scratch = torch.empty(room, dtype=torch.uint8, device=a.device)
+                _check(self.lib.ifx_gemm_f32_split(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), T, N, K, _ptr(scratch), _LL(room),
+                                                   _ptr(self.error_flag), _stream()), "gemm (float32 by parts)")
+                self.launches += self.lib.ifx_gemm_f32_split_launches(T, N, K)
+                return out
             _check(self.lib.ifx_gemm_generic(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), T, N, K, 0, 0, _stream()),
                    "gemm (float32)")
             self.launches += 1
@@ -408,6 +416,15 @@ class CudaKernels:
         if bias is not None:
             out += bias.to(out.dtype)
         return out
+
+    @staticmethod
+    def float32_by_parts(n, k):
+        """Whether a float32 product runs on the tensor cores, its operands cut into three bfloat16 numbers each
+        (csrc/gemm_f32_split.cu).  By the weight's sizes alone: a row's bits must not depend on how many there are.  Parts
+        against the chain of multiply-adds, us, 1 / 16 / 100 / 512 rows: 1,536 x 1,368 17 17 22 37 against 21 21 37 74;
+        2,048 x 1,024 17 17 22 39 against 16 17 28 67; 4,096 x 512 17 16 22 38 against 10 10 22 60; 1,024 x 1,024
+        21 17 22 26 against 15 16 19 39; 256 x 8,192 18 18 25 37 against 96 98 123 123."""
+        return k % 8 == 0 and k >= 1280 and n * k >= 1 << 21
 
     # The many-rows tcgen05 product with SiLU(gate)*up in its epilogue against cuBLAS followed by the activation
     # kernel, measured on a B200 (us a layer, 256 / 512 / 2,048 rows): Qwen2.5-1.5B sizes 21 vs 27, 31 vs 37, 94 vs 110;

@@ -1,0 +1,70 @@
+"""The float32 product on the tensor cores (operands in three bfloat16 parts) at its edges: rows around its tiles of tokens and
+the blocks of rows worked on at a time, columns and K that fill no tile, K whole and in slices."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def operands(M, N, K, seed=0):
+    g = torch.Generator().manual_seed(M * 7 + N + K + seed)
+    return tuple(torch.randn(n, generator=g).to(DEV) for n in ((M, K), (N, K), (N,)))
+
+
+def bound(a, w):
+    """Products left out: three below 2^-24 of one each.  A chunk of 64 k: 24 additions into its accumulator that may cut off up
+    to 2^-22 each (aligned products, then the sum).  The chunks' and slices' rounded additions: 2^-24 each."""
+    K = a.shape[1]
+    return (3 * 2.0 ** -24 + 24 * 2.0 ** -22 + (K / 64 + 150) * 2.0 ** -24) * (a.double().abs() @ w.double().abs().t()) + 1e-30
+
+
+# 1,700 columns: slices of K; 19,000: 149 tiles of columns, K whole
+@pytest.mark.parametrize("M,N,K", [(1, 1700, 1288), (16, 1700, 1280), (17, 1699, 1344), (33, 1700, 4104), (64, 19000, 1280),
+                                   (65, 18951, 1288), (127, 1700, 1288), (129, 1700, 1288), (333, 19000, 1288), (1030, 1700, 1288),
+                                   (2, 70, 30008)])
+def test_against_64_bits(cuda_kernels, M, N, K):
+    assert cuda_kernels.float32_by_parts(N, K)
+    a, w, bias = operands(M, N, K)
+    want, chain = a.double() @ w.double().t(), cuda_kernels.linear_generic(a, w)
+    for b in (None, bias):
+        got = cuda_kernels.linear(a, w, b).double()
+        exact = want if b is None else want + b.double()
+        assert bool(((got - exact).abs() <= bound(a, w) + 2.0 ** -24 * exact.abs()).all())
+    assert float((cuda_kernels.linear(a, w).double() - want).norm()) <= float((chain.double() - want).norm())
+    cuda_kernels.check_errors()
+
+
+@pytest.mark.parametrize("N,K", [(1700, 1288), (19000, 1280)])
+def test_rows_do_not_depend_on_their_number(cuda_kernels, N, K):
+    a, w, bias = operands(1100, N, K)
+    whole = cuda_kernels.linear(a, w, bias)
+    for n in (1, 16, 40, 97, 200, 1024):
+        assert torch.equal(cuda_kernels.linear(a[:n].contiguous(), w, bias), whole[:n])
+
+
+@pytest.mark.parametrize("N", [1700, 19000])
+def test_not_finite_tiny_and_huge(cuda_kernels, N):
+    """Rows whose parts leave bfloat16's range, or are no numbers, come out as from the chain of multiply-adds; the others as ever."""
+    a, w, _ = operands(40, N, 1288, seed=1)
+    clean = cuda_kernels.linear(a, w)
+    a[3, 7], a[4, 1287], a[5, 0] = float("inf"), float("nan"), -float("inf")
+    w[11, 3] = float("inf")
+    a[6] *= 2.0 ** -118
+    a[7] *= 2.0 ** 122                                        # sums beyond the largest float32 in some columns
+    a[8] = 0.0
+    a[9, :], a[9, 2] = 0.0, 3.4e38
+    got, chain = cuda_kernels.linear(a, w), cuda_kernels.linear_generic(a, w)
+    for r in (3, 4, 5, 6, 8):
+        assert torch.equal(got[r].nan_to_num(nan=7.0), chain[r].nan_to_num(nan=7.0)) and torch.equal(got[r].isnan(), chain[r].isnan())
+    # a sum that goes beyond the largest float32 and comes back within a chunk may be finite here alone: then it is the right one
+    want, most = a.double() @ w.double().t(), bound(a, w)
+    for r in (7, 9):
+        f = got[r].isfinite()
+        assert bool(f[chain[r].isfinite()].all()) and torch.equal(got[r][~f].nan_to_num(nan=7.0), chain[r][~f].nan_to_num(nan=7.0))
+        assert bool(f.any()) and bool(((got[r].double() - want[r]).abs() <= most[r])[f].all())
+    keep = torch.ones(40, dtype=torch.bool, device=DEV)
+    keep[3:10] = False
+    cols = torch.arange(N, device=DEV) != 11
+    assert torch.equal(got[keep][:, cols], clean[keep][:, cols])
+    assert not bool(got[keep][:, 11].isfinite().any())
