@@ -12,20 +12,21 @@
 //   moe_down      out[t] = sum over the token's choices, in their order, of weight * (W_down[e] act[p]), or
 //                 weight * h[t] for an expert without weights
 //
-// In bfloat16 the work goes one of three ways (CudaKernels.moe_kernels has the rule and its measurements): the kernels of this file
-// for a few tokens, the stream of moe_stream_tcgen05.cu up to a few hundred pairs, whole tiles above.  The tiles sort their
-// (token, choice) pairs by expert first and multiply on the tensor cores (the grouped modes of gemm_tcgen05.cu):
+// In bfloat16 the work goes one of two ways (the rule and its measurements stand at CudaKernels.moe_kernels): the kernels of this
+// file for a little work, sorted rows above.  These sort the (token, choice) pairs by expert first and multiply on the tensor
+// cores (gemm_pair_tcgen05.cu):
 //
-//   moe_sort      every expert's pairs get a stretch of rows that starts on a multiple of 128; per row the pair it
-//                 holds (or -1) and the pair's weight (or 0); per 128-row tile its expert (or -1); per pair its row
-//   moe_gather    rows[r] = h[token of the pair in row r], zeros for a row without a pair
-//   moe_combine   out[t] = sum over the token's choices, in their order, of y[row of the pair] (already weighted), or
+//   moe_sort      every expert's pairs get a stretch of rows, one behind the other, cut into tiles of up to 256 rows of about the
+//                 same size; per pair its row (or -1: an expert without weights)
+//   moe_gather    rows[row of the pair] = h[token]
+//   moe_combine   out[t] = sum over the token's choices, in their order, of weight * y[row of the pair], or
 //                 weight * h[t] for an expert without weights
 //
 // The kernels below the sort are those of the float32 run and of steps with few tokens: a warp makes one output number as a dot
 // product (lanes stride the inner size, then a shuffle tree), so every sum has an order that depends on the sizes
 // alone.  Expert weights are stacked: up [experts, ff, width], down [experts, width, ff].
 #include "common.cuh"
+#include "moe_items.cuh"
 
 namespace ifx {
 
@@ -318,72 +319,117 @@ __global__ void moe_down_kernel(const T* __restrict__ h, const T* __restrict__ a
   }
 }
 
-// One block.  counts/offset/cursor live in shared memory: experts <= kMaxRouterOutputs.
-__global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ ids, const float* __restrict__ weights,
-                                                        int pairs, int experts, int* __restrict__ row_pair,
-                                                        float* __restrict__ row_scale, int* __restrict__ tile_group,
-                                                        int* __restrict__ pair_row, int rows_cap) {
-  __shared__ int count_s[kMaxRouterOutputs], offset_s[kMaxRouterOutputs], cursor_s[kMaxRouterOutputs];
-  for (int e = threadIdx.x; e < experts; e += blockDim.x) count_s[e] = cursor_s[e] = 0;
-  for (int r = threadIdx.x; r < rows_cap; r += blockDim.x) {
-    row_pair[r] = -1;
-    row_scale[r] = 0.0f;
+// One block.  Pairs of one expert inside a warp draw their places with one addition (an addition a pair: 8,192 pairs of 16 experts
+// 10.7 us, so 5.0); experts' stretches are found by a scan over all of them (one thread walking 1,024 experts: 20 us more).
+__global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ ids, int pairs, int experts, PairItem* __restrict__ items,
+                                                        int* __restrict__ pair_row) {
+  static_assert(kMaxRouterOutputs == 1024, "a thread an expert");
+  __shared__ int count_s[kMaxRouterOutputs], row_s[kMaxRouterOutputs], warp_rows[32], warp_items[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  count_s[threadIdx.x] = 0;
+  __syncthreads();
+  pdl_launch_dependents();
+  pdl_wait();
+  for (int p0 = 0; p0 < pairs; p0 += 1024) {
+    const int p = p0 + threadIdx.x;
+    int e = p < pairs ? ids[p] : -1;
+    if (e < 0 || e >= experts) e = -1;
+    const unsigned same = __match_any_sync(0xffffffffu, e);
+    int base = 0;
+    if (e >= 0 && lane == __ffs(same) - 1) base = atomicAdd(&count_s[e], __popc(same));
+    base = __shfl_sync(0xffffffffu, base, __ffs(same) - 1);
+    // which row inside the stretch does not change a row's result
+    if (p < pairs) pair_row[p] = e >= 0 ? base + __popc(same & ((1u << lane) - 1)) : -1;
   }
   __syncthreads();
-  for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-    const int e = ids[p];
-    if (e >= 0 && e < experts) atomicAdd(&count_s[e], 1);
+  const int count = count_s[threadIdx.x], tiles = (count + kItemTokens - 1) / kItemTokens;
+  int rows_to = count, items_to = tiles;                     // sums up to and with this expert
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int r = __shfl_up_sync(0xffffffffu, rows_to, o), i = __shfl_up_sync(0xffffffffu, items_to, o);
+    if (lane >= o) rows_to += r, items_to += i;
   }
+  if (lane == 31) warp_rows[warp] = rows_to, warp_items[warp] = items_to;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int row = 0;
-    for (int e = 0; e < experts; ++e) {
-      offset_s[e] = row;
-      const int tiles = (count_s[e] + 127) / 128;
-      for (int i = 0; i < tiles; ++i) tile_group[row / 128 + i] = e;
-      row += tiles * 128;
-    }
-    for (int tile = row / 128; tile < rows_cap / 128; ++tile) tile_group[tile] = -1;
+  int rows_before = 0, items_before = 0;
+  for (int w = 0; w < warp; ++w) rows_before += warp_rows[w], items_before += warp_items[w];
+  const int first = rows_before + rows_to - count;
+  row_s[threadIdx.x] = first;
+  int at = 1 + items_before + items_to - tiles, begin = 0;
+  for (int i = 0; i < tiles; ++i) {                          // the tiles' sizes differ by one at most
+    const int n = (count - begin + tiles - i - 1) / (tiles - i);
+    items[at + i] = PairItem{(int)threadIdx.x, first + begin, n, (n + 31) / 32 * 32};
+    begin += n;
   }
+  if (threadIdx.x == 1023) items[0] = PairItem{items_before + items_to, 0, 0, 0};
   __syncthreads();
-  for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-    const int e = ids[p];
-    int row = -1;
-    if (e >= 0 && e < experts) {
-      row = offset_s[e] + atomicAdd(&cursor_s[e], 1);      // which row inside the stretch does not change a row's result
-      row_pair[row] = p;
-      row_scale[row] = weights[p];
-    }
-    pair_row[p] = row;
+  for (int p = threadIdx.x; p < pairs; p += 1024) {
+    const int place = pair_row[p];
+    if (place >= 0) pair_row[p] = row_s[ids[p]] + place;
   }
 }
 
-__global__ void moe_gather_kernel(const __nv_bfloat16* __restrict__ h, const int* __restrict__ row_pair,
+// A block a token: its row is read once.
+__global__ void moe_gather_kernel(const __nv_bfloat16* __restrict__ h, const int* __restrict__ pair_row,
                                   __nv_bfloat16* __restrict__ rows, int top, int width8) {
-  const int r = blockIdx.x;
-  const int p = row_pair[r];
-  const uint4* src = p >= 0 ? reinterpret_cast<const uint4*>(h) + (size_t)(p / top) * width8 : nullptr;
-  uint4* dst = reinterpret_cast<uint4*>(rows) + (size_t)r * width8;
-  for (int i = threadIdx.x; i < width8; i += blockDim.x) dst[i] = src ? src[i] : make_uint4(0u, 0u, 0u, 0u);
+  pdl_launch_dependents();
+  pdl_wait();
+  const uint4* src = reinterpret_cast<const uint4*>(h) + (size_t)blockIdx.x * width8;
+  const int* row = pair_row + (size_t)blockIdx.x * top;
+  for (int i = threadIdx.x; i < width8; i += blockDim.x) {
+    const uint4 v = src[i];
+    for (int k = 0; k < top; ++k)
+      if (row[k] >= 0) reinterpret_cast<uint4*>(rows)[(size_t)row[k] * width8 + i] = v;
+  }
 }
 
+// Eight columns a thread: two loads of 16 bytes a choice, all choices' in flight.
 template <typename TO>
 __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ h, const float* __restrict__ y,
-                                   const int* __restrict__ ids, const float* __restrict__ weights,
-                                   const int* __restrict__ pair_row, TO* __restrict__ out, int top, int experts,
-                                   int width) {
+                                   const float* __restrict__ weights, const int* __restrict__ pair_row, TO* __restrict__ out,
+                                   int top, int width) {
+  pdl_wait();
   const int t = blockIdx.x;
-  for (int c = threadIdx.x; c < width; c += blockDim.x) {
-    float acc = 0.0f;
+  for (int c = threadIdx.x * 8; c < width; c += blockDim.x * 8) {
+    float acc[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] = 0.0f;
+#pragma unroll 4
     for (int k = 0; k < top; ++k) {
-      const int p = t * top + k;
-      const int row = pair_row[p];
-      if (row >= 0) acc += y[(size_t)row * width + c];
-      else acc = fmaf(weights[p], to_f32(h[(size_t)t * width + c]), acc);
+      const int p = t * top + k, row = pair_row[p];
+      const float w = weights[p];
+      float v[8];
+      if (row >= 0) {
+        const float4* src = reinterpret_cast<const float4*>(y + (size_t)row * width + c);
+        reinterpret_cast<float4*>(v)[0] = src[0];
+        reinterpret_cast<float4*>(v)[1] = src[1];
+      } else {
+        const uint4 raw = *reinterpret_cast<const uint4*>(h + (size_t)t * width + c);
+        const __nv_bfloat16* b = reinterpret_cast<const __nv_bfloat16*>(&raw);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = to_f32(b[i]);
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] = fmaf(w, v[i], acc[i]);
     }
-    out[(size_t)t * width + c] = from_f32<TO>(acc);
+    TO* dst = out + (size_t)t * width + c;
+    if constexpr (sizeof(TO) == 4) {
+      reinterpret_cast<float4*>(dst)[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+      reinterpret_cast<float4*>(dst)[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+    } else {
+      __nv_bfloat162 b[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) b[i] = __floats2bfloat162_rn(acc[2 * i], acc[2 * i + 1]);
+      *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<uint4*>(b);
+    }
   }
 }
+
+int gemm_pair(int mode, const void* tokens, const void* W, void* out, int rows, int N, int K, int stack, const PairItem* items,
+              int most_items, float limit, float slope, float offset, int* error_flag, cudaStream_t stream);
+
+static long long moe_aligned(long long bytes) { return (bytes + 255) / 256 * 256; }
+static int moe_most_items(int pairs, int experts) { return pairs / kItemTokens + (experts < pairs ? experts : pairs); }
 
 }  // namespace ifx
 
@@ -468,41 +514,49 @@ int ifx_moe_experts_glu(const void* h, const void* w_up, const void* w_down, con
   return 0;
 }
 
-// Rows that the sorted form needs at most: every expert's stretch is rounded up to whole tiles of 128.
-int ifx_moe_sorted_rows(int pairs, int experts) {
-  return (pairs + experts * 127 + 127) / 128 * 128;
+// Bytes of scratch of ifx_moe_sorted: the list of tiles, the pairs' rows, gathered rows, activations, the experts' outputs.
+long long ifx_moe_sorted_scratch(int T, int top, int experts, int width, int ff) {
+  const long long pairs = (long long)T * top;
+  return moe_aligned((1 + moe_most_items((int)pairs, experts)) * (long long)sizeof(PairItem)) + moe_aligned(pairs * 4) +
+         moe_aligned(pairs * width * 2) + moe_aligned(pairs * ff * 2) + pairs * width * 4;
 }
 
-int ifx_moe_sort(const int* ids, const float* weights, int pairs, int experts, int* row_pair, float* row_scale,
-                 int* tile_group, int* pair_row, int rows_cap, cudaStream_t stream) {
-  if (pairs <= 0) return 0;
-  if (experts <= 0 || experts > kMaxRouterOutputs || rows_cap % 128 || rows_cap < ifx_moe_sorted_rows(pairs, experts))
-    return IFX_E_BADARG;
-  moe_sort_kernel<<<1, 1024, 0, stream>>>(ids, weights, pairs, experts, row_pair, row_scale, tile_group, pair_row, rows_cap);
-  IFX_CHECK_LAUNCH();
-  return 0;
-}
-
-int ifx_moe_gather(const void* h, const int* row_pair, void* rows, int rows_cap, int top, int width, cudaStream_t stream) {
-  if (rows_cap <= 0) return 0;
-  if (width % 8 || (uintptr_t)h % 16 || (uintptr_t)rows % 16) return IFX_E_ALIGN;
-  moe_gather_kernel<<<rows_cap, 128, 0, stream>>>((const __nv_bfloat16*)h, row_pair, (__nv_bfloat16*)rows, top, width / 8);
-  IFX_CHECK_LAUNCH();
-  return 0;
-}
-
-int ifx_moe_combine(const void* h, const float* y, const int* ids, const float* weights, const int* pair_row, void* out,
-                    int T, int top, int experts, int width, int out_dtype, cudaStream_t stream) {
+// The experts of a bfloat16 step over sorted rows.  h [T, width]; w_up [experts, ff, width] (glu: [experts, 2 ff, width], gate rows
+// above up rows); w_down [experts, width, ff]; ids, weights [T, top]; out [T, width] in out_dtype.  width and ff multiples of 8;
+// matrices, h, out and scratch on 16-byte boundaries.
+int ifx_moe_sorted(const void* h, const void* w_up, const void* w_down, const int* ids, const float* weights, void* out, int T, int top,
+                   int experts, int width, int ff, int out_dtype, int glu, float limit, float slope, float offset, void* scratch,
+                   long long scratch_bytes, int* error_flag, cudaStream_t stream) {
   if (T <= 0) return 0;
+  if (top <= 0 || experts <= 0 || experts > kMaxRouterOutputs || width <= 0 || ff <= 0 || width % 8 || ff % 8 || error_flag == nullptr)
+    return IFX_E_BADARG;
+  if (out_dtype != IFX_DT_F32 && out_dtype != IFX_DT_BF16) return IFX_E_DTYPE;
+  if (((uintptr_t)h | (uintptr_t)w_up | (uintptr_t)w_down | (uintptr_t)out | (uintptr_t)scratch) % 16) return IFX_E_ALIGN;
+  if ((long long)T * top > 0x7fffffffll || scratch_bytes < ifx_moe_sorted_scratch(T, top, experts, width, ff)) return IFX_E_TOOBIG;
+  const int pairs = T * top, most = moe_most_items(pairs, experts);
+  unsigned char* at = reinterpret_cast<unsigned char*>(scratch);
+  auto take = [&](long long bytes) {
+    unsigned char* p = at;
+    at += moe_aligned(bytes);
+    return p;
+  };
+  PairItem* items = reinterpret_cast<PairItem*>(take((1 + most) * (long long)sizeof(PairItem)));
+  int* pair_row = reinterpret_cast<int*>(take(pairs * 4ll));
+  __nv_bfloat16* rows = reinterpret_cast<__nv_bfloat16*>(take((long long)pairs * width * 2));
+  __nv_bfloat16* act = reinterpret_cast<__nv_bfloat16*>(take((long long)pairs * ff * 2));
+  float* y = reinterpret_cast<float*>(at);
+  int rc = launch_pdl(moe_sort_kernel, dim3(1), dim3(1024), 0, stream, 1, ids, pairs, experts, items, pair_row);
+  if (rc) return rc;
+  rc = launch_pdl(moe_gather_kernel, dim3(T), dim3(192), 0, stream, 1, (const __nv_bfloat16*)h, pair_row, rows, top, width / 8);
+  if (rc) return rc;
+  rc = gemm_pair(glu ? 2 : 0, rows, w_up, act, pairs, ff, width, experts, items, most, limit, slope, offset, error_flag, stream);
+  if (rc) return rc;
+  rc = gemm_pair(1, act, w_down, y, pairs, width, ff, experts, items, most, 0.0f, 0.0f, 0.0f, error_flag, stream);
+  if (rc) return rc;
+  const __nv_bfloat16* hb = reinterpret_cast<const __nv_bfloat16*>(h);
   if (out_dtype == IFX_DT_BF16)
-    moe_combine_kernel<__nv_bfloat16><<<T, 256, 0, stream>>>((const __nv_bfloat16*)h, y, ids, weights, pair_row,
-                                                             (__nv_bfloat16*)out, top, experts, width);
-  else if (out_dtype == IFX_DT_F32)
-    moe_combine_kernel<float><<<T, 256, 0, stream>>>((const __nv_bfloat16*)h, y, ids, weights, pair_row, (float*)out, top,
-                                                     experts, width);
-  else return IFX_E_DTYPE;
-  IFX_CHECK_LAUNCH();
-  return 0;
+    return launch_pdl(moe_combine_kernel<__nv_bfloat16>, dim3(T), dim3(192), 0, stream, 1, hb, y, weights, pair_row, (__nv_bfloat16*)out, top, width);
+  return launch_pdl(moe_combine_kernel<float>, dim3(T), dim3(192), 0, stream, 1, hb, y, weights, pair_row, (float*)out, top, width);
 }
 
 }  // extern "C"

@@ -159,18 +159,18 @@ class CudaKernels:
                    "ifx_latent_attention_mma_supports", "ifx_gemm_cublas_bf16_batched", "ifx_gemm_skinny_act",
                    "ifx_attention_generic_ex", "ifx_norm_rope_append", "ifx_token_shift_mix", "ifx_cast_rows",
                    "ifx_wkv_scan", "ifx_moe_route", "ifx_moe_experts", "ifx_tanh_rows",
-                   "ifx_attention_prefill_bf16_ex", "ifx_attention_decode_bf16_ex", "ifx_moe_sorted_rows", "ifx_moe_sort",
-                   "ifx_moe_gather", "ifx_moe_combine", "ifx_gemm_tcgen05_grouped", "ifx_attention_prefill_tcgen05_ex",
+                   "ifx_attention_prefill_bf16_ex", "ifx_attention_decode_bf16_ex", "ifx_moe_sorted",
+                   "ifx_attention_prefill_tcgen05_ex",
                    "ifx_groupnorm_stream", "ifx_residual_add_scaled", "ifx_gelu_mul_table", "ifx_embed_scaled", "ifx_scale_f32",
                    "ifx_delta_rule_scan", "ifx_latent_rope_append", "ifx_latent_attention_generic_rot", "ifx_moe_route_ex",
-                   "ifx_moe_experts_ex", "ifx_gemm_tcgen05_grouped_glu", "ifx_latent_attention_mma_rot", "ifx_latent_attention_mma_supports_rot",
-                   "ifx_moe_route_kind", "ifx_moe_experts_glu", "ifx_gemm_tcgen05_grouped_glu_offset", "ifx_norm_rope_append_ex",
+                   "ifx_moe_experts_ex", "ifx_latent_attention_mma_rot", "ifx_latent_attention_mma_supports_rot",
+                   "ifx_moe_route_kind", "ifx_moe_experts_glu", "ifx_norm_rope_append_ex",
                    "ifx_attention_generic_sink", "ifx_short_conv_ex", "ifx_decay_scan", "ifx_decay_scan_split", "ifx_bigram_add",
                    "ifx_rmsnorm_pair", "ifx_gate_mul", "ifx_gated_groupnorm", "ifx_pair_combine", "ifx_residual_add_vectors",
                    "ifx_attention_prefill_tcgen05_sink", "ifx_attention_prefill_bf16_sink", "ifx_attention_decode_bf16_sink",
                    "ifx_norm_of_sum", "ifx_row_norm_rope_append", "ifx_rotate_rows", "ifx_gated_scan", "ifx_decay_scan_rate",
-                   "ifx_geglu_mul", "ifx_gemm_skinny_geglu", "ifx_gemm_tcgen05_geglu", "ifx_relu2", "ifx_silu_columns", "ifx_moe_stream",
-                   "ifx_moe_stream_slices", "ifx_chunk_scan_supports", "ifx_chunk_decay_scan", "ifx_chunk_wkv_scan", "ifx_wkv_norm",
+                   "ifx_geglu_mul", "ifx_gemm_skinny_geglu", "ifx_gemm_tcgen05_geglu", "ifx_relu2", "ifx_silu_columns",
+                   "ifx_chunk_scan_supports", "ifx_chunk_decay_scan", "ifx_chunk_wkv_scan", "ifx_wkv_norm",
                    "ifx_latent_decode", "ifx_latent_decode_supports", "ifx_latent_decode_stretch",
                    "ifx_latent_prompt", "ifx_latent_prompt_supports", "ifx_delta_chunks_supports", "ifx_delta_chunks_scan",
                    "ifx_attention_prefill_tcgen05_parts", "ifx_gemm_f32_split", "ifx_gemm_f32_split_launches"):
@@ -180,6 +180,7 @@ class CudaKernels:
         self.lib.ifx_delta_chunks_scratch_floats.restype = ctypes.c_longlong
         self.lib.ifx_attention_prefill_tcgen05_parts_bytes.restype = ctypes.c_longlong
         self.lib.ifx_gemm_f32_split_scratch.restype = ctypes.c_longlong
+        self.lib.ifx_moe_sorted_scratch.restype = ctypes.c_longlong
         # long spans of a bfloat16 run's recurrences by stretches of 64 tokens (0: token after token, for comparisons)
         self.chunk_scans = os.environ.get("INFERFLUX_B200_CHUNK_SCANS", "1") != "0"
         self.lib.ifx_sample_scratch_bytes.restype = ctypes.c_longlong
@@ -1679,10 +1680,9 @@ class CudaKernels:
                   and w_down.is_contiguous() and tuple(w_up.shape) == (experts, 2 * ff, width)
                   and tuple(w_down.shape) == (experts, width, ff), "moe_experts: stacked expert weights in the activations' dtype")
             if h.dtype == torch.bfloat16:
-                way = self.moe_kernels(T * top, int(experts), width, ff, True)
-                if way != "tokens" and self._moe_on_tensor_cores(h, w_up, w_down, ff, width):
-                    return (self._moe_experts_tiles if way == "tiles" else self._moe_experts_stream)(
-                        h, w_up, w_down, ids, weights, experts, out_dtype, glu=glu)
+                if (self._moe_by_sorted_rows(T * top, int(experts), width, ff, True)
+                        and self._moe_on_tensor_cores(h, w_up, w_down, ff, width)):
+                    return self._moe_experts_tiles(h, w_up, w_down, ids, weights, experts, out_dtype, glu=glu)
             act = torch.empty(T * top, ff, dtype=h.dtype, device=h.device)
             out = torch.empty(T, width, dtype=out_dtype, device=h.device)
             _check(self.lib.ifx_moe_experts_glu(_ptr(h), _ptr(w_up), _ptr(w_down), _ptr(ids), _ptr(weights), _ptr(act), _ptr(out),
@@ -1696,10 +1696,9 @@ class CudaKernels:
               and w_down.is_contiguous() and tuple(w_up.shape) == (experts, ff, width) and tuple(w_down.shape) == (experts, width, ff))),
               "moe_experts: stacked expert weights in the activations' dtype")
         if experts and h.dtype == torch.bfloat16:
-            way = self.moe_kernels(T * top, int(experts), width, ff, False)
-            if way != "tokens" and self._moe_on_tensor_cores(h, w_up, w_down, ff, width):
-                return (self._moe_experts_tiles if way == "tiles" else self._moe_experts_stream)(
-                    h, w_up, w_down, ids, weights, experts, out_dtype)
+            if (self._moe_by_sorted_rows(T * top, int(experts), width, ff, False)
+                    and self._moe_on_tensor_cores(h, w_up, w_down, ff, width)):
+                return self._moe_experts_tiles(h, w_up, w_down, ids, weights, experts, out_dtype)
         act = torch.empty(T * top, ff, dtype=h.dtype, device=h.device)
         out = torch.empty(T, width, dtype=out_dtype, device=h.device)
         _check(self.lib.ifx_moe_experts(_ptr(h), _ptr(w_up if experts else None), _ptr(w_down if experts else None), _ptr(ids),
@@ -1708,26 +1707,24 @@ class CudaKernels:
         self.launches += 2 if experts else 1
         return out
 
-    # Which kernels make the experts of a bfloat16 step, by the number of (token, choice) pairs.  Measured on a B200 with every
-    # expert's weights in HBM (us; per token / every chosen expert's weights once / sorted 128-row tiles):
-    #    16 experts, 1,536 x 2,240 gated, four a token   1 token 71 / 48 / 69, 8: 122 / 93 / 111, 24: 255 / 95 / 118, 64: 560 / 114 / 116
-    #     8 experts, the same, two a token               1 token 46 / 46 / 62, 16: 108 / 52 / 87, 64: 300 / 60 / 87
-    #    32 experts, the same, four a token              8 tokens 132 / 128 / 150, 24: 279 / 169 / 177, 64: 585 / 167 / 185
-    #    64 experts, 2,048 x 1,408 gated, six a token    1 token 83 / 54 / 99, 4: 124 / 118 / 144, 16: 290 / 230 / 251, 48: 610 / 267 / 280
-    #   128 experts, 2,048 x 768 gated, eight a token    4 tokens 88 / 116 / 134, 16: 216 / 249 / 255, 32: 343 / 308 / 329
-    #   256 experts, 2,048 x 1,024 gated, eight a token  1 token 75 / 60 / 110, 8: 196 / 216 / 245, 32: 494 / 572 / 607, 48: 669 / 621 / 710
-    #   256 experts, 3,584 x 1,024, eight a token        1 token 79 / 85 / 153, 16: 364 / 388 / 464, 48: 844 / 724 / 851
-    #    64 experts, 1,536 x 512, four a token           4 tokens 34 / 42 / 65, 16: 58 / 54 / 89, 64: 134 / 62 / 103
-    # (3,584 x 4,736 gated, 16 experts: 1 token 150 / 109 / 110, 8: 514 / 312 / 299, 24: 1,100 / 329 / 323, from L2.)
-    # Per token, where an expert seldom has more than one pair: nothing is read twice then, and the other two have a block for every
-    # tile of an expert all the same; and where the work is a few megabytes, which end before the other two have filled their
-    # pipelines.  Tiles once an expert has a dozen tokens (their rows then are not mostly padding, and the stream's gathering grows), or
-    # once its matrices are large enough to keep every SM at whole tiles.
+    # Which kernels make the experts of a bfloat16 step, by the number of (token, choice) pairs: per token, or, once the work is
+    # MOE_TOKENS_MAX_WORK multiply-adds or there are MOE_STREAM_MAX_PAIRS pairs, over rows sorted by expert, where every chosen
+    # expert's weights are read once.  Measured on a B200, weights of two layers in turn (us, per token / sorted rows):
+    #     4 experts, 2,048 x 2,048, one a token           1 token (8M) 18 / 25, 4 (34M): 22 / 26, 16 (134M): 52 / 28, 64: 140 / 29
+    #     8 experts, 1,536 x 2,240 gated, two a token     1 token (21M) 37 / 30, 2 (41M): 42 / 30, 8: 64 / 39, 32: 169 / 42
+    #    16 experts, the same, one a token                1 token (10M) 20 / 24, 2 (21M): 27 / 28, 4 (41M): 34 / 30, 8: 47 / 41
+    #    16 experts, the same, four a token               1 token (41M) 63 / 31, 4: 81 / 48
+    #    64 experts, 1,536 x 512, four a token            1 token (9M) 19 / 21, 4 (38M): 29 / 26, 8: 44 / 38, 16: 66 / 51
+    #    64 experts, 2,048 x 1,408 gated, six a token     1 token (52M) 73 / 36, 4: 112 / 81
+    #   256 experts, 2,048 x 1,024 gated, eight a token   1 token (50M) 63 / 35, 4: 103 / 84, 16: 281 / 203
+    # (A stream of blocks that each find their expert and its pairs in the step's choices, without a sort, lay between: 44, 80, 46 and
+    # 55, 116 us for the sixteen experts' 1 and 4 tokens, the eight's 32 and the 256's 1 and 4.)
+    # `moe_kernels` tells apart three sizes of step by the pairs an expert has; "stream" and "tiles" are sorted rows alike.
     MOE_TILES_MIN_PAIRS = 192
     MOE_TILES_LARGE_EXPERT = 1 << 23
     MOE_TOKENS_MAX_WORK = 40_000_000
     MOE_STREAM_MAX_PAIRS = 512
-    MOE_MAX_EXPERTS = 1024     # of the stream and the tiles
+    MOE_MAX_EXPERTS = 1024     # of sorted rows
 
     @classmethod
     def moe_kernels(cls, pairs, experts, width, ff, gated):
@@ -1748,56 +1745,28 @@ class CudaKernels:
                 and w_up.data_ptr() % 16 == 0 and w_down.data_ptr() % 16 == 0
                 and os.environ.get("INFERFLUX_B200_MOE_TILES", "1") != "0")
 
+    def _moe_by_sorted_rows(self, pairs, experts, width, ff, gated):
+        way = self.moe_kernels(pairs, experts, width, ff, gated)
+        work = pairs * ff * width * (3 if gated else 2)
+        return way != "tokens" or (experts <= self.MOE_MAX_EXPERTS and work >= self.MOE_TOKENS_MAX_WORK)
+
     def _moe_experts_stream(self, h, w_up, w_down, ids, weights, experts, out_dtype, glu=None):
-        """bfloat16, few tokens: every chosen expert's weights once through the tensor cores (csrc/moe_stream_tcgen05.cu)."""
-        T, width = h.shape
-        top, ff = ids.shape[1], w_up.shape[1] // (2 if glu is not None else 1)
-        sums = int(self.lib.ifx_moe_stream_slices(ff)) * T * top * width           # float32, then the activations in bfloat16
-        room = torch.empty(sums + T * top * ff // 2, dtype=torch.float32, device=h.device)
-        out = torch.empty(T, width, dtype=out_dtype, device=h.device)
-        limit, slope, offset = glu if glu is not None else (0.0, 0.0, 0.0)
-        act = ctypes.c_void_p(room.data_ptr() + 4 * sums)
-        _check(self.lib.ifx_moe_stream(_ptr(h), _ptr(w_up), _ptr(w_down), _ptr(ids), _ptr(weights), act, _ptr(room), _ptr(out),
-                                       T, top, int(experts), width, ff, _DT[out_dtype], int(glu is not None), ctypes.c_float(limit),
-                                       ctypes.c_float(slope), ctypes.c_float(offset), _ptr(self.error_flag), _stream()),
-               "moe experts (stream)")
-        self.launches += 3
-        return out
+        """bfloat16, few tokens: every chosen expert's weights once through the tensor cores, as with many tokens."""
+        return self._moe_experts_tiles(h, w_up, w_down, ids, weights, experts, out_dtype, glu=glu)
 
     def _moe_experts_tiles(self, h, w_up, w_down, ids, weights, experts, out_dtype, glu=None):
-        """bfloat16, many tokens: pairs sorted by expert into stretches of whole 128-row tiles, two grouped tcgen05
-        products (the activation, relu^2 or the gated one of `glu` over tiles of 128 gate rows and their 128 up rows, in
-        the first one's epilogue, the pair's weight in the second's), then the sum per token."""
+        """bfloat16: pairs sorted by expert, two tcgen05 products over the sorted rows by pairs of SMs (the
+        activation, relu^2 or the gated one of `glu`, in the first one's epilogue), then the weighted sum per token."""
         T, width = h.shape
         top, ff = ids.shape[1], w_up.shape[1] // (2 if glu is not None else 1)
-        pairs = T * top
-        cap = int(self.lib.ifx_moe_sorted_rows(pairs, int(experts)))
-        dev = h.device
-        row_pair = torch.empty(cap, dtype=torch.int32, device=dev)
-        row_scale = torch.empty(cap, dtype=torch.float32, device=dev)
-        tile_group = torch.empty(cap // 128, dtype=torch.int32, device=dev)
-        pair_row = torch.empty(pairs, dtype=torch.int32, device=dev)
-        _check(self.lib.ifx_moe_sort(_ptr(ids), _ptr(weights), pairs, int(experts), _ptr(row_pair), _ptr(row_scale),
-                                     _ptr(tile_group), _ptr(pair_row), cap, _stream()), "moe_sort")
-        rows = torch.empty(cap, width, dtype=torch.bfloat16, device=dev)
-        _check(self.lib.ifx_moe_gather(_ptr(h), _ptr(row_pair), _ptr(rows), cap, top, width, _stream()), "moe_gather")
-        act = torch.empty(cap, ff, dtype=torch.bfloat16, device=dev)
-        if glu is not None:
-            _check(self.lib.ifx_gemm_tcgen05_grouped_glu_offset(
-                _ptr(rows), _ptr(w_up), _ptr(act), cap, ff, width, int(experts), _ptr(tile_group), ctypes.c_float(glu[0]),
-                ctypes.c_float(glu[1]), ctypes.c_float(glu[2] if len(glu) > 2 else 1.0), _ptr(self.error_flag), _stream()),
-                "moe experts (gate and up, tiles)")
-        else:
-            _check(self.lib.ifx_gemm_tcgen05_grouped(_ptr(rows), _ptr(w_up), _ptr(act), cap, ff, width, int(experts), ff,
-                                                     _ptr(tile_group), _ptr(None), 2, _ptr(self.error_flag), _stream()),
-                   "moe experts (up, tiles)")
-        y = torch.empty(cap, width, dtype=torch.float32, device=dev)
-        _check(self.lib.ifx_gemm_tcgen05_grouped(_ptr(act), _ptr(w_down), _ptr(y), cap, width, ff, int(experts), width,
-                                                 _ptr(tile_group), _ptr(row_scale), 3, _ptr(self.error_flag), _stream()),
-               "moe experts (down, tiles)")
-        out = torch.empty(T, width, dtype=out_dtype, device=dev)
-        _check(self.lib.ifx_moe_combine(_ptr(h), _ptr(y), _ptr(ids), _ptr(weights), _ptr(pair_row), _ptr(out), T, top,
-                                        int(experts), width, _DT[out_dtype], _stream()), "moe_combine")
+        room = self.lib.ifx_moe_sorted_scratch(T, top, int(experts), width, ff)
+        scratch = torch.empty(room, dtype=torch.uint8, device=h.device)
+        out = torch.empty(T, width, dtype=out_dtype, device=h.device)
+        limit, slope, offset = (glu if len(glu) > 2 else (*glu, 1.0)) if glu is not None else (0.0, 0.0, 0.0)
+        _check(self.lib.ifx_moe_sorted(_ptr(h), _ptr(w_up), _ptr(w_down), _ptr(ids), _ptr(weights), _ptr(out), T, top, int(experts),
+                                       width, ff, _DT[out_dtype], int(glu is not None), ctypes.c_float(limit), ctypes.c_float(slope),
+                                       ctypes.c_float(offset), _ptr(scratch), _LL(room), _ptr(self.error_flag), _stream()),
+               "moe experts (sorted rows)")
         self.launches += 5
         return out
 
