@@ -2,12 +2,14 @@
 // (tcgen05 cta_group::2), operands swapped so that the weight rows are the lanes of tensor memory and the tokens the columns.
 //
 // Token rows lie sorted in stretches, one per matrix of a stack (experts); a device list (PairItem) says which matrix a stretch
-// takes, and cuts it into tiles of about the same width, a multiple of 32: no row is padded to 128.
+// takes, and cuts it into tiles of about the same width, a multiple of 32: no row is padded to 128.  Without a list all rows take
+// the one matrix there is.
 //
 //   PAIR_RELU2  out[row, n] = max(acc, 0)^2                                        (bfloat16)
 //   PAIR_F32    out[row, n] = acc                                                  (float32)
 //   PAIR_GLU    the matrix holds `n` gate rows above `n` up rows; out[row, n] = g sigmoid(slope g) (u + offset) with
 //               g = min(acc_gate, limit), u = clamp(acc_up, -limit, limit)         (bfloat16)
+//   PAIR_SWIGLU the same without limits, slope 1 and offset 0: silu(acc_gate) acc_up, NaN included
 //
 // A persistent grid of one block per SM, two of them a cluster.  Both blocks load half of the weight rows and half of the tokens
 // of a tile; the tensor cores of both read both halves of the tokens.  Per block:
@@ -28,6 +30,8 @@
 // tokens: a stream of single blocks that gathered each expert's pairs) -> this (us): 2,048 tokens, 1,536 x 3,328: 260 -> 208;
 // 24 tokens, 1,536 x 2,240 gated: 100 -> 82; 700 tokens, 3,584 x 4,736 gated: 466 -> 354.
 //
+// One matrix: 1,531 rows, 1,536 -> 2 x 8,960: 65 -> 59; 4,096, 3,584 -> 2 x 18,944: 811 -> 675 (1.65 PFLOP/s).
+//
 // No load has a multicast form; the commits that arrive at both blocks' barriers do.  Every wait on an mbarrier is bounded.
 #include "common.cuh"
 #include "ptx_sm100.cuh"
@@ -38,7 +42,7 @@ namespace ifx {
 constexpr int kPairRows = 256, kPairTokens = 256, kPairK = 64, kPairStages = 6;   // weight rows and tokens of a tile, k of a stage
 constexpr uint32_t kPairWBytes = 128 * kPairK * 2, kPairStageBytes = 2 * kPairWBytes;
 constexpr int kPairThreads = 192;
-enum { PAIR_RELU2 = 0, PAIR_F32 = 1, PAIR_GLU = 2 };
+enum { PAIR_RELU2 = 0, PAIR_F32 = 1, PAIR_GLU = 2, PAIR_SWIGLU = 3 };
 
 // The token rows in boxes of 32, 64 and 128: a block's share of a tile is one copy.
 struct TokenMaps {
@@ -46,7 +50,8 @@ struct TokenMaps {
 };
 
 struct PairArgs {
-  const PairItem* items;             // items[0].matrix: how many follow
+  const PairItem* items;             // items[0].matrix: how many follow; null: `rows` rows in `row_tiles` tiles
+  int rows, row_tiles;
   void* out;
   int N, kblocks, w_tiles, half_rows, band;
   float limit, slope, offset;
@@ -129,6 +134,12 @@ __device__ __forceinline__ uint32_t pair_pack(float a, float b) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// Tile i of `tiles` that share `rows` rows: sizes differ by one at most.
+__device__ __forceinline__ PairItem even_share(int rows, int tiles, int i) {
+  const int base = rows / tiles, more = rows % tiles, n = base + (i < more);
+  return PairItem{0, i * base + min(i, more), n, (n + 31) / 32 * 32};
+}
+
 template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ TokenMaps map_t, const PairArgs args) {
@@ -168,11 +179,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   const uint32_t tmem = tmem_holder;
   pdl_wait();
 
-  const int items = args.items[0].matrix, tiles = items * args.w_tiles, pairs = gridDim.x >> 1;
+  const int items = args.items ? args.items[0].matrix : args.row_tiles, tiles = items * args.w_tiles, pairs = gridDim.x >> 1;
   // Bands of `band` items with all their weight tiles, items fastest.
   auto tile_at = [&](int t, PairItem& item, int& wt) {
     const int first = t / (args.band * args.w_tiles) * args.band, rows = min(args.band, items - first), in = t - first * args.w_tiles;
-    item = args.items[1 + first + in % rows];
+    item = args.items ? args.items[1 + first + in % rows] : even_share(args.rows, items, first + in % rows);
     wt = in / rows;
   };
 
@@ -194,7 +205,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
           if (!ok) break;
           if (rank == 0) mbar_expect_tx(full + 8 * s, 2 * bytes);
           const uint32_t dst = ring + s * kPairStageBytes, bar = full_first + 8 * s;
-          if (MODE == PAIR_GLU) pair_load_5d(dst, &map_w, kb * kPairK, (wt * 128 + rank * 64) / args.half_rows, item.matrix, bar);
+          if (MODE >= PAIR_GLU) pair_load_5d(dst, &map_w, kb * kPairK, (wt * 128 + rank * 64) / args.half_rows, item.matrix, bar);
           else pair_load_3d(dst, &map_w, kb * kPairK, wt * kPairRows + rank * 128, item.matrix, bar);
           pair_load_2d(dst + kPairWBytes, &map_t.rows[box], kb * kPairK, item.row + rank * half, bar);
         }
@@ -292,6 +303,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
           __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(args.out) + row * args.N + n;
           auto made = [&](float lo, float hi) {        // of columns j (lo) and j + 1 (hi)
             const float other = __shfl_xor_sync(0xffffffffu, up ? lo : hi, half);
+            if (MODE == PAIR_SWIGLU) {
+              const float gate = up ? other : lo;
+              return __fdividef(gate, 1.0f + __expf(-gate)) * (up ? hi : other);
+            }
             const float gate = fminf(up ? other : lo, args.limit), u = fminf(fmaxf(up ? hi : other, -args.limit), args.limit);
             return __fdividef(gate, 1.0f + __expf(-args.slope * gate)) * (u + args.offset);
           };
@@ -348,7 +363,7 @@ static int launch_pair(const CUtensorMap& mw, const TokenMaps& mt, PairArgs args
   if (e != cudaSuccess) return (int)e;
   const long long tiles = (long long)most_items * args.w_tiles;
   const int most = pair_sm_count() / 2, pairs = tiles < most ? (int)tiles : most;
-  args.band = (pairs + args.w_tiles - 1) / args.w_tiles;
+  args.band = args.items ? (pairs + args.w_tiles - 1) / args.w_tiles : most_items;     // one matrix: all tokens against a tile of it
   return launch_pdl(gemm_pair_kernel<MODE>, dim3(2 * pairs), dim3(kPairThreads), smem, stream, 1, mw, mt, args);
 }
 
@@ -362,10 +377,10 @@ int gemm_pair(int mode, const void* tokens, const void* W, void* out, int rows, 
   TokenMaps mt;
   const cuuint64_t k = (cuuint64_t)K, pitch = k * 2;
   PairArgs args = {};
-  args.items = items, args.out = out, args.N = N, args.kblocks = (K + kPairK - 1) / kPairK;
+  args.items = items, args.rows = rows, args.row_tiles = most_items, args.out = out, args.N = N, args.kblocks = (K + kPairK - 1) / kPairK;
   args.limit = limit, args.slope = slope, args.offset = offset, args.error_flag = error_flag;
   int rc;
-  if (mode == PAIR_GLU) {
+  if (mode >= PAIR_GLU) {
     args.half_rows = N % 16 ? 8 : 16;
     args.w_tiles = (N + 127) / 128;
     const cuuint64_t h = (cuuint64_t)args.half_rows;
@@ -388,7 +403,14 @@ int gemm_pair(int mode, const void* tokens, const void* W, void* out, int rows, 
   if (mode == PAIR_RELU2) return launch_pair<PAIR_RELU2>(mw, mt, args, most_items, stream);
   if (mode == PAIR_F32) return launch_pair<PAIR_F32>(mw, mt, args, most_items, stream);
   if (mode == PAIR_GLU) return launch_pair<PAIR_GLU>(mw, mt, args, most_items, stream);
+  if (mode == PAIR_SWIGLU) return launch_pair<PAIR_SWIGLU>(mw, mt, args, most_items, stream);
   return IFX_E_BADARG;
+}
+
+// The same for rows that all take the one matrix W.
+int gemm_pair_rows(int mode, const void* tokens, const void* W, void* out, int rows, int N, int K, int* error_flag, cudaStream_t stream) {
+  return gemm_pair(mode, tokens, W, out, rows, N, K, 1, nullptr, (rows + kItemTokens - 1) / kItemTokens, 0.0f, 0.0f, 0.0f, error_flag,
+                   stream);
 }
 
 }  // namespace ifx

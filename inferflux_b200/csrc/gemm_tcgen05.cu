@@ -29,6 +29,9 @@
 
 namespace ifx {
 
+int gemm_pair_rows(int mode, const void* tokens, const void* W, void* out, int rows, int N, int K, int* error_flag,
+                   cudaStream_t stream);      // gemm_pair_tcgen05.cu
+
 constexpr int kBM = 128, kBN = 256, kBK = 64, kGemmStages = 4;
 constexpr uint32_t kABytes = kBM * kBK * 2, kBBytes = kBN * kBK * 2, kStageBytes = kABytes + kBBytes;
 
@@ -268,6 +271,13 @@ extern "C" int ifx_gemm_tcgen05(const void* act, const void* W, void* out, int M
   if (K <= 0 || error_flag == nullptr || out == nullptr) return IFX_E_BADARG;
   if (mode == GEMM_SWIGLU && (up_row_offset < N || up_row_offset + N > w_rows)) return IFX_E_BADARG;
   if ((mode == GEMM_STORE || mode == GEMM_RELU2) && N > w_rows) return IFX_E_BADARG;
+  // By pairs of SMs wherever outputs come in eights: the same bits, sooner (us, single blocks -> pairs, 200 / 512 / 1,531 / 4,096
+  // rows): 1,536 -> 2 x 8,960: 21 27 65 163 -> 18 25 59 147; 3,584 -> 2 x 18,944: 61 106 287 811 -> 54 100 271 675; 1,024 ->
+  // 2 x 4,096 17 19 29 58 -> 17 21 28 53.
+  if (N % 8 == 0 && (reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(act)) % 16 == 0 && K % 8 == 0) {
+    if (mode == GEMM_SWIGLU && up_row_offset == N) return gemm_pair_rows(3, act, W, out, M, N, K, error_flag, stream);
+    if (mode == GEMM_RELU2) return gemm_pair_rows(0, act, W, out, M, N, K, error_flag, stream);
+  }
   CUtensorMap ma, mw;
   int rc = weight_tensor_map(&mw, W, w_rows, K, 128);
   if (rc) return rc;
