@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(256) chunk_carry_kernel(const ChunkArgs a, int
 
 // out += (queries times decays)^T state.  CHANNEL: the decays are in `reach` already; else its number scales a token's row.
 template <int DK, bool CHANNEL>
-__global__ void __launch_bounds__(256) chunk_reach_kernel(const ChunkArgs a) {
+__global__ void __launch_bounds__(256, 3) chunk_reach_kernel(const ChunkArgs a) {
   constexpr int PK = DK + 8;
   extern __shared__ __align__(16) float smem[];
   float *q_s = smem, *s_s = smem + kChunk * PK;
@@ -493,6 +493,7 @@ __global__ void __launch_bounds__(256) chunk_reach_kernel(const ChunkArgs a) {
   if (!chunk_of(a.cu_seqlens, a.requests, a.min_span, blockIdx.x, first, n)) return;
   const float* state = a.local + (((size_t)blockIdx.x * a.heads + h) * dv + z * 64) * DK;
   bool bad = false;
+#pragma unroll
   for (int e = tid; e < kChunk * DK / 4; e += 256) {
     const int t = e / (DK / 4), c = e % (DK / 4) * 4;
     float4 q = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -524,6 +525,17 @@ __global__ void __launch_bounds__(256) chunk_reach_kernel(const ChunkArgs a) {
     return;
   }
   const int t0 = (warp >> 2) * 32, c0 = (warp & 3) * 16;   // a warp's 32 tokens and 16 value channels
+  float2 before[2][2][2];                                  // the outputs so far: on their way under the products
+  float scale[2][2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int t = min(t0 + i * 16 + half * 8 + (lane >> 2), n - 1);
+      scale[i][half] = CHANNEL ? 1.0f : a.reach[(size_t)(first + t) * a.heads + h];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) before[i][half][j] = *reinterpret_cast<const float2*>(out + t * out_row + c0 + j * 8 + 2 * (lane & 3));
+    }
   float acc[2][2][4] = {};
 #pragma unroll 2
   for (int kk = 0; kk < DK; kk += 16) {
@@ -544,12 +556,12 @@ __global__ void __launch_bounds__(256) chunk_reach_kernel(const ChunkArgs a) {
     for (int half = 0; half < 2; ++half) {
       const int t = t0 + i * 16 + half * 8 + (lane >> 2);
       if (t < n) {
-        const float f = CHANNEL ? 1.0f : a.reach[(size_t)(first + t) * a.heads + h];
+        const float f = scale[i][half];
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
-          float2* to = reinterpret_cast<float2*>(out + t * out_row + c0 + j * 8 + 2 * (lane & 3));
-          const float2 o = *to;
-          *to = make_float2(fmaf(f, acc[i][j][2 * half], o.x), fmaf(f, acc[i][j][2 * half + 1], o.y));
+          const float2 o = before[i][half][j];
+          *reinterpret_cast<float2*>(out + t * out_row + c0 + j * 8 + 2 * (lane & 3)) =
+              make_float2(fmaf(f, acc[i][j][2 * half], o.x), fmaf(f, acc[i][j][2 * half + 1], o.y));
         }
       }
     }
