@@ -8,7 +8,7 @@
 //   S = Q . K^T     tcgen05.mma, M 128 (queries = TMEM lanes) x N 128 (keys), K = head size;
 //                   Q and the key tile are K-major in shared memory (128-byte swizzle)
 //   softmax         one group of four warps per query tile, one thread per query row: the row
-//                   of S is read from TMEM (tcgen05.ld), masked on edge tiles, exponentiated
+//                   of S is read from TMEM once (tcgen05.ld), masked on edge tiles, exponentiated
 //                   against the row's reference maximum (log2 domain, one FFMA + one ex2 per
 //                   score), and written back over S as bfloat16 pairs (tcgen05.st): the A
 //                   operand of the next product
@@ -28,6 +28,8 @@
 // Bound: the tensor pipe and the exponentials, each busy 43 % of the time a block is resident (a key tile takes a block 2.1 us),
 // waiting for one another at the hand-overs.  A warp in step issues the products, one lane of it by predicate: with a single thread in a
 // branch of its own a product took 108 clocks to issue instead of 65 (2,500 tokens behind 4,000, 28 heads: 211 us, then 192).
+// A row's 128 scores stay in registers between the maximum and the exponentials (they were read twice), and the product with the
+// values begins with the first 64 keys' probabilities: 162 -> 151; 900 tokens of 12 heads behind 1,500: 25.1 -> 23.5; 447: 16.9 -> 16.2.
 // A block has an SM to itself, so blocks left over behind whole rounds of 148 cost a round: they are cut into parts of their keys
 // that prefill_merge_kernel adds up (192 -> 162; 512 tokens behind 3,000 of 12 heads, where 24 blocks are all there is, 62 -> 30).
 //
@@ -84,6 +86,13 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
+// The largest of three.
+__device__ __forceinline__ float max3(float x, float y, float z) {
+  float m;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(x), "f"(y), "f"(z));
+  return m;
+}
+
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&u)[32]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -112,7 +121,7 @@ struct PrefillLayout {
   static constexpr uint32_t Q_BYTES = HALVES * kBM * 128;     // one query tile: [half][128 rows][128 B]
   static constexpr uint32_t SLOT_BYTES = HALVES * kBN * 128;  // the keys or the values of one tile
   static constexpr int B_Q = 0, B_FULL = 1, B_EMPTY = B_FULL + SLOTS, B_S_FULL = B_EMPTY + SLOTS,
-                       B_P_FULL = B_S_FULL + 2, B_O_FULL = B_P_FULL + 2, B_COUNT = B_O_FULL + 2;
+                       B_P_HALF = B_S_FULL + 2, B_P_FULL = B_P_HALF + 2, B_O_FULL = B_P_FULL + 2, B_COUNT = B_O_FULL + 2;
   static constexpr size_t SMEM = 1024 + 2 * Q_BYTES + (size_t)SLOTS * SLOT_BYTES + B_COUNT * 8 + 16;
 };
 
@@ -155,6 +164,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
     }
     for (int q = 0; q < 2; ++q) {
       mbar_init(bar(L::B_S_FULL + q), 1);
+      mbar_init(bar(L::B_P_HALF + q), 4);
       mbar_init(bar(L::B_P_FULL + q), 4);
       mbar_init(bar(L::B_O_FULL + q), 1);
     }
@@ -284,14 +294,17 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
       int done[2] = {0, 0};                                // key tiles of each query tile so far
       auto issue_pv = [&](int q, int kt) -> bool {        // O_q += P_q . V(kt)
         const int j = 2 * visited(kt) + 1, s = j % SLOTS;
-        if (!wait(L::B_P_FULL + q, done[q] & 1) || !wait(L::B_FULL + s, (j / SLOTS) & 1))
-          return false;
-        tc_fence_after();
+        if (!wait(L::B_FULL + s, (j / SLOTS) & 1)) return false;
         const uint32_t v_src = kv_s + s * SLOT_BYTES;
 #pragma unroll
-        for (int k = 0; k < kBN / 16; ++k)                 // 16 keys (8 columns of pairs) a step
-          umma_ts(tmem_o + q * D, tmem_s + q * kBN + k * 8, desc_mnmajor_sw128(v_src + k * 2048, kBN * 128),
-                       idesc_o, (done[q] > 0 || k > 0) ? 1u : 0u, elected);
+        for (int half = 0; half < 2; ++half) {             // the first 64 keys' probabilities are used while the others are made
+          if (!wait((half ? L::B_P_FULL : L::B_P_HALF) + q, done[q] & 1)) return false;
+          tc_fence_after();
+#pragma unroll
+          for (int k = half * (kBN / 32); k < (half + 1) * (kBN / 32); ++k)       // 16 keys (8 columns of pairs) a step
+            umma_ts(tmem_o + q * D, tmem_s + q * kBN + k * 8, desc_mnmajor_sw128(v_src + k * 2048, kBN * 128),
+                         idesc_o, (done[q] > 0 || k > 0) ? 1u : 0u, elected);
+        }
         umma_commit(bar(L::B_O_FULL + q), elected);
         if (q == last_q(kt)) umma_commit(bar(L::B_EMPTY + s), elected);      // the values have been read
         ++done[q];
@@ -335,25 +348,24 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
       tc_fence_after();
       const bool edge = key0 + kBN - 1 > pos0_q ||
                         (window.any() && key0 < window.first(pos0_q + kBM - 1) && (!KEPT || key0 + kBN > keep));
-      // pass 1: the row's maximum
-      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      // the row's scores stay in registers: 128 of them
+      float s[kBN];
 #pragma unroll
-      for (int c = 0; c < kBN; c += 64) {
-        float s[64];
-        tmem_ld32(s_addr + c, *reinterpret_cast<float(*)[32]>(&s[0]));
-        tmem_ld32(s_addr + c + 32, *reinterpret_cast<float(*)[32]>(&s[32]));
-        tmem_wait_ld();
-        if (edge) {
+      for (int c = 0; c < kBN; c += 32) tmem_ld32(s_addr + c, *reinterpret_cast<float(*)[32]>(&s[c]));
+      tmem_wait_ld();
+      if (edge) {
 #pragma unroll
-          for (int j = 0; j < 64; ++j) {
-            const int key = key0 + c + j;
-            if (key > pos || (key < wfirst && (!KEPT || key >= keep))) s[j] = -INFINITY;
-          }
+        for (int j = 0; j < kBN; ++j) {
+          const int key = key0 + j;
+          if (key > pos || (key < wfirst && (!KEPT || key >= keep))) s[j] = -INFINITY;
         }
-#pragma unroll
-        for (int j = 0; j < 64; ++j) mx4[j & 3] = fmaxf(mx4[j & 3], s[j]);
       }
-      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+      float mx4[4] = {s[0], s[1], s[2], s[3]};
+#pragma unroll
+      for (int j = 4; j + 7 < kBN; j += 8)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) mx4[e] = max3(mx4[e], s[j + e], s[j + 4 + e]);
+      const float mx = fmaxf(max3(mx4[0], mx4[1], max3(s[kBN - 4], s[kBN - 3], s[kBN - 2])), max3(mx4[2], mx4[3], s[kBN - 1]));
       // the reference maximum moves only when the row's maximum has outgrown it
       const bool outgrown = m_ref > -INFINITY && (mx - m_ref) * scale_log2 > kRescaleStep;
       float factor = 1.0f;
@@ -380,38 +392,27 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
         }
         tmem_wait_st();
       }
-      // pass 2: probabilities over the scores, 64 keys (32 columns of bfloat16 pairs) at a time
+      // probabilities over the scores, 64 keys (32 columns of bfloat16 pairs) at a time
       const float bias = m_ref == -INFINITY ? 0.0f : -m_ref * scale_log2;
       float sum4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
       for (int c = 0; c < kBN; c += 64) {
-        float s[64];
-        tmem_ld32(s_addr + c, *reinterpret_cast<float(*)[32]>(&s[0]));
-        tmem_ld32(s_addr + c + 32, *reinterpret_cast<float(*)[32]>(&s[32]));
-        tmem_wait_ld();
-        if (edge) {
-#pragma unroll
-          for (int j = 0; j < 64; ++j) {
-            const int key = key0 + c + j;
-            if (key > pos || (key < wfirst && (!KEPT || key >= keep))) s[j] = -INFINITY;
-          }
-        }
         uint32_t packed[32];
 #pragma unroll
         for (int j = 0; j < 64; j += 2) {
-          const float p0 = ex2(fmaf(s[j], scale_log2, bias));
-          const float p1 = ex2(fmaf(s[j + 1], scale_log2, bias));
+          const float p0 = ex2(fmaf(s[c + j], scale_log2, bias));
+          const float p1 = ex2(fmaf(s[c + j + 1], scale_log2, bias));
           sum4[(j >> 1) & 3] += p0 + p1;
           __nv_bfloat162 b2 = __floats2bfloat162_rn(p0, p1);
           packed[j >> 1] = *reinterpret_cast<uint32_t*>(&b2);
         }
         tmem_st32(s_addr + (c >> 1), packed);              // columns whose scores have been read already
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar((c == 0 ? L::B_P_HALF : L::B_P_FULL) + q));
       }
       l_run += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
-      tmem_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(L::B_P_FULL + q));
       ++i;
     }
     if (ok && i > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar(L::B_O_FULL + q), (i - 1) & 1));
