@@ -329,6 +329,20 @@ __global__ void silu_mul_kernel(const T* __restrict__ in, T* __restrict__ out, i
   out[idx] = from_f32<T>(g / (1.0f + expf(-g)) * u);
 }
 
+// float32, inter % 4 == 0: 16-byte loads (333 rows of 8,960: 12.6 -> 6.2 us).
+__global__ void __launch_bounds__(256) silu_mul_f32x4_kernel(const float4* __restrict__ in, float4* __restrict__ out, int inter4, size_t total4) {
+  const size_t idx = (size_t)blockIdx.x * 256 + threadIdx.x;
+  if (idx >= total4) return;
+  const size_t r = idx / inter4, i = idx - r * inter4;
+  const float4 g = in[r * 2 * inter4 + i], u = in[r * 2 * inter4 + inter4 + i];
+  float4 o;
+  o.x = g.x / (1.0f + expf(-g.x)) * u.x;
+  o.y = g.y / (1.0f + expf(-g.y)) * u.y;
+  o.z = g.z / (1.0f + expf(-g.z)) * u.z;
+  o.w = g.w / (1.0f + expf(-g.w)) * u.w;
+  out[idx] = o;
+}
+
 // bf16, inter % 8 == 0: 16-byte loads, two chunks of 8 elements a thread (four loads in flight).
 __global__ void __launch_bounds__(256)
 silu_mul_bf16x8_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, int inter,
@@ -397,10 +411,13 @@ __global__ void residual_add_partial_kernel(float* __restrict__ x, const float* 
 template <typename T>
 __global__ void reduce_partial_kernel(const float* __restrict__ part, const float* __restrict__ bias,
                                       T* __restrict__ out, size_t total, int cols, int num_splits) {
+  pdl_launch_dependents();
+  pdl_wait();
   size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= total) return;
   float d = 0.0f;
-  for (int s = 0; s < num_splits; ++s) d += part[(size_t)s * total + idx];
+#pragma unroll 5
+  for (int s = 0; s < num_splits; ++s) d += part[(size_t)s * total + idx];       // (slices come in up to ten)
   if (bias) d += bias[idx % cols];
   out[idx] = from_f32<T>(d);
 }
@@ -567,15 +584,13 @@ int ifx_reduce_partial(const float* part, const float* bias, void* out, int rows
   if (rows <= 0 || num_splits <= 0) return 0;
   const size_t total = (size_t)rows * cols;
   const unsigned blocks = (unsigned)((total + 255) / 256);
+  // behind a product whose blocks let it in early: its launch is not waited for
   if (dtype == IFX_DT_F32)
-    reduce_partial_kernel<float><<<blocks, 256, 0, stream>>>(part, bias, (float*)out, total, cols, num_splits);
-  else if (dtype == IFX_DT_BF16)
-    reduce_partial_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(part, bias, (__nv_bfloat16*)out, total, cols,
-                                                                     num_splits);
-  else
-    return IFX_E_DTYPE;
-  IFX_CHECK_LAUNCH();
-  return 0;
+    return launch_pdl(reduce_partial_kernel<float>, dim3(blocks), dim3(256), 0, stream, 1, part, bias, (float*)out, total, cols, num_splits);
+  if (dtype == IFX_DT_BF16)
+    return launch_pdl(reduce_partial_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, 1, part, bias, (__nv_bfloat16*)out, total,
+                      cols, num_splits);
+  return IFX_E_DTYPE;
 }
 
 // gate_up [rows, 2 inter] (+ bias [2 inter], may be null) -> gelu_tanh(gate) * up, in the same dtype
@@ -605,6 +620,8 @@ int ifx_silu_mul(const void* gate_up, void* out, int rows, int inter, int dtype,
   } else if (dtype == IFX_DT_BF16) {
     silu_mul_kernel<__nv_bfloat16><<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(
         (const __nv_bfloat16*)gate_up, (__nv_bfloat16*)out, inter, total);
+  } else if (dtype == IFX_DT_F32 && inter % 4 == 0 && (((uintptr_t)gate_up | (uintptr_t)out) & 15) == 0) {
+    silu_mul_f32x4_kernel<<<(unsigned)((total / 4 + 255) / 256), 256, 0, stream>>>((const float4*)gate_up, (float4*)out, inter / 4, total / 4);
   } else if (dtype == IFX_DT_F32) {
     silu_mul_kernel<float><<<(unsigned)((total + 255) / 256), 256, 0, stream>>>((const float*)gate_up, (float*)out,
                                                                                inter, total);

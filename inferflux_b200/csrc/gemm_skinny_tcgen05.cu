@@ -414,6 +414,18 @@ extern "C" int ifx_gemm_skinny(const void* act, const void* W, const float* bias
                          sumsq_chunks, eps, error_flag, stream, ACT_NONE, 0.0f, 0.0f);
 }
 
+// A feed-forward of few rows, both products in one call from the host: hidden [M, inter] = silu(act . Wg^T) * (act . Wu^T) with
+// w_gate_up [2 inter, K], then hidden . w_down^T with w_down [N, inter] as out [M, N] (splits 1) or partials [splits, M, N].
+extern "C" int ifx_swiglu_few(const void* act, const void* w_gate_up, const void* w_down, void* hidden, void* out, float* partials, int M,
+                              int K, int inter, int N, int splits, const float* row_sumsq, int sumsq_chunks, float eps, int* error_flag,
+                              cudaStream_t stream) {
+  const int rc = gemm_skinny_any(act, w_gate_up, nullptr, hidden, nullptr, M, inter, K, 2 * inter, 1, MODE_SWIGLU, inter, 0, row_sumsq,
+                                 sumsq_chunks, eps, error_flag, stream, ACT_NONE, 0.0f, 0.0f);
+  if (rc) return rc;
+  return gemm_skinny_any(hidden, w_down, nullptr, out, partials, M, N, inter, N, splits, splits > 1 ? MODE_PARTIAL : MODE_STORE, 0, 0,
+                         nullptr, 0, 0.0f, error_flag, stream, ACT_NONE, 0.0f, 0.0f);
+}
+
 // mode 0 with an activation on the result before it is stored: act_kind 1 = xIELU with its two factors
 // (act_a z^2 + z/2 for z > 0, act_b (e^z - 1 - z) + z/2 otherwise), 3 = max(z, 0)^2.
 extern "C" int ifx_gemm_skinny_act(const void* act, const void* W, const float* bias, void* out, int M, int N, int K,

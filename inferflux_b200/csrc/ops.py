@@ -173,7 +173,7 @@ class CudaKernels:
                    "ifx_chunk_scan_supports", "ifx_chunk_decay_scan", "ifx_chunk_wkv_scan", "ifx_wkv_norm",
                    "ifx_latent_decode", "ifx_latent_decode_supports", "ifx_latent_decode_stretch",
                    "ifx_latent_prompt", "ifx_latent_prompt_supports", "ifx_delta_chunks_supports", "ifx_delta_chunks_scan",
-                   "ifx_attention_prefill_tcgen05_parts", "ifx_gemm_f32_split", "ifx_gemm_f32_split_launches"):
+                   "ifx_attention_prefill_tcgen05_parts", "ifx_gemm_f32_split", "ifx_swiglu_few", "ifx_gemm_f32_split_launches"):
             getattr(self.lib, fn).restype = ctypes.c_int
         self.lib.ifx_delta_rule_scratch_floats.restype = ctypes.c_longlong
         self.lib.ifx_chunk_scan_scratch_floats.restype = ctypes.c_longlong
@@ -400,11 +400,7 @@ class CudaKernels:
             return out
         if T <= self.SKINNY_MAX_ROWS and K % 8 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0:
             tiles = -(-N // 128)
-            kblocks = -(-K // 64)
-            # up to 128 rows: two blocks a SM and up to 10 K slices; above, a block owns its SM (32 KB of
-            # activations a stage) and every slice costs a [T, N] float32 round trip: at most 5
-            slots, most = (296, 10) if T <= 128 else (148, 5)
-            splits = max(1, min(slots // tiles, most, kblocks // 4)) if allow_partial and bias is None else 1
+            splits = self.skinny_slices(T, N, K) if allow_partial and bias is None else 1
             if splits > 1:
                 parts = self.linear_skinny(a, w, None, splits=splits, mode=1, rows=rows)
                 return PartialSum(parts, out_dtype)
@@ -417,6 +413,37 @@ class CudaKernels:
         if bias is not None:
             out += bias.to(out.dtype)
         return out
+
+    @staticmethod
+    def skinny_slices(rows, n, k):
+        """Slices of K of a few-rows product whose consumer adds them.  Up to 128 rows: two blocks a SM and up to 10 slices;
+        above, a block owns its SM (32 KB of activations a stage) and every slice costs a [rows, n] float32 round trip: at most 5."""
+        slots, most = (296, 10) if rows <= 128 else (148, 5)
+        return max(1, min(slots // -(-n // 128), most, -(-k // 64) // 4))
+
+    def swiglu_few(self, a, w_gate_up, w_down):
+        """A whole SwiGLU feed-forward of few bfloat16 rows, its two products launched by one call: what
+        `linear(linear_swiglu(a, w_gate_up), w_down, allow_partial=True)` gives, or None where that does not take the
+        few-rows kernels twice.  The host's time bounds such a call on small layers."""
+        rows = a if isinstance(a, ScaledRows) else None
+        if rows is not None:
+            a = rows.pre
+        T, K = a.shape
+        N, inter = w_down.shape
+        if not (a.dtype == w_gate_up.dtype == w_down.dtype == torch.bfloat16 and 0 < T <= self.SKINNY_MAX_ROWS and K % 8 == 0
+                and inter % 8 == 0 and tuple(w_gate_up.shape) == (2 * inter, K) and a.is_contiguous() and w_gate_up.is_contiguous()
+                and w_down.is_contiguous() and (a.data_ptr() | w_gate_up.data_ptr() | w_down.data_ptr()) % 16 == 0):
+            return None
+        splits = self.skinny_slices(T, N, inter)
+        hidden = torch.empty(T, inter, dtype=torch.bfloat16, device=a.device)
+        out = (torch.empty(splits, T, N, dtype=torch.float32, device=a.device) if splits > 1
+               else torch.empty(T, N, dtype=torch.bfloat16, device=a.device))
+        _check(self.lib.ifx_swiglu_few(_ptr(a), _ptr(w_gate_up), _ptr(w_down), _ptr(hidden), _ptr(out), _ptr(out), T, K, inter, N, splits,
+                                       _ptr(None if rows is None else rows.sumsq), 0 if rows is None else rows.sumsq.shape[1],
+                                       ctypes.c_float(0.0 if rows is None else rows.eps), _ptr(self.error_flag), _stream()),
+               "swiglu (few rows)")
+        self.launches += 2
+        return PartialSum(out, torch.bfloat16) if splits > 1 else out
 
     @staticmethod
     def float32_by_parts(n, k):

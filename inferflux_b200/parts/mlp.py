@@ -46,6 +46,10 @@ class SwiGLU(FeedForward):
 
     def forward(self, h, ctx):
         k = ctx.kernels
+        few = getattr(k, "swiglu_few", None)             # both products by one call, for few rows
+        y = few(h, self.w_gate_up, self.w_down) if few is not None else None
+        if y is not None:
+            return y
         act = k.linear_swiglu(h, self.w_gate_up)         # [T, I] = silu(h Wg^T) * (h Wu^T)
         return k.linear(act, self.w_down, allow_partial=True)
 
