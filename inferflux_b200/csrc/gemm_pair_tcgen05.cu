@@ -6,9 +6,10 @@
 // the one matrix there is.
 //
 //   PAIR_RELU2  out[row, n] = max(acc, 0)^2                                        (bfloat16)
-//   PAIR_F32    out[row, n] = acc                                                  (float32)
+//   PAIR_F32    out[row, n] = acc, or [slices, row, n] with K in slices            (float32)
 //   PAIR_GLU    the matrix holds `n` gate rows above `n` up rows; out[row, n] = g sigmoid(slope g) (u + offset) with
 //               g = min(acc_gate, limit), u = clamp(acc_up, -limit, limit)         (bfloat16)
+//   PAIR_GLU_EXACT  the same without the fast exponential and division
 //   PAIR_SWIGLU the same without limits, slope 1 and offset 0: silu(acc_gate) acc_up, NaN included
 //
 // A persistent grid of one block per SM, two of them a cluster.  Both blocks load half of the weight rows and half of the tokens
@@ -28,7 +29,7 @@
 // matrices of 4,096: 170 us, 1.62 PFLOP/s, the library's best; with few tiles what is lost is the last wave (192 tiles on 74 pairs).
 // Measured, all kernels of a mixture of 16 experts, four a token, 128 x 256 tiles of single blocks with rows padded to 128 (few
 // tokens: a stream of single blocks that gathered each expert's pairs) -> this (us): 2,048 tokens, 1,536 x 3,328: 260 -> 208;
-// 24 tokens, 1,536 x 2,240 gated: 100 -> 82; 700 tokens, 3,584 x 4,736 gated: 466 -> 354.
+// 24 tokens, 1,536 x 2,240 gated: 99 -> 84 (82 with K whole in the second product); 700 tokens, 3,584 x 4,736 gated: 478 -> 362.
 //
 // One matrix: 1,531 rows, 1,536 -> 2 x 8,960: 65 -> 59; 4,096, 3,584 -> 2 x 18,944: 811 -> 675 (1.65 PFLOP/s).
 //
@@ -42,7 +43,7 @@ namespace ifx {
 constexpr int kPairRows = 256, kPairTokens = 256, kPairK = 64, kPairStages = 6;   // weight rows and tokens of a tile, k of a stage
 constexpr uint32_t kPairWBytes = 128 * kPairK * 2, kPairStageBytes = 2 * kPairWBytes;
 constexpr int kPairThreads = 192;
-enum { PAIR_RELU2 = 0, PAIR_F32 = 1, PAIR_GLU = 2, PAIR_SWIGLU = 3 };
+enum { PAIR_RELU2 = 0, PAIR_F32 = 1, PAIR_GLU = 2, PAIR_SWIGLU = 3, PAIR_GLU_EXACT = 4 };
 
 // The token rows in boxes of 32, 64 and 128: a block's share of a tile is one copy.
 struct TokenMaps {
@@ -54,6 +55,7 @@ struct PairArgs {
   int rows, row_tiles;
   void* out;
   int N, kblocks, w_tiles, half_rows, band;
+  int slices, slice_kblocks;         // PAIR_F32: K in slices, each with its own [rows, N] of `out`
   float limit, slope, offset;
   int* error_flag;
 };
@@ -179,9 +181,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   const uint32_t tmem = tmem_holder;
   pdl_wait();
 
-  const int items = args.items ? args.items[0].matrix : args.row_tiles, tiles = items * args.w_tiles, pairs = gridDim.x >> 1;
-  // Bands of `band` items with all their weight tiles, items fastest.
-  auto tile_at = [&](int t, PairItem& item, int& wt) {
+  const int items = args.items ? args.items[0].matrix : args.row_tiles, tiles = items * args.w_tiles * (MODE == PAIR_F32 ? args.slices : 1), pairs = gridDim.x >> 1;
+  // Bands of `band` items with all their weight tiles: slices of K fastest, then items.
+  auto tile_at = [&](int t, PairItem& item, int& wt, int& slice) {
+    slice = 0;
+    if (MODE == PAIR_F32) {
+      slice = t % args.slices;
+      t /= args.slices;
+    }
     const int first = t / (args.band * args.w_tiles) * args.band, rows = min(args.band, items - first), in = t - first * args.w_tiles;
     item = args.items ? args.items[1 + first + in % rows] : even_share(args.rows, items, first + in % rows);
     wt = in / rows;
@@ -195,11 +202,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       bool ok = true;
       for (int t = blockIdx.x >> 1; t < tiles && ok; t += pairs) {
         PairItem item;
-        int wt;
-        tile_at(t, item, wt);
+        int wt, slice;
+        tile_at(t, item, wt, slice);
+        const int kb0 = slice * args.slice_kblocks, kb1 = min(args.kblocks, kb0 + args.slice_kblocks);
         const int half = item.width / 2, box = half <= 32 ? 0 : (half <= 64 ? 1 : 2);
         const uint32_t bytes = kPairWBytes + (32u << box) * kPairK * 2;
-        for (int kb = 0; kb < args.kblocks; ++kb, ++idx) {
+        for (int kb = kb0; kb < kb1; ++kb, ++idx) {
           const int s = idx % kPairStages;
           if (idx >= kPairStages) ok = pair_wait(empty + 8 * s, ((idx / kPairStages) & 1) ^ 1);
           if (!ok) break;
@@ -229,22 +237,23 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       bool ok = true;
       for (int t = blockIdx.x >> 1; t < tiles && ok; t += pairs, ++tile) {
         PairItem item;
-        int wt;
-        tile_at(t, item, wt);
+        int wt, slice;
+        tile_at(t, item, wt, slice);
+        const int kb0 = slice * args.slice_kblocks, kb1 = min(args.kblocks, kb0 + args.slice_kblocks);
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(item.width >> 3) << 17) | ((uint32_t)(kPairRows >> 4) << 24);
         const int buf = tile & 1, use = tile >> 1;
         if (use > 0) ok = pair_wait(acc_empty + 8 * buf, (use & 1) ^ 1);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t acc = tmem + buf * kPairTokens;
-        for (int kb = 0; kb < args.kblocks; ++kb, ++idx) {
+        for (int kb = kb0; kb < kb1; ++kb, ++idx) {
           const int s = idx % kPairStages;
           ok = pair_wait(full + 8 * s, (idx / kPairStages) & 1);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint64_t a = pair_desc(ring + s * kPairStageBytes), b = pair_desc(ring + s * kPairStageBytes + kPairWBytes);
 #pragma unroll
-          for (int k = 0; k < kPairK / 16; ++k) pair_mma(acc, a + 2 * k, b + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u, elected);
+          for (int k = 0; k < kPairK / 16; ++k) pair_mma(acc, a + 2 * k, b + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u, elected);
           pair_commit(empty + 8 * s, elected);
         }
         if (ok) pair_commit(acc_full + 8 * buf, elected);
@@ -261,8 +270,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     for (int t = blockIdx.x >> 1; t < tiles && ok; t += pairs, ++tile) {
       const int buf = tile & 1, use = tile >> 1;
       PairItem item;
-      int wt;
-      tile_at(t, item, wt);
+      int wt, slice;
+      tile_at(t, item, wt, slice);
       ok = pair_wait(acc_full + 8 * buf, use & 1);
       if (!ok) {
         if (lane == 0) atomicExch(args.error_flag, 73);
@@ -277,7 +286,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         const int left = item.count - c;             // columns that are somebody's
         if (MODE == PAIR_F32) {
           const int n = wt * kPairRows + rank * 128 + quarter * 32 + lane;
-          float* out = reinterpret_cast<float*>(args.out) + row * args.N + n;
+          float* out = reinterpret_cast<float*>(args.out) + ((size_t)slice * args.rows + row) * args.N + n;
           if (n < args.N) {
 #pragma unroll
             for (int j = 0; j < 16; ++j)
@@ -308,6 +317,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
               return __fdividef(gate, 1.0f + __expf(-gate)) * (up ? hi : other);
             }
             const float gate = fminf(up ? other : lo, args.limit), u = fminf(fmaxf(up ? hi : other, -args.limit), args.limit);
+            if (MODE == PAIR_GLU_EXACT) return gate / (1.0f + expf(-args.slope * gate)) * (u + args.offset);
             return __fdividef(gate, 1.0f + __expf(-args.slope * gate)) * (u + args.offset);
           };
 #pragma unroll
@@ -361,23 +371,25 @@ static int launch_pair(const CUtensorMap& mw, const TokenMaps& mt, PairArgs args
   const size_t smem = 1024 + (size_t)kPairStages * kPairStageBytes;
   cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  const long long tiles = (long long)most_items * args.w_tiles;
+  const long long tiles = (long long)most_items * args.w_tiles * args.slices;
   const int most = pair_sm_count() / 2, pairs = tiles < most ? (int)tiles : most;
   args.band = args.items ? (pairs + args.w_tiles - 1) / args.w_tiles : most_items;     // one matrix: all tokens against a tile of it
   return launch_pdl(gemm_pair_kernel<MODE>, dim3(2 * pairs), dim3(kPairThreads), smem, stream, 1, mw, mt, args);
 }
 
 // tokens [rows, K] bfloat16 sorted in stretches; W: `stack` matrices of [N, K] (GLU: [2 N, K]) bfloat16; K and N multiples of 8;
-// items on the device, at most `most_items` of them.
+// items on the device, at most `most_items` of them.  slice_kblocks: 64s of K in a slice (0: all; PAIR_F32 then fills [slices, rows, N]).
 int gemm_pair(int mode, const void* tokens, const void* W, void* out, int rows, int N, int K, int stack, const PairItem* items,
-              int most_items, float limit, float slope, float offset, int* error_flag, cudaStream_t stream) {
+              int most_items, int slice_kblocks, float limit, float slope, float offset, int* error_flag, cudaStream_t stream) {
   if (rows <= 0 || N <= 0 || most_items <= 0) return 0;
-  if (K <= 0 || K % 8 || N % 8 || stack <= 0) return IFX_E_BADARG;
+  if (K <= 0 || K % 8 || N % 8 || stack <= 0 || slice_kblocks < 0 || (slice_kblocks && mode != PAIR_F32)) return IFX_E_BADARG;
   CUtensorMap mw;
   TokenMaps mt;
   const cuuint64_t k = (cuuint64_t)K, pitch = k * 2;
   PairArgs args = {};
   args.items = items, args.rows = rows, args.row_tiles = most_items, args.out = out, args.N = N, args.kblocks = (K + kPairK - 1) / kPairK;
+  args.slice_kblocks = slice_kblocks ? slice_kblocks : args.kblocks;
+  args.slices = (args.kblocks + args.slice_kblocks - 1) / args.slice_kblocks;
   args.limit = limit, args.slope = slope, args.offset = offset, args.error_flag = error_flag;
   int rc;
   if (mode >= PAIR_GLU) {
@@ -403,13 +415,14 @@ int gemm_pair(int mode, const void* tokens, const void* W, void* out, int rows, 
   if (mode == PAIR_RELU2) return launch_pair<PAIR_RELU2>(mw, mt, args, most_items, stream);
   if (mode == PAIR_F32) return launch_pair<PAIR_F32>(mw, mt, args, most_items, stream);
   if (mode == PAIR_GLU) return launch_pair<PAIR_GLU>(mw, mt, args, most_items, stream);
+  if (mode == PAIR_GLU_EXACT) return launch_pair<PAIR_GLU_EXACT>(mw, mt, args, most_items, stream);
   if (mode == PAIR_SWIGLU) return launch_pair<PAIR_SWIGLU>(mw, mt, args, most_items, stream);
   return IFX_E_BADARG;
 }
 
 // The same for rows that all take the one matrix W.
 int gemm_pair_rows(int mode, const void* tokens, const void* W, void* out, int rows, int N, int K, int* error_flag, cudaStream_t stream) {
-  return gemm_pair(mode, tokens, W, out, rows, N, K, 1, nullptr, (rows + kItemTokens - 1) / kItemTokens, 0.0f, 0.0f, 0.0f, error_flag,
+  return gemm_pair(mode, tokens, W, out, rows, N, K, 1, nullptr, (rows + kItemTokens - 1) / kItemTokens, 0, 0.0f, 0.0f, 0.0f, error_flag,
                    stream);
 }
 

@@ -383,13 +383,14 @@ __global__ void moe_gather_kernel(const __nv_bfloat16* __restrict__ h, const int
   }
 }
 
-// Eight columns a thread: two loads of 16 bytes a choice, all choices' in flight.
-template <typename TO>
+// Eight columns a thread: two loads of 16 bytes a choice, all choices' in flight.  SLICED: y is [slices, rows, width].
+template <typename TO, bool SLICED>
 __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ h, const float* __restrict__ y,
                                    const float* __restrict__ weights, const int* __restrict__ pair_row, TO* __restrict__ out,
-                                   int top, int width) {
+                                   int top, int width, int slices) {
   pdl_wait();
   const int t = blockIdx.x;
+  const size_t slice = (size_t)gridDim.x * top * width;
   for (int c = threadIdx.x * 8; c < width; c += blockDim.x * 8) {
     float acc[8];
 #pragma unroll
@@ -398,19 +399,21 @@ __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ h, const fl
     for (int k = 0; k < top; ++k) {
       const int p = t * top + k, row = pair_row[p];
       const float w = weights[p];
-      float v[8];
-      if (row >= 0) {
-        const float4* src = reinterpret_cast<const float4*>(y + (size_t)row * width + c);
-        reinterpret_cast<float4*>(v)[0] = src[0];
-        reinterpret_cast<float4*>(v)[1] = src[1];
+      if (row >= 0) {                                        // a product, then a sum, each rounded: the same sums however K is cut
+        const float* src = y + (size_t)row * width + c;
+        for (int s = 0; s < (SLICED ? slices : 1); ++s, src += slice) {
+          float v[8];
+          reinterpret_cast<float4*>(v)[0] = reinterpret_cast<const float4*>(src)[0];
+          reinterpret_cast<float4*>(v)[1] = reinterpret_cast<const float4*>(src)[1];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) acc[i] = __fadd_rn(acc[i], __fmul_rn(v[i], w));
+        }
       } else {
         const uint4 raw = *reinterpret_cast<const uint4*>(h + (size_t)t * width + c);
         const __nv_bfloat16* b = reinterpret_cast<const __nv_bfloat16*>(&raw);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = to_f32(b[i]);
+        for (int i = 0; i < 8; ++i) acc[i] = fmaf(w, to_f32(b[i]), acc[i]);
       }
-#pragma unroll
-      for (int i = 0; i < 8; ++i) acc[i] = fmaf(w, v[i], acc[i]);
     }
     TO* dst = out + (size_t)t * width + c;
     if constexpr (sizeof(TO) == 4) {
@@ -426,10 +429,17 @@ __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ h, const fl
 }
 
 int gemm_pair(int mode, const void* tokens, const void* W, void* out, int rows, int N, int K, int stack, const PairItem* items,
-              int most_items, float limit, float slope, float offset, int* error_flag, cudaStream_t stream);
+              int most_items, int slice_kblocks, float limit, float slope, float offset, int* error_flag, cudaStream_t stream);
 
 static long long moe_aligned(long long bytes) { return (bytes + 255) / 256 * 256; }
 static int moe_most_items(int pairs, int experts) { return pairs / kItemTokens + (experts < pairs ? experts : pairs); }
+
+// Slices of K of a few tokens' second product: three, or one of a short K.  None is empty.
+static int moe_slice_kblocks(int ff) {
+  const int kblocks = (ff + 63) / 64, want = kblocks < 12 ? 1 : 3;
+  return (kblocks + want - 1) / want;
+}
+static int moe_slices(int ff, int few) { return few ? ((ff + 63) / 64 + moe_slice_kblocks(ff) - 1) / moe_slice_kblocks(ff) : 1; }
 
 }  // namespace ifx
 
@@ -515,24 +525,25 @@ int ifx_moe_experts_glu(const void* h, const void* w_up, const void* w_down, con
 }
 
 // Bytes of scratch of ifx_moe_sorted: the list of tiles, the pairs' rows, gathered rows, activations, the experts' outputs.
-long long ifx_moe_sorted_scratch(int T, int top, int experts, int width, int ff) {
+long long ifx_moe_sorted_scratch(int T, int top, int experts, int width, int ff, int few) {
   const long long pairs = (long long)T * top;
   return moe_aligned((1 + moe_most_items((int)pairs, experts)) * (long long)sizeof(PairItem)) + moe_aligned(pairs * 4) +
-         moe_aligned(pairs * width * 2) + moe_aligned(pairs * ff * 2) + pairs * width * 4;
+         moe_aligned(pairs * width * 2) + moe_aligned(pairs * ff * 2) + pairs * width * 4 * moe_slices(ff, few);
 }
 
 // The experts of a bfloat16 step over sorted rows.  h [T, width]; w_up [experts, ff, width] (glu: [experts, 2 ff, width], gate rows
 // above up rows); w_down [experts, width, ff]; ids, weights [T, top]; out [T, width] in out_dtype.  width and ff multiples of 8;
-// matrices, h, out and scratch on 16-byte boundaries.
+// matrices, h, out and scratch on 16-byte boundaries.  few: a step of few tokens, whose second product's K is cut into slices that
+// are added in float32, and whose gates' exponentials and divisions are not the fast ones.
 int ifx_moe_sorted(const void* h, const void* w_up, const void* w_down, const int* ids, const float* weights, void* out, int T, int top,
-                   int experts, int width, int ff, int out_dtype, int glu, float limit, float slope, float offset, void* scratch,
-                   long long scratch_bytes, int* error_flag, cudaStream_t stream) {
+                   int experts, int width, int ff, int out_dtype, int glu, int few, float limit, float slope, float offset,
+                   void* scratch, long long scratch_bytes, int* error_flag, cudaStream_t stream) {
   if (T <= 0) return 0;
   if (top <= 0 || experts <= 0 || experts > kMaxRouterOutputs || width <= 0 || ff <= 0 || width % 8 || ff % 8 || error_flag == nullptr)
     return IFX_E_BADARG;
   if (out_dtype != IFX_DT_F32 && out_dtype != IFX_DT_BF16) return IFX_E_DTYPE;
   if (((uintptr_t)h | (uintptr_t)w_up | (uintptr_t)w_down | (uintptr_t)out | (uintptr_t)scratch) % 16) return IFX_E_ALIGN;
-  if ((long long)T * top > 0x7fffffffll || scratch_bytes < ifx_moe_sorted_scratch(T, top, experts, width, ff)) return IFX_E_TOOBIG;
+  if ((long long)T * top > 0x7fffffffll || scratch_bytes < ifx_moe_sorted_scratch(T, top, experts, width, ff, few)) return IFX_E_TOOBIG;
   const int pairs = T * top, most = moe_most_items(pairs, experts);
   unsigned char* at = reinterpret_cast<unsigned char*>(scratch);
   auto take = [&](long long bytes) {
@@ -549,14 +560,17 @@ int ifx_moe_sorted(const void* h, const void* w_up, const void* w_down, const in
   if (rc) return rc;
   rc = launch_pdl(moe_gather_kernel, dim3(T), dim3(192), 0, stream, 1, (const __nv_bfloat16*)h, pair_row, rows, top, width / 8);
   if (rc) return rc;
-  rc = gemm_pair(glu ? 2 : 0, rows, w_up, act, pairs, ff, width, experts, items, most, limit, slope, offset, error_flag, stream);
+  rc = gemm_pair(!glu ? 0 : few ? 4 : 2, rows, w_up, act, pairs, ff, width, experts, items, most, 0, limit, slope, offset, error_flag, stream);
   if (rc) return rc;
-  rc = gemm_pair(1, act, w_down, y, pairs, width, ff, experts, items, most, 0.0f, 0.0f, 0.0f, error_flag, stream);
+  const int slices = moe_slices(ff, few), per = slices > 1 ? moe_slice_kblocks(ff) : 0;
+  rc = gemm_pair(1, act, w_down, y, pairs, width, ff, experts, items, most, per, 0.0f, 0.0f, 0.0f, error_flag, stream);
   if (rc) return rc;
   const __nv_bfloat16* hb = reinterpret_cast<const __nv_bfloat16*>(h);
-  if (out_dtype == IFX_DT_BF16)
-    return launch_pdl(moe_combine_kernel<__nv_bfloat16>, dim3(T), dim3(192), 0, stream, 1, hb, y, weights, pair_row, (__nv_bfloat16*)out, top, width);
-  return launch_pdl(moe_combine_kernel<float>, dim3(T), dim3(192), 0, stream, 1, hb, y, weights, pair_row, (float*)out, top, width);
+#define IFX_COMBINE(TO, SLICED)                                                                                                      \
+  launch_pdl(moe_combine_kernel<TO, SLICED>, dim3(T), dim3(192), 0, stream, 1, hb, y, weights, pair_row, (TO*)out, top, width, slices)
+  if (out_dtype == IFX_DT_BF16) return slices > 1 ? IFX_COMBINE(__nv_bfloat16, true) : IFX_COMBINE(__nv_bfloat16, false);
+  return slices > 1 ? IFX_COMBINE(float, true) : IFX_COMBINE(float, false);
+#undef IFX_COMBINE
 }
 
 }  // extern "C"

@@ -1709,7 +1709,7 @@ class CudaKernels:
             if h.dtype == torch.bfloat16:
                 if (self._moe_by_sorted_rows(T * top, int(experts), width, ff, True)
                         and self._moe_on_tensor_cores(h, w_up, w_down, ff, width)):
-                    return self._moe_experts_tiles(h, w_up, w_down, ids, weights, experts, out_dtype, glu=glu)
+                    return self._moe_sorted(h, w_up, w_down, ids, weights, experts, out_dtype, glu)
             act = torch.empty(T * top, ff, dtype=h.dtype, device=h.device)
             out = torch.empty(T, width, dtype=out_dtype, device=h.device)
             _check(self.lib.ifx_moe_experts_glu(_ptr(h), _ptr(w_up), _ptr(w_down), _ptr(ids), _ptr(weights), _ptr(act), _ptr(out),
@@ -1725,7 +1725,7 @@ class CudaKernels:
         if experts and h.dtype == torch.bfloat16:
             if (self._moe_by_sorted_rows(T * top, int(experts), width, ff, False)
                     and self._moe_on_tensor_cores(h, w_up, w_down, ff, width)):
-                return self._moe_experts_tiles(h, w_up, w_down, ids, weights, experts, out_dtype)
+                return self._moe_sorted(h, w_up, w_down, ids, weights, experts, out_dtype, None)
         act = torch.empty(T * top, ff, dtype=h.dtype, device=h.device)
         out = torch.empty(T, width, dtype=out_dtype, device=h.device)
         _check(self.lib.ifx_moe_experts(_ptr(h), _ptr(w_up if experts else None), _ptr(w_down if experts else None), _ptr(ids),
@@ -1777,23 +1777,29 @@ class CudaKernels:
         work = pairs * ff * width * (3 if gated else 2)
         return way != "tokens" or (experts <= self.MOE_MAX_EXPERTS and work >= self.MOE_TOKENS_MAX_WORK)
 
-    def _moe_experts_stream(self, h, w_up, w_down, ids, weights, experts, out_dtype, glu=None):
-        """bfloat16, few tokens: every chosen expert's weights once through the tensor cores, as with many tokens."""
-        return self._moe_experts_tiles(h, w_up, w_down, ids, weights, experts, out_dtype, glu=glu)
+    def _moe_sorted(self, h, w_up, w_down, ids, weights, experts, out_dtype, glu):
+        ff = w_up.shape[1] // (2 if glu is not None else 1)
+        many = self.moe_kernels(ids.numel(), int(experts), h.shape[1], ff, glu is not None) == "tiles"
+        return (self._moe_experts_tiles if many else self._moe_experts_stream)(h, w_up, w_down, ids, weights, experts, out_dtype, glu=glu)
 
-    def _moe_experts_tiles(self, h, w_up, w_down, ids, weights, experts, out_dtype, glu=None):
+    def _moe_experts_stream(self, h, w_up, w_down, ids, weights, experts, out_dtype, glu=None):
+        """bfloat16, few tokens: over sorted rows too, but K of the second product in up to three slices whose sums are added in
+        float32, and a gate's exponential and division are not the fast ones."""
+        return self._moe_experts_tiles(h, w_up, w_down, ids, weights, experts, out_dtype, glu=glu, few=True)
+
+    def _moe_experts_tiles(self, h, w_up, w_down, ids, weights, experts, out_dtype, glu=None, few=False):
         """bfloat16: pairs sorted by expert, two tcgen05 products over the sorted rows by pairs of SMs (the
         activation, relu^2 or the gated one of `glu`, in the first one's epilogue), then the weighted sum per token."""
         T, width = h.shape
         top, ff = ids.shape[1], w_up.shape[1] // (2 if glu is not None else 1)
-        room = self.lib.ifx_moe_sorted_scratch(T, top, int(experts), width, ff)
+        room = self.lib.ifx_moe_sorted_scratch(T, top, int(experts), width, ff, int(few))
         scratch = torch.empty(room, dtype=torch.uint8, device=h.device)
         out = torch.empty(T, width, dtype=out_dtype, device=h.device)
         limit, slope, offset = (glu if len(glu) > 2 else (*glu, 1.0)) if glu is not None else (0.0, 0.0, 0.0)
         _check(self.lib.ifx_moe_sorted(_ptr(h), _ptr(w_up), _ptr(w_down), _ptr(ids), _ptr(weights), _ptr(out), T, top, int(experts),
-                                       width, ff, _DT[out_dtype], int(glu is not None), ctypes.c_float(limit), ctypes.c_float(slope),
-                                       ctypes.c_float(offset), _ptr(scratch), _LL(room), _ptr(self.error_flag), _stream()),
-               "moe experts (sorted rows)")
+                                       width, ff, _DT[out_dtype], int(glu is not None), int(few), ctypes.c_float(limit),
+                                       ctypes.c_float(slope), ctypes.c_float(offset), _ptr(scratch), _LL(room), _ptr(self.error_flag),
+                                       _stream()), "moe experts (sorted rows)")
         self.launches += 5
         return out
 

@@ -1,5 +1,7 @@
 """The experts over sorted rows, products by pairs of SMs: pairs of an expert around the tiles' widths (16, 32, 256 rows), matrices
 that fill no tile of 128 or 256 outputs or 64 of K, experts without a pair, one with all of them, experts without weights."""
+import math
+
 import pytest
 import torch
 from test_moe_stream_gpu import BF, DEV, _inputs, _plain
@@ -49,3 +51,41 @@ def test_rows_that_are_no_numbers_stay_alone(cuda_kernels):
     keep = torch.ones(T, dtype=torch.bool, device=DEV)
     keep[[7, 100]] = False
     assert torch.equal(got[keep], clean[keep])
+
+
+@pytest.mark.parametrize("T,width,ff,slices", [(5, 64, 704, 1), (3, 64, 712, 3), (40, 136, 768, 3), (33, 72, 840, 3)])
+def test_few_tokens_add_slices_of_the_second_product_in_float32(cuda_kernels, T, width, ff, slices):
+    """Bit for bit: a slice is the same product over a part of the inner size; weighted, then added, each step rounded."""
+    experts, top = 4, 2
+    h, up, down, ids, weights = (t.to(DEV) for t in _inputs(T, width, ff, experts, experts + 1, top, None, T))
+    per = -(-(-(-ff // 64)) // slices) * 64
+    parts = []
+    for k in range(0, ff, per):
+        w_up, w_down = up[:, k:k + per].contiguous(), down[:, :, k:k + per].contiguous()
+        parts.append([cuda_kernels._moe_experts_tiles(h, w_up, w_down, ids[:, c:c + 1].contiguous(), torch.ones(T, 1, device=DEV), experts,
+                                                      torch.float32) for c in range(top)])
+    assert len(parts) == slices
+    want = torch.zeros(T, width, device=DEV)
+    for c in range(top):
+        w = weights[:, c:c + 1]
+        sums = want
+        for part in parts:
+            sums = sums + part[c] * w
+        plain = torch.addcmul(want, w, h.float())                            # an expert without weights
+        want = torch.where(ids[:, c:c + 1] < experts, sums, plain)
+    for out_dtype in (torch.float32, BF):
+        got = cuda_kernels._moe_experts_stream(h, up, down, ids, weights, experts, out_dtype)
+        assert torch.equal(got, want.to(out_dtype))
+    cuda_kernels.check_errors()
+
+
+def test_gates_of_few_tokens_are_divided_exactly(cuda_kernels):
+    """silu(-88) is 5e-37, which a fast division by 1 + e^88 takes for 0."""
+    experts, width, ff = 2, 64, 64
+    h, up, down = torch.zeros(3, width), torch.zeros(experts, 2 * ff, width), torch.zeros(experts, width, ff)
+    h[:, 0], up[:, :ff, 0], up[:, ff:, 0], down[:, :, 5] = 1.0, -88.0, 1.0, 2.0 ** 100
+    ids, weights = torch.zeros(3, 1, dtype=torch.int32, device=DEV), torch.ones(3, 1, device=DEV)
+    got = cuda_kernels._moe_experts_stream(h.to(BF).to(DEV), up.to(BF).to(DEV), down.to(BF).to(DEV), ids, weights, experts, torch.float32,
+                                           glu=(float("inf"), 1.0, 0.0))
+    want = -88.0 * math.exp(-88.0) * 2.0 ** 100
+    assert bool(((got.double() - want).abs() <= 2.0 ** -8 * abs(want)).all())
