@@ -1,30 +1,37 @@
 // Float32 matrix product C[M, N] = A[M, K] . W[N, K]^T (+ bias[N]) on the 5th-generation tensor cores, at 32-bit precision.
 //
-// Every operand is cut into three bfloat16 numbers that add up to it exactly (24 = 8 + 8 + 8 bits: the upper 16 bits of the
-// number, of what is left, and of what is left then), and an output is the sum of the six products of parts that reach 2^-16 of
-// it: hi hi, hi mid, mid hi, mid mid, hi lo, lo hi.  What is left out is below 2^-23 of a product's size.  The tensor cores cut
-// off when they add, so a chunk of 64 k gets an accumulator of its own, small products first, and the chunks' sums are added up
-// in registers with rounded float32 additions, k ascending: fewer roundings than a chain of K multiply-adds.  Errors against 64
-// bits (2-norm, normal rows; the same for 1 to 1,000 of them): K 1,536 chain of multiply-adds 7.0e-7, this 1.5e-7; K 3,584
-// 10.7e-7 and 1.9e-7; K 8,960 16.9e-7 and 1.6e-7; K 18,944 24.7e-7 and 1.9e-7.
+// Every operand is cut into three bfloat16 numbers that add up to it exactly: the number rounded to 8 bits, what is left rounded to 8
+// bits, and what is left then (7 bits at most).  An output is the sum of six products of parts: hi hi; mid hi, hi mid, mid mid, lo hi,
+// hi lo.  What is left out (mid lo, lo mid, lo lo) is below 2^-23.9 of a product's size, of either sign.  The tensor cores cut off
+// when they add.  So products hi hi, which have 16 bits, get an accumulator of their own, and a fresh one every 64 k, whose sums are
+// added up in registers with rounded float32 additions, k ascending; the other five, 2^-8 of them, run in a second accumulator that is
+// added every 16 chunks.
+// Errors against 64 bits (2-norm, normal numbers; chain of multiply-adds and this): K 1,288 6.5e-7 and 1.0e-7; 8,960 17e-7 and 1.2e-7
+// (2.3e-7 where K is not in slices); 18,944 25e-7 and 1.7e-7.  Rows with one, two, four, eight numbers that are not 0: 2.5e-8 and
+// 2.6e-8; 3.0 and 3.0 to 4.1; 4.0 and 3.4 to 4.9; 5.3 and 4.0 to 5.9: the slices and the second accumulator round once more.  (Parts
+// cut off instead of rounded, all six products in one accumulator: 1.0e-7 in these four, 4.6e-7 at most; dense rows 1.4e-7 to 2.5e-7.)
 //
 // An output's additions depend on K and N alone (how K is cut into slices does), never on the number of rows, so a row's bits
-// are the same whatever other rows share the launch.  A result that is not finite, or is tiny enough for a part to have fallen
-// below bfloat16's range, is made again as the plain chain of multiply-adds: infinities, NaN and overflow behave as there (a sum that leaves float32's range and
-// returns within one chunk stays finite here).
+// are the same whatever other rows share the launch.  Parts of a number below 2^-109 end at bfloat16's smallest, 2^-133.  That is
+// nothing in a result of 2^-60 or more whose operands are below 2^35.  All other results are made again as the plain chain of
+// multiply-adds, a tile at a time by the block that made them: those below 2^-60, those that are not finite, and those of a row (of
+// either operand) with a number of 2^35 or more, which puts a NaN into its row's first part.  So infinities, NaN and overflow behave
+// as there.
 //
 // Swapped operands: 128 weight rows are the lanes of tensor memory, up to 128 token rows the columns.  Persistent blocks:
 //
 //   warp 0        TMA: weights as they are (float32, [128 x 64] a chunk), the tokens' three planes (split_rows_kernel) as bfloat16
 //   warps 2-9     cut a chunk's weight rows, read from shared memory, and store the three parts into tensor memory (the products'
 //                 A operand); four warps the even chunks, four the odd ones (one group of four: 121 us instead of 109)
-//   warp 1        24 tcgen05.mma a chunk (M 128, N tokens, K 16, A from tensor memory) into one of two accumulators
-//   warps 10-17   add a finished chunk's accumulator to their registers, half the columns each four; behind the last chunk store,
+//   warp 1        24 tcgen05.mma a chunk (M 128, N tokens, K 16, A from tensor memory), hi hi first: its accumulator is read while the
+//                 other twenty run
+//   warps 10-17   add finished accumulators to their registers, half the columns each four; behind the last chunk store,
 //                 neighbouring lanes neighbouring columns of a row
 //
-// Bound: the tensor pipe for many rows (1,000 rows of 3,584 -> 37,888: 1,313 us, six products at 1.24 PFLOP/s); cutting and
+// Bound: the tensor pipe for many rows (1,000 rows of 3,584 -> 37,888: 1,216 us, six products at 1.34 PFLOP/s); cutting and
 // reading the weights for few.  Measured, gemm_f32_tiles_kernel -> this with both kernels beside it (us): 333 rows, 1,536 ->
-// 17,920: 485 -> 109; 8,960 -> 1,536: 310 -> 79; one row: 33 -> 32 and 107 -> 25; 150 rows, 18,944 -> 3,584: 650 -> 143.
+// 17,920: 485 -> 99; 8,960 -> 1,536: 310 -> 70; one row: 33 -> 32 and 107 -> 23; 150 rows, 18,944 -> 3,584: 650 -> 143.  Of 333 rows
+// one that is not finite: 233 and 358; all of them: 1,258 and 697.  Weights that are all zero: 3 times the time of others.
 #include "common.cuh"
 #include "ptx_sm100.cuh"
 
@@ -36,20 +43,25 @@ constexpr int kSplitMaxStages = 4;
 constexpr int kSplitThreads = 576;
 constexpr int kSplitPartCols = kSplitK / 2;                      // tensor memory columns of one part of a chunk
 constexpr int kSplitACols = 3 * kSplitPartCols;
+constexpr int kSplitDrain = 16;                                  // chunks of the five smaller products between two additions
 
-// Upper 16 bits of two numbers as a pair of bfloat16 (a below, b above).
-__device__ __forceinline__ uint32_t upper_halves(float a, float b) {
-  return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+// a, b -> three pairs of bfloat16 (a below, b above); `largest` of the magnitudes so far (NaN do not count).
+__device__ __forceinline__ void cut_pair(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo, float& largest) {
+  auto rounded = [](float x, float y) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
+    return *reinterpret_cast<const uint32_t*>(&v);
+  };
+  auto below = [](uint32_t pair) { return __uint_as_float(pair << 16); };
+  auto above = [](uint32_t pair) { return __uint_as_float(pair & 0xffff0000u); };
+  hi = rounded(a, b);
+  const float ra = a - below(hi), rb = b - above(hi);
+  mid = rounded(ra, rb);
+  lo = __byte_perm(__float_as_uint(ra - below(mid)), __float_as_uint(rb - above(mid)), 0x7632);
+  asm("{\n\t.reg .f32 x, y;\n\tabs.f32 x, %1;\n\tabs.f32 y, %2;\n\tmax.f32 %0, %0, x, y;\n\t}" : "+f"(largest) : "f"(a), "f"(b));
 }
-__device__ __forceinline__ float upper_part(float a) { return __uint_as_float(__float_as_uint(a) & 0xffff0000u); }
-
-// a, b -> three pairs of bfloat16.  What is not finite leaves NaN in the lower parts; the result is then made again.
-__device__ __forceinline__ void cut_pair(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  hi = upper_halves(a, b);
-  const float ra = a - upper_part(a), rb = b - upper_part(b);
-  mid = upper_halves(ra, rb);
-  lo = upper_halves(ra - upper_part(ra), rb - upper_part(rb));
-}
+constexpr uint32_t kNanPair = 0x7fff7fffu;
+constexpr float kSplitLargest = 34359738368.0f;                  // 2^35: from here on a row is made again
+constexpr float kSplitSmallest = 8.673617379884035e-19f;         // 2^-60: results below are
 
 // planes [3, rows, K] bfloat16 <- x [rows, K] float32, eight numbers a thread.
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ planes, long long n8) {
@@ -57,25 +69,127 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict
   if (i >= n8) return;
   const float4 a = reinterpret_cast<const float4*>(x)[2 * i], b = reinterpret_cast<const float4*>(x)[2 * i + 1];
   uint4 hi, mid, lo;
-  cut_pair(a.x, a.y, hi.x, mid.x, lo.x);
-  cut_pair(a.z, a.w, hi.y, mid.y, lo.y);
-  cut_pair(b.x, b.y, hi.z, mid.z, lo.z);
-  cut_pair(b.z, b.w, hi.w, mid.w, lo.w);
+  float largest = 0.0f;
+  cut_pair(a.x, a.y, hi.x, mid.x, lo.x, largest);
+  cut_pair(a.z, a.w, hi.y, mid.y, lo.y, largest);
+  cut_pair(b.x, b.y, hi.z, mid.z, lo.z, largest);
+  cut_pair(b.z, b.w, hi.w, mid.w, lo.w, largest);
+  if (!(largest < kSplitLargest)) hi.x = kNanPair;
   uint4* out = reinterpret_cast<uint4*>(planes);
   out[i] = hi;
   out[n8 + i] = mid;
   out[2 * n8 + i] = lo;
 }
 
-// Whether a result has to be made again (see the top).  2^-100: parts of a number above 2^-109 are whole.
-__device__ __forceinline__ bool made_again(float v) { return !(fabsf(v) < INFINITY) || (v != 0.0f && fabsf(v) < 7.9e-31f); }
-__device__ __noinline__ float chain_of_products(const float* __restrict__ a, const float* __restrict__ w, int K) {
-  float acc = 0.0f;
-  for (int k = 0; k < K; k += 4) {
-    const float4 x = *reinterpret_cast<const float4*>(a + k), y = *reinterpret_cast<const float4*>(w + k);
-    acc = fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, fmaf(x.x, y.x, acc))));
+// Whether a result has to be made again (see the top), and what stands in its place until then.
+__device__ __forceinline__ bool made_again(float v) { return !(fabsf(v) < INFINITY) || fabsf(v) < kSplitSmallest; }
+constexpr uint32_t kWasZero = 0x7fc00001u, kWasOther = 0x7fffffffu;              // NaN both
+__device__ __forceinline__ float placeholder(float v) { return __uint_as_float(v == 0.0f ? kWasZero : kWasOther); }
+
+// Results [m0 .. m0 + 32) x [n0 .. n0 + COLS) that are NaN, made again as the chain of multiply-adds (k ascending, then the bias).
+// All threads of a block fetch, four warps multiply: 8 rows and every 32nd column a thread.  smem: again_floats(COLS), free.  Zeros of
+// rows that hold nothing else are not multiplied out: they are the results that come here in earnest.
+constexpr int kAgainRows = 32, kAgainK = 32, kAgainPitch = kAgainK + 4, kAgainStages = 3;
+constexpr int again_floats(int cols) { return (kAgainRows + cols) * (kAgainStages * kAgainPitch + 1); }
+template <int COLS, int THREADS>
+__device__ __noinline__ void make_again(float* smem, const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
+                                        float* out, int M, int N, int K, int m0, int n0) {
+  constexpr int LINES = kAgainRows + COLS, EACH = COLS / 32;                     // lines: rows of A, then rows of W
+  static_assert(EACH <= 4 && THREADS >= 128, "");
+  const int tid = threadIdx.x, lane = tid & 31, row = (tid >> 5) * 8;
+  uint32_t* line_s = reinterpret_cast<uint32_t*>(smem + LINES * kAgainStages * kAgainPitch);          // the largest magnitude of a line
+  auto place = [&](int r, int j) { return out + (size_t)(m0 + row + r) * N + n0 + j * 32 + lane; };
+  unsigned need = 0, zeros = 0;                                                  // bit 8 j + r
+  if (tid < 128) {
+#pragma unroll
+    for (int j = 0; j < EACH; ++j)
+#pragma unroll
+      for (int r = 0; r < 8; ++r)
+        if (m0 + row + r < M && n0 + j * 32 + lane < N) {
+          const float v = *place(r, j);
+          if (isnan(v)) need |= 1u << (8 * j + r);
+          if (__float_as_uint(v) == kWasZero) zeros |= 1u << (8 * j + r);
+        }
   }
-  return acc;
+  if (!__syncthreads_or(need != 0)) return;
+  auto line = [&](int i) {
+    return i < kAgainRows ? A + (size_t)min(m0 + i, M - 1) * K : W + (size_t)min(n0 + i - kAgainRows, N - 1) * K;
+  };
+  const unsigned all = need;
+  if (__syncthreads_or(zeros != 0)) {                                            // of these, the ones of a line of zeros stay
+    for (int e = tid; e < LINES; e += THREADS) line_s[e] = 0;
+    __syncthreads();
+    for (int e = tid; e < LINES * 16; e += THREADS) {
+      const float* src = line(e >> 4);
+      uint32_t most = 0;
+#pragma unroll 4
+      for (int k = (e & 15) * 4; k < K; k += 64) {
+        const uint4 v = *reinterpret_cast<const uint4*>(src + k);
+        most = max(max(most, max(v.x & 0x7fffffffu, v.y & 0x7fffffffu)), max(v.z & 0x7fffffffu, v.w & 0x7fffffffu));
+      }
+      atomicMax(&line_s[e >> 4], most);
+    }
+    __syncthreads();
+    if (zeros) {
+#pragma unroll
+      for (int i = 0; i < 8 * EACH; ++i)
+        if ((zeros >> i & 1u) && (line_s[row + i % 8] == 0 || line_s[kAgainRows + i / 8 * 32 + lane] == 0)) need &= ~(1u << i);
+    }
+  }
+  float acc[EACH][8] = {};
+  if (__syncthreads_or(need != 0)) {
+    unsigned rows = __reduce_or_sync(0xffffffffu, need);
+    rows = (rows | rows >> 8 | rows >> 16 | rows >> 24) & 0xffu;
+    auto fetch = [&](int k0) {
+      float* to = smem + k0 / kAgainK % kAgainStages * LINES * kAgainPitch;
+      for (int e = tid; e < LINES * (kAgainK / 4); e += THREADS) {
+        const int i = e / (kAgainK / 4), k = e % (kAgainK / 4) * 4;
+        if (k0 + k < K)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(to + i * kAgainPitch + k)), "l"(line(i) + k0 + k) : "memory");
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int k0 = 0; k0 < (kAgainStages - 1) * kAgainK; k0 += kAgainK) fetch(k0);
+    for (int k0 = 0; k0 < K; k0 += kAgainK) {
+      fetch(k0 + (kAgainStages - 1) * kAgainK);
+      asm volatile("cp.async.wait_group %0;" ::"n"(kAgainStages - 1) : "memory");
+      __syncthreads();
+      const float* from = smem + k0 / kAgainK % kAgainStages * LINES * kAgainPitch;
+      const int left = min(kAgainK, K - k0);
+      auto step = [&](int k, unsigned which) {
+        float4 w[EACH];
+#pragma unroll
+        for (int j = 0; j < EACH; ++j) w[j] = *reinterpret_cast<const float4*>(from + (kAgainRows + j * 32 + lane) * kAgainPitch + k);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          if (which >> r & 1u) {
+            const float4 x = *reinterpret_cast<const float4*>(from + (row + r) * kAgainPitch + k);
+#pragma unroll
+            for (int j = 0; j < EACH; ++j)
+              acc[j][r] = fmaf(x.w, w[j].w, fmaf(x.z, w[j].z, fmaf(x.y, w[j].y, fmaf(x.x, w[j].x, acc[j][r]))));
+          }
+        }
+      };
+      if (rows & (rows - 1)) {                                     // more than one row: all eight
+#pragma unroll 1
+        for (int k = 0; k < left; k += 4) step(k, 0xffu);
+      } else if (rows) {
+#pragma unroll 1
+        for (int k = 0; k < left; k += 4) step(k, rows);
+      }
+      __syncthreads();
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+  }
+#pragma unroll
+  for (int j = 0; j < EACH; ++j)
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+      if (all >> (8 * j + r) & 1u) {
+        const float v = need >> (8 * j + r) & 1u ? acc[j][r] : 0.0f;
+        *place(r, j) = bias ? v + bias[n0 + j * 32 + lane] : v;
+      }
+  __syncthreads();
 }
 
 __device__ __forceinline__ void split_tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
@@ -112,14 +226,16 @@ template <int NT>
 __global__ void __launch_bounds__(kSplitThreads, 1)
 gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_t, const SplitArgs args) {
   extern __shared__ unsigned char smem_raw[];
-  __shared__ uint64_t bars[4 * kSplitMaxStages + 6];
+  __shared__ uint64_t bars[4 * kSplitMaxStages + 8];
   __shared__ uint32_t tmem_holder;
+  __shared__ int again_s;                                          // a result of this block has to be made again
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int nt = args.nt, w_stages = args.w_stages, t_stages = args.t_stages;
   const uint32_t plane_bytes = (uint32_t)nt * kSplitK * 2, t_bytes = 3 * plane_bytes;
   const uint32_t w_smem = smem_addr(smem), t_smem = w_smem + w_stages * kSplitWBytes;
   const uint32_t w_full = smem_addr(bars), w_empty = w_full + 8 * kSplitMaxStages, t_full = w_empty + 8 * kSplitMaxStages,
-                 t_empty = t_full + 8 * kSplitMaxStages, a_full = t_empty + 8 * kSplitMaxStages, done = a_full + 16, acc_empty = done + 16;
+                 t_empty = t_full + 8 * kSplitMaxStages, a_full = t_empty + 8 * kSplitMaxStages, a_empty = a_full + 16, big_full = a_empty + 16, big_empty = big_full + 8,
+                 small_full = big_empty + 8, small_empty = small_full + 8;
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int tiles = args.m_tiles * args.n_tiles * args.slices;
 
@@ -132,9 +248,13 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(a_full + 8 * b, 4);
-      mbar_init(done + 8 * b, 1);
-      mbar_init(acc_empty + 8 * b, 8);
+      mbar_init(a_empty + 8 * b, 1);
     }
+    mbar_init(big_full, 1);
+    mbar_init(big_empty, 8);
+    mbar_init(small_full, 1);
+    mbar_init(small_empty, 8);
+    again_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -145,7 +265,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_holder;
-  const uint32_t a_tmem = tmem + 256;                              // accumulators: columns 0 and 128; parts: 256 and 352
+  const uint32_t small = tmem + 128, a_tmem = tmem + 256;          // accumulators: hi hi at 0, the rest at 128; parts: 256 and 352
 
   // A tile: token tiles fastest, so that blocks running at a time read the same weights; then slices of K, then weight rows.
   auto slice_of = [&](int t, int& m_tile, int& n_tile, int& slice, int& c0, int& c1) {
@@ -195,28 +315,39 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nt >> 3) << 17) | ((uint32_t)(kSplitRows >> 4) << 24);
     const uint32_t elected = elect_one();
     const uint64_t plane_step = plane_bytes >> 4;
-    int i = 0;
+    int i = 0, sums = 0;                                           // chunks, uses of the second accumulator so far
     bool ok = true;
     for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
       int mt, ntile, slice, c0, c1;
       slice_of(t, mt, ntile, slice, c0, c1);
       for (int c = c0; c < c1; ++c, ++i) {
         const int buf = i & 1, ts = i % t_stages;
+        const bool fresh = (c - c0) % kSplitDrain == 0;
         ok = mbar_wait(t_full + 8 * ts, (i / t_stages) & 1) && mbar_wait(a_full + 8 * buf, (i >> 1) & 1);
-        if (ok && i >= 2) ok = mbar_wait(acc_empty + 8 * buf, ((i >> 1) & 1) ^ 1);
+        if (ok && i > 0) ok = mbar_wait(big_empty, (i & 1) ^ 1);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t acc = tmem + buf * 128, a = a_tmem + buf * kSplitACols;
+        const uint32_t a = a_tmem + buf * kSplitACols;
         const uint64_t b = split_smem_desc(t_smem + ts * t_bytes);
-        // (part of the weights, part of the tokens): 0 hi, 1 mid, 2 lo; the smallest products first
-        constexpr int WP[6] = {2, 0, 1, 1, 0, 0}, TP[6] = {0, 2, 1, 0, 1, 0};
 #pragma unroll
-        for (int p = 0; p < 6; ++p)
+        for (int k = 0; k < kSplitK / 16; ++k) umma_ts(tmem, a + k * 8, b + 2 * k, idesc, k > 0 ? 1u : 0u, elected);
+        umma_commit(big_full, elected);
+        if (fresh && sums > 0) ok = mbar_wait(small_empty, (sums & 1) ^ 1);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        // (part of the weights, part of the tokens): 0 hi, 1 mid, 2 lo; the smallest products first
+        constexpr int WP[5] = {2, 0, 1, 1, 0}, TP[5] = {0, 2, 1, 0, 1};
+#pragma unroll
+        for (int p = 0; p < 5; ++p)
 #pragma unroll
           for (int k = 0; k < kSplitK / 16; ++k)
-            umma_ts(acc, a + WP[p] * kSplitPartCols + k * 8, b + TP[p] * plane_step + 2 * k, idesc, (p > 0 || k > 0) ? 1u : 0u, elected);
+            umma_ts(small, a + WP[p] * kSplitPartCols + k * 8, b + TP[p] * plane_step + 2 * k, idesc, (!fresh || p > 0 || k > 0) ? 1u : 0u, elected);
         umma_commit(t_empty + 8 * ts, elected);
-        umma_commit(done + 8 * buf, elected);
+        umma_commit(a_empty + 8 * buf, elected);
+        if (c + 1 == c1 || (c + 1 - c0) % kSplitDrain == 0) {
+          umma_commit(small_full, elected);
+          ++sums;
+        }
       }
     }
     if (!ok && lane == 0) atomicExch(args.error_flag, 62);
@@ -233,7 +364,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         const int buf = i & 1, ws = i % w_stages;
         if (buf != group) continue;
         ok = mbar_wait(w_full + 8 * ws, (i / w_stages) & 1);
-        if (ok && i >= 2) ok = mbar_wait(done + 8 * buf, ((i >> 1) & 1) ^ 1);
+        if (ok && i >= 2) ok = mbar_wait(a_empty + 8 * buf, ((i >> 1) & 1) ^ 1);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t base = a_tmem + ((uint32_t)((warp & 3) * 32) << 16) + buf * kSplitACols;
@@ -241,12 +372,14 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         for (int h = 0; h < 2; ++h) {                              // 32 k: a row of 128 bytes, 16-byte pieces swizzled
           const unsigned char* src = smem + (size_t)ws * kSplitWBytes + h * (kSplitWBytes / 2) + row * 128;
           uint32_t hi[16], mid[16], lo[16];
+          float largest = 0.0f;
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
             const float4 v = *reinterpret_cast<const float4*>(src + ((q ^ (row & 7)) << 4));
-            cut_pair(v.x, v.y, hi[2 * q], mid[2 * q], lo[2 * q]);
-            cut_pair(v.z, v.w, hi[2 * q + 1], mid[2 * q + 1], lo[2 * q + 1]);
+            cut_pair(v.x, v.y, hi[2 * q], mid[2 * q], lo[2 * q], largest);
+            cut_pair(v.z, v.w, hi[2 * q + 1], mid[2 * q + 1], lo[2 * q + 1], largest);
           }
+          if (!(largest < kSplitLargest)) hi[0] = kNanPair;
           split_tmem_st16(base + h * 16, hi);
           split_tmem_st16(base + kSplitPartCols + h * 16, mid);
           split_tmem_st16(base + 2 * kSplitPartCols + h * 16, lo);
@@ -266,7 +399,8 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     // ------------------------------------------------------------------ sums of chunks, results
     constexpr int COLS = NT / 2;
     const int quarter = warp & 3, first = (warp - 10) / 4 * COLS;    // token columns first .. first + COLS
-    int i = 0;
+    const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
+    int i = 0, sums = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
       int mt, ntile, slice, c0, c1;
@@ -274,17 +408,14 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
       float sum[COLS];
 #pragma unroll
       for (int j = 0; j < COLS; ++j) sum[j] = 0.0f;
-      for (int c = c0; c < c1; ++c, ++i) {
-        const int buf = i & 1;
-        ok = mbar_wait(done + 8 * buf, (i >> 1) & 1);
-        if (!ok) break;
+      auto add = [&](uint32_t acc, uint32_t full, uint32_t empty, int use) {
+        if (!mbar_wait(full, use & 1)) return false;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + buf * 128 + first;
 #pragma unroll
         for (int j0 = 0; j0 < COLS; j0 += 16) {
           if (first + j0 < nt) {
             uint32_t r[16];
-            split_tmem_ld16(taddr + j0, r);
+            split_tmem_ld16(acc + lanes + first + j0, r);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
             for (int j = 0; j < 16; ++j) sum[j0 + j] += __uint_as_float(r[j]);
@@ -292,7 +423,12 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
-        if (lane == 0) split_arrive(acc_empty + 8 * buf);
+        if (lane == 0) split_arrive(empty);
+        return true;
+      };
+      for (int c = c0; c < c1 && ok; ++c, ++i) {
+        ok = add(tmem, big_full, big_empty, i);
+        if (ok && (c + 1 == c1 || (c + 1 - c0) % kSplitDrain == 0)) ok = add(small, small_full, small_empty, sums++);
       }
       if (!ok) break;
       const int n = ntile * kSplitRows + quarter * 32 + lane, m0 = mt * nt + first;
@@ -305,15 +441,12 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
 #pragma unroll
         for (int j = 0; j < COLS; ++j) {
           if (j < cols) {
-            again = again || made_again(sum[j]);
-            out[(size_t)(m0 + j) * args.N] = sum[j] + b;
+            const bool lost = whole && made_again(sum[j]);
+            again = again || lost;
+            out[(size_t)(m0 + j) * args.N] = lost ? placeholder(sum[j]) : sum[j] + b;
           }
         }
-        if (whole && again) {                                      // rare: which of them they were is seen from the results
-          for (int j = 0; j < cols; ++j)
-            if (made_again(out[(size_t)(m0 + j) * args.N] - b))
-              out[(size_t)(m0 + j) * args.N] = chain_of_products(args.A + (size_t)(m0 + j) * args.K, args.W + (size_t)n * args.K, args.K) + b;
-        }
+        if (again) again_s = 1;
       }
     }
     if (!ok && lane == 0) atomicExch(args.error_flag, 64);
@@ -324,20 +457,44 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
   }
+  if (again_s == 0) return;                                        // (set in front of the barrier above)
+  for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+    int mt, ntile, slice, c0, c1;
+    slice_of(t, mt, ntile, slice, c0, c1);
+    for (int r = 0; r < nt && mt * nt + r < args.M; r += kAgainRows)
+      make_again<kSplitRows, kSplitThreads>(reinterpret_cast<float*>(smem), args.A, args.W, args.bias, args.out, min(args.M, (mt + 1) * nt), args.N, args.K,
+                             mt * nt + r, ntile * kSplitRows);
+  }
 }
 
-// C [M, N] = the slices' sums in order (+ bias).
-__global__ void __launch_bounds__(256) split_slices_kernel(const float* __restrict__ parts, int slices, const float* __restrict__ A,
-                                                           const float* __restrict__ W, const float* __restrict__ bias,
-                                                           float* __restrict__ C, int M, int N, int K) {
-  const long long i = (long long)blockIdx.x * 256 + threadIdx.x, total = (long long)M * N;
-  if (i >= total) return;
-  float v = parts[i];
+// C [M, N] = the slices' sums in order (+ bias): 32 rows x 64 columns a block, 4 rows a thread.
+constexpr int kSumCols = 64, kSumRows = 4, kSumThreads = kSumCols * kAgainRows / kSumRows;
+__global__ void __launch_bounds__(kSumThreads) split_slices_kernel(const float* __restrict__ parts, int slices, const float* __restrict__ A,
+                                                                   const float* __restrict__ W, const float* __restrict__ bias, float* C,
+                                                                   int M, int N, int K) {
+  __shared__ __align__(16) float smem[again_floats(kSumCols)];
+  const int n0 = blockIdx.x * kSumCols, m0 = blockIdx.y * kAgainRows, n = n0 + threadIdx.x % kSumCols, m = m0 + threadIdx.x / kSumCols * kSumRows;
+  const int rows = n < N ? min(kSumRows, M - m) : 0;
+  const size_t total = (size_t)M * N;
+  const float* from = parts + (size_t)m * N + n;
+  float v[kSumRows] = {};
 #pragma unroll 4
-  for (int s = 1; s < slices; ++s) v += parts[s * total + i];
-  const int n = (int)(i % N);
-  if (made_again(v)) v = chain_of_products(A + i / N * K, W + (size_t)n * K, K);
-  C[i] = bias ? v + bias[n] : v;
+  for (int s = 0; s < slices; ++s) {
+#pragma unroll
+    for (int r = 0; r < kSumRows; ++r)
+      if (r < rows) v[r] = s == 0 ? from[(size_t)r * N] : v[r] + from[s * total + (size_t)r * N];
+  }
+  const float b = bias && rows > 0 ? bias[n] : 0.0f;
+  bool again = false;
+#pragma unroll
+  for (int r = 0; r < kSumRows; ++r) {
+    if (r < rows) {
+      const bool lost = made_again(v[r]);
+      again = again || lost;
+      C[(size_t)(m + r) * N + n] = lost ? placeholder(v[r]) : bias ? v[r] + b : v[r];
+    }
+  }
+  if (__syncthreads_or(again)) make_again<kSumCols, kSumThreads>(smem, A, W, bias, C, M, N, K, m0, n0);
 }
 
 static int split_sm_count() {
@@ -446,8 +603,8 @@ int ifx_gemm_f32_split(const float* A, const float* W, const float* bias, float*
     else rc = launch_split<128>(mw, mt, args, smem, stream);
     if (rc) return rc;
     if (args.slices > 1) {
-      const long long total = (long long)m * N;
-      split_slices_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(parts, args.slices, a, W, bias, C + (size_t)r0 * N, m, N, K);
+      const dim3 grid((N + kSumCols - 1) / kSumCols, (m + kAgainRows - 1) / kAgainRows);
+      split_slices_kernel<<<grid, kSumThreads, 0, stream>>>(parts, args.slices, a, W, bias, C + (size_t)r0 * N, m, N, K);
       IFX_CHECK_LAUNCH();
     }
   }

@@ -13,10 +13,11 @@ def operands(M, N, K, seed=0):
 
 
 def bound(a, w):
-    """Products left out: three below 2^-24 of one each.  A chunk of 64 k: 24 additions into its accumulator that may cut off up
-    to 2^-22 each (aligned products, then the sum).  The chunks' and slices' rounded additions: 2^-24 each."""
+    """Products left out: three below 2^-24 of one each.  A chunk of 64 k: 4 additions of its largest products into its accumulator that
+    may cut off up to 2^-22 each (aligned products, then the sum), 320 of the others, 2^-7 of them, into theirs.  The chunks' and
+    slices' rounded additions: 2^-24 each."""
     K = a.shape[1]
-    return (3 * 2.0 ** -24 + 24 * 2.0 ** -22 + (K / 64 + 150) * 2.0 ** -24) * (a.double().abs() @ w.double().abs().t()) + 1e-30
+    return (3 * 2.0 ** -24 + (4 + 320 * 2.0 ** -7) * 2.0 ** -22 + (K / 64 + 150) * 2.0 ** -24) * (a.double().abs() @ w.double().abs().t()) + 1e-30
 
 
 # 1,700 columns: slices of K; 19,000: 149 tiles of columns, K whole
@@ -68,3 +69,46 @@ def test_not_finite_tiny_and_huge(cuda_kernels, N):
     cols = torch.arange(N, device=DEV) != 11
     assert torch.equal(got[keep][:, cols], clean[keep][:, cols])
     assert not bool(got[keep][:, 11].isfinite().any())
+
+
+@pytest.mark.parametrize("N,K", [(1700, 1288), (19000, 1280), (1536, 8960)])
+@pytest.mark.parametrize("terms", [1, 2, 4, 8])
+def test_rows_of_few_terms_round_as_the_chain(cuda_kernels, N, K, terms):
+    """Errors that do not average out.  One term: what is left out (2^-24) and one rounding, the smaller products' cut off below; more:
+    a rounding or two beyond the chain's (2-norm up to 1.5 of its, 2 to 4 where parts are cut off instead of rounded)."""
+    a, w, _ = operands(40, N, K, seed=terms)
+    g = torch.Generator().manual_seed(terms)
+    keep = torch.zeros(40, K).scatter_(1, torch.rand(40, K, generator=g).argsort(1)[:, :terms], 1.0).to(DEV)
+    a *= keep
+    a[0], w[:8] = keep[0] * (1 + 2.0 ** -7 - 2.0 ** -23), 1 + 2.0 ** -7 - 2.0 ** -23      # what mantissas of this kind leave out adds up
+    want = a.double() @ w.double().t()
+    got, chain = cuda_kernels.linear(a, w).double() - want, cuda_kernels.linear_generic(a, w).double() - want
+    assert float(got.norm()) <= 1.5 * float(chain.norm())
+    if terms == 1:
+        assert bool((got.abs() <= (2 * 2.0 ** -24 + 20 * 2.0 ** -30) * want.abs()).all())
+
+
+@pytest.mark.parametrize("N", [1700, 19000])
+@pytest.mark.parametrize("small,large", [(-118, 100), (-125, 110), (-128, 60), (-140, 120), (-146, 20), (-133, 0), (-100, 4), (-70, -60)])
+def test_tiny_numbers_against_large_ones(cuda_kernels, N, small, large):
+    """Their lower parts are below bfloat16's range, whatever the result is."""
+    a, w, bias = operands(33, N, 1288, seed=2)
+    for x, y in ((a * 2.0 ** small, w * 2.0 ** large), (a * 2.0 ** large, w * 2.0 ** small)):
+        for b in (None, bias):
+            got, chain = cuda_kernels.linear(x, y, b), cuda_kernels.linear_generic(x, y, b)
+            assert bool(chain.isfinite().all()) and bool((chain != 0).any()) and torch.equal(got, chain)
+    # among numbers of ordinary size they are next to nothing, and stay that
+    x, y = a.clone(), w * 2.0 ** min(large, 28)
+    x[:, ::3] *= 2.0 ** small
+    assert bool(((cuda_kernels.linear(x, y).double() - x.double() @ y.double().t()).abs() <= bound(x, y)).all())
+    cuda_kernels.check_errors()
+
+
+@pytest.mark.parametrize("N", [1700, 19000])
+def test_rows_of_zeros(cuda_kernels, N):
+    a, w, bias = operands(100, N, 1288, seed=3)
+    a[5:50], w[7], w[9], w[N - 1] = 0.0, 0.0, -0.0, 0.0
+    a[60, 3], w[30, 5], a[99, :], a[99, 1287] = float("inf"), float("nan"), 0.0, 2.0 ** -140
+    got, chain = cuda_kernels.linear(a, w, bias), cuda_kernels.linear_generic(a, w, bias)
+    for x, y in ((got[5:50], chain[5:50]), (got[:, [7, 9, 30, N - 1]], chain[:, [7, 9, 30, N - 1]]), (got[60], chain[60]), (got[99], chain[99])):
+        assert torch.equal(x.nan_to_num(nan=7.0), y.nan_to_num(nan=7.0)) and torch.equal(x.isnan(), y.isnan())
