@@ -507,7 +507,6 @@ static int split_sm_count() {
   return sms;
 }
 
-constexpr int kSplitRowBlock = 1024;         // token rows worked on at a time: bounds the scratch
 
 // Chunks of 64 k in a slice: enough slices for about one block an SM with a single tile of tokens, at least four chunks each.
 // From N and K alone, so that the order of additions does not depend on the rows.
@@ -521,6 +520,18 @@ static int split_slice_chunks(int N, int K) {
 static int split_slices(int N, int K) {
   const int per = split_slice_chunks(N, K);
   return ((K + kSplitK - 1) / kSplitK + per - 1) / per;
+}
+
+// Token rows worked on at a time: up to 1,024, fewer where their planes and slices would take more than 64 MB (18,944 -> 3,584 takes
+// 185 KB a row: 256; one tile of 128 rows has a block for every SM, so that smaller portions cost launches alone).
+constexpr int kSplitRowBlock = 1024;
+constexpr long long kSplitScratch = 64ll << 20;
+static long long split_planes(long long rows, int K) { return (rows * K * 6 + 255) / 256 * 256; }
+static int split_row_block(int M, int N, int K) {
+  const int slices = split_slices(N, K);
+  const long long row = (long long)K * 6 + (slices > 1 ? (long long)slices * N * 4 : 0), fit = (kSplitScratch - 256) / row;
+  const int most = fit >= kSplitRowBlock ? kSplitRowBlock : fit >= kSplitRows ? (int)fit / kSplitRows * kSplitRows : fit >= 16 ? (int)fit / 16 * 16 : 16;
+  return M < most ? M : most;
 }
 
 template <int NT>
@@ -552,15 +563,16 @@ using namespace ifx;
 
 extern "C" {
 
-// Bytes of scratch that ifx_gemm_f32_split needs.
+// Bytes of scratch that ifx_gemm_f32_split needs: 64 MB at most, or what 16 rows take.
 long long ifx_gemm_f32_split_scratch(int M, int N, int K) {
-  const long long m = M < kSplitRowBlock ? M : kSplitRowBlock;
+  const long long m = split_row_block(M, N, K);
   const int slices = split_slices(N, K);
-  return ((m * K * 6 + 255) / 256) * 256 + (slices > 1 ? slices * m * N * 4 : 0);
+  return split_planes(m, K) + (slices > 1 ? slices * m * N * 4 : 0);
 }
 
 int ifx_gemm_f32_split_launches(int M, int N, int K) {
-  return (M + kSplitRowBlock - 1) / kSplitRowBlock * (split_slices(N, K) > 1 ? 3 : 2);
+  const int block = split_row_block(M, N, K);
+  return (M + block - 1) / block * (split_slices(N, K) > 1 ? 3 : 2);
 }
 
 // A [M, K], W [N, K], C [M, N] float32, K a multiple of 8, A, W and scratch on 16-byte boundaries.
@@ -573,8 +585,9 @@ int ifx_gemm_f32_split(const float* A, const float* W, const float* bias, float*
   CUtensorMap mw;
   int rc = make_f32_map(&mw, W, N, K);
   if (rc) return rc;
-  for (int r0 = 0; r0 < M; r0 += kSplitRowBlock) {
-    const int m = M - r0 < kSplitRowBlock ? M - r0 : kSplitRowBlock;
+  const int block = split_row_block(M, N, K);
+  for (int r0 = 0; r0 < M; r0 += block) {
+    const int m = M - r0 < block ? M - r0 : block;
     const float* a = A + (size_t)r0 * K;
     __nv_bfloat16* planes = reinterpret_cast<__nv_bfloat16*>(scratch);
     const long long n8 = (long long)m * K / 8;
@@ -592,7 +605,7 @@ int ifx_gemm_f32_split(const float* A, const float* W, const float* bias, float*
     args.w_stages = args.nt <= 64 ? 4 : 2;                                         // 64: 128 + 72 KB; 128: 64 + 144 KB
     args.t_stages = 3;
     args.error_flag = error_flag;
-    float* parts = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(scratch) + ((long long)m * K * 6 + 255) / 256 * 256);
+    float* parts = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(scratch) + split_planes(m, K));
     args.out = args.slices > 1 ? parts : C + (size_t)r0 * N;
     CUtensorMap mt;
     rc = make_tensor_map_bf16(&mt, planes, 3LL * m, K, args.nt);

@@ -112,3 +112,20 @@ def test_rows_of_zeros(cuda_kernels, N):
     got, chain = cuda_kernels.linear(a, w, bias), cuda_kernels.linear_generic(a, w, bias)
     for x, y in ((got[5:50], chain[5:50]), (got[:, [7, 9, 30, N - 1]], chain[:, [7, 9, 30, N - 1]]), (got[60], chain[60]), (got[99], chain[99])):
         assert torch.equal(x.nan_to_num(nan=7.0), y.nan_to_num(nan=7.0)) and torch.equal(x.isnan(), y.isnan())
+
+
+@pytest.mark.parametrize("N,K,rows", [(1536, 8960, 512), (3584, 18944, 256), (1700, 1288, 1024), (256, 16384, 384), (40, 262144, 32)])
+def test_scratch_is_bounded(cuda_kernels, N, K, rows):
+    """64 MB: more rows go in portions, whose results are the same bits."""
+    assert cuda_kernels.float32_by_parts(N, K)
+    a, w, bias = operands(rows + 5, N, K)
+    room = cuda_kernels.lib.ifx_gemm_f32_split_scratch
+    assert room(rows + 5, N, K) == room(rows, N, K) > room(rows - 1, N, K) and room(5000, N, K) <= 64 << 20
+    whole = cuda_kernels.linear(a, w, bias)
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    out = cuda_kernels.linear(a, w, bias)
+    assert torch.cuda.max_memory_allocated() - before - out.numel() * 4 <= room(rows, N, K) + 4096
+    assert torch.equal(out, whole) and torch.equal(cuda_kernels.linear(a[rows - 3:].contiguous(), w, bias), whole[rows - 3:])
+    cuda_kernels.check_errors()
