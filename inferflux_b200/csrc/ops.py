@@ -1707,9 +1707,10 @@ class CudaKernels:
                   and w_down.is_contiguous() and tuple(w_up.shape) == (experts, 2 * ff, width)
                   and tuple(w_down.shape) == (experts, width, ff), "moe_experts: stacked expert weights in the activations' dtype")
             if h.dtype == torch.bfloat16:
-                if (self._moe_by_sorted_rows(T * top, int(experts), width, ff, True)
-                        and self._moe_on_tensor_cores(h, w_up, w_down, ff, width)):
-                    return self._moe_sorted(h, w_up, w_down, ids, weights, experts, out_dtype, glu)
+                way = self.moe_kernels(T * top, int(experts), width, ff, True)
+                if way != "tokens" and self._moe_on_tensor_cores(h, w_up, w_down, ff, width):
+                    return (self._moe_experts_tiles if way == "tiles" else self._moe_experts_stream)(
+                        h, w_up, w_down, ids, weights, experts, out_dtype, glu=glu)
             act = torch.empty(T * top, ff, dtype=h.dtype, device=h.device)
             out = torch.empty(T, width, dtype=out_dtype, device=h.device)
             _check(self.lib.ifx_moe_experts_glu(_ptr(h), _ptr(w_up), _ptr(w_down), _ptr(ids), _ptr(weights), _ptr(act), _ptr(out),
@@ -1723,9 +1724,10 @@ class CudaKernels:
               and w_down.is_contiguous() and tuple(w_up.shape) == (experts, ff, width) and tuple(w_down.shape) == (experts, width, ff))),
               "moe_experts: stacked expert weights in the activations' dtype")
         if experts and h.dtype == torch.bfloat16:
-            if (self._moe_by_sorted_rows(T * top, int(experts), width, ff, False)
-                    and self._moe_on_tensor_cores(h, w_up, w_down, ff, width)):
-                return self._moe_sorted(h, w_up, w_down, ids, weights, experts, out_dtype, None)
+            way = self.moe_kernels(T * top, int(experts), width, ff, False)
+            if way != "tokens" and self._moe_on_tensor_cores(h, w_up, w_down, ff, width):
+                return (self._moe_experts_tiles if way == "tiles" else self._moe_experts_stream)(
+                    h, w_up, w_down, ids, weights, experts, out_dtype)
         act = torch.empty(T * top, ff, dtype=h.dtype, device=h.device)
         out = torch.empty(T, width, dtype=out_dtype, device=h.device)
         _check(self.lib.ifx_moe_experts(_ptr(h), _ptr(w_up if experts else None), _ptr(w_down if experts else None), _ptr(ids),
@@ -1735,31 +1737,31 @@ class CudaKernels:
         return out
 
     # Which kernels make the experts of a bfloat16 step, by the number of (token, choice) pairs: per token, or, once the work is
-    # MOE_TOKENS_MAX_WORK multiply-adds or there are MOE_STREAM_MAX_PAIRS pairs, over rows sorted by expert, where every chosen
+    # MOE_TOKENS_MAX_WORK multiply-adds or there are MOE_TOKENS_MAX_PAIRS pairs, over rows sorted by expert, where every chosen
     # expert's weights are read once.  Measured on a B200, weights of two layers in turn (us, per token / sorted rows):
-    #     4 experts, 2,048 x 2,048, one a token           1 token (8M) 18 / 25, 4 (34M): 22 / 26, 16 (134M): 52 / 28, 64: 140 / 29
-    #     8 experts, 1,536 x 2,240 gated, two a token     1 token (21M) 37 / 30, 2 (41M): 42 / 30, 8: 64 / 39, 32: 169 / 42
-    #    16 experts, the same, one a token                1 token (10M) 20 / 24, 2 (21M): 27 / 28, 4 (41M): 34 / 30, 8: 47 / 41
-    #    16 experts, the same, four a token               1 token (41M) 63 / 31, 4: 81 / 48
-    #    64 experts, 1,536 x 512, four a token            1 token (9M) 19 / 21, 4 (38M): 29 / 26, 8: 44 / 38, 16: 66 / 51
-    #    64 experts, 2,048 x 1,408 gated, six a token     1 token (52M) 73 / 36, 4: 112 / 81
-    #   256 experts, 2,048 x 1,024 gated, eight a token   1 token (50M) 63 / 35, 4: 103 / 84, 16: 281 / 203
-    # (A stream of blocks that each find their expert and its pairs in the step's choices, without a sort, lay between: 44, 80, 46 and
-    # 55, 116 us for the sixteen experts' 1 and 4 tokens, the eight's 32 and the 256's 1 and 4.)
-    # `moe_kernels` tells apart three sizes of step by the pairs an expert has; "stream" and "tiles" are sorted rows alike.
+    #     4 experts, 2,048 x 2,048, one a token           1 token (8M) 21 / 31, 4 (34M): 26 / 31, 16 (134M): 52 / 31, 64: 137 / 31
+    #     8 experts, 1,536 x 2,240 gated, two a token     1 token (21M) 33 / 26, 2 (41M): 42 / 32, 8: 62 / 44, 32: 166 / 45
+    #    16 experts, the same, one a token                1 token (10M) 19 / 23, 2 (21M): 24 / 25, 4 (41M): 33 / 31, 8: 45 / 41
+    #    16 experts, the same, four a token               1 token (41M) 62 / 34, 4: 82 / 55, 24: 243 / 72
+    #    64 experts, 1,536 x 512, four a token            1 token (6M) 17 / 22, 4 (25M): 26 / 26, 8 (50M): 30 / 31, 16: 48 / 42
+    #    64 experts, 2,048 x 1,408 gated, six a token     1 token (52M) 70 / 46, 4: 106 / 84
+    #   256 experts, 2,048 x 1,024 gated, eight a token   1 token (50M) 64 / 48, 4: 103 / 101, 16: 293 / 252
+    #    16 experts, 3,584 x 4,736 gated, four a token    1 token (204M) 154 / 93, 8: 506 / 266
+    # Of the sorted rows, steps of few pairs an expert ("stream") cut the second product's K into slices and take the exact
+    # exponential and division; the others ("tiles") do not.  A result's bits depend on that line, which lies where a kernel of its
+    # own for few pairs was slower than tiles; the time does so little (the last row 251 instead of 266).
     MOE_TILES_MIN_PAIRS = 192
     MOE_TILES_LARGE_EXPERT = 1 << 23
     MOE_TOKENS_MAX_WORK = 40_000_000
-    MOE_STREAM_MAX_PAIRS = 512
+    MOE_TOKENS_MAX_PAIRS = 512
     MOE_MAX_EXPERTS = 1024     # of sorted rows
 
     @classmethod
     def moe_kernels(cls, pairs, experts, width, ff, gated):
-        """"tokens", "stream" or "tiles"."""
-        if pairs >= cls.MOE_STREAM_MAX_PAIRS:
+        """"tokens", or over sorted rows "stream" or "tiles"."""
+        if pairs >= cls.MOE_TOKENS_MAX_PAIRS:
             return "tiles"
-        if (experts > cls.MOE_MAX_EXPERTS or pairs * ff * width * (3 if gated else 2) < cls.MOE_TOKENS_MAX_WORK
-                or not (4 * pairs >= 5 * experts or (pairs <= 16 and experts <= 64))):
+        if experts > cls.MOE_MAX_EXPERTS or pairs * ff * width * (3 if gated else 2) < cls.MOE_TOKENS_MAX_WORK:
             return "tokens"
         if ((pairs >= cls.MOE_TILES_MIN_PAIRS and pairs >= 12 * experts)
                 or (ff * width >= cls.MOE_TILES_LARGE_EXPERT and pairs >= 2 * experts)):
@@ -1771,16 +1773,6 @@ class CudaKernels:
         return (h.shape[0] > 0 and h.dtype == torch.bfloat16 and width % 8 == 0 and ff % 8 == 0 and h.data_ptr() % 16 == 0
                 and w_up.data_ptr() % 16 == 0 and w_down.data_ptr() % 16 == 0
                 and os.environ.get("INFERFLUX_B200_MOE_TILES", "1") != "0")
-
-    def _moe_by_sorted_rows(self, pairs, experts, width, ff, gated):
-        way = self.moe_kernels(pairs, experts, width, ff, gated)
-        work = pairs * ff * width * (3 if gated else 2)
-        return way != "tokens" or (experts <= self.MOE_MAX_EXPERTS and work >= self.MOE_TOKENS_MAX_WORK)
-
-    def _moe_sorted(self, h, w_up, w_down, ids, weights, experts, out_dtype, glu):
-        ff = w_up.shape[1] // (2 if glu is not None else 1)
-        many = self.moe_kernels(ids.numel(), int(experts), h.shape[1], ff, glu is not None) == "tiles"
-        return (self._moe_experts_tiles if many else self._moe_experts_stream)(h, w_up, w_down, ids, weights, experts, out_dtype, glu=glu)
 
     def _moe_experts_stream(self, h, w_up, w_down, ids, weights, experts, out_dtype, glu=None):
         """bfloat16, few tokens: over sorted rows too, but K of the second product in up to three slices whose sums are added in

@@ -85,13 +85,34 @@ def test_which_kernels_run(cuda_kernels, pairs, experts, width, ff, gated, want)
 
 
 @pytest.mark.parametrize("pairs,experts,width,ff,gated,want", [
-    (8, 64, 2048, 1408, True, "stream"), (24, 64, 2048, 1408, True, "tokens"), (96, 64, 2048, 1408, True, "stream"),
-    (300, 64, 2048, 1408, True, "stream"), (64, 256, 2048, 1024, True, "tokens"), (192, 256, 2048, 1024, True, "tokens"),
+    (8, 64, 2048, 1408, True, "stream"), (24, 64, 2048, 1408, True, "stream"), (96, 64, 2048, 1408, True, "stream"),
+    (300, 64, 2048, 1408, True, "stream"), (64, 256, 2048, 1024, True, "stream"), (192, 256, 2048, 1024, True, "stream"),
     (384, 256, 2048, 1024, True, "stream"), (511, 16, 2048, 1024, True, "tiles"), (200, 1025, 1024, 512, True, "tokens"),
-    (512, 256, 2048, 1024, True, "tiles")])
+    (512, 256, 2048, 1024, True, "tiles"),
+    (1, 1024, 8000, 2500, False, "stream"), (1, 1024, 8000, 2499, False, "tokens"), (1, 1025, 8000, 2500, False, "tokens"),
+    (511, 1024, 128, 128, True, "tokens"), (512, 1024, 128, 128, True, "tiles")])
 def test_which_kernels_run_with_many_experts(cuda_kernels, pairs, experts, width, ff, gated, want):
-    """An expert that has one pair at most is read once per token too, without a block for every tile of every expert."""
+    """From 40M multiply-adds or 512 pairs on over sorted rows, up to 1,024 experts below 512 pairs."""
     assert cuda_kernels.moe_kernels(pairs, experts, width, ff, gated) == want
+
+
+@pytest.mark.parametrize("T,experts,ff", [(1, 4, 72), (2, 3, 1032), (255, 4, 72), (256, 4, 72), (60, 8, 640), (100, 8, 640)])
+def test_the_rule_is_what_runs(cuda_kernels, T, experts, ff, monkeypatch):
+    """Per token two launches, over sorted rows five; and the bits of the kernels that the rule names."""
+    width, top = 256, 2
+    monkeypatch.setattr(type(cuda_kernels), "MOE_TOKENS_MAX_WORK", 1_000_000)      # both sides of the line with small matrices
+    for glu in (None, (7.0, 1.702, 1.0)):
+        h, up, down, ids, weights = (t.to(DEV) for t in _inputs(T, width, ff, experts, experts, top, glu, T))
+        way = cuda_kernels.moe_kernels(T * top, experts, width, ff, glu is not None)
+        before = cuda_kernels.launches
+        got = cuda_kernels.moe_experts(h, up, down, ids, weights, experts, BF, glu=glu)
+        assert cuda_kernels.launches - before == (2 if way == "tokens" else 5)
+        if way != "tokens":
+            by = cuda_kernels._moe_experts_stream if way == "stream" else cuda_kernels._moe_experts_tiles
+            assert torch.equal(got, by(h, up, down, ids, weights, experts, BF, glu=glu))
+        assert way == {(1, 72): "tokens", (2, 1032): "stream", (255, 72): "tiles", (256, 72): "tiles", (60, 640): "stream",
+                       (100, 640): "tiles"}[T, ff]
+    cuda_kernels.check_errors()
 
 
 def test_more_experts_than_the_stream_and_the_tiles_take(cuda_kernels):
