@@ -33,7 +33,9 @@
 //
 // One matrix: 1,531 rows, 1,536 -> 2 x 8,960: 65 -> 59; 4,096, 3,584 -> 2 x 18,944: 811 -> 675 (1.65 PFLOP/s).
 //
-// No load has a multicast form; the commits that arrive at both blocks' barriers do.  Every wait on an mbarrier is bounded.
+// No load has a multicast form; the commits that arrive at both blocks' barriers do.  Every wait on an mbarrier is bounded.  Two waits
+// are not: the cluster's barriers, which both blocks reach whatever their waits came to, and tcgen05.alloc, which waits for what
+// another kernel's blocks still hold on the SM.
 #include "common.cuh"
 #include "ptx_sm100.cuh"
 #include "moe_items.cuh"
