@@ -13,7 +13,7 @@
 // a unit lower triangular system, solved for the columns of [N V | U] so that everything is linear in S_0.  Four kernels:
 //
 //   delta_local   per stretch and head: outputs without S_0, the queries that meet S_0, the matrix that carries S_0 on, what is added
-//   delta_carry   the states in front of every stretch, one small product a stretch, 16 value channels a block
+//   delta_carry   the states in front of every stretch, one small product a stretch, 8 value channels a block
 //   chunk_reach   (chunk_scan.cu) adds what S_0 brings to the outputs
 //   delta_finish  (delta_rule.cu) norm and gate
 //
@@ -433,9 +433,8 @@ __global__ void __launch_bounds__(kCarryThreads) delta_carry_kernel(const DeltaC
   auto hand_on = [&](int buf) {                            // true: a number that is not finite, which parts would lose
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      auto whole = [](float y) { return y == y ? y : __uint_as_float(0x7fffffffu); };      // a NaN that its upper half still is
       Split p;
-      p.set(whole(x[i]), whole(x[2 + i]));
+      p.set(x[i], x[2 + i]);
       const int to = (2 * (lane & 3) + i) * 8 + lr;        // the word of the lane (value channel, lr / 2) for its odd or even key channel
       reinterpret_cast<uint32_t*>(s_s[buf][0][warp])[to] = p.hi;
       reinterpret_cast<uint32_t*>(s_s[buf][1][warp])[to] = p.mid;
@@ -475,10 +474,9 @@ __global__ void __launch_bounds__(kCarryThreads) delta_carry_kernel(const DeltaC
         const int upper = (j >> 3) & 1;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const int at = (2 * (lane & 3) + (i & 1)) * 8 + (j & 7), word = i >> 1;
-          const float s = from_parts(reinterpret_cast<const uint32_t*>(s_s[buf][0][j >> 4])[at], reinterpret_cast<const uint32_t*>(s_s[buf][1][j >> 4])[at],
-                                     reinterpret_cast<const uint32_t*>(s_s[buf][2][j >> 4])[at], upper);
-          acc[0][i] = fmaf(from_parts(m[word], m[word + 128], m[word + 256], upper), s, acc[0][i]);
+          const int word = i >> 1;
+          // (the state in front of the stretch, stored above: parts lose what lies below 2^-133)
+          acc[0][i] = fmaf(from_parts(m[word], m[word + 128], m[word + 256], upper), a.local[item * kDcD * kDcD + (vc + (i & 1)) * kDcD + j], acc[0][i]);
         }
       }
     } else {

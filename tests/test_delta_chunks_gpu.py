@@ -67,6 +67,28 @@ def test_a_number_that_is_not_finite_reaches_what_follows_it(cuda_kernels, block
     assert float((y.float() - walk.float())[fine].abs().max()) <= 2.0 ** -7 * float(walk.float()[fine].abs().max())
 
 
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_a_tiny_state_beside_one_that_is_not_finite(cuda_kernels, value):
+    """Columns of a state do not meet.  Those beside an infinity are multiplied in float32, in which a sum of 64 terms around 2^-130
+    is off by 64 halves of 2^-149 at most, in each of four stretches and their erased parts."""
+    H, D, T = 2, 64, 200
+    HD = H * D
+    g = torch.Generator().manual_seed(9)
+    proj, w_raw = torch.randn(T, 5 * HD, generator=g), torch.randn(T, HD, generator=g) - 6.0
+    proj[:, 2 * HD:3 * HD] = 0.0
+    vec = [torch.randn(HD, generator=g) for _ in range(3)]
+    first = torch.randn(HD * D, generator=g) * 2.0 ** -130
+    state, state_p = first[None].to(DEV).clone(), first[None].double()
+    state[0, 5] = value                                                         # head 0, key channel 0, value channel 5
+    PlainKernels(wide=True).delta_rule_scan(proj.double(), w_raw.double(), *vec, 1e-6, H, D, state_p, _Ctx((T,), (0,), "cpu"), F64)
+    _scan(cuda_kernels, True, proj.to(DEV), w_raw.to(DEV), *(t.to(DEV) for t in vec), 1e-6, H, D, state, _Ctx((T,), (0,), DEV), BF)
+    got, want = state.view(H, D, D).double().cpu(), state_p.view(H, D, D)
+    assert not bool(got[0, :, 5].isfinite().any())
+    beside = [0, 1, 2, 3, 4, 6, 7]
+    assert float(want[0, :, beside].abs().max()) > 2.0 ** -136
+    assert float((got - want)[0, :, beside].abs().max()) <= 4 * 2 * 64 * 2.0 ** -150
+
+
 @pytest.mark.parametrize("tokens", [130, 640])
 def test_no_less_exact_than_the_scan(cuda_kernels, tokens):
     """Parameters where trained models have them.  Both make float32 sums of the same numbers; a tenth for chance."""
