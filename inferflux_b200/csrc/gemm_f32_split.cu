@@ -23,15 +23,15 @@
 //   warp 0        TMA: weights as they are (float32, [128 x 64] a chunk), the tokens' three planes (split_rows_kernel) as bfloat16
 //   warps 2-9     cut a chunk's weight rows, read from shared memory, and store the three parts into tensor memory (the products'
 //                 A operand); four warps the even chunks, four the odd ones (one group of four: 121 us instead of 109)
-//   warp 1        24 tcgen05.mma a chunk (M 128, N tokens, K 16, A from tensor memory), hi hi first: its accumulator is read while the
-//                 other twenty run
+//   warp 1        24 tcgen05.mma a chunk (M 128, N tokens, K 16, A from tensor memory), hi hi first: its accumulator is read while
+//                 others run
 //   warps 10-17   add finished accumulators to their registers, half the columns each four; behind the last chunk store,
 //                 neighbouring lanes neighbouring columns of a row
 //
-// Bound: the tensor pipe for many rows (1,000 rows of 3,584 -> 37,888: 1,216 us, six products at 1.34 PFLOP/s); cutting and
+// Bound: the tensor pipe for many rows (1,000 rows of 3,584 -> 37,888: 1,148 us, six products at 1.42 PFLOP/s); cutting and
 // reading the weights for few.  Measured, gemm_f32_tiles_kernel -> this with both kernels beside it (us): 333 rows, 1,536 ->
-// 17,920: 485 -> 99; 8,960 -> 1,536: 310 -> 70; one row: 33 -> 32 and 107 -> 23; 150 rows, 18,944 -> 3,584: 650 -> 143.  Of 333 rows
-// one that is not finite: 233 and 358; all of them: 1,258 and 697.  Weights that are all zero: 3 times the time of others.
+// 17,920: 485 -> 95; 8,960 -> 1,536: 310 -> 71; one row: 33 -> 30 and 107 -> 23; 150 rows, 18,944 -> 3,584: 650 -> 141.  Of 333 rows
+// one that is not finite: 232 and 357; all of them: 1,259 and 534.  Weights that are all zero: 3 times the time of others.
 #include "common.cuh"
 #include "ptx_sm100.cuh"
 
@@ -39,10 +39,11 @@ namespace ifx {
 
 constexpr int kSplitRows = 128, kSplitK = 64;                    // weight rows of a tile, k of a chunk
 constexpr uint32_t kSplitWBytes = kSplitRows * kSplitK * 4;      // a chunk of float32 weights
-constexpr int kSplitMaxStages = 4;
+constexpr int kSplitMaxStages = 4, kSplitTStages = 3;            // of the weights' ring at most, of the tokens'
 constexpr int kSplitThreads = 576;
 constexpr int kSplitPartCols = kSplitK / 2;                      // tensor memory columns of one part of a chunk
 constexpr int kSplitACols = 3 * kSplitPartCols;
+constexpr int kSplitBig = 96;                                    // columns of the first of two accumulators
 constexpr int kSplitDrain = 16;                                  // chunks of the five smaller products between two additions
 
 // a, b -> three pairs of bfloat16 (a below, b above); `largest` of the magnitudes so far (NaN do not count).
@@ -217,7 +218,7 @@ __device__ __forceinline__ void split_arrive(uint32_t bar) {
 struct SplitArgs {
   const float *A, *W, *bias;
   float* out;                          // [M, N], or [slices, M, N] where slices > 1
-  int M, N, K, m_tiles, n_tiles, slices, slice_chunks, chunks, nt, w_stages, t_stages;
+  int M, N, K, m_tiles, n_tiles, slices, slice_chunks, chunks, nt, w_log;     // w_log: log2 of the weights' stages
   int* error_flag;
 };
 
@@ -226,16 +227,17 @@ template <int NT>
 __global__ void __launch_bounds__(kSplitThreads, 1)
 gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_t, const SplitArgs args) {
   extern __shared__ unsigned char smem_raw[];
-  __shared__ uint64_t bars[4 * kSplitMaxStages + 8];
+  __shared__ uint64_t bars[4 * kSplitMaxStages + 10];
   __shared__ uint32_t tmem_holder;
   __shared__ int again_s;                                          // a result of this block has to be made again
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  const int nt = args.nt, w_stages = args.w_stages, t_stages = args.t_stages;
+  const int nt = args.nt, w_log = args.w_log, w_stages = 1 << w_log;
+  constexpr int t_stages = kSplitTStages;
   const uint32_t plane_bytes = (uint32_t)nt * kSplitK * 2, t_bytes = 3 * plane_bytes;
   const uint32_t w_smem = smem_addr(smem), t_smem = w_smem + w_stages * kSplitWBytes;
   const uint32_t w_full = smem_addr(bars), w_empty = w_full + 8 * kSplitMaxStages, t_full = w_empty + 8 * kSplitMaxStages,
-                 t_empty = t_full + 8 * kSplitMaxStages, a_full = t_empty + 8 * kSplitMaxStages, a_empty = a_full + 16, big_full = a_empty + 16, big_empty = big_full + 8,
-                 small_full = big_empty + 8, small_empty = small_full + 8;
+                 t_empty = t_full + 8 * kSplitMaxStages, a_full = t_empty + 8 * kSplitMaxStages, a_empty = a_full + 16, big_full = a_empty + 16, big_empty = big_full + 16,
+                 small_full = big_empty + 16, small_empty = small_full + 8;
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int tiles = args.m_tiles * args.n_tiles * args.slices;
 
@@ -249,9 +251,9 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     for (int b = 0; b < 2; ++b) {
       mbar_init(a_full + 8 * b, 4);
       mbar_init(a_empty + 8 * b, 1);
+      mbar_init(big_full + 8 * b, 1);
+      mbar_init(big_empty + 8 * b, 8);
     }
-    mbar_init(big_full, 1);
-    mbar_init(big_empty, 8);
     mbar_init(small_full, 1);
     mbar_init(small_empty, 8);
     again_s = 0;
@@ -265,7 +267,10 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_holder;
-  const uint32_t small = tmem + 128, a_tmem = tmem + 256;          // accumulators: hi hi at 0, the rest at 128; parts: 256 and 352
+  // Tensor memory: hi hi, twice where three accumulators of a tile fit (few tokens, whose products do not last until the first has
+  // been read: one row, 3,584 -> 37,888, 104 -> 97 us), the rest of the products, the parts twice.
+  const int bigs = nt <= kSplitBig ? 2 : 1;
+  const uint32_t small = tmem + (bigs == 2 ? 2 * kSplitBig : kSplitRows), a_tmem = tmem + 512 - 2 * kSplitACols;
 
   // A tile: token tiles fastest, so that blocks running at a time read the same weights; then slices of K, then weight rows.
   auto slice_of = [&](int t, int& m_tile, int& n_tile, int& slice, int& c0, int& c1) {
@@ -286,8 +291,8 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         int mt, ntile, slice, c0, c1;
         slice_of(t, mt, ntile, slice, c0, c1);
         for (int c = c0; c < c1; ++c, ++i) {
-          const int ws = i % w_stages, ts = i % t_stages;
-          if (i >= w_stages) ok = mbar_wait(w_empty + 8 * ws, ((i / w_stages) & 1) ^ 1);
+          const int ws = i & (w_stages - 1), ts = i % t_stages;
+          if (i >= w_stages) ok = mbar_wait(w_empty + 8 * ws, ((i >> w_log) & 1) ^ 1);
           if (!ok) break;
           mbar_expect_tx(w_full + 8 * ws, kSplitWBytes);
           const uint32_t dst = w_smem + ws * kSplitWBytes;
@@ -295,7 +300,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
           tma_load_2d(dst + kSplitWBytes / 2, &map_w, c * kSplitK + 32, ntile * kSplitRows, w_full + 8 * ws);
           if (i >= t_stages) ok = mbar_wait(t_empty + 8 * ts, ((i / t_stages) & 1) ^ 1);
           if (!ok) {
-            mbar_wait(w_full + 8 * ws, (i / w_stages) & 1);        // not counted below: it has no tokens
+            mbar_wait(w_full + 8 * ws, (i >> w_log) & 1);        // not counted below: it has no tokens
             break;
           }
           mbar_expect_tx(t_full + 8 * ts, t_bytes);
@@ -305,7 +310,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
       }
       if (!ok) {
         atomicExch(args.error_flag, 61);
-        for (int j = max(0, i - w_stages); j < i; ++j) mbar_wait(w_full + 8 * (j % w_stages), (j / w_stages) & 1);
+        for (int j = max(0, i - w_stages); j < i; ++j) mbar_wait(w_full + 8 * (j & (w_stages - 1)), (j >> w_log) & 1);
         for (int j = max(0, i - t_stages); j < i; ++j) mbar_wait(t_full + 8 * (j % t_stages), (j / t_stages) & 1);
       }
     }
@@ -324,14 +329,15 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         const int buf = i & 1, ts = i % t_stages;
         const bool fresh = (c - c0) % kSplitDrain == 0;
         ok = mbar_wait(t_full + 8 * ts, (i / t_stages) & 1) && mbar_wait(a_full + 8 * buf, (i >> 1) & 1);
-        if (ok && i > 0) ok = mbar_wait(big_empty, (i & 1) ^ 1);
+        const int big = i & (bigs - 1), use = i >> (bigs - 1);
+        if (ok && use > 0) ok = mbar_wait(big_empty + 8 * big, (use & 1) ^ 1);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t a = a_tmem + buf * kSplitACols;
         const uint64_t b = split_smem_desc(t_smem + ts * t_bytes);
 #pragma unroll
-        for (int k = 0; k < kSplitK / 16; ++k) umma_ts(tmem, a + k * 8, b + 2 * k, idesc, k > 0 ? 1u : 0u, elected);
-        umma_commit(big_full, elected);
+        for (int k = 0; k < kSplitK / 16; ++k) umma_ts(tmem + big * kSplitBig, a + k * 8, b + 2 * k, idesc, k > 0 ? 1u : 0u, elected);
+        umma_commit(big_full + 8 * big, elected);
         if (fresh && sums > 0) ok = mbar_wait(small_empty, (sums & 1) ^ 1);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -361,9 +367,9 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
       int mt, ntile, slice, c0, c1;
       slice_of(t, mt, ntile, slice, c0, c1);
       for (int c = c0; c < c1; ++c, ++i) {
-        const int buf = i & 1, ws = i % w_stages;
+        const int buf = i & 1, ws = i & (w_stages - 1);
         if (buf != group) continue;
-        ok = mbar_wait(w_full + 8 * ws, (i / w_stages) & 1);
+        ok = mbar_wait(w_full + 8 * ws, (i >> w_log) & 1);
         if (ok && i >= 2) ok = mbar_wait(a_empty + 8 * buf, ((i >> 1) & 1) ^ 1);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -427,7 +433,8 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         return true;
       };
       for (int c = c0; c < c1 && ok; ++c, ++i) {
-        ok = add(tmem, big_full, big_empty, i);
+        const int big = i & (bigs - 1);
+        ok = add(tmem + big * kSplitBig, big_full + 8 * big, big_empty + 8 * big, i >> (bigs - 1));
         if (ok && (c + 1 == c1 || (c + 1 - c0) % kSplitDrain == 0)) ok = add(small, small_full, small_empty, sums++);
       }
       if (!ok) break;
@@ -478,7 +485,7 @@ __global__ void __launch_bounds__(kSumThreads) split_slices_kernel(const float* 
   const size_t total = (size_t)M * N;
   const float* from = parts + (size_t)m * N + n;
   float v[kSumRows] = {};
-#pragma unroll 4
+#pragma unroll 6
   for (int s = 0; s < slices; ++s) {
 #pragma unroll
     for (int r = 0; r < kSumRows; ++r)
@@ -602,15 +609,14 @@ int ifx_gemm_f32_split(const float* A, const float* W, const float* bias, float*
     args.chunks = (K + kSplitK - 1) / kSplitK;
     args.slice_chunks = split_slice_chunks(N, K);
     args.slices = split_slices(N, K);
-    args.w_stages = args.nt <= 64 ? 4 : 2;                                         // 64: 128 + 72 KB; 128: 64 + 144 KB
-    args.t_stages = 3;
+    args.w_log = args.nt <= 64 ? 2 : 1;                                            // 64: 128 + 72 KB; 128: 64 + 144 KB
     args.error_flag = error_flag;
     float* parts = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(scratch) + split_planes(m, K));
     args.out = args.slices > 1 ? parts : C + (size_t)r0 * N;
     CUtensorMap mt;
     rc = make_tensor_map_bf16(&mt, planes, 3LL * m, K, args.nt);
     if (rc) return rc;
-    const size_t smem = 1024 + (size_t)args.w_stages * kSplitWBytes + (size_t)args.t_stages * 3 * args.nt * kSplitK * 2;
+    const size_t smem = 1024 + ((size_t)kSplitWBytes << args.w_log) + (size_t)kSplitTStages * 3 * args.nt * kSplitK * 2;
     if (args.nt <= 32) rc = launch_split<32>(mw, mt, args, smem, stream);
     else if (args.nt <= 64) rc = launch_split<64>(mw, mt, args, smem, stream);
     else rc = launch_split<128>(mw, mt, args, smem, stream);

@@ -129,3 +129,12 @@ def test_scratch_is_bounded(cuda_kernels, N, K, rows):
     assert torch.cuda.max_memory_allocated() - before - out.numel() * 4 <= room(rows, N, K) + 4096
     assert torch.equal(out, whole) and torch.equal(cuda_kernels.linear(a[rows - 3:].contiguous(), w, bias), whole[rows - 3:])
     cuda_kernels.check_errors()
+
+
+@pytest.mark.parametrize("M,N,K", [(33, 19000, 2048), (40, 18950, 2112), (17, 1536, 12288), (5, 1536, 12352)])
+def test_whole_groups_of_chunks(cuda_kernels, M, N, K):
+    """The smaller products' accumulator is added every 16 chunks of 64: 32 and 33 chunks, slices of 16 and of 17."""
+    a, w, bias = operands(M, N, K)
+    want = a.double() @ w.double().t() + bias.double()
+    assert bool(((cuda_kernels.linear(a, w, bias).double() - want).abs() <= bound(a, w) + 2.0 ** -24 * want.abs()).all())
+    cuda_kernels.check_errors()
