@@ -366,8 +366,8 @@ class CudaKernels:
 
     def linear(self, a, w, bias=None, out_dtype=None, allow_partial=False):
         """out[T, N] = a[T, K] . w[N, K]^T (+ bias), float32 accumulation.  float32 runs use
-        the CUDA-core product, or operands in parts on the tensor cores (`float32_by_parts`).  bfloat16 runs with up to 256 rows use the tcgen05 weight-streaming
-        kernel; with `allow_partial` a narrow product is split over K and comes back as a
+        the CUDA-core product, or for large weights operands in parts on the tensor cores (`float32_by_parts`).  bfloat16 runs
+        with up to SKINNY_MAX_ROWS rows use the tcgen05 weight-streaming kernel; with `allow_partial` a narrow product is split over K and comes back as a
         PartialSum for a consumer that adds the slices itself.  More rows go to cuBLAS."""
         rows = a if isinstance(a, ScaledRows) else None
         if rows is not None:
@@ -449,15 +449,17 @@ class CudaKernels:
     def float32_by_parts(n, k):
         """Whether a float32 product runs on the tensor cores, its operands cut into three bfloat16 numbers each
         (csrc/gemm_f32_split.cu).  By the weight's sizes alone: a row's bits must not depend on how many there are.  Parts
-        against the chain of multiply-adds, us, 1 / 16 / 100 / 512 rows: 1,536 x 1,368 17 17 22 37 against 21 21 37 74;
-        2,048 x 1,024 17 17 22 39 against 16 17 28 67; 4,096 x 512 17 16 22 38 against 10 10 22 60; 1,024 x 1,024
-        21 17 22 26 against 15 16 19 39; 256 x 8,192 18 18 25 37 against 96 98 123 123."""
+        against the chain of multiply-adds, us, 1 / 16 / 100 / 512 rows: 1,536 x 1,368 24 25 27 41 against 29 25 45 81;
+        2,048 x 1,024 18 17 21 34 against 17 17 29 70; 4,096 x 512 17 17 21 35 against 10 10 22 60; 1,024 x 1,024
+        17 17 20 24 against 16 17 19 39; 256 x 8,192 20 24 29 41 against 97 99 123 123."""
         return k % 8 == 0 and k >= 1280 and n * k >= 1 << 21
 
     # The many-rows tcgen05 product with SiLU(gate)*up in its epilogue against cuBLAS followed by the activation
-    # kernel, measured on a B200 (us a layer, 256 / 512 / 2,048 rows): Qwen2.5-1.5B sizes 21 vs 27, 31 vs 37, 94 vs 110;
-    # 7B sizes 63 vs 79, 107 vs 107, 373 vs 381; 32B sizes (inner size 5120) 126 vs 136, 217 vs 212, 851 vs 779.
-    # So it is used up to an inner size of 4096.
+    # kernel, measured on a B200 (us a layer, 256 / 512 / 2,048 rows): Qwen2.5-1.5B sizes 18 vs 29, 25 vs 31, 77 vs 95;
+    # 7B sizes 57 vs 79, 99 vs 106, 340 vs 382; 32B sizes (inner size 5,120) 111 vs 144, 197 vs 218, 767 vs 961; inner size
+    # 8,192 (28,672 outputs) 208 vs 221, 347 vs 397, 1,297 vs 1,564.  The line comes from tiles of single SMs, which were
+    # slower than the library's at 5,120 (851 vs 779 us at 2,048 rows); by pairs of SMs they are ahead there too.  It stays for
+    # what it does to results: beyond it gate and up are rounded to bfloat16 in front of the activation.
     SWIGLU_TILES_MAX_K = 4096
 
     def linear_swiglu(self, a, w_gate_up):
