@@ -29,7 +29,7 @@
 // matrices of 4,096: 170 us, 1.62 PFLOP/s, the library's best; with few tiles what is lost is the last wave (192 tiles on 74 pairs).
 // Measured, all kernels of a mixture of 16 experts, four a token, 128 x 256 tiles of single blocks with rows padded to 128 (few
 // tokens: a stream of single blocks that gathered each expert's pairs) -> this (us): 2,048 tokens, 1,536 x 3,328: 260 -> 208;
-// 24 tokens, 1,536 x 2,240 gated: 99 -> 84 (82 with K whole in the second product); 700 tokens, 3,584 x 4,736 gated: 478 -> 362.
+// 24 tokens, 1,536 x 2,240 gated: 98 -> 80; 700 tokens, 3,584 x 4,736 gated: 478 -> 362.
 //
 // One matrix: 1,531 rows, 1,536 -> 2 x 8,960: 65 -> 59; 4,096, 3,584 -> 2 x 18,944: 811 -> 675 (1.65 PFLOP/s).
 //

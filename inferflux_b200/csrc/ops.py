@@ -1741,17 +1741,17 @@ class CudaKernels:
     # Which kernels make the experts of a bfloat16 step, by the number of (token, choice) pairs: per token, or, once the work is
     # MOE_TOKENS_MAX_WORK multiply-adds or there are MOE_TOKENS_MAX_PAIRS pairs, over rows sorted by expert, where every chosen
     # expert's weights are read once.  Measured on a B200, weights of two layers in turn (us, per token / sorted rows):
-    #     4 experts, 2,048 x 2,048, one a token           1 token (8M) 21 / 31, 4 (34M): 26 / 31, 16 (134M): 52 / 31, 64: 137 / 31
-    #     8 experts, 1,536 x 2,240 gated, two a token     1 token (21M) 33 / 26, 2 (41M): 42 / 32, 8: 62 / 44, 32: 166 / 45
-    #    16 experts, the same, one a token                1 token (10M) 19 / 23, 2 (21M): 24 / 25, 4 (41M): 33 / 31, 8: 45 / 41
-    #    16 experts, the same, four a token               1 token (41M) 62 / 34, 4: 82 / 55, 24: 243 / 72
-    #    64 experts, 1,536 x 512, four a token            1 token (6M) 17 / 22, 4 (25M): 26 / 26, 8 (50M): 30 / 31, 16: 48 / 42
-    #    64 experts, 2,048 x 1,408 gated, six a token     1 token (52M) 70 / 46, 4: 106 / 84
-    #   256 experts, 2,048 x 1,024 gated, eight a token   1 token (50M) 64 / 48, 4: 103 / 101, 16: 293 / 252
-    #    16 experts, 3,584 x 4,736 gated, four a token    1 token (204M) 154 / 93, 8: 506 / 266
+    #     4 experts, 2,048 x 2,048, one a token           1 token (8M) 21 / 31, 4 (34M): 21 / 31, 16 (134M): 52 / 30, 64: 137 / 30
+    #     8 experts, 1,536 x 2,240 gated, two a token     1 token (21M) 38 / 25, 2 (41M): 42 / 31, 8: 63 / 43, 32: 166 / 44
+    #    16 experts, the same, one a token                1 token (10M) 19 / 22, 2 (21M): 19 / 22, 4 (41M): 30 / 27, 8: 45 / 40
+    #    16 experts, the same, four a token               1 token (41M) 61 / 31, 4: 85 / 53, 24: 243 / 70
+    #    64 experts, 1,536 x 512, four a token            1 token (6M) 17 / 21, 4 (25M): 25 / 25, 8 (50M): 31 / 31, 16: 48 / 42
+    #    64 experts, 2,048 x 1,408 gated, six a token     1 token (52M) 70 / 40, 4: 111 / 88
+    #   256 experts, 2,048 x 1,024 gated, eight a token   1 token (50M) 64 / 42, 4: 103 / 94, 16: 282 / 221
+    #    16 experts, 3,584 x 4,736 gated, four a token    1 token (204M) 153 / 88, 8: 520 / 257
     # Of the sorted rows, steps of few pairs an expert ("stream") cut the second product's K into slices and take the exact
     # exponential and division; the others ("tiles") do not.  A result's bits depend on that line, which lies where a kernel of its
-    # own for few pairs was slower than tiles; the time does so little (the last row 251 instead of 266).
+    # own for few pairs was slower than tiles; the time does so little (the last row 252 instead of 257).
     MOE_TILES_MIN_PAIRS = 192
     MOE_TILES_LARGE_EXPERT = 1 << 23
     MOE_TOKENS_MAX_WORK = 40_000_000
