@@ -242,36 +242,14 @@ __global__ void __launch_bounds__(kDeltaThreads) delta_scan_kernel(
   }
 }
 
-// y = o / rms(o) per head * norm_w * sigmoid(g): a warp per (token, head).
-template <typename TO>
-__global__ void delta_finish_kernel(const float* __restrict__ o, const float* __restrict__ proj, int ld,
-                                    const float* __restrict__ norm_w, float eps, TO* __restrict__ y, int num_tokens,
-                                    int heads, int dim) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + warp;
-  if (item >= (long long)num_tokens * heads) return;
-  const int t = (int)(item / heads), h = (int)(item % heads);
-  const int HD = heads * dim;
-  const float* orow = o + (size_t)t * HD + h * dim;
-  const float* g = proj + (size_t)t * ld + 3 * HD + h * dim;
-  float ss = 0.0f;
-  for (int i = lane; i < dim; i += 32) ss = fmaf(orow[i], orow[i], ss);
-  ss = warp_sum(ss);
-  const float r = rsqrtf(ss / (float)dim + eps);
-  for (int i = lane; i < dim; i += 32)
-    y[(size_t)t * HD + h * dim + i] = from_f32<TO>(orow[i] * r * norm_w[h * dim + i] * sigmoid_f(g[i]));
-}
+int launch_gated_heads(const float* y, const float* gate, long long gate_stride, const float* w, int w_size, float eps, void* out, int T,
+                       int C, int groups, int gate_first, int sigmoid, int root, int out_dtype, cudaStream_t stream);      // pair_mixer.cu
 
+// y = o / rms(o) per head * norm_w * sigmoid(g)
 int launch_delta_finish(const float* o, const float* proj, int ld, const float* norm_w, float eps, void* y, int num_tokens, int heads,
                         int dim, int out_dtype, cudaStream_t stream) {
-  const unsigned blocks = (unsigned)(((long long)num_tokens * heads + 3) / 4);
-  if (out_dtype == IFX_DT_F32)
-    delta_finish_kernel<float><<<blocks, 128, 0, stream>>>(o, proj, ld, norm_w, eps, (float*)y, num_tokens, heads, dim);
-  else if (out_dtype == IFX_DT_BF16)
-    delta_finish_kernel<__nv_bfloat16><<<blocks, 128, 0, stream>>>(o, proj, ld, norm_w, eps, (__nv_bfloat16*)y, num_tokens, heads, dim);
-  else return IFX_E_DTYPE;
-  IFX_CHECK_LAUNCH();
-  return 0;
+  return launch_gated_heads(o, proj + 3 * (size_t)heads * dim, ld, norm_w, heads * dim, eps, y, num_tokens, heads * dim, heads, 0, 1, 0,
+                            out_dtype, stream);
 }
 
 // Preparation and scan of the spans of up to max_span tokens: their rows of o and their states.  scratch: as

@@ -12,6 +12,8 @@
 // Norms, sums and gates are float32 whatever the dtype of what comes in or goes out.
 #include "common.cuh"
 
+#include <type_traits>
+
 namespace ifx {
 
 __device__ __forceinline__ float load_as_f32(const void* p, int dtype, size_t i) {
@@ -96,40 +98,208 @@ __global__ void gate_mul_kernel(const void* __restrict__ a, const void* __restri
 
 __device__ __forceinline__ float gate_value(float g, int sigmoid) { return (sigmoid ? 1.0f : g) / (1.0f + expf(-g)); }
 
-// One block a row, a warp a part at a time.  y [T, C] float32 contiguous; gate float32 with a row stride.
-__global__ void __launch_bounds__(256) gated_groupnorm_kernel(const float* __restrict__ y, const float* __restrict__ gate,
-                                                              long long gate_stride, const float* __restrict__ w, int w_size,
-                                                              float eps, void* __restrict__ out, int C, int groups,
-                                                              int gate_first, int sigmoid, int out_dtype) {
-  const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-  const int part = C / groups;
-  const float* yr = y + (size_t)t * C;
-  const float* gr = gate + (size_t)t * gate_stride;
-  for (int p = warp; p < groups; p += nwarps) {
+// Parts of up to 256 numbers: a warp takes up to four neighbouring parts and has the reads of all of them on their way before it sums
+// the first.  ROOT: one over a square root in the place of rsqrtf (wkv.cu's norm, which its scan makes too: the same bits).
+// Bound: instructions (an exponential and a division a number), then HBM.  A warp a part, its two reads after one another, a 64-bit
+// division a part -> the kernel below, us: 1,500 rows of 24 parts of 64 16.5 -> 9.7; of 12 of 128 11.1 -> 6.5 (4.2 TB/s).
+constexpr int kHeadsAtOnce = 4;
+template <typename TO, int PER, bool ROOT>
+__global__ void __launch_bounds__(256) gated_heads_kernel(const float* __restrict__ y, const float* __restrict__ gate, long long gate_stride,
+                                                          const float* __restrict__ w, int w_wide, float eps, TO* __restrict__ out,
+                                                          unsigned items, unsigned groups, int part, int gate_first, int sigmoid, unsigned each) {
+  const int lane = threadIdx.x & 31;
+  const unsigned first = (blockIdx.x * 8 + (threadIdx.x >> 5)) * each;
+  pdl_launch_dependents();
+  pdl_wait();
+  if (first >= items) return;
+  float v[kHeadsAtOnce][PER], g[kHeadsAtOnce][PER];
+  int p[kHeadsAtOnce];
+  unsigned t = first / groups, at = first - t * groups;      // (one division: they cost more than the reads)
+#pragma unroll
+  for (unsigned k = 0; k < kHeadsAtOnce; ++k) {
+    const unsigned item = first + k;
+    const bool live = k < each && item < items;
+    p[k] = (int)at;
+    const float* yr = y + (size_t)item * part;
+    const float* gr = gate + (long long)t * gate_stride + (size_t)at * part;
+    if (++at == groups) at = 0, ++t;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const int e = lane + 32 * j;
+      v[k][j] = live && e < part ? yr[e] : 0.0f;
+      g[k][j] = live && e < part ? gr[e] : 0.0f;
+    }
+  }
+#pragma unroll
+  for (unsigned k = 0; k < kHeadsAtOnce; ++k) {
+    const unsigned item = first + k;
+    if (k >= each || item >= items) break;
     float ss = 0.0f;
-    for (int e = lane; e < part; e += 32) {
-      const int c = p * part + e;
-      float v = yr[c];
-      if (gate_first) {
-        v *= gate_value(gr[c], sigmoid);
-      }
-      ss = fmaf(v, v, ss);
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      g[k][j] = gate_value(g[k][j], sigmoid);
+      if (gate_first) v[k][j] *= g[k][j];
+      ss = lane + 32 * j < part ? fmaf(v[k][j], v[k][j], ss) : ss;
     }
     ss = warp_sum(ss);
-    const float inv = rsqrtf(ss / (float)part + eps);
-    for (int e = lane; e < part; e += 32) {
-      const int c = p * part + e;
-      const float sg = gate_value(gr[c], sigmoid);
-      float v = yr[c];
-      if (gate_first) v *= sg;
-      v = v * inv * (w ? w[w_size == C ? c : e] : 1.0f);
-      if (!gate_first) v *= sg;
-      store_from_f32(out, out_dtype, (size_t)t * C + c, v);
+    const float mean = ss / (float)part + eps, inv = ROOT ? 1.0f / sqrtf(mean) : rsqrtf(mean);
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const int e = lane + 32 * j;
+      if (e >= part) continue;
+      float o = v[k][j] * inv * (w ? w[(w_wide ? p[k] * part : 0) + e] : 1.0f);
+      if (!gate_first) o *= g[k][j];
+      out[(size_t)item * part + e] = from_f32<TO>(o);
     }
   }
 }
 
-// The same for few, long parts: the whole block works on one part after the other.
+// The same for parts of 64 (sixteen lanes a part) and 128, without a look at any bound but the last part's: the same sums in the same
+// order, so the same bits.
+template <typename TO, int PART, bool ROOT>
+__global__ void __launch_bounds__(256) gated_heads_full_kernel(const float* __restrict__ y, const float* __restrict__ gate, long long gate_stride,
+                                                               const float* __restrict__ w, int w_wide, float eps, TO* __restrict__ out,
+                                                               unsigned items, unsigned groups, int gate_first, int sigmoid, unsigned each) {
+  constexpr int LANES = PART / 4, ACROSS = 32 / LANES;
+  const unsigned lane = threadIdx.x & (LANES - 1), warp = threadIdx.x >> 5;
+  unsigned item = (blockIdx.x * 8 + warp) * (each * ACROSS) + (threadIdx.x & 31) / LANES;
+  pdl_launch_dependents();
+  pdl_wait();
+  unsigned t = item / groups, at = item - t * groups;
+  float v[kHeadsAtOnce][4], g[kHeadsAtOnce][4];
+  const float* yr = y + (size_t)item * PART + lane;
+  unsigned place[kHeadsAtOnce];
+#pragma unroll
+  for (unsigned k = 0; k < kHeadsAtOnce; ++k) {
+    place[k] = at;
+    if (k < each && item + k * ACROSS < items) {
+      const float* gr = gate + (long long)t * gate_stride + at * PART + lane;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        v[k][j] = yr[k * ACROSS * PART + LANES * j];
+        g[k][j] = gr[LANES * j];
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[k][j] = g[k][j] = 0.0f;
+    }
+    at += ACROSS;
+    while (at >= groups) at -= groups, ++t;
+  }
+  TO* to = out + (size_t)item * PART + lane;
+#pragma unroll
+  for (unsigned k = 0; k < kHeadsAtOnce; ++k) {
+    if (k >= each) break;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      g[k][j] = gate_value(g[k][j], sigmoid);
+      if (gate_first) v[k][j] *= g[k][j];
+    }
+    float ss;
+    if (LANES == 16) ss = fmaf(v[k][2], v[k][2], v[k][0] * v[k][0]) + fmaf(v[k][3], v[k][3], v[k][1] * v[k][1]);
+    else ss = fmaf(v[k][3], v[k][3], fmaf(v[k][2], v[k][2], fmaf(v[k][1], v[k][1], v[k][0] * v[k][0])));
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float mean = ss / (float)PART + eps, inv = ROOT ? 1.0f / sqrtf(mean) : rsqrtf(mean);
+    if (item + k * ACROSS >= items) continue;
+    const float* wr = w + (w_wide ? place[k] * PART : 0) + lane;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float o = v[k][j] * inv * (w ? wr[LANES * j] : 1.0f);
+      if (!gate_first) o *= g[k][j];
+      to[k * ACROSS * PART + LANES * j] = from_f32<TO>(o);
+    }
+  }
+}
+
+// w_size: numbers of w, a row's or a part's.  Parts of up to 256.
+int launch_gated_heads(const float* y, const float* gate, long long gate_stride, const float* w, int w_size, float eps, void* out, int T,
+                       int C, int groups, int gate_first, int sigmoid, int root, int out_dtype, cudaStream_t stream) {
+  const int part = C / groups;
+  if (part > 256 || (long long)T * groups > 0x7fffffffLL - 32) return IFX_E_TOOBIG;
+  if (out_dtype != IFX_DT_F32 && out_dtype != IFX_DT_BF16) return IFX_E_DTYPE;
+  const unsigned items = (unsigned)T * (unsigned)groups;
+  // several parts a warp only where all SMs have their fill of warps without
+  const unsigned across = part == 64 ? 2 : 1, turns = items / across;
+  const unsigned each = turns >= 148 * 64 * 2 ? 4 : turns >= 148 * 64 ? 2 : 1;
+  const unsigned blocks = (items + 8 * each * across - 1) / (8 * each * across);
+  static_assert(kHeadsAtOnce == 4, "each");
+  auto full = [&](auto* to, auto kern) {
+    return launch_pdl(kern, dim3(blocks), dim3(256), 0, stream, 1, y, gate, gate_stride, w, w_size == C ? 1 : 0, eps, to, items, (unsigned)groups,
+                      gate_first, sigmoid, each);
+  };
+  auto run = [&](auto* to, auto kern) {
+    return launch_pdl(kern, dim3(blocks), dim3(256), 0, stream, 1, y, gate, gate_stride, w, w_size == C ? 1 : 0, eps, to, items, (unsigned)groups, part,
+                      gate_first, sigmoid, each);
+  };
+  auto with = [&](auto* to) {
+    using TO = std::remove_pointer_t<decltype(to)>;
+    if (part == 64) return root ? full(to, gated_heads_full_kernel<TO, 64, true>) : full(to, gated_heads_full_kernel<TO, 64, false>);
+    if (part == 128) return root ? full(to, gated_heads_full_kernel<TO, 128, true>) : full(to, gated_heads_full_kernel<TO, 128, false>);
+    return root ? run(to, gated_heads_kernel<TO, 8, true>) : run(to, gated_heads_kernel<TO, 8, false>);
+  };
+  return out_dtype == IFX_DT_F32 ? with(static_cast<float*>(out)) : with(static_cast<__nv_bfloat16*>(out));
+}
+
+// Longer parts on 16-byte boundaries: a block a part, which stays in registers between the sum and the store.
+// Bound: HBM.  1,901 rows of 1,536: 16.1 us with a number a thread at a time, read twice, so 8.8 (3.3 TB/s).
+constexpr int kPartKept = 4;
+template <typename TO>
+__global__ void __launch_bounds__(512) gated_part_kernel(const float* __restrict__ y, const float* __restrict__ gate, long long gate_stride,
+                                                         const float* __restrict__ w, int w_wide, float eps, TO* __restrict__ out, int C,
+                                                         int part, int gate_first, int sigmoid) {
+  __shared__ float scratch[32];
+  const int t = blockIdx.x, p = blockIdx.y, step = blockDim.x * 4;
+  pdl_launch_dependents();
+  pdl_wait();
+  const float* yr = y + (size_t)t * C + (size_t)p * part;
+  const float* gr = gate + (size_t)t * gate_stride + (size_t)p * part;
+  const float* wr = w ? w + (w_wide ? (size_t)p * part : 0) : nullptr;
+  float4 v[kPartKept], g[kPartKept];
+#pragma unroll
+  for (int c = 0; c < kPartKept; ++c) {
+    const int e = threadIdx.x * 4 + c * step;
+    v[c] = g[c] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (e < part) {
+      v[c] = *reinterpret_cast<const float4*>(yr + e);
+      g[c] = *reinterpret_cast<const float4*>(gr + e);
+    }
+  }
+  float ss = 0.0f;
+#pragma unroll
+  for (int c = 0; c < kPartKept; ++c) {
+    if (threadIdx.x * 4 + c * step >= part) continue;
+    g[c] = make_float4(gate_value(g[c].x, sigmoid), gate_value(g[c].y, sigmoid), gate_value(g[c].z, sigmoid), gate_value(g[c].w, sigmoid));
+    if (gate_first) {
+      v[c].x *= g[c].x; v[c].y *= g[c].y; v[c].z *= g[c].z; v[c].w *= g[c].w;
+    }
+    ss = fmaf(v[c].x, v[c].x, ss);
+    ss = fmaf(v[c].y, v[c].y, ss);
+    ss = fmaf(v[c].z, v[c].z, ss);
+    ss = fmaf(v[c].w, v[c].w, ss);
+  }
+  ss = block_sum(ss, scratch);
+  const float inv = rsqrtf(ss / (float)part + eps);
+#pragma unroll
+  for (int c = 0; c < kPartKept; ++c) {
+    const int e = threadIdx.x * 4 + c * step;
+    if (e >= part) continue;
+    const float4 x = wr ? *reinterpret_cast<const float4*>(wr + e) : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+    float4 o = make_float4(v[c].x * inv * x.x, v[c].y * inv * x.y, v[c].z * inv * x.z, v[c].w * inv * x.w);
+    if (!gate_first) {
+      o.x *= g[c].x; o.y *= g[c].y; o.z *= g[c].z; o.w *= g[c].w;
+    }
+    TO* to = out + (size_t)t * C + (size_t)p * part + e;
+    if constexpr (sizeof(TO) == 4) {
+      *reinterpret_cast<float4*>(to) = o;
+    } else {
+      __nv_bfloat162 b[2] = {__floats2bfloat162_rn(o.x, o.y), __floats2bfloat162_rn(o.z, o.w)};
+      *reinterpret_cast<uint2*>(to) = *reinterpret_cast<uint2*>(b);
+    }
+  }
+}
+
+// Any part and alignment: the whole block works on one part after the other.  y [T, C] float32 contiguous; gate float32 with a row stride.
 __global__ void __launch_bounds__(512) gated_groupnorm_wide_kernel(const float* __restrict__ y, const float* __restrict__ gate,
                                                                    long long gate_stride, const float* __restrict__ w,
                                                                    int w_size, float eps, void* __restrict__ out, int C,
@@ -263,15 +433,18 @@ int ifx_gated_groupnorm(const float* y, const float* gate, long long gate_stride
   if (C <= 0 || groups <= 0 || C % groups || (w != nullptr && w_size != C && w_size != C / groups) || gate_stride < C) return IFX_E_BADARG;
   if (out_dtype != IFX_DT_F32 && out_dtype != IFX_DT_BF16) return IFX_E_DTYPE;
   const int part = C / groups;
-  if (groups < 8 && part > 64) {                            // few long parts: a block per row takes them in turn
-    const int threads = part >= 2048 ? 512 : (part >= 256 ? 256 : ((part + 31) / 32) * 32);
-    gated_groupnorm_wide_kernel<<<T, threads, 0, stream>>>(y, gate, gate_stride, w, w_size, eps, out, C, groups, gate_first,
-                                                           sigmoid, out_dtype);
-  } else {
-    const int warps = groups >= 8 ? 8 : groups;
-    gated_groupnorm_kernel<<<T, warps * 32, 0, stream>>>(y, gate, gate_stride, w, w_size, eps, out, C, groups, gate_first,
-                                                        sigmoid, out_dtype);
+  if (part <= 256 && (long long)T * groups <= 0x7fffffffLL - 32) return launch_gated_heads(y, gate, gate_stride, w, w_size, eps, out, T, C, groups, gate_first, sigmoid, 0, out_dtype, stream);
+  const bool aligned = part % 4 == 0 && gate_stride % 4 == 0 && ((uintptr_t)y | (uintptr_t)gate | (uintptr_t)w | (uintptr_t)out) % 16 == 0;
+  if (aligned && part <= 512 * 4 * kPartKept && groups <= 65535) {
+    const int threads = ((part + 4 * kPartKept - 1) / (4 * kPartKept) + 31) / 32 * 32;      // of the part's size alone, as the sum's order
+    if (out_dtype == IFX_DT_F32)
+      return launch_pdl(gated_part_kernel<float>, dim3(T, groups), dim3(threads), 0, stream, 1, y, gate, gate_stride, w, w_size == C ? 1 : 0, eps,
+                        (float*)out, C, part, gate_first, sigmoid);
+    return launch_pdl(gated_part_kernel<__nv_bfloat16>, dim3(T, groups), dim3(threads), 0, stream, 1, y, gate, gate_stride, w, w_size == C ? 1 : 0,
+                      eps, (__nv_bfloat16*)out, C, part, gate_first, sigmoid);
   }
+  const int threads = part >= 2048 ? 512 : 256;
+  gated_groupnorm_wide_kernel<<<T, threads, 0, stream>>>(y, gate, gate_stride, w, w_size, eps, out, C, groups, gate_first, sigmoid, out_dtype);
   IFX_CHECK_LAUNCH();
   return 0;
 }
