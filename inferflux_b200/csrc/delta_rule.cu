@@ -11,8 +11,8 @@
 // request's tokens: a column of S (one value channel, all key channels) never meets another column, so the grid is
 // (requests, heads, groups of columns); a column's key channels are cut into slices of 8 that neighbouring lanes keep
 // in registers, and the two sums over key channels are added across a column's lanes by shuffles.  The step's vectors
-// of a stretch of tokens arrive by cp.async in one of two buffers while the other is worked on.  delta_finish (a warp
-// per token and head) norms and gates.  Everything is float32, and every sum's order is a function of the head size
+// of a stretch of tokens arrive by cp.async in one of two buffers while the other is worked on.  A warp
+// per token and head norms and gates.  Everything is float32, and every sum's order is a function of the head size
 // alone, so a token's result does not depend on how its request's tokens were cut into steps or on what else is in the
 // batch.
 //

@@ -32,20 +32,15 @@ namespace ifx {
 
 constexpr int kMaxRouterOutputs = 1024;
 
-__global__ void moe_route_kernel(const float* __restrict__ z, const float* __restrict__ correction,
-                                 int* __restrict__ ids, float* __restrict__ weights, int T, int n, int top, int of_chosen,
-                                 float floor) {
+// One token's choice by a warp: zr its n logits, score_s and choice_s room for n numbers each.
+__device__ __forceinline__ void route_token(const float* zr, const float* __restrict__ correction, float* score_s, float* choice_s,
+                                            int* __restrict__ ids, float* __restrict__ weights, int n, int top, int of_chosen, float floor,
+                                            int lane) {
   const bool sigmoid = of_chosen == 2;
-  __shared__ float score_s[4][kMaxRouterOutputs];
-  __shared__ float choice_s[4][kMaxRouterOutputs];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t = blockIdx.x * 4 + warp;
-  if (t >= T) return;
-  const float* zr = z + (size_t)t * n;
   if (of_chosen == 1) {
     for (int i = lane; i < n; i += 32) {
-      score_s[warp][i] = zr[i];
-      choice_s[warp][i] = zr[i] + (correction ? correction[i] : 0.0f);
+      score_s[i] = zr[i];
+      choice_s[i] = zr[i] + (correction ? correction[i] : 0.0f);
     }
     __syncwarp();
     float m = -INFINITY;                                // the largest chosen logit, known to lane 0
@@ -53,7 +48,7 @@ __global__ void moe_route_kernel(const float* __restrict__ z, const float* __res
       float best = -INFINITY;
       int at = 0x7fffffff;
       for (int i = lane; i < n; i += 32) {
-        const float v = choice_s[warp][i];
+        const float v = choice_s[i];
         if (v > best) { best = v; at = i; }
       }
 #pragma unroll
@@ -64,20 +59,20 @@ __global__ void moe_route_kernel(const float* __restrict__ z, const float* __res
       }
       if (at >= n) at = 0;
       if (lane == 0) {
-        ids[(size_t)t * top + c] = at;
-        m = fmaxf(m, score_s[warp][at]);
-        choice_s[warp][at] = -INFINITY;
+        ids[c] = at;
+        m = fmaxf(m, score_s[at]);
+        choice_s[at] = -INFINITY;
       }
       __syncwarp();
     }
     if (lane == 0) {                                     // softmax over the chosen alone, in the order of the choice
       float sum = 0.0f;
       for (int c = 0; c < top; ++c) {
-        const float e = expf(score_s[warp][ids[(size_t)t * top + c]] - m);
-        weights[(size_t)t * top + c] = e;
+        const float e = expf(score_s[ids[c]] - m);
+        weights[c] = e;
         sum += e;
       }
-      for (int c = 0; c < top; ++c) weights[(size_t)t * top + c] /= sum;
+      for (int c = 0; c < top; ++c) weights[c] /= sum;
     }
     return;
   }
@@ -87,21 +82,21 @@ __global__ void moe_route_kernel(const float* __restrict__ z, const float* __res
   float sum = 0.0f;
   for (int i = lane; i < n; i += 32) {
     const float e = sigmoid ? 1.0f / (1.0f + expf(-zr[i])) : expf(zr[i] - m);
-    score_s[warp][i] = e;
+    score_s[i] = e;
     sum += e;
   }
   sum = sigmoid ? 1.0f : warp_sum(sum);
   for (int i = lane; i < n; i += 32) {
-    const float sc = score_s[warp][i] / sum;
-    score_s[warp][i] = sc;
-    choice_s[warp][i] = sc + (correction ? correction[i] : 0.0f);
+    const float sc = score_s[i] / sum;
+    score_s[i] = sc;
+    choice_s[i] = sc + (correction ? correction[i] : 0.0f);
   }
   __syncwarp();
   for (int c = 0; c < top; ++c) {
     float best = -INFINITY;
     int at = 0x7fffffff;
     for (int i = lane; i < n; i += 32) {
-      const float v = choice_s[warp][i];
+      const float v = choice_s[i];
       if (v > best) { best = v; at = i; }              // i ascends: the earlier index stays on a tie
     }
 #pragma unroll
@@ -112,17 +107,168 @@ __global__ void moe_route_kernel(const float* __restrict__ z, const float* __res
     }
     if (at >= n) at = 0;                               // only if every score is NaN
     if (lane == 0) {
-      ids[(size_t)t * top + c] = at;
-      weights[(size_t)t * top + c] = score_s[warp][at];
-      choice_s[warp][at] = -INFINITY;
+      ids[c] = at;
+      weights[c] = score_s[at];
+      choice_s[at] = -INFINITY;
     }
     __syncwarp();
   }
   if (sigmoid && lane == 0) {                            // the chosen scores over their sum, added in the order of the choice
     float total = 0.0f;
-    for (int c = 0; c < top; ++c) total += weights[(size_t)t * top + c];
+    for (int c = 0; c < top; ++c) total += weights[c];
     total += floor;
-    for (int c = 0; c < top; ++c) weights[(size_t)t * top + c] /= total;
+    for (int c = 0; c < top; ++c) weights[c] /= total;
+  }
+}
+
+__global__ void moe_route_kernel(const float* __restrict__ z, const float* __restrict__ correction,
+                                 int* __restrict__ ids, float* __restrict__ weights, int T, int n, int top, int of_chosen,
+                                 float floor) {
+  __shared__ float score_s[4][kMaxRouterOutputs];
+  __shared__ float choice_s[4][kMaxRouterOutputs];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int t = blockIdx.x * 4 + warp;
+  if (t >= T) return;
+  route_token(z + (size_t)t * n, correction, score_s[warp], choice_s[warp], ids + (size_t)t * top, weights + (size_t)t * top, n, top, of_chosen,
+              floor, lane);
+}
+
+// The same for up to 64 outputs and 32 choices without memory in between: a lane keeps two outputs' scores and one choice.  The largest is
+// found by one reduction of ordered bits, and on a tie the earlier index by one vote.
+__device__ __forceinline__ void route_token_small(const float* z_s, const float* __restrict__ correction, int* __restrict__ ids,
+                                                  float* __restrict__ weights, int n, int top, int of_chosen, float floor, int lane) {
+  const unsigned all = 0xffffffffu;
+  float score[2], choice[2];
+  bool in[2];
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    in[j] = lane + 32 * j < n;
+    score[j] = in[j] ? z_s[lane + 32 * j] : -INFINITY;
+  }
+  if (of_chosen == 2) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j) score[j] = 1.0f / (1.0f + expf(-score[j]));
+  } else if (of_chosen == 0) {
+    const float m = warp_max(fmaxf(score[0], score[1]));
+    float sum = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      if (in[j]) sum += score[j] = expf(score[j] - m);
+    sum = warp_sum(sum);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) score[j] /= sum;
+  }
+  unsigned key[2];                                         // ordered as the numbers are; 0: not to be chosen (NaN, -inf, chosen before)
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    choice[j] = (in[j] && correction ? score[j] + correction[lane + 32 * j] : score[j]) + 0.0f;       // (one zero)
+    const unsigned u = __float_as_uint(choice[j]);
+    key[j] = in[j] && choice[j] > -INFINITY ? (u & 0x80000000u ? ~u : u | 0x80000000u) : 0u;
+  }
+  float mine = -INFINITY;                                  // the lane-th choice's score
+  int at_mine = 0;
+  for (int c = 0; c < top; ++c) {
+    const unsigned best = __reduce_max_sync(all, max(key[0], key[1]));
+    const unsigned first = __ballot_sync(all, key[0] == best), second = __ballot_sync(all, key[1] == best);
+    const int at = best == 0 ? 0 : first ? __ffs(first) - 1 : 31 + __ffs(second);
+    const float s = __shfl_sync(all, at < 32 ? score[0] : score[1], at & 31);
+    if (lane == c) mine = s, at_mine = at;
+    if (lane == at) key[0] = 0;
+    if (lane + 32 == at) key[1] = 0;
+  }
+  if (of_chosen) {                                         // in the order of the choice
+    float m = warp_max(mine), sum = 0.0f;
+    if (of_chosen == 1) mine = lane < top ? expf(mine - m) : 0.0f;
+    for (int c = 0; c < top; ++c) sum += __shfl_sync(all, mine, c);
+    mine /= of_chosen == 2 ? sum + floor : sum;
+  }
+  if (lane < top) {
+    ids[lane] = at_mine;
+    weights[lane] = mine;
+  }
+}
+
+// Router and choice of a bfloat16 step in one launch, up to 64 outputs: 16 tokens a block, whose sixteen warps (eight for more than 32 outputs) share the inner size 32 numbers
+// at a time and add up in the order of the warps, so a token's logits depend on nothing else in the step.  A lane reads 16 bytes of a
+// row, of which it feeds the first half to one mma.sync of 16 and the second to the next: both operands are permuted alike.
+// Bound: latency (the rows' reads, then the choice).  Library product (with its own sum of slices for 18 outputs) and the kernel above -> this,
+// us: 24 tokens of 1,536 to 16 outputs 7.2 -> 3.4; 2,048 to 18 12.4 -> 4.1.
+constexpr int kRouterMost = 64, kRouterAhead = 3;
+template <int NT>
+struct RouterWarps { static constexpr int N = NT <= 4 ? 16 : 8; };      // (shared memory)
+template <int NT>
+__global__ void __launch_bounds__(RouterWarps<NT>::N * 32) moe_choose_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restrict__ w,
+                                                                       const float* __restrict__ correction, int* __restrict__ ids,
+                                                                       float* __restrict__ weights, int T, int K, int n, int top, int kind,
+                                                                       float floor) {
+  constexpr int kRouterWarps = RouterWarps<NT>::N;
+  __shared__ __align__(16) float part_s[kRouterWarps][16][NT * 8];
+  __shared__ float z_s[16][NT * 8], score_s[kRouterWarps][NT * 8], choice_s[kRouterWarps][NT * 8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = lane >> 2, t0 = blockIdx.x * 16, units = (K + 31) / 32;
+  const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+  uint4 a[kRouterAhead][2], b[kRouterAhead][NT];
+  auto column = [&](int u) { return u * 32 + 8 * (lane & 3); };
+  auto fetch_w = [&](int u0) {
+#pragma unroll
+    for (int i = 0; i < kRouterAhead; ++i) {
+      const int k = column(u0 + i * kRouterWarps);
+#pragma unroll
+      for (int j = 0; j < NT; ++j) b[i][j] = k < K && j * 8 + row < n ? __ldg(reinterpret_cast<const uint4*>(w + (size_t)(j * 8 + row) * K + k)) : none;
+    }
+  };
+  fetch_w(warp);                                           // (weights do not come from the kernel in front)
+  pdl_launch_dependents();
+  pdl_wait();
+  float acc[NT][4];
+#pragma unroll
+  for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
+  for (int u = warp; u < units; u += kRouterAhead * kRouterWarps) {
+#pragma unroll
+    for (int i = 0; i < kRouterAhead; ++i) {
+      const int k = column(u + i * kRouterWarps);
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int t = t0 + row + 8 * half;
+        a[i][half] = k < K && t < T ? *reinterpret_cast<const uint4*>(h + (size_t)t * K + k) : none;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kRouterAhead; ++i)
+#pragma unroll
+      for (int j = 0; j < NT; ++j) {
+        auto mma = [&](uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+          asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                       : "+f"(acc[j][0]), "+f"(acc[j][1]), "+f"(acc[j][2]), "+f"(acc[j][3])
+                       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+        };
+        mma(a[i][0].x, a[i][1].x, a[i][0].y, a[i][1].y, b[i][j].x, b[i][j].y);
+        mma(a[i][0].z, a[i][1].z, a[i][0].w, a[i][1].w, b[i][j].z, b[i][j].w);
+      }
+    if (u + kRouterAhead * kRouterWarps < units) fetch_w(u + kRouterAhead * kRouterWarps);
+  }
+#pragma unroll
+  for (int j = 0; j < NT; ++j) {
+    float* to = &part_s[warp][row][j * 8 + 2 * (lane & 3)];
+    *reinterpret_cast<float2*>(to) = make_float2(acc[j][0], acc[j][1]);
+    *reinterpret_cast<float2*>(to + 8 * NT * 8) = make_float2(acc[j][2], acc[j][3]);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 16 * NT * 8; i += kRouterWarps * 32) {
+    float z = (&part_s[0][0][0])[i];
+#pragma unroll
+    for (int v = 1; v < kRouterWarps; ++v) z += (&part_s[v][0][0])[i];
+    (&z_s[0][0])[i] = z;
+  }
+  __syncthreads();
+  for (int i = warp; i < 16 && t0 + i < T; i += kRouterWarps) {
+    int* to = ids + (size_t)(t0 + i) * top;
+    float* wt = weights + (size_t)(t0 + i) * top;
+    if (top <= 32) {
+      route_token_small(z_s[i], correction, to, wt, n, top, kind, floor, lane);
+    } else {
+      route_token(z_s[i], correction, score_s[warp], choice_s[warp], to, wt, n, top, kind, floor, lane);
+      __syncwarp();
+    }
   }
 }
 
@@ -465,6 +611,24 @@ int ifx_moe_route_kind(const float* z, const float* correction, int* ids, float*
   moe_route_kernel<<<(T + 3) / 4, 128, 0, stream>>>(z, correction, ids, weights, T, n, top, kind, floor);
   IFX_CHECK_LAUNCH();
   return 0;
+}
+
+// The same with the router in front of it: z = h [T, K] . w [n, K]^T, both bfloat16 on 16-byte boundaries, K a multiple of 8, n up to 64.
+int ifx_moe_choose(const void* h, const void* w, const float* correction, int* ids, float* weights, int T, int K, int n, int top, int kind,
+                   float floor, cudaStream_t stream) {
+  if (T <= 0) return 0;
+  if (K <= 0 || K % 8 || n <= 0 || top <= 0 || top > n || kind < 0 || kind > 2) return IFX_E_BADARG;
+  if (n > kRouterMost) return IFX_E_TOOBIG;
+  if (((uintptr_t)h | (uintptr_t)w) % 16) return IFX_E_ALIGN;
+  auto run = [&](auto kern, int warps = 16) {
+    return launch_pdl(kern, dim3((T + 15) / 16), dim3(warps * 32), 0, stream, 1, (const __nv_bfloat16*)h, (const __nv_bfloat16*)w, correction,
+                      ids, weights, T, K, n, top, kind, floor);
+  };
+  if (n <= 8) return run(moe_choose_kernel<1>);
+  if (n <= 16) return run(moe_choose_kernel<2>);
+  if (n <= 24) return run(moe_choose_kernel<3>);
+  if (n <= 32) return run(moe_choose_kernel<4>);
+  return run(moe_choose_kernel<8>, RouterWarps<8>::N);
 }
 
 int ifx_moe_route_ex(const float* z, const float* correction, int* ids, float* weights, int T, int n, int top,

@@ -164,7 +164,7 @@ class CudaKernels:
                    "ifx_groupnorm_stream", "ifx_residual_add_scaled", "ifx_gelu_mul_table", "ifx_embed_scaled", "ifx_scale_f32",
                    "ifx_delta_rule_scan", "ifx_latent_rope_append", "ifx_latent_attention_generic_rot", "ifx_moe_route_ex",
                    "ifx_moe_experts_ex", "ifx_latent_attention_mma_rot", "ifx_latent_attention_mma_supports_rot",
-                   "ifx_moe_route_kind", "ifx_moe_experts_glu", "ifx_norm_rope_append_ex",
+                   "ifx_moe_route_kind", "ifx_moe_choose", "ifx_moe_experts_glu", "ifx_norm_rope_append_ex",
                    "ifx_attention_generic_sink", "ifx_short_conv_ex", "ifx_decay_scan", "ifx_decay_scan_split", "ifx_bigram_add",
                    "ifx_rmsnorm_pair", "ifx_gate_mul", "ifx_gated_groupnorm", "ifx_pair_combine", "ifx_residual_add_vectors",
                    "ifx_attention_prefill_tcgen05_sink", "ifx_attention_prefill_bf16_sink", "ifx_attention_decode_bf16_sink",
@@ -1689,6 +1689,24 @@ class CudaKernels:
         _check(self.lib.ifx_moe_route_kind(_ptr(z), _ptr(correction), _ptr(ids), _ptr(weights), T, n, int(top),
                                            2 if kind == "sigmoid_normalized" else int(bool(of_chosen)), ctypes.c_float(floor),
                                            _stream()), "moe_route")
+        self.launches += 1
+        return ids, weights
+
+    def moe_choose(self, h, w_router, correction, top, of_chosen=False, kind=None, floor=0.0):
+        """`moe_route` of the router's logits h . w_router^T.  A bfloat16 router of up to 64 outputs takes one launch for both."""
+        n = w_router.shape[0]
+        if not (h.dtype == w_router.dtype == torch.bfloat16 and n <= 64 and h.is_contiguous() and w_router.is_contiguous()
+                and h.shape[1] == w_router.shape[1] and h.shape[1] % 8 == 0 and (h.data_ptr() | w_router.data_ptr()) % 16 == 0):
+            return self.moe_route(self.linear(h, w_router, out_dtype=torch.float32), correction, top, of_chosen=of_chosen, kind=kind, floor=floor)
+        _need(kind in (None, "sigmoid_normalized"), f"moe_choose: unknown kind {kind!r}")
+        _need(correction is None or (correction.dtype == torch.float32 and correction.is_contiguous() and correction.numel() == n),
+              "moe_choose: float32 corrections")
+        T = h.shape[0]
+        ids = torch.empty(T, top, dtype=torch.int32, device=h.device)
+        weights = torch.empty(T, top, dtype=torch.float32, device=h.device)
+        _check(self.lib.ifx_moe_choose(_ptr(h), _ptr(w_router), _ptr(correction), _ptr(ids), _ptr(weights), T, h.shape[1], n, int(top),
+                                       2 if kind == "sigmoid_normalized" else int(bool(of_chosen)), ctypes.c_float(floor), _stream()),
+               "moe_choose")
         self.launches += 1
         return ids, weights
 

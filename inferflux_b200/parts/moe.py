@@ -109,18 +109,21 @@ class MixtureOfExperts(FeedForward):
 
     def forward(self, h, ctx):
         k = ctx.kernels
-        z = k.linear(h, self.w_router, out_dtype=torch.float32)                   # [T, experts + identity]
+
+        def choose(correction, **kind):                                           # ids, weights [T, top]
+            both = getattr(k, "moe_choose", None)
+            if both is not None:
+                return both(h, self.w_router, correction, self.top, **kind)
+            return k.moe_route(k.linear(h, self.w_router, out_dtype=torch.float32), correction, self.top, **kind)
         if self.routing == "sigmoid_normalized":
-            ids, weights = k.moe_route(z, self.correction if self.has_correction else None, self.top,
-                                       kind="sigmoid_normalized", floor=self.weight_floor)
+            ids, weights = choose(self.correction if self.has_correction else None, kind="sigmoid_normalized", floor=self.weight_floor)
             y = k.moe_experts(h, self.w_up, self.w_down, ids, weights, self.experts, ctx.dtype, glu=self.glu)
             return y if self.shared is None else (y, self.shared.forward(h, ctx))
         if self.shared is not None:
             raise ValueError("moe: a shared expert beside softmax routing is not built")
         if self.routing == "softmax_of_chosen" or self.gated:
-            ids, weights = k.moe_route(z, self.correction if self.has_correction else None, self.top,
-                                       of_chosen=self.routing == "softmax_of_chosen")
+            ids, weights = choose(self.correction if self.has_correction else None, of_chosen=self.routing == "softmax_of_chosen")
             return k.moe_experts(h, self.w_up, self.w_down, ids, weights, self.experts, ctx.dtype,
                                  glu=self.glu)
-        ids, weights = k.moe_route(z, self.correction, self.top)
+        ids, weights = choose(self.correction)
         return k.moe_experts(h, self.w_up, self.w_down, ids, weights, self.experts, ctx.dtype)
