@@ -37,30 +37,6 @@
 
 namespace ifx {
 
-enum { CHUNK_CHANNEL = 0, CHUNK_STEP = 1, CHUNK_CONSTANT = 2, CHUNK_WKV = 3 };
-
-struct ChunkArgs {
-  const float* q; long long q_stride;
-  const float* k; long long k_stride;
-  const float* v; long long v_stride;
-  const float* raw; long long raw_stride;
-  float* state; long long state_slot_stride;
-  const int* req_slot; const int* cu_seqlens;
-  float* out;                                   // [T, heads dv]
-  const float* step_bias; const float* log_rate; const float* skip; const float* rate;      // per head
-  const float* w0; const float* u;              // CHUNK_WKV: per head and key channel
-  int requests, min_span, heads, groups, dv;    // shorter spans are left to the scans token by token
-  float inv_tau, q_scale;
-  float* local;                                 // [stretches, heads, dv, dk]: what a stretch adds, then the state in front of it
-  float* total;                                 // decays of a whole stretch: [stretches, heads, dk], or [stretches, heads] as two numbers each
-  float* reach;                                 // queries times decays since the stretch's beginning [T, heads dk], or decays [T, heads]
-  int key_rows;                                 // the request's state is [head, key channel, value channel]
-  const float* x; float* prev_state; int C;     // CHUNK_WKV: the step's input rows, where the last one of a request goes
-};
-
-__device__ __forceinline__ float chunk_log_sigmoid(float x) { return fminf(x, 0.0f) - log1pf(expf(-fabsf(x))); }
-__device__ __forceinline__ float chunk_softplus(float x) { return x > 20.0f ? x : log1pf(expf(x)); }
-
 template <int DK, int MODE>
 struct ChunkLayout {
   static constexpr bool CHANNEL = MODE == CHUNK_CHANNEL || MODE == CHUNK_WKV;
@@ -427,7 +403,7 @@ __global__ void __launch_bounds__(256) chunk_local_kernel(const ChunkArgs a) {
 template <bool CHANNEL>
 __global__ void __launch_bounds__(256) chunk_carry_kernel(const ChunkArgs a, int dk) {
   const int r = blockIdx.x, h = blockIdx.y, e = blockIdx.z * 256 + threadIdx.x;
-  const int lo = a.cu_seqlens[r], span = a.cu_seqlens[r + 1] - lo, chunks = chunks_of(span, a.min_span);
+  const int lo = a.cu_seqlens[r], span = a.cu_seqlens[r + 1] - lo, chunks = chunks_of(span, a.min_span, a.per);
   if (chunks == 0) return;
   if (a.x != nullptr && h == 0 && blockIdx.z == 0) {                       // the step's last input row
     float* to = a.prev_state + (long long)a.req_slot[r] * a.state_slot_stride;
@@ -439,7 +415,7 @@ __global__ void __launch_bounds__(256) chunk_carry_kernel(const ChunkArgs a, int
   float4 S;
   if (a.key_rows) S = make_float4(st[(size_t)c * a.dv + v], st[(size_t)(c + 1) * a.dv + v], st[(size_t)(c + 2) * a.dv + v], st[(size_t)(c + 3) * a.dv + v]);
   else S = make_float4(st[(size_t)v * dk + c], st[(size_t)v * dk + c + 1], st[(size_t)v * dk + c + 2], st[(size_t)v * dk + c + 3]);
-  const size_t base = (size_t)chunks_before(a.cu_seqlens, a.min_span, r) * a.heads + h;
+  const size_t base = (size_t)chunks_before(a.cu_seqlens, a.min_span, r, a.per) * a.heads + h;
   constexpr int U = 8;
   for (int c0 = 0; c0 < chunks; c0 += U) {
     float4 add[U], w[U];
@@ -586,6 +562,15 @@ static int launch_chunks(const ChunkArgs& a, int chunks, cudaStream_t stream) {
   return 0;
 }
 
+// The states in front of every stretch, for chunk_tcgen05.cu's stretches.
+int launch_chunk_carry(const ChunkArgs& a, int dk, cudaStream_t stream) {
+  chunk_carry_kernel<false><<<dim3(a.requests, a.heads, (a.dv * (dk / 4) + 255) / 256), 256, 0, stream>>>(a, dk);
+  IFX_CHECK_LAUNCH();
+  return 0;
+}
+int launch_chunks_of_128(const ChunkArgs& a, int dk, int mode, int chunks, int* error_flag, cudaStream_t stream);      // chunk_tcgen05.cu
+bool chunks_of_128_take(int mode, int dk, int dv);
+
 static int run_chunks(const ChunkArgs& a, int dk, int mode, int chunks, cudaStream_t stream) {
   if (dk == 64) {
     if (mode == CHUNK_CHANNEL) return launch_chunks<64, CHUNK_CHANNEL>(a, chunks, stream);
@@ -637,12 +622,20 @@ long long ifx_chunk_scan_scratch_floats(int num_tokens, int requests, int min_sp
   return chunks * heads * dv * dk + total + (per_channel ? (long long)num_tokens * heads * dk : (long long)num_tokens * heads);
 }
 
-// As ifx_decay_scan_rate (decay_scan.cu), with scratch as above; every row on a 16-byte boundary (IFX_E_ALIGN otherwise).
+// Whether a decay per head goes by stretches of 128 tokens (chunk_tcgen05.cu) where they take the sizes: when the blocks of the stretches of
+// 64 would not all have an SM of their own.  us, by 64 and by 128: 12 heads of 128 x 128, one span of 300 tokens 31 / 34, 512 43 / 35,
+// 2,048 120 / 62; 12 of 64 x 128 22 / 27, 29 / 27, 69 / 47; 24 of 128 x 64 31 / 31, 44 / 31, 115 / 78; 28 of 128 x 128, 128 tokens 44 / 35.
+int ifx_chunk_scan_takes_128(int num_tokens, int num_requests, int min_span, int heads, int dv) {
+  return (long long)chunks_at_most(num_tokens, num_requests, min_span) * heads * (dv / 64) > 148;
+}
+
+// As ifx_decay_scan_rate (decay_scan.cu), with scratch as above; every row on a 16-byte boundary (IFX_E_ALIGN otherwise).  stretch: 64 or 128
+// tokens (where those take the sizes), or 0 for what ifx_chunk_scan_takes_128 says.
 int ifx_chunk_decay_scan(const float* q, long long q_stride, const float* k, long long k_stride, const float* v, long long v_stride,
                          const float* raw, long long raw_stride, float* state, long long state_slot_stride, const int* req_slot,
                          const int* cu_seqlens, float* out, const float* step_bias, const float* log_rate, const float* skip,
                          int num_requests, int num_tokens, int min_span, int heads, int groups, int dk, int dv, int mode, float tau,
-                         float q_scale, float* scratch, const float* rate, cudaStream_t stream) {
+                         float q_scale, float* scratch, const float* rate, int stretch, int* error_flag, cudaStream_t stream) {
   if (num_requests <= 0 || num_tokens <= 0 || num_tokens < min_span) return 0;
   if (!ifx_chunk_scan_supports(num_requests, heads, dk, dv) || groups <= 0 || heads % groups || mode < 0 || mode > 2 || scratch == nullptr)
     return IFX_E_BADARG;
@@ -651,7 +644,9 @@ int ifx_chunk_decay_scan(const float* q, long long q_stride, const float* k, lon
   if (!rows_fit(q, q_stride) || !rows_fit(k, k_stride) || !rows_fit(v, v_stride) || (mode == 0 && !rows_fit(raw, raw_stride)) ||
       !rows_fit(scratch, 0) || !rows_fit(out, 0))
     return IFX_E_ALIGN;
-  const int chunks = chunks_at_most(num_tokens, num_requests, min_span);
+  const int per = (stretch == 128 || (stretch == 0 && ifx_chunk_scan_takes_128(num_tokens, num_requests, min_span, heads, dv))) &&
+                          chunks_of_128_take(mode, dk, dv) && error_flag != nullptr ? 128 : kChunk;
+  const int chunks = chunks_at_most(num_tokens, num_requests, min_span, per);
   ChunkArgs a = {};
   a.q = q; a.q_stride = q_stride; a.k = k; a.k_stride = k_stride; a.v = v; a.v_stride = v_stride; a.raw = raw; a.raw_stride = raw_stride;
   a.state = state; a.state_slot_stride = state_slot_stride; a.req_slot = req_slot; a.cu_seqlens = cu_seqlens; a.out = out;
@@ -659,9 +654,11 @@ int ifx_chunk_decay_scan(const float* q, long long q_stride, const float* k, lon
   a.requests = num_requests; a.min_span = min_span; a.heads = heads; a.groups = groups; a.dv = dv;
   a.inv_tau = mode == 0 ? 1.0f / tau : 0.0f;
   a.q_scale = q_scale;
+  a.per = per;
   a.local = scratch;
   a.total = scratch + (size_t)chunks * heads * dv * dk;
   a.reach = a.total + ((mode == 0 ? (size_t)chunks * heads * dk : (size_t)2 * chunks * heads) + 3) / 4 * 4;
+  if (per == 128) return launch_chunks_of_128(a, dk, mode, chunks, error_flag, stream);
   return run_chunks(a, dk, mode, chunks, stream);
 }
 
@@ -682,6 +679,7 @@ int ifx_chunk_wkv_scan(const float* r, const float* k, const float* v, const flo
   a.w0 = w0; a.u = u; a.x = x; a.prev_state = prev_state; a.C = C;
   a.requests = num_requests; a.min_span = min_span; a.heads = heads; a.groups = heads; a.dv = dim;
   a.q_scale = 1.0f;
+  a.per = kChunk;
   a.key_rows = 1;
   a.local = scratch;
   a.total = scratch + (size_t)chunks * heads * dim * dim;

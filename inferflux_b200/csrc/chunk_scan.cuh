@@ -113,29 +113,56 @@ __device__ __forceinline__ void load_b_columns(FragB& f, const float* p, int pit
 
 // Stretch `index` of the step's spans of min_span tokens and more: its request, first flat token and tokens.  Stretches of a
 // request lie side by side.
-__device__ __forceinline__ int chunks_of(int span, int min_span) { return span < min_span ? 0 : (span + kChunk - 1) / kChunk; }
-__device__ __forceinline__ bool chunk_of(const int* __restrict__ cu_seqlens, int requests, int min_span, int index, int& first, int& n) {
+// (`per`: tokens of a stretch)
+__device__ __forceinline__ int chunks_of(int span, int min_span, int per = kChunk) { return span < min_span ? 0 : (span + per - 1) / per; }
+__device__ __forceinline__ bool chunk_of(const int* __restrict__ cu_seqlens, int requests, int min_span, int index, int& first, int& n,
+                                         int per = kChunk) {
   int before = 0;
   for (int r = 0; r < requests; ++r) {
-    const int lo = cu_seqlens[r], span = cu_seqlens[r + 1] - lo, chunks = chunks_of(span, min_span);
+    const int lo = cu_seqlens[r], span = cu_seqlens[r + 1] - lo, chunks = chunks_of(span, min_span, per);
     if (index < before + chunks) {
-      first = lo + (index - before) * kChunk;
-      n = min(kChunk, span - (index - before) * kChunk);
+      first = lo + (index - before) * per;
+      n = min(per, span - (index - before) * per);
       return true;
     }
     before += chunks;
   }
   return false;
 }
-__device__ __forceinline__ int chunks_before(const int* __restrict__ cu_seqlens, int min_span, int request) {
+__device__ __forceinline__ int chunks_before(const int* __restrict__ cu_seqlens, int min_span, int request, int per = kChunk) {
   int before = 0;
-  for (int r = 0; r < request; ++r) before += chunks_of(cu_seqlens[r + 1] - cu_seqlens[r], min_span);
+  for (int r = 0; r < request; ++r) before += chunks_of(cu_seqlens[r + 1] - cu_seqlens[r], min_span, per);
   return before;
 }
 // The most stretches that num_tokens of num_requests can make.
-inline int chunks_at_most(int num_tokens, int num_requests, int min_span) {
+inline int chunks_at_most(int num_tokens, int num_requests, int min_span, int per = kChunk) {
   const int spans = num_tokens / (min_span > 1 ? min_span : 1);
-  return num_tokens / kChunk + (spans < num_requests ? spans : num_requests);
+  return num_tokens / per + (spans < num_requests ? spans : num_requests);
 }
+
+enum { CHUNK_CHANNEL = 0, CHUNK_STEP = 1, CHUNK_CONSTANT = 2, CHUNK_WKV = 3 };
+
+struct ChunkArgs {
+  const float* q; long long q_stride;
+  const float* k; long long k_stride;
+  const float* v; long long v_stride;
+  const float* raw; long long raw_stride;
+  float* state; long long state_slot_stride;
+  const int* req_slot; const int* cu_seqlens;
+  float* out;                                   // [T, heads dv]
+  const float* step_bias; const float* log_rate; const float* skip; const float* rate;      // per head
+  const float* w0; const float* u;              // CHUNK_WKV: per head and key channel
+  int requests, min_span, heads, groups, dv;    // shorter spans are left to the scans token by token
+  float inv_tau, q_scale;
+  float* local;                                 // [stretches, heads, dv, dk]: what a stretch adds, then the state in front of it
+  float* total;                                 // decays of a whole stretch: [stretches, heads, dk], or [stretches, heads] as two numbers each
+  float* reach;                                 // queries times decays since the stretch's beginning [T, heads dk], or decays [T, heads]
+  int key_rows;                                 // the request's state is [head, key channel, value channel]
+  int per;                                      // tokens of a stretch
+  const float* x; float* prev_state; int C;     // CHUNK_WKV: the step's input rows, where the last one of a request goes
+};
+
+__device__ __forceinline__ float chunk_log_sigmoid(float x) { return fminf(x, 0.0f) - log1pf(expf(-fabsf(x))); }
+__device__ __forceinline__ float chunk_softplus(float x) { return x > 20.0f ? x : log1pf(expf(x)); }
 
 }  // namespace ifx

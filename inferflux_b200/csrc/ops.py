@@ -170,7 +170,7 @@ class CudaKernels:
                    "ifx_attention_prefill_tcgen05_sink", "ifx_attention_prefill_bf16_sink", "ifx_attention_decode_bf16_sink",
                    "ifx_norm_of_sum", "ifx_row_norm_rope_append", "ifx_rotate_rows", "ifx_gated_scan", "ifx_decay_scan_rate",
                    "ifx_geglu_mul", "ifx_gemm_skinny_geglu", "ifx_gemm_tcgen05_geglu", "ifx_relu2", "ifx_silu_columns",
-                   "ifx_chunk_scan_supports", "ifx_chunk_decay_scan", "ifx_chunk_wkv_scan", "ifx_wkv_norm",
+                   "ifx_chunk_scan_supports", "ifx_chunk_scan_takes_128", "ifx_chunk_decay_scan", "ifx_chunk_wkv_scan", "ifx_wkv_norm",
                    "ifx_latent_decode", "ifx_latent_decode_supports", "ifx_latent_decode_stretch",
                    "ifx_latent_prompt", "ifx_latent_prompt_supports", "ifx_delta_chunks_supports", "ifx_delta_chunks_scan",
                    "ifx_attention_prefill_tcgen05_parts", "ifx_gemm_f32_split", "ifx_swiglu_few", "ifx_gemm_f32_split_launches"):
@@ -1524,6 +1524,8 @@ class CudaKernels:
                                     sum(-(-n // 64) for _s, n in ctx.spans if n >= self.CHUNK_SCAN_MIN_SPAN))
         return got
 
+    stretch = 0                # tokens of a stretch of a decay per head: 64, 128, or 0 for the kernels' own rule
+
     def _scans_by_chunks(self, dtype, ctx, heads, dk, dv, *rows, constant=False):
         """Which of a recurrence's spans go by stretches of tokens: False, none; else (the fewest tokens of one that does, the most
         tokens of one that does not or 0).  Where that pays, with sizes the kernels are made for, rows on 16-byte boundaries (those
@@ -1905,7 +1907,8 @@ class CudaKernels:
             room = torch.empty(int(self.lib.ifx_chunk_scan_scratch_floats(T, ctx.num_requests, least, heads, dk, dv, int(mode == 0))),
                                dtype=torch.float32, device=q.device)
             rc = self.lib.ifx_chunk_decay_scan(*rows, ctx.num_requests, T, least, int(heads), int(groups), int(dk), int(dv), mode,
-                                               ctypes.c_float(tau), ctypes.c_float(q_scale), _ptr(room), _ptr(rate), _stream())
+                                               ctypes.c_float(tau), ctypes.c_float(q_scale), _ptr(room), _ptr(rate),
+                                               self.stretch, _ptr(self.error_flag), _stream())
             if rc != _MISALIGNED:
                 _check(rc, "decay_scan (stretches)")
                 self.launches += 3
