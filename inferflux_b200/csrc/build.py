@@ -2,7 +2,7 @@
 
 Every .cu file of this folder is compiled to an object (`-gencode
 arch=compute_100a,code=sm_100a`) and the objects are linked into one shared
-library.  The library lives in `_build/` beside the sources when that folder can be
+library; host_call.cpp becomes the extension module that calls it.  Both live in `_build/` beside the sources when that folder can be
 written, else in a per-user folder under the system's temporary directory.  A
 stamp of the sources' contents and the flags decides whether a build is current, so
 a fresh checkout compiles once, at its first call, and prints a line per file
@@ -12,10 +12,12 @@ from __future__ import annotations
 
 import ctypes
 import hashlib
+import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import time
 from concurrent.futures import ThreadPoolExecutor
@@ -23,6 +25,7 @@ from pathlib import Path
 
 HERE = Path(__file__).resolve().parent
 LIB_NAME = "libinferflux_b200.so"
+HOST_NAME = "_ifx_host" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
               "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
 LINK_LIBS = ["-lcublas"]
@@ -50,7 +53,7 @@ def sources():
 
 def _stamp() -> str:
     h = hashlib.sha256()
-    for p in sorted(list(HERE.glob("*.cu")) + list(HERE.glob("*.cuh")) + list(HERE.glob("*.h"))):
+    for p in sorted(list(HERE.glob("*.cu")) + list(HERE.glob("*.cuh")) + list(HERE.glob("*.h")) + list(HERE.glob("*.cpp"))):
         h.update(p.name.encode())
         h.update(p.read_bytes())
     h.update(" ".join(NVCC_FLAGS + LINK_LIBS).encode())
@@ -99,12 +102,27 @@ def _compile_one(nvcc: str, src: Path, obj: Path, verbose_ptxas: bool) -> str:
     return proc.stderr
 
 
+def _compile_host(out: Path) -> None:
+    gxx = os.environ.get("CXX") or shutil.which("g++")
+    include = sysconfig.get_paths()["include"]
+    if not gxx or not (Path(include) / "Python.h").is_file():
+        raise BuildError(f"host_call.cpp needs g++ and Python.h ({include}): there is no other way to call the kernels")
+    tmp = out / (HOST_NAME + f".tmp{os.getpid()}")
+    proc = subprocess.run([gxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-I", include, str(HERE / "host_call.cpp"), "-o", str(tmp)],
+                          capture_output=True, text=True)
+    if proc.returncode != 0:
+        raise BuildError(f"g++ failed on host_call.cpp:\n{proc.stdout}\n{proc.stderr}")
+    os.replace(tmp, out / HOST_NAME)
+
+
 def build(force: bool = False, verbose_ptxas: bool = False) -> Path:
     """Compile what is stale and return the path of the shared library."""
     out = build_dir()
     lib, stamp_file = out / LIB_NAME, out / "stamp.txt"
     stamp = _stamp()
     if not force and lib.is_file() and stamp_file.is_file() and stamp_file.read_text().strip() == stamp:
+        if not (out / HOST_NAME).is_file():                  # built by another interpreter
+            _compile_host(out)
         return lib
     nvcc = find_nvcc()
     srcs = sources()
@@ -123,6 +141,7 @@ def build(force: bool = False, verbose_ptxas: bool = False) -> Path:
     if proc.returncode != 0:
         raise BuildError(f"linking {LIB_NAME} failed:\n{proc.stdout}\n{proc.stderr}")
     os.replace(tmp, lib)
+    _compile_host(out)
     stamp_file.write_text(stamp + "\n")
     if verbose_ptxas:
         (out / "ptxas.log").write_text("\n".join(logs))
@@ -145,3 +164,22 @@ def load_library() -> ctypes.CDLL:
         except OSError as e:
             raise BuildError(f"cannot load {path}: {e}") from e
     return _LIB
+
+
+class HostLibrary:
+    """The kernel library's entry points as callables that take tensors, integers, floats and None as they are.  `wide`: the names of those
+    that return long long; all others return int.  Names that are not listed are ctypes functions."""
+
+    def __init__(self, library, names, wide):
+        import torch
+        self._ctypes = library
+        spec = importlib.util.spec_from_file_location("_ifx_host", build_dir() / HOST_NAME)
+        host = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(host)
+        for name in (*names, *wide):
+            fn = getattr(self._ctypes, name)
+            fn.restype = ctypes.c_longlong if name in wide else ctypes.c_int
+            setattr(self, name, host.Function(ctypes.cast(fn, ctypes.c_void_p).value, name in wide, torch.Tensor))
+
+    def __getattr__(self, name):
+        return getattr(self._ctypes, name)

@@ -4,7 +4,7 @@ where the reference uses it too).
 
 There is no CPU path and no library model code here: making a `CudaKernels`
 without a CUDA device, or without being able to build or load the library, raises.
-Tensors are passed as raw device pointers on torch's current stream.  What a call costs the host
+Tensors are passed as raw device pointers (host_call.cpp) on torch's current stream.  What a call costs the host
 matters where a layer's kernels are short: sizes go to `torch.empty` one by one (as a tuple they
 take a microsecond more), and messages with values in them are made when something is wrong.
 """
@@ -12,11 +12,10 @@ from __future__ import annotations
 
 import ctypes
 import os
-from typing import Optional
 
 import torch
 
-from .build import BuildError, load_library
+from .build import BuildError, HostLibrary, load_library
 
 _DT = {torch.float32: 0, torch.bfloat16: 1}
 _MISALIGNED = -3             # what the kernels of long spans say of rows off a 16-byte boundary, before they touch anything
@@ -67,10 +66,6 @@ class PartialSum:
         return self.parts.shape[0]
 
 
-def _ptr(t: Optional[torch.Tensor]):
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
-
-
 # The current stream's handle of the current device, asked for at every launch: torch's own accessors
 # when they are there (plain integers, a fraction of a microsecond), else through the Stream object
 # (several microseconds).
@@ -80,8 +75,8 @@ _RAW_DEVICE = getattr(torch._C, "_cuda_getDevice", None)
 
 def _stream():
     if _RAW_STREAM is not None and _RAW_DEVICE is not None:
-        return ctypes.c_void_p(_RAW_STREAM(_RAW_DEVICE()))
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        return _RAW_STREAM(_RAW_DEVICE())
+    return torch.cuda.current_stream().cuda_stream
 
 
 def _check(rc: int, what: str) -> None:
@@ -99,7 +94,7 @@ def _need(cond: bool, msg: str) -> None:
         raise KernelError(msg)
 
 
-_I, _F, _P, _LL = ctypes.c_int, ctypes.c_float, ctypes.c_void_p, ctypes.c_longlong
+_I, _F, _P, _LL = ctypes.c_int, ctypes.c_float, ctypes.c_void_p, ctypes.c_longlong       # of the structures below
 
 
 class TurnedQueries:
@@ -146,8 +141,9 @@ class CudaKernels:
         if not torch.cuda.is_available():
             raise BuildError("no CUDA device: the engine has no CPU path")
         self.device = torch.device(device)
-        self.lib = load_library()
-        for fn in ("ifx_embed", "ifx_rmsnorm", "ifx_silu_mul", "ifx_residual_add", "ifx_gather_rows",
+        self.lib = HostLibrary(
+                  load_library(),
+                  ("ifx_embed", "ifx_rmsnorm", "ifx_silu_mul", "ifx_residual_add", "ifx_gather_rows",
                    "ifx_scatter_i32", "ifx_rope_append", "ifx_attention_generic", "ifx_gemm_generic",
                    "ifx_gemm_cublas_bf16", "ifx_cublas_init", "ifx_argmax", "ifx_penalties", "ifx_logit_bias",
                    "ifx_sample", "ifx_sample_blocks", "ifx_attention_mma_supports", "ifx_attention_prefill_bf16",
@@ -173,18 +169,13 @@ class CudaKernels:
                    "ifx_chunk_scan_supports", "ifx_chunk_scan_takes_128", "ifx_chunk_decay_scan", "ifx_chunk_wkv_scan", "ifx_wkv_norm",
                    "ifx_latent_decode", "ifx_latent_decode_supports", "ifx_latent_decode_stretch",
                    "ifx_latent_prompt", "ifx_latent_prompt_supports", "ifx_delta_chunks_supports", "ifx_delta_chunks_scan",
-                   "ifx_attention_prefill_tcgen05_parts", "ifx_gemm_f32_split", "ifx_swiglu_few", "ifx_gemm_f32_split_launches"):
-            getattr(self.lib, fn).restype = ctypes.c_int
-        self.lib.ifx_delta_rule_scratch_floats.restype = ctypes.c_longlong
-        self.lib.ifx_chunk_scan_scratch_floats.restype = ctypes.c_longlong
-        self.lib.ifx_delta_chunks_scratch_floats.restype = ctypes.c_longlong
-        self.lib.ifx_attention_prefill_tcgen05_parts_bytes.restype = ctypes.c_longlong
-        self.lib.ifx_gemm_f32_split_scratch.restype = ctypes.c_longlong
-        self.lib.ifx_moe_sorted_scratch.restype = ctypes.c_longlong
+                   "ifx_attention_prefill_tcgen05_parts", "ifx_gemm_f32_split", "ifx_swiglu_few", "ifx_gemm_f32_split_launches",
+                   "ifx_set_shared_carveout", "ifx_set_pdl"),
+                  ("ifx_delta_rule_scratch_floats", "ifx_chunk_scan_scratch_floats", "ifx_delta_chunks_scratch_floats",
+                   "ifx_attention_prefill_tcgen05_parts_bytes", "ifx_gemm_f32_split_scratch", "ifx_moe_sorted_scratch",
+                   "ifx_sample_scratch_bytes", "ifx_latent_attention_mma_workspace", "ifx_layer_workspace_bytes"))
         # long spans of a bfloat16 run's recurrences by stretches of 64 tokens (0: token after token, for comparisons)
         self.chunk_scans = os.environ.get("INFERFLUX_B200_CHUNK_SCANS", "1") != "0"
-        self.lib.ifx_sample_scratch_bytes.restype = ctypes.c_longlong
-        self.lib.ifx_latent_attention_mma_workspace.restype = ctypes.c_longlong
         self._latent_sizes = {}
         # latent attention on the tensor-core tiles (0: the per-token kernel, for comparisons)
         self.latent_tiles = os.environ.get("INFERFLUX_B200_LATENT_TILES", "1") != "0"
@@ -216,8 +207,7 @@ class CudaKernels:
         self.native_layers = os.environ.get("INFERFLUX_B200_NATIVE_LAYER", "1") != "0"
         # in a natively run layer of a mixed step, the two attention kernels side by side on two streams
         self.overlap_attention = os.environ.get("INFERFLUX_B200_ATTENTION_OVERLAP", "1") != "0"
-        self.lib.ifx_layer_forward.restype = ctypes.c_int
-        self.lib.ifx_layer_workspace_bytes.restype = ctypes.c_longlong
+        self.lib.ifx_layer_forward.restype = ctypes.c_int          # (takes structures: a ctypes function)
         self._layer_ws, self._layer_ws_all, self._layer_views = None, [], {}
         self._layer_io = _LayerIO()
         self._layer_io_ref = ctypes.byref(self._layer_io)
@@ -229,11 +219,11 @@ class CudaKernels:
         T, H = token_ids.numel(), table.shape[1]
         out = torch.empty(T, H, dtype=torch.float32, device=table.device)
         if scale != 1.0:
-            _check(self.lib.ifx_embed_scaled(_ptr(table), _ptr(token_ids), _ptr(out), T, H, int(vocab), ctypes.c_float(scale),
+            _check(self.lib.ifx_embed_scaled(table, token_ids, out, T, H, int(vocab), float(scale),
                                              _DT[table.dtype], _stream()), "embed")
             self.launches += 1
             return out
-        _check(self.lib.ifx_embed(_ptr(table), _ptr(token_ids), _ptr(out), T, H, int(vocab), _DT[table.dtype],
+        _check(self.lib.ifx_embed(table, token_ids, out, T, H, int(vocab), _DT[table.dtype],
                                   _stream()), "embed")
         self.launches += 1
         return out
@@ -245,12 +235,12 @@ class CudaKernels:
         if groups > 1:
             _need(x.is_contiguous() and H % groups == 0, "rmsnorm: the groups must cut a contiguous row evenly")
             _check(self.lib.ifx_groupnorm_stream(
-                _ptr(x), _ptr(None), _ptr(None), ctypes.c_float(0.0), _ptr(w), ctypes.c_float(eps), int(groups), _ptr(out),
-                _ptr(None), T, H, 0, _DT[out_dtype], 1, _ptr(None), 0, _ptr(None), ctypes.c_longlong(0), _ptr(None),
-                _ptr(None), _stream()), "rmsnorm (groups)")
+                x, None, None, 0.0, w, float(eps), int(groups), out,
+                None, T, H, 0, _DT[out_dtype], 1, None, 0, None, 0, None,
+                None, _stream()), "rmsnorm (groups)")
             self.launches += 1
             return out
-        _check(self.lib.ifx_rmsnorm(_ptr(x), _ptr(None), _ptr(w), _ptr(out), T, H, ctypes.c_float(eps), 0,
+        _check(self.lib.ifx_rmsnorm(x, None, w, out, T, H, float(eps), 0,
                                     _DT[out_dtype], _stream()), "rmsnorm")
         self.launches += 1
         return out
@@ -266,15 +256,15 @@ class CudaKernels:
             chunks = -(-H // 512)
             if T <= self._norm_tickets.numel() and T * chunks <= self._norm_sumsq.numel():
                 _check(self.lib.ifx_reduce_add_rmsnorm(
-                    _ptr(x), _ptr(delta.parts), _ptr(w), _ptr(out), T, H, ctypes.c_float(eps), delta.splits,
-                    _ptr(self._norm_sumsq), _ptr(self._norm_tickets), _DT[out_dtype], _stream()), "reduce_add_rmsnorm")
+                    x, delta.parts, w, out, T, H, float(eps), delta.splits,
+                    self._norm_sumsq, self._norm_tickets, _DT[out_dtype], _stream()), "reduce_add_rmsnorm")
                 self.launches += 1
                 return out
             src, splits = delta.parts, delta.splits
         else:
             _need(delta.dtype == out_dtype and delta.shape == x.shape, "add_rmsnorm: delta must match x and the dtype")
             src, splits = delta, 0
-        _check(self.lib.ifx_rmsnorm(_ptr(x), _ptr(src), _ptr(w), _ptr(out), T, H, ctypes.c_float(eps), splits,
+        _check(self.lib.ifx_rmsnorm(x, src, w, out, T, H, float(eps), splits,
                                     _DT[out_dtype], _stream()), "add_rmsnorm")
         self.launches += 1
         return out
@@ -294,7 +284,7 @@ class CudaKernels:
         else:
             _need(delta is None or (delta.dtype == out_dtype and delta.shape == x.shape), "prenorm: delta must match x")
             src, splits = delta, 0
-        _check(self.lib.ifx_prenorm(_ptr(x), _ptr(src), _ptr(w), _ptr(pre), _ptr(sumsq), T, H, splits, _DT[out_dtype],
+        _check(self.lib.ifx_prenorm(x, src, w, pre, sumsq, T, H, splits, _DT[out_dtype],
                                     _stream()), "prenorm")
         self.launches += 1
         return ScaledRows(pre, sumsq, eps)
@@ -305,7 +295,7 @@ class CudaKernels:
             return h
         T, H = h.shape
         out = torch.empty(T, H, dtype=h.dtype, device=h.pre.device)
-        _check(self.lib.ifx_scale_rows(_ptr(h.pre), _ptr(h.sumsq), _ptr(out), T, H, ctypes.c_float(h.eps),
+        _check(self.lib.ifx_scale_rows(h.pre, h.sumsq, out, T, H, float(h.eps),
                                        _DT[h.dtype], _stream()), "scale_rows")
         self.launches += 1
         return out
@@ -313,10 +303,10 @@ class CudaKernels:
     def residual_add(self, x, delta):
         T, H = x.shape
         if isinstance(delta, PartialSum):
-            _check(self.lib.ifx_residual_add_partial(_ptr(x), _ptr(delta.parts), T, H, delta.splits, _stream()),
+            _check(self.lib.ifx_residual_add_partial(x, delta.parts, T, H, delta.splits, _stream()),
                    "residual_add")
         else:
-            _check(self.lib.ifx_residual_add(_ptr(x), _ptr(delta), T, H, _DT[delta.dtype], _stream()), "residual_add")
+            _check(self.lib.ifx_residual_add(x, delta, T, H, _DT[delta.dtype], _stream()), "residual_add")
         self.launches += 1
 
     def materialize(self, value, bias=None):
@@ -325,7 +315,7 @@ class CudaKernels:
             return value if bias is None else value + bias.to(value.dtype)
         T, N = value.shape
         out = torch.empty(T, N, dtype=value.dtype, device=value.parts.device)
-        _check(self.lib.ifx_reduce_partial(_ptr(value.parts), _ptr(bias), _ptr(out), T, N, value.splits,
+        _check(self.lib.ifx_reduce_partial(value.parts, bias, out, T, N, value.splits,
                                            _DT[value.dtype], _stream()), "reduce_partial")
         self.launches += 1
         return out
@@ -333,7 +323,7 @@ class CudaKernels:
     def silu_mul(self, gate_up):
         T, two_i = gate_up.shape
         out = torch.empty(T, two_i // 2, dtype=gate_up.dtype, device=gate_up.device)
-        _check(self.lib.ifx_silu_mul(_ptr(gate_up), _ptr(out), T, two_i // 2, _DT[gate_up.dtype], _stream()),
+        _check(self.lib.ifx_silu_mul(gate_up, out, T, two_i // 2, _DT[gate_up.dtype], _stream()),
                "silu_mul")
         self.launches += 1
         return out
@@ -341,21 +331,21 @@ class CudaKernels:
     def gather_rows(self, x, rows):
         R, H = rows.numel(), x.shape[1]
         out = torch.empty(R, H, dtype=torch.float32, device=x.device)
-        _check(self.lib.ifx_gather_rows(_ptr(x), _ptr(rows), _ptr(out), R, H, x.shape[0], _stream()), "gather_rows")
+        _check(self.lib.ifx_gather_rows(x, rows, out, R, H, x.shape[0], _stream()), "gather_rows")
         self.launches += 1
         return out
 
     def scatter_i32(self, table, index, value):
         n = index.numel()
         if n:
-            _check(self.lib.ifx_scatter_i32(_ptr(table), _ptr(index), _ptr(value), n, table.numel(), _stream()),
+            _check(self.lib.ifx_scatter_i32(table, index, value, n, table.numel(), _stream()),
                    "scatter_i32")
             self.launches += 1
 
     def relay_i32(self, dst, dst_index, src, src_index):
         n = dst_index.numel()
         if n:
-            _check(self.lib.ifx_relay_i32(_ptr(dst), _ptr(dst_index), _ptr(src), _ptr(src_index), n, dst.numel(),
+            _check(self.lib.ifx_relay_i32(dst, dst_index, src, src_index, n, dst.numel(),
                                           src.numel(), _stream()), "relay_i32")
             self.launches += 1
 
@@ -390,11 +380,11 @@ class CudaKernels:
             if self.float32_by_parts(N, K) and (a.data_ptr() | w.data_ptr()) % 16 == 0:
                 room = self.lib.ifx_gemm_f32_split_scratch(T, N, K)
                 scratch = torch.empty(room, dtype=torch.uint8, device=a.device)
-                _check(self.lib.ifx_gemm_f32_split(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), T, N, K, _ptr(scratch), _LL(room),
-                                                   _ptr(self.error_flag), _stream()), "gemm (float32 by parts)")
+                _check(self.lib.ifx_gemm_f32_split(a, w, bias, out, T, N, K, scratch, room,
+                                                   self.error_flag, _stream()), "gemm (float32 by parts)")
                 self.launches += self.lib.ifx_gemm_f32_split_launches(T, N, K)
                 return out
-            _check(self.lib.ifx_gemm_generic(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), T, N, K, 0, 0, _stream()),
+            _check(self.lib.ifx_gemm_generic(a, w, bias, out, T, N, K, 0, 0, _stream()),
                    "gemm (float32)")
             self.launches += 1
             return out
@@ -407,7 +397,7 @@ class CudaKernels:
             if tiles >= 74 or allow_partial or rows is not None:
                 return self.linear_skinny(a, w, bias, out_dtype=out_dtype, splits=1, mode=0, rows=rows)
         out = torch.empty(T, N, dtype=out_dtype, device=a.device)
-        _check(self.lib.ifx_gemm_cublas_bf16(_ptr(a), _ptr(w), _ptr(out), T, N, K, _DT[out_dtype], _stream()),
+        _check(self.lib.ifx_gemm_cublas_bf16(a, w, out, T, N, K, _DT[out_dtype], _stream()),
                "gemm (bfloat16)")
         self.library_calls += 1
         if bias is not None:
@@ -438,9 +428,9 @@ class CudaKernels:
         hidden = torch.empty(T, inter, dtype=torch.bfloat16, device=a.device)
         out = (torch.empty(splits, T, N, dtype=torch.float32, device=a.device) if splits > 1
                else torch.empty(T, N, dtype=torch.bfloat16, device=a.device))
-        _check(self.lib.ifx_swiglu_few(_ptr(a), _ptr(w_gate_up), _ptr(w_down), _ptr(hidden), _ptr(out), _ptr(out), T, K, inter, N, splits,
-                                       _ptr(None if rows is None else rows.sumsq), 0 if rows is None else rows.sumsq.shape[1],
-                                       ctypes.c_float(0.0 if rows is None else rows.eps), _ptr(self.error_flag), _stream()),
+        _check(self.lib.ifx_swiglu_few(a, w_gate_up, w_down, hidden, out, out, T, K, inter, N, splits,
+                                       (None if rows is None else rows.sumsq), 0 if rows is None else rows.sumsq.shape[1],
+                                       float(0.0 if rows is None else rows.eps), self.error_flag, _stream()),
                "swiglu (few rows)")
         self.launches += 2
         return PartialSum(out, torch.bfloat16) if splits > 1 else out
@@ -494,13 +484,13 @@ class CudaKernels:
             if few or (self.swiglu_tiles and K <= self.SWIGLU_TILES_MAX_K):
                 out = torch.empty(T, inter, dtype=torch.bfloat16, device=a.device)
                 product = self.lib.ifx_gemm_skinny_geglu if few else self.lib.ifx_gemm_tcgen05_geglu
-                _check(product(_ptr(a), _ptr(w_gate_up), _ptr(bias), _ptr(out), T, inter, K, _ptr(self.error_flag), _stream()),
+                _check(product(a, w_gate_up, bias, out, T, inter, K, self.error_flag, _stream()),
                        "linear_geglu")
                 self.launches += 1
                 return out
         both = self.linear(a, w_gate_up)
         out = torch.empty(T, inter, dtype=a.dtype, device=a.device)
-        _check(self.lib.ifx_geglu_mul(_ptr(both), _ptr(bias), _ptr(out), T, inter, _DT[a.dtype], _stream()), "geglu_mul")
+        _check(self.lib.ifx_geglu_mul(both, bias, out, T, inter, _DT[a.dtype], _stream()), "geglu_mul")
         self.launches += 1
         return out
 
@@ -514,9 +504,9 @@ class CudaKernels:
                 and a.is_contiguous() and w.is_contiguous() and w.shape[1] == K and a.data_ptr() % 16 == 0
                 and w.data_ptr() % 16 == 0 and -(-N // 128) >= 74):
             out = torch.empty(T, N, dtype=torch.bfloat16, device=a.device)
-            _check(self.lib.ifx_gemm_skinny_act(_ptr(a), _ptr(w), _ptr(None), _ptr(out), T, N, K, w.shape[0], 0, _ptr(None), 0,
-                                                ctypes.c_float(0.0), 1, ctypes.c_float(a_pos), ctypes.c_float(a_neg),
-                                                _ptr(self.error_flag), _stream()), "gemm_skinny (xielu)")
+            _check(self.lib.ifx_gemm_skinny_act(a, w, None, out, T, N, K, w.shape[0], 0, None, 0,
+                                                0.0, 1, float(a_pos), float(a_neg),
+                                                self.error_flag, _stream()), "gemm_skinny (xielu)")
             self.launches += 1
             return out
         return self.xielu(self.linear(a, w, allow_partial=True), a_pos, a_neg)
@@ -531,12 +521,12 @@ class CudaKernels:
             out = None
             if T <= self.SKINNY_MAX_ROWS and -(-N // 128) >= 74:
                 out = torch.empty(T, N, dtype=torch.bfloat16, device=a.device)
-                _check(self.lib.ifx_gemm_skinny_act(_ptr(a), _ptr(w), _ptr(None), _ptr(out), T, N, K, N, 0, _ptr(None), 0,
-                                                    ctypes.c_float(0.0), 3, ctypes.c_float(0.0), ctypes.c_float(0.0),
-                                                    _ptr(self.error_flag), _stream()), "gemm_skinny (relu2)")
+                _check(self.lib.ifx_gemm_skinny_act(a, w, None, out, T, N, K, N, 0, None, 0,
+                                                    0.0, 3, 0.0, 0.0,
+                                                    self.error_flag, _stream()), "gemm_skinny (relu2)")
             elif T > self.SKINNY_MAX_ROWS and self.swiglu_tiles and K <= self.SWIGLU_TILES_MAX_K:
                 out = torch.empty(T, N, dtype=torch.bfloat16, device=a.device)
-                _check(self.lib.ifx_gemm_tcgen05(_ptr(a), _ptr(w), _ptr(out), T, N, K, N, 6, 0, _ptr(self.error_flag), _stream()),
+                _check(self.lib.ifx_gemm_tcgen05(a, w, out, T, N, K, N, 6, 0, self.error_flag, _stream()),
                        "gemm_tcgen05 (relu2)")
             if out is not None:
                 self.launches += 1
@@ -550,7 +540,7 @@ class CudaKernels:
             out_dtype, splits, z = z.dtype, z.splits, z.parts
         _need(z.is_contiguous(), "relu2: contiguous input")
         out = torch.empty(tuple(z.shape[-2:]), dtype=out_dtype, device=z.device)
-        _check(self.lib.ifx_relu2(_ptr(z), _ptr(out), ctypes.c_longlong(out.numel()), _DT[z.dtype], _DT[out_dtype], splits,
+        _check(self.lib.ifx_relu2(z, out, (out.numel()), _DT[z.dtype], _DT[out_dtype], splits,
                                   _stream()), "relu2")
         self.launches += 1
         return out
@@ -576,12 +566,12 @@ class CudaKernels:
             partials = torch.empty(splits, T, N, dtype=torch.float32, device=a.device)
         else:
             out = torch.empty(T, N, dtype=out_dtype, device=a.device)
-        _check(self.lib.ifx_gemm_skinny(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), _ptr(partials), T, N, K, w.shape[0],
+        _check(self.lib.ifx_gemm_skinny(a, w, bias, out, partials, T, N, K, w.shape[0],
                                         splits, mode, up_row_offset, int(out_dtype == torch.float32),
-                                        _ptr(None if rows is None else rows.sumsq),
+                                        (None if rows is None else rows.sumsq),
                                         0 if rows is None else rows.sumsq.shape[1],
-                                        ctypes.c_float(0.0 if rows is None else rows.eps),
-                                        _ptr(self.error_flag), _stream()), "gemm_skinny")
+                                        float(0.0 if rows is None else rows.eps),
+                                        self.error_flag, _stream()), "gemm_skinny")
         self.launches += 1
         return partials if mode == 1 else out
 
@@ -593,8 +583,8 @@ class CudaKernels:
         _need(a.is_contiguous() and w.is_contiguous() and w.shape[1] == K and K % 8 == 0, "linear_tiles: bad operands")
         N = w.shape[0] // 2 if swiglu else w.shape[0]
         out = torch.empty(T, N, dtype=torch.bfloat16, device=a.device)
-        _check(self.lib.ifx_gemm_tcgen05(_ptr(a), _ptr(w), _ptr(out), T, N, K, w.shape[0], int(bool(swiglu)),
-                                         N if swiglu else 0, _ptr(self.error_flag), _stream()), "gemm_tcgen05")
+        _check(self.lib.ifx_gemm_tcgen05(a, w, out, T, N, K, w.shape[0], int(bool(swiglu)),
+                                         N if swiglu else 0, self.error_flag, _stream()), "gemm_tcgen05")
         self.launches += 1
         return out
 
@@ -604,7 +594,7 @@ class CudaKernels:
         N = w.shape[0]
         out_dtype = out_dtype or a.dtype
         out = torch.empty(T, N, dtype=out_dtype, device=a.device)
-        _check(self.lib.ifx_gemm_generic(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), T, N, K, _DT[a.dtype],
+        _check(self.lib.ifx_gemm_generic(a, w, bias, out, T, N, K, _DT[a.dtype],
                                          _DT[out_dtype], _stream()), "gemm_generic")
         self.launches += 1
         return out
@@ -736,7 +726,7 @@ class CudaKernels:
         io.least_decode_splits = self.least_decode_splits(ctx, ctx.extra_len.get("attn.decode_rows", 0), m.nkv, m.d, int(m.window or 0))
         io.prefill_parts = self.prefill_parts(ctx, m.nq, int(m.window or 0))
         io.ws, io.ws_bytes = ws.data_ptr(), ws.numel()
-        rc = self.lib.ifx_layer_forward(step, layer, self._layer_io_ref, _stream())
+        rc = self.lib.ifx_layer_forward(step, layer, self._layer_io_ref, ctypes.c_void_p(_stream()))
         self.launches += io.launches
         self.library_calls += io.library_calls
         self.native_layer_calls += 1
@@ -818,11 +808,11 @@ class CudaKernels:
         rot = 0 if rotary is None else int(rotary.rotary_dim)
         _need(rot <= d, "rope_append: rotary_dim exceeds the head size")
         _check(self.lib.ifx_rope_append(
-            _ptr(qkv), _ptr(partial), splits, _ptr(bias), _ptr(None if rotary is None else rotary.inv_freq), rot,
+            qkv, partial, splits, bias, (None if rotary is None else rotary.inv_freq), rot,
             int(bool(rotary.interleaved)) if rotary is not None else 0,
-            _ptr(ctx.positions), _ptr(ctx.token_req), _ptr(ctx.req_slot), _ptr(table),
+            ctx.positions, ctx.token_req, ctx.req_slot, table,
             0 if table is None else table.shape[1], cache.page_size, 0 if kv is None else kv.shape[0],
-            _ptr(kv), _ptr(q_out), T, nq, nkv, d, int(write), self.small_attention_grid(ctx, nkv), _DT[dtype],
+            kv, q_out, T, nq, nkv, d, int(write), self.small_attention_grid(ctx, nkv), _DT[dtype],
             _stream()), "rope_append")
         self.launches += 1
         return q_out
@@ -853,13 +843,13 @@ class CudaKernels:
         rot = 0 if rotary is None else int(rotary.rotary_dim)
         _need(rot <= d, "rope_append: rotary_dim exceeds the head size")
         _check(self.lib.ifx_norm_rope_append_ex(
-            _ptr(qkv), _ptr(partial), splits, _ptr(q_norm), _ptr(k_norm), ctypes.c_float(norm_eps),
-            _ptr(None if rotary is None else rotary.inv_freq), rot,
-            int(bool(rotary.interleaved)) if rotary is not None else 0, _ptr(ctx.positions), _ptr(ctx.token_req),
-            _ptr(ctx.req_slot), _ptr(table), 0 if table is None else table.shape[1], cache.page_size,
-            0 if kv is None else kv.shape[0], _ptr(kv if write else None), _ptr(q_out), T, nq, src_kv, nkv, d, dv, d_row,
-            int(write), ctypes.c_float(1.0 if rotary is None else rotary.magnitude),
-            ctypes.c_float(0.0 if q_temp is None else q_temp[0]), 0 if q_temp is None else int(q_temp[1]),
+            qkv, partial, splits, q_norm, k_norm, float(norm_eps),
+            (None if rotary is None else rotary.inv_freq), rot,
+            int(bool(rotary.interleaved)) if rotary is not None else 0, ctx.positions, ctx.token_req,
+            ctx.req_slot, table, 0 if table is None else table.shape[1], cache.page_size,
+            0 if kv is None else kv.shape[0], (kv if write else None), q_out, T, nq, src_kv, nkv, d, dv, d_row,
+            int(write), float(1.0 if rotary is None else rotary.magnitude),
+            float(0.0 if q_temp is None else q_temp[0]), 0 if q_temp is None else int(q_temp[1]),
             _DT[dtype], _stream()), "rope_append (normed heads)")
         self.launches += 1
         return q_out
@@ -890,7 +880,7 @@ class CudaKernels:
         _need(q.is_contiguous() and q.shape[1] == nq * d, "attention: queries must be one [tokens, heads * size] block")
         out = torch.empty(T, nq * d, dtype=q.dtype, device=q.device)
         win = 0 if window is None else int(window)
-        common = (cache.page_size, table.shape[1], kv.shape[0], win, ctypes.c_float(scale))
+        common = (cache.page_size, table.shape[1], kv.shape[0], win, float(scale))
         tiled = q.dtype == torch.bfloat16 and bool(self.lib.ifx_attention_mma_supports(d))
         if "attn.prefill_tiles" not in ctx.extra:          # a step context built without the mixer as a provider
             for name, vals in self.attention_sections(ctx).items():
@@ -909,14 +899,14 @@ class CudaKernels:
                 room = torch.empty(self.prefill_parts_bytes(num_tiles, nq, d, parts), dtype=torch.uint8, device=q.device)
                 self.launches += 1
             _check(self.lib.ifx_attention_prefill_tcgen05_parts(
-                _ptr(q), T, _ptr(kv), _ptr(table), _ptr(tiles), _ptr(ctx.req_slot), _ptr(out),
-                num_tiles, nq, nkv, d, *common, parts, _ptr(room), _ptr(self.error_flag), _stream()),
+                q, T, kv, table, tiles, ctx.req_slot, out,
+                num_tiles, nq, nkv, d, *common, parts, room, self.error_flag, _stream()),
                 "attention (prompt portions, tcgen05)")
             self.launches += 1
         elif num_tiles:
             _check(self.lib.ifx_attention_prefill_bf16(
-                _ptr(q), _ptr(kv), _ptr(table), _ptr(tiles), _ptr(ctx.req_slot), _ptr(out),
-                num_tiles, nq, nkv, d, *common, int(ctx.max_kv_len), _ptr(self.error_flag), _stream()),
+                q, kv, table, tiles, ctx.req_slot, out,
+                num_tiles, nq, nkv, d, *common, int(ctx.max_kv_len), self.error_flag, _stream()),
                 "attention (prompt portions)")
             self.launches += 1
         n = ctx.extra_len["attn.decode_rows"]
@@ -928,8 +918,8 @@ class CudaKernels:
             most = int(self.lib.ifx_attention_decode_max_splits(d, cache.page_size))
             splits = max(self.decode_splits(n, nkv, max_keys, most), min(most, self.least_decode_splits(ctx, n, nkv, d, win)))
             _check(self.lib.ifx_attention_decode_bf16(
-                _ptr(q), _ptr(kv), _ptr(table), _ptr(decode_meta), _ptr(out), n, nq, nkv, d, *common, splits,
-                max_keys, _ptr(self.error_flag), _stream()), "attention (decoded tokens)")
+                q, kv, table, decode_meta, out, n, nq, nkv, d, *common, splits,
+                max_keys, self.error_flag, _stream()), "attention (decoded tokens)")
             self.launches += 1
         return out
 
@@ -1036,18 +1026,18 @@ class CudaKernels:
                     ctx.extra_len[name] = len(vals)
             num_tiles = ctx.extra_len["attn.prefill_tiles"] // 4
             common = (cache.page_size, table.shape[1], kv.shape[0], win, int(chunk or 0),
-                      int(sink_values is not None or bool(sink)), _ptr(sink_values), ctypes.c_float(scale), _ptr(back), neighbours,
-                      keep_first, _ptr(head_gate))
+                      int(sink_values is not None or bool(sink)), sink_values, float(scale), back, neighbours,
+                      keep_first, head_gate)
             if num_tiles and self.tensor_core_prefill and self.lib.ifx_attention_prefill_tcgen05_supports(d, cache.page_size):
                 _check(self.lib.ifx_attention_prefill_tcgen05_sink(
-                    _ptr(q), T, _ptr(kv), _ptr(table), _ptr(ctx.extra["attn.prefill_tiles"]), _ptr(ctx.req_slot), _ptr(out),
-                    num_tiles, nq, nkv, d, *common, _ptr(self.error_flag), _stream()),
+                    q, T, kv, table, ctx.extra["attn.prefill_tiles"], ctx.req_slot, out,
+                    num_tiles, nq, nkv, d, *common, self.error_flag, _stream()),
                     "attention (masked, prompt portions, tcgen05)")
                 self.launches += 1
             elif num_tiles:
                 _check(self.lib.ifx_attention_prefill_bf16_sink(
-                    _ptr(q), _ptr(kv), _ptr(table), _ptr(ctx.extra["attn.prefill_tiles"]), _ptr(ctx.req_slot), _ptr(out),
-                    num_tiles, nq, nkv, d, *common, int(ctx.max_kv_len), _ptr(self.error_flag), _stream()),
+                    q, kv, table, ctx.extra["attn.prefill_tiles"], ctx.req_slot, out,
+                    num_tiles, nq, nkv, d, *common, int(ctx.max_kv_len), self.error_flag, _stream()),
                     "attention (masked, prompt portions)")
                 self.launches += 1
             n = ctx.extra_len["attn.decode_rows"]
@@ -1061,23 +1051,23 @@ class CudaKernels:
                     max_keys = min(int(ctx.max_kv_len), max_keys + -(-keep_first // 16) * 16)
                 splits = self.decode_splits(n, nkv, max_keys, int(self.lib.ifx_attention_decode_max_splits(d, cache.page_size)))
                 _check(self.lib.ifx_attention_decode_bf16_sink(
-                    _ptr(q), _ptr(kv), _ptr(table), _ptr(ctx.extra["attn.decode_meta"]), _ptr(out), n, nq, nkv, d, *common,
-                    splits, max_keys, _ptr(self.error_flag), _stream()), "attention (masked, decoded tokens)")
+                    q, kv, table, ctx.extra["attn.decode_meta"], out, n, nq, nkv, d, *common,
+                    splits, max_keys, self.error_flag, _stream()), "attention (masked, decoded tokens)")
                 self.launches += 1
             return out
         _check(self.lib.ifx_attention_generic_sink(
-            _ptr(q), _ptr(kv), _ptr(table), _ptr(ctx.positions), _ptr(ctx.token_req), _ptr(ctx.req_slot), _ptr(None),
-            _ptr(out), T, nq, nkv, d, dv, d_row, cache.page_size, table.shape[1], kv.shape[0],
+            q, kv, table, ctx.positions, ctx.token_req, ctx.req_slot, None,
+            out, T, nq, nkv, d, dv, d_row, cache.page_size, table.shape[1], kv.shape[0],
             0 if window is None else int(window), int(chunk or 0), int(sink_values is not None or bool(sink)),
-            _ptr(sink_values), ctypes.c_float(scale), _ptr(back), neighbours, keep_first, _ptr(head_gate),
+            sink_values, float(scale), back, neighbours, keep_first, head_gate,
             _DT[q.dtype], _stream()), "attention (masked)")
         self.launches += 1
         return out
 
     def _attention_generic(self, q, kv, table, ctx, rows, count, out, nq, nkv, d, common):
         _check(self.lib.ifx_attention_generic(
-            _ptr(q), _ptr(kv), _ptr(table), _ptr(ctx.positions), _ptr(ctx.token_req), _ptr(ctx.req_slot),
-            _ptr(rows), _ptr(out), count, nq, nkv, d, *common, _DT[q.dtype], _stream()), "attention")
+            q, kv, table, ctx.positions, ctx.token_req, ctx.req_slot,
+            rows, out, count, nq, nkv, d, *common, _DT[q.dtype], _stream()), "attention")
         self.launches += 1
 
     # ------------------------------------------- layers that norm a sublayer's output
@@ -1104,7 +1094,7 @@ class CudaKernels:
               "postnorm_add: norm weights must be float32")
         T, H = x.shape
         out = None if (w_next is None and not cast_out) else torch.empty(T, H, dtype=out_dtype or y.dtype, device=x.device)
-        cw, taps, st_ptr, stride, treq, rslot = None, 0, ctypes.c_void_p(0), 0, None, None
+        cw, taps, st_ptr, stride, treq, rslot = None, 0, 0, 0, None, None
         if conv is not None:
             cw, taps, state, index, ctx = conv
             _need(w_next is not None and ctx.max_span == 1 and tuple(cw.shape) == (H, taps) and cw.dtype == torch.float32,
@@ -1114,12 +1104,12 @@ class CudaKernels:
                       and tuple(state.shape[2:]) == (taps - 1, H) and 0 <= index < state.shape[1],
                       "postnorm_add: the state does not fit the convolution")
                 stride = state.shape[1] * (taps - 1) * H
-                st_ptr = ctypes.c_void_p(state.data_ptr() + 4 * index * (taps - 1) * H)
+                st_ptr = state.data_ptr() + 4 * index * (taps - 1) * H
             treq, rslot = ctx.token_req, ctx.req_slot
         _check(self.lib.ifx_postnorm_add_rmsnorm(
-            _ptr(x), _ptr(y), _ptr(w_post), ctypes.c_float(eps_post), _ptr(w_next), ctypes.c_float(eps_next), _ptr(out),
-            T, H, _DT[y.dtype], _DT[(out_dtype or y.dtype)], splits, _ptr(cw), taps, st_ptr, ctypes.c_longlong(stride),
-            _ptr(treq), _ptr(rslot), _stream()), "postnorm_add")
+            x, y, w_post, float(eps_post), w_next, float(eps_next), out,
+            T, H, _DT[y.dtype], _DT[(out_dtype or y.dtype)], splits, cw, taps, st_ptr, stride,
+            treq, rslot, _stream()), "postnorm_add")
         self.launches += 1
         return out
 
@@ -1136,7 +1126,7 @@ class CudaKernels:
         T, H = x.shape
         out_dtype = out_dtype or y.dtype
         out = torch.empty(T, H, dtype=out_dtype, device=x.device)
-        out2, cw, taps, st_ptr, stride, treq, rslot = None, None, 0, ctypes.c_void_p(0), 0, None, None
+        out2, cw, taps, st_ptr, stride, treq, rslot = None, None, 0, 0, 0, None, None
         if conv is not None:
             cw, taps, state, index, ctx = conv
             _need(ctx.max_span == 1 and tuple(cw.shape) == (H, taps) and cw.dtype == torch.float32,
@@ -1146,13 +1136,13 @@ class CudaKernels:
                       and state.stride(3) == 1 and state.stride(2) == H and 0 <= index < state.shape[1],
                       "postnorm_add: the state does not fit the convolution")
                 stride = state.stride(0)
-                st_ptr = ctypes.c_void_p(state.data_ptr() + 4 * index * state.stride(1))
+                st_ptr = state.data_ptr() + 4 * index * state.stride(1)
             treq, rslot = ctx.token_req, ctx.req_slot
             out2 = torch.empty(T, H, dtype=out_dtype, device=x.device)
         _check(self.lib.ifx_groupnorm_stream(
-            _ptr(x), _ptr(y), _ptr(w_post), ctypes.c_float(eps_post), _ptr(w_next), ctypes.c_float(eps_next), int(groups),
-            _ptr(out), _ptr(out2), T, H, _DT[y.dtype], _DT[out_dtype], splits, _ptr(cw), taps, st_ptr,
-            ctypes.c_longlong(stride), _ptr(treq), _ptr(rslot), _stream()), "postnorm_add (groups)")
+            x, y, w_post, float(eps_post), w_next, float(eps_next), int(groups),
+            out, out2, T, H, _DT[y.dtype], _DT[out_dtype], splits, cw, taps, st_ptr,
+            stride, treq, rslot, _stream()), "postnorm_add (groups)")
         self.launches += 1
         if conv is None:
             return out
@@ -1175,7 +1165,7 @@ class CudaKernels:
         pa, da, sa = operand(a)
         pb, db, sb = operand(b)
         out = None if out_dtype is None else torch.empty(T, H, dtype=out_dtype, device=x.device)
-        _check(self.lib.ifx_residual_add_scaled(_ptr(x), _ptr(pa), da, sa, _ptr(pb), db, sb, ctypes.c_float(scale), _ptr(out),
+        _check(self.lib.ifx_residual_add_scaled(x, pa, da, sa, pb, db, sb, float(scale), out,
                                                 0 if out is None else _DT[out_dtype], T, H, _stream()), "residual_add_scaled")
         self.launches += 1
         return out
@@ -1183,7 +1173,7 @@ class CudaKernels:
     def scale_(self, values, factor):
         """values *= factor, in place (float32)."""
         _need(values.dtype == torch.float32 and values.is_contiguous(), "scale_: contiguous float32 values")
-        _check(self.lib.ifx_scale_f32(_ptr(values), ctypes.c_longlong(values.numel()), ctypes.c_float(factor), _stream()), "scale_")
+        _check(self.lib.ifx_scale_f32(values, (values.numel()), float(factor), _stream()), "scale_")
         self.launches += 1
 
     def gelu_mul_table(self, z, table, token_ids, first_column):
@@ -1192,8 +1182,8 @@ class CudaKernels:
         _need(z.is_contiguous() and table.is_contiguous() and table.dtype == z.dtype and token_ids.numel() == T
               and first_column + dim <= table.shape[1], "gelu_mul_table: rows and table of one dtype, columns inside the table")
         out = torch.empty_like(z)
-        _check(self.lib.ifx_gelu_mul_table(_ptr(z), _ptr(table), _ptr(token_ids), table.shape[1], int(first_column),
-                                           table.shape[0], _ptr(out), T, dim, _DT[z.dtype], _stream()), "gelu_mul_table")
+        _check(self.lib.ifx_gelu_mul_table(z, table, token_ids, table.shape[1], int(first_column),
+                                           table.shape[0], out, T, dim, _DT[z.dtype], _stream()), "gelu_mul_table")
         self.launches += 1
         return out
 
@@ -1204,8 +1194,8 @@ class CudaKernels:
               "rmsnorm_columns: the columns must lie inside contiguous rows")
         out = torch.empty(T, n, dtype=rows.dtype, device=rows.device)
         _check(self.lib.ifx_latent_norm_append(
-            _ptr(rows), ld, int(col0), _ptr(w), ctypes.c_float(eps), _ptr(None), _ptr(None), _ptr(None), _ptr(None), 0, 0, 0,
-            _ptr(None), _ptr(out), T, n, _DT[rows.dtype], _stream()), "rmsnorm_columns")
+            rows, ld, int(col0), w, float(eps), None, None, None, None, 0, 0, 0,
+            None, out, T, n, _DT[rows.dtype], _stream()), "rmsnorm_columns")
         self.launches += 1
         return out
 
@@ -1215,7 +1205,7 @@ class CudaKernels:
               and b.is_contiguous(), "concat_cast: two float32 tensors of one shape")
         T, H = a.shape
         out = torch.empty(T, 2 * H, dtype=dtype, device=a.device)
-        _check(self.lib.ifx_concat_cast(_ptr(a), _ptr(b), _ptr(out), T, H, _DT[dtype], _stream()), "concat_cast")
+        _check(self.lib.ifx_concat_cast(a, b, out, T, H, _DT[dtype], _stream()), "concat_cast")
         self.launches += 1
         return out
 
@@ -1226,15 +1216,15 @@ class CudaKernels:
             out_dtype, splits, z = z.dtype, z.splits, z.parts
         _need(z.is_contiguous(), "xielu: contiguous input")
         out = torch.empty(tuple(z.shape[-2:]), dtype=out_dtype, device=z.device)
-        _check(self.lib.ifx_xielu(_ptr(z), _ptr(out), ctypes.c_longlong(out.numel()), ctypes.c_float(a_pos),
-                                  ctypes.c_float(a_neg), _DT[z.dtype], _DT[out_dtype], splits, _stream()), "xielu")
+        _check(self.lib.ifx_xielu(z, out, (out.numel()), float(a_pos),
+                                  float(a_neg), _DT[z.dtype], _DT[out_dtype], splits, _stream()), "xielu")
         self.launches += 1
         return out
 
     def softcap(self, logits, cap):
         """logits <- cap tanh(logits / cap), in place (float32)."""
         _need(logits.dtype == torch.float32 and logits.is_contiguous(), "softcap: float32 logits")
-        _check(self.lib.ifx_softcap(_ptr(logits), ctypes.c_longlong(logits.numel()), ctypes.c_float(cap), _stream()),
+        _check(self.lib.ifx_softcap(logits, (logits.numel()), float(cap), _stream()),
                "softcap")
         self.launches += 1
 
@@ -1248,18 +1238,18 @@ class CudaKernels:
         _need(h.is_contiguous() and w.dtype == torch.float32 and tuple(w.shape) == (C, taps) and w.is_contiguous()
               and 0 <= col0 and col0 + C <= width and act in (None, "silu")
               and (bias is None or (bias.dtype == torch.float32 and bias.numel() == C)), "short_conv: bad operands")
-        st_ptr, stride = ctypes.c_void_p(0), 0
+        st_ptr, stride = 0, 0
         if taps > 1:
             _need(state is not None and state.dtype == torch.float32 and tuple(state.shape[2:]) == (taps - 1, C)
                   and state.stride(3) == 1 and state.stride(2) == C and 0 <= index < state.shape[1],
                   "short_conv: the state does not fit the convolution")
             stride = state.stride(0)                       # a slot's rows may be part of a longer state row
-            st_ptr = ctypes.c_void_p(state.data_ptr() + 4 * index * state.stride(1))
+            st_ptr = state.data_ptr() + 4 * index * state.stride(1)
         out = torch.empty(T, C, dtype=h.dtype, device=h.device)
-        _check(self.lib.ifx_short_conv_ex(ctypes.c_void_p(h.data_ptr() + col0 * h.element_size()), ctypes.c_longlong(width),
-                                          _ptr(w), _ptr(bias), st_ptr, ctypes.c_longlong(stride), _ptr(ctx.token_req),
-                                          _ptr(ctx.req_slot), _ptr(ctx.cu_seqlens), _ptr(out), T, ctx.num_requests, C,
-                                          taps, int(ctx.max_span > 1), ctypes.c_float(1.0 if add_input else 0.0),
+        _check(self.lib.ifx_short_conv_ex(h.data_ptr() + col0 * h.element_size(), width,
+                                          w, bias, st_ptr, stride, ctx.token_req,
+                                          ctx.req_slot, ctx.cu_seqlens, out, T, ctx.num_requests, C,
+                                          taps, int(ctx.max_span > 1), float(1.0 if add_input else 0.0),
                                           int(act == "silu"), _DT[h.dtype], _stream()), "short_conv")
         self.launches += 1 + int(taps > 1 and ctx.max_span > 1)
         return out
@@ -1297,7 +1287,7 @@ class CudaKernels:
               and out.shape[1] >= (heads - 1) * so + n, "linear_heads: the output does not fit")
         ldw = k if w_is_nk else n
         _check(self.lib.ifx_gemm_cublas_bf16_batched(
-            _ptr(a), _LL(lda), _LL(sa), _ptr(w), _LL(ldw), _LL(k * n), _ptr(out), _LL(out.shape[1]), _LL(so), T, n, k, heads,
+            a, lda, sa, w, ldw, (k * n), out, out.shape[1], so, T, n, k, heads,
             int(bool(w_is_nk)), _stream()), "linear_heads")
         self.library_calls += 1
         return out
@@ -1311,9 +1301,9 @@ class CudaKernels:
         _need(kv.shape[1] == 1 and kv.shape[2] == 1 and kv.shape[4] == rank, "latent_norm_append: the cache is not one latent plane")
         write = bool(cache.writes)
         _check(self.lib.ifx_latent_norm_append(
-            _ptr(rows), ld, col0, _ptr(w), ctypes.c_float(eps), _ptr(ctx.positions), _ptr(ctx.token_req),
-            _ptr(ctx.req_slot), _ptr(table), table.shape[1], cache.page_size, kv.shape[0], _ptr(kv if write else None),
-            _ptr(None), T, rank, _DT[rows.dtype], _stream()), "latent_norm_append")
+            rows, ld, col0, w, float(eps), ctx.positions, ctx.token_req,
+            ctx.req_slot, table, table.shape[1], cache.page_size, kv.shape[0], (kv if write else None),
+            None, T, rank, _DT[rows.dtype], _stream()), "latent_norm_append")
         self.launches += 1
 
     def latent_rope_append(self, rows, col0, rank, rot, w, eps, q, heads, dim, rotary, ctx, cache, vdim=None, gate_col=None):
@@ -1344,10 +1334,10 @@ class CudaKernels:
             dst = torch.empty(T, heads * (rank + rot), dtype=torch.bfloat16, device=rows.device)
             ld_dst, head_stride, offset, result = heads * (rank + rot), rank + rot, rank, TurnedQueries(q, dst)
         _check(self.lib.ifx_latent_rope_append(
-            _ptr(rows), ld, int(col0), _ptr(w), ctypes.c_float(eps), _ptr(q), q.shape[1], _ptr(dst), ld_dst, head_stride, offset,
-            _ptr(freq), used, inter, ctypes.c_float(mag), _ptr(ctx.positions), _ptr(ctx.token_req), _ptr(ctx.req_slot),
-            _ptr(table), table.shape[1], cache.page_size, kv.shape[0], _ptr(kv if write else None), T, rank, rot, heads, dim,
-            _ptr(gate), int(gate_col or 0), _DT[rows.dtype], _stream()), "latent_rope_append")
+            rows, ld, int(col0), w, float(eps), q, q.shape[1], dst, ld_dst, head_stride, offset,
+            freq, used, inter, float(mag), ctx.positions, ctx.token_req, ctx.req_slot,
+            table, table.shape[1], cache.page_size, kv.shape[0], (kv if write else None), T, rank, rot, heads, dim,
+            gate, int(gate_col or 0), _DT[rows.dtype], _stream()), "latent_rope_append")
         self.launches += 1
         return result if gate_col is None else (result, gate)
 
@@ -1377,10 +1367,10 @@ class CudaKernels:
         if rot or (head_gate is not None and not tiled):
             out = torch.empty(T, heads * vdim, dtype=q_rows.dtype, device=q_rows.device)
             _check(self.lib.ifx_latent_attention_generic_rot(
-                _ptr(q_rows), ldq, _ptr(w_uk), _ptr(w_uv), _ptr(sinks), _ptr(kv), _ptr(table), _ptr(ctx.positions),
-                _ptr(ctx.token_req), _ptr(ctx.req_slot), _ptr(None), _ptr(out), T, heads, dim, vdim, rank, cache.page_size,
-                table.shape[1], kv.shape[0], 0 if window is None else int(window), ctypes.c_float(scale), int(rot),
-                _ptr(head_gate), _DT[q_rows.dtype], _stream()), "latent_attention (turned part)")
+                q_rows, ldq, w_uk, w_uv, sinks, kv, table, ctx.positions,
+                ctx.token_req, ctx.req_slot, None, out, T, heads, dim, vdim, rank, cache.page_size,
+                table.shape[1], kv.shape[0], 0 if window is None else int(window), float(scale), int(rot),
+                head_gate, _DT[q_rows.dtype], _stream()), "latent_attention (turned part)")
             self.launches += 1
             return out
         if tiled:
@@ -1388,9 +1378,9 @@ class CudaKernels:
                                                 head_gate=head_gate)
         out = torch.empty(T, heads * vdim, dtype=q_rows.dtype, device=q_rows.device)
         _check(self.lib.ifx_latent_attention_generic(
-            _ptr(q_rows), ldq, _ptr(w_uk), _ptr(w_uv), _ptr(sinks), _ptr(kv), _ptr(table), _ptr(ctx.positions),
-            _ptr(ctx.token_req), _ptr(ctx.req_slot), _ptr(None), _ptr(out), T, heads, dim, vdim, rank, cache.page_size,
-            table.shape[1], kv.shape[0], 0 if window is None else int(window), ctypes.c_float(scale), _DT[q_rows.dtype],
+            q_rows, ldq, w_uk, w_uv, sinks, kv, table, ctx.positions,
+            ctx.token_req, ctx.req_slot, None, out, T, heads, dim, vdim, rank, cache.page_size,
+            table.shape[1], kv.shape[0], 0 if window is None else int(window), float(scale), _DT[q_rows.dtype],
             _stream()), "latent_attention")
         self.launches += 1
         return out
@@ -1458,19 +1448,19 @@ class CudaKernels:
         olat = torch.empty(T, heads * rank, dtype=torch.bfloat16, device=q_rows.device)
         if decode:
             _check(self.lib.ifx_latent_decode(
-                _ptr(ql), _ptr(kv), _ptr(table), _ptr(items), num_items, _ptr(sinks), _ptr(olat), _ptr(ws), T, heads, rank, int(rot),
-                cache.page_size, table.shape[1], kv.shape[0], win, ctypes.c_float(scale), stretch, splits, _ptr(head_gate),
-                _ptr(self.error_flag), _stream()), "latent_attention (decode)")
+                ql, kv, table, items, num_items, sinks, olat, ws, T, heads, rank, int(rot),
+                cache.page_size, table.shape[1], kv.shape[0], win, float(scale), stretch, splits, head_gate,
+                self.error_flag, _stream()), "latent_attention (decode)")
         elif prompt:
             _check(self.lib.ifx_latent_prompt(
-                _ptr(ql), _ptr(kv), _ptr(table), _ptr(items), num_items, int(min(self.LATENT_TILE, ctx.max_span)), _ptr(sinks),
-                _ptr(olat), _ptr(ws), T, heads, rank, int(rot), cache.page_size, table.shape[1], kv.shape[0], win,
-                ctypes.c_float(scale), splits, _ptr(head_gate), _ptr(self.error_flag), _stream()), "latent_attention (prompt)")
+                ql, kv, table, items, num_items, int(min(self.LATENT_TILE, ctx.max_span)), sinks,
+                olat, ws, T, heads, rank, int(rot), cache.page_size, table.shape[1], kv.shape[0], win,
+                float(scale), splits, head_gate, self.error_flag, _stream()), "latent_attention (prompt)")
         else:
             _check(self.lib.ifx_latent_attention_mma_rot(
-                _ptr(ql), _ptr(kv), _ptr(table), _ptr(items), num_items, int(min(self.LATENT_TILE, ctx.max_span)), _ptr(sinks),
-                _ptr(olat), _ptr(ws), T, heads, rank, int(rot), cache.page_size, table.shape[1], kv.shape[0], win,
-                ctypes.c_float(scale), splits, _ptr(head_gate), _stream()), "latent_attention (tiles)")
+                ql, kv, table, items, num_items, int(min(self.LATENT_TILE, ctx.max_span)), sinks,
+                olat, ws, T, heads, rank, int(rot), cache.page_size, table.shape[1], kv.shape[0], win,
+                float(scale), splits, head_gate, _stream()), "latent_attention (tiles)")
         self.launches += 1 + int(splits > 1)
         return self.linear_heads(olat, w_uv, heads, rank, vdim, w_is_nk=True)               # [T, heads * vdim]
 
@@ -1481,14 +1471,14 @@ class CudaKernels:
             return x
         _need(x.dtype == torch.float32 and x.is_contiguous(), "cast_rows: contiguous float32 rows")
         out = torch.empty(x.shape, dtype=dtype, device=x.device)
-        _check(self.lib.ifx_cast_rows(_ptr(x), _ptr(out), ctypes.c_longlong(x.numel()), _DT[dtype], _stream()), "cast_rows")
+        _check(self.lib.ifx_cast_rows(x, out, (x.numel()), _DT[dtype], _stream()), "cast_rows")
         self.launches += 1
         return out
 
     def tanh(self, z):
         """tanh of every element, in place."""
         _need(z.is_contiguous(), "tanh: contiguous input")
-        _check(self.lib.ifx_tanh_rows(_ptr(z), ctypes.c_longlong(z.numel()), _DT[z.dtype], _stream()), "tanh")
+        _check(self.lib.ifx_tanh_rows(z, (z.numel()), _DT[z.dtype], _stream()), "tanh")
         self.launches += 1
         return z
 
@@ -1503,8 +1493,8 @@ class CudaKernels:
               and prev_offset + C <= state.shape[1], "token_shift_mix: the state does not hold a row")
         out = torch.empty(mu.shape[0], T, C, dtype=out_dtype, device=x.device)
         _check(self.lib.ifx_token_shift_mix(
-            _ptr(x), _ptr(mu), ctypes.c_void_p(state.data_ptr() + 4 * prev_offset), ctypes.c_longlong(state.shape[1]),
-            _ptr(ctx.token_req), _ptr(ctx.req_slot), _ptr(ctx.cu_seqlens), _ptr(out), T, C, mu.shape[0], _DT[out_dtype],
+            x, mu, state.data_ptr() + 4 * prev_offset, state.shape[1],
+            ctx.token_req, ctx.req_slot, ctx.cu_seqlens, out, T, C, mu.shape[0], _DT[out_dtype],
             _stream()), "token_shift_mix")
         self.launches += 1
         return out
@@ -1580,25 +1570,25 @@ class CudaKernels:
             size += int(self.lib.ifx_chunk_scan_scratch_floats(T, ctx.num_requests, least, heads, dim, dim, 1))
         scratch = torch.empty(size, dtype=torch.float32, device=r.device)         # the sums, and what the stretches need
         y = torch.empty(T, HD, dtype=out_dtype, device=r.device)
-        common = (_ptr(state), ctypes.c_void_p(state.data_ptr() + 4 * prev_offset), _LL(state.shape[1]), _ptr(x), C, _ptr(ctx.cu_seqlens),
-                  _ptr(ctx.req_slot), _ptr(scratch))
-        rows = (_ptr(r), _ptr(k), _ptr(v), _ptr(w_raw))
+        common = (state, state.data_ptr() + 4 * prev_offset, state.shape[1], x, C, ctx.cu_seqlens,
+                  ctx.req_slot, scratch)
+        rows = (r, k, v, w_raw)
         if by_chunks:
-            room = ctypes.c_void_p(scratch.data_ptr() + 4 * T * HD)               # (heads of 64 or 128: still on 16 bytes)
-            rc = self.lib.ifx_chunk_wkv_scan(*rows, _ptr(w0), _ptr(u), *common, ctx.num_requests, T, least, heads, dim, ld, ld_w, room,
+            room = scratch.data_ptr() + 4 * T * HD               # (heads of 64 or 128: still on 16 bytes)
+            rc = self.lib.ifx_chunk_wkv_scan(*rows, w0, u, *common, ctx.num_requests, T, least, heads, dim, ld, ld_w, room,
                                              _stream())
             if rc != _MISALIGNED:
                 _check(rc, "wkv_scan (stretches)")
                 if short:
-                    _check(self.lib.ifx_wkv_scan(*rows, _ptr(g), _ptr(w0), _ptr(u), _ptr(norm_w), ctypes.c_float(eps), *common, _ptr(y),
+                    _check(self.lib.ifx_wkv_scan(*rows, g, w0, u, norm_w, float(eps), *common, y,
                                                  ctx.num_requests, T, heads, dim, ld, ld_w, _DT[out_dtype], short, _stream()),
                            "wkv_scan (short spans)")
                     self.launches += 1
-                _check(self.lib.ifx_wkv_norm(_ptr(scratch), _ptr(g), _ptr(norm_w), ctypes.c_float(eps), _ptr(y), T, heads, dim, ld,
+                _check(self.lib.ifx_wkv_norm(scratch, g, norm_w, float(eps), y, T, heads, dim, ld,
                                              _DT[out_dtype], _stream()), "wkv_norm")
                 self.launches += 4
                 return y
-        _check(self.lib.ifx_wkv_scan(*rows, _ptr(g), _ptr(w0), _ptr(u), _ptr(norm_w), ctypes.c_float(eps), *common, _ptr(y), ctx.num_requests,
+        _check(self.lib.ifx_wkv_scan(*rows, g, w0, u, norm_w, float(eps), *common, y, ctx.num_requests,
                                      T, heads, dim, ld, ld_w, _DT[out_dtype], 0, _stream()), "wkv_scan")
         self.launches += 1
         return y
@@ -1660,17 +1650,17 @@ class CudaKernels:
             if short:
                 scan_room = torch.empty(int(self.lib.ifx_delta_rule_scratch_floats(T, heads, dim)), dtype=torch.float32, device=proj.device)
             rc = self.lib.ifx_delta_chunks_scan(
-                _ptr(proj), proj.shape[1], _ptr(w_raw), _ptr(w0), _ptr(a_bias), _ptr(norm_w), ctypes.c_float(eps), _ptr(state),
-                ctypes.c_longlong(state.stride(0)), _ptr(ctx.cu_seqlens), _ptr(ctx.req_slot), _ptr(room), _ptr(y), ctx.num_requests, T,
-                least, heads, dim, _DT[out_dtype], _ptr(scan_room), _stream())
+                proj, proj.shape[1], w_raw, w0, a_bias, norm_w, float(eps), state,
+                state.stride(0), ctx.cu_seqlens, ctx.req_slot, room, y, ctx.num_requests, T,
+                least, heads, dim, _DT[out_dtype], scan_room, _stream())
             if rc != _MISALIGNED:
                 _check(rc, "delta_rule_scan (stretches)")
                 self.launches += 6 if short else 4
                 return y
         scratch = torch.empty(int(self.lib.ifx_delta_rule_scratch_floats(T, heads, dim)), dtype=torch.float32, device=proj.device)
         _check(self.lib.ifx_delta_rule_scan(
-            _ptr(proj), proj.shape[1], _ptr(w_raw), _ptr(w0), _ptr(a_bias), _ptr(norm_w), ctypes.c_float(eps), _ptr(state),
-            ctypes.c_longlong(state.stride(0)), _ptr(ctx.cu_seqlens), _ptr(ctx.req_slot), _ptr(scratch), _ptr(y),
+            proj, proj.shape[1], w_raw, w0, a_bias, norm_w, float(eps), state,
+            state.stride(0), ctx.cu_seqlens, ctx.req_slot, scratch, y,
             ctx.num_requests, T, heads, dim, _DT[out_dtype], _stream()), "delta_rule_scan")
         self.launches += 3
         return y
@@ -1688,8 +1678,8 @@ class CudaKernels:
               and correction.numel() == n)), "moe_route: float32 logits and corrections")
         ids = torch.empty(T, top, dtype=torch.int32, device=z.device)
         weights = torch.empty(T, top, dtype=torch.float32, device=z.device)
-        _check(self.lib.ifx_moe_route_kind(_ptr(z), _ptr(correction), _ptr(ids), _ptr(weights), T, n, int(top),
-                                           2 if kind == "sigmoid_normalized" else int(bool(of_chosen)), ctypes.c_float(floor),
+        _check(self.lib.ifx_moe_route_kind(z, correction, ids, weights, T, n, int(top),
+                                           2 if kind == "sigmoid_normalized" else int(bool(of_chosen)), float(floor),
                                            _stream()), "moe_route")
         self.launches += 1
         return ids, weights
@@ -1706,8 +1696,8 @@ class CudaKernels:
         T = h.shape[0]
         ids = torch.empty(T, top, dtype=torch.int32, device=h.device)
         weights = torch.empty(T, top, dtype=torch.float32, device=h.device)
-        _check(self.lib.ifx_moe_choose(_ptr(h), _ptr(w_router), _ptr(correction), _ptr(ids), _ptr(weights), T, h.shape[1], n, int(top),
-                                       2 if kind == "sigmoid_normalized" else int(bool(of_chosen)), ctypes.c_float(floor), _stream()),
+        _check(self.lib.ifx_moe_choose(h, w_router, correction, ids, weights, T, h.shape[1], n, int(top),
+                                       2 if kind == "sigmoid_normalized" else int(bool(of_chosen)), float(floor), _stream()),
                "moe_choose")
         self.launches += 1
         return ids, weights
@@ -1735,9 +1725,9 @@ class CudaKernels:
                         h, w_up, w_down, ids, weights, experts, out_dtype, glu=glu)
             act = torch.empty(T * top, ff, dtype=h.dtype, device=h.device)
             out = torch.empty(T, width, dtype=out_dtype, device=h.device)
-            _check(self.lib.ifx_moe_experts_glu(_ptr(h), _ptr(w_up), _ptr(w_down), _ptr(ids), _ptr(weights), _ptr(act), _ptr(out),
+            _check(self.lib.ifx_moe_experts_glu(h, w_up, w_down, ids, weights, act, out,
                                                 T, top, int(experts), width, ff, _DT[h.dtype], _DT[out_dtype], 1,
-                                                ctypes.c_float(glu[0]), ctypes.c_float(glu[1]), ctypes.c_float(glu[2]),
+                                                float(glu[0]), float(glu[1]), float(glu[2]),
                                                 _stream()), "moe_experts (gated)")
             self.launches += 2
             return out
@@ -1752,8 +1742,8 @@ class CudaKernels:
                     h, w_up, w_down, ids, weights, experts, out_dtype)
         act = torch.empty(T * top, ff, dtype=h.dtype, device=h.device)
         out = torch.empty(T, width, dtype=out_dtype, device=h.device)
-        _check(self.lib.ifx_moe_experts(_ptr(h), _ptr(w_up if experts else None), _ptr(w_down if experts else None), _ptr(ids),
-                                        _ptr(weights), _ptr(act), _ptr(out), T, top, int(experts), width, ff, _DT[h.dtype],
+        _check(self.lib.ifx_moe_experts(h, (w_up if experts else None), (w_down if experts else None), ids,
+                                        weights, act, out, T, top, int(experts), width, ff, _DT[h.dtype],
                                         _DT[out_dtype], _stream()), "moe_experts")
         self.launches += 2 if experts else 1
         return out
@@ -1810,9 +1800,9 @@ class CudaKernels:
         scratch = torch.empty(room, dtype=torch.uint8, device=h.device)
         out = torch.empty(T, width, dtype=out_dtype, device=h.device)
         limit, slope, offset = (glu if len(glu) > 2 else (*glu, 1.0)) if glu is not None else (0.0, 0.0, 0.0)
-        _check(self.lib.ifx_moe_sorted(_ptr(h), _ptr(w_up), _ptr(w_down), _ptr(ids), _ptr(weights), _ptr(out), T, top, int(experts),
-                                       width, ff, _DT[out_dtype], int(glu is not None), int(few), ctypes.c_float(limit),
-                                       ctypes.c_float(slope), ctypes.c_float(offset), _ptr(scratch), _LL(room), _ptr(self.error_flag),
+        _check(self.lib.ifx_moe_sorted(h, w_up, w_down, ids, weights, out, T, top, int(experts),
+                                       width, ff, _DT[out_dtype], int(glu is not None), int(few), float(limit),
+                                       float(slope), float(offset), scratch, room, self.error_flag,
                                        _stream()), "moe experts (sorted rows)")
         self.launches += 5
         return out
@@ -1824,9 +1814,9 @@ class CudaKernels:
         T, H = x.shape
         _need(x.dtype == torch.float32 and x.is_contiguous() and table.is_contiguous() and tuple(table.shape) == (buckets + 1, H)
               and state is not None and state.dtype == torch.int32, "bigram_add: bad operands")
-        _check(self.lib.ifx_bigram_add(_ptr(x), _ptr(table), _ptr(token_ids), _ptr(ctx.positions), _ptr(ctx.token_req),
-                                       _ptr(ctx.req_slot), _ptr(ctx.cu_seqlens), _ptr(state), ctypes.c_longlong(state.stride(0)),
-                                       T, H, int(vocab), ctypes.c_longlong(mul_prev), ctypes.c_longlong(mul_cur), int(buckets),
+        _check(self.lib.ifx_bigram_add(x, table, token_ids, ctx.positions, ctx.token_req,
+                                       ctx.req_slot, ctx.cu_seqlens, state, state.stride(0),
+                                       T, H, int(vocab), mul_prev, mul_cur, int(buckets),
                                        _DT[table.dtype], _stream()), "bigram_add")
         self.launches += 1
 
@@ -1849,9 +1839,9 @@ class CudaKernels:
               and w_a.dtype == torch.float32 and w_b.dtype == torch.float32, "rmsnorm_pair: bad operands")
         out_a = torch.empty(T, H, dtype=out_dtype, device=x.device)
         out_b = torch.empty(T, H, dtype=out_dtype, device=x.device)
-        _check(self.lib.ifx_rmsnorm_pair(_ptr(x), _ptr(w_a), ctypes.c_float(eps_a), _ptr(w_b), ctypes.c_float(eps_b), _ptr(out_a),
-                                         _ptr(out_b), T, H, _DT[out_dtype], _ptr(va), _DT[va.dtype] if va is not None else 0,
-                                         _ptr(vsa), _ptr(vb), _ptr(vb2), _DT[vb.dtype] if vb is not None else 0, _ptr(vsb),
+        _check(self.lib.ifx_rmsnorm_pair(x, w_a, float(eps_a), w_b, float(eps_b), out_a,
+                                         out_b, T, H, _DT[out_dtype], va, _DT[va.dtype] if va is not None else 0,
+                                         vsa, vb, vb2, _DT[vb.dtype] if vb is not None else 0, vsb,
                                          _stream()), "rmsnorm_pair")
         self.launches += 1
         return out_a, out_b
@@ -1861,7 +1851,7 @@ class CudaKernels:
         _need(kind in ("sigmoid", "silu") and a.shape == g.shape and a.dtype == g.dtype and a.is_contiguous() and g.is_contiguous(),
               "gate_mul: bad operands")
         out = torch.empty_like(a)
-        _check(self.lib.ifx_gate_mul(_ptr(a), _ptr(g), _ptr(out), ctypes.c_longlong(a.numel()), _DT[a.dtype], int(kind == "silu"),
+        _check(self.lib.ifx_gate_mul(a, g, out, (a.numel()), _DT[a.dtype], int(kind == "silu"),
                                      _stream()), "gate_mul")
         self.launches += 1
         return out
@@ -1870,7 +1860,7 @@ class CudaKernels:
     def _rows_f32(t, what):
         if t.dtype != torch.float32 or t.dim() != 2 or t.stride(1) != 1:
             raise KernelError(f"{what}: float32 rows with unit column stride")
-        return ctypes.c_void_p(t.data_ptr()), ctypes.c_longlong(t.stride(0))
+        return t.data_ptr(), t.stride(0)
 
     def decay_scan(self, q, k, v, raw, state, ctx, heads, groups, dk, dv, decay, tau=1.0, q_scale=1.0, step_bias=None,
                    log_rate=None, skip=None, rate=None):
@@ -1898,8 +1888,8 @@ class CudaKernels:
                   "decay_scan: per-head vectors are float32 [heads]")
         out = torch.empty(T, heads * dv, dtype=torch.float32, device=q.device)
         rows = (*self._rows_f32(q, "decay_scan q"), *self._rows_f32(k, "decay_scan k"), *self._rows_f32(v, "decay_scan v"),
-                *(self._rows_f32(raw, "decay_scan raw") if raw is not None else (_ptr(None), _LL(0))), _ptr(state), _LL(state.stride(0)),
-                _ptr(ctx.req_slot), _ptr(ctx.cu_seqlens), _ptr(out), _ptr(step_bias), _ptr(log_rate), _ptr(skip))
+                *(self._rows_f32(raw, "decay_scan raw") if raw is not None else (None, 0)), state, state.stride(0),
+                ctx.req_slot, ctx.cu_seqlens, out, step_bias, log_rate, skip)
         longest = int(ctx.max_span)
         by_chunks = self._scans_by_chunks(getattr(ctx, "dtype", None), ctx, heads, dk, dv, constant=mode == 2)
         if by_chunks:
@@ -1907,8 +1897,8 @@ class CudaKernels:
             room = torch.empty(int(self.lib.ifx_chunk_scan_scratch_floats(T, ctx.num_requests, least, heads, dk, dv, int(mode == 0))),
                                dtype=torch.float32, device=q.device)
             rc = self.lib.ifx_chunk_decay_scan(*rows, ctx.num_requests, T, least, int(heads), int(groups), int(dk), int(dv), mode,
-                                               ctypes.c_float(tau), ctypes.c_float(q_scale), _ptr(room), _ptr(rate),
-                                               self.stretch, _ptr(self.error_flag), _stream())
+                                               float(tau), float(q_scale), room, rate,
+                                               self.stretch, self.error_flag, _stream())
             if rc != _MISALIGNED:
                 _check(rc, "decay_scan (stretches)")
                 self.launches += 3
@@ -1919,7 +1909,7 @@ class CudaKernels:
         if longest >= 64 and mode != 2:
             scratch = torch.empty(T * (heads * dk if mode == 0 else 2 * heads), dtype=torch.float32, device=q.device)
         _check(self.lib.ifx_decay_scan_rate(*rows, ctx.num_requests, T, longest, int(longest < ctx.max_span), int(heads), int(groups), int(dk),
-                                            int(dv), mode, ctypes.c_float(tau), ctypes.c_float(q_scale), 296, _ptr(scratch), _ptr(rate), _stream()),
+                                            int(dv), mode, float(tau), float(q_scale), 296, scratch, rate, _stream()),
                "decay_scan")
         self.launches += 1 + int(scratch is not None)
         return out
@@ -1934,7 +1924,7 @@ class CudaKernels:
               and kind in ("silu", "sigmoid"), "gated_groupnorm: bad operands")
         out = torch.empty(T, C, dtype=out_dtype, device=y.device)
         gp, gs = self._rows_f32(gate, "gated_groupnorm gate")
-        _check(self.lib.ifx_gated_groupnorm(_ptr(y), gp, gs, _ptr(w), 0 if w is None else int(w.numel()), ctypes.c_float(eps), _ptr(out), T, C,
+        _check(self.lib.ifx_gated_groupnorm(y, gp, gs, w, 0 if w is None else int(w.numel()), float(eps), out, T, C,
                                             int(groups), int(bool(gate_first)), int(kind == "sigmoid"), _DT[out_dtype], _stream()),
                "gated_groupnorm")
         self.launches += 1
@@ -1946,8 +1936,8 @@ class CudaKernels:
         _need(a.is_contiguous() and b.is_contiguous() and a.shape == b.shape and (w_a is None) == (w_b is None),
               "pair_combine: rows of one shape")
         out = torch.empty(T, C, dtype=torch.float32, device=a.device)
-        _check(self.lib.ifx_pair_combine(_ptr(a), _DT[a.dtype], _ptr(b), _DT[b.dtype], _ptr(w_a), _ptr(w_b), ctypes.c_float(c_a),
-                                         ctypes.c_float(c_b), ctypes.c_float(eps), _ptr(out), T, C, _stream()), "pair_combine")
+        _check(self.lib.ifx_pair_combine(a, _DT[a.dtype], b, _DT[b.dtype], w_a, w_b, float(c_a),
+                                         float(c_b), float(eps), out, T, C, _stream()), "pair_combine")
         self.launches += 1
         return out
 
@@ -1962,8 +1952,8 @@ class CudaKernels:
         _need(x.dtype == torch.float32 and x.is_contiguous() and a.shape == x.shape and a.is_contiguous()
               and (b is None or (b.shape == x.shape and b.is_contiguous())) and (b2 is None or (b is not None and b2.is_contiguous())),
               "residual_add_vectors: bad operands")
-        _check(self.lib.ifx_residual_add_vectors(_ptr(x), _ptr(a), _DT[a.dtype], _ptr(s_a), _ptr(b), _ptr(b2),
-                                                 _DT[b.dtype] if b is not None else 0, _ptr(s_b), T, C, _stream()),
+        _check(self.lib.ifx_residual_add_vectors(x, a, _DT[a.dtype], s_a, b, b2,
+                                                 _DT[b.dtype] if b is not None else 0, s_b, T, C, _stream()),
                "residual_add_vectors")
         self.launches += 1
 
@@ -1984,9 +1974,9 @@ class CudaKernels:
             _need((y is None or (tuple(y.shape[-2:]) == (T, H) and y.is_contiguous()))
                   and (bias is None or (bias.dtype == torch.float32 and bias.numel() == H and bias.is_contiguous())),
                   "norm_of_sum: a term does not match x")
-            flat += [_ptr(y), 0 if y is None else _DT[y.dtype], splits, ctypes.c_float(c), _ptr(bias)]
+            flat += [y, 0 if y is None else _DT[y.dtype], splits, float(c), bias]
         out = None if out_dtype is None else torch.empty(T, H, dtype=out_dtype, device=x.device)
-        _check(self.lib.ifx_norm_of_sum(_ptr(x), ctypes.c_float(alpha), *flat, _ptr(w), ctypes.c_float(eps), _ptr(out),
+        _check(self.lib.ifx_norm_of_sum(x, float(alpha), *flat, w, float(eps), out,
                                         0 if out is None else _DT[out_dtype], T, H, _stream()), "norm_of_sum")
         self.launches += 1
         return out
@@ -2000,9 +1990,9 @@ class CudaKernels:
     def _row_source(rows):
         """(plain pointer, dtype code, partial pointer, splits, row length) of a tensor or PartialSum."""
         if isinstance(rows, PartialSum):
-            return _ptr(None), 0, _ptr(rows.parts), rows.splits, rows.parts.shape[-1]
+            return None, 0, rows.parts, rows.splits, rows.parts.shape[-1]
         _need(rows.is_contiguous(), "projected rows must be contiguous")
-        return _ptr(rows), _DT[rows.dtype], _ptr(None), 1, rows.shape[-1]
+        return rows, _DT[rows.dtype], None, 1, rows.shape[-1]
 
     def row_norm_rope_append(self, rows, col0, bias, rotary, turn, temp, nq, nkv, d, dv, ctx, cache, q_norm=None, k_norm=None,
                              norm_eps=0.0, v_from_k=False, gate_col=None):
@@ -2029,12 +2019,12 @@ class CudaKernels:
         back = None if turn is None else torch.empty(T, dv // 2, 2, dtype=torch.float32, device=dev)
         gate = None if gate_col is None else torch.empty(T, nq, dtype=torch.float32, device=dev)
         _check(self.lib.ifx_row_norm_rope_append(
-            src, code, part, splits, _LL(ld), int(col0), _ptr(bias), _ptr(q_norm), _ptr(k_norm), ctypes.c_float(norm_eps),
-            _ptr(None if rotary is None else rotary.inv_freq), 0 if rotary is None else int(rotary.rotary_dim),
-            int(rotary is not None and rotary.interleaved), _ptr(None if turn is None else turn.inv_freq),
-            int(turn is not None and turn.interleaved), _ptr(temp), _ptr(ctx.positions), _ptr(ctx.token_req), _ptr(ctx.req_slot),
-            _ptr(table), table.shape[1], cache.page_size, kv.shape[0], _ptr(kv), _ptr(q_out), _ptr(back), T, nq, nkv, d, dv,
-            kv.shape[-1], int(bool(cache.writes)), int(bool(v_from_k)), _ptr(gate), int(gate_col or 0), _DT[kv.dtype], _stream()),
+            src, code, part, splits, ld, int(col0), bias, q_norm, k_norm, float(norm_eps),
+            (None if rotary is None else rotary.inv_freq), 0 if rotary is None else int(rotary.rotary_dim),
+            int(rotary is not None and rotary.interleaved), (None if turn is None else turn.inv_freq),
+            int(turn is not None and turn.interleaved), temp, ctx.positions, ctx.token_req, ctx.req_slot,
+            table, table.shape[1], cache.page_size, kv.shape[0], kv, q_out, back, T, nq, nkv, d, dv,
+            kv.shape[-1], int(bool(cache.writes)), int(bool(v_from_k)), gate, int(gate_col or 0), _DT[kv.dtype], _stream()),
             "row_norm_rope_append")
         self.launches += 1
         turned = None if back is None else (back, turn.interleaved)
@@ -2048,7 +2038,7 @@ class CudaKernels:
         plain = not isinstance(rows, PartialSum)
         _need(not plain or rows.dtype == torch.float32, "silu_columns: float32 rows")
         out = rows if plain else torch.empty(T, ld, dtype=torch.float32, device=rows.parts.device)
-        _check(self.lib.ifx_silu_columns(src, part, splits, _LL(ld), 0, _ptr(out), T, int(ld), int(acted), _stream()), "silu_columns")
+        _check(self.lib.ifx_silu_columns(src, part, splits, ld, 0, out, T, int(ld), int(acted), _stream()), "silu_columns")
         self.launches += 1
         return out
 
@@ -2064,9 +2054,9 @@ class CudaKernels:
         device = rows.device if plain else rows.parts.device
         out = rows if plain and ld == width and col0 == 0 else torch.empty(T, width, dtype=torch.float32, device=device)
         _check(self.lib.ifx_rotate_rows(
-            src, part, splits, _LL(ld), int(col0), _ptr(None if rotary is None else rotary.inv_freq),
-            0 if rotary is None else int(rotary.rotary_dim), int(rotary is not None and rotary.interleaved), _ptr(ctx.positions),
-            _ptr(out), T, int(width), int(heads), int(dk), ctypes.c_float(k_scale), _stream()), "rotate_rows")
+            src, part, splits, ld, int(col0), (None if rotary is None else rotary.inv_freq),
+            0 if rotary is None else int(rotary.rotary_dim), int(rotary is not None and rotary.interleaved), ctx.positions,
+            out, T, int(width), int(heads), int(dk), float(k_scale), _stream()), "rotate_rows")
         self.launches += 1
         return out
 
@@ -2081,8 +2071,8 @@ class CudaKernels:
         src, splits = (rows.parts, rows.splits) if isinstance(rows, PartialSum) else (rows, 1)
         _need(src.dtype == torch.float32 and src.is_contiguous(), "gated_scan: float32 rows")
         out = torch.empty(T, width, dtype=out_dtype, device=src.device)
-        _check(self.lib.ifx_gated_scan(_ptr(src), splits, _ptr(bias), _ptr(state), _LL(state.stride(0)), _ptr(ctx.req_slot),
-                                       _ptr(ctx.cu_seqlens), _ptr(out), ctx.num_requests, T, int(ctx.max_span), int(width),
+        _check(self.lib.ifx_gated_scan(src, splits, bias, state, state.stride(0), ctx.req_slot,
+                                       ctx.cu_seqlens, out, ctx.num_requests, T, int(ctx.max_span), int(width),
                                        _DT[out_dtype], _stream()), "gated_scan")
         self.launches += 1
         return out
@@ -2092,23 +2082,23 @@ class CudaKernels:
         R, V = logits.shape
         out = torch.empty(R, dtype=torch.int32, device=logits.device)
         if V >= 16384 and R <= 256:                      # long rows, few of them: many blocks per row
-            _check(self.lib.ifx_argmax_chunks(_ptr(logits), _ptr(out), R, V, 32, _ptr(self._argmax_val),
-                                              _ptr(self._argmax_idx), _ptr(self._argmax_tickets), _stream()), "argmax")
+            _check(self.lib.ifx_argmax_chunks(logits, out, R, V, 32, self._argmax_val,
+                                              self._argmax_idx, self._argmax_tickets, _stream()), "argmax")
             self.launches += 1
             return out
-        _check(self.lib.ifx_argmax(_ptr(logits), _ptr(out), R, V, _stream()), "argmax")
+        _check(self.lib.ifx_argmax(logits, out, R, V, _stream()), "argmax")
         self.launches += 1
         return out
 
     def penalties(self, logits, tokens, counts, rep, freq, pres):
         R, V = logits.shape
-        _check(self.lib.ifx_penalties(_ptr(logits), _ptr(tokens), _ptr(counts), _ptr(rep), _ptr(freq), _ptr(pres),
+        _check(self.lib.ifx_penalties(logits, tokens, counts, rep, freq, pres,
                                       R, tokens.shape[1], V, _stream()), "penalties")
         self.launches += 1
 
     def logit_bias(self, logits, rows, tokens, bias):
         R, V = logits.shape
-        _check(self.lib.ifx_logit_bias(_ptr(logits), _ptr(rows), _ptr(tokens), _ptr(bias), rows.numel(), R, V,
+        _check(self.lib.ifx_logit_bias(logits, rows, tokens, bias, rows.numel(), R, V,
                                        _stream()), "logit_bias")
         self.launches += 1
 
@@ -2122,9 +2112,9 @@ class CudaKernels:
             self._sample_scratch = torch.zeros(int(self.lib.ifx_sample_scratch_bytes(self._sample_capacity)),
                                                dtype=torch.uint8, device=logits.device)
         passes = 3 + (1 if features & 3 else 0) + (2 if features & 1 else 0) + (3 if features & 2 else 0)
-        _check(self.lib.ifx_sample_blocks(_ptr(logits), _ptr(temperature), _ptr(top_k), _ptr(top_p), _ptr(min_p),
-                                          _ptr(seed_lo), _ptr(seed_hi), _ptr(step), _ptr(out), R, V, int(features),
-                                          _ptr(self._sample_scratch), self._sample_capacity, _stream()), "sample")
+        _check(self.lib.ifx_sample_blocks(logits, temperature, top_k, top_p, min_p,
+                                          seed_lo, seed_hi, step, out, R, V, int(features),
+                                          self._sample_scratch, self._sample_capacity, _stream()), "sample")
         self.launches += passes
         return out
 
@@ -2133,8 +2123,8 @@ class CudaKernels:
         R, V = logits.shape
         probs = torch.empty(R, V, dtype=torch.float32, device=logits.device)
         out = torch.empty(R, dtype=torch.int32, device=logits.device)
-        _check(self.lib.ifx_sample(_ptr(logits), _ptr(probs), _ptr(temperature), _ptr(top_k), _ptr(top_p),
-                                   _ptr(min_p), _ptr(seed_lo), _ptr(seed_hi), _ptr(step), _ptr(out), R, V,
+        _check(self.lib.ifx_sample(logits, probs, temperature, top_k, top_p,
+                                   min_p, seed_lo, seed_hi, step, out, R, V,
                                    _stream()), "sample")
         self.launches += 1
         return out

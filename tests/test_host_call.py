@@ -1,0 +1,78 @@
+"""Calls of C entry points by host_call.cpp against the same calls through ctypes (no GPU: a small library of its own)."""
+import ctypes
+import importlib
+import importlib.util
+import random
+import shutil
+import subprocess
+
+import pytest
+import torch
+
+build = importlib.import_module("inferflux_b200.csrc.build")
+# p pointer, i int, l long long, f float; more integers than registers, floats between them, both many
+SIGNATURES = ["i", "p", "f", "pilf", "pppppp", "ppppppp", "fiiiiiiiiif", "pppllliiifffpppiiilllfffpp", "l" * 54, "f" * 8 + "p" * 30, "ilp" * 18]
+
+
+@pytest.fixture(scope="module")
+def library(tmp_path_factory):
+    if shutil.which("g++") is None:
+        pytest.skip("no g++")
+    d = tmp_path_factory.mktemp("host_call")
+    types = {"p": "const void*", "i": "int", "l": "long long", "f": "float"}
+    code = ["#include <stdint.h>"]
+    for n, sig in enumerate(SIGNATURES):
+        args = ", ".join(f"{types[c]} a{i}" for i, c in enumerate(sig))
+        terms = "".join(f" h = h * 1000003 + (long long){'(uintptr_t)' if c == 'p' else ''}a{i}{' * 4096.0f' if c == 'f' else ''};".replace(
+            f"(long long)a{i} * 4096.0f", f"(long long)(a{i} * 4096.0f)") for i, c in enumerate(sig))
+        code.append(f'extern "C" long long w{n}({args}) {{ unsigned long long h = 1;{terms} return (long long)h; }}')
+        code.append(f'extern "C" int n{n}({args}) {{ return (int)w{n}({", ".join(f"a{i}" for i in range(len(sig)))}); }}')
+    (d / "f.cpp").write_text("\n".join(code))
+    subprocess.run(["g++", "-shared", "-fPIC", "-O1", str(d / "f.cpp"), "-o", str(d / "f.so")], check=True)
+    build._compile_host(d)
+    spec = importlib.util.spec_from_file_location("_ifx_host", d / build.HOST_NAME)
+    host = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(host)
+    return ctypes.CDLL(str(d / "f.so")), host
+
+
+def _arguments(sig, r):
+    """(as a program passes them, as ctypes wants them)"""
+    plain, wrapped = [], []
+    for c in sig:
+        if c == "p":
+            t = None if r.random() < 0.2 else torch.zeros(3)
+            plain.append(t)
+            wrapped.append(ctypes.c_void_p(0 if t is None else t.data_ptr()))
+        elif c == "f":
+            x = r.choice([0.0, -1.5, 0.1, 3e5])
+            plain.append(x)
+            wrapped.append(ctypes.c_float(x))
+        else:
+            x = r.choice([0, -1, True, 7, -(1 << 31), (1 << 31) - 1] + ([1 << 40, -(1 << 45)] if c == "l" else []))
+            plain.append(x)
+            wrapped.append((ctypes.c_int if c == "i" else ctypes.c_longlong)(x))
+    return plain, wrapped
+
+
+@pytest.mark.parametrize("n", range(len(SIGNATURES)))
+def test_as_through_ctypes(library, n):
+    lib, host = library
+    r = random.Random(n)
+    for name, kind in ((f"w{n}", ctypes.c_longlong), (f"n{n}", ctypes.c_int)):
+        fn = getattr(lib, name)
+        fn.restype = kind
+        fast = host.Function(ctypes.cast(fn, ctypes.c_void_p).value, kind is ctypes.c_longlong, torch.Tensor)
+        for _ in range(20):
+            plain, wrapped = _arguments(SIGNATURES[n], r)
+            assert fast(*plain) == fn(*wrapped) == fast(*wrapped)
+
+
+def test_what_it_refuses(library):
+    lib, host = library
+    fast = host.Function(ctypes.cast(lib.w0, ctypes.c_void_p).value, True, torch.Tensor)
+    for args, error in ((("x",), AttributeError), (([1],), AttributeError), ((1.0,) * 9, TypeError), ((1,) * 55, TypeError)):
+        with pytest.raises(error):
+            fast(*args)
+    with pytest.raises(TypeError):
+        fast(a=1)
