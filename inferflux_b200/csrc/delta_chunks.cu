@@ -30,11 +30,11 @@
 // Error of the state against 64 bits (2-norm, scan and this, 2,048 tokens): parameters where trained models have them 5.2e-7 and
 // 4.6e-7, decays near one 1.76e-6 and 1.70e-6, random ones 0.95e-7 and 1.00e-7.  (With operands of 22 bits 241 us, 1.4e-7 in the last
 // case, and 1.0e-6 in place of the scan's 4.6e-7 where 130 keys are nearly the same.)
-#include "chunk_scan.cuh"
+#include "parts_tcgen05.cuh"
 
 namespace ifx {
 
-constexpr int kDcThreads = 256, kDcD = 64, kDcP = kPitchV;
+constexpr int kDcThreads = 512, kDcD = 64, kDcP = kPitchV;
 constexpr float kDcFloor = 0.6065306597126334f;            // exp(-1/2)
 
 struct DeltaChunkArgs {
@@ -61,126 +61,112 @@ __device__ __forceinline__ float from_parts(uint32_t hi, uint32_t mid, uint32_t 
   return splits(h) ? h + (part(mid) + part(lo)) : h;
 }
 
-struct DeltaChunkLayout {
+// Shared memory of delta_local, bytes from the first 1,024 boundary.  Tiles as in parts_tcgen05.cuh, rows of 64 numbers.
+struct DeltaLayout {
+  static constexpr int P = kPitchA, FLOATS = kChunk * P * 4;                // a float32 matrix of 64 x 64
+  static constexpr uint32_t UR = 0, KE = UR + 3 * 128 * 128, V = KE + 3 * 128 * 128, B = V + 3 * 64 * 128, U32 = B + 3 * 64 * 128, R32 = U32 + FLOATS,
+                            M = R32 + FLOATS, MP = M + FLOATS, MID = MP + 3 * 64 * 128, END = MID + 256, BYTES = END + 256;
+  static constexpr uint32_t NA = UR, X = UR, W = M;        // in their places later, or before
+  static_assert(MP % 1024 == 0, "a tile's place");
+  static constexpr size_t SMEM = 1024 + BYTES + 4096;     // (48 rows of M from row 48 on are read up to row 95)
+};
+// The same rows as float32, for a stretch that is walked token by token.
+struct DeltaWalkLayout {
   static constexpr int TILE = kChunk * kDcP;
-  static constexpr int R = 0, U = TILE, K = 2 * TILE, E = 3 * TILE, V = 4 * TILE, A = 5 * TILE, MID = A + kChunk * kPitchA,
-                       END = MID + kDcD, FLOATS = END + kDcD;
-  static constexpr size_t BYTES = (size_t)FLOATS * sizeof(float);
+  static constexpr int R = 0, U = TILE, K = 2 * TILE, E = 3 * TILE, V = 4 * TILE, W = 5 * TILE, FLOATS = W + kChunk * kPitchA;
+  static_assert(FLOATS * 4 <= (int)DeltaLayout::BYTES, "room");
 };
-
-// A warp makes 16 columns of two blocks of 16 rows: the first and the last, or the two in the middle.  Both halves of the warps then
-// have the same share of what lies below a diagonal, and split a column operand once for both.
-struct DcTile {
-  int r0, r1, c;                                            // rows of the two blocks, columns
-  __device__ __forceinline__ DcTile(int warp) : r0((warp >> 2) * 16), r1(48 - (warp >> 2) * 16), c((warp & 3) * 16) {}
-  __device__ __forceinline__ int row(int b) const { return b ? r1 : r0; }
-};
-typedef float DcAcc[2][2][4];                               // block of rows, 8 columns, the product's own order
-
-// acc = rows . columns^T of two tiles whose inner size runs along the rows, in the blocks on and below the diagonal.
-__device__ __forceinline__ void dc_pairs(DcAcc& acc, const float* x, const float* y, const DcTile& w, int lane) {
-  if (w.c > w.r1) return;
-#pragma unroll 2
-  for (int kk = 0; kk < kDcD; kk += 16) {
-    FragA fa;
-    FragB fb[2];
-#pragma unroll
-    for (int j = 0; j < 2; ++j) load_b_rows(fb[j], y + (w.c + j * 8) * kDcP + kk, kDcP, lane);
-#pragma unroll
-    for (int b = 0; b < 2; ++b) {
-      if (w.c > w.row(b)) continue;
-      load_a_rows(fa, x + w.row(b) * kDcP + kk, kDcP, lane);
-#pragma unroll
-      for (int j = 0; j < 2; ++j) mma_split(acc[b][j], fa, fb[j]);
-    }
-  }
-}
-// acc += the lower triangle of a matrix times the rows of a tile.
-__device__ __forceinline__ void dc_times(DcAcc& acc, const float* m, const float* tile, const DcTile& w, int lane) {
-  for (int s = 0; s <= w.r1; s += 16) {
-    FragA fa;
-    FragB fb[2];
-#pragma unroll
-    for (int j = 0; j < 2; ++j) load_b_columns(fb[j], tile + s * kDcP + w.c + j * 8, kDcP, lane);
-#pragma unroll
-    for (int b = 0; b < 2; ++b) {
-      if (s > w.row(b)) continue;
-      load_a_single(fa, m + w.row(b) * kPitchA + s, kPitchA, lane);
-#pragma unroll
-      for (int j = 0; j < 2; ++j) mma_split(acc[b][j], fa, fb[j]);
-    }
-  }
-}
-// acc = columns of one tile . columns of another, over the tokens.
-__device__ __forceinline__ void dc_over_tokens(DcAcc& acc, const float* x, const float* y, const DcTile& w, int lane) {
-#pragma unroll 2
-  for (int s = 0; s < kChunk; s += 16) {
-    FragA fa;
-    FragB fb[2];
-#pragma unroll
-    for (int j = 0; j < 2; ++j) load_b_columns(fb[j], y + s * kDcP + w.c + j * 8, kDcP, lane);
-#pragma unroll
-    for (int b = 0; b < 2; ++b) {
-      load_a_columns(fa, x + s * kDcP + w.row(b), kDcP, lane);
-#pragma unroll
-      for (int j = 0; j < 2; ++j) mma_split(acc[b][j], fa, fb[j]);
-    }
-  }
-}
 __device__ __forceinline__ float dc_sigmoid(float z) { return 1.0f / (1.0f + expf(-z)); }
 
-__global__ void __launch_bounds__(kDcThreads, 2) delta_local_kernel(const DeltaChunkArgs a) {
-  using L = DeltaChunkLayout;
-  extern __shared__ __align__(16) float smem[];
-  float *r_s = smem + L::R, *u_s = smem + L::U, *k_s = smem + L::K, *e_s = smem + L::E, *v_s = smem + L::V,
-        *a_s = smem + L::A, *mid = smem + L::MID, *end = smem + L::END;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y, HD = a.heads * kDcD;
+// With [U; R] the 64 tokens' unit keys and queries as rows one below the other, decays counted from the middle:
+//
+//   [U; R] [K; E]^T                 = [N M; A B], of which the triangles count            rows are lanes of tensor memory
+//   [V . ]^T [N; A]^T               = (N V)^T | (A V)^T                                   value channels are lanes from here on
+//   (1 + M) [X | U]                 by substitution, a thread a column, in float32
+//   [X | U]^T B^T, [X | U]^T E, V^T K     what outputs, what is left to the state before, and what is added are short of or made of
+//
+// All 512 threads add up products (16 columns of a lane, or twice 16); the four warps whose lanes are the columns substitute, under V^T K.
+__global__ void __launch_bounds__(kDcThreads, 1) delta_local_kernel(const DeltaChunkArgs a, int* error_flag) {
+  using L = DeltaLayout;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ uint64_t bar_s[3];
+  __shared__ uint32_t tmem_holder;
+  const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31, h = blockIdx.y, HD = a.heads * kDcD;
   int first, n;
   if (!chunk_of(a.cu_seqlens, a.requests, a.min_span, blockIdx.x, first, n)) return;
   const size_t item = (size_t)blockIdx.x * a.heads + h;
+  unsigned char* smem = smem_raw + ((1024 - (smem_addr(smem_raw) & 1023)) & 1023);
+  const uint32_t base = smem_addr(smem), bar = smem_addr(bar_s);
+  float *u32 = reinterpret_cast<float*>(smem + L::U32), *r32 = reinterpret_cast<float*>(smem + L::R32), *w_s = reinterpret_cast<float*>(smem + L::W),
+        *m_s = reinterpret_cast<float*>(smem + L::M), *x_s = reinterpret_cast<float*>(smem + L::X), *mid = reinterpret_cast<float*>(smem + L::MID),
+        *end = reinterpret_cast<float*>(smem + L::END);
+  if (tid == 0) {
+    mbar_init(bar, 1);
+    mbar_init(bar + 8, 1);
+    mbar_init(bar + 16, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_holder)), "r"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_before();
 
   // ---------------------------------------------------------- rows: queries, keys, values, how much is erased, unit keys, decays
-  auto load = [&]() {
-    bool bad = false;
-#pragma unroll 2
-    for (int part = 0; part < 4; ++part) {
-      const int t = part * 16 + (tid >> 4), c = (tid & 15) * 4;             // sixteen neighbouring lanes a token
-      float4 r = make_float4(0.0f, 0.0f, 0.0f, 0.0f), k = r, v = r, e = r, w = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
-      if (t < n) {
-        const float* row = a.proj + (size_t)(first + t) * a.ld + h * kDcD + c;
-        r = *reinterpret_cast<const float4*>(row);
-        k = *reinterpret_cast<const float4*>(row + HD);
-        v = *reinterpret_cast<const float4*>(row + 2 * HD);
-        e = *reinterpret_cast<const float4*>(row + 4 * HD);
-        w = *reinterpret_cast<const float4*>(a.w_raw + (size_t)(first + t) * HD + h * kDcD + c);
-        const float4 b = *reinterpret_cast<const float4*>(a.a_bias + h * kDcD + c), w0 = *reinterpret_cast<const float4*>(a.w0 + h * kDcD + c);
-        e.x = dc_sigmoid(e.x + b.x); e.y = dc_sigmoid(e.y + b.y); e.z = dc_sigmoid(e.z + b.z); e.w = dc_sigmoid(e.w + b.w);
-        w.x = expf(-kDcFloor * dc_sigmoid(w.x + w0.x)); w.y = expf(-kDcFloor * dc_sigmoid(w.y + w0.y));
-        w.z = expf(-kDcFloor * dc_sigmoid(w.z + w0.z)); w.w = expf(-kDcFloor * dc_sigmoid(w.w + w0.w));
-      }
-      float ss = fmaf(k.x, k.x, fmaf(k.y, k.y, fmaf(k.z, k.z, k.w * k.w)));
-#pragma unroll
-      for (int o = 1; o < 16; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-      const float inv = 1.0f / sqrtf(ss + 1e-6f);
-      const float4 u = make_float4(k.x * inv, k.y * inv, k.z * inv, k.w * inv);
-      e.x *= u.x; e.y *= u.y; e.z *= u.z; e.w *= u.w;
-      bad = bad || !splits(r) || !splits(k) || !splits(v) || !splits(e) || !splits(w) || !isfinite(ss);
-      *reinterpret_cast<float4*>(r_s + t * kDcP + c) = r;
-      *reinterpret_cast<float4*>(k_s + t * kDcP + c) = k;
-      *reinterpret_cast<float4*>(v_s + t * kDcP + c) = v;
-      *reinterpret_cast<float4*>(e_s + t * kDcP + c) = e;
-      *reinterpret_cast<float4*>(u_s + t * kDcP + c) = u;
-      *reinterpret_cast<float4*>(a_s + t * kPitchA + c) = w;
+  struct Rows { float4 r, k, v, e, u, w; };
+  auto token = [&](int piece) { return piece * 32 + (tid >> 4); };         // sixteen neighbouring lanes a token, four channels each
+  const int c = (tid & 15) * 4;
+  auto fetch = [&](int piece, Rows& x) {                                   // true: a number that is not finite
+    const int t = token(piece);
+    x.r = x.k = x.v = x.e = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    x.w = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+    if (t < n) {
+      const float* row = a.proj + (size_t)(first + t) * a.ld + h * kDcD + c;
+      x.r = *reinterpret_cast<const float4*>(row);
+      x.k = *reinterpret_cast<const float4*>(row + HD);
+      x.v = *reinterpret_cast<const float4*>(row + 2 * HD);
+      x.e = *reinterpret_cast<const float4*>(row + 4 * HD);
+      x.w = *reinterpret_cast<const float4*>(a.w_raw + (size_t)(first + t) * HD + h * kDcD + c);
     }
-    return bad;
   };
-  bool bad = __syncthreads_or(load());
+  auto finish = [&](int piece, Rows& x) {
+    if (token(piece) < n) {
+      const float4 b = *reinterpret_cast<const float4*>(a.a_bias + h * kDcD + c), w0 = *reinterpret_cast<const float4*>(a.w0 + h * kDcD + c);
+      x.e.x = dc_sigmoid(x.e.x + b.x); x.e.y = dc_sigmoid(x.e.y + b.y); x.e.z = dc_sigmoid(x.e.z + b.z); x.e.w = dc_sigmoid(x.e.w + b.w);
+      x.w.x = expf(-kDcFloor * dc_sigmoid(x.w.x + w0.x)); x.w.y = expf(-kDcFloor * dc_sigmoid(x.w.y + w0.y));
+      x.w.z = expf(-kDcFloor * dc_sigmoid(x.w.z + w0.z)); x.w.w = expf(-kDcFloor * dc_sigmoid(x.w.w + w0.w));
+    }
+    float ss = fmaf(x.k.x, x.k.x, fmaf(x.k.y, x.k.y, fmaf(x.k.z, x.k.z, x.k.w * x.k.w)));
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float inv = 1.0f / sqrtf(ss + 1e-6f);
+    x.u = make_float4(x.k.x * inv, x.k.y * inv, x.k.z * inv, x.k.w * inv);
+    x.e.x *= x.u.x; x.e.y *= x.u.y; x.e.z *= x.u.z; x.e.w *= x.u.w;
+    return !splits(x.r) || !splits(x.k) || !splits(x.v) || !splits(x.e) || !splits(x.w) || !isfinite(ss);
+  };
   float* out = a.out + (size_t)first * HD + h * kDcD;
   float* reach = a.reach + (size_t)first * HD + h * kDcD;
   float* local = a.local + item * kDcD * kDcD;
   uint32_t* trans = a.trans + item * kTransWords;
 
   auto walk = [&]() {                                      // token by token: 64 columns of values, 64 of the unit matrix
+    using W = DeltaWalkLayout;
+    float* f = reinterpret_cast<float*>(smem);
+    __syncthreads();                                       // (what lies there has been read)
+#pragma unroll 1
+    for (int piece = 0; piece < 2; ++piece) {
+      Rows x;
+      fetch(piece, x);
+      finish(piece, x);
+      const int t = token(piece);
+      *reinterpret_cast<float4*>(f + W::R + t * kDcP + c) = x.r;
+      *reinterpret_cast<float4*>(f + W::K + t * kDcP + c) = x.k;
+      *reinterpret_cast<float4*>(f + W::V + t * kDcP + c) = x.v;
+      *reinterpret_cast<float4*>(f + W::E + t * kDcP + c) = x.e;
+      *reinterpret_cast<float4*>(f + W::U + t * kDcP + c) = x.u;
+      *reinterpret_cast<float4*>(f + W::W + t * kPitchA + c) = x.w;
+    }
+    __syncthreads();
     if (tid < 2 * kDcD) {
       const bool unit = tid >= kDcD;
       const int j = tid & (kDcD - 1);
@@ -190,19 +176,19 @@ __global__ void __launch_bounds__(kDcThreads, 2) delta_local_kernel(const DeltaC
 #pragma unroll 1
       for (int t = 0; t < n; ++t) {
         float x = 0.0f, kept = 0.0f, c1 = 0.0f, c2 = 0.0f;  // the output from the state in front of the token, as delta_scan_kernel takes it
-        const float v = unit ? 0.0f : v_s[t * kDcP + j];
+        const float v = unit ? 0.0f : f[W::V + t * kDcP + j];
 #pragma unroll 1
         for (int i = 0; i < kDcD; ++i) {
-          const float r = r_s[t * kDcP + i];
-          x = fmaf(u_s[t * kDcP + i], S[i], x);
-          kept = fmaf(r * a_s[t * kPitchA + i], S[i], kept);
-          c1 = fmaf(r, e_s[t * kDcP + i], c1);
-          c2 = fmaf(r, k_s[t * kDcP + i], c2);
+          const float r = f[W::R + t * kDcP + i];
+          x = fmaf(f[W::U + t * kDcP + i], S[i], x);
+          kept = fmaf(r * f[W::W + t * kPitchA + i], S[i], kept);
+          c1 = fmaf(r, f[W::E + t * kDcP + i], c1);
+          c2 = fmaf(r, f[W::K + t * kDcP + i], c2);
         }
 #pragma unroll 1
         for (int i = 0; i < kDcD; ++i) {
-          const float w = a_s[t * kPitchA + i] * S[i];
-          S[i] = fmaf(-e_s[t * kDcP + i], x, unit ? w : fmaf(k_s[t * kDcP + i], v, w));
+          const float w = f[W::W + t * kPitchA + i] * S[i];
+          S[i] = fmaf(-f[W::E + t * kDcP + i], x, unit ? w : fmaf(f[W::K + t * kDcP + i], v, w));
         }
         const float o = fmaf(-c1, x, unit ? kept : fmaf(c2, v, kept));
         (unit ? reach : out)[(size_t)t * HD + j] = o;
@@ -222,191 +208,277 @@ __global__ void __launch_bounds__(kDcThreads, 2) delta_local_kernel(const DeltaC
     }
     if (tid == 0) a.bad[item] = 1;
   };
-  if (bad) {
-    walk();
-    return;
-  }
 
-  // ---------------------------------------------------------- decays from the middle: a_s then holds G_t / G_31 for t > 31, its reciprocal up to there
-  if (tid < 2 * kDcD) {
-    const int c = tid & (kDcD - 1);
-    Product p;
-    if (tid < kDcD) {
-      float w = a_s[31 * kPitchA + c];
-      a_s[31 * kPitchA + c] = 1.0f;
-#pragma unroll 8
-      for (int t = 30; t >= 0; --t) {
-        p.times(w);
-        w = a_s[t * kPitchA + c];
-        a_s[t * kPitchA + c] = p.value();
+  bool ok = true;
+  auto fast = [&]() -> bool {                              // false: to be walked
+    uint32_t largest = 0;                                  // of what is made here to be cut
+    auto note = [&](float x) { largest = max(largest, magnitude(x)); };
+    {
+      Rows x[2];
+      bool bad = false;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) fetch(i, x[i]);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        bad = finish(i, x[i]) || bad;
+        *reinterpret_cast<float4*>(w_s + token(i) * L::P + c) = x[i].w;
       }
-      p.times(w);
-      mid[c] = p.value();                                  // from the stretch's beginning to the middle
+      if (__syncthreads_or(bad)) return false;
+      // decays from the middle: w_s then holds G_t / G_31 for t > 31, its reciprocal up to there
+      if (tid < 2 * kDcD) {
+        const int ch = tid & (kDcD - 1);
+        Product p;
+        if (tid < kDcD) {
+          float w = w_s[31 * L::P + ch];
+          w_s[31 * L::P + ch] = 1.0f;
+#pragma unroll 8
+          for (int t = 30; t >= 0; --t) {
+            p.times(w);
+            w = w_s[t * L::P + ch];
+            w_s[t * L::P + ch] = p.value();
+          }
+          p.times(w);
+          mid[ch] = p.value();                             // from the stretch's beginning to the middle
+        } else {
+#pragma unroll 8
+          for (int t = 32; t < kChunk; ++t) {
+            p.times(w_s[t * L::P + ch]);
+            w_s[t * L::P + ch] = p.value();
+          }
+          end[ch] = p.value();
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int t = token(i);
+        const float4 p = *reinterpret_cast<const float4*>(w_s + t * L::P + c), q = make_float4(1.0f / p.x, 1.0f / p.y, 1.0f / p.z, 1.0f / p.w);
+        const bool late = t > 31;
+        const float4 f = late ? p : q, back = late ? q : p;
+        const float4 b4 = *reinterpret_cast<const float4*>((t == 0 ? mid : w_s + (t - 1) * L::P) + c);
+        const float4 before = t > 32 ? b4 : make_float4(1.0f / b4.x, 1.0f / b4.y, 1.0f / b4.z, 1.0f / b4.w);
+        auto times = [&](float4& y, const float4& g) {
+          y.x *= g.x; y.y *= g.y; y.z *= g.z; y.w *= g.w;
+          largest = tc_largest(largest, y);
+        };
+        times(x[i].r, f);
+        times(x[i].u, before);
+        times(x[i].k, back);
+        times(x[i].e, back);
+        largest = tc_largest(largest, x[i].v);
+        *reinterpret_cast<float4*>(u32 + t * L::P + c) = x[i].u;
+        *reinterpret_cast<float4*>(r32 + t * L::P + c) = x[i].r;
+        tc_put<128, 64>(smem + L::UR, t, c, x[i].u);
+        tc_put<128, 64>(smem + L::UR, 64 + t, c, x[i].r);
+        tc_put<128, 64>(smem + L::KE, t, c, x[i].k);
+        tc_put<128, 64>(smem + L::KE, 64 + t, c, x[i].e);
+        tc_put<64, 64>(smem + L::V, t, c, x[i].v);
+      }
+    }
+    fence_proxy_async_smem();
+    if (__syncthreads_or(largest >= kTcCut)) return false;
+    tc_after();
+    const uint32_t tmem = tmem_holder, lanes = (uint32_t)((warp & 3) * 32) << 16;
+    const int row = (warp & 3) * 32 + lane, quarter = warp >> 2, q0 = quarter * 16;
+    const bool lower = row >= kDcD, issuer = warp == 0;    // of the 128 lanes: queries, or key channels
+    const int own = row & (kDcD - 1);
+    uint2 phase = make_uint2(0u, 0u);
+    const uint64_t d_ur = tc_k_major(base + L::UR), d_ke = tc_k_major(base + L::KE), d_b = tc_k_major(base + L::B),
+                   d_v = tc_mn_major(base + L::V, 64 * 128), d_keys = tc_mn_major(base + L::KE, 128 * 128);
+    constexpr uint32_t kWide = 128 * 128, kNarrow = 64 * 128;                // a part of a tile of 128 or 64 rows
+    auto ss = [&](int cols, int a_mn, int b_mn) {
+      return [=](uint32_t d, uint64_t x, uint64_t y, uint32_t on, uint32_t elected) { umma_ss(d, x, y, tc_idesc(cols, a_mn, b_mn), on, elected); };
+    };
+    auto nothing = [] {};
+    float made[32] = {};
+    ok = tc_product<128, 4, 4, 64>(made, tmem, lanes + q0, bar, phase, issuer, [&](int p, int ks) { return d_ur + ((p * kWide + ks * 32) >> 4); },
+                                   [&](int p, int ks) { return d_ke + ((p * kWide + ks * 32) >> 4); }, ss(128, 0, 0), false, nothing) && ok;
+    tc_add_small<64>(made, tmem, lanes + q0);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const bool counts = lower ? q0 + i <= own : q0 + i < own;
+      made[i] = counts ? made[i] : 0.0f;                   // N, A
+      made[16 + i] = counts ? made[16 + i] : 0.0f;         // M, B
+      note(made[i]);
+      note(made[16 + i]);
+    }
+    auto put_row = [&](unsigned char* tile, uint32_t part, int at_row, const float* v) {      // 16 numbers of a row from column q0
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const Cut c0(v[8 * j], v[8 * j + 1]), c1(v[8 * j + 2], v[8 * j + 3]), c2(v[8 * j + 4], v[8 * j + 5]), c3(v[8 * j + 6], v[8 * j + 7]);
+        unsigned char* to = tile + at_row * 128 + (((quarter * 2 + j) ^ (at_row & 7)) << 4);
+#pragma unroll
+        for (int p = 0; p < 3; ++p) *reinterpret_cast<uint4*>(to + p * part) = make_uint4(c0.part[p], c1.part[p], c2.part[p], c3.part[p]);
+      }
+    };
+    put_row(smem + L::NA, kWide, row, made);
+    if (lower) {
+      put_row(smem + L::B, kNarrow, own, made + 16);
     } else {
-#pragma unroll 8
-      for (int t = 32; t < kChunk; ++t) {
-        p.times(a_s[t * kPitchA + c]);
-        a_s[t * kPitchA + c] = p.value();
-      }
-      end[c] = p.value();
-    }
-  }
-  __syncthreads();
-  uint32_t largest = 0;                                    // of what is made here to be split
-  auto note = [&](float x) { largest = max(largest, magnitude(x)); };
-#pragma unroll 4
-  for (int e8 = 0; e8 < kChunk * kDcD / kDcThreads; ++e8) {
-    const int e = e8 * kDcThreads + tid, t = e >> 6, c = e & 63;
-    const float p = a_s[t * kPitchA + c], q = 1.0f / p, f = t > 31 ? p : q, back = t > 31 ? q : p;
-    const float before = t == 0 ? 1.0f / mid[c] : (t > 32 ? a_s[(t - 1) * kPitchA + c] : 1.0f / a_s[(t - 1) * kPitchA + c]);
-    r_s[t * kDcP + c] *= f;
-    u_s[t * kDcP + c] *= before;
-    k_s[t * kDcP + c] *= back;
-    e_s[t * kDcP + c] *= back;
-    note(r_s[t * kDcP + c]);
-    note(u_s[t * kDcP + c]);
-    note(k_s[t * kDcP + c]);
-    note(e_s[t * kDcP + c]);
-  }
-  __syncthreads();
-
-  const DcTile w(warp);
-  const int lr = lane >> 2, lc = w.c + 2 * (lane & 3);              // a product's numbers: rows + lr and + lr + 8, columns lc + 8 j, + 1
-  auto lower = [&](const float* rows, const float* cols, bool strict) {   // a_s = the lower triangle of rows . cols^T
-    DcAcc acc = {};
-    dc_pairs(acc, rows, cols, w, lane);
+      put_row(smem + L::MP, kNarrow, own, made + 16);
+      if (quarter == own >> 4) {
 #pragma unroll
-    for (int b = 0; b < 2; ++b) {
-      if (w.c > w.row(b)) continue;
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int t = w.row(b) + lr + (i >> 1) * 8, s = lc + j * 8 + (i & 1);
-          const float x = (strict ? s < t : s <= t) ? acc[b][j][i] : 0.0f;
-          a_s[t * kPitchA + s] = x;
-          note(x);
-        }
-    }
-  };
-  float* x_s = v_s;                                        // X takes the values' place once they have been used
-  DcAcc kv = {}, o = {};
-  {
-    DcAcc nv = {};
-    dc_over_tokens(kv, v_s, k_s, w, lane);                 // [v, k]
-    lower(u_s, k_s, true);                                 // N
-    __syncthreads();
-    dc_times(nv, a_s, v_s, w, lane);
-    __syncthreads();
-    lower(r_s, k_s, false);                                // A
-    __syncthreads();
-    dc_times(o, a_s, v_s, w, lane);
-    __syncthreads();
-#pragma unroll
-    for (int b = 0; b < 2; ++b)
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) x_s[(w.row(b) + lr + (i >> 1) * 8) * kDcP + lc + j * 8 + (i & 1)] = nv[b][j][i];
-  }
-  lower(u_s, e_s, true);                                   // M
-  __syncthreads();
-  for (int e = tid; e < kChunk * kDcD; e += kDcThreads) u_s[(e >> 6) * kDcP + (e & 63)] *= mid[e & 63];     // U, counted from the beginning
-  __syncthreads();
-  for (int i = 0; i < 4; ++i) {                            // [x_s | u_s] <- (1 + M)^-1 [x_s | u_s], 16 rows at a time
-    if (tid < 2 * kDcD) {
-      float* col = (tid < kDcD ? x_s : u_s) + i * 16 * kDcP + (tid & (kDcD - 1));
-      const float* m = a_s + i * 16 * kPitchA + i * 16;
-      float x[16];
-#pragma unroll
-      for (int r = 0; r < 16; ++r) x[r] = col[r * kDcP];
-      note(x[0]);
-#pragma unroll
-      for (int r = 1; r < 16; ++r) {
-#pragma unroll
-        for (int q = 0; q < r; ++q) x[r] = fmaf(-m[r * kPitchA + q], x[q], x[r]);
-        col[r * kDcP] = x[r];
-        note(x[r]);
+        for (int i = 0; i < 16; ++i)                       // what lies within 16 tokens in float32, by columns from the diagonal on
+          if (q0 + i < own) m_s[(q0 + i) * L::P + own - (q0 + i) - 1] = made[16 + i];
       }
     }
-    __syncthreads();
-    const int c = warp * 16;                               // what these rows take off the ones below, 16 of the 128 columns a warp
-    float* tile = (c < kDcD ? x_s : u_s) + (c & (kDcD - 1));
-    if (i < 3) {
-      FragA fa;
-      FragB fb[2];
+    fence_proxy_async_smem();
+    tc_before();
+    if (__syncthreads_or(largest >= kTcCut || !ok)) return false;
 #pragma unroll
-      for (int x = 0; x < 2; ++x) load_b_columns(fb[x], tile + i * 16 * kDcP + x * 8, kDcP, lane);
-      for (int j = i + 1; j < 4; ++j) {
-        load_a_single(fa, a_s + j * 16 * kPitchA + i * 16, kPitchA, lane);
+    for (int i = 0; i < 32; ++i) made[i] = 0.0f;
+    ok = tc_product<128, 4, 4, 64>(made, tmem, lanes + q0, bar, phase, issuer, [&](int p, int ks) { return d_v + ((p * kNarrow + ks * 2048) >> 4); },
+                                   [&](int p, int ks) { return d_ur + ((p * kWide + ks * 32) >> 4); }, ss(128, 1, 0), false, nothing) && ok;
+    tc_add_small<64>(made, tmem, lanes + q0);
+    if (!lower) {
 #pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          float acc[4] = {};
-          mma_split(acc, fa, fb[x]);
-#pragma unroll
-          for (int q = 0; q < 4; ++q) tile[(j * 16 + lr + (q >> 1) * 8) * kDcP + x * 8 + 2 * (lane & 3) + (q & 1)] -= acc[q];
-        }
-      }
+      for (int i = 0; i < 16; ++i) x_s[(q0 + i) * L::P + own] = made[i];
     }
-    __syncthreads();
-  }
-  lower(r_s, e_s, false);                                  // B
-  if (__syncthreads_or(largest >= kSplitLimit)) {
-    load();
-    __syncthreads();
-    walk();
-    return;
-  }
-  {
-    DcAcc bx = {}, bu = {};
-    dc_times(bx, a_s, x_s, w, lane);
-    dc_times(bu, a_s, u_s, w, lane);
+    float o[16], kv[16] = {};
 #pragma unroll
-    for (int b = 0; b < 2; ++b)
+    for (int i = 0; i < 16; ++i) o[i] = made[16 + i];
+    if (__syncthreads_or(!ok)) return false;
+    constexpr uint32_t kAt = 96, kTake = kAt + 5 * 64;      // behind the parts of [X | U]^T; what solved tokens take off others
+    bool taken = true;
+    ok = tc_product<64, 4, 5>(kv, tmem + kAt, lanes + q0, bar, phase, issuer, [&](int p, int ks) { return d_v + ((p * kNarrow + ks * 2048) >> 4); },
+                              [&](int p, int ks) { return d_keys + ((p * kWide + ks * 2048) >> 4); }, ss(64, 1, 1), false, [&] {
+      if (tid >= 2 * kDcD) return;
+      // Sixteen tokens at a time in float32; what they take off those behind them is a product with 48 rows of M (beyond the last token:
+      // whatever lies there, for columns that nobody looks at), and the others move up.  (All in float32, one by one: 11,000 cycles, and
+      // 33,000 written out, which does not fit the instruction cache.)
+      float x[kChunk];
+      const float* column = (lower ? u32 : x_s) + own;
+      const float f = lower ? mid[own] : 1.0f;             // U, counted from the beginning
 #pragma unroll
-      for (int j = 0; j < 2; ++j)
+      for (int t = 0; t < kChunk; ++t) x[t] = column[t * L::P] * f;
+      const uint64_t d_m = tc_k_major(base + L::MP);
+#pragma unroll 1
+      for (int s = 0; s < 4; ++s) {
+        const float* m = m_s + s * 16 * L::P;
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          const int t = w.row(b) + lr + half * 8, c = lc + j * 8;
-          if (t < n) {
-            *reinterpret_cast<float2*>(out + (size_t)t * HD + c) =
-                make_float2(o[b][j][2 * half] - bx[b][j][2 * half], o[b][j][2 * half + 1] - bx[b][j][2 * half + 1]);
-            *reinterpret_cast<float2*>(reach + (size_t)t * HD + c) =
-                make_float2(fmaf(r_s[t * kDcP + c], mid[c], -bu[b][j][2 * half]), fmaf(r_s[t * kDcP + c + 1], mid[c + 1], -bu[b][j][2 * half + 1]));
+        for (int q = 0; q < 15; ++q) {
+#pragma unroll
+          for (int j = 0; j < 15 - q; j += 4) {
+            const float4 m4 = *reinterpret_cast<const float4*>(m + q * L::P + j);
+            x[q + 1 + j] = fmaf(-m4.x, x[q], x[q + 1 + j]);
+            if (q + 2 + j < 16) x[q + 2 + j] = fmaf(-m4.y, x[q], x[q + 2 + j]);
+            if (q + 3 + j < 16) x[q + 3 + j] = fmaf(-m4.z, x[q], x[q + 3 + j]);
+            if (q + 4 + j < 16) x[q + 4 + j] = fmaf(-m4.w, x[q], x[q + 4 + j]);
           }
         }
-  }
-  {
-    DcAcc ex = {}, eu = {};
-    dc_over_tokens(ex, x_s, e_s, w, lane);                 // [v, k]
-    dc_over_tokens(eu, e_s, u_s, w, lane);                 // [k, k]
-    bool lost = false;
+        uint32_t pairs[3][8];
 #pragma unroll
-    for (int b = 0; b < 2; ++b) {
+        for (int i = 0; i < 8; ++i) {
+          note(x[2 * i]);
+          note(x[2 * i + 1]);
+          const Cut cut(x[2 * i], x[2 * i + 1]);
 #pragma unroll
-      for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          const int row = w.row(b) + lr + half * 8, c = lc + j * 8;
-          *reinterpret_cast<float2*>(local + row * kDcD + c) = make_float2((kv[b][j][2 * half] - ex[b][j][2 * half]) * end[c],
-                                                                           (kv[b][j][2 * half + 1] - ex[b][j][2 * half + 1]) * end[c + 1]);
-          const float f = end[row], g = f * mid[row];
-          eu[b][j][2 * half] = (row == c ? g : 0.0f) - f * eu[b][j][2 * half];
-          eu[b][j][2 * half + 1] = (row == c + 1 ? g : 0.0f) - f * eu[b][j][2 * half + 1];
-          lost = lost || !splits(eu[b][j][2 * half]) || !splits(eu[b][j][2 * half + 1]);
+          for (int p = 0; p < 3; ++p) pairs[p][i] = cut.part[p];
         }
-      Split x[4];
-      x[0].set(eu[b][0][0], eu[b][1][0]);
-      x[1].set(eu[b][0][2], eu[b][1][2]);
-      x[2].set(eu[b][0][1], eu[b][1][1]);
-      x[3].set(eu[b][0][3], eu[b][1][3]);
-      uint32_t* to = trans + trans_word(w.row(b) >> 4, w.c >> 4, 0, lane);
-      *reinterpret_cast<uint4*>(to) = make_uint4(x[0].hi, x[1].hi, x[2].hi, x[3].hi);
-      *reinterpret_cast<uint4*>(to + 128) = make_uint4(x[0].mid, x[1].mid, x[2].mid, x[3].mid);
-      *reinterpret_cast<uint4*>(to + 256) = make_uint4(x[0].lo, x[1].lo, x[2].lo, x[3].lo);
+#pragma unroll
+        for (int p = 0; p < 3; ++p) tc_st8(tmem + lanes + p * 32 + s * 8, pairs[p]);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        if (s == 3) break;
+        tc_before();
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (issuer) {
+          tc_after();
+          const uint32_t elected = elect_one();
+          constexpr int PX[6] = {0, 2, 0, 1, 1, 0}, PY[6] = {0, 0, 2, 1, 0, 1};
+#pragma unroll
+          for (int i = 0; i < 6; ++i)
+            umma_ts(tmem + (i == 0 ? kTake : kTake + 48), tmem + PX[i] * 32 + s * 8,
+                    d_m + ((PY[i] * kNarrow + (s + 1) * 2048 + s * 32) >> 4), tc_idesc(48, 0, 0), i > 1 ? 1u : 0u, elected);
+          umma_commit(bar + 16, elected);
+          __syncwarp();
+        }
+        taken = __all_sync(0xffffffffu, mbar_wait(bar + 16, s & 1)) && taken;
+        tc_after();
+#pragma unroll
+        for (int j = 0; j < 48; j += 8) {
+          float big[8], small[8];
+          tc_ld8(tmem + lanes + kTake + j, big);
+          tc_ld8(tmem + lanes + kTake + 48 + j, small);
+          tc_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 8; ++i) x[j + i] = x[j + i + 16] - (big[i] + small[i]);
+        }
+      }
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    }) && ok;
+    ok = ok && taken;
+    tc_add_small(kv, tmem + kAt, lanes + q0);
+    if (__syncthreads_or(largest >= kTcCut || !ok)) return false;
+    auto ts = [&](int b_mn) {
+      return [=](uint32_t d, uint32_t x, uint64_t y, uint32_t on, uint32_t elected) { umma_ts(d, x, y, tc_idesc(64, 0, b_mn), on, elected); };
+    };
+    auto x_u = [&](int p, int ks) { return tmem + p * 32 + ks * 8; };
+    float b[16] = {}, e[16] = {};
+    ok = tc_product<64, 4, 5>(b, tmem + kAt, lanes + q0, bar, phase, issuer, x_u, [&](int p, int ks) { return d_b + ((p * kNarrow + ks * 32) >> 4); },
+                              ts(0), false, nothing) && ok;
+    tc_add_small(b, tmem + kAt, lanes + q0);
+    __syncthreads();                                       // the accumulators are free again
+    ok = tc_product<64, 4, 5>(e, tmem + kAt, lanes + q0, bar, phase, issuer, x_u,
+                              [&](int p, int ks) { return d_keys + ((kNarrow + p * kWide + ks * 2048) >> 4); }, ts(1), false, [&] {
+      const float f = mid[own];
+      float* to = (lower ? reach : out) + (size_t)q0 * HD + own;
+      const float* r = r32 + q0 * L::P + own;
+#pragma unroll
+      for (int i = 0; i < 16; ++i, to += HD)
+        if (q0 + i < n) *to = lower ? fmaf(r[i * L::P], f, -b[i]) : o[i] - b[i];
+    }) && ok;
+    tc_add_small(e, tmem + kAt, lanes + q0);
+    bool lost = false;
+    if (!lower) {
+#pragma unroll
+      for (int i = 0; i < 16; i += 4) {
+        const float4 f = *reinterpret_cast<const float4*>(end + q0 + i);
+        *reinterpret_cast<float4*>(local + own * kDcD + q0 + i) =
+            make_float4((kv[i] - e[i]) * f.x, (kv[i + 1] - e[i + 1]) * f.y, (kv[i + 2] - e[i + 2]) * f.z, (kv[i + 3] - e[i + 3]) * f.w);
+      }
+    } else {
+      // numbers (row q0 + i, column own) of the matrix; words hold two columns eight apart, and two rows eight apart are neighbours: a lane
+      // takes four pairs of rows of its column and the one eight away
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const float f = end[q0 + i];
+        e[i] = (q0 + i == own ? f * mid[own] : 0.0f) - f * e[i];
+        lost = lost || !splits(e[i]);
+      }
+      const bool second = lane & 8;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        // the first lane of a pair keeps rows 0 .. 3 and 8 .. 11, the second one the others
+        const float give_lo = second ? e[i] : e[i + 4], give_hi = second ? e[i + 8] : e[i + 12];
+        const float got_lo = __shfl_xor_sync(0xffffffffu, give_lo, 8), got_hi = __shfl_xor_sync(0xffffffffu, give_hi, 8);
+        const int r = i + (second ? 4 : 0);
+        Split lo, hi;
+        lo.set(second ? got_lo : e[i], second ? e[i + 4] : got_lo);
+        hi.set(second ? got_hi : e[i + 8], second ? e[i + 12] : got_hi);
+        uint32_t* to = trans + trans_word(quarter, own >> 4, 0, r * 4 + ((own & 7) >> 1)) + (own & 1) * 2;
+        *reinterpret_cast<uint2*>(to) = make_uint2(lo.hi, hi.hi);
+        *reinterpret_cast<uint2*>(to + 128) = make_uint2(lo.mid, hi.mid);
+        *reinterpret_cast<uint2*>(to + 256) = make_uint2(lo.lo, hi.lo);
+      }
     }
     lost = __syncthreads_or(lost);
     if (tid == 0) a.bad[item] = lost;
+    return true;
+  };
+  if (!fast()) {
+    if (__syncthreads_or(!ok)) {
+      if (tid == 0) atomicExch(error_flag, 83);
+    } else {
+      walk();
+    }
+  } else if (!ok && lane == 0) {
+    atomicExch(error_flag, 83);
+  }
+  tc_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_holder), "r"(512) : "memory");
   }
 }
 
@@ -535,7 +607,7 @@ long long ifx_delta_chunks_scratch_floats(int num_tokens, int requests, int min_
 int ifx_delta_chunks_scan(const float* proj, int ld, const float* w_raw, const float* w0, const float* a_bias, const float* norm_w,
                           float eps, float* state, long long slot_stride, const int* cu_seqlens, const int* req_slot, float* scratch,
                           void* y, int num_requests, int num_tokens, int min_span, int heads, int dim, int out_dtype, float* scan_scratch,
-                          cudaStream_t stream) {
+                          int* error_flag, cudaStream_t stream) {
   if (num_tokens <= 0 || num_requests <= 0) return 0;
   if (!ifx_delta_chunks_supports(num_requests, heads, dim) || ld < 5 * heads * dim || slot_stride < (long long)heads * dim * dim ||
       scratch == nullptr || min_span < 1 || min_span > num_tokens)
@@ -552,14 +624,14 @@ int ifx_delta_chunks_scan(const float* proj, int ld, const float* w_raw, const f
   a.bad = reinterpret_cast<int*>(a.trans + items * kTransWords);
   a.reach = reinterpret_cast<float*>(a.bad + (items + 3) / 4 * 4);
   a.out = a.reach + rows;
-  cudaError_t e = cudaFuncSetAttribute(delta_local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DeltaChunkLayout::BYTES);
+  cudaError_t e = cudaFuncSetAttribute(delta_local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DeltaLayout::SMEM);
   if (e != cudaSuccess) return (int)e;
   if (scan_scratch != nullptr) {
     const int rc = launch_delta_scan(proj, ld, w_raw, w0, a_bias, state, slot_stride, cu_seqlens, req_slot, scan_scratch, a.out, num_requests,
                                      num_tokens, heads, dim, min_span - 1, stream);
     if (rc) return rc;
   }
-  delta_local_kernel<<<dim3(chunks, heads), kDcThreads, DeltaChunkLayout::BYTES, stream>>>(a);
+  delta_local_kernel<<<dim3(chunks, heads), kDcThreads, DeltaLayout::SMEM, stream>>>(a, error_flag);
   IFX_CHECK_LAUNCH();
   delta_carry_kernel<<<dim3(num_requests, heads, kDcD / kCarryV), kCarryThreads, 0, stream>>>(a);
   IFX_CHECK_LAUNCH();

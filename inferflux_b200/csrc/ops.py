@@ -1652,7 +1652,7 @@ class CudaKernels:
             rc = self.lib.ifx_delta_chunks_scan(
                 proj, proj.shape[1], w_raw, w0, a_bias, norm_w, float(eps), state,
                 state.stride(0), ctx.cu_seqlens, ctx.req_slot, room, y, ctx.num_requests, T,
-                least, heads, dim, _DT[out_dtype], scan_room, _stream())
+                least, heads, dim, _DT[out_dtype], scan_room, self.error_flag, _stream())
             if rc != _MISALIGNED:
                 _check(rc, "delta_rule_scan (stretches)")
                 self.launches += 6 if short else 4
