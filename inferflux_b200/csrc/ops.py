@@ -1608,25 +1608,26 @@ class CudaKernels:
     def delta_stretches_pay(cls, heads, tokens, requests, longest, short, short_tokens, short_spans, short_stretches, stretches):
         """A stretch of the delta rule does several times a token's work of the scan; what is gained is that the tokens of one span run
         side by side, so this compares what the ways take: the scan for all, stretches for all, stretches for the long spans beside
-        the scan for the others.  us, fitted to what follows within a tenth: the scan walks its longest span at 0.3 a token and more
-        with more columns at once; the stretches go in rounds of 148 blocks (a head's stretch each).
-        us, 24 heads of 64, the scan alone and the stretches (beside the scan): 128 tokens 47 / 48; 256 87 / 53; 512 165 / 96; 2,048
-        659 / 304; two of 256 99 / 92; four of 256 128 / 139; four of 512 262 / 277; eight of 512 377 / 509; with 31 of one 128 68 / 72,
-        256 115 / 81, 512 211 / 129; with 63 of one 512 225 / 144; 256 and 100 106 / 102; 512, 100, 80 and 29 of one 222 / 176.
-        56 heads: 192 82 / 90; 256 105 / 93; 2,048 841 / 608; four of 256 267 / 320; with 31 of one 512 280 / 249."""
+        the scan for the others.  us, fitted to what follows within a sixth: the scan walks its longest span at 0.3 a token and more
+        with more columns at once; the stretches go in rounds of 148 blocks (a head's stretch each), and every block walks the requests.
+        us, 24 heads of 64, the scan alone and the stretches (beside the scan): 128 tokens 46 / 31; 256 86 / 34; 512 164 / 59; 2,048
+        656 / 189; two of 256 98 / 60; four of 256 126 / 91; four of 512 259 / 185; eight of 512 365 / 333; eight of 128 92 / 98; sixteen of
+        150 223 / 254; with 31 of one 128 67 / 178 (57), 512 212 / 214 (87); with 63 of one 512 227 / 452 (110); 256 and 100 94 / 39 (80);
+        512, 100, 80 and 29 of one 211 / 85 (112).  56 heads: 128 56 / 37; 256 104 / 61; 2,048 830 / 386; four of 256 263 / 213; four of
+        512 513 / 384; with 31 of one 512 296 / 540 (180)."""
         def scan(longest, tokens, requests):
             columns = tokens * heads / longest             # heads at work at once, on average
             return longest * max(0.3 + 0.0019 * columns, columns / 275) + 0.018 * requests * heads
 
         def chunks(blocks):
-            return 37 * -(-blocks // 148) + 1.5 * (longest / 64) + 0.055 * blocks + 8
+            return 20.6 * -(-blocks // 148) + 0.6 * (longest / 64) + 0.07 * blocks + 4 + 1.5 * max(0, requests - 4)
         least, alone = 1, 6 + scan(longest, tokens, requests - 1)
         best = chunks((stretches + short_stretches) * heads)
         if short:
             beside = chunks(stretches * heads) + 10 + scan(short, short_tokens, short_spans)
             if beside < best:
                 least, best = cls.CHUNK_SCAN_MIN_SPAN, beside
-        return 1.1 * best < alone and (least, short if least > 1 else 0)
+        return best < alone and (least, short if least > 1 else 0)
 
     def delta_rule_scan(self, proj, w_raw, w0, a_bias, norm_w, eps, heads, dim, state, ctx, out_dtype):
         """The recurrence of csrc/delta_rule.cu over every request's tokens.  `proj`: float32 [T, 5 heads dim], the
