@@ -519,22 +519,37 @@ __global__ void __launch_bounds__(256) prefill_merge_kernel(const int* __restric
   const int* tile = tiles + (size_t)(num_tiles - 1 - block / nq) * 4;
   if (row >= tile[2]) return;
   const size_t at = (size_t)blockIdx.x * split.parts * 2 * kBM + row;
-  float m = -INFINITY, l = 0.0f;
-  for (int p = 0; p < split.parts; ++p) m = fmaxf(m, split.ml[at + (size_t)p * 2 * kBM].x);
+  // a lane a part's reference and sum (16 parts at most); then the parts' rows, four on their way at a time, added in order
+  float2 mine = make_float2(-INFINITY, 0.0f);
+  if (lane < split.parts) mine = split.ml[at + (size_t)lane * 2 * kBM];
+  const float m = warp_max(mine.x);
+  // a part without a key: its sums were not written (weight 0, and the row is not read)
+  const bool there = lane < split.parts && !(mine.x == -INFINITY && !isnan(mine.y));
+  const float w_mine = !there ? 0.0f : mine.x == -INFINITY ? 1.0f : exp2f(mine.x - m);
+  const unsigned parts = __ballot_sync(0xffffffffu, there);
+  float l = 0.0f;
   float acc[D / 32];
 #pragma unroll
   for (int j = 0; j < D / 32; ++j) acc[j] = 0.0f;
-  for (int p = 0; p < split.parts; ++p) {
-    const float2 ml = split.ml[at + (size_t)p * 2 * kBM];
-    if (ml.x == -INFINITY && !isnan(ml.y)) continue;       // no key of this part: its sums were not written
-    const float w = ml.x == -INFINITY ? 1.0f : exp2f(ml.x - m);
-    l = fmaf(ml.y, w, l);
-    const float* o = split.o + (at + (size_t)p * 2 * kBM) * D + lane * (D / 32);
+  for (int p0 = 0; p0 < split.parts; p0 += 4) {
+    float2 v[4][D / 64];
 #pragma unroll
-    for (int j = 0; j < D / 32; j += 2) {
-      const float2 v = *reinterpret_cast<const float2*>(o + j);
-      acc[j] = fmaf(v.x, w, acc[j]);
-      acc[j + 1] = fmaf(v.y, w, acc[j + 1]);
+    for (int k = 0; k < 4; ++k)
+      if (parts >> (p0 + k) & 1) {
+        const float* o = split.o + (at + (size_t)(p0 + k) * 2 * kBM) * D + lane * (D / 32);
+#pragma unroll
+        for (int j = 0; j < D / 64; ++j) v[k][j] = *reinterpret_cast<const float2*>(o + 2 * j);
+      }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float w = __shfl_sync(0xffffffffu, w_mine, (p0 + k) & 31), sum = __shfl_sync(0xffffffffu, mine.y, (p0 + k) & 31);
+      if (!(parts >> (p0 + k) & 1)) continue;
+      l = fmaf(sum, w, l);
+#pragma unroll
+      for (int j = 0; j < D / 64; ++j) {
+        acc[2 * j] = fmaf(v[k][j].x, w, acc[2 * j]);
+        acc[2 * j + 1] = fmaf(v[k][j].y, w, acc[2 * j + 1]);
+      }
     }
   }
   const float inv = l > 0.0f || isnan(l) ? 1.0f / l : 0.0f;
