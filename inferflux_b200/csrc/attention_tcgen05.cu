@@ -1,6 +1,6 @@
 // Attention of prompt portions on the 5th-generation tensor cores.
 //
-// A thread block takes up to 256 query tokens of one query head, as two tiles of 128, and
+// A block of the grid is up to 256 query tokens of one query head, as two tiles of 128; it
 // walks the keys they may see in tiles of 128; both query tiles use each key/value tile that
 // is fetched, which halves the traffic from L2.  Tensor memory holds, per query tile, the
 // scores and the output:
@@ -23,14 +23,25 @@
 //
 // Warp 0 fetches: the query tiles once, then per key tile the pages of K and of V as TMA boxes
 // [16 keys x 64 elements] through the block table, into a ring of slots (a slot holds the keys
-// or the values of one tile).  Warp 1 issues the MMAs.  Warps 2-5 and 6-9 are the softmax groups.
+// or the values of one tile).  Warp 1 issues the MMAs.  Warps 4-7 and 8-11 are the softmax groups, with 208 registers a thread
+// (setmaxnreg), since a row's scores take 128.
 //
-// Bound: the tensor pipe and the exponentials, each busy 43 % of the time a block is resident (a key tile takes a block 2.1 us),
-// waiting for one another at the hand-overs.  A warp in step issues the products, one lane of it by predicate: with a single thread in a
+// A block has an SM to itself.  When its last keys are on their way it takes a block that has not begun off the grid
+// (clusterlaunchcontrol) and goes on with that one: its keys and, once the output rows that lay in their place have left, its queries
+// are fetched while the last tile's softmax and the output are still at work.  A block of its own would begin 5 us later (exit, launch
+// 0.7, barriers, tensor memory, tile, slot, page and keys one after the other 2.7).  A grid of no more than 148 blocks takes none.
+// The output leaves through shared memory in whole rows (a thread's own row, 16 bytes of 32 rows a store, took 2 us a tile).
+//
+// Bound: the tensor pipe: a key tile takes a block 1.87 us at the 1.65 GHz that the SMs keep under it, 1.3 PFLOP/s while a block
+// walks its keys; the rest is heads and tails of blocks.  Blocks behind one another, whole rows of output, registers for the scores
+// and two scores an instruction, us: 2,500 tokens of 28 heads behind 4,000 149 -> 132, behind none 61 -> 52; 2,200 in five prompts
+// 38.7 -> 30.7; 900 of 12 heads behind 1,500 (one round) 20.1 -> 17.3, 447 behind none 16.0 -> 13.8.  A quarter of the
+// exponentials by multiply-adds was slower (149 -> 153), probabilities of the first 96 keys instead of 64 handed over first the same.
+// A warp in step issues the products, one lane of it by predicate: with a single thread in a
 // branch of its own a product took 108 clocks to issue instead of 65 (2,500 tokens behind 4,000, 28 heads: 211 us, then 192).
 // A row's 128 scores stay in registers between the maximum and the exponentials (they were read twice), and the product with the
-// values begins with the first 64 keys' probabilities: 162 -> 151; 900 tokens of 12 heads behind 1,500: 25.1 -> 23.5; 447: 16.9 -> 16.2.
-// A block has an SM to itself, so blocks left over behind whole rounds of 148 cost a round: they are cut into parts of their keys
+// values begins with the first 64 keys' probabilities: 162 -> 151.
+// Blocks left over behind whole rounds of 148 would cost a round: they are cut into parts of their keys
 // that prefill_merge_kernel adds up (192 -> 162; 512 tokens behind 3,000 of 12 heads, where 24 blocks are all there is, 62 -> 30).
 //
 // Keys outside a row's range get weight zero; what the cache holds there is finite (the pool
@@ -86,6 +97,18 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{.reg .b64 a,b,c,d; mov.b64 a,{%2,%3}; mov.b64 b,{%4,%5}; mov.b64 c,{%6,%7}; fma.rn.f32x2 d,a,b,c; mov.b64 {%0,%1},d;}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{.reg .b64 a,b,d; mov.b64 a,{%2,%3}; mov.b64 b,{%4,%5}; add.rn.f32x2 d,a,b; mov.b64 {%0,%1},d;}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
 // The largest of three.
 __device__ __forceinline__ float max3(float x, float y, float z) {
   float m;
@@ -112,7 +135,11 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 constexpr int kSms = 148;                  // blocks of a round: one an SM
 constexpr float kRescaleStep = 8.0f;      // log2 units the maximum may outgrow its reference before O is rescaled
 constexpr uint32_t kTmemCols = 512;       // per query tile: scores (128 columns) and output (head size)
-constexpr int kThreads = 320;             // fetch warp, MMA warp, two softmax groups of four warps
+constexpr int kThreads = 384;             // fetch warp, MMA warp, two that rest, two softmax groups of four warps
+constexpr int kNextSlots = 4;             // answers about the next block that are kept (see next_block)
+// Registers a thread: the launch's 168 x 384 shared out anew, the softmax groups' 256 threads 208 and the others 88.
+constexpr int kRegsSoftmax = 208, kRegsOther = 88;
+static_assert(256 * kRegsSoftmax + 128 * kRegsOther <= 168 * kThreads, "no more than the block was launched with");
 
 template <int D>
 struct PrefillLayout {
@@ -120,9 +147,12 @@ struct PrefillLayout {
   static constexpr int SLOTS = D == 128 ? 5 : 8;              // key or value tiles in flight
   static constexpr uint32_t Q_BYTES = HALVES * kBM * 128;     // one query tile: [half][128 rows][128 B]
   static constexpr uint32_t SLOT_BYTES = HALVES * kBN * 128;  // the keys or the values of one tile
-  static constexpr int B_Q = 0, B_FULL = 1, B_EMPTY = B_FULL + SLOTS, B_S_FULL = B_EMPTY + SLOTS,
-                       B_P_HALF = B_S_FULL + 2, B_P_FULL = B_P_HALF + 2, B_O_FULL = B_P_FULL + 2, B_COUNT = B_O_FULL + 2;
-  static constexpr size_t SMEM = 1024 + 2 * Q_BYTES + (size_t)SLOTS * SLOT_BYTES + B_COUNT * 8 + 16;
+  // barriers: queries there, their place free again, slots there and free, scores, probabilities of the first keys and of all,
+  // output, the next block's number
+  static constexpr int B_Q = 0, B_Q_FREE = B_Q + 2, B_FULL = B_Q_FREE + 2, B_EMPTY = B_FULL + SLOTS, B_S_FULL = B_EMPTY + SLOTS,
+                       B_P_HALF = B_S_FULL + 2, B_P_FULL = B_P_HALF + 2, B_O_FULL = B_P_FULL + 2, B_NEXT = B_O_FULL + 2,
+                       B_COUNT = B_NEXT + kNextSlots;
+  static constexpr size_t SMEM = 1024 + 2 * Q_BYTES + (size_t)SLOTS * SLOT_BYTES + kNextSlots * 16 + B_COUNT * 8 + 16;
 };
 
 // What is left over when whole rounds of blocks, one an SM, have been taken off a grid runs as `parts` blocks each, every one over a
@@ -134,22 +164,96 @@ struct PrefillParts {
   float2* ml;                // [left over x parts][256]: reference in units of log2, sum
 };
 
-// KEPT: the mask has kept first keys (without them the walk over the key tiles is a plain range).
+// A block that has not begun is taken off the grid, and its number written to `answer` (16 bytes of shared memory).
+__device__ __forceinline__ void take_next_block(uint32_t answer, uint32_t bar) {
+  mbar_expect_tx(bar, 16);
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(answer), "r"(bar)
+               : "memory");
+}
+// The number taken, -1 where every block had begun (or, with `ok` false, the answer never came).
+__device__ __forceinline__ int next_block(uint32_t answer, uint32_t bar, uint32_t parity, bool& ok) {
+  ok = __all_sync(0xffffffffu, mbar_wait(bar, parity));
+  if (!ok) return -1;
+  uint32_t there, x;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 a;\n\t"
+      "ld.shared.b128 a, [%2];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, a;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\tmov.u32 %1, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, a;\n\t}"
+      : "=r"(there), "=r"(x)
+      : "r"(answer)
+      : "memory");
+  fence_proxy_async_smem();
+  return there ? (int)x : -1;
+}
+
+// What a block of the grid has to do.  KEPT: the mask has kept first keys (without them the walk over the key tiles is a plain range).
+template <bool KEPT>
+struct PrefillItem {
+  int r, row0, rows, pos0, h, slot;        // request, rows of the step, position of the first; slot < 0: a block with all of its keys
+  int rows_1;                              // rows of query tile 1
+  int tb_0, te_0, tb_1, te_1, te;          // key tiles [tb_q, te_q) of query tile q (rows q * 128 ...); tile 1 may be absent
+  int keep, keep_tiles, nk, tb;
+
+  __device__ __forceinline__ PrefillItem(int block, const int* __restrict__ tiles, int num_tiles, int nq, const KeyMask& window,
+                                         const PrefillParts& split) {
+    // the last items of a prompt see the most keys: they go first; the heads of an item run side by side
+    int part = 0;
+    slot = block - split.full;
+    if (slot >= 0) {
+      block = split.full + slot / split.parts;
+      part = slot % split.parts;
+    }
+    const int* tile = tiles + (size_t)(num_tiles - 1 - block / nq) * 4;
+    r = tile[0], row0 = tile[1], rows = tile[2], pos0 = tile[3];
+    h = block % nq;
+    rows_1 = max(rows - kBM, 0);
+    tb_0 = window.first(pos0) / kBN;
+    te_0 = (pos0 + min(rows, kBM) + kBN - 1) / kBN;
+    tb_1 = window.first(pos0 + kBM) / kBN;
+    te_1 = rows_1 > 0 ? (pos0 + rows + kBN - 1) / kBN : tb_1;
+    if (!KEPT && slot >= 0) {                              // this block's part of the key tiles (tile 0 begins first)
+      const int last = max(te_0, te_1), per = (last - tb_0 + split.parts - 1) / split.parts;
+      const int lo = min(last, tb_0 + part * per), hi = min(last, lo + per);
+      tb_0 = lo;
+      te_0 = max(lo, min(te_0, hi));
+      tb_1 = max(lo, min(tb_1, hi));
+      te_1 = max(tb_1, min(te_1, hi));
+    }
+    te = max(te_0, te_1);
+    // Key tiles are visited in order: with kept keys first [0, nk), then [tb_0, te); query tile q uses those that hold kept keys
+    // and those of its own window.
+    keep = KEPT ? window.keep : 0, keep_tiles = (keep + kBN - 1) / kBN, nk = min(keep_tiles, tb_0);
+    tb = KEPT && nk > 0 ? 0 : tb_0;
+  }
+  __device__ __forceinline__ int next_tile(int kt) const { return KEPT && kt + 1 == nk ? tb_0 : kt + 1; }
+  __device__ __forceinline__ int visited(int kt) const { return KEPT && kt < nk ? kt : kt - tb_0 + nk; }   // tiles that come before kt
+  __device__ __forceinline__ int visits() const { return te - tb_0 + nk; }
+  __device__ __forceinline__ bool active(int q, int kt) const {
+    if (KEPT && kt < keep_tiles && kt < te_0 && (q == 0 || rows_1 > 0)) return true;      // (kept keys lie in front of te_0)
+    return q == 0 ? (kt >= tb_0 && kt < te_0) : (kt >= tb_1 && kt < te_1);
+  }
+  __device__ __forceinline__ bool has(int q) const { return q == 0 || rows_1 > 0; }
+};
+
 template <int D, bool KEPT>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 1)
 attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap pool_map,
                             const int* __restrict__ block_table, const int* __restrict__ tiles,
                             const int* __restrict__ req_slot, bf16* __restrict__ out, int nq, int nkv, int page_size,
                             int page_shift, int max_blocks, int num_pages, KeyMask window, HeadOutput post, float scale_log2,
                             int* __restrict__ error_flag, int num_tiles, PrefillParts split) {
   using L = PrefillLayout<D>;
+  using Item = PrefillItem<KEPT>;
   constexpr int HALVES = L::HALVES, SLOTS = L::SLOTS;
   constexpr uint32_t Q_BYTES = L::Q_BYTES, SLOT_BYTES = L::SLOT_BYTES;
   extern __shared__ unsigned char smem_dyn[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
   const uint32_t q_s = smem_addr(smem);                  // two query tiles
   const uint32_t kv_s = q_s + 2 * Q_BYTES;               // the ring of slots
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 2 * Q_BYTES + SLOTS * SLOT_BYTES);
+  const uint32_t next_s = kv_s + SLOTS * SLOT_BYTES;     // answers about the next block
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 2 * Q_BYTES + SLOTS * SLOT_BYTES + kNextSlots * 16);
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + L::B_COUNT);
   const uint32_t bar0 = smem_addr(bars);
   auto bar = [&](int i) { return bar0 + 8 * i; };
@@ -157,17 +261,19 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
   pdl_launch_dependents();
   if (threadIdx.x == 0) {
-    mbar_init(bar(L::B_Q), 1);
     for (int s = 0; s < SLOTS; ++s) {
       mbar_init(bar(L::B_FULL + s), 1);
       mbar_init(bar(L::B_EMPTY + s), 1);
     }
     for (int q = 0; q < 2; ++q) {
+      mbar_init(bar(L::B_Q + q), 1);
+      mbar_init(bar(L::B_Q_FREE + q), 4);
       mbar_init(bar(L::B_S_FULL + q), 1);
       mbar_init(bar(L::B_P_HALF + q), 4);
       mbar_init(bar(L::B_P_FULL + q), 4);
       mbar_init(bar(L::B_O_FULL + q), 1);
     }
+    for (int s = 0; s < kNextSlots; ++s) mbar_init(bar(L::B_NEXT + s), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -183,291 +289,321 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
   const uint32_t tmem_s = tmem_base, tmem_o = tmem_base + 2 * kBN;       // S of tile q: + q * 128; O: + q * D
   pdl_wait();
 
-  // the last items of a prompt see the most keys: they go first; the heads of an item run side by side
-  int block = blockIdx.x, part = 0;
-  const int slot = block - split.full;                     // < 0: a block with all of its keys
-  if (slot >= 0) {
-    block = split.full + slot / split.parts;
-    part = slot % split.parts;
-  }
-  const int* tile = tiles + (size_t)(num_tiles - 1 - block / nq) * 4;
-  const int r = tile[0], row0 = tile[1], rows = tile[2], pos0 = tile[3];
-  const int h = block % nq;
-  const int g = h / (nq / nkv);
-  // key tiles [tb_q, te_q) of query tile q (rows q * 128 ...); tile 1 may be absent
-  const int rows_1 = max(rows - kBM, 0);
-  int tb_0 = window.first(pos0) / kBN;
-  int te_0 = (pos0 + min(rows, kBM) + kBN - 1) / kBN;
-  int tb_1 = window.first(pos0 + kBM) / kBN;
-  int te_1 = rows_1 > 0 ? (pos0 + rows + kBN - 1) / kBN : tb_1;
-  if (!KEPT && slot >= 0) {                                // this block's part of the key tiles (tile 0 begins first)
-    const int last = max(te_0, te_1), per = (last - tb_0 + split.parts - 1) / split.parts;
-    const int lo = min(last, tb_0 + part * per), hi = min(last, lo + per);
-    tb_0 = lo;
-    te_0 = max(lo, min(te_0, hi));
-    tb_1 = max(lo, min(tb_1, hi));
-    te_1 = max(tb_1, min(te_1, hi));
-  }
-  const int te = max(te_0, te_1);
-  // Key tiles are visited in order: with kept keys first [0, nk), then [tb_0, te); query tile q uses those that hold kept keys
-  // and those of its own window.
-  const int keep = KEPT ? window.keep : 0, keep_tiles = (keep + kBN - 1) / kBN, nk = min(keep_tiles, tb_0);
-  const int tb = KEPT && nk > 0 ? 0 : tb_0;
-  auto next_tile = [&](int kt) { return KEPT && kt + 1 == nk ? tb_0 : kt + 1; };
-  auto visited = [&](int kt) { return KEPT && kt < nk ? kt : kt - tb_0 + nk; };          // how many tiles come before kt
-  auto active = [&](int q, int kt) {
-    if (KEPT && kt < keep_tiles && kt < te_0 && (q == 0 || rows_1 > 0)) return true;      // (kept keys lie in front of te_0)
-    return q == 0 ? (kt >= tb_0 && kt < te_0) : (kt >= tb_1 && kt < te_1);
+  // Every role goes through the same blocks: this one, then those that the fetching warp takes off the grid.
+  auto next_of = [&](int n, bool& ok) {                    // the block behind the n-th
+    return next_block(next_s + (n % kNextSlots) * 16, bar(L::B_NEXT + n % kNextSlots), (n / kNextSlots) & 1, ok);
   };
-  const int kfirst = window.first(pos0), kend = pos0 + rows;
 
-  if (warp == 0) {
-    // ------------------------------------------------------------------ fetching
-    const int* table = block_table + (size_t)req_slot[r] * max_blocks;
-    if (lane == 0) {
-      mbar_expect_tx(bar(L::B_Q), rows_1 > 0 ? 2 * Q_BYTES : Q_BYTES);
-      for (int q = 0; q < (rows_1 > 0 ? 2 : 1); ++q)
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
+    if (warp == 0) {
+      // ---------------------------------------------------------------- fetching
+      bool ok = true;
+      int base = 0;                                         // slots used by the blocks before
+      int loads[2] = {0, 0};                                // of query tile q
+      int issued = 0;                                       // slots filled so far
+      for (int n = 0, block = blockIdx.x; ok && block >= 0; ++n) {
+        const Item it(block, tiles, num_tiles, nq, window, split);
+        const int* table = block_table + (size_t)req_slot[it.r] * max_blocks;
+        const int g = it.h / (nq / nkv);
+        const int kfirst = window.first(it.pos0), kend = it.pos0 + it.rows;
+        // the queries go over the output rows of the block before once those have left
+        auto fetch_queries = [&]() {
+          for (int q = 0; q < 2 && ok; ++q) {
+            if (!it.has(q)) continue;
+            if (loads[q] > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar(L::B_Q_FREE + q), (loads[q] - 1) & 1));
+            if (!ok) break;
+            if (lane == 0) {
+              mbar_expect_tx(bar(L::B_Q + q), Q_BYTES);
 #pragma unroll
-        for (int hh = 0; hh < HALVES; ++hh)
-          tma_load_2d(q_s + q * Q_BYTES + hh * kBM * 128, &q_map, h * D + hh * 64, row0 + q * kBM, bar(L::B_Q));
-    }
-    bool ok = true;
-    int issued = 0;                                       // slots filled so far
-    for (int kt = tb; kt < te && ok; kt = next_tile(kt)) {
-      // lanes 0-7 take one 16-key block each; its page is looked up before the wait for a free slot
-      const int key = kt * kBN + lane * 16;
-      int page = 0, off = 0;
-      // no visible key among the 16: any valid page, its keys get weight zero
-      if (lane < kBN / 16 && key < kend && (key + 16 > kfirst || key < keep)) {
-        page = table[key >> page_shift];
-        if (page < 0 || page >= num_pages) page = 0;
-        off = key & (page_size - 1);
-      }
+              for (int hh = 0; hh < HALVES; ++hh)
+                tma_load_2d(q_s + q * Q_BYTES + hh * kBM * 128, &q_map, it.h * D + hh * 64, it.row0 + q * kBM, bar(L::B_Q + q));
+            }
+            ++loads[q];
+          }
+        };
+        if (it.tb >= it.te) fetch_queries();               // (a part without keys)
+        for (int kt = it.tb; kt < it.te && ok; kt = it.next_tile(kt)) {
+          // lanes 0-7 take one 16-key block each; its page is looked up before the wait for a free slot
+          const int key = kt * kBN + lane * 16;
+          int page = 0, off = 0;
+          // no visible key among the 16: any valid page, its keys get weight zero
+          if (lane < kBN / 16 && key < kend && (key + 16 > kfirst || key < it.keep)) {
+            page = table[key >> page_shift];
+            if (page < 0 || page >= num_pages) page = 0;
+            off = key & (page_size - 1);
+          }
 #pragma unroll 1
-      for (int kv = 0; kv < 2; ++kv) {                     // the keys, then the values
-        const int j = 2 * visited(kt) + kv, s = j % SLOTS;
-        ok = __all_sync(0xffffffffu, mbar_wait(bar(L::B_EMPTY + s), ((j / SLOTS) & 1) ^ 1));
-        if (!ok) break;
-        const uint32_t fb = bar(L::B_FULL + s);
-        if (lane == 0) mbar_expect_tx(fb, SLOT_BYTES);
-        __syncwarp();
-        if (lane < kBN / 16) {
-          const uint32_t dst = kv_s + s * SLOT_BYTES + lane * 2048;
-          const int y = ((page * 2 + kv) * nkv + g) * page_size + off;
+          for (int kv = 0; kv < 2 && ok; ++kv) {             // the keys, then the values
+            if (kt == it.tb && kv == (n > 0 ? 1 : 0)) fetch_queries();     // (behind keys whose slot is free sooner)
+            const int j = base + 2 * it.visited(kt) + kv, s = j % SLOTS;
+            ok = ok && __all_sync(0xffffffffu, mbar_wait(bar(L::B_EMPTY + s), ((j / SLOTS) & 1) ^ 1));
+            if (!ok) break;
+            const uint32_t fb = bar(L::B_FULL + s);
+            if (lane == 0) mbar_expect_tx(fb, SLOT_BYTES);
+            __syncwarp();
+            if (lane < kBN / 16) {
+              const uint32_t dst = kv_s + s * SLOT_BYTES + lane * 2048;
+              const int y = ((page * 2 + kv) * nkv + g) * page_size + off;
 #pragma unroll
-          for (int hh = 0; hh < HALVES; ++hh) tma_load_2d(dst + hh * kBN * 128, &pool_map, hh * 64, y, fb);
+              for (int hh = 0; hh < HALVES; ++hh) tma_load_2d(dst + hh * kBN * 128, &pool_map, hh * 64, y, fb);
+            }
+            issued = j + 1;
+          }
         }
-        issued = j + 1;
+        base += 2 * it.visits();
+        // the next block is taken when this one's last tiles are on their way: late, so that SMs that are done sooner take more
+        block = -1;
+        if (ok) {
+          if (lane == 0) take_next_block(next_s + (n % kNextSlots) * 16, bar(L::B_NEXT + n % kNextSlots));
+          __syncwarp();
+          block = next_of(n, ok);
+        }
       }
-    }
-    if (!ok && lane == 0) {
-      atomicExch(error_flag, 7);
-      for (int j = max(0, issued - SLOTS); j < issued; ++j)        // let the copies in flight land
-        mbar_wait(bar(L::B_FULL + j % SLOTS), (j / SLOTS) & 1);
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------------- MMA issue: the warp in step, one lane's instructions by predicate
-    {
+      if (!ok && lane == 0) {
+        atomicExch(error_flag, 7);
+        for (int j = max(0, issued - SLOTS); j < issued; ++j)        // let the copies in flight land
+          mbar_wait(bar(L::B_FULL + j % SLOTS), (j / SLOTS) & 1);
+        for (int q = 0; q < 2; ++q)
+          if (loads[q] > 0) mbar_wait(bar(L::B_Q + q), (loads[q] - 1) & 1);
+      }
+    } else if (warp == 1) {
+      // ----------------------------------------------------- MMA issue: the warp in step, one lane's instructions by predicate
       const uint32_t elected = elect_one();
       const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kBN >> 3) << 17) |
                                ((uint32_t)(kBM >> 4) << 24);                       // both operands K-major
       const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(D >> 3) << 17) |
                                ((uint32_t)(kBM >> 4) << 24);                       // B (values) MN-major
-      auto last_q = [&](int kt) { return active(1, kt) ? 1 : 0; };    // the query tile that uses a key tile last
       auto wait = [&](int b, int parity) { return (bool)__all_sync(0xffffffffu, mbar_wait(bar(b), parity)); };
-      bool ok = wait(L::B_Q, 0);
-      auto issue_s = [&](int q, int kt) -> bool {         // S_q = Q_q . K(kt)^T
-        const int j = 2 * visited(kt), s = j % SLOTS;
-        if (!wait(L::B_FULL + s, (j / SLOTS) & 1)) return false;
-        tc_fence_after();
-        const uint32_t k_src = kv_s + s * SLOT_BYTES, q_src = q_s + q * Q_BYTES;
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t half = k / 4, inner = (k % 4) * 32;
-          umma_ss(tmem_s + q * kBN, desc_kmajor_sw128(q_src + half * kBM * 128) + (inner >> 4),
-                    desc_kmajor_sw128(k_src + half * kBN * 128) + (inner >> 4), idesc_s, k > 0 ? 1u : 0u, elected);
-        }
-        umma_commit(bar(L::B_S_FULL + q), elected);
-        if (q == last_q(kt)) umma_commit(bar(L::B_EMPTY + s), elected);      // the keys have been read
-        return true;
-      };
+      bool ok = true;
+      int base = 0, loads[2] = {0, 0};
       int done[2] = {0, 0};                                // key tiles of each query tile so far
-      auto issue_pv = [&](int q, int kt) -> bool {        // O_q += P_q . V(kt)
-        const int j = 2 * visited(kt) + 1, s = j % SLOTS;
-        if (!wait(L::B_FULL + s, (j / SLOTS) & 1)) return false;
-        const uint32_t v_src = kv_s + s * SLOT_BYTES;
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {             // the first 64 keys' probabilities are used while the others are made
-          if (!wait((half ? L::B_P_FULL : L::B_P_HALF) + q, done[q] & 1)) return false;
+      for (int n = 0, block = blockIdx.x; ok && block >= 0; ++n) {
+        const Item it(block, tiles, num_tiles, nq, window, split);
+        auto last_q = [&](int kt) { return it.active(1, kt) ? 1 : 0; };    // the query tile that uses a key tile last
+        auto issue_s = [&](int q, int kt) -> bool {         // S_q = Q_q . K(kt)^T
+          const int j = base + 2 * it.visited(kt), s = j % SLOTS;
+          if (!wait(L::B_FULL + s, (j / SLOTS) & 1)) return false;
           tc_fence_after();
+          const uint32_t k_src = kv_s + s * SLOT_BYTES, q_src = q_s + q * Q_BYTES;
 #pragma unroll
-          for (int k = half * (kBN / 32); k < (half + 1) * (kBN / 32); ++k)       // 16 keys (8 columns of pairs) a step
-            umma_ts(tmem_o + q * D, tmem_s + q * kBN + k * 8, desc_mnmajor_sw128(v_src + k * 2048, kBN * 128),
-                         idesc_o, (done[q] > 0 || k > 0) ? 1u : 0u, elected);
-        }
-        umma_commit(bar(L::B_O_FULL + q), elected);
-        if (q == last_q(kt)) umma_commit(bar(L::B_EMPTY + s), elected);      // the values have been read
-        ++done[q];
-        return true;
-      };
-      for (int q = 0; q < 2 && ok; ++q)
-        if (active(q, tb)) ok = issue_s(q, tb);
-      for (int kt = tb, before = tb; kt < te && ok; before = kt, kt = next_tile(kt)) {
+          for (int k = 0; k < D / 16; ++k) {
+            const uint32_t half = k / 4, inner = (k % 4) * 32;
+            umma_ss(tmem_s + q * kBN, desc_kmajor_sw128(q_src + half * kBM * 128) + (inner >> 4),
+                      desc_kmajor_sw128(k_src + half * kBN * 128) + (inner >> 4), idesc_s, k > 0 ? 1u : 0u, elected);
+          }
+          umma_commit(bar(L::B_S_FULL + q), elected);
+          if (q == last_q(kt)) umma_commit(bar(L::B_EMPTY + s), elected);      // the keys have been read
+          return true;
+        };
+        bool begun[2] = {false, false};
+        auto issue_pv = [&](int q, int kt) -> bool {        // O_q += P_q . V(kt)
+          const int j = base + 2 * it.visited(kt) + 1, s = j % SLOTS;
+          if (!wait(L::B_FULL + s, (j / SLOTS) & 1)) return false;
+          const uint32_t v_src = kv_s + s * SLOT_BYTES;
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {             // the first 64 keys' probabilities are used while the others are made
+            if (!wait((half ? L::B_P_FULL : L::B_P_HALF) + q, done[q] & 1)) return false;
+            tc_fence_after();
+#pragma unroll
+            for (int k = half * (kBN / 32); k < (half + 1) * (kBN / 32); ++k)       // 16 keys (8 columns of pairs) a step
+              umma_ts(tmem_o + q * D, tmem_s + q * kBN + k * 8, desc_mnmajor_sw128(v_src + k * 2048, kBN * 128),
+                           idesc_o, (begun[q] || k > 0) ? 1u : 0u, elected);
+          }
+          umma_commit(bar(L::B_O_FULL + q), elected);
+          if (q == last_q(kt)) umma_commit(bar(L::B_EMPTY + s), elected);      // the values have been read
+          begun[q] = true;
+          ++done[q];
+          return true;
+        };
+        // The queries are waited for once a block, whether or not a part of it has keys for them.
         for (int q = 0; q < 2 && ok; ++q) {
-          if (!active(q, kt)) continue;
-          // a query tile that starts, or behind the kept keys goes on, later (window)
-          if (kt != tb && (KEPT ? !active(q, before) : kt == (q == 0 ? tb_0 : tb_1))) ok = issue_s(q, kt);
-          if (ok) ok = issue_pv(q, kt);
-          // the next scores of this query tile go over its probabilities: the product that reads them
-          // was issued just before and runs first; meanwhile the other tile's softmax is at work
-          if (ok && active(q, next_tile(kt))) ok = issue_s(q, next_tile(kt));
+          if (!it.has(q)) continue;
+          ok = wait(L::B_Q + q, loads[q]++ & 1);
+          if (ok && it.active(q, it.tb)) ok = issue_s(q, it.tb);
         }
+        for (int kt = it.tb, before = it.tb; kt < it.te && ok; before = kt, kt = it.next_tile(kt)) {
+          for (int q = 0; q < 2 && ok; ++q) {
+            if (!it.active(q, kt)) continue;
+            // a query tile that starts, or behind the kept keys goes on, later (window)
+            if (kt != it.tb && (KEPT ? !it.active(q, before) : kt == (q == 0 ? it.tb_0 : it.tb_1))) ok = issue_s(q, kt);
+            if (ok) ok = issue_pv(q, kt);
+            // the next scores of this query tile go over its probabilities: the product that reads them
+            // was issued just before and runs first; meanwhile the other tile's softmax is at work
+            if (ok && it.active(q, it.next_tile(kt))) ok = issue_s(q, it.next_tile(kt));
+          }
+        }
+        base += 2 * it.visits();
+        block = -1;
+        if (ok) block = next_of(n, ok);
       }
       if (!ok && lane == 0) atomicExch(error_flag, 8);
+      __syncwarp();
     }
-    __syncwarp();
   } else {
     // ------------------------------------------------------------------ softmax: one query tile, one row per thread
-    const int q = (warp - 2) >> 2;
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax));
+    const int q = (warp - 4) >> 2;
     const int quarter = warp & 3;
     const int row = quarter * 32 + lane;                  // TMEM lane = query row of the tile
-    const int rows_q = q == 0 ? min(rows, kBM) : rows_1;
-    const int pos0_q = pos0 + q * kBM;
-    const int pos = pos0_q + row;
-    const int wfirst = window.first(pos);
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     const uint32_t s_addr = tmem_s + q * kBN + lane_addr, o_addr = tmem_o + q * D + lane_addr;
-    float m_ref = -INFINITY, l_run = 0.0f;
+    // where the warp's 32 rows of output lie before they leave: the place of its queries, which no product reads any more
+    unsigned char* stage = smem + q * Q_BYTES + quarter * (32 * D * 2);
+    constexpr int CHUNKS = D / 8;                          // of 16 bytes, in a row of 2 D bytes
+    auto stage_at = [&](int r, int c) { return reinterpret_cast<uint4*>(stage + r * (D * 2) + ((c ^ (r & 7)) * 16)); };
     bool ok = true;
-    int i = 0;                                            // key tiles of this query tile so far
-    for (int kt = KEPT ? tb : (q == 0 ? tb_0 : tb_1); kt < (KEPT ? te : (q == 0 ? te_0 : te_1)); kt = next_tile(kt)) {
-      if (KEPT && !active(q, kt)) continue;
-      const int key0 = kt * kBN;
-      ok = __all_sync(0xffffffffu, mbar_wait(bar(L::B_S_FULL + q), i & 1));
-      if (!ok) break;
-      tc_fence_after();
-      const bool edge = key0 + kBN - 1 > pos0_q ||
-                        (window.any() && key0 < window.first(pos0_q + kBM - 1) && (!KEPT || key0 + kBN > keep));
-      // the row's scores stay in registers: 128 of them
-      float s[kBN];
-#pragma unroll
-      for (int c = 0; c < kBN; c += 32) tmem_ld32(s_addr + c, *reinterpret_cast<float(*)[32]>(&s[c]));
-      tmem_wait_ld();
-      if (edge) {
-#pragma unroll
-        for (int j = 0; j < kBN; ++j) {
-          const int key = key0 + j;
-          if (key > pos || (key < wfirst && (!KEPT || key >= keep))) s[j] = -INFINITY;
-        }
-      }
-      float mx4[4] = {s[0], s[1], s[2], s[3]};
-#pragma unroll
-      for (int j = 4; j + 7 < kBN; j += 8)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) mx4[e] = max3(mx4[e], s[j + e], s[j + 4 + e]);
-      const float mx = fmaxf(max3(mx4[0], mx4[1], max3(s[kBN - 4], s[kBN - 3], s[kBN - 2])), max3(mx4[2], mx4[3], s[kBN - 1]));
-      // the reference maximum moves only when the row's maximum has outgrown it
-      const bool outgrown = m_ref > -INFINITY && (mx - m_ref) * scale_log2 > kRescaleStep;
-      float factor = 1.0f;
-      if (outgrown) {
-        factor = ex2((m_ref - mx) * scale_log2);
-        m_ref = mx;
-        l_run *= factor;
-      } else if (m_ref == -INFINITY) {
-        m_ref = mx;                                        // nothing accumulated for this row so far
-      }
-      if (i > 0 && __any_sync(0xffffffffu, outgrown)) {    // rescale this warp's rows of O in tensor memory
-        ok = __all_sync(0xffffffffu, mbar_wait(bar(L::B_O_FULL + q), (i - 1) & 1));   // the products so far are done
+    int i0 = 0, loads = 0;                                // key tiles, and blocks with rows, of this query tile before this block
+    for (int n = 0, block = blockIdx.x; ok && block >= 0; ++n) {
+      const Item it(block, tiles, num_tiles, nq, window, split);
+      const int rows_q = q == 0 ? min(it.rows, kBM) : it.rows_1;
+      const int pos0_q = it.pos0 + q * kBM;
+      const int pos = pos0_q + row;
+      const int wfirst = window.first(pos);
+      float m_ref = -INFINITY, l_run = 0.0f;
+      int i = 0;                                            // key tiles of this query tile so far
+      for (int kt = KEPT ? it.tb : (q == 0 ? it.tb_0 : it.tb_1); kt < (KEPT ? it.te : (q == 0 ? it.te_0 : it.te_1)); kt = it.next_tile(kt)) {
+        if (KEPT && !it.active(q, kt)) continue;
+        const int key0 = kt * kBN;
+        ok = __all_sync(0xffffffffu, mbar_wait(bar(L::B_S_FULL + q), (i0 + i) & 1));
         if (!ok) break;
         tc_fence_after();
-#pragma unroll 1
-        for (int c = 0; c < D; c += 32) {
-          float t[32];
-          tmem_ld32(o_addr + c, t);
-          tmem_wait_ld();
-          uint32_t u[32];
+        const bool edge = key0 + kBN - 1 > pos0_q ||
+                          (window.any() && key0 < window.first(pos0_q + kBM - 1) && (!KEPT || key0 + kBN > it.keep));
+        // the row's scores stay in registers: 128 of them
+        float s[kBN];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) u[j] = __float_as_uint(t[j] * factor);
-          tmem_st32(o_addr + c, u);
-        }
-        tmem_wait_st();
-      }
-      // probabilities over the scores, 64 keys (32 columns of bfloat16 pairs) at a time
-      const float bias = m_ref == -INFINITY ? 0.0f : -m_ref * scale_log2;
-      float sum4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        for (int c = 0; c < kBN; c += 32) tmem_ld32(s_addr + c, *reinterpret_cast<float(*)[32]>(&s[c]));
+        tmem_wait_ld();
+        if (edge) {
 #pragma unroll
-      for (int c = 0; c < kBN; c += 64) {
-        uint32_t packed[32];
-#pragma unroll
-        for (int j = 0; j < 64; j += 2) {
-          const float p0 = ex2(fmaf(s[c + j], scale_log2, bias));
-          const float p1 = ex2(fmaf(s[c + j + 1], scale_log2, bias));
-          sum4[(j >> 1) & 3] += p0 + p1;
-          __nv_bfloat162 b2 = __floats2bfloat162_rn(p0, p1);
-          packed[j >> 1] = *reinterpret_cast<uint32_t*>(&b2);
-        }
-        tmem_st32(s_addr + (c >> 1), packed);              // columns whose scores have been read already
-        tmem_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar((c == 0 ? L::B_P_HALF : L::B_P_FULL) + q));
-      }
-      l_run += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
-      ++i;
-    }
-    if (ok && i > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar(L::B_O_FULL + q), (i - 1) & 1));
-    if (!ok && lane == 0) atomicExch(error_flag, 9);
-    if (!KEPT && slot >= 0) {                              // the sum as it is, for the merge
-      const size_t at = (size_t)slot * 2 * kBM + q * kBM + row;
-      if (row < rows_q)
-        split.ml[at] = ok && i > 0 ? make_float2(m_ref > -INFINITY ? m_ref * scale_log2 : -INFINITY, l_run) : make_float2(-INFINITY, 0.0f);
-      if (ok && i > 0) {
-        tc_fence_after();
-#pragma unroll 1
-        for (int c = 0; c < D; c += 32) {
-          float t[32];
-          tmem_ld32(o_addr + c, t);
-          tmem_wait_ld();
-          if (row < rows_q) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 4)
-              *reinterpret_cast<float4*>(split.o + at * D + c + j) = make_float4(t[j], t[j + 1], t[j + 2], t[j + 3]);
+          for (int j = 0; j < kBN; ++j) {
+            const int key = key0 + j;
+            if (key > pos || (key < wfirst && (!KEPT || key >= it.keep))) s[j] = -INFINITY;
           }
         }
+        float mx4[4] = {s[0], s[1], s[2], s[3]};
+#pragma unroll
+        for (int j = 4; j + 7 < kBN; j += 8)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) mx4[e] = max3(mx4[e], s[j + e], s[j + 4 + e]);
+        const float mx = fmaxf(max3(mx4[0], mx4[1], max3(s[kBN - 4], s[kBN - 3], s[kBN - 2])), max3(mx4[2], mx4[3], s[kBN - 1]));
+        // the reference maximum moves only when the row's maximum has outgrown it
+        const bool outgrown = m_ref > -INFINITY && (mx - m_ref) * scale_log2 > kRescaleStep;
+        float factor = 1.0f;
+        if (outgrown) {
+          factor = ex2((m_ref - mx) * scale_log2);
+          m_ref = mx;
+          l_run *= factor;
+        } else if (m_ref == -INFINITY) {
+          m_ref = mx;                                        // nothing accumulated for this row so far
+        }
+        if (i > 0 && __any_sync(0xffffffffu, outgrown)) {    // rescale this warp's rows of O in tensor memory
+          ok = __all_sync(0xffffffffu, mbar_wait(bar(L::B_O_FULL + q), (i0 + i - 1) & 1));   // the products so far are done
+          if (!ok) break;
+          tc_fence_after();
+#pragma unroll 1
+          for (int c = 0; c < D; c += 32) {
+            float t[32];
+            tmem_ld32(o_addr + c, t);
+            tmem_wait_ld();
+            uint32_t u[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) u[j] = __float_as_uint(t[j] * factor);
+            tmem_st32(o_addr + c, u);
+          }
+          tmem_wait_st();
+        }
+        // probabilities over the scores, 64 keys (32 columns of bfloat16 pairs) at a time; two scores an instruction
+        const float bias = m_ref == -INFINITY ? 0.0f : -m_ref * scale_log2;
+        const float2 scale2 = make_float2(scale_log2, scale_log2), bias2 = make_float2(bias, bias);
+        float2 sum2[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+#pragma unroll
+        for (int c = 0; c < kBN; c += 64) {
+          uint32_t packed[32];
+#pragma unroll
+          for (int j = 0; j < 64; j += 2) {
+            const float2 x = fma2(make_float2(s[c + j], s[c + j + 1]), scale2, bias2);
+            const float2 p = make_float2(ex2(x.x), ex2(x.y));
+            sum2[(j >> 1) & 1] = add2(sum2[(j >> 1) & 1], p);
+            __nv_bfloat162 b2 = __floats2bfloat162_rn(p.x, p.y);
+            packed[j >> 1] = *reinterpret_cast<uint32_t*>(&b2);
+          }
+          tmem_st32(s_addr + (c >> 1), packed);              // columns whose scores have been read already
+          tmem_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar((c == 0 ? L::B_P_HALF : L::B_P_FULL) + q));
+        }
+        l_run += (sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y);
+        ++i;
       }
-    } else if (ok && i > 0) {
+      if (ok && i > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar(L::B_O_FULL + q), (i0 + i - 1) & 1));
+      if (ok && i == 0 && it.has(q)) ok = __all_sync(0xffffffffu, mbar_wait(bar(L::B_Q + q), loads & 1));
+      if (!ok) {
+        if (lane == 0) atomicExch(error_flag, 9);
+        break;
+      }
+      i0 += i;
       tc_fence_after();
-      if (window.sink && m_ref > -INFINITY) l_run += exp2f(window.sink_log2(h) - m_ref * scale_log2);     // the sink's share
-      const float inv = (l_run > 0.0f ? 1.0f / l_run : 0.0f) * post.factor(row0 + q * kBM + min(row, max(rows_q - 1, 0)), h);
-      bf16* dst = out + ((size_t)(row0 + q * kBM + row) * nq + h) * D;
-      if (post.table != nullptr) {                         // 16 pairs at a time: 32 columns, or 16 and their 16 partners
-        const float4* cs4 = reinterpret_cast<const float4*>(post.table + (size_t)(row0 + q * kBM + min(row, max(rows_q - 1, 0))) * (D / 2));
-        const int apart = post.interleaved ? 16 : D / 2;
+      const int rows_w = rows_q - quarter * 32;             // rows of this warp
+      if (!KEPT && it.slot >= 0) {                          // the sum as it is, for the merge
+        const size_t at = (size_t)it.slot * 2 * kBM + q * kBM + quarter * 32;
+        if (lane < rows_w)
+          split.ml[at + lane] = i > 0 ? make_float2(m_ref > -INFINITY ? m_ref * scale_log2 : -INFINITY, l_run) : make_float2(-INFINITY, 0.0f);
+        if (i > 0) {
 #pragma unroll 1
-        for (int m0 = 0; m0 < D / 2; m0 += 16) {
-          const int c = post.interleaved ? 2 * m0 : m0;
-          float lo[16], hi[16];
-          tmem_ld16f(o_addr + c, lo);
-          tmem_ld16f(o_addr + c + apart, hi);
-          tmem_wait_ld();
-          if (post.interleaved) {
+          for (int half = 0; half < 2; ++half) {            // rows of D / 2 float32 numbers
 #pragma unroll
-            for (int j = 0; j < 8; j += 2) {
-              const float4 a = cs4[(m0 + j) >> 1], b = cs4[(m0 + 8 + j) >> 1];
-              HeadOutput::apply(make_float2(a.x, a.y), lo[2 * j], lo[2 * j + 1]);
-              HeadOutput::apply(make_float2(a.z, a.w), lo[2 * j + 2], lo[2 * j + 3]);
-              HeadOutput::apply(make_float2(b.x, b.y), hi[2 * j], hi[2 * j + 1]);
-              HeadOutput::apply(make_float2(b.z, b.w), hi[2 * j + 2], hi[2 * j + 3]);
-            }
-          } else {
+            for (int c = 0; c < D / 2; c += 32) {
+              float t[32];
+              tmem_ld32(o_addr + half * (D / 2) + c, t);
+              tmem_wait_ld();
 #pragma unroll
-            for (int j = 0; j < 16; j += 2) {
-              const float4 a = cs4[(m0 + j) >> 1];
-              HeadOutput::apply(make_float2(a.x, a.y), lo[j], hi[j]);
-              HeadOutput::apply(make_float2(a.z, a.w), lo[j + 1], hi[j + 1]);
+              for (int j = 0; j < 32; j += 4)
+                *stage_at(lane, (c + j) / 4) = make_uint4(__float_as_uint(t[j]), __float_as_uint(t[j + 1]), __float_as_uint(t[j + 2]),
+                                                          __float_as_uint(t[j + 3]));
             }
+            __syncwarp();
+#pragma unroll 4
+            for (int e = lane; e < 32 * CHUNKS; e += 32) {
+              const int r = e / CHUNKS, c = e % CHUNKS;
+              if (r < rows_w) *reinterpret_cast<uint4*>(split.o + (at + r) * D + half * (D / 2) + c * 4) = *stage_at(r, c);
+            }
+            __syncwarp();
           }
-          if (row < rows_q) {
+        }
+      } else if (i > 0) {
+        if (window.sink && m_ref > -INFINITY) l_run += exp2f(window.sink_log2(it.h) - m_ref * scale_log2);     // the sink's share
+        const int t_row = it.row0 + q * kBM + min(row, max(rows_q - 1, 0));
+        const float inv = (l_run > 0.0f ? 1.0f / l_run : 0.0f) * post.factor(t_row, it.h);
+        if (post.table != nullptr) {                         // 16 pairs at a time: 32 columns, or 16 and their 16 partners
+          const float4* cs4 = reinterpret_cast<const float4*>(post.table + (size_t)t_row * (D / 2));
+          const int apart = post.interleaved ? 16 : D / 2;
+#pragma unroll 1
+          for (int m0 = 0; m0 < D / 2; m0 += 16) {
+            const int c = post.interleaved ? 2 * m0 : m0;
+            float lo[16], hi[16];
+            tmem_ld16f(o_addr + c, lo);
+            tmem_ld16f(o_addr + c + apart, hi);
+            tmem_wait_ld();
+            if (post.interleaved) {
+#pragma unroll
+              for (int j = 0; j < 8; j += 2) {
+                const float4 a = cs4[(m0 + j) >> 1], b = cs4[(m0 + 8 + j) >> 1];
+                HeadOutput::apply(make_float2(a.x, a.y), lo[2 * j], lo[2 * j + 1]);
+                HeadOutput::apply(make_float2(a.z, a.w), lo[2 * j + 2], lo[2 * j + 3]);
+                HeadOutput::apply(make_float2(b.x, b.y), hi[2 * j], hi[2 * j + 1]);
+                HeadOutput::apply(make_float2(b.z, b.w), hi[2 * j + 2], hi[2 * j + 3]);
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < 16; j += 2) {
+                const float4 a = cs4[(m0 + j) >> 1];
+                HeadOutput::apply(make_float2(a.x, a.y), lo[j], hi[j]);
+                HeadOutput::apply(make_float2(a.z, a.w), lo[j + 1], hi[j + 1]);
+              }
+            }
 #pragma unroll
             for (int j = 0; j < 16; j += 8) {
               uint4 vl, vh;
@@ -478,28 +614,43 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
                 l2[e] = __floats2bfloat162_rn(lo[j + 2 * e] * inv, lo[j + 2 * e + 1] * inv);
                 h2[e] = __floats2bfloat162_rn(hi[j + 2 * e] * inv, hi[j + 2 * e + 1] * inv);
               }
-              *reinterpret_cast<uint4*>(dst + c + j) = vl;
-              *reinterpret_cast<uint4*>(dst + c + apart + j) = vh;
+              *stage_at(lane, (c + j) / 8) = vl;
+              *stage_at(lane, (c + apart + j) / 8) = vh;
+            }
+          }
+        } else {
+#pragma unroll
+          for (int c = 0; c < D; c += 32) {
+            float t[32];
+            tmem_ld32(o_addr + c, t);
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 32; j += 8) {
+              uint4 v;
+              __nv_bfloat162* v2 = reinterpret_cast<__nv_bfloat162*>(&v);
+#pragma unroll
+              for (int e = 0; e < 4; ++e) v2[e] = __floats2bfloat162_rn(t[j + 2 * e] * inv, t[j + 2 * e + 1] * inv);
+              *stage_at(lane, (c + j) / 8) = v;
             }
           }
         }
-      } else
-#pragma unroll 1
-      for (int c = 0; c < D; c += 32) {
-        float t[32];
-        tmem_ld32(o_addr + c, t);
-        tmem_wait_ld();
-        if (row < rows_q) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 8) {
-            uint4 v;
-            __nv_bfloat162* v2 = reinterpret_cast<__nv_bfloat162*>(&v);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) v2[e] = __floats2bfloat162_rn(t[j + 2 * e] * inv, t[j + 2 * e + 1] * inv);
-            *reinterpret_cast<uint4*>(dst + c + j) = v;
-          }
+        __syncwarp();
+        bf16* dst = out + ((size_t)(it.row0 + q * kBM + quarter * 32) * nq + it.h) * D;
+#pragma unroll 4
+        for (int e = lane; e < 32 * CHUNKS; e += 32) {       // whole rows, 16 bytes a lane
+          const int r = e / CHUNKS, c = e % CHUNKS;
+          if (r < rows_w) *reinterpret_cast<uint4*>(dst + (size_t)r * nq * D + c * 8) = *stage_at(r, c);
         }
       }
+      if (it.has(q)) {                                       // the next queries may come
+        ++loads;
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(L::B_Q_FREE + q));
+      }
+      tc_fence_before();
+      block = next_of(n, ok);
+      if (!ok && lane == 0) atomicExch(error_flag, 9);
     }
   }
   tc_fence_before();

@@ -1,0 +1,52 @@
+"""Prompt attention of more blocks than SMs: a resident block that goes through several blocks of the grid gives every one of them
+the bits it has in a grid of its own."""
+import math
+
+import pytest
+import torch
+
+from tests.test_kernels_gpu import DEV, _Ctx, fill_cache, make_cache_case
+
+pytestmark = pytest.mark.gpu
+
+LENS = [1024, 130, 1003, 5, 640, 300, 900, 129, 1024, 257, 512]
+SPANS = [256, 130, 1000, 5, 128, 300, 1, 129, 2, 257, 131]          # one and two query tiles, one row of a second, a decoded token
+
+
+def _alone(ctx, r):
+    from inferflux_b200.csrc import CudaKernels
+    one, first = _Ctx(), sum(n for _s, n in ctx.spans[:r])
+    one.spans, one.slots_host = [ctx.spans[r]], [ctx.slots_host[r]]
+    one.num_tokens = ctx.spans[r][1]
+    one.positions = ctx.positions[first:first + one.num_tokens].clone()
+    one.token_req = torch.zeros(one.num_tokens, dtype=torch.int32, device=DEV)
+    one.req_slot = ctx.req_slot[r:r + 1].clone()
+    one.extra, one.extra_len = {}, {}
+    for name, vals in CudaKernels.attention_sections(CudaKernels, one).items():
+        one.extra[name] = torch.tensor(vals, dtype=torch.int32, device=DEV)
+        one.extra_len[name] = len(vals)
+    one.max_kv_len = sum(ctx.spans[r])
+    return one, slice(first, first + one.num_tokens)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("window,keep", [(None, 0), (200, 0), (200, 300)])
+def test_blocks_behind_one_another(cuda_kernels, d, window, keep):
+    nq, nkv, page = 36, 4, 16
+    ctx, cache, slots = make_cache_case(torch.bfloat16, nkv, d, page, LENS, SPANS, num_pages=sum(-(-n // page) for n in LENS) + 3, seed=3)
+    fill_cache(cache, LENS, slots, nkv, d, torch.bfloat16, seed=4)
+    blocks = ctx.extra_len["attn.prefill_tiles"] // 4 * nq
+    assert blocks > 3 * 148 and cuda_kernels.prefill_parts(ctx, nq, window or 0) == 1
+    q = torch.randn(ctx.num_tokens, nq * d, generator=torch.Generator().manual_seed(5)).bfloat16().to(DEV)
+    args = (nq, nkv, d, window, 2.0 / math.sqrt(d))
+    got = [cuda_kernels.attention(q, *args, ctx, cache, keep_first=keep) for _ in range(3)]
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])          # whichever SM takes which block
+    for r, span in enumerate(SPANS):
+        one, rows = _alone(ctx, r)
+        assert one.extra_len["attn.prefill_tiles"] // 4 * nq <= 148
+        want = cuda_kernels.attention(q[rows].contiguous(), *args, one, cache, keep_first=keep)
+        if span > 1:
+            assert torch.equal(got[0][rows], want), r
+        else:                                       # (a decoded token's keys are cut by how many tokens there are)
+            assert (got[0][rows].float() - want.float()).abs().max() <= 2 ** -6
+    cuda_kernels.check_errors()
