@@ -11,8 +11,10 @@
 //
 //   warp 0     TMA: the rows' queries once; per tile the pages' latents as boxes [16 keys x 64] into one of two buffers of 64 KB,
 //              their rotated parts into one of 16 KB, which is free again as soon as the scores are made
+//              (a buffer's first 64 keys leave when the first half of the weighted sum is done, and the next ones come in their place)
 //   warp 1     MMA issue: the next tile's scores go in front of a tile's weighted sum, so that the exponentials of one tile run
-//              under the products of the other
+//              under the products of the other; where the weights are there before the next tile's keys, the sum goes first,
+//              since it frees the buffer that the tile behind that one waits for
 //   warps 2-9  softmax: warps w and w + 4 share rows and meet once a tile for the maximum
 //
 // Shared memory is one block's (80 KB of queries, 144 KB of keys), tensor memory too (256 + 256 columns).
@@ -24,9 +26,12 @@
 //
 // Every wait is bounded; a wait that runs out sets *error_flag.
 //
-// Bound: the tensor pipe (576 multiply-adds a score) beside 64 exponentials a thread and tile.  2,048 tokens of 12 heads:
-// latent_attention_mma_kernel and its merge 302 us, this 55 (192 blocks on 148 SMs; one that holds the last tokens
-// walks 16 tiles at 3.2 us).  100 tokens behind 2,000: 17 us and 4 of merge.
+// Bound: 2,304 cycles of the tensor pipe (576 multiply-adds a score) of the 3,830 that a tile takes, the rest the fetch of a tile,
+// which begins only when one of the two buffers is free.  2,048 tokens of 12 heads (192 blocks on 148 SMs; one that holds the last
+// tokens walks 16 tiles), us: latent_attention_mma_kernel and its merge 302; this with the scores always first, so that every sum
+// waited for the next tile's fetch, 52.9 (3.2 a tile); whichever can go first 45.5 (2.3); fetched by halves, two scores an
+// instruction and rows stored whole 44.4 (2.14).  1,000 tokens in three requests of 28 heads behind 1,500: 78.7, now 66.9; 300 of
+// 12 heads behind 500 19.4 and 17.8.  Blocks of more than 12 tiles in two parts would save 5 and cost 3.5 for adding them up.
 #include "common.cuh"
 #include "ptx_sm100.cuh"
 
@@ -84,7 +89,8 @@ struct LatentPromptLayout {
   static constexpr int BOXES = (kLpRank + ROT) / 64, ROT_BOXES = ROT / 64;
   static constexpr uint32_t Q = 0, KV = Q + BOXES * kLpBox, KV_BYTES = 4 * kLpBox, TURNED = KV + 2 * KV_BYTES,
                             BARS = TURNED + ROT_BOXES * kLpBox;
-  enum { B_Q = 0, B_KV_FULL = 1, B_KV_EMPTY = 3, B_ROT_FULL = 5, B_ROT_EMPTY = 6, B_S_FULL = 7, B_P_FULL = 9, B_O_FULL = 11, B_COUNT = 12 };
+  // B_KV_EMPTY: of a buffer's first 64 keys, + 2: of the others
+  enum { B_Q = 0, B_KV_FULL = 1, B_KV_EMPTY = 3, B_ROT_FULL = 7, B_ROT_EMPTY = 8, B_S_FULL = 9, B_P_FULL = 11, B_O_FULL = 13, B_COUNT = 14 };
   static constexpr uint32_t HOLDER = BARS + B_COUNT * 8, MAXIMA = HOLDER + 8, END = MAXIMA + 2 * kLpRows * 4;
   static constexpr size_t BYTES = 1024 + END;
 };
@@ -158,16 +164,20 @@ __global__ void __launch_bounds__(kLpThreads, 1) latent_prompt_kernel(
         if (page < 0 || page >= num_pages) page = 0;
         y = page * page_size + (seen & ~15) % page_size;
       }
-      ok = __all_sync(0xffffffffu, mbar_wait(bar(L::B_KV_EMPTY + (i & 1)), ((i >> 1) & 1) ^ 1));
-      if (!ok) break;
-      if (lane == 0) mbar_expect_tx(bar(L::B_KV_FULL + (i & 1)), L::KV_BYTES);
-      __syncwarp();
-      if (lane < 8) {
-        const uint32_t dst = base + L::KV + (i & 1) * L::KV_BYTES + lane * 2048;
+#pragma unroll 1
+      for (int part = 0; part < 2; ++part) {                           // 64 keys each, as the sums that read their places come to an end
+        ok = __all_sync(0xffffffffu, mbar_wait(bar(L::B_KV_EMPTY + 2 * part + (i & 1)), ((i >> 1) & 1) ^ 1));
+        if (!ok && part == 0) break;                                   // (a tile that has begun is fetched whole, so that its copies land)
+        if (part == 0 && lane == 0) mbar_expect_tx(bar(L::B_KV_FULL + (i & 1)), L::KV_BYTES);
+        __syncwarp();
+        if (lane >> 2 == part) {
+          const uint32_t dst = base + L::KV + (i & 1) * L::KV_BYTES + lane * 2048;
 #pragma unroll
-        for (int b = 0; b < 4; ++b) tma_load_2d(dst + b * kLpBox, &pool_map, b * 64, y, bar(L::B_KV_FULL + (i & 1)));
+          for (int b = 0; b < 4; ++b) tma_load_2d(dst + b * kLpBox, &pool_map, b * 64, y, bar(L::B_KV_FULL + (i & 1)));
+        }
+        kv_issued = i + 1;
       }
-      kv_issued = i + 1;
+      if (!ok) break;
       if (ROT) {
         ok = __all_sync(0xffffffffu, mbar_wait(bar(L::B_ROT_EMPTY), (i & 1) ^ 1));
         if (!ok) break;
@@ -189,6 +199,7 @@ __global__ void __launch_bounds__(kLpThreads, 1) latent_prompt_kernel(
     {
       const uint32_t elected = elect_one();
       auto wait = [&](int b, int parity) { return (bool)__all_sync(0xffffffffu, mbar_wait(bar(b), parity)); };
+      auto ready = [&](int b, int parity) { return (bool)__all_sync(0xffffffffu, mbar_test(bar(b), parity)); };
       const uint32_t common = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kLpRows >> 4) << 24);
       const uint32_t idesc_s = common | ((uint32_t)(kLpKeys >> 3) << 17), idesc_o = common | (1u << 16) | ((uint32_t)(kLpRank >> 3) << 17);
       bool ok = wait(L::B_Q, 0);
@@ -213,15 +224,27 @@ __global__ void __launch_bounds__(kLpThreads, 1) latent_prompt_kernel(
       };
       if (ok) ok = scores(0);
       for (int i = 0; i < n && ok; ++i) {
-        if (i + 1 < n) ok = scores(i + 1);                             // over the weights of tile i - 1, whose product was issued before
+        // whichever can go first: the next tile's scores (over the weights of tile i - 1, whose product was issued before) or this
+        // tile's sum, which frees the buffer that the tile behind waits for
+        bool made = i + 1 >= n;
+        for (int tries = 0; !made && tries < kWaitLimit; ++tries) {
+          if (ready(L::B_KV_FULL + ((i + 1) & 1), ((i + 1) >> 1) & 1)) {
+            ok = scores(i + 1);
+            made = true;
+          } else if (ready(L::B_P_FULL + (i & 1), (i >> 1) & 1))
+            break;
+        }
         if (!ok || !(ok = wait(L::B_P_FULL + (i & 1), (i >> 1) & 1))) break;
         lp_after();
         const uint32_t v_src = base + L::KV + (i & 1) * L::KV_BYTES;
 #pragma unroll
-        for (int k = 0; k < kLpKeys / 16; ++k)
+        for (int k = 0; k < kLpKeys / 16; ++k) {
           umma_ts(tmem_o, tmem + (i & 1) * kLpKeys + k * 8, lp_desc_mn(v_src + k * 2048), idesc_o, (i > 0 || k > 0) ? 1u : 0u, elected);
-        umma_commit(bar(L::B_KV_EMPTY + (i & 1)), elected);
+          if (k == kLpKeys / 32 - 1) umma_commit(bar(L::B_KV_EMPTY + (i & 1)), elected);
+        }
+        umma_commit(bar(L::B_KV_EMPTY + 2 + (i & 1)), elected);
         umma_commit(bar(L::B_O_FULL), elected);
+        if (!made) ok = scores(i + 1);
       }
       if (!ok && lane == 0) atomicExch(error_flag, 62);
     }
@@ -300,17 +323,18 @@ __global__ void __launch_bounds__(kLpThreads, 1) latent_prompt_kernel(
         }
       }
       const float bias = m_ref == -INFINITY ? 0.0f : -m_ref * scale_log2;
-      float sum4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      const float2 scale2 = make_float2(scale_log2, scale_log2), bias2 = make_float2(bias, bias);
+      float2 sum2[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
       uint32_t packed[32];
 #pragma unroll
-      for (int j = 0; j < 64; j += 2) {
-        const float p0 = lp_ex2(fmaf(s[j], scale_log2, bias)), p1 = lp_ex2(fmaf(s[j + 1], scale_log2, bias));
-        sum4[(j >> 1) & 3] += p0 + p1;
-        __nv_bfloat162 b2 = __floats2bfloat162_rn(p0, p1);
+      for (int j = 0; j < 64; j += 2) {                                // two scores an instruction
+        const float2 x = fma2(make_float2(s[j], s[j + 1]), scale2, bias2), p = make_float2(lp_ex2(x.x), lp_ex2(x.y));
+        sum2[(j >> 1) & 1] = add2(sum2[(j >> 1) & 1], p);
+        __nv_bfloat162 b2 = __floats2bfloat162_rn(p.x, p.y);
         packed[j >> 1] = *reinterpret_cast<uint32_t*>(&b2);
       }
       lp_st32(s_addr + half * 32, packed);                             // columns whose scores both halves have read
-      l_run += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+      l_run += (sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y);
       lp_wait_st();
       lp_before();
       __syncwarp();
@@ -330,28 +354,50 @@ __global__ void __launch_bounds__(kLpThreads, 1) latent_prompt_kernel(
       l += exp2f(sinks[grow % heads] * 1.4426950408889634f - m_ref * scale_log2);
     }
     const float inv = (l > 0.0f || isnan(l) ? 1.0f / l : 0.0f) * (gate != nullptr ? gate[grow] : 1.0f);
+    // Out through shared memory in whole rows of 256 bytes, where the queries lay: the products that read them are done.  (A
+    // thread's own row, 16 bytes of 32 rows a store, took 2 us.)
+    unsigned char* stage = smem + L::Q + (warp - 2) * (32 * 256);
+    auto stage_at = [&](int r, int c) { return reinterpret_cast<uint4*>(stage + r * 256 + ((c ^ (r & 7)) * 16)); };
+    const int rows_w = rows - quarter * 32;                            // rows of this warp
+    if (gridDim.z > 1) {
 #pragma unroll 1
-    for (int c = half * 128; c < half * 128 + 128; c += 32) {
-      float t[32];
-      lp_ld32(tmem_o + lane_addr + c, t);
-      lp_wait_ld();
-      if (row < rows) {
-        if (gridDim.z > 1) {
-          float* to = part_o + ((size_t)blockIdx.z * total_rows + grow) * kLpRank + c;
+      for (int c0 = half * 128; c0 < half * 128 + 128; c0 += 64) {
 #pragma unroll
-          for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(to + j) = make_float4(t[j], t[j + 1], t[j + 2], t[j + 3]);
-        } else {
-          __nv_bfloat16* to = out + grow * kLpRank + c;
+        for (int c = 0; c < 64; c += 32) {
+          float t[32];
+          lp_ld32(tmem_o + lane_addr + c0 + c, t);
+          lp_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 32; j += 8) {
-            uint4 v;
-            __nv_bfloat162* v2 = reinterpret_cast<__nv_bfloat162*>(&v);
+          for (int j = 0; j < 32; j += 4)
+            *reinterpret_cast<float4*>(stage_at(lane, (c + j) / 4)) = make_float4(t[j], t[j + 1], t[j + 2], t[j + 3]);
+        }
+        __syncwarp();
+        float* to = part_o + ((size_t)blockIdx.z * total_rows + row0 + quarter * 32) * kLpRank + c0;
+#pragma unroll 4
+        for (int e = lane; e < 32 * 16; e += 32)
+          if ((e >> 4) < rows_w) *reinterpret_cast<uint4*>(to + (size_t)(e >> 4) * kLpRank + (e & 15) * 4) = *stage_at(e >> 4, e & 15);
+        __syncwarp();
+      }
+    } else {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) v2[e] = __floats2bfloat162_rn(t[j + 2 * e] * inv, t[j + 2 * e + 1] * inv);
-            *reinterpret_cast<uint4*>(to + j) = v;
-          }
+      for (int c = 0; c < 128; c += 32) {
+        float t[32];
+        lp_ld32(tmem_o + lane_addr + half * 128 + c, t);
+        lp_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 32; j += 8) {
+          uint4 v;
+          __nv_bfloat162* v2 = reinterpret_cast<__nv_bfloat162*>(&v);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) v2[e] = __floats2bfloat162_rn(t[j + 2 * e] * inv, t[j + 2 * e + 1] * inv);
+          *stage_at(lane, (c + j) / 8) = v;
         }
       }
+      __syncwarp();
+      __nv_bfloat16* to = out + (row0 + quarter * 32) * kLpRank + half * 128;
+#pragma unroll 4
+      for (int e = lane; e < 32 * 16; e += 32)
+        if ((e >> 4) < rows_w) *reinterpret_cast<uint4*>(to + (size_t)(e >> 4) * kLpRank + (e & 15) * 8) = *stage_at(e >> 4, e & 15);
     }
   }
   lp_before();
