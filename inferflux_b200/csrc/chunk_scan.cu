@@ -1,4 +1,5 @@
-// The scans of decay_scan.cu and wkv.cu over long spans, a stretch of 64 tokens at a time instead of token after token.
+// The scans of decay_scan.cu and wkv.cu over long spans, a stretch of 64 tokens at a time instead of token after token.  (One decay
+// per head with keys or values of 128: chunk_tcgen05.cu, 128 tokens at a time, with this file's carry.)
 // With S_0 the state in front of a stretch, and products of decays w over the tokens between,
 //
 //   o_t  = (q_t * prod w_1..t)^T S_0  +  sum over s <= t of (q_t . (k_s * prod w_s+1..t)) v_s

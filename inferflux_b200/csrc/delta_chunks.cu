@@ -10,26 +10,30 @@
 //   O = A V - B X + R S_0          A[t, s] = r_t . (k_s G_t / G_s),      B[t, s] = r_t . (e_s G_t / G_s)          s <= t
 //   S = diag(G_64) S_0 + K^T V - E^T X                                   K, E: keys and e times G_64 / G_s
 //
-// a unit lower triangular system, solved for the columns of [N V | U] so that everything is linear in S_0.  Four kernels:
+// a unit lower triangular system, solved for the columns of [N V | U] so that everything is linear in S_0.  Three kernels, and the norm:
 //
 //   delta_local   per stretch and head: outputs without S_0, the queries that meet S_0, the matrix that carries S_0 on, what is added
 //   delta_carry   the states in front of every stretch, one small product a stretch, 8 value channels a block
 //   chunk_reach   (chunk_scan.cu) adds what S_0 brings to the outputs
-//   delta_finish  (delta_rule.cu) norm and gate
+//   gated_heads_full  (pair_mixer.cu) norm and gate
 //
 // A decay lies between 0.545 and 1, so products over half a stretch and their reciprocals stay below 3e8: G_t / G_s is taken as
-// a product on the one side and a reciprocal on the other, both counted from the middle of the stretch.  Products run on the tensor
-// cores with split operands (chunk_scan.cuh); the triangular system goes by blocks of 16 rows, substituted in the blocks.
+// a product on the one side and a reciprocal on the other, both counted from the middle of the stretch.  Products of operands in
+// three bfloat16 parts: delta_local's on the 5th-generation tensor cores (parts_tcgen05.cuh), the carry's and reach's by mma.sync
+// (chunk_scan.cuh).  The triangular system goes by blocks of 16 rows: a block is substituted, and what it changes in the rows behind
+// it is a product.
 //
 // A stretch that holds a number that is not finite, or in which one comes up that a scan would not have formed, is walked token by
 // token.  The order of the sums depends on where a span is cut into steps, so the float32 run keeps the scan.
 //
-// Bound: delta_local, two blocks of 8 warps an SM (110 KB each: X in the values' place, decays in the matrix's): barriers and the chain
-// split -> product -> sum between them (issue slots 49 % busy, tensor pipe 35 %; one block of 16 warps with a tile more 206 us, so
-// 165).  2,048 tokens of 24 heads: delta_rule.cu's three kernels 658 us, these 232.
-// Error of the state against 64 bits (2-norm, scan and this, 2,048 tokens): parameters where trained models have them 5.2e-7 and
-// 4.6e-7, decays near one 1.76e-6 and 1.70e-6, random ones 0.95e-7 and 1.00e-7.  (With operands of 22 bits 241 us, 1.4e-7 in the last
-// case, and 1.0e-6 in place of the scan's 4.6e-7 where 130 keys are nearly the same.)
+// Bound: delta_local, one block of 16 warps an SM (200 KB of operands): operands are cut, multiplied and added up in phases that wait
+// for one another, and the substitution is a chain of four blocks.  2,048 tokens of 24 heads: 165.6 us with products by mma.sync, two
+// blocks of 8 warps an SM; 123.7 on tcgen05.  On the way: the substitution of all 64 rows written out took 33,000 cycles (40 KB of
+// code, the instruction cache), one by one in a loop 11,000, by blocks of 16 with products behind them 4,000.  delta_rule.cu's three
+// kernels take 658 us there, these with the norm 189.
+// Error against 64 bits (2-norm, 2,048 tokens), products by mma.sync and these: state 5.43e-7 and 5.43e-7, outputs 5.10e-7 and 5.09e-7.
+// Scan and products by mma.sync: parameters where trained models have them 5.2e-7 and 4.6e-7, decays near one 1.76e-6 and 1.70e-6,
+// random ones 0.95e-7 and 1.00e-7.
 #include "parts_tcgen05.cuh"
 
 namespace ifx {

@@ -17,7 +17,7 @@
 // batch.
 //
 // Long spans of a bfloat16 run go to delta_chunks.cu instead of delta_scan (delta_stretches_pay in ops.py), where stretches of 64
-// tokens are products on the tensor cores; preparation and finish are these.
+// tokens are products on the tensor cores; norm and gate (pair_mixer.cu) are the same.
 #include "common.cuh"
 
 namespace ifx {

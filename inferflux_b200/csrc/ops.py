@@ -174,7 +174,7 @@ class CudaKernels:
                   ("ifx_delta_rule_scratch_floats", "ifx_chunk_scan_scratch_floats", "ifx_delta_chunks_scratch_floats",
                    "ifx_attention_prefill_tcgen05_parts_bytes", "ifx_gemm_f32_split_scratch", "ifx_moe_sorted_scratch",
                    "ifx_sample_scratch_bytes", "ifx_latent_attention_mma_workspace", "ifx_layer_workspace_bytes"))
-        # long spans of a bfloat16 run's recurrences by stretches of 64 tokens (0: token after token, for comparisons)
+        # long spans of a bfloat16 run's recurrences by stretches of 64 or 128 tokens (0: token after token, for comparisons)
         self.chunk_scans = os.environ.get("INFERFLUX_B200_CHUNK_SCANS", "1") != "0"
         self._latent_sizes = {}
         # latent attention on the tensor-core tiles (0: the per-token kernel, for comparisons)
@@ -1499,9 +1499,9 @@ class CudaKernels:
         self.launches += 1
         return out
 
-    # Spans of this many tokens and more can go by stretches of 64 tokens in a bfloat16 run (csrc/chunk_scan.cu, delta_chunks.cu).  The
-    # other spans of the same step then go along, or through the scans token by token in launches of their own: a stretch costs the
-    # same with one token as with 64.
+    # Spans of this many tokens and more can go by stretches of 64 tokens in a bfloat16 run (csrc/chunk_scan.cu, delta_chunks.cu), of 128
+    # with one decay per head (csrc/chunk_tcgen05.cu).  The other spans of the same step then go along, or through the scans token by
+    # token in launches of their own: a stretch costs the same with one token as with all of them.
     CHUNK_SCAN_MIN_SPAN = 128
 
     def _long_spans(self, ctx):
