@@ -148,6 +148,7 @@ struct PrefillLayout {
 // full = its blocks.  (28 heads x 11 items on 148 SMs are two rounds and 12 blocks, which alone took a third round.)
 struct PrefillParts {
   int full, parts;
+  int halves;                // 1: the grid has a block for each of an item's query tiles (parts is 1)
   float* o;                  // [left over x parts][256][D]
   float2* ml;                // [left over x parts][256]: reference in units of log2, sum
 };
@@ -193,8 +194,14 @@ struct PrefillItem {
       block = split.full + slot / split.parts;
       part = slot % split.parts;
     }
+    int half = 0;                                          // (an item's second tile sees more keys: it goes first)
+    if (split.halves) {
+      half = 1 - block / nq % 2;
+      block = block / (2 * nq) * nq + block % nq;
+    }
     const int* tile = tiles + (size_t)(num_tiles - 1 - block / nq) * 4;
-    r = tile[0], row0 = tile[1], rows = tile[2], pos0 = tile[3];
+    r = tile[0], row0 = tile[1] + half * kBM, rows = tile[2] - half * kBM, pos0 = tile[3] + half * kBM;
+    if (split.halves) rows = min(max(rows, 0), kBM);
     h = block % nq;
     rows_1 = max(rows - kBM, 0);
     tb_0 = window.first(pos0) / kBN;
@@ -209,6 +216,7 @@ struct PrefillItem {
       tb_1 = max(lo, min(tb_1, hi));
       te_1 = max(tb_1, min(te_1, hi));
     }
+    if (rows == 0) te_0 = tb_0;                            // a second query tile that is not there
     te = max(te_0, te_1);
     // Key tiles are visited in order: with kept keys first [0, nk), then [tb_0, te); query tile q uses those that hold kept keys
     // and those of its own window.
@@ -222,7 +230,7 @@ struct PrefillItem {
     if (KEPT && kt < keep_tiles && kt < te_0 && (q == 0 || rows_1 > 0)) return true;      // (kept keys lie in front of te_0)
     return q == 0 ? (kt >= tb_0 && kt < te_0) : (kt >= tb_1 && kt < te_1);
   }
-  __device__ __forceinline__ bool has(int q) const { return q == 0 || rows_1 > 0; }
+  __device__ __forceinline__ bool has(int q) const { return q == 0 ? rows > 0 : rows_1 > 0; }
 };
 
 template <int D, bool KEPT>
@@ -716,7 +724,7 @@ static int launch_prefill_tcgen05(const bf16* q, int num_tokens, const bf16* kv_
     configured = true;
   }
   const int blocks = nq * num_tiles, left = parts > 1 ? blocks % kSms : 0;
-  PrefillParts split{blocks - left, parts, (float*)workspace, nullptr};
+  PrefillParts split{parts == -1 ? 2 * blocks : blocks - left, parts, parts == -1, (float*)workspace, nullptr};
   if (left) split.ml = reinterpret_cast<float2*>(split.o + (size_t)left * parts * 2 * kBM * D);
   rc = launch_pdl(attn_prefill_tcgen05_kernel<D, KEPT>, dim3(split.full + left * parts), dim3(kThreads), smem, stream, 1, q_map,
                   pool_map, block_table, tiles, req_slot, out, nq, nkv, page_size, page_shift, max_blocks,
@@ -786,17 +794,18 @@ long long ifx_attention_prefill_tcgen05_parts_bytes(int num_tiles, int nq, int d
   return parts > 1 ? (long long)((long long)num_tiles * nq % kSms) * parts * 2 * kBM * (d + 2) * 4 : 0;
 }
 
-// The plain form with the blocks left over behind whole rounds cut into `parts` parts of their keys (1: none; two launches with more).
+// The plain form with the blocks left over behind whole rounds cut into `parts` parts of their keys (1: none; two launches with more), or
+// (-1) with a block for each 128 rows.
 int ifx_attention_prefill_tcgen05_parts(const void* q, int num_tokens, const void* kv_pool, const int* block_table, const int* tiles,
                                         const int* req_slot, void* out, int num_tiles, int nq, int nkv, int d, int page_size,
                                         int max_blocks, int num_pages, int window, float scale, int parts, void* workspace,
                                         int* error_flag, cudaStream_t stream) {
-  if (parts <= 1)
+  if (parts <= 1 && parts != -1)
     return ifx_attention_prefill_tcgen05(q, num_tokens, kv_pool, block_table, tiles, req_slot, out, num_tiles, nq, nkv, d, page_size,
                                          max_blocks, num_pages, window, scale, error_flag, stream);
   if (num_tiles <= 0) return 0;
   if (!ifx_attention_prefill_tcgen05_supports(d, page_size) || nq <= 0 || nkv <= 0 || nq % nkv || max_blocks <= 0 || num_tiles > 65535 ||
-      !(scale > 0.0f) || error_flag == nullptr || parts > 16 || workspace == nullptr || (uintptr_t)workspace % 16)
+      !(scale > 0.0f) || error_flag == nullptr || parts > 16 || (parts > 1 && (workspace == nullptr || (uintptr_t)workspace % 16)))
     return IFX_E_BADARG;
   int ps = 0;
   while ((1 << ps) < page_size) ++ps;

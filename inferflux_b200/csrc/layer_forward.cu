@@ -75,7 +75,7 @@ struct IfxLayerIO {
   void* out_tensor;           // this layer's last delta, unadded: one of the two forms again
   float* out_parts;
   int out_splits, launches, library_calls;
-  int prefill_parts;          // in: parts of the prompt attention's left over blocks (CudaKernels.prefill_parts)
+  int prefill_parts;          // in: parts of the prompt attention's left over blocks, or -1 (CudaKernels.prefill_cut)
   int least_decode_splits, pad0;   // in: parts of a decoded token's keys at least (CudaKernels.least_decode_splits)
 };
 
@@ -314,7 +314,7 @@ extern "C" int ifx_layer_forward(const IfxStepArgs* s, const IfxLayerArgs* l, If
         if (bytes && !room) return IFX_E_TOOBIG;
         RUN(ifx_attention_prefill_tcgen05_parts(q, T, l->kv_pool, l->block_table, s->prefill_tiles, s->req_slot, attn, s->num_tiles, nq,
                                                 nkv, d, l->page_size, l->max_blocks, l->num_pages, l->window, l->scale,
-                                                bytes ? io->prefill_parts : 1, room, s->error_flag, st));
+                                                bytes || io->prefill_parts < 0 ? io->prefill_parts : 1, room, s->error_flag, st));
         if (bytes) ++io->launches;
       } else
         RUN(ifx_attention_prefill_bf16(q, l->kv_pool, l->block_table, s->prefill_tiles, s->req_slot, attn, s->num_tiles, nq,

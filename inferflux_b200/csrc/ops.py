@@ -724,7 +724,7 @@ class CudaKernels:
         parity = self._layer_parity = 1 - self._layer_parity
         io.parity = parity
         io.least_decode_splits = self.least_decode_splits(ctx, ctx.extra_len.get("attn.decode_rows", 0), m.nkv, m.d, int(m.window or 0))
-        io.prefill_parts = self.prefill_parts(ctx, m.nq, int(m.window or 0))
+        io.prefill_parts = self.prefill_cut(ctx, m.nq, int(m.window or 0))
         io.ws, io.ws_bytes = ws.data_ptr(), ws.numel()
         rc = self.lib.ifx_layer_forward(step, layer, self._layer_io_ref, ctypes.c_void_p(_stream()))
         self.launches += io.launches
@@ -893,7 +893,7 @@ class CudaKernels:
             return out
         if num_tiles and self.tensor_core_prefill and self.lib.ifx_attention_prefill_tcgen05_supports(
                 d, cache.page_size):
-            parts = self.prefill_parts(ctx, nq, win)
+            parts = self.prefill_cut(ctx, nq, win)
             room = None
             if parts > 1:
                 room = torch.empty(self.prefill_parts_bytes(num_tiles, nq, d, parts), dtype=torch.uint8, device=q.device)
@@ -937,6 +937,27 @@ class CudaKernels:
         if parts is None:
             parts = known[nq, window] = self._prefill_parts(ctx, nq, window)
         return parts
+
+    def prefill_cut(self, ctx, nq, window):
+        """What the kernel is told: prefill_parts, or -1 for a block for each 128 rows; found once a step and kind of layer."""
+        known = ctx.__dict__.setdefault("prefill_parts", {})
+        cut = known.get((nq, window, "cut"))
+        if cut is None:
+            cut = self.prefill_parts(ctx, nq, window)
+            if cut == 1 and self._prefill_by_tiles(ctx, nq):
+                cut = -1
+            known[nq, window, "cut"] = cut
+        return cut
+
+    @staticmethod
+    def _prefill_by_tiles(ctx, nq):
+        """Whether each 128 rows get a block of their own instead of 256 rows: while all of those fit on the SMs at once.  A key tile takes
+        one query tile as long as two (1.6 us: hand-overs between products and exponentials), but the second tile's last keys and its
+        output come behind the first one's.  us, 256 and 128 rows a block: 12 heads, 447 tokens 14.2 and 12.4, 1,000 20.7 and 18.9,
+        four times 256 behind 700 21.9 and 19.5; 28 heads, 300 behind 500 17.9 and 17.5; heads of 64, 16 of them, 1,000 tokens 19.6
+        and 16.4.  With more blocks than SMs: four times 300 tokens of 12 heads 11.2 and 12.4, 1,000 of 28 21.4 and 21.8, behind 2,000
+        48.8 and 69.7 (one long prompt gains, its last blocks alone being long: 2,000 of 12 heads 33.8 and 30.9)."""
+        return sum(-(-n // 128) for _s, n in ctx.spans if n > 1) * nq <= 148
 
     def _prefill_parts(self, ctx, nq, window):
         """A block takes up to 256 tokens of a head and an SM to itself, so what is left behind whole rounds of 148 blocks leaves SMs idle

@@ -50,3 +50,22 @@ def test_blocks_behind_one_another(cuda_kernels, d, window, keep):
         else:                                       # (a decoded token's keys are cut by how many tokens there are)
             assert (got[0][rows].float() - want.float()).abs().max() <= 2 ** -6
     cuda_kernels.check_errors()
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("window", [None, 200])
+@pytest.mark.parametrize("lens,spans", [([300], [257]), ([128, 129, 700, 5], [128, 129, 130, 1]), ([1000], [1000]), ([60, 256], [60, 256])])
+def test_a_block_for_each_128_rows(cuda_kernels, monkeypatch, d, window, lens, spans):
+    """The same bits as with 256 rows a block; second query tiles that are there, of one row, and not there."""
+    nq, nkv, page = 12, 4, 16
+    ctx, cache, slots = make_cache_case(torch.bfloat16, nkv, d, page, lens, spans, num_pages=sum(-(-n // page) for n in lens) + 3, seed=3)
+    fill_cache(cache, lens, slots, nkv, d, torch.bfloat16, seed=4)
+    assert cuda_kernels.prefill_parts(ctx, nq, window or 0) == 1 and cuda_kernels.prefill_cut(ctx, nq, window or 0) == -1
+    q = torch.randn(ctx.num_tokens, nq * d, generator=torch.Generator().manual_seed(5)).bfloat16().to(DEV)
+    args = (nq, nkv, d, window, 2.0 / math.sqrt(d), ctx, cache)
+    got = cuda_kernels.attention(q, *args)
+    monkeypatch.setattr(type(cuda_kernels), "_prefill_by_tiles", staticmethod(lambda ctx, nq: False))
+    ctx.__dict__.pop("prefill_parts")
+    assert cuda_kernels.prefill_cut(ctx, nq, window or 0) == 1
+    assert torch.equal(got, cuda_kernels.attention(q, *args))
+    cuda_kernels.check_errors()
