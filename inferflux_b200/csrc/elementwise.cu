@@ -493,10 +493,12 @@ int ifx_rmsnorm(float* x, const void* delta, const float* w, void* out, int rows
                 int num_splits, int dtype, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (hidden <= 0 || num_splits < 0) return IFX_E_BADARG;
-  // Of the width alone, as the order of a row's sum.  bfloat16: four reads of 16 bytes a thread, and blocks so small that every SM holds a
-  // round of prompt rows (1,531 rows of 1,536 with their sum: 7.1 us with 256 threads a row, so 6.0).
-  const int threads = dtype == IFX_DT_BF16 && hidden >= 512 && hidden <= 8192 ? ((hidden + 15) / 16 + 31) / 32 * 32
-                      : hidden >= 2048 ? 512 : (hidden >= 512 ? 256 : 128);
+  // float32: of the width alone, as the order of a row's sum.  bfloat16, more than the SMs hold at a time: four reads of 16 bytes a thread,
+  // and blocks so small that every SM holds a round of prompt rows.  us with the sum, larger and smaller blocks: 1,536 wide, 8 rows 2.3
+  // and 2.9, 600 3.1 and 3.3, 1,000 4.7 and 3.6, 1,531 5.4 and 4.3; 3,584 wide, 8 rows 2.3 and 2.8, 400 3.5 and 3.4, 600 5.2 and 4.1,
+  // 1,531 9.9 and 8.5.
+  const bool many = dtype == IFX_DT_BF16 && hidden >= 512 && hidden <= 8192 && (long long)rows * hidden >= 1300000;
+  const int threads = many ? ((hidden + 15) / 16 + 31) / 32 * 32 : hidden >= 2048 ? 512 : (hidden >= 512 ? 256 : 128);
   const size_t stride = (size_t)rows * hidden;
 #define IFX_NORM(T, ADD)                                                                                        \
   return launch_pdl(rmsnorm_kernel<T, ADD>, dim3(rows), dim3(threads), 0, stream, 1, x, delta, w, (T*)out, hidden, eps, \
