@@ -518,12 +518,17 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
         for (int c = 0; c < kBN; c += 64) {
           uint32_t packed[32];
 #pragma unroll
-          for (int j = 0; j < 64; j += 2) {
-            const float2 x = fma2(make_float2(s[c + j], s[c + j + 1]), scale2, bias2);
-            const float2 p = make_float2(ex2(x.x), ex2(x.y));
-            sum2[(j >> 1) & 1] = add2(sum2[(j >> 1) & 1], p);
-            __nv_bfloat162 b2 = __floats2bfloat162_rn(p.x, p.y);
-            packed[j >> 1] = *reinterpret_cast<uint32_t*>(&b2);
+          for (int j = 0; j < 64; j += 4) {
+            float pair[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const float2 x = fma2(make_float2(s[c + j + 2 * e], s[c + j + 2 * e + 1]), scale2, bias2);
+              const float2 p = make_float2(ex2(x.x), ex2(x.y));
+              pair[e] = p.x + p.y;
+              __nv_bfloat162 b2 = __floats2bfloat162_rn(p.x, p.y);
+              packed[(j >> 1) + e] = *reinterpret_cast<uint32_t*>(&b2);
+            }
+            sum2[(j >> 2) & 1] = add2(sum2[(j >> 2) & 1], make_float2(pair[0], pair[1]));
           }
           tmem_st32(s_addr + (c >> 1), packed);              // columns whose scores have been read already
           tmem_wait_st();

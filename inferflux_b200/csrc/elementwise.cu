@@ -50,7 +50,9 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, float4 v) {
   *reinterpret_cast<uint2*>(p) = raw;
 }
 
-template <typename T, int ADD>
+// SHARE: a thread does the work of so many threads of a block SHARE times as large, blockDim.x apart, whose sums it keeps apart: the
+// bits are those of the larger block.  (Rows of up to 8 elements for each thread of that one, in whole fours, and no slices to add.)
+template <typename T, int ADD, int SHARE>
 __global__ void rmsnorm_kernel(float* __restrict__ x, const void* __restrict__ delta_raw,
                                const float* __restrict__ w, T* __restrict__ out, int hidden, float eps,
                                int num_splits, size_t split_stride) {
@@ -63,9 +65,9 @@ __global__ void rmsnorm_kernel(float* __restrict__ x, const void* __restrict__ d
   const float* pr = ADD == 2 ? reinterpret_cast<const float*>(delta_raw) + row * hidden : nullptr;
   T* o = out + row * hidden;
   const bool vec = (hidden & 3) == 0;                    // rows start 16-byte aligned then (8-byte for bfloat16)
-  constexpr int KEEP = 4;                                // the row's elements stay in registers between the passes
-  float4 keep[KEEP];
-  float ss = 0.0f;
+  constexpr int KEEP = SHARE > 1 ? 2 : 4;                // the row's elements stay in registers between the passes
+  float4 keep[KEEP][SHARE];
+  float ss = 0.0f, others[SHARE] = {};                   // others: of the threads blockDim.x, 2 blockDim.x ... behind this one
   auto take = [&](int i) -> float4 {                     // x (+ delta) at columns i .. i + 3, written back
     float4 v = *reinterpret_cast<const float4*>(xr + i);
     if (ADD == 1) {
@@ -83,14 +85,40 @@ __global__ void rmsnorm_kernel(float* __restrict__ x, const void* __restrict__ d
     }
     return v;
   };
-  const int step4 = blockDim.x * 4;
-  if (vec) {
+  const int step4 = blockDim.x * 4 * SHARE;
+  if (SHARE > 1) {
+    float4 add[KEEP][SHARE];
+#pragma unroll
+    for (int c = 0; c < KEEP; ++c)
+#pragma unroll
+      for (int g = 0; g < SHARE; ++g) {
+        const int i = (threadIdx.x + g * blockDim.x) * 4 + c * step4;
+        keep[c][g] = i < hidden ? *reinterpret_cast<const float4*>(xr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (ADD == 1) add[c][g] = i < hidden ? load4(dr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    if (ADD == 1)                                        // (every read is on its way before the first write)
+#pragma unroll
+      for (int c = 0; c < KEEP; ++c)
+#pragma unroll
+        for (int g = 0; g < SHARE; ++g) {
+          const int i = (threadIdx.x + g * blockDim.x) * 4 + c * step4;
+          keep[c][g].x += add[c][g].x; keep[c][g].y += add[c][g].y; keep[c][g].z += add[c][g].z; keep[c][g].w += add[c][g].w;
+          if (i < hidden) *reinterpret_cast<float4*>(xr + i) = keep[c][g];
+        }
+#pragma unroll
+    for (int c = 0; c < KEEP; ++c)
+#pragma unroll
+      for (int g = 0; g < SHARE; ++g) {
+        const float4 v = keep[c][g];
+        others[g] += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+      }
+  } else if (vec) {
 #pragma unroll
     for (int c = 0; c < KEEP; ++c) {
       const int i = threadIdx.x * 4 + c * step4;
-      keep[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (i < hidden) keep[c] = take(i);
-      ss += keep[c].x * keep[c].x + keep[c].y * keep[c].y + keep[c].z * keep[c].z + keep[c].w * keep[c].w;
+      keep[c][0] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (i < hidden) keep[c][0] = take(i);
+      ss += keep[c][0].x * keep[c][0].x + keep[c][0].y * keep[c][0].y + keep[c][0].z * keep[c][0].z + keep[c][0].w * keep[c][0].w;
     }
     for (int i = threadIdx.x * 4 + KEEP * step4; i < hidden; i += step4) {
       const float4 v = take(i);
@@ -111,18 +139,30 @@ __global__ void rmsnorm_kernel(float* __restrict__ x, const void* __restrict__ d
       ss += v * v;
     }
   }
-  ss = block_sum(ss, scratch);
+  if (SHARE > 1) {                                       // block_sum of the larger block
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+#pragma unroll
+    for (int g = 0; g < SHARE; ++g) {
+      const float s = warp_sum(others[g]);
+      if (lane == 0) scratch[warp + g * warps] = s;
+    }
+    __syncthreads();
+    ss = warp_sum(lane < SHARE * warps ? scratch[lane] : 0.0f);
+  } else
+    ss = block_sum(ss, scratch);
   const float r = rsqrtf(ss / (float)hidden + eps);
-  if (vec) {
+  if (SHARE > 1 || vec) {
     auto put = [&](int i, float4 v) {
       const float4 wv = *reinterpret_cast<const float4*>(w + i);
       store4(o + i, make_float4(v.x * r * wv.x, v.y * r * wv.y, v.z * r * wv.z, v.w * r * wv.w));
     };
 #pragma unroll
-    for (int c = 0; c < KEEP; ++c) {
-      const int i = threadIdx.x * 4 + c * step4;
-      if (i < hidden) put(i, keep[c]);
-    }
+    for (int c = 0; c < KEEP; ++c)
+#pragma unroll
+      for (int g = 0; g < SHARE; ++g) {
+        const int i = (threadIdx.x + g * blockDim.x) * 4 + c * step4;
+        if (i < hidden) put(i, keep[c][g]);
+      }
     for (int i = threadIdx.x * 4 + KEEP * step4; i < hidden; i += step4) put(i, *reinterpret_cast<const float4*>(xr + i));
   } else {
     for (int i = threadIdx.x; i < hidden; i += blockDim.x) o[i] = from_f32<T>(xr[i] * r * w[i]);
@@ -493,24 +533,28 @@ int ifx_rmsnorm(float* x, const void* delta, const float* w, void* out, int rows
                 int num_splits, int dtype, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (hidden <= 0 || num_splits < 0) return IFX_E_BADARG;
-  // float32: of the width alone, as the order of a row's sum.  bfloat16, more than the SMs hold at a time: four reads of 16 bytes a thread,
-  // and blocks so small that every SM holds a round of prompt rows.  us with the sum, larger and smaller blocks: 1,536 wide, 8 rows 2.3
-  // and 2.9, 600 3.1 and 3.3, 1,000 4.7 and 3.6, 1,531 5.4 and 4.3; 3,584 wide, 8 rows 2.3 and 2.8, 400 3.5 and 3.4, 600 5.2 and 4.1,
-  // 1,531 9.9 and 8.5.
-  const bool many = dtype == IFX_DT_BF16 && hidden >= 512 && hidden <= 8192 && (long long)rows * hidden >= 1300000;
-  const int threads = many ? ((hidden + 15) / 16 + 31) / 32 * 32 : hidden >= 2048 ? 512 : (hidden >= 512 ? 256 : 128);
+  // Of the width alone, as the order of a row's sum.
+  const int threads = hidden >= 2048 ? 512 : (hidden >= 512 ? 256 : 128);
+  // More rows than the SMs hold at a time: half as many threads with twice the reads each, so that every SM holds a round of prompt rows.
+  // us with the sum, before and with them: 1,536 wide, 600 rows 2.8 (not so many), 1,000 4.5 and 3.3, 1,531 5.2 and 4.2; 3,584 wide,
+  // 400 rows 3.7 and 3.6, 600 5.3 and 4.2, 1,000 7.6 and 7.6, 1,531 10.0 and 8.7; below the line they take 0.3 to 0.6 longer.
+  const bool many = dtype == IFX_DT_BF16 && num_splits == 0 && hidden >= 512 && hidden <= 4096 && hidden % 4 == 0 &&
+                    (long long)rows * hidden >= 1300000;
   const size_t stride = (size_t)rows * hidden;
-#define IFX_NORM(T, ADD)                                                                                        \
-  return launch_pdl(rmsnorm_kernel<T, ADD>, dim3(rows), dim3(threads), 0, stream, 1, x, delta, w, (T*)out, hidden, eps, \
+#define IFX_NORM(T, ADD, SHARE)                                                                                             \
+  return launch_pdl(rmsnorm_kernel<T, ADD, SHARE>, dim3(rows), dim3(threads / SHARE), 0, stream, 1, x, delta, w, (T*)out, hidden, eps, \
                     num_splits, stride)
   if (dtype == IFX_DT_F32) {
-    if (!delta) IFX_NORM(float, 0);
-    else if (num_splits > 0) IFX_NORM(float, 2);
-    else IFX_NORM(float, 1);
+    if (!delta) IFX_NORM(float, 0, 1);
+    else if (num_splits > 0) IFX_NORM(float, 2, 1);
+    else IFX_NORM(float, 1, 1);
+  } else if (many) {
+    if (!delta) IFX_NORM(__nv_bfloat16, 0, 2);
+    else IFX_NORM(__nv_bfloat16, 1, 2);
   } else if (dtype == IFX_DT_BF16) {
-    if (!delta) IFX_NORM(__nv_bfloat16, 0);
-    else if (num_splits > 0) IFX_NORM(__nv_bfloat16, 2);
-    else IFX_NORM(__nv_bfloat16, 1);
+    if (!delta) IFX_NORM(__nv_bfloat16, 0, 1);
+    else if (num_splits > 0) IFX_NORM(__nv_bfloat16, 2, 1);
+    else IFX_NORM(__nv_bfloat16, 1, 1);
   }
 #undef IFX_NORM
   return IFX_E_DTYPE;

@@ -327,11 +327,16 @@ __global__ void __launch_bounds__(kLpThreads, 1) latent_prompt_kernel(
       float2 sum2[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
       uint32_t packed[32];
 #pragma unroll
-      for (int j = 0; j < 64; j += 2) {                                // two scores an instruction
-        const float2 x = fma2(make_float2(s[j], s[j + 1]), scale2, bias2), p = make_float2(lp_ex2(x.x), lp_ex2(x.y));
-        sum2[(j >> 1) & 1] = add2(sum2[(j >> 1) & 1], p);
-        __nv_bfloat162 b2 = __floats2bfloat162_rn(p.x, p.y);
-        packed[j >> 1] = *reinterpret_cast<uint32_t*>(&b2);
+      for (int j = 0; j < 64; j += 4) {                                // two scores an instruction
+        float2 p[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float2 x = fma2(make_float2(s[j + 2 * e], s[j + 2 * e + 1]), scale2, bias2);
+          p[e] = make_float2(lp_ex2(x.x), lp_ex2(x.y));
+          __nv_bfloat162 b2 = __floats2bfloat162_rn(p[e].x, p[e].y);
+          packed[(j >> 1) + e] = *reinterpret_cast<uint32_t*>(&b2);
+        }
+        sum2[(j >> 2) & 1] = add2(sum2[(j >> 2) & 1], add2(make_float2(p[0].x, p[1].x), make_float2(p[0].y, p[1].y)));
       }
       lp_st32(s_addr + half * 32, packed);                             // columns whose scores both halves have read
       l_run += (sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y);
