@@ -34,9 +34,10 @@
 //
 // Bound: the tensor pipe: a key tile takes a block 1.87 us at the 1.65 GHz that the SMs keep under it, 1.3 PFLOP/s while a block
 // walks its keys; the rest is heads and tails of blocks.  Blocks behind one another, whole rows of output, registers for the scores
-// and two scores an instruction, us: 2,500 tokens of 28 heads behind 4,000 149 -> 132, behind none 61 -> 52; 2,200 in five prompts
-// 38.7 -> 30.7; 900 of 12 heads behind 1,500 (one round) 20.1 -> 17.3, 447 behind none 16.0 -> 13.8.  A quarter of the
-// exponentials by multiply-adds was slower (149 -> 153), probabilities of the first 96 keys instead of 64 handed over first the same.
+// and two scores an instruction, us: 2,500 tokens of 28 heads behind 4,000 153 -> 139, behind none 61 -> 55; 2,200 in five prompts
+// 38.5 -> 31.3; 900 of 12 heads behind 1,500 (one round) 20.5 -> 18.3, eight layers of 1,531 in three prompts 146 -> 127.  A quarter of
+// the exponentials by multiply-adds was slower (149 -> 153), probabilities of the first 96 keys instead of 64 handed over first the same,
+// sums of probabilities two an instruction in another order 2 % faster.
 // A warp in step issues the products, one lane of it by predicate: with a single thread in a
 // branch of its own a product took 108 clocks to issue instead of 65 (2,500 tokens behind 4,000, 28 heads: 211 us, then 192).
 // A row's 128 scores stay in registers between the maximum and the exponentials (they were read twice), and the product with the
