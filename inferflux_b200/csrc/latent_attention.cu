@@ -61,6 +61,9 @@ __global__ void latent_norm_append_kernel(const T* __restrict__ rows, int ld, in
 }
 
 // ------------------------------------------------- norm + rotation + append
+// x cos + y sin, rounded in one way wherever a row lies.
+__device__ __forceinline__ float turned(float x, float c, float y, float s) { return fmaf(x, c, __fmul_rn(y, s)); }
+
 // A warp per token and stretch of `per` heads (blockIdx.y; the first stretch's also makes the cached row and the gates).  The
 // cached row is [c; k_t]: c = x / rms(x) * w over `lat` columns starting at `col0` of `rows`,
 // k_t the `rot` columns behind them turned by the token's position.  Every query head's last `rot` elements (heads of
@@ -82,7 +85,7 @@ __device__ __forceinline__ void turn_store(const T* src, T* dst, int rot, int ro
       const int i = interleaved ? (e >> 1) : (e < half ? e : e - half);
       const bool first = interleaved ? !(e & 1) : e < half;
       const float m = held[interleaved ? (e ^ 1) : (first ? e + half : e - half)];
-      v = first ? v * cs[i] - m * cs[half + i] : v * cs[i] + m * cs[half + i];
+      v = turned(v, cs[i], first ? -m : m, cs[half + i]);
     }
     dst[e] = from_f32<T>(v);
   }
@@ -139,14 +142,15 @@ __global__ void latent_rope_append_kernel(const T* __restrict__ rows, int ld, in
 }
 
 // The two above for bfloat16 rows on 16-byte boundaries.  Eight numbers a read, a row's in registers from the sum to the store; a lane
-// keeps its pair of turned elements and their angle and has four heads' pairs on their way.
+// keeps its pair of turned elements and their angle and has four heads' pairs on their way.  The squares are added up in the order of
+// the kernels above (a lane every 32nd number, by way of shared memory), so a row's bits do not depend on where it lies.
 // Bound: HBM and the latency of few tokens' reads.  2,048 tokens, 1,536 numbers normed: 9.0 us a number at a time, so 5.2; 64 of 12
 // heads' numbers turned beside latents of 256: 10.7, so 6.5.  64 decoded tokens: 7 us less for the two in their chain.
 constexpr int kLatentKept = 8;                           // reads of a lane: rows of up to 2,048
 template <int KEPT>
 __device__ __forceinline__ void latent_norm_row(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w, float eps, int rank,
-                                                __nv_bfloat16* dst, __nv_bfloat16* also, int lane) {
-  uint4 raw[KEPT];
+                                                __nv_bfloat16* dst, __nv_bfloat16* also, uint4* held, int lane) {
+  uint4 raw[KEPT];                                       // held: the warp's room for KEPT * 32 of them
   float ss = 0.0f;
 #pragma unroll
   for (int k = 0; k < KEPT; ++k) {
@@ -155,14 +159,12 @@ __device__ __forceinline__ void latent_norm_row(const __nv_bfloat16* __restrict_
     if (e < rank) raw[k] = *reinterpret_cast<const uint4*>(x + e);
   }
 #pragma unroll
-  for (int k = 0; k < KEPT; ++k) {
-    const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(&raw[k]);
+  for (int k = 0; k < KEPT; ++k) held[lane + 32 * k] = raw[k];
+  __syncwarp();
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 v = __bfloat1622float2(b[i]);
-      ss = fmaf(v.x, v.x, ss);
-      ss = fmaf(v.y, v.y, ss);
-    }
+  for (int k = 0; k < 8 * KEPT; ++k) {                   // (zeros behind the row change no sum)
+    const float v = to_f32(reinterpret_cast<const __nv_bfloat16*>(held)[lane + 32 * k]);
+    ss = fmaf(v, v, ss);
   }
   ss = warp_sum(ss);
   const float r = rsqrtf(ss / (float)rank + eps);
@@ -190,6 +192,7 @@ __global__ void __launch_bounds__(128) latent_norm_append_vec_kernel(
     const __nv_bfloat16* __restrict__ rows, int ld, int col0, const float* __restrict__ w, float eps, const int* __restrict__ positions,
     const int* __restrict__ token_req, const int* __restrict__ req_slot, const int* __restrict__ block_table, int max_blocks, int page_size,
     int num_pages, __nv_bfloat16* __restrict__ pool, __nv_bfloat16* __restrict__ c_out, int num_tokens, int rank) {
+  __shared__ uint4 held[4][KEPT * 32];
   const int t = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   pdl_launch_dependents();
   pdl_wait();
@@ -199,7 +202,8 @@ __global__ void __launch_bounds__(128) latent_norm_append_vec_kernel(
     const int pos = positions[t], slot = req_slot[token_req[t]], page = block_table[(size_t)slot * max_blocks + pos / page_size];
     if (page >= 0 && page < num_pages) dst = pool + ((size_t)page * page_size + pos % page_size) * rank;
   }
-  latent_norm_row<KEPT>(rows + (size_t)t * ld + col0, w, eps, rank, dst, c_out ? c_out + (size_t)t * rank : nullptr, lane);
+  latent_norm_row<KEPT>(rows + (size_t)t * ld + col0, w, eps, rank, dst, c_out ? c_out + (size_t)t * rank : nullptr,
+                        held[threadIdx.x >> 5], lane);
 }
 
 // rot <= 64: a pair of elements a lane.
@@ -209,6 +213,7 @@ __global__ void __launch_bounds__(128) latent_rope_append_vec_kernel(
     float magnitude, const int* __restrict__ positions, const int* __restrict__ token_req, const int* __restrict__ req_slot,
     const int* __restrict__ block_table, int max_blocks, int page_size, int num_pages, __nv_bfloat16* __restrict__ pool, int num_tokens,
     int lat, int rot, int heads, int dim, float* __restrict__ gate_out, int gate_col, int per) {
+  __shared__ uint4 held[4][2 * 32];
   const int t = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   pdl_launch_dependents();
   const int half = rot_used >> 1, h_end = min(heads, (int)(blockIdx.y + 1) * per);
@@ -227,7 +232,7 @@ __global__ void __launch_bounds__(128) latent_rope_append_vec_kernel(
   }
   auto turn = [&](__nv_bfloat16 a, __nv_bfloat16 b, __nv_bfloat16* to) {
     const float x = to_f32(a), y = to_f32(b);
-    const float rx = turns ? x * c - y * s : x, ry = turns ? y * c + x * s : y;
+    const float rx = turns ? turned(x, c, -y, s) : x, ry = turns ? turned(y, c, x, s) : y;
     const __nv_bfloat16 u = from_f32<__nv_bfloat16>(rx), v = from_f32<__nv_bfloat16>(ry);
     if (e1 == e0 + 1) {
       *reinterpret_cast<__nv_bfloat162*>(to + e0) = __nv_bfloat162(u, v);
@@ -257,7 +262,7 @@ __global__ void __launch_bounds__(128) latent_rope_append_vec_kernel(
         __nv_bfloat16* dst = pool + ((size_t)page * page_size + pos % page_size) * (lat + rot);
         __nv_bfloat16 a, b;
         if (live) fetch(x + lat, a, b);
-        latent_norm_row<2>(x, w, eps, lat, dst, nullptr, lane);
+        latent_norm_row<2>(x, w, eps, lat, dst, nullptr, held[threadIdx.x >> 5], lane);
         if (live) turn(a, b, dst + lat);
       }
     }

@@ -119,3 +119,36 @@ def test_turned_latents(cuda_kernels, rot, used, interleaved, heads, lat):
     pos, slot = ctx.positions.cpu().long(), torch.tensor([1] * 3 + [0] * 150)
     held = kv.cpu().view(20, page, -1)[table.cpu()[slot, pos // page].long(), pos % page]
     _close(held, row, torch.bfloat16)
+
+
+@pytest.mark.parametrize("rank", [8, 256, 264, 512, 520, 1536, 2040, 2048])
+def test_a_normed_row_has_its_bits_wherever_it_lies(cuda_kernels, rank):
+    """Rows on 16-byte boundaries and the same rows off them: one order of sums.  (700 rows: a sum in another order rounds some of their
+    numbers differently.)"""
+    g = torch.Generator().manual_seed(rank)
+    rows, w = torch.randn(700, rank, generator=g).to(torch.bfloat16), (1 + 0.2 * torch.randn(rank, generator=g)).to(DEV)
+    off = torch.zeros(700, rank + 1, dtype=torch.bfloat16)
+    off[:, 1:] = rows
+    assert torch.equal(cuda_kernels.rmsnorm_columns(rows.to(DEV), 0, rank, w, 1e-6), cuda_kernels.rmsnorm_columns(off.to(DEV), 1, rank, w, 1e-6))
+
+
+@pytest.mark.parametrize("rot,used,interleaved", [(0, 0, False), (64, 64, True), (64, 32, False), (8, 2, False)])
+@pytest.mark.parametrize("lat", [8, 256, 504, 512])
+def test_a_turned_latent_has_its_bits_wherever_it_lies(cuda_kernels, rot, used, interleaved, lat):
+    from types import SimpleNamespace
+    g = torch.Generator().manual_seed(rot + lat)
+    T, heads, dim, page = 700, 5, 64, 16
+    rows, q = torch.randn(T, lat + rot, generator=g).to(torch.bfloat16), torch.randn(T, heads * (dim + rot), generator=g).to(torch.bfloat16)
+    off = torch.zeros(T, lat + rot + 1, dtype=torch.bfloat16)
+    off[:, 1:] = rows
+    w, freq = (1 + 0.2 * torch.randn(lat, generator=g)).to(DEV), (10.0 ** (-4 * torch.arange(used // 2) / max(1, used // 2))).to(DEV)
+    ctx = _Ctx([(31, T)], [0], DEV)
+    table = torch.arange(46, dtype=torch.int32, device=DEV).view(1, 46)
+    rotary = SimpleNamespace(rotary_dim=used, interleaved=interleaved, magnitude=0.75, inv_freq=freq) if used else None
+    results = []
+    for x, col0 in ((rows, 0), (off, 1)):
+        kv = torch.zeros(46, 1, 1, page, lat + rot, dtype=torch.bfloat16, device=DEV)
+        turned = cuda_kernels.latent_rope_append(x.to(DEV), col0, lat, rot, w, 1e-6, q.to(DEV), heads, dim, rotary, ctx,
+                                                 SimpleNamespace(kv=kv, block_table=table, writes=True, page_size=page))
+        results.append((turned, kv))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
