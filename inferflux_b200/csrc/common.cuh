@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "key_mask.cuh"
+
 #define IFX_DT_F32 0
 #define IFX_DT_BF16 1
 
@@ -77,28 +79,6 @@ inline int launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t sm
   cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
   return e == cudaSuccess ? 0 : (int)e;
 }
-
-// Which keys a query sees besides "not later than itself": the last `window` of them (> 0), only those of its own
-// stretch of `chunk` positions (> 0), or both; the first `keep` keys of a sequence stay visible whatever the window or the
-// stretch.  A query's keys are therefore [0, kept(first)) and [first, pos].  `sink`: the softmax's denominator holds one more unit, a key of score 0
-// that brings no value; with `sink_values` (one learned number per query head) the unit is exp(that number) instead.
-struct KeyMask {
-  int window, chunk, sink;
-  const float* sink_values;
-  int keep;
-  // the sink's score in units of log2, for kernels that keep maxima and sums as powers of two
-  __device__ __forceinline__ float sink_log2(int head) const {
-    return sink_values ? sink_values[head] * 1.4426950408889634f : 0.0f;
-  }
-  __device__ __forceinline__ int first(int pos) const {          // the first key the query at `pos` sees
-    int f = window > 0 ? max(0, pos - window + 1) : 0;
-    if (chunk > 0) f = max(f, pos / chunk * chunk);
-    return f;
-  }
-  __device__ __forceinline__ bool any() const { return window > 0 || chunk > 0; }
-  __device__ __forceinline__ int kept(int first) const { return min(keep, first); }      // keys in front of `first` that stay
-  __device__ __forceinline__ bool sees(int key, int first) const { return key >= first || key < keep; }
-};
 
 // What happens to a head's finished sum of values before it is rounded and stored.
 // Values that were turned by their own position before they were summed: the sum is turned back by the query's.  `table`
