@@ -123,7 +123,7 @@ constexpr int kSms = 148;                  // blocks of a round: one an SM
 constexpr float kRescaleStep = 8.0f;      // log2 units the maximum may outgrow its reference before O is rescaled
 constexpr uint32_t kTmemCols = 512;       // per query tile: scores (128 columns) and output (head size)
 constexpr int kThreads = 384;             // fetch warp, MMA warp, two that rest, two softmax groups of four warps
-constexpr int kNextSlots = 4;             // answers about the next block that are kept (see next_block)
+constexpr int kNextSlots = 4;             // answers about the next block that are kept (see next_of)
 // Registers a thread: the launch's 168 x 384 shared out anew, the softmax groups' 256 threads 208 and the others 88.
 constexpr int kRegsSoftmax = 208, kRegsOther = 88;
 static_assert(256 * kRegsSoftmax + 128 * kRegsOther <= 168 * kThreads, "no more than the block was launched with");
@@ -135,10 +135,10 @@ struct PrefillLayout {
   static constexpr uint32_t Q_BYTES = HALVES * kBM * 128;     // one query tile: [half][128 rows][128 B]
   static constexpr uint32_t SLOT_BYTES = HALVES * kBN * 128;  // the keys or the values of one tile
   // barriers: queries there, their place free again, slots there and free, scores, probabilities of the first keys and of all,
-  // output, the next block's number
+  // output, the next block's number there and read by every role
   static constexpr int B_Q = 0, B_Q_FREE = B_Q + 2, B_FULL = B_Q_FREE + 2, B_EMPTY = B_FULL + SLOTS, B_S_FULL = B_EMPTY + SLOTS,
                        B_P_HALF = B_S_FULL + 2, B_P_FULL = B_P_HALF + 2, B_O_FULL = B_P_FULL + 2, B_NEXT = B_O_FULL + 2,
-                       B_COUNT = B_NEXT + kNextSlots;
+                       B_NEXT_FREE = B_NEXT + kNextSlots, B_COUNT = B_NEXT_FREE + kNextSlots;
   static constexpr size_t SMEM = 1024 + 2 * Q_BYTES + (size_t)SLOTS * SLOT_BYTES + kNextSlots * 16 + B_COUNT * 8 + 16;
 };
 
@@ -202,7 +202,10 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
       mbar_init(bar(L::B_P_FULL + q), 4);
       mbar_init(bar(L::B_O_FULL + q), 1);
     }
-    for (int s = 0; s < kNextSlots; ++s) mbar_init(bar(L::B_NEXT + s), 1);
+    for (int s = 0; s < kNextSlots; ++s) {
+      mbar_init(bar(L::B_NEXT + s), 1);
+      mbar_init(bar(L::B_NEXT_FREE + s), 9);               // the MMA warp and the softmax groups' eight
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -218,9 +221,14 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
   const uint32_t tmem_s = tmem_base, tmem_o = tmem_base + 2 * kBN;       // S of tile q: + q * 128; O: + q * D
   pdl_wait();
 
-  // Every role goes through the same blocks: this one, then those that the fetching warp takes off the grid.
+  // Every role goes through the same blocks: this one, then those that the fetching warp takes off the grid.  An answer's place is
+  // free for the fourth one behind it when all others have read it: a softmax group without rows may be that far behind.
   auto next_of = [&](int n, bool& ok) {                    // the block behind the n-th
     return next_block(next_s + (n % kNextSlots) * 16, bar(L::B_NEXT + n % kNextSlots), (n / kNextSlots) & 1, ok);
+  };
+  auto next_read = [&](int n) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar(L::B_NEXT_FREE + n % kNextSlots));
   };
 
   if (warp < 4) {
@@ -283,6 +291,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
         base += 2 * it.visits();
         // the next block is taken when this one's last tiles are on their way: late, so that SMs that are done sooner take more
         block = -1;
+        if (ok && n >= kNextSlots) ok = __all_sync(0xffffffffu, mbar_wait(bar(L::B_NEXT_FREE + n % kNextSlots), (n / kNextSlots - 1) & 1));
         if (ok) {
           if (lane == 0) take_next_block(next_s + (n % kNextSlots) * 16, bar(L::B_NEXT + n % kNextSlots));
           __syncwarp();
@@ -364,7 +373,10 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
         }
         base += 2 * it.visits();
         block = -1;
-        if (ok) block = next_of(n, ok);
+        if (ok) {
+          block = next_of(n, ok);
+          next_read(n);
+        }
       }
       if (!ok && lane == 0) atomicExch(error_flag, 8);
       __syncwarp();
@@ -584,6 +596,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
       }
       tc_fence_before();
       block = next_of(n, ok);
+      next_read(n);
       if (!ok && lane == 0) atomicExch(error_flag, 9);
     }
   }

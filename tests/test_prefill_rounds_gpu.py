@@ -1,6 +1,7 @@
 """Prompt attention of more blocks than SMs: a resident block that goes through several blocks of the grid gives every one of them
 the bits it has in a grid of its own."""
 import math
+import random
 
 import pytest
 import torch
@@ -68,4 +69,46 @@ def test_a_block_for_each_128_rows(cuda_kernels, monkeypatch, d, window, lens, s
     ctx.__dict__.pop("prefill_parts")
     assert cuda_kernels.prefill_cut(ctx, nq, window or 0) == 1
     assert torch.equal(got, cuda_kernels.attention(q, *args))
+    cuda_kernels.check_errors()
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("window", [None, 200])
+def test_blocks_of_one_query_tile_behind_one_another(cuda_kernels, d, window):
+    """Many rounds of blocks without a second query tile (whose softmax group only reads which block is next), a few with one between them."""
+    nq, nkv, page = 36, 4, 16
+    r = random.Random(7)
+    spans = [256 if i % 23 == 5 else 130 if i % 23 == 6 else r.randint(2, 128) for i in range(92)]
+    lens = [n + r.choice([0, 0, 30, 500]) for n in spans]
+    ctx, cache, slots = make_cache_case(torch.bfloat16, nkv, d, page, lens, spans, num_pages=sum(-(-n // page) for n in lens) + 3, seed=3)
+    fill_cache(cache, lens, slots, nkv, d, torch.bfloat16, seed=4)
+    assert ctx.extra_len["attn.prefill_tiles"] // 4 * nq > 20 * 148
+    q = torch.randn(ctx.num_tokens, nq * d, generator=torch.Generator().manual_seed(5)).bfloat16().to(DEV)
+    args = (nq, nkv, d, window, 2.0 / math.sqrt(d))
+    got = [cuda_kernels.attention(q, *args, ctx, cache) for _ in range(5)]
+    assert all(torch.equal(g, got[0]) for g in got)
+    for i in range(0, len(spans), 5):
+        one, rows = _alone(ctx, i)
+        assert torch.equal(got[0][rows], cuda_kernels.attention(q[rows].contiguous(), *args, one, cache)), i
+    cuda_kernels.check_errors()
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("window", [None, 60, 200])
+@pytest.mark.parametrize("lens,spans", [([700] * 12, [100] * 12), ([128 + 3 * i for i in range(40)], [2 + 3 * i for i in range(40)]),
+                                        ([900, 300, 400], [256, 1 + 128, 100])])
+def test_second_query_tiles_that_are_not_there(cuda_kernels, monkeypatch, d, window, lens, spans):
+    """A block for each 128 rows in grids of more blocks than SMs, items of 128 rows and fewer behind more keys than a window holds."""
+    nq, nkv, page = 24, 4, 16
+    ctx, cache, slots = make_cache_case(torch.bfloat16, nkv, d, page, lens, spans, num_pages=sum(-(-n // page) for n in lens) + 3, seed=3)
+    fill_cache(cache, lens, slots, nkv, d, torch.bfloat16, seed=4)
+    monkeypatch.setattr(cuda_kernels, "prefill_parts", lambda *a: 1)
+    q = torch.randn(ctx.num_tokens, nq * d, generator=torch.Generator().manual_seed(5)).bfloat16().to(DEV)
+    results = []
+    for by_tiles in (True, False):
+        ctx.__dict__.pop("prefill_parts", None)
+        monkeypatch.setattr(type(cuda_kernels), "_prefill_by_tiles", staticmethod(lambda ctx, nq: by_tiles))
+        assert cuda_kernels.prefill_cut(ctx, nq, window or 0) == (-1 if by_tiles else 1)
+        results += [cuda_kernels.attention(q, nq, nkv, d, window, 2.0 / math.sqrt(d), ctx, cache) for _ in range(3)]
+    assert all(torch.equal(g, results[0]) for g in results)
     cuda_kernels.check_errors()
