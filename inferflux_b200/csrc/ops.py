@@ -951,13 +951,26 @@ class CudaKernels:
 
     @staticmethod
     def _prefill_by_tiles(ctx, nq):
-        """Whether each 128 rows get a block of their own instead of 256 rows: while all of those fit on the SMs at once.  A key tile takes
-        one query tile as long as two (1.6 us: hand-overs between products and exponentials), but the second tile's last keys and its
-        output come behind the first one's.  us, 256 and 128 rows a block: 12 heads, 447 tokens 14.2 and 12.4, 1,000 20.7 and 18.9,
-        four times 256 behind 700 21.9 and 19.5; 28 heads, 300 behind 500 17.9 and 17.5; heads of 64, 16 of them, 1,000 tokens 19.6
-        and 16.4.  With more blocks than SMs: four times 300 tokens of 12 heads 11.2 and 12.4, 1,000 of 28 21.4 and 21.8, behind 2,000
-        48.8 and 69.7 (one long prompt gains, its last blocks alone being long: 2,000 of 12 heads 33.8 and 30.9)."""
-        return sum(-(-n // 128) for _s, n in ctx.spans if n > 1) * nq <= 148
+        """Whether each 128 rows get a block of their own instead of 256 rows: while all of those fit on the SMs at once, and the block that
+        walks the most keys is one of two query tiles.  Such a block takes an eighth longer a key tile, and the second tile's last keys
+        and its output come behind the first one's, two thirds of a key tile.  Where a block of one query tile walks longer, nothing is
+        gained, and the second query tiles that are not there, which are launched all the same and leave at once, cost up to 4 us.
+        us, 256 and 128 rows a block: 12 heads, 447 tokens 14.9 and 13.3, 1,000 21.5 and 19.5, with four of 50 beside 22.0 and 20.0, four
+        times 256 behind 700 23.1 and 20.5; 28 heads, 300 behind 500 19.5 and 18.9, 640 behind 1,500 37.9 and 34.3; heads of 64, 16 of
+        them, 1,000 tokens 20.5 and 17.4; and those that stay: 12 heads, 300 tokens 11.0 and 11.8, four times 300 12.6 and 13.8, twelve times
+        100 10.2 and 13.8, behind 700 19.5 and 23.1.  With more blocks than SMs: 1,000 of 28 heads behind 2,000 51.7 and 72.2, 3,500 of 12
+        57.4 and 67.6 (the last blocks of 2,000 of 12 alone are long enough to gain, 35.9 and 32.3, and are left)."""
+        tiles = two = one = 0                              # 128-row tiles; keys to the end of the longest item of two tiles, and of one
+        for s, n in ctx.spans:
+            if n > 1:
+                tiles += -(-n // 128)
+                rest = n % 256
+                if 0 < rest <= 128:
+                    one = max(one, s + n)
+                    n -= rest
+                if n:
+                    two = max(two, s + n)
+        return tiles * nq <= 148 and two > 0 and 1.12 * -(-two // 128) + 0.7 > -(-one // 128)
 
     def _prefill_parts(self, ctx, nq, window):
         """A block takes up to 256 tokens of a head and an SM to itself, so what is left behind whole rounds of 148 blocks leaves SMs idle
