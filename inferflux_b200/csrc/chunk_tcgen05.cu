@@ -15,7 +15,7 @@
 // Bound: chunk_outputs (one block an SM, 192 KB of operands) by phases that wait for one another: of 40,000 cycles a block of 128 x 128, reads
 // and cuts of queries and keys 5,000, three products 5,600 to 7,000 each (3,100 of them the tensor pipe's), the state's and values' cuts
 // 4,600 and 5,200, stores 5,800; all blocks meet each phase together, so memory is idle during products.  12 heads, 1,901 tokens of two
-// requests: chunk_local 74.6, carry 11.5, reach 30.9 us -> 15.6, 8.0 and 42.3.
+// requests: chunk_local 74.6, carry 11.5, reach 30.9 us -> 16.4, 8.0 and 43.9.
 #include "parts_tcgen05.cuh"
 
 namespace ifx {

@@ -28,9 +28,9 @@
 //
 // Bound: delta_local, one block of 16 warps an SM (200 KB of operands): operands are cut, multiplied and added up in phases that wait
 // for one another, and the substitution is a chain of four blocks.  2,048 tokens of 24 heads: 165.6 us with products by mma.sync, two
-// blocks of 8 warps an SM; 123.7 on tcgen05.  On the way: the substitution of all 64 rows written out took 33,000 cycles (40 KB of
+// blocks of 8 warps an SM; 127.0 on tcgen05 (123.7 with six products of parts instead of eight).  On the way: the substitution of all 64 rows written out took 33,000 cycles (40 KB of
 // code, the instruction cache), one by one in a loop 11,000, by blocks of 16 with products behind them 4,000.  delta_rule.cu's three
-// kernels take 658 us there, these with the norm 189.
+// kernels take 658 us there, these with the norm 193.
 // Error against 64 bits (2-norm, 2,048 tokens), products by mma.sync and these: state 5.43e-7 and 5.43e-7, outputs 5.10e-7 and 5.09e-7.
 // Scan and products by mma.sync: parameters where trained models have them 5.2e-7 and 4.6e-7, decays near one 1.76e-6 and 1.70e-6,
 // random ones 0.95e-7 and 1.00e-7.
@@ -284,7 +284,8 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_local_kernel(const DeltaC
     tc_after();
     const uint32_t tmem = tmem_holder, lanes = (uint32_t)((warp & 3) * 32) << 16;
     const int row = (warp & 3) * 32 + lane, quarter = warp >> 2, q0 = quarter * 16;
-    const bool lower = row >= kDcD, issuer = warp == 0;    // of the 128 lanes: queries, or key channels
+    const bool lower = row >= kDcD;                        // of the 128 lanes: queries, or key channels
+    const bool issuer = warp == 4;                         // (the first four substitute: issued by one of them, 4 us a layer more)
     const int own = row & (kDcD - 1);
     uint2 phase = make_uint2(0u, 0u);
     const uint64_t d_ur = tc_k_major(base + L::UR), d_ke = tc_k_major(base + L::KE), d_b = tc_k_major(base + L::B),
@@ -385,12 +386,12 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_local_kernel(const DeltaC
         if (s == 3) break;
         tc_before();
         asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (issuer) {
+        if (warp == 0) {
           tc_after();
           const uint32_t elected = elect_one();
-          constexpr int PX[6] = {0, 2, 0, 1, 1, 0}, PY[6] = {0, 0, 2, 1, 0, 1};
+          constexpr int PX[8] = {0, 1, 2, 2, 0, 1, 1, 0}, PY[8] = {0, 2, 1, 0, 2, 1, 0, 1};
 #pragma unroll
-          for (int i = 0; i < 6; ++i)
+          for (int i = 0; i < 8; ++i)
             umma_ts(tmem + (i == 0 ? kTake : kTake + 48), tmem + PX[i] * 32 + s * 8,
                     d_m + ((PY[i] * kNarrow + (s + 1) * 2048 + s * 32) >> 4), tc_idesc(48, 0, 0), i > 1 ? 1u : 0u, elected);
           umma_commit(bar + 16, elected);

@@ -144,8 +144,8 @@ __global__ void latent_rope_append_kernel(const T* __restrict__ rows, int ld, in
 // The two above for bfloat16 rows on 16-byte boundaries.  Eight numbers a read, a row's in registers from the sum to the store; a lane
 // keeps its pair of turned elements and their angle and has four heads' pairs on their way.  The squares are added up in the order of
 // the kernels above (a lane every 32nd number, by way of shared memory), so a row's bits do not depend on where it lies.
-// Bound: HBM and the latency of few tokens' reads.  2,048 tokens, 1,536 numbers normed: 9.0 us a number at a time, so 5.2; 64 of 12
-// heads' numbers turned beside latents of 256: 10.7, so 6.5.  64 decoded tokens: 7 us less for the two in their chain.
+// Bound: HBM and the latency of few tokens' reads.  2,048 tokens, 1,536 numbers normed: 9.0 us a number at a time, so 5.6; 64 of 12
+// heads' numbers turned beside latents of 256: 10.7, so 6.6.  64 decoded tokens: 7 us less for the two in their chain.
 constexpr int kLatentKept = 8;                           // reads of a lane: rows of up to 2,048
 template <int KEPT>
 __device__ __forceinline__ void latent_norm_row(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w, float eps, int rank,

@@ -1,11 +1,16 @@
 // Products of float32 operands on the 5th-generation tensor cores, for recurrences by stretches (chunk_tcgen05.cu, delta_chunks.cu).
 //
-// Operands are float32 cut into three bfloat16 numbers each, rounded at every cut, so that the six largest of the nine products leave out
-// less than 2^-26 of the whole.  They lie in shared memory as [part][64 columns][rows of 128 bytes], 128-byte swizzle: such a tile is a
-// K-major operand of its rows and an MN-major one of its columns.  The tensor cores cut off what a sum cannot hold instead of rounding it.
-// So every step of 16 of the two upper parts' product has an accumulator of its own, and registers add them up, rounding, while the five
-// small products of those steps (a 2^-8th of it) are made into one that they share.  With the upper product's steps in one accumulator
-// too, outputs of constant decays (12 heads of 128 x 128, 2,048 tokens) were off by 2.0e-7 instead of 6.1e-8.
+// Operands are float32 cut into three bfloat16 numbers each, rounded at every cut, so that a part is at most 2^-8 of the one before and the
+// three hold all 24 bits.  Eight of the nine products of parts are made, as by mma_split (chunk_scan.cuh): what is left out is below 2^-32
+// of a product.  (With six it is up to 2^-24.2, rms 2^-27.5: a product of two numbers no longer rounds to its float32 neighbour.)
+// Operands lie in shared memory as [part][64 columns][rows of 128 bytes], 128-byte swizzle: such a tile is a K-major operand of its rows
+// and an MN-major one of its columns.  The tensor cores cut off what a sum cannot hold instead of rounding it.  So every step of 16 of the
+// two upper parts' product has an accumulator of its own, and registers add them up, rounding, while the seven small products of those
+// steps (2^-7 of it at most) are made into one that they share: over eight steps 56 times a last place of theirs, 2^-24 of the whole at
+// most and 2^-27 on average, is cut off, where a rounding after every step could cost eight times 2^-24.  With the upper product's steps
+// in one accumulator too, outputs of constant decays (12 heads of 128 x 128, 2,048 tokens) were off by 2.0e-7 instead of 6.1e-8.
+// The two products from six to eight cost 1.5 % of a delta rule layer (2,048 tokens, 24 heads: 269.0 us, so 273.2) and 0.8 % of one with
+// constant decays (1,901 tokens, 12 heads of 128 x 128: 132.5, so 133.6).
 #pragma once
 
 #include "chunk_scan.cuh"
@@ -81,7 +86,8 @@ struct TcTile {
 
 // acc += x y^T over KSTEPS steps of 16 (x(part, step), y(part, step): operands).  Tensor memory from `at`: SLOTS accumulators of N columns, the
 // first for the small products.  A thread adds up COLS columns of its lane from `col`, groups of 16 that lie SPREAD apart.  `meanwhile` runs under the first products.
-// A warp of its own issues: among the others, which are short of registers, an M 128, N 128, K 16 product took 110 to 190 cycles.
+// One warp issues, the upper products first: with the small ones by a second warp they delay the sums of the upper ones (139.6 us a layer
+// of constant decays instead of 133.6).
 // Two barriers, for the upper products of a round and for the end: one alone could complete twice before a thread looks.
 // By all threads of the block, operands in place and in sight of the tensor cores; at the end nothing is at work any more as far as the
 // others are concerned, and the issuer meets them at the next barrier.
@@ -89,7 +95,7 @@ template <int N, int KSTEPS, int SLOTS, int SPREAD = 16, int COLS, typename X, t
 __device__ __forceinline__ bool tc_product(float (&acc)[COLS], uint32_t at, uint32_t col, uint32_t bar, uint2& phase, bool issuer, X x, Y y, Issue issue,
                                            bool more, Meanwhile meanwhile) {
   constexpr int EACH = SLOTS - 1 < KSTEPS ? SLOTS - 1 : KSTEPS, ROUNDS = (KSTEPS + EACH - 1) / EACH;
-  constexpr int PX[5] = {2, 0, 1, 1, 0}, PY[5] = {0, 2, 1, 0, 1};
+  constexpr int SMALL = 7, PX[SMALL] = {1, 2, 2, 0, 1, 1, 0}, PY[SMALL] = {2, 1, 0, 2, 1, 0, 1};
   bool ok = true;
   // a round's accumulators among themselves first: one rounding of the whole sum a round
   auto column = [&](int c) { return col + (c / 16) * SPREAD + c % 16; };
@@ -124,7 +130,7 @@ __device__ __forceinline__ bool tc_product(float (&acc)[COLS], uint32_t at, uint
 #pragma unroll
       for (int ks = k0; ks < k1; ++ks)
 #pragma unroll
-        for (int i = 0; i < 5; ++i) issue(at, x(PX[i], ks), y(PY[i], ks), more || ks > 0 || i > 0 ? 1u : 0u, elected);
+        for (int i = 0; i < SMALL; ++i) issue(at, x(PX[i], ks), y(PY[i], ks), more || ks > 0 || i > 0 ? 1u : 0u, elected);
       if (r == ROUNDS - 1) umma_commit(bar + 8, elected);
       __syncwarp();
     }

@@ -88,3 +88,35 @@ def test_which_steps_take_them(cuda_kernels):
     rule = cuda_kernels.lib.ifx_chunk_scan_takes_128
     assert not rule(300, 1, 1, 12, 128) and rule(512, 1, 1, 12, 128) and rule(128, 1, 1, 28, 128)
     assert not rule(300, 32, 128, 12, 64)
+
+
+def _off_by(got, want):
+    """The largest relative error in units of 2^-24 (one rounding is at most one of them)."""
+    at = want != 0
+    return float(((got.double() - want).abs()[at] / want.abs()[at]).max()) * 2.0 ** 24
+
+
+@pytest.mark.parametrize("H,G,dk,dv", [(2, 2, 64, 128), (2, 2, 128, 128), (6, 2, 128, 64)])
+def test_one_product_is_rounded_once(cuda_kernels, H, G, dk, dv):
+    """Without decay, one token's key and value alone: the state is their products, and one channel of a query alone reads products of the
+    state.  Whatever parts operands are cut into, a product of two numbers is off by its rounding (2^-24) and by what is left out of and
+    cut off the small parts (eight ends of sums of 2^-8, 2^-28; six products of parts instead of eight leave out up to 2^-24.2)."""
+    T = 300
+    g = torch.Generator().manual_seed(dk + dv)
+    q, k, v = torch.zeros(T, G, dk), torch.zeros(T, G, dk), torch.zeros(T, H, dv)
+    k[290], v[290] = torch.randn(G, dk, generator=g), torch.randn(H, dv, generator=g)
+    rate = torch.ones(H, device=DEV)
+    kw = dict(heads=H, groups=G, dk=dk, dv=dv, decay="constant", rate=rate)
+    state = torch.zeros(1, H * dk * dv, device=DEV)
+    cuda_kernels.decay_scan(q.view(T, -1).to(DEV), k.view(T, -1).to(DEV), v.view(T, -1).to(DEV), None, state, by_64._Ctx((T,), (0,), DEV), **kw)
+    keys = k[290].repeat_interleave(H // G, 0).double()
+    want = v[290].double()[:, :, None] * keys[:, None]                           # [head, value channel, key channel]
+    assert _off_by(state.cpu().view(H, dv, dk), want) <= 1.07
+    q = torch.zeros(T, G, dk)
+    which = torch.randint(0, dk, (T, G, 1), generator=g)
+    q.scatter_(2, which, torch.randn(T, G, 1, generator=g))
+    held = torch.randn(H, dv, dk, generator=g)
+    out = cuda_kernels.decay_scan(q.view(T, -1).to(DEV), torch.zeros(T, G * dk, device=DEV), v.view(T, -1).to(DEV), None,
+                                  held.reshape(1, -1).to(DEV), by_64._Ctx((T,), (0,), DEV), **kw)
+    want = torch.einsum("thk,hvk->thv", q.double().repeat_interleave(H // G, 1), held.double())
+    assert _off_by(out.cpu().view(T, H, dv)[:128], want[:128]) <= 1.07          # (the first stretch: the state as it was)

@@ -150,3 +150,21 @@ def test_long_spans_by_stretches_beside_short_ones(cuda_kernels, monkeypatch, be
         # the norm divides by the size of a head's sums, which may be small
         assert float((y.double().cpu() - want).abs().max()) <= 2.0 ** -8 * max(1.0, float(want.abs().max()))
         assert float((state.double().cpu() - state_p).abs().max()) <= 5e-6 * max(1.0, float(state_p.abs().max()))
+
+
+def test_one_product_is_rounded_once(cuda_kernels, monkeypatch):
+    """Nothing decays and nothing is erased, one token's key and value alone: the state is their products, each off by its rounding (2^-24)
+    and by what the small parts' sum cuts off (2^-28); six products of parts instead of eight leave out up to 2^-24.2."""
+    H, D, T = 6, 64, 128
+    HD = H * D
+    g = torch.Generator().manual_seed(3)
+    proj = torch.zeros(T, 5, H, D)
+    proj[100, 1], proj[:, 2] = torch.randn(H, D, generator=g), torch.randn(T, H, D, generator=g)
+    never = torch.full((HD,), -200.0, device=DEV)             # (sigmoid: 0)
+    monkeypatch.setattr(cuda_kernels, "_delta_by_chunks", lambda *a: (1, 0))
+    state = torch.zeros(1, HD * D, device=DEV)
+    cuda_kernels.delta_rule_scan(proj.view(T, -1).to(DEV), torch.zeros(T, HD, device=DEV), never, never, torch.ones(HD, device=DEV), 1e-6, H, D,
+                                 state, _Ctx((T,), (0,), DEV), BF)
+    want = proj[100, 1].double()[:, :, None] * proj[100, 2].double()[:, None]    # [head, key channel, value channel]
+    got = state.double().cpu().view(H, D, D)
+    assert float(((got - want).abs() / want.abs()).max()) * 2.0 ** 24 <= 1.07
