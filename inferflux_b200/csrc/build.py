@@ -14,6 +14,7 @@ import ctypes
 import hashlib
 import importlib.util
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -166,20 +167,45 @@ def load_library() -> ctypes.CDLL:
     return _LIB
 
 
-class HostLibrary:
-    """The kernel library's entry points as callables that take tensors, integers, floats and None as they are.  `wide`: the names of those
-    that return long long; all others return int.  Names that are not listed are ctypes functions."""
+_ENTRY = re.compile(r"\b(int|long long)\s+(ifx_\w+)\s*\(([^()]*)\)\s*\{")
 
-    def __init__(self, library, names, wide):
+
+def signatures() -> dict:
+    """The C entry points as the sources define them: name -> (whether it returns long long, a letter an argument: p pointer or stream,
+    i int, l long long, f float; ? a structure's address, which only ctypes passes)."""
+    found = {}
+    for src in sources():
+        for wide, name, arguments in _ENTRY.findall(re.sub(r"//[^\n]*", "", src.read_text())):
+            letters = ""
+            for a in filter(None, (a.strip() for a in arguments.split(","))):
+                kind = re.sub(r"\s*\w+$", "", a).strip()           # without the argument's name
+                if kind.endswith("*"):
+                    letters += "?" if "Ifx" in kind else "p"
+                else:
+                    letters += {"int": "i", "unsigned": "i", "long long": "l", "float": "f", "cudaStream_t": "p"}[kind]
+            found[name] = (wide != "int", letters)
+    return found
+
+
+class HostLibrary:
+    """The kernel library's entry points as callables that take tensors, integers, floats and None as they are, in the count and of the
+    kinds that the sources say (TypeError otherwise).  `wide`: the names of those that return long long; all others return int.  Names
+    that are not listed are ctypes functions."""
+
+    def __init__(self, library, names, wide, known=None):
         import torch
+        known = signatures() if known is None else known
         self._ctypes = library
         spec = importlib.util.spec_from_file_location("_ifx_host", build_dir() / HOST_NAME)
         host = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(host)
         for name in (*names, *wide):
             fn = getattr(self._ctypes, name)
-            fn.restype = ctypes.c_longlong if name in wide else ctypes.c_int
-            setattr(self, name, host.Function(ctypes.cast(fn, ctypes.c_void_p).value, name in wide, torch.Tensor))
+            returns_wide, letters = known[name]
+            if returns_wide != (name in wide) or "?" in letters:
+                raise BuildError(f"{name} is listed with another result than the sources give it, or takes structures")
+            fn.restype = ctypes.c_longlong if returns_wide else ctypes.c_int
+            setattr(self, name, host.Function(ctypes.cast(fn, ctypes.c_void_p).value, returns_wide, torch.Tensor, letters))
 
     def __getattr__(self, name):
         return getattr(self._ctypes, name)

@@ -1,8 +1,12 @@
 // Calls of the kernel library's C entry points from Python, in place of ctypes: a small layer's launches take the GPU a few microseconds
 // each, and ctypes an object an argument and as long a call.
 //
-//   Function(address, wide, tensor_type)(...)    integers, floats (as float32), None (null) and tensors (their data_ptr()); also objects
-//                                                with a `value` of those (ctypes' own)
+//   Function(address, wide, tensor_type, signature)(...)    integers, floats (as float32), None (null) and tensors (their data_ptr());
+//                                                           also objects with a `value` of those (ctypes' own)
+//
+// signature: a letter an argument, p pointer, i int, l long long, f float.  A call with another count of arguments or with an argument of
+// another kind raises TypeError; a pointer may be an integer, and an integer in the place of a float is passed as a float.  (Without a
+// signature arguments are passed as what they are.)
 //
 // The entry points take pointers, integers and up to eight floats.  By the System V convention of x86-64 the first six integers and
 // pointers go to general registers, floats to vector registers and further integers to the stack, eight bytes each and in order, so one
@@ -31,6 +35,7 @@ struct Function {
   vectorcallfunc vectorcall;
   void* address;
   PyObject* tensor_type;
+  PyObject* signature;                                     // ASCII, or null
   int wide;                                                // returns long long, not int
 };
 
@@ -54,20 +59,33 @@ bool add_integer(Arguments& a, PyObject* v) {
   return true;
 }
 
-bool add(Arguments& a, PyObject* v, PyObject* tensor_type, int depth) {
-  if (v == Py_None) return add_integer(a, Py_False);
-  if (PyLong_Check(v)) return add_integer(a, v);
-  if (PyFloat_Check(v)) {
-    if (a.real == kFloats) {
-      PyErr_SetString(PyExc_TypeError, "more than eight floats");
-      return false;
-    }
-    const float f = (float)PyFloat_AS_DOUBLE(v);
-    std::memcpy(&a.floats[a.real++], &f, sizeof f);
-    return true;
+bool add_float(Arguments& a, double v) {
+  if (a.real == kFloats) {
+    PyErr_SetString(PyExc_TypeError, "more than eight floats");
+    return false;
   }
+  const float f = (float)v;
+  std::memcpy(&a.floats[a.real++], &f, sizeof f);
+  return true;
+}
+
+bool refuse(PyObject* v, char kind) {
+  PyErr_Format(PyExc_TypeError, "cannot pass a %s as %s", Py_TYPE(v)->tp_name, kind == 'p' ? "a pointer" : kind == 'f' ? "a float" : "an integer");
+  return false;
+}
+
+// kind: a signature's letter, or 0
+bool add(Arguments& a, PyObject* v, PyObject* tensor_type, char kind, int depth) {
+  if (v == Py_None) return kind == 0 || kind == 'p' ? add_integer(a, Py_False) : refuse(v, kind);
+  if (PyLong_Check(v)) {
+    if (kind != 'f') return add_integer(a, v);
+    const double x = PyLong_AsDouble(v);
+    return x == -1.0 && PyErr_Occurred() ? false : add_float(a, x);
+  }
+  if (PyFloat_Check(v)) return kind == 0 || kind == 'f' ? add_float(a, PyFloat_AS_DOUBLE(v)) : refuse(v, kind);
   PyObject* inner;
   if (PyObject_TypeCheck(v, (PyTypeObject*)tensor_type)) {
+    if (kind != 0 && kind != 'p') return refuse(v, kind);
     PyObject* self[1] = {v};
     inner = PyObject_VectorcallMethod(g_data_ptr, self, 1 | PY_VECTORCALL_ARGUMENTS_OFFSET, nullptr);
   } else {
@@ -75,7 +93,7 @@ bool add(Arguments& a, PyObject* v, PyObject* tensor_type, int depth) {
     if (!inner && !PyErr_Occurred()) PyErr_Format(PyExc_TypeError, "cannot pass a %s", Py_TYPE(v)->tp_name);
   }
   if (!inner) return false;
-  const bool ok = add(a, inner, tensor_type, 1);
+  const bool ok = add(a, inner, tensor_type, kind, 1);
   Py_DECREF(inner);
   return ok;
 }
@@ -104,8 +122,16 @@ PyObject* call(PyObject* callable, PyObject* const* args, size_t nargsf, PyObjec
   }
   Arguments a;
   const Py_ssize_t n = PyVectorcall_NARGS(nargsf);
+  const char* kinds = nullptr;
+  if (self->signature) {
+    kinds = reinterpret_cast<const char*>(PyUnicode_1BYTE_DATA(self->signature));
+    if (n != PyUnicode_GET_LENGTH(self->signature)) {
+      PyErr_Format(PyExc_TypeError, "%zd arguments instead of %zd", n, PyUnicode_GET_LENGTH(self->signature));
+      return nullptr;
+    }
+  }
   for (Py_ssize_t i = 0; i < n; ++i)
-    if (!add(a, args[i], self->tensor_type, 0)) return nullptr;
+    if (!add(a, args[i], self->tensor_type, kinds ? kinds[i] : 0, 0)) return nullptr;
   int64_t result;
   Py_BEGIN_ALLOW_THREADS
   result = invoke(self->address, a);
@@ -116,8 +142,12 @@ PyObject* call(PyObject* callable, PyObject* const* args, size_t nargsf, PyObjec
 PyObject* make(PyTypeObject* type, PyObject* args, PyObject*) {
   unsigned long long address;
   int wide;
-  PyObject* tensor_type;
-  if (!PyArg_ParseTuple(args, "KpO!", &address, &wide, &PyType_Type, &tensor_type)) return nullptr;
+  PyObject *tensor_type, *signature = nullptr;
+  if (!PyArg_ParseTuple(args, "KpO!|U", &address, &wide, &PyType_Type, &tensor_type, &signature)) return nullptr;
+  if (signature && !PyUnicode_IS_ASCII(signature)) {
+    PyErr_SetString(PyExc_ValueError, "a signature has the letters p, i, l and f");
+    return nullptr;
+  }
   Function* self = reinterpret_cast<Function*>(type->tp_alloc(type, 0));
   if (!self) return nullptr;
   self->vectorcall = call;
@@ -125,11 +155,14 @@ PyObject* make(PyTypeObject* type, PyObject* args, PyObject*) {
   self->wide = wide;
   Py_INCREF(tensor_type);
   self->tensor_type = tensor_type;
+  Py_XINCREF(signature);
+  self->signature = signature;
   return reinterpret_cast<PyObject*>(self);
 }
 
 void drop(PyObject* o) {
   Py_XDECREF(reinterpret_cast<Function*>(o)->tensor_type);
+  Py_XDECREF(reinterpret_cast<Function*>(o)->signature);
   Py_TYPE(o)->tp_free(o);
 }
 

@@ -76,3 +76,44 @@ def test_what_it_refuses(library):
             fast(*args)
     with pytest.raises(TypeError):
         fast(a=1)
+
+
+@pytest.mark.parametrize("n", range(len(SIGNATURES)))
+def test_a_signature_changes_no_call(library, n):
+    lib, host = library
+    r = random.Random(100 + n)
+    fn = getattr(lib, f"w{n}")
+    fn.restype = ctypes.c_longlong
+    fast = host.Function(ctypes.cast(fn, ctypes.c_void_p).value, True, torch.Tensor, SIGNATURES[n])
+    for _ in range(20):
+        plain, wrapped = _arguments(SIGNATURES[n], r)
+        assert fast(*plain) == fn(*wrapped) == fast(*wrapped)
+        assert fast(*[p.data_ptr() if isinstance(p, torch.Tensor) else p for p in plain]) == fn(*wrapped)
+
+
+@pytest.mark.parametrize("n", range(len(SIGNATURES)))
+def test_another_count_or_kind_is_refused(library, n):
+    """What a call without a signature reads from the wrong register, or from whatever lies on the stack."""
+    lib, host = library
+    r = random.Random(200 + n)
+    sig, fn = SIGNATURES[n], getattr(lib, f"w{n}")
+    fn.restype = ctypes.c_longlong
+    fast = host.Function(ctypes.cast(fn, ctypes.c_void_p).value, True, torch.Tensor, sig)
+    plain, wrapped = _arguments(sig, r)
+    for wrong in (plain[:-1], plain + [1], plain + [None]):
+        with pytest.raises(TypeError):
+            fast(*wrong)
+    for i, c in enumerate(sig):
+        for wrong in {"p": (1.5,), "i": (1.5, None, torch.zeros(1)), "l": (1.5, None, torch.zeros(1)), "f": (None, torch.zeros(1))}[c]:
+            with pytest.raises(TypeError):
+                fast(*plain[:i], wrong, *plain[i + 1:])
+    if "f" in sig:                                           # an integer in the place of a float is one
+        whole, as_float = ([7 if c == "f" else p for c, p in zip(sig, plain)], [ctypes.c_float(7.0) if c == "f" else w for c, w in zip(sig, wrapped)])
+        assert fast(*whole) == fn(*as_float)
+
+
+def test_signatures_as_the_sources_have_them():
+    known = build.signatures()
+    assert known["ifx_embed"] == (False, "pppiiiip") and known["ifx_moe_route_kind"] == (False, "ppppiiiifp")
+    assert known["ifx_gemm_f32_split_scratch"] == (True, "iii") and "?" in known["ifx_layer_forward"][1]
+    assert sum(letters.count("f") for _wide, letters in known.values()) > 50
