@@ -2,11 +2,12 @@
 
 Every .cu file of this folder is compiled to an object (`-gencode
 arch=compute_100a,code=sm_100a`) and the objects are linked into one shared
-library; host_call.cpp becomes the extension module that calls it.  Both live in `_build/` beside the sources when that folder can be
-written, else in a per-user folder under the system's temporary directory.  A
-stamp of the sources' contents and the flags decides whether a build is current, so
-a fresh checkout compiles once, at its first call, and prints a line per file
-while it does.
+library; host_call.cpp becomes the extension module that calls it, on hosts it is written for
+(x86-64 Linux with g++ and Python.h; on others ctypes calls it, more slowly).  Both live in
+`_build/` beside the sources when that folder can be written, else in a per-user folder under
+the system's temporary directory.  A stamp of the sources' contents and the flags decides
+whether a build is current, so a fresh checkout compiles once, at its first call, and prints a
+line per file while it does.
 """
 from __future__ import annotations
 
@@ -14,6 +15,7 @@ import ctypes
 import hashlib
 import importlib.util
 import os
+import platform
 import re
 import shutil
 import subprocess
@@ -103,11 +105,23 @@ def _compile_one(nvcc: str, src: Path, obj: Path, verbose_ptxas: bool) -> str:
     return proc.stderr
 
 
+def _no_extension() -> str:
+    """Why host_call.cpp cannot be had on this host, or nothing."""
+    if platform.machine() not in ("x86_64", "AMD64") or not sys.platform.startswith("linux"):
+        return f"it is written for x86-64 Linux, not for {platform.machine()} {sys.platform}"
+    if not (os.environ.get("CXX") or shutil.which("g++")):
+        return "no g++"
+    include = Path(sysconfig.get_paths()["include"])
+    return "" if (include / "Python.h").is_file() else f"no Python.h in {include}"
+
+
 def _compile_host(out: Path) -> None:
+    why = _no_extension()
+    if why:
+        _say(f"host_call.cpp is left out ({why}): kernels are called through ctypes, which takes the host some microseconds more a call")
+        return
     gxx = os.environ.get("CXX") or shutil.which("g++")
     include = sysconfig.get_paths()["include"]
-    if not gxx or not (Path(include) / "Python.h").is_file():
-        raise BuildError(f"host_call.cpp needs g++ and Python.h ({include}): there is no other way to call the kernels")
     tmp = out / (HOST_NAME + f".tmp{os.getpid()}")
     proc = subprocess.run([gxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-I", include, str(HERE / "host_call.cpp"), "-o", str(tmp)],
                           capture_output=True, text=True)
@@ -122,7 +136,7 @@ def build(force: bool = False, verbose_ptxas: bool = False) -> Path:
     lib, stamp_file = out / LIB_NAME, out / "stamp.txt"
     stamp = _stamp()
     if not force and lib.is_file() and stamp_file.is_file() and stamp_file.read_text().strip() == stamp:
-        if not (out / HOST_NAME).is_file():                  # built by another interpreter
+        if not (out / HOST_NAME).is_file() and not _no_extension():        # built by another interpreter
             _compile_host(out)
         return lib
     nvcc = find_nvcc()
@@ -187,6 +201,23 @@ def signatures() -> dict:
     return found
 
 
+class _ThroughCtypes:
+    """One entry point, called as the extension's Function is."""
+    KINDS = {"p": ctypes.c_void_p, "i": ctypes.c_int, "l": ctypes.c_longlong, "f": ctypes.c_float}
+
+    def __init__(self, fn, tensor_type, letters):
+        fn.argtypes = [self.KINDS[c] for c in letters]
+        self._fn, self._tensor, self._letters = fn, tensor_type, letters
+
+    def __call__(self, *args):
+        if len(args) != len(self._letters):
+            raise TypeError(f"{len(args)} arguments instead of {len(self._letters)}")
+        try:
+            return self._fn(*[a.data_ptr() if c == "p" and isinstance(a, self._tensor) else a for a, c in zip(args, self._letters)])
+        except ctypes.ArgumentError as e:
+            raise TypeError(str(e)) from e
+
+
 class HostLibrary:
     """The kernel library's entry points as callables that take tensors, integers, floats and None as they are, in the count and of the
     kinds that the sources say (TypeError otherwise).  `wide`: the names of those that return long long; all others return int.  Names
@@ -196,16 +227,19 @@ class HostLibrary:
         import torch
         known = signatures() if known is None else known
         self._ctypes = library
-        spec = importlib.util.spec_from_file_location("_ifx_host", build_dir() / HOST_NAME)
-        host = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(host)
+        host, path = None, build_dir() / HOST_NAME
+        if path.is_file():
+            spec = importlib.util.spec_from_file_location("_ifx_host", path)
+            host = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(host)
         for name in (*names, *wide):
             fn = getattr(self._ctypes, name)
             returns_wide, letters = known[name]
             if returns_wide != (name in wide) or "?" in letters:
                 raise BuildError(f"{name} is listed with another result than the sources give it, or takes structures")
             fn.restype = ctypes.c_longlong if returns_wide else ctypes.c_int
-            setattr(self, name, host.Function(ctypes.cast(fn, ctypes.c_void_p).value, returns_wide, torch.Tensor, letters))
+            setattr(self, name, _ThroughCtypes(fn, torch.Tensor, letters) if host is None else
+                    host.Function(ctypes.cast(fn, ctypes.c_void_p).value, returns_wide, torch.Tensor, letters))
 
     def __getattr__(self, name):
         return getattr(self._ctypes, name)

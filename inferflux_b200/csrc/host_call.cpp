@@ -23,7 +23,7 @@
 #include <cstring>
 
 #if !defined(__x86_64__) || !defined(__linux__)
-#error "host_call.cpp is written for the System V calling convention of x86-64"
+#error "host_call.cpp is written for the System V calling convention of x86-64 (build.py leaves it out elsewhere)"
 #endif
 
 namespace {

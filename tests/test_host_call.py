@@ -117,3 +117,32 @@ def test_signatures_as_the_sources_have_them():
     assert known["ifx_embed"] == (False, "pppiiiip") and known["ifx_moe_route_kind"] == (False, "ppppiiiifp")
     assert known["ifx_gemm_f32_split_scratch"] == (True, "iii") and "?" in known["ifx_layer_forward"][1]
     assert sum(letters.count("f") for _wide, letters in known.values()) > 50
+
+
+@pytest.mark.parametrize("without", ["extension", "python.h", "x86"])
+def test_hosts_without_the_extension(library, monkeypatch, tmp_path, capsys, without):
+    """Another processor, no g++ or no Python.h: nothing is built and nothing raised, and ctypes makes the same calls and refusals."""
+    lib, _ = library
+    monkeypatch.setattr(build, "build_dir", lambda: tmp_path)
+    if without == "x86":
+        monkeypatch.setattr(build.platform, "machine", lambda: "aarch64")
+    elif without == "python.h":
+        monkeypatch.setattr(build.sysconfig, "get_paths", lambda: {"include": str(tmp_path)})
+    else:
+        monkeypatch.delenv("CXX", raising=False)
+        monkeypatch.setattr(build.shutil, "which", lambda name: None)
+    build._compile_host(tmp_path)
+    assert not list(tmp_path.iterdir())
+    names = [f"n{n}" for n in range(len(SIGNATURES))], [f"w{n}" for n in range(len(SIGNATURES))]
+    known = {f"{c}{n}": (c == "w", sig) for c in "nw" for n, sig in enumerate(SIGNATURES)}
+    host = build.HostLibrary(ctypes.CDLL(lib._name), *names, known)
+    for n, sig in enumerate(SIGNATURES):
+        r = random.Random(300 + n)
+        for name in (f"n{n}", f"w{n}"):
+            plain, wrapped = _arguments(sig, r)
+            fn = getattr(lib, name)
+            fn.restype = ctypes.c_longlong if name[0] == "w" else ctypes.c_int
+            assert getattr(host, name)(*plain) == fn(*wrapped)
+            for wrong in (plain[:-1], plain + [1], [1.5 if c != "f" else None for c in sig]):
+                with pytest.raises(TypeError):
+                    getattr(host, name)(*wrong)
