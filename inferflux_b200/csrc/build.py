@@ -29,6 +29,7 @@ from pathlib import Path
 HERE = Path(__file__).resolve().parent
 LIB_NAME = "libinferflux_b200.so"
 HOST_NAME = "_ifx_host" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so")
+HOST_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-shared"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
               "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
 LINK_LIBS = ["-lcublas"]
@@ -56,7 +57,7 @@ def sources():
 
 def _stamp() -> str:
     h = hashlib.sha256()
-    for p in sorted(list(HERE.glob("*.cu")) + list(HERE.glob("*.cuh")) + list(HERE.glob("*.h")) + list(HERE.glob("*.cpp"))):
+    for p in sorted(list(HERE.glob("*.cu")) + list(HERE.glob("*.cuh")) + list(HERE.glob("*.h"))):
         h.update(p.name.encode())
         h.update(p.read_bytes())
     h.update(" ".join(NVCC_FLAGS + LINK_LIBS).encode())
@@ -115,7 +116,22 @@ def _no_extension() -> str:
     return "" if (include / "Python.h").is_file() else f"no Python.h in {include}"
 
 
+def _host_stamp() -> str:
+    """Of the extension alone: interpreters share a folder and the library, and each has an extension of its own."""
+    h = hashlib.sha256((HERE / "host_call.cpp").read_bytes())
+    h.update(" ".join(HOST_FLAGS).encode())
+    return h.hexdigest()
+
+
+def _host_is_current(out: Path) -> bool:
+    stamp_file = out / (HOST_NAME + ".stamp")
+    return (out / HOST_NAME).is_file() and stamp_file.is_file() and stamp_file.read_text().strip() == _host_stamp()
+
+
 def _compile_host(out: Path) -> None:
+    """The extension, unless it is there from these sources."""
+    if _host_is_current(out):
+        return
     why = _no_extension()
     if why:
         _say(f"host_call.cpp is left out ({why}): kernels are called through ctypes, which takes the host some microseconds more a call")
@@ -123,11 +139,12 @@ def _compile_host(out: Path) -> None:
     gxx = os.environ.get("CXX") or shutil.which("g++")
     include = sysconfig.get_paths()["include"]
     tmp = out / (HOST_NAME + f".tmp{os.getpid()}")
-    proc = subprocess.run([gxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-I", include, str(HERE / "host_call.cpp"), "-o", str(tmp)],
+    proc = subprocess.run([gxx, *HOST_FLAGS, "-I", include, str(HERE / "host_call.cpp"), "-o", str(tmp)],
                           capture_output=True, text=True)
     if proc.returncode != 0:
         raise BuildError(f"g++ failed on host_call.cpp:\n{proc.stdout}\n{proc.stderr}")
     os.replace(tmp, out / HOST_NAME)
+    (out / (HOST_NAME + ".stamp")).write_text(_host_stamp() + "\n")
 
 
 def build(force: bool = False, verbose_ptxas: bool = False) -> Path:
@@ -136,8 +153,7 @@ def build(force: bool = False, verbose_ptxas: bool = False) -> Path:
     lib, stamp_file = out / LIB_NAME, out / "stamp.txt"
     stamp = _stamp()
     if not force and lib.is_file() and stamp_file.is_file() and stamp_file.read_text().strip() == stamp:
-        if not (out / HOST_NAME).is_file() and not _no_extension():        # built by another interpreter
-            _compile_host(out)
+        _compile_host(out)                                   # another interpreter may have built the library
         return lib
     nvcc = find_nvcc()
     srcs = sources()
@@ -227,9 +243,9 @@ class HostLibrary:
         import torch
         known = signatures() if known is None else known
         self._ctypes = library
-        host, path = None, build_dir() / HOST_NAME
-        if path.is_file():
-            spec = importlib.util.spec_from_file_location("_ifx_host", path)
+        host = None
+        if _host_is_current(build_dir()):
+            spec = importlib.util.spec_from_file_location("_ifx_host", build_dir() / HOST_NAME)
             host = importlib.util.module_from_spec(spec)
             spec.loader.exec_module(host)
         for name in (*names, *wide):

@@ -146,3 +146,34 @@ def test_hosts_without_the_extension(library, monkeypatch, tmp_path, capsys, wit
             for wrong in (plain[:-1], plain + [1], [1.5 if c != "f" else None for c in sig]):
                 with pytest.raises(TypeError):
                     getattr(host, name)(*wrong)
+
+
+def test_an_extension_of_earlier_sources_is_made_again(monkeypatch, tmp_path):
+    """The library's stamp is every interpreter's; each one's extension has its own.  One of earlier sources that cannot be made again is
+    not loaded."""
+    if shutil.which("g++") is None:
+        pytest.skip("no g++")
+    import os
+    monkeypatch.setattr(build, "build_dir", lambda: tmp_path)
+    monkeypatch.setattr(build, "HERE", tmp_path / "sources")
+    (tmp_path / "sources").mkdir()
+    own = tmp_path / "sources" / "host_call.cpp"
+    shutil.copy(os.path.join(os.path.dirname(build.__file__), "host_call.cpp"), own)
+    (tmp_path / build.LIB_NAME).write_bytes(b"")
+    (tmp_path / "stamp.txt").write_text(build._stamp() + "\n")                # another interpreter has built the library
+    host = tmp_path / build.HOST_NAME
+    host.write_bytes(b"an extension of earlier sources")
+    assert build.build() == tmp_path / build.LIB_NAME
+    made = host.stat()
+    assert made.st_size > 1000
+    build.build()
+    assert host.stat().st_mtime_ns == made.st_mtime_ns and host.stat().st_ino == made.st_ino
+    own.write_text(own.read_text() + "// and more\n")
+    (tmp_path / "stamp.txt").write_text(build._stamp() + "\n")
+    build.build()
+    assert host.stat().st_ino != made.st_ino or host.stat().st_mtime_ns != made.st_mtime_ns
+    own.write_text(own.read_text() + "// and more\n")
+    (tmp_path / "stamp.txt").write_text(build._stamp() + "\n")
+    monkeypatch.setattr(build, "_no_extension", lambda: "no g++")
+    build.build()
+    assert host.is_file() and build.HostLibrary(ctypes.CDLL(None), (), (), {}) is not None and not build._host_is_current(tmp_path)
