@@ -1566,14 +1566,16 @@ class CudaKernels:
     @classmethod
     def stretches_pay(cls, longest, blocks, cheap, short, short_tokens, short_spans, short_stretches, stretches):
         """The plan for a step whose longest span has `longest` tokens, with `blocks` blocks a stretch.  Short spans go along where their
-        stretches (0.13 us a block) take less than a launch of the scan for them.  Otherwise what is gained is the time between the
-        longest span and the longest short one.  us, the scan alone and this (12 heads of 128 x 128 with a constant decay; wkv, 24
-        heads of 64): 128 tokens 41 / 32; 40 / 29; sixteen of 128 213 / 152; 183 / 148; short spans along: 128 and 20 46 / 33; 44 / 30;
-        228 and 100 80 / 45 (81 beside); 73 / 42 (74); beside the scan: 128 and 31 of one 75 / 66; 96 / 62 (146; 121 along); 512 and 31
-        of one 239 / 79; 260 / 76; 512, 100, 80 and 29 of one 226 / 124; 267 / 127.  At 56 heads 128 and 31 of one 123 / 117; 154 / 109,
-        but 63 of one 187 / 199; 242 / 174: what the launch for very many states costs has to be gained.  `cheap`, a constant decay and
-        keys of 64 numbers: its scan wins where very many stretches are of short spans (28 heads, 32 of 128 442 / 493; sixteen of 256
-        456 / 374)."""
+        stretches (0.13 us a block of 64 tokens) take less than a launch of the scan for them.  Otherwise what is gained is the time between
+        the longest span and the longest short one.  us, the scan alone and all by stretches (the long ones beside the scan), 12 heads of
+        128 x 128 with a constant decay; wkv, 24 heads of 64: 128 tokens 40 / 30; 39 / 28; sixteen of 128 212 / 92; 183 / 143; 128 and 20
+        46 / 31 (41); 43 / 29 (39); 228 and 100 79 / 36 (73); 71 / 39 (72); 128 and 31 of one token 75 / 149 (63); 95 / 135 (60); 512 and
+        31 of one token 223 / 152 (69); 260 / 151 (74); 512, 100, 80 and 29 of one token 234 / 154 (107); 267 / 154 (122).  At 56 and 28
+        heads 128 and 31 of one token 154 / 285 (105) and 124 / 367 (109), but 63 of one token 28 heads of 128 x 128 188 / 896 (194): what the
+        launch for very many states costs has to be gained.  `cheap`, a constant decay and keys of 64 numbers, whose scan wins over
+        stretches of 64 where very many are of short spans.  The lines were drawn for stretches of 64 tokens, which wkv and decays per
+        channel have; no step takes longer than the scan alone.  Stretches of 128 take about half as long, so that more steps with a
+        decay per head would gain: 300 and eight of 100 tokens 174 / 55 (138); `cheap`, 28 heads, 32 of 128 441 / 300."""
         if cheap and stretches > 24 + longest // 4:
             return False
         if 0.13 * short_stretches * blocks <= 8 + 0.22 * short + 0.035 * short_spans * blocks:
@@ -1643,22 +1645,25 @@ class CudaKernels:
         """A stretch of the delta rule does several times a token's work of the scan; what is gained is that the tokens of one span run
         side by side, so this compares what the ways take: the scan for all, stretches for all, stretches for the long spans beside
         the scan for the others.  us, fitted to what follows within a sixth: the scan walks its longest span at 0.3 a token and more
-        with more columns at once; the stretches go in rounds of 148 blocks (a head's stretch each), and every block walks the requests.
-        us, 24 heads of 64, the scan alone and the stretches (beside the scan): 128 tokens 46 / 31; 256 86 / 34; 512 164 / 59; 2,048
-        656 / 189; two of 256 98 / 60; four of 256 126 / 91; four of 512 259 / 185; eight of 512 365 / 333; eight of 128 92 / 98; sixteen of
-        150 223 / 254; with 31 of one 128 67 / 178 (57), 512 212 / 214 (87); with 63 of one 512 227 / 452 (110); 256 and 100 94 / 39 (80);
-        512, 100, 80 and 29 of one 211 / 85 (112).  56 heads: 128 56 / 37; 256 104 / 61; 2,048 830 / 386; four of 256 263 / 213; four of
-        512 513 / 384; with 31 of one 512 296 / 540 (180)."""
+        with more columns at once; the stretches go in rounds of 148 blocks (a head's stretch each), every block walks the requests, each
+        span behind the eighth costs its heads' carries, and beyond 3,000 blocks what they hand on (40 KB each) does not stay in L2.
+        us, 24 heads of 64, the scan alone and the stretches for all (for the long ones beside the scan): 128 tokens 46 / 32; 256 85 / 34;
+        512 164 / 60; 2,048 658 / 193; two of 256 98 / 61; four of 256 125 / 93; four of 512 261 / 190; eight of 512 368 / 341; eight of 128
+        92 / 101; sixteen of 150 224 / 260; 128 and 31 of one token 66 / 181 (58, left: what it gains is within the fit's error); 512 and 31
+        of one token 216 / 221 (89), 63 228 / 469 (111); 256 and 100 94 / 40 (80); four spans of 512, 100, 80 and 29 212 / 87 (114).
+        56 heads: 128 56 / 38; 256 104 / 62; 2,048 833 / 396; four of 256 265 / 219; four of 512 516 / 394; sixteen of 128 420 / 469,
+        thirty-two 794 / 1,013; sixteen of 256 817 / 833; 512 and 31 of one token 297 / 560 (183), 63 321 / 1,196 (230, left)."""
         def scan(longest, tokens, requests):
             columns = tokens * heads / longest             # heads at work at once, on average
             return longest * max(0.3 + 0.0019 * columns, columns / 275) + 0.018 * requests * heads
 
-        def chunks(blocks):
-            return 20.6 * -(-blocks // 148) + 0.6 * (longest / 64) + 0.07 * blocks + 4 + 1.5 * max(0, requests - 4)
+        def chunks(blocks, spans):
+            return (20.6 * -(-blocks // 148) + 0.6 * (longest / 64) + 0.07 * blocks + 4 + 1.5 * max(0, requests - 4)
+                    + 0.06 * heads * max(0, spans - 8) + 0.1 * max(0, blocks - 3000))
         least, alone = 1, 6 + scan(longest, tokens, requests - 1)
-        best = chunks((stretches + short_stretches) * heads)
+        best = chunks((stretches + short_stretches) * heads, requests)
         if short:
-            beside = chunks(stretches * heads) + 10 + scan(short, short_tokens, short_spans)
+            beside = chunks(stretches * heads, requests - short_spans) + 10 + scan(short, short_tokens, short_spans)
             if beside < best:
                 least, best = cls.CHUNK_SCAN_MIN_SPAN, beside
         return best < alone and (least, short if least > 1 else 0)
