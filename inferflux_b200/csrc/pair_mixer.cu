@@ -98,12 +98,14 @@ __global__ void gate_mul_kernel(const void* __restrict__ a, const void* __restri
 
 __device__ __forceinline__ float gate_value(float g, int sigmoid) { return (sigmoid ? 1.0f : g) / (1.0f + expf(-g)); }
 
-// Parts of up to 256 numbers: a warp takes up to four neighbouring parts and has the reads of all of them on their way before it sums
+// Parts of up to 32 PER numbers: a warp takes up to AT neighbouring parts and has the reads of all of them on their way before it sums
 // the first.  ROOT: one over a square root in the place of rsqrtf (wkv.cu's norm, which its scan makes too: the same bits).
-// Bound: instructions (an exponential and a division a number), then HBM.  A warp a part, its two reads after one another, a 64-bit
-// division a part -> the kernel below, us: 1,500 rows of 24 parts of 64 16.5 -> 9.7; of 12 of 128 11.1 -> 6.5 (4.2 TB/s).
+// Bound: instructions (an exponential and a division a number), then HBM.  A block a row, a warp a part, its two reads after one another, a
+// 64-bit division a part -> the kernels below, us: 1,500 rows of 24 parts of 64 16.5 -> 9.7; of 12 of 128 11.1 -> 6.5 (4.2 TB/s); 2,048 of
+// 48 of 32 18.5 -> 14.6, of 96 of 16 35.0 -> 34.7, of 16 of 96 12.8 -> 11.8, of 14 of 256 21.9 -> 22.3 (29.1 -> 22.8 with the gate first).
+// PER is the part's own: with room for 256 numbers in every case, parts of 32 took 105 us, of 16 217, of 96 38.
 constexpr int kHeadsAtOnce = 4;
-template <typename TO, int PER, bool ROOT>
+template <typename TO, int PER, int AT, bool ROOT>
 __global__ void __launch_bounds__(256) gated_heads_kernel(const float* __restrict__ y, const float* __restrict__ gate, long long gate_stride,
                                                           const float* __restrict__ w, int w_wide, float eps, TO* __restrict__ out,
                                                           unsigned items, unsigned groups, int part, int gate_first, int sigmoid, unsigned each) {
@@ -112,11 +114,11 @@ __global__ void __launch_bounds__(256) gated_heads_kernel(const float* __restric
   pdl_launch_dependents();
   pdl_wait();
   if (first >= items) return;
-  float v[kHeadsAtOnce][PER], g[kHeadsAtOnce][PER];
-  int p[kHeadsAtOnce];
+  float v[AT][PER], g[AT][PER];
+  int p[AT];
   unsigned t = first / groups, at = first - t * groups;      // (one division: they cost more than the reads)
 #pragma unroll
-  for (unsigned k = 0; k < kHeadsAtOnce; ++k) {
+  for (unsigned k = 0; k < AT; ++k) {
     const unsigned item = first + k;
     const bool live = k < each && item < items;
     p[k] = (int)at;
@@ -131,12 +133,13 @@ __global__ void __launch_bounds__(256) gated_heads_kernel(const float* __restric
     }
   }
 #pragma unroll
-  for (unsigned k = 0; k < kHeadsAtOnce; ++k) {
+  for (unsigned k = 0; k < AT; ++k) {
     const unsigned item = first + k;
     if (k >= each || item >= items) break;
     float ss = 0.0f;
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
+      if (32 * j >= part) break;
       g[k][j] = gate_value(g[k][j], sigmoid);
       if (gate_first) v[k][j] *= g[k][j];
       ss = lane + 32 * j < part ? fmaf(v[k][j], v[k][j], ss) : ss;
@@ -221,7 +224,7 @@ int launch_gated_heads(const float* y, const float* gate, long long gate_stride,
   const unsigned items = (unsigned)T * (unsigned)groups;
   // several parts a warp only where all SMs have their fill of warps without
   const unsigned across = part == 64 ? 2 : 1, turns = items / across;
-  const unsigned each = turns >= 148 * 64 * 2 ? 4 : turns >= 148 * 64 ? 2 : 1;
+  const unsigned most = part > 128 ? 2 : 4, each = turns >= 148 * 64 * 2 ? most : turns >= 148 * 64 ? 2 : 1;
   const unsigned blocks = (items + 8 * each * across - 1) / (8 * each * across);
   static_assert(kHeadsAtOnce == 4, "each");
   auto full = [&](auto* to, auto kern) {
@@ -236,7 +239,10 @@ int launch_gated_heads(const float* y, const float* gate, long long gate_stride,
     using TO = std::remove_pointer_t<decltype(to)>;
     if (part == 64) return root ? full(to, gated_heads_full_kernel<TO, 64, true>) : full(to, gated_heads_full_kernel<TO, 64, false>);
     if (part == 128) return root ? full(to, gated_heads_full_kernel<TO, 128, true>) : full(to, gated_heads_full_kernel<TO, 128, false>);
-    return root ? run(to, gated_heads_kernel<TO, 8, true>) : run(to, gated_heads_kernel<TO, 8, false>);
+    if (part <= 32) return root ? run(to, gated_heads_kernel<TO, 1, 4, true>) : run(to, gated_heads_kernel<TO, 1, 4, false>);
+    if (part < 64) return root ? run(to, gated_heads_kernel<TO, 2, 4, true>) : run(to, gated_heads_kernel<TO, 2, 4, false>);
+    if (part < 128) return root ? run(to, gated_heads_kernel<TO, 4, 4, true>) : run(to, gated_heads_kernel<TO, 4, 4, false>);
+    return root ? run(to, gated_heads_kernel<TO, 8, 2, true>) : run(to, gated_heads_kernel<TO, 8, 2, false>);
   };
   return out_dtype == IFX_DT_F32 ? with(static_cast<float*>(out)) : with(static_cast<__nv_bfloat16*>(out));
 }

@@ -152,3 +152,12 @@ def test_a_turned_latent_has_its_bits_wherever_it_lies(cuda_kernels, rot, used, 
                                                  SimpleNamespace(kv=kv, block_table=table, writes=True, page_size=page))
         results.append((turned, kv))
     assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
+@pytest.mark.parametrize("T,groups,part", [(3, 9, 1), (5, 9, 20), (700, 40, 31), (700, 40, 32), (700, 40, 33), (41, 7, 63), (600, 40, 65), (600, 40, 127),
+                                           (9, 3, 129), (2100, 10, 200), (2100, 10, 255), (4, 40, 16)])
+@pytest.mark.parametrize("gate_first", [False, True])
+def test_norm_and_gate_of_parts_of_any_size(cuda_kernels, T, groups, part, gate_first):
+    """Sizes around those for which a lane has room; few rows, and so many that a warp takes several parts."""
+    test_norm_and_gate(cuda_kernels, torch.bfloat16, T, groups, part, gate_first, "silu", 1)
+    test_norm_and_gate(cuda_kernels, torch.float32, T, groups, part, gate_first, "sigmoid", 0)
