@@ -192,7 +192,8 @@ __device__ __forceinline__ void route_token_small(const float* z_s, const float*
 // at a time and add up in the order of the warps, so a token's logits depend on nothing else in the step.  A lane reads 16 bytes of a
 // row, of which it feeds the first half to one mma.sync of 16 and the second to the next: both operands are permuted alike.
 // Bound: latency (the rows' reads, then the choice).  Library product (with its own sum of slices for 18 outputs) and the kernel above -> this,
-// us: 24 tokens of 1,536 to 16 outputs 7.2 -> 3.4; 2,048 to 18 12.4 -> 4.1.
+// us: 24 tokens of 1,536 to 16 outputs 7.2 -> 3.4; 2,048 to 18 12.4 -> 4.1.  More tokens than run at once, and long routers of more than 32
+// outputs, are faster by the library (CudaKernels._one_launch_router).
 constexpr int kRouterMost = 64, kRouterAhead = 3;
 template <int NT>
 struct RouterWarps { static constexpr int N = NT <= 4 ? 16 : 8; };      // (shared memory)

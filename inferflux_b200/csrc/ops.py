@@ -1724,10 +1724,25 @@ class CudaKernels:
         self.launches += 1
         return ids, weights
 
+    @staticmethod
+    def _one_launch_router(T, K, n):
+        """Whether router and choice in one launch take less than the library's product and the choice behind it.  The kernel has 16 tokens
+        a block, so up to 2,368 tokens run at once, and each block reads the whole router; the library is slow for outputs that are no
+        multiple of eight.  Up to 2,368 tokens the router's sizes alone decide, so that a token's choice depends on nothing else in the step.
+        us, the two ways: 16 outputs, 24 tokens of 1,536 7.2 / 3.4, 4,096 of 2,880 11.8 / 9.1, 8,192 of 7,168 30.7 / 48.7; 24, 2,368 of 3,584
+        10.4 / 9.0, 2,369 10.4 / 13.8, 24 of 7,168 13.3 / 11.3 (but 2 to 16 of them 8.8 / 10.4: the library has a kernel for those); 20, 4,096
+        of 3,584 22.2 / 15.5; 64, 64 of 768 6.6 / 5.5, of 1,536 7.6 / 7.5, of 2,048 8.1 / 9.3, of 7,168 14.0 / 22.9; 33, 64 of 2,048 10.0 / 8.8,
+        of 7,168 13.0 / 19.9."""
+        odd = n % 8 != 0
+        if T <= 2368:
+            return n <= 32 or (n <= 64 and K <= (2048 if odd else 1536))
+        return T <= 4736 and (n <= 8 or (n <= 16 and (odd or K <= 3072)) or (n <= 32 and (odd or K <= 512)))
+
     def moe_choose(self, h, w_router, correction, top, of_chosen=False, kind=None, floor=0.0):
-        """`moe_route` of the router's logits h . w_router^T.  A bfloat16 router of up to 64 outputs takes one launch for both."""
+        """`moe_route` of the router's logits h . w_router^T.  A bfloat16 router of up to 64 outputs takes one launch for both where that
+        takes less."""
         n = w_router.shape[0]
-        if not (h.dtype == w_router.dtype == torch.bfloat16 and n <= 64 and h.is_contiguous() and w_router.is_contiguous()
+        if not (h.dtype == w_router.dtype == torch.bfloat16 and self._one_launch_router(*h.shape, n) and h.is_contiguous() and w_router.is_contiguous()
                 and h.shape[1] == w_router.shape[1] and h.shape[1] % 8 == 0 and (h.data_ptr() | w_router.data_ptr()) % 16 == 0):
             return self.moe_route(self.linear(h, w_router, out_dtype=torch.float32), correction, top, of_chosen=of_chosen, kind=kind, floor=floor)
         _need(kind in (None, "sigmoid_normalized"), f"moe_choose: unknown kind {kind!r}")
