@@ -128,10 +128,11 @@ __global__ void rope_append_kernel(const T* __restrict__ qkv, const float* __res
 // all its heads, so they are computed once into shared memory, by as many threads as there are angles; then every thread moves 8 + 8
 // elements (a 16-byte chunk and its rotation partner half a head away) of every token per step.  Takes the common case only:
 // bfloat16 activations (not partial sums), whole-head split-half rotation, head sizes that are multiples of 16.
-// Bound: HBM, and the chains position -> angles and token -> slot -> page.  Eight layers of 1,531 tokens, 12 + 4 heads of 128: 52.5 us with a token a
-// block, 57.6 with a programmatic launch, 48.9 with two tokens, 71.5 with four (registers).
-template <int TOKENS>
-__global__ void __launch_bounds__(TOKENS > 1 ? 512 : 1024)
+// Bound: HBM, and the chains position -> angles and token -> slot -> page, which different warps follow (by one warp after each other they
+// took 5 % of a step of prompts' rotations and 20 % where an SM holds one block).  Eight layers of 1,531 tokens, 12 + 4 heads of 128: 52.5 us with a
+// token a block, 57.6 with a programmatic launch (EARLY) too, 48.9 with two tokens, 71.5 with four (registers).
+template <int TOKENS, bool EARLY>
+__global__ void __launch_bounds__(1024)
 rope_append_rows_kernel(const __nv_bfloat16* __restrict__ qkv, const float* __restrict__ bias,
                         const float* __restrict__ inv_freq, const int* __restrict__ positions,
                         const int* __restrict__ token_req, const int* __restrict__ req_slot,
@@ -140,8 +141,10 @@ rope_append_rows_kernel(const __nv_bfloat16* __restrict__ qkv, const float* __re
                         int write_cache, int num_tokens) {
   __shared__ float cs[TOKENS][128], sn[TOKENS][128];    // d / 2 <= 128
   __shared__ long long page_base[TOKENS];               // < 0: no page
-  pdl_launch_dependents();
-  pdl_wait();
+  if (EARLY) {
+    pdl_launch_dependents();
+    pdl_wait();
+  }
   const int t0 = blockIdx.x * TOKENS, tokens = min(TOKENS, num_tokens - t0);
   const int half = d / 2;
   const int width = (nq + 2 * nkv) * d;
@@ -167,14 +170,15 @@ rope_append_rows_kernel(const __nv_bfloat16* __restrict__ qkv, const float* __re
     const int k = j / half, a = j - k * half;
     sincosf((float)positions[t0 + k] * inv_freq[a], &sn[k][a], &cs[k][a]);
   }
-  if ((int)threadIdx.x < tokens) {
+  const int last = (int)(blockDim.x - 1 - threadIdx.x);    // (not the warps that make angles, if there are others)
+  if (last < tokens) {
     long long base = -1;
     if (write_cache) {
-      const int t = t0 + threadIdx.x, pos = positions[t], slot = req_slot[token_req[t]];
+      const int t = t0 + last, pos = positions[t], slot = req_slot[token_req[t]];
       const int page = block_table[(size_t)slot * max_blocks + pos / page_size];
       if (page >= 0 && page < num_pages) base = (long long)page * 2 * nkv * page_size * d + (long long)(pos % page_size) * d;
     }
-    page_base[threadIdx.x] = base;
+    page_base[last] = base;
   }
   __syncthreads();
   for (; it < items; it += blockDim.x) {
@@ -351,12 +355,32 @@ extern "C" int ifx_rope_append(const void* qkv, const float* qkv_partial, int nu
       (bias == nullptr || reinterpret_cast<uintptr_t>(bias) % 16 == 0)) {
     const int items = (nq + 2 * nkv) * (d / 16);
     const int threads = items >= 1024 ? 1024 : (items + 31) / 32 * 32;
+    const dim3 block(threads);
     auto run = [&](auto kern, int tokens) {
-      return launch_pdl(kern, dim3((num_tokens + tokens - 1) / tokens), dim3(threads), 0, stream, 1, (const __nv_bfloat16*)qkv, bias, inv_freq,
+      return launch_pdl(kern, dim3((num_tokens + tokens - 1) / tokens), block, 0, stream, 1, (const __nv_bfloat16*)qkv, bias, inv_freq,
                         positions, token_req, req_slot, block_table, max_blocks, page_size, num_pages, (__nv_bfloat16*)kv_pool,
                         (__nv_bfloat16*)q_out, nq, nkv, d, write_cache, num_tokens);
     };
-    return num_tokens >= 4 * 148 && threads <= 512 ? run(rope_append_rows_kernel<2>, 2) : run(rope_append_rows_kernel<1>, 1);
+    // More than 512 threads, one block an SM: nothing starts early, and waiting for it costs 4 %.  us, a token a block and two: 64 + 16 heads
+    // of 128, 592 tokens 9.0 and 7.1, 2,048 30.1 and 22.4, 8,192 133 and 97; 40 + 80 heads 2,048 43.3 and 34.2.
+    if (threads > 512) {
+      auto plain = [&](auto kern, int tokens) {
+        kern<<<(num_tokens + tokens - 1) / tokens, block, 0, stream>>>(
+            (const __nv_bfloat16*)qkv, bias, inv_freq, positions, token_req, req_slot, block_table, max_blocks, page_size, num_pages,
+            (__nv_bfloat16*)kv_pool, (__nv_bfloat16*)q_out, nq, nkv, d, write_cache, num_tokens);
+        const cudaError_t e = cudaGetLastError();
+        return e == cudaSuccess ? 0 : (int)e;
+      };
+      return num_tokens > 148 ? plain(rope_append_rows_kernel<2, false>, 2) : plain(rope_append_rows_kernel<1, false>, 1);
+    }
+    // Rounds of blocks (an SM holds as many as their 56 or 64 registers a thread let it): one with two tokens a block takes a third longer and
+    // more.  us, one and two: 16 heads of 128, 1,000 tokens 3.1 and 3.7, 2,048 4.9 and 4.7, 8,192 14.9 and 14.0; 36 heads 1,000 5.1 and 5.8,
+    // 2,048 9.1 and 8.7; 48 of 64, 1,000 4.5 and 4.1; 24 of 256, 592 4.7 and 4.0, 2,048 12.0 and 12.4.
+    auto rounds = [&](int registers, int tokens) {
+      const int at_once = 148 * tokens * (65536 / (registers * threads));
+      return (num_tokens + at_once - 1) / at_once;
+    };
+    return 4 * rounds(64, 2) < 3 * rounds(56, 1) ? run(rope_append_rows_kernel<2, true>, 2) : run(rope_append_rows_kernel<1, true>, 1);
   }
   dim3 grid(num_tokens, nq + 2 * nkv);
   int threads = d / 2 >= 64 ? 64 : 32;

@@ -161,3 +161,33 @@ def test_norm_and_gate_of_parts_of_any_size(cuda_kernels, T, groups, part, gate_
     """Sizes around those for which a lane has room; few rows, and so many that a warp takes several parts."""
     test_norm_and_gate(cuda_kernels, torch.bfloat16, T, groups, part, gate_first, "silu", 1)
     test_norm_and_gate(cuda_kernels, torch.float32, T, groups, part, gate_first, "sigmoid", 0)
+
+
+@pytest.mark.parametrize("nq,nkv,d,T", [(64, 8, 128, 149), (40, 40, 128, 301), (65, 31, 128, 300), (12, 2, 128, 1333), (12, 2, 128, 2369), (28, 4, 128, 1777),
+                                        (8, 8, 256, 593), (1, 1, 16, 9500)])
+def test_turned_rows_have_their_bits_in_steps_of_any_size(cuda_kernels, nq, nkv, d, T):
+    """One token a block and two, rows of one block an SM and of several: as in steps of 100 tokens, where every block has one."""
+    from types import SimpleNamespace
+    g = torch.Generator().manual_seed(T)
+    qkv = torch.randn(T, (nq + 2 * nkv) * d, generator=g).to(torch.bfloat16).to(DEV)
+    bias = torch.randn((nq + 2 * nkv) * d, generator=g).to(DEV)
+    rotary = SimpleNamespace(rotary_dim=d, interleaved=False, magnitude=1.0, inv_freq=torch.rand(d // 2, generator=g).to(DEV))
+    pages = -(-(T + 5) // 16)
+    results = []
+    for step in (T, 100):
+        kv = torch.zeros(pages + 3, 2, nkv, 16, d, dtype=torch.bfloat16, device=DEV)
+        table = torch.randperm(pages, generator=torch.Generator().manual_seed(1)).to(torch.int32).view(1, -1).to(DEV)
+        cache = SimpleNamespace(kv=kv, block_table=table, writes=True, page_size=16)
+        out = []
+        for t0 in range(0, T, step):
+            ctx = _Ctx([(5 + t0, min(step, T - t0))], [0], DEV)
+            ctx.extra_len = {"attn.prefill_tiles": 4, "attn.decode_rows": 0}
+            out.append(cuda_kernels.rope_append(qkv[t0:t0 + step], bias, rotary, nq, nkv, d, ctx, cache))
+        results.append((torch.cat(out), kv))
+    if T % 100 >= 64 or T % 100 == 0:
+        assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+    else:                                                    # (fewer than 64 tokens: another kernel, with its own order of roundings)
+        n = T - T % 100
+        assert torch.equal(results[0][0][:n], results[1][0][:n])
+        assert float((results[0][0].float() - results[1][0].float()).abs().max()) <= 2.0 ** -5
+        assert float((results[0][1].float() - results[1][1].float()).abs().max()) <= 2.0 ** -5
