@@ -544,7 +544,9 @@ int ifx_silu_columns(const float* rows, const float* partial, int splits, long l
   const int rc = make_source(&src, rows, IFX_DT_F32, partial, splits, num_tokens, ld, col0);
   if (rc) return rc;
   const int stop = in_place ? acted : width;
-  if (partial == nullptr && num_tokens >= 128 && stop > 0 && ((long long)width | acted | col0 | ld) % 4 == 0 && ((uintptr_t)rows | (uintptr_t)out) % 16 == 0)
+  // (a block of the kernel for 16-byte reads does four times as much: with few of them the SMs idle.  us, by the other and by it: 200 rows of
+  // 4,608 columns 3.5 and 4.6, 600 7.6 and 7.7, 2,048 22.3 and 18.2; 600 of 1,024 2.7 and 2.9, 2,048 6.2 and 5.4)
+  if (partial == nullptr && num_tokens >= 128 && stop > 0 && (stop <= 512 || (long long)num_tokens * ((stop + 2047) / 2048) >= 1536) && ((long long)width | acted | col0 | ld) % 4 == 0 && ((uintptr_t)rows | (uintptr_t)out) % 16 == 0)
     return launch_pdl(silu_columns_vec_kernel, dim3(num_tokens, (stop + 2047) / 2048), dim3(128), 0, stream, 1, rows + col0, (size_t)ld, out, width,
                       acted, stop);
   int blocks = (stop + 511) / 512;
