@@ -66,15 +66,18 @@ __global__ void short_conv_kernel(const T* __restrict__ h, const float* __restri
 // The same for up to 4 taps and channel counts that are multiples of 16 bytes' worth of elements: a thread owns
 // VEC consecutive channels (one 16-byte load per input row) and, in steps of many tokens, walks up to kConvRows
 // consecutive tokens, so that the chain of metadata loads (token -> request -> span and slot) is paid once per
-// request a block meets and a token's earlier inputs stay in registers for the next token.  Bound: HBM, and the latency of
-// the reads (1,500 tokens of 1,792 float32 channels: 15.5 us with a token's read behind the token before, so 14.3).
+// request a block meets and a token's earlier inputs stay in registers for the next token.  Bound: the latency of the reads, then HBM.
+// Four taps come by 16 bytes (one by one: 16 or 32 reads of a lane's own lines).  us, before and so: 1,792 float32 channels, 300 tokens 9.1
+// and 5.9, 2,048 13.5 and 10.4; 3,072 bfloat16 channels 300 tokens 23.7 and 12.2, 2,048 33.9 and 23.5.  All of a block's rows on their way
+// before the first is worked on, blocks of 128: 11.1 and 29.3 for 2,048 tokens, and slower with two or three taps; not kept.
 constexpr int kConvRows = 8;
 
 template <typename T> struct ConvVec;
 template <> struct ConvVec<float> {
   static constexpr int N = 4;
-  static __device__ __forceinline__ void spread(const uint4& raw, float (&v)[4]) {
-    v[0] = __uint_as_float(raw.x); v[1] = __uint_as_float(raw.y); v[2] = __uint_as_float(raw.z); v[3] = __uint_as_float(raw.w);
+  static __device__ __forceinline__ void load(const float* p, float (&v)[4]) {
+    const float4 a = *reinterpret_cast<const float4*>(p);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
   }
   static __device__ __forceinline__ void store(float* p, const float (&v)[4]) {
     *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
@@ -82,7 +85,8 @@ template <> struct ConvVec<float> {
 };
 template <> struct ConvVec<__nv_bfloat16> {
   static constexpr int N = 8;
-  static __device__ __forceinline__ void spread(const uint4& raw, float (&v)[8]) {
+  static __device__ __forceinline__ void load(const __nv_bfloat16* p, float (&v)[8]) {
+    const uint4 raw = *reinterpret_cast<const uint4*>(p);
     const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -100,7 +104,7 @@ template <> struct ConvVec<__nv_bfloat16> {
 };
 
 template <typename T>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 4) short_conv_vec_kernel(
+__global__ void __launch_bounds__(256) short_conv_vec_kernel(
     const T* __restrict__ h, const float* __restrict__ w, float* __restrict__ state, long long state_slot_stride,
     const int* __restrict__ token_req, const int* __restrict__ req_slot, const int* __restrict__ cu_seqlens,
     T* __restrict__ out, int num_tokens, int channels, int taps, int inline_single, int rows_per_block,
@@ -109,26 +113,24 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 4) short_conv_vec_ke
   const int c0 = (blockIdx.y * blockDim.x + threadIdx.x) * V;
   if (c0 >= channels) return;
   float wr[V][4];                                        // wr[v][k]: the tap of the input k steps back
+  if (taps == 4 && (uintptr_t)w % 16 == 0) {             // (a number at a time 16 or 32 reads of a lane's own lines)
 #pragma unroll
-  for (int v = 0; v < V; ++v)
-#pragma unroll
-    for (int k = 0; k < 4; ++k) wr[v][k] = k < taps ? w[(size_t)(c0 + v) * taps + (taps - 1 - k)] : 0.0f;
-  const int t0 = blockIdx.x * rows_per_block, t_end = min(num_tokens, t0 + rows_per_block);
-  uint4 raw[kConvRows];                                  // all rows and their requests are on their way before the first is worked on
-  int req[kConvRows];
-#pragma unroll
-  for (int j = 0; j < kConvRows; ++j)
-    if (t0 + j < t_end) {
-      raw[j] = *reinterpret_cast<const uint4*>(h + (size_t)(t0 + j) * in_stride + c0);
-      req[j] = token_req[t0 + j];
+    for (int v = 0; v < V; ++v) {
+      const float4 f = reinterpret_cast<const float4*>(w)[c0 + v];
+      wr[v][0] = f.w; wr[v][1] = f.z; wr[v][2] = f.y; wr[v][3] = f.x;
     }
+  } else {
+#pragma unroll
+    for (int v = 0; v < V; ++v)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) wr[v][k] = k < taps ? w[(size_t)(c0 + v) * taps + (taps - 1 - k)] : 0.0f;
+  }
+  const int t_end = min(num_tokens, (int)(blockIdx.x + 1) * rows_per_block);
   int r_at = -1, first = 0, n = 0;
   float* st = nullptr;
   float in[4][V];                                        // in[k]: the input k steps back
-#pragma unroll
-  for (int j = 0; j < kConvRows; ++j) {
-    const int t = t0 + j, r = req[j];
-    if (t >= t_end) break;
+  for (int t = blockIdx.x * rows_per_block; t < t_end; ++t) {
+    const int r = token_req[t];
     const bool carry = r == r_at;                        // the token before is this request's too: its inputs are in registers
     if (!carry) {
       r_at = r;
@@ -143,12 +145,12 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 4) short_conv_vec_ke
 #pragma unroll
         for (int v = 0; v < V; ++v) in[k][v] = in[k - 1][v];
     }
-    ConvVec<T>::spread(raw[j], in[0]);
+    ConvVec<T>::load(h + (size_t)t * in_stride + c0, in[0]);
 #pragma unroll
     for (int k = 1; k < 4; ++k) {
       if (k < taps && !carry) {
         if (k <= i) {
-          ConvVec<T>::spread(*reinterpret_cast<const uint4*>(h + (size_t)(t - k) * in_stride + c0), in[k]);
+          ConvVec<T>::load(h + (size_t)(t - k) * in_stride + c0, in[k]);
         } else {
           const float* cell = st + (size_t)((taps - 1) - (k - i)) * channels + c0;
 #pragma unroll
@@ -232,7 +234,7 @@ int ifx_short_conv_ex(const void* h, long long in_stride, const float* w, const 
   const int vec = dtype == IFX_DT_F32 ? 4 : 8;
   const bool wide = taps <= 4 && channels % vec == 0 && in_stride % vec == 0 && ((uintptr_t)h % 16 == 0) && ((uintptr_t)out % 16 == 0) &&
                     (state == nullptr || ((uintptr_t)state % 16 == 0 && state_slot_stride % 4 == 0));
-  const int vthreads = channels / vec >= 128 ? 128 : ((channels / vec + 31) / 32) * 32;
+  const int vthreads = channels / vec >= 256 ? 256 : ((channels / vec + 31) / 32) * 32;
   const int rows_per_block = T >= 256 * kConvRows ? kConvRows : (T >= 256 ? T / 256 : 1);
   dim3 vgrid((unsigned)((T + rows_per_block - 1) / rows_per_block), wide ? (unsigned)((channels / vec + vthreads - 1) / vthreads) : 1u);
 #define IFX_LAUNCH(TT)                                                                                              \

@@ -191,3 +191,28 @@ def test_turned_rows_have_their_bits_in_steps_of_any_size(cuda_kernels, nq, nkv,
         assert torch.equal(results[0][0][:n], results[1][0][:n])
         assert float((results[0][0].float() - results[1][0].float()).abs().max()) <= 2.0 ** -5
         assert float((results[0][1].float() - results[1][1].float()).abs().max()) <= 2.0 ** -5
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("taps", [2, 3, 4])
+@pytest.mark.parametrize("lens", [(1, 3, 1), (300,), (2049, 17)])
+def test_a_convolution_has_its_bits_wherever_its_taps_lie(cuda_kernels, dtype, taps, lens):
+    """Taps on a 16-byte boundary, read whole where there are four, and off it."""
+    C, T = 264, sum(lens)
+    g = torch.Generator().manual_seed(T + taps)
+    x, w, st = torch.randn(T, C, generator=g).to(dtype).to(DEV), torch.randn(C, taps, generator=g).to(DEV), torch.randn(4, 1, taps - 1, C, generator=g)
+    off = torch.zeros(C * taps + 1, device=DEV)
+    off[1:] = w.reshape(-1)
+    results = []
+    for taken in (w, off[1:].view(C, taps)):
+        state = st.to(DEV)
+        out = cuda_kernels.short_conv(x, taken, taps, state, 0, _Ctx([(0, n) for n in lens], [2, 0, 3][:len(lens)], DEV))
+        results.append((out, state))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+    want = torch.zeros(T, C, dtype=F64)
+    at = 0
+    for n, slot in zip(lens, [2, 0, 3]):
+        rows = torch.cat([st[slot, 0].double(), x[at:at + n].double().cpu()])
+        want[at:at + n] = x[at:at + n].double().cpu() + sum(rows[k:k + n] * w.double().cpu()[:, k] for k in range(taps))
+        at += n
+    _close(results[0][0], want, dtype)
