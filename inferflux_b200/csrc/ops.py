@@ -955,11 +955,11 @@ class CudaKernels:
         walks the most keys is one of two query tiles.  Such a block takes an eighth longer a key tile, and the second tile's last keys
         and its output come behind the first one's, two thirds of a key tile.  Where a block of one query tile walks longer, nothing is
         gained, and the second query tiles that are not there, which are launched all the same and leave at once, cost up to 4 us.
-        us, 256 and 128 rows a block: 12 heads, 447 tokens 14.9 and 13.3, 1,000 21.5 and 19.5, with four of 50 beside 22.0 and 20.0, four
-        times 256 behind 700 23.1 and 20.5; 28 heads, 300 behind 500 19.5 and 18.9, 640 behind 1,500 37.9 and 34.3; heads of 64, 16 of
-        them, 1,000 tokens 20.5 and 17.4; and those that stay: 12 heads, 300 tokens 11.0 and 11.8, four times 300 12.6 and 13.8, twelve times
-        100 10.2 and 13.8, behind 700 19.5 and 23.1.  With more blocks than SMs: 1,000 of 28 heads behind 2,000 51.7 and 72.2, 3,500 of 12
-        57.4 and 67.6 (the last blocks of 2,000 of 12 alone are long enough to gain, 35.9 and 32.3, and are left)."""
+        us, 256 and 128 rows a block: 12 heads, 447 tokens 13.3 and 11.8, 1,000 20.0 and 18.2, with four of 50 beside 20.0 and 18.4, four
+        times 256 behind 700 20.7 and 18.7; 28 heads, 300 behind 500 17.4 and 17.1, 640 behind 1,500 35.1 and 32.8; heads of 64, 16 of
+        them, 1,000 tokens 19.2 and 15.9; and those that stay: 12 heads, 300 tokens 10.2 and 10.2, four times 300 10.8 and 12.0, twelve times
+        100 8.6 and 11.8, behind 700 17.4 and 21.3.  With more blocks than SMs: 1,000 of 28 heads behind 2,000 48.4 and 68.6, 3,500 of 12
+        55.0 and 65.0 (the last blocks of 2,000 of 12 alone are long enough to gain, 33.9 and 31.0, and are left)."""
         tiles = two = one = 0                              # 128-row tiles; keys to the end of the longest item of two tiles, and of one
         for s, n in ctx.spans:
             if n > 1:
