@@ -401,10 +401,10 @@ __global__ void __launch_bounds__(256) chunk_local_kernel(const ChunkArgs a) {
 
 // grid (requests, heads, pieces of a state): four key channels of a value channel a thread.  The reads of eight stretches are
 // on their way together; only the multiply-adds are in sequence.
-template <bool CHANNEL>
+template <bool CHANNEL, int PER>
 __global__ void __launch_bounds__(256) chunk_carry_kernel(const ChunkArgs a, int dk) {
   const int r = blockIdx.x, h = blockIdx.y, e = blockIdx.z * 256 + threadIdx.x;
-  const int lo = a.cu_seqlens[r], span = a.cu_seqlens[r + 1] - lo, chunks = chunks_of(span, a.min_span, a.per);
+  const int lo = a.cu_seqlens[r], span = a.cu_seqlens[r + 1] - lo, chunks = chunks_of(span, a.min_span, PER);
   if (chunks == 0) return;
   if (a.x != nullptr && h == 0 && blockIdx.z == 0) {                       // the step's last input row
     float* to = a.prev_state + (long long)a.req_slot[r] * a.state_slot_stride;
@@ -416,7 +416,7 @@ __global__ void __launch_bounds__(256) chunk_carry_kernel(const ChunkArgs a, int
   float4 S;
   if (a.key_rows) S = make_float4(st[(size_t)c * a.dv + v], st[(size_t)(c + 1) * a.dv + v], st[(size_t)(c + 2) * a.dv + v], st[(size_t)(c + 3) * a.dv + v]);
   else S = make_float4(st[(size_t)v * dk + c], st[(size_t)v * dk + c + 1], st[(size_t)v * dk + c + 2], st[(size_t)v * dk + c + 3]);
-  const size_t base = (size_t)chunks_before(a.cu_seqlens, a.min_span, r, a.per) * a.heads + h;
+  const size_t base = (size_t)chunks_before(a.cu_seqlens, a.min_span, r, PER) * a.heads + h;
   constexpr int U = 8;
   for (int c0 = 0; c0 < chunks; c0 += U) {
     float4 add[U], w[U];
@@ -556,16 +556,17 @@ static int launch_chunks(const ChunkArgs& a, int chunks, cudaStream_t stream) {
   const dim3 grid(chunks, a.heads, a.dv / 64);
   local<<<grid, 256, L::BYTES, stream>>>(a);
   IFX_CHECK_LAUNCH();
-  chunk_carry_kernel<L::CHANNEL><<<dim3(a.requests, a.heads, (a.dv * (DK / 4) + 255) / 256), 256, 0, stream>>>(a, DK);
+  chunk_carry_kernel<L::CHANNEL, kChunk><<<dim3(a.requests, a.heads, (a.dv * (DK / 4) + 255) / 256), 256, 0, stream>>>(a, DK);
   IFX_CHECK_LAUNCH();
   reach<<<grid, 256, reach_bytes, stream>>>(a);
   IFX_CHECK_LAUNCH();
   return 0;
 }
 
-// The states in front of every stretch, for chunk_tcgen05.cu's stretches.
+// The states in front of every stretch, for chunk_tcgen05.cu's stretches.  (Their size is a constant of the kernel: every block counts the
+// stretches of the requests in front of its own, and with a division by a variable 32 requests took 3 to 5 % longer.)
 int launch_chunk_carry(const ChunkArgs& a, int dk, cudaStream_t stream) {
-  chunk_carry_kernel<false><<<dim3(a.requests, a.heads, (a.dv * (dk / 4) + 255) / 256), 256, 0, stream>>>(a, dk);
+  chunk_carry_kernel<false, 128><<<dim3(a.requests, a.heads, (a.dv * (dk / 4) + 255) / 256), 256, 0, stream>>>(a, dk);
   IFX_CHECK_LAUNCH();
   return 0;
 }
@@ -624,8 +625,9 @@ long long ifx_chunk_scan_scratch_floats(int num_tokens, int requests, int min_sp
 }
 
 // Whether a decay per head goes by stretches of 128 tokens (chunk_tcgen05.cu) where they take the sizes: when the blocks of the stretches of
-// 64 would not all have an SM of their own.  us, by 64 and by 128: 12 heads of 128 x 128, one span of 300 tokens 31 / 34, 512 43 / 35,
-// 2,048 120 / 62; 12 of 64 x 128 22 / 27, 29 / 27, 69 / 47; 24 of 128 x 64 31 / 31, 44 / 31, 115 / 78; 28 of 128 x 128, 128 tokens 44 / 35.
+// 64 would not all have an SM of their own.  us, by 64 and by 128: 12 heads of 128 x 128, one span of 300 tokens 30 / 35, 512 43 / 36,
+// 2,048 119 / 64; 12 of 64 x 128 22 / 28, 29 / 29, 69 / 49; 24 of 128 x 64 31 / 32, 44 / 33, 115 / 67; 28 of 128 x 128, 128 tokens 44 / 36; but 56
+// of 128 x 64, 256 tokens 45.5 / 47.0.
 int ifx_chunk_scan_takes_128(int num_tokens, int num_requests, int min_span, int heads, int dv) {
   return (long long)chunks_at_most(num_tokens, num_requests, min_span) * heads * (dv / 64) > 148;
 }
@@ -655,7 +657,6 @@ int ifx_chunk_decay_scan(const float* q, long long q_stride, const float* k, lon
   a.requests = num_requests; a.min_span = min_span; a.heads = heads; a.groups = groups; a.dv = dv;
   a.inv_tau = mode == 0 ? 1.0f / tau : 0.0f;
   a.q_scale = q_scale;
-  a.per = per;
   a.local = scratch;
   a.total = scratch + (size_t)chunks * heads * dv * dk;
   a.reach = a.total + ((mode == 0 ? (size_t)chunks * heads * dk : (size_t)2 * chunks * heads) + 3) / 4 * 4;
@@ -680,7 +681,6 @@ int ifx_chunk_wkv_scan(const float* r, const float* k, const float* v, const flo
   a.w0 = w0; a.u = u; a.x = x; a.prev_state = prev_state; a.C = C;
   a.requests = num_requests; a.min_span = min_span; a.heads = heads; a.groups = heads; a.dv = dim;
   a.q_scale = 1.0f;
-  a.per = kChunk;
   a.key_rows = 1;
   a.local = scratch;
   a.total = scratch + (size_t)chunks * heads * dim * dim;

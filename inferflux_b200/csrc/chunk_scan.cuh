@@ -158,7 +158,6 @@ struct ChunkArgs {
   float* total;                                 // decays of a whole stretch: [stretches, heads, dk], or [stretches, heads] as two numbers each
   float* reach;                                 // queries times decays since the stretch's beginning [T, heads dk], or decays [T, heads]
   int key_rows;                                 // the request's state is [head, key channel, value channel]
-  int per;                                      // tokens of a stretch
   const float* x; float* prev_state; int C;     // CHUNK_WKV: the step's input rows, where the last one of a request goes
 };
 
