@@ -1550,6 +1550,11 @@ class CudaKernels:
 
     stretch = 0                # tokens of a stretch of a decay per head: 64, 128, or 0 for the kernels' own rule
 
+    def _stretch_beside(self, ctx, heads, dv):
+        """The same where short spans go through the scan: the kernels' rule (ifx_chunk_scan_takes_128), which knows a step's tokens alone, of
+        the long spans' stretches.  us, 24 heads of 128 x 64, 300 tokens beside eight spans of 100: 171 by 64, 180 by 128."""
+        return 128 if self._long_spans(ctx)[4] * heads * (dv // 64) > 148 else 64
+
     def _scans_by_chunks(self, dtype, ctx, heads, dk, dv, *rows, constant=False):
         """Which of a recurrence's spans go by stretches of tokens: False, none; else (the fewest tokens of one that does, the most
         tokens of one that does not or 0).  Where that pays, with sizes the kernels are made for, rows on 16-byte boundaries (those
@@ -1951,9 +1956,10 @@ class CudaKernels:
             least, short = by_chunks
             room = torch.empty(int(self.lib.ifx_chunk_scan_scratch_floats(T, ctx.num_requests, least, heads, dk, dv, int(mode == 0))),
                                dtype=torch.float32, device=q.device)
+            stretch = self.stretch or (self._stretch_beside(ctx, heads, dv) if short else 0)
             rc = self.lib.ifx_chunk_decay_scan(*rows, ctx.num_requests, T, least, int(heads), int(groups), int(dk), int(dv), mode,
                                                float(tau), float(q_scale), room, rate,
-                                               self.stretch, self.error_flag, _stream())
+                                               stretch, self.error_flag, _stream())
             if rc != _MISALIGNED:
                 _check(rc, "decay_scan (stretches)")
                 self.launches += 3
