@@ -218,6 +218,13 @@ __global__ void __launch_bounds__(RouterWarps<NT>::N * 32) moe_choose_kernel(con
     }
   };
   fetch_w(warp);                                           // (weights do not come from the kernel in front)
+  if (gridDim.x <= 8)                                      // the other rounds' weights on their way into L2: behind a step's experts they
+    for (int u = warp + kRouterAhead * kRouterWarps; u < units; u += kRouterWarps) {      // are in DRAM, and few blocks wait for them in turn
+      const int k = column(u);
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+        if (k < K && j * 8 + row < n) asm volatile("prefetch.global.L2 [%0];" ::"l"(w + (size_t)(j * 8 + row) * K + k));
+    }
   pdl_launch_dependents();
   pdl_wait();
   float acc[NT][4];

@@ -1737,7 +1737,8 @@ class CudaKernels:
         us, the two ways: 16 outputs, 24 tokens of 1,536 7.2 / 3.4, 4,096 of 2,880 11.8 / 9.1, 8,192 of 7,168 30.7 / 48.7; 24, 2,368 of 3,584
         10.4 / 9.0, 2,369 10.4 / 13.8, 24 of 7,168 13.3 / 11.3 (but 2 to 16 of them 8.8 / 10.4: the library has a kernel for those); 20, 4,096
         of 3,584 22.2 / 15.5; 64, 64 of 768 6.6 / 5.5, of 1,536 7.6 / 7.5, of 2,048 8.1 / 9.3, of 7,168 14.0 / 22.9; 33, 64 of 2,048 10.0 / 8.8,
-        of 7,168 13.0 / 19.9."""
+        of 7,168 13.0 / 19.9.  (Router in L2.  Behind experts that push it out, layers of 18 outputs of 3,584 and up to 16 tokens take 1 % longer in one
+        launch, 149.4 / 150.8, all others less or the same: 24 tokens 189.9 / 187.5, 16 outputs of 1,536 and 8 tokens 77.0 / 73.5.)"""
         odd = n % 8 != 0
         if T <= 2368:
             return n <= 32 or (n <= 64 and K <= (2048 if odd else 1536))
