@@ -28,9 +28,9 @@
 //
 // Bound: delta_local, one block of 16 warps an SM (200 KB of operands): operands are cut, multiplied and added up in phases that wait
 // for one another, and the substitution is a chain of four blocks.  2,048 tokens of 24 heads: 165.6 us with products by mma.sync, two
-// blocks of 8 warps an SM; 127.0 on tcgen05 (123.7 with six products of parts instead of eight).  On the way: the substitution of all 64 rows written out took 33,000 cycles (40 KB of
-// code, the instruction cache), one by one in a loop 11,000, by blocks of 16 with products behind them 4,000.  delta_rule.cu's three
-// kernels take 658 us there, these with the norm 193.
+// blocks of 8 warps an SM; 127.0 on tcgen05 (123.7 with six products of parts instead of eight).  On the way: the substitution of all
+// 64 rows written out took 33,000 cycles (40 KB of code, the instruction cache), one by one in a loop 11,000, by blocks of 16 with
+// products behind them 4,000.  delta_rule.cu's three kernels take 658 us there, these with the norm 193.
 // Error against 64 bits (2-norm, 2,048 tokens), products by mma.sync and these: state 5.43e-7 and 5.43e-7, outputs 5.10e-7 and 5.09e-7.
 // Scan and products by mma.sync: parameters where trained models have them 5.2e-7 and 4.6e-7, decays near one 1.76e-6 and 1.70e-6,
 // random ones 0.95e-7 and 1.00e-7.
